@@ -62,10 +62,12 @@ SIGNATURES: Dict[str, Tuple[object, List[object]]] = {
                                    _i, _i, _l, _i, _i, _f, _f, _p]),
     "dsa_latent_append": (_i, [_p, _p, _f, _p, _p, _p, _p, _p, _i, _l, _l, _i, _i, _i, _p]),
     "dsa_decode_prep": (_i, [_p, _p, _p, _p, _p, _p, _l] + [_p] * 12 + [_i, _i, _i, _l, _i, _f, _p]),
+    "dsa_prefill_latents": (_i, [_p, _l, _p, _l, _p, _l] + [_p] * 8 + [_l, _p, _p, _l, _l] + [_i] * 6 + [_f, _i, _p]),
+    "dsa_prefill_queries": (_i, [_p, _l, _l, _i, _p, _l, _p, _l] + [_p] * 7 + [_l] + [_i] * 8 + [_p]),
     "dsa_quantize_e4m3_rowwise": (_i, [_p, _p, _p, _l, _i, _f, _p]),
 }
 
-ABI_VERSION = 9
+ABI_VERSION = 10
 
 
 class DsaError(RuntimeError):

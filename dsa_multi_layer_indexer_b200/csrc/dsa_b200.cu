@@ -14,6 +14,7 @@
 #include "fused_decode.cuh"
 #include "indexer_scan.cuh"
 #include "peer_allreduce.cuh"
+#include "prefill_prep.cuh"
 #include "sparse_mla.cuh"
 #include "sparse_mla_tc.cuh"
 #include "topk_select.cuh"
@@ -1168,6 +1169,77 @@ int dsa_decode_prep(const void* iq_raw, const void* w_raw, const void* ik_raw, c
   const int items = n_index_heads + 2 + H;
   DSA_CUDA(launch_pdl(prep::decode_prep_kernel, dim3((items + 3) / 4, B), dim3(128), 0,
                       static_cast<cudaStream_t>(stream), p));
+  return DSA_OK;
+}
+
+// ------------------------------------------------------------------ full-sequence preparation
+int dsa_prefill_latents(const void* qa, int64_t qa_stride, const void* kv_a, int64_t kv_a_stride, const void* ik,
+                        int64_t ik_stride, const void* q_norm_w, const void* kv_norm_w, const void* mla_cos,
+                        const void* mla_sin, const void* idx_cos, const void* idx_sin, void* c_q, void* kv_out,
+                        int64_t kv_cap, void* ik_out, float* ik_scale, int64_t ik_cap, int64_t rows, int seq,
+                        int q_rank, int kv_rank, int rope_dim, int idx_dim, int interleave, float eps, int dtype,
+                        void* stream) {
+  DSA_REQUIRE(dtype == 0 || dtype == 1, "prefill latents: dtype must be 0 (fp32) or 1 (bf16)");
+  DSA_REQUIRE(rows > 0 && rows < (int64_t(1) << 31) && seq > 0 && rows % seq == 0, "prefill latents: bad rows / seq");
+  DSA_REQUIRE(!qa || (q_norm_w && c_q && q_rank > 0 && qa_stride >= q_rank), "prefill latents: bad query latent");
+  DSA_REQUIRE(!kv_a || (kv_norm_w && mla_cos && mla_sin && kv_out && kv_rank > 0 && rope_dim > 0 && rope_dim % 2 == 0 &&
+                        kv_a_stride >= kv_rank + rope_dim && kv_cap >= seq),
+              "prefill latents: bad latent rows");
+  DSA_REQUIRE(!ik || (idx_cos && idx_sin && ik_out && idx_dim > 0 && idx_dim % 2 == 0 && ik_stride >= idx_dim && ik_cap >= seq),
+              "prefill latents: bad index keys");
+  DSA_REQUIRE(!ik || !ik_scale || (dtype == 1 && idx_dim == DSA_INDEX_DIM && aligned16(ik_out)),
+              "prefill latents: e4m3 index keys need bf16 rows of %d", DSA_INDEX_DIM);
+  prep::LatentsParams p{};
+  p.qa = qa, p.kv_a = kv_a, p.ik = ik, p.q_norm_w = q_norm_w, p.kv_norm_w = kv_norm_w;
+  p.mla_cos = mla_cos, p.mla_sin = mla_sin, p.idx_cos = idx_cos, p.idx_sin = idx_sin;
+  p.c_q = c_q, p.kv_out = kv_out, p.ik_out = ik_out, p.ik_scale = ik_scale;
+  p.qa_stride = qa_stride, p.kv_a_stride = kv_a_stride, p.ik_stride = ik_stride, p.kv_cap = kv_cap, p.ik_cap = ik_cap;
+  p.rows = rows, p.seq = seq, p.q_rank = q_rank, p.kv_rank = kv_rank, p.rope_dim = rope_dim, p.idx_dim = idx_dim;
+  p.interleave = interleave, p.eps = eps;
+  const dim3 grid(unsigned((rows * 3 + prep::kLatentWarps - 1) / prep::kLatentWarps)), block(prep::kLatentWarps * 32);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dtype == 1) DSA_CUDA(launch_pdl(prep::prefill_latents_kernel<__nv_bfloat16>, grid, block, 0, st, p));
+  else DSA_CUDA(launch_pdl(prep::prefill_latents_kernel<float>, grid, block, 0, st, p));
+  return DSA_OK;
+}
+
+int dsa_prefill_queries(const void* q, int64_t q_stride, int64_t q_head_stride, int nope, const void* iq,
+                        int64_t iq_stride, const void* w, int64_t w_stride, const void* mla_cos, const void* mla_sin,
+                        const void* idx_cos, const void* idx_sin, void* q_full, void* index_q, float* index_w,
+                        int64_t rows, int seq, int H, int n_index_heads, int kv_rank, int rope_dim, int idx_dim,
+                        int interleave, int dtype, void* stream) {
+  DSA_REQUIRE(dtype == 0 || dtype == 1, "prefill queries: dtype must be 0 (fp32) or 1 (bf16)");
+  DSA_REQUIRE(rows > 0 && rows < (int64_t(1) << 31) && seq > 0 && rows % seq == 0, "prefill queries: bad rows / seq");
+  DSA_REQUIRE(q_full || iq, "prefill queries: nothing to do");
+  DSA_REQUIRE(!q_full || (q && mla_cos && mla_sin && H > 0 && nope >= 0 && kv_rank > 0 && rope_dim > 0 && rope_dim % 2 == 0 &&
+                          q_head_stride >= nope + rope_dim),
+              "prefill queries: bad attention query");
+  DSA_REQUIRE(!iq || (index_q && idx_cos && idx_sin && n_index_heads > 0 && idx_dim > 0 && idx_dim % 2 == 0 &&
+                      iq_stride >= int64_t(n_index_heads) * idx_dim),
+              "prefill queries: bad indexer query");
+  auto aligned8 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 7u) == 0; };
+  if (dtype == 1) {
+    DSA_REQUIRE(!q_full || (kv_rank == DSA_VALUE_DIM && rope_dim == DSA_LATENT_DIM - DSA_VALUE_DIM && aligned8(q) &&
+                            aligned16(q_full) && aligned8(mla_cos) && aligned8(mla_sin) && q_stride % 4 == 0 &&
+                            q_head_stride % 4 == 0 && nope % 4 == 0),
+                "prefill queries: bf16 needs the %d + 64 latent and 8-byte aligned rows", DSA_VALUE_DIM);
+    DSA_REQUIRE(!iq || (idx_dim == DSA_INDEX_DIM && w && index_w && aligned8(iq) && iq_stride % 4 == 0 && aligned16(index_q) &&
+                        aligned8(idx_cos) && aligned8(idx_sin)),
+                "prefill queries: bf16 needs %d-wide indexer heads, head weights and 8-byte aligned rows", DSA_INDEX_DIM);
+  } else {
+    DSA_REQUIRE(!iq || !index_w, "prefill queries: e4m3 indexer queries need bf16 operands");
+  }
+  prep::QueriesParams p{};
+  p.q = q, p.iq = iq, p.w = w, p.mla_cos = mla_cos, p.mla_sin = mla_sin, p.idx_cos = idx_cos, p.idx_sin = idx_sin;
+  p.q_full = q_full, p.index_q = index_q, p.index_w = index_w;
+  p.q_stride = q_stride, p.q_head_stride = q_head_stride, p.iq_stride = iq_stride, p.w_stride = w_stride, p.rows = rows;
+  p.seq = seq, p.H = H, p.Hidx = n_index_heads, p.nope = nope, p.kv_rank = kv_rank, p.rope_dim = rope_dim, p.idx_dim = idx_dim;
+  p.interleave = interleave;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dtype == 1)
+    DSA_CUDA(launch_pdl(prep::prefill_queries_bf16_kernel, dim3(unsigned(rows)), dim3(prep::kQueryWarps * 32), 0, st, p));
+  else
+    DSA_CUDA(launch_pdl(prep::prefill_queries_f32_kernel, dim3(unsigned(rows)), dim3(256), 0, st, p));
   return DSA_OK;
 }
 

@@ -99,6 +99,25 @@ class IndexerWorkspace:
             torch.full((n_seq, topk), -1, dtype=torch.int32, device=device))
 
 
+@dataclasses.dataclass
+class FullOperands:
+    """A full-sequence layer's operands of the scan and the attention (``DSALayer.full_operands``).
+
+    fused: ready for the kernels -- q [B*S,H,Dqk], kv [B,cap,Dqk], iq / iw / ik (/ ik_scale) of the FP8
+    scan (ik [B,cap,128] e4m3 bytes) or of the fp32 scan. Otherwise the torch tensors as computed."""
+
+    b: int
+    s: int
+    lens: torch.Tensor  # int32 [B*S]: causally visible keys of every row
+    fused: bool
+    q: Optional[torch.Tensor]
+    kv: Optional[torch.Tensor]
+    iq: Optional[torch.Tensor]
+    iw: Optional[torch.Tensor]
+    ik: Optional[torch.Tensor]
+    ik_scale: Optional[torch.Tensor]
+
+
 def _pad_heads(t: torch.Tensor, multiple: int) -> torch.Tensor:
     """Zero-pads dim 1 (heads) to a multiple; zero queries attend uniformly and
     are dropped by the caller (reference fused_decode.py:38-43)."""
@@ -249,33 +268,149 @@ class DSALayer(nn.Module):
                                  self.sm_scale, seq_lens, rows_per_seq=rows_per_seq)
         return out.to(q.dtype)
 
+    # ------------------------------------------------------------------ full sequence
+    def full_operands(self, x_norm, rope: RopeCaches, c_q=None, attention: bool = True, indexer: bool = True,
+                      cache: Optional["LayerDecodeCache"] = None) -> "FullOperands":
+        """Everything a full-sequence layer computes from x_norm [B,S,hidden] before its scan and its
+        attention, once for both. With a ``cache`` the latent rows and index keys are written to (and
+        read from) the first S rows of the cache."""
+        c = self.config
+        b, s, _ = x_norm.shape
+        if self._fused_full(x_norm) and (cache is None or (cache.k_scale is not None) == self._fast_path(x_norm)):
+            return self._full_operands_fused(x_norm, rope, c_q, attention, indexer, cache)
+        if c_q is None:
+            c_q = self.q_latent(x_norm)
+        q = kv = iq = ik = w = None
+        if attention or cache is not None:
+            q, kv = self._mla_qkv(x_norm, c_q, rope)
+            q = q.reshape(b * s, *q.shape[2:])
+        if indexer or cache is not None:
+            iq, ik, w = self._indexer_qkw(x_norm, c_q, rope)
+            iq, w = iq.reshape(b * s, *iq.shape[2:]), w.reshape(b * s, -1)
+        if cache is not None:
+            cache.kv[:, :s] = kv.to(cache.kv.dtype)
+            if cache.k_scale is not None:
+                ik8, sk = ops.quantize_e4m3_rowwise(ik.float().contiguous())
+                cache.index_k[:, :s] = ik8.view(torch.uint8)
+                cache.k_scale[:, :s] = sk
+            else:
+                cache.index_k[:, :s] = ik.float()
+        return FullOperands(b, s, self._causal_lens(b, s, x_norm.device), False, q, kv, iq, w, ik, None)
+
+    def _fused_full(self, t: torch.Tensor) -> bool:
+        """True when the fused full-sequence preparation applies: it has no autograd, and knows the
+        fp32 form of any geometry and the bf16 / e4m3 form of the production geometry."""
+        return (t.is_cuda and not torch.is_grad_enabled() and (t.dtype == torch.float32 or self._fast_path(t))
+                and self.q_a_proj.weight.dtype == t.dtype)
+
+    def _full_operands_fused(self, x_norm, rope, c_q, attention, indexer, cache) -> "FullOperands":
+        c = self.config
+        b, s, _ = x_norm.shape
+        rows, h, dev, dt = b * s, c.num_attention_heads, x_norm.device, x_norm.dtype
+        fp8 = self._fast_path(x_norm)
+        linear = torch.nn.functional.linear
+        x2 = x_norm.reshape(rows, -1)
+        if rope.mla_cos.dtype != dt:
+            rope = RopeCaches(*(t.to(dt) for t in (rope.mla_cos, rope.mla_sin, rope.idx_cos, rope.idx_sin)))
+        stacked = fp8 and self._stacked()
+        keep_kv, keep_ik = attention or cache is not None, indexer or cache is not None
+        # ---- what reads x_norm
+        qa = kv_a = ik_raw = kv = ik = ik_scale = None
+        if stacked and c_q is None and keep_kv and keep_ik:
+            qa, kv_a, ik_raw = linear(x2, self._wx).split([c.q_lora_rank, c.qk_head_dim, c.index_head_dim], dim=1)
+        else:
+            if c_q is None:
+                qa = self.q_a_proj(x2)
+            if keep_kv:
+                kv_a = self.kv_a_proj(x2)
+            if keep_ik:
+                ik_raw = self.index_k_proj(x2)
+        if qa is not None:
+            c_q = torch.empty(rows, c.q_lora_rank, dtype=dt, device=dev)
+        else:
+            c_q = c_q.reshape(rows, -1)
+        if cache is not None:
+            kv, ik, ik_scale = cache.kv, cache.index_k, cache.k_scale
+        else:
+            if keep_kv:
+                kv = torch.empty(b, s, c.qk_head_dim, dtype=dt, device=dev)
+            if keep_ik:
+                ik = torch.empty(b, s, c.index_head_dim, dtype=torch.uint8 if fp8 else dt, device=dev)
+                ik_scale = torch.empty(b, s, dtype=torch.float32, device=dev) if fp8 else None
+        il = c.indexer_rope_interleave
+        if qa is not None or keep_kv or keep_ik:
+            ops.prefill_latents(qa, kv_a, ik_raw, self.q_a_layernorm.weight, self.kv_a_layernorm.weight, rope, c_q, kv, ik,
+                                ik_scale, s, il, c.rms_norm_eps)
+        # ---- what reads c_q
+        nope, rd = c.qk_nope_head_dim, c.qk_rope_head_dim
+        q = iq_raw = w = q_full = iq = iw = None
+        if stacked and attention and indexer:
+            q, iq_raw, w = linear(c_q, self._wc).split(
+                [h * (nope + rd), c.index_n_heads * c.index_head_dim, c.index_n_heads], dim=1)
+        else:
+            if attention:
+                q = self.q_b_proj(c_q)
+            if indexer:
+                iq_raw, w = self.index_q_proj(c_q), self.index_weights_proj(c_q)
+        if attention:
+            q = q.unflatten(1, (h, nope + rd))
+            q_full = torch.empty(rows, h, c.qk_head_dim, dtype=dt, device=dev)
+            w_uk, _ = self._w_uk_uv()  # absorb W_UK into the query: the GEMM writes its columns of q_full in place
+            torch.bmm(q[:, :, :nope].transpose(0, 1), w_uk, out=q_full[:, :, :c.kv_lora_rank].transpose(0, 1))
+        if indexer:
+            iq = torch.empty(rows, c.index_n_heads, c.index_head_dim, dtype=torch.uint8 if fp8 else dt, device=dev)
+            iw = torch.empty(rows, c.index_n_heads, dtype=torch.float32, device=dev) if fp8 else w.contiguous()
+        if attention or indexer:
+            ops.prefill_queries(q, nope, iq_raw, w, rope, q_full, iq, iw if fp8 else None, s, il)
+        return FullOperands(b, s, self._causal_lens(b, s, dev), True, q_full, kv, iq, iw, ik, ik_scale)
+
+    def full_select(self, op: "FullOperands", pad_value: int = -1, padded: bool = True) -> torch.Tensor:
+        """int32 [B*S, topk] selected key positions of every row. ``padded`` False: without the columns
+        that no row of a short sequence can fill (min(topk, S) columns)."""
+        if not op.fused:
+            return self._select(op.iq, op.ik, op.iw, op.lens, op.s, pad_value)
+        topk = self.config.index_topk if padded else min(self.config.index_topk, op.s)
+        if op.ik_scale is not None:
+            logits = ops.indexer_scan_fp8(op.iq, op.iw, op.ik, op.ik_scale, op.lens, rows_per_seq=op.s, ctx=op.s)
+        else:
+            logits = ops.indexer_scan_f32(op.iq, op.iw, op.ik, op.lens, rows_per_seq=op.s, ctx=op.s)
+        return ops.topk_select(logits, topk, op.lens, pad_value=pad_value)
+
+    def full_attend(self, op: "FullOperands", indices: Optional[torch.Tensor]) -> torch.Tensor:
+        """Attention hidden output [B,S,hidden]; indices int32 [B*S, topk] or None (dense causal)."""
+        c = self.config
+        if not op.fused:
+            o = self._attend(op.q, op.kv, indices, op.lens, op.s)
+            return self._project_output(o.view(op.b, op.s, *o.shape[1:]))
+        h = op.q.shape[1]
+        if op.q.dtype == torch.bfloat16:
+            o = ops.sparse_mla_decode(_pad_heads(op.q, ops.HEAD_BLOCK), op.kv, indices, self.sm_scale, op.lens,
+                                      rows_per_seq=op.s, dense_keys=op.s)
+        else:
+            o = ops.sparse_mla_f32(op.q, op.kv, indices, c.kv_lora_rank, self.sm_scale, op.lens, rows_per_seq=op.s)
+        _, w_uv = self._w_uk_uv()
+        ov = torch.empty(o.shape[0], h, c.v_head_dim, dtype=o.dtype, device=o.device)
+        torch.bmm(o[:, :h].transpose(0, 1), w_uv.transpose(1, 2), out=ov.transpose(0, 1))
+        return self._reduced(self.o_proj(ov.view(op.b, op.s, h * c.v_head_dim)))
+
     # ------------------------------------------------------------------ reference API (full sequence)
     def indexer_indices(self, x_norm, rope: RopeCaches, c_q=None) -> torch.Tensor:
         """int64 [B,S,topk] selected key positions, padded with S (reference :145-153)."""
-        if c_q is None:
-            c_q = self.q_latent(x_norm)
-        iq, ik, w = self._indexer_qkw(x_norm, c_q, rope)
-        b, s = x_norm.shape[0], x_norm.shape[1]
-        lens = self._causal_lens(b, s, x_norm.device)
-        idx = self._select(iq.reshape(b * s, *iq.shape[2:]), ik, w.reshape(b * s, -1), lens, s, pad_value=s)
-        return idx.view(b, s, -1).long()
+        op = self.full_operands(x_norm, rope, c_q, attention=False)
+        return self.full_select(op, pad_value=op.s).view(op.b, op.s, -1).long()
 
     def attention_output(self, x_norm, rope: RopeCaches, indices, c_q=None) -> torch.Tensor:
         """Attention hidden output; ``indices=None`` is dense causal (reference :156-171)."""
-        if c_q is None:
-            c_q = self.q_latent(x_norm)
-        q, kv = self._mla_qkv(x_norm, c_q, rope)
-        b, s, h = q.shape[0], q.shape[1], q.shape[2]
-        lens = self._causal_lens(b, s, x_norm.device)
-        idx32 = None if indices is None else indices.reshape(b * s, -1).to(torch.int32).contiguous()
-        o = self._attend(q.reshape(b * s, h, -1), kv, idx32, lens, s)
-        return self._project_output(o.view(b, s, h, -1))
+        op = self.full_operands(x_norm, rope, c_q, indexer=False)
+        idx32 = None if indices is None else indices.reshape(op.b * op.s, -1).to(torch.int32).contiguous()
+        return self.full_attend(op, idx32)
 
     def fused_attention_and_indices(self, x_norm, rope: RopeCaches, attn_indices, produce_indexer: bool = True):
         """One shared query latent for both consumers (reference :173-192)."""
-        c_q = self.q_latent(x_norm)
-        attn_hidden = self.attention_output(x_norm, rope, attn_indices, c_q=c_q)
-        nxt = self.indexer_indices(x_norm, rope, c_q=c_q) if produce_indexer else None
+        op = self.full_operands(x_norm, rope, indexer=produce_indexer)
+        idx32 = None if attn_indices is None else attn_indices.reshape(op.b * op.s, -1).to(torch.int32).contiguous()
+        attn_hidden = self.full_attend(op, idx32)
+        nxt = self.full_select(op, pad_value=op.s).view(op.b, op.s, -1).long() if produce_indexer else None
         return attn_hidden, nxt
 
     def mlp(self, h_norm: torch.Tensor) -> torch.Tensor:
@@ -302,17 +437,7 @@ class DSALayer(nn.Module):
 
     def fill_cache(self, cache: LayerDecodeCache, x_norm: torch.Tensor, rope: RopeCaches) -> None:
         """Writes the keys of a whole prefix x_norm [B,S,hidden] (prefill)."""
-        c_q = self.q_latent(x_norm)
-        _, kv = self._mla_qkv(x_norm, c_q, rope)
-        _, ik, _ = self._indexer_qkw(x_norm, c_q, rope)
-        s = x_norm.shape[1]
-        cache.kv[:, :s] = kv.to(cache.kv.dtype)
-        if cache.k_scale is not None:
-            ik8, sk = ops.quantize_e4m3_rowwise(ik.float().contiguous())
-            cache.index_k[:, :s] = ik8.view(torch.uint8)
-            cache.k_scale[:, :s] = sk
-        else:
-            cache.index_k[:, :s] = ik.float()
+        self.full_operands(x_norm, rope, attention=False, indexer=False, cache=cache)
 
     def decode_project(self, x_norm, rope: RopeCaches, positions, cache: LayerDecodeCache, batch_index):
         """Projections of one new token per sequence, and its keys appended to

@@ -129,13 +129,6 @@ class DSAModel(nn.Module):
                                    interleave=c.indexer_rope_interleave)
         return RopeCaches(mc, ms, ic, is_)
 
-    def _cold_start_indices(self, layer: DSALayer, x_norm, rope, cold_start: ColdStartPolicy):
-        if cold_start is ColdStartPolicy.DENSE:
-            return None
-        if cold_start is ColdStartPolicy.EAGER:
-            return layer.indexer_indices(x_norm, rope)
-        raise ValueError(f"unknown cold start policy: {cold_start}")
-
     def _lagged_indexer_layers(self, types) -> List[bool]:
         return lagged_producers(types)
 
@@ -147,41 +140,46 @@ class DSAModel(nn.Module):
         if not inputs_embeds.is_cuda:
             raise RuntimeError("this implementation runs on a CUDA device only (there is no CPU path)")
         rope = self._build_rope(inputs_embeds.shape[1], inputs_embeds.device, inputs_embeds.dtype)
+        used, produced = ([], []) if record else (None, None)
+        x = self._run_full(inputs_embeds, rope, mode, cold_start, None, used, produced)
+        return ForwardTrace(x, used, produced) if record else x
+
+    def _run_full(self, x, rope, mode: ScheduleMode, cold_start: ColdStartPolicy,
+                  caches: Optional[List[LayerDecodeCache]], used=None, produced=None) -> torch.Tensor:
+        """The full-sequence layers under a schedule (reference model.py:92-144), filling ``caches`` on
+        the way if given; returns the final norm's output. A layer's projections are computed once for
+        the caches, its indexer and its attention; the selections stay int32 between the layers."""
+        if mode not in (ScheduleMode.BASELINE, ScheduleMode.LAGGED_REFERENCE, ScheduleMode.LAGGED_FUSED):
+            raise ValueError(f"unknown schedule mode: {mode}")
+        b, s, _ = x.shape
         types = self.config.resolved_attention_types
         produces = lagged_producers(types)
-        x = inputs_embeds
+        lagged = mode is not ScheduleMode.BASELINE
         prev: Optional[torch.Tensor] = None
-        used, produced = [], []
+        x_norm = self.layers[0].attn_norm(x)
         for li, layer in enumerate(self.layers):
-            x_norm = layer.attn_norm(x)
             is_dsa = types[li] is AttentionType.DSA
-            if mode is ScheduleMode.BASELINE:
-                made = layer.indexer_indices(x_norm, rope) if is_dsa else None
-                attend = made
-                attn = layer.attention_output(x_norm, rope, attend)
-            elif mode in (ScheduleMode.LAGGED_REFERENCE, ScheduleMode.LAGGED_FUSED):
-                if not is_dsa:
-                    attend = None
-                elif li == 0:
-                    attend = self._cold_start_indices(layer, x_norm, rope, cold_start)
-                else:
-                    attend = prev
-                if mode is ScheduleMode.LAGGED_REFERENCE:
-                    attn = layer.attention_output(x_norm, rope, attend)
-                    made = layer.indexer_indices(x_norm, rope) if produces[li] else None
-                else:
-                    attn, made = layer.fused_attention_and_indices(x_norm, rope, attend,
-                                                                   produce_indexer=produces[li])
+            cold = lagged and is_dsa and li == 0
+            if cold and cold_start not in (ColdStartPolicy.DENSE, ColdStartPolicy.EAGER):
+                raise ValueError(f"unknown cold start policy: {cold_start}")
+            eager = cold and cold_start is ColdStartPolicy.EAGER  # layer 0 attends its own selection
+            makes = produces[li] if lagged else is_dsa
+            op = layer.full_operands(x_norm, rope, indexer=makes or eager, cache=None if caches is None else caches[li])
+            own = layer.full_select(op, pad_value=s, padded=used is not None) if makes or eager else None
+            made = own if makes else None
+            if not is_dsa:
+                attend = None
+            elif not lagged or eager:
+                attend = own
             else:
-                raise ValueError(f"unknown schedule mode: {mode}")
-            h = x + attn
-            x = h + layer.mlp(layer.ffn_norm(h))
+                attend = prev  # (None at layer 0 with a dense cold start)
+            attn = layer.full_attend(op, attend)
+            x, x_norm = self._residual_tail(li, x, attn)
             prev = made
-            if record:
-                used.append(attend)
-                produced.append(made)
-        x = self.final_norm(x)
-        return ForwardTrace(x, used, produced) if record else x
+            if used is not None:
+                used.append(None if attend is None else attend.view(b, s, -1).long())
+                produced.append(None if made is None else made.view(b, s, -1).long())
+        return x_norm  # the last layer's tail applied the final norm
 
     # ------------------------------------------------------------------ decode
     def init_decode(self, batch: int, capacity: int, fp8: Optional[bool] = None,
@@ -224,26 +222,10 @@ class DSAModel(nn.Module):
         layer's caches on the way; returns the final hidden states."""
         b, s, _ = inputs_embeds.shape
         rope = RopeCaches(state.rope.mla_cos[:s], state.rope.mla_sin[:s], state.rope.idx_cos[:s], state.rope.idx_sin[:s])
-        types = self.config.resolved_attention_types
-        produces = lagged_producers(types)
-        x, prev = inputs_embeds, None
-        for li, layer in enumerate(self.layers):
-            x_norm = layer.attn_norm(x)
-            layer.fill_cache(state.caches[li], x_norm, rope)
-            is_dsa = types[li] is AttentionType.DSA
-            if mode is ScheduleMode.BASELINE:
-                made = layer.indexer_indices(x_norm, rope) if is_dsa else None
-                attend = made
-            else:
-                attend = (None if not is_dsa else
-                          self._cold_start_indices(layer, x_norm, rope, cold_start) if li == 0 else prev)
-                made = layer.indexer_indices(x_norm, rope) if produces[li] else None
-            h = x + layer.attention_output(x_norm, rope, attend)
-            x = h + layer.mlp(layer.ffn_norm(h))
-            prev = made
+        x = self._run_full(inputs_embeds, rope, mode, cold_start, state.caches)
         state.positions.fill_(s)
         state.seq_lens.fill_(s)
-        return self.final_norm(x)
+        return x
 
     @torch.no_grad()
     def decode_step(self, state: DecodeState, x: torch.Tensor, mode: ScheduleMode,

@@ -171,15 +171,19 @@ def indexer_scan_f32(
     seq_lens: Optional[torch.Tensor] = None,
     *,
     rows_per_seq: int = 1,
+    ctx: Optional[int] = None,
     out: Optional[torch.Tensor] = None,
 ) -> torch.Tensor:
-    """fp32 logits for any head count / key width: q ``[R, H, D]``, k ``[n_seq, ctx, D]``."""
+    """fp32 logits for any head count / key width: q ``[R, H, D]``, k ``[n_seq, cap, D]`` of which
+    the first ``ctx`` keys are scanned (default: all)."""
     for t, n in ((index_q, "index_q"), (index_w, "index_w"), (index_k, "index_k")):
         _cuda_contig(t, n, (torch.float32,))
     R, n_heads, d = index_q.shape
     if index_k.dim() == 2:
         index_k = index_k.unsqueeze(0)
-    n_seq, ctx = index_k.shape[0], index_k.shape[1]
+    n_seq, cap = index_k.shape[0], index_k.shape[1]
+    ctx = cap if ctx is None else int(ctx)
+    _need(0 < ctx <= cap, "ctx must be in (0, cap]")
     _need(index_k.shape[2] == d, "index_k width differs from index_q")
     _need(R == n_seq * rows_per_seq, "R must equal n_seq * rows_per_seq")
     seq_lens = _lens(seq_lens, R)
@@ -187,7 +191,7 @@ def indexer_scan_f32(
         out = torch.empty(R, (ctx + 3) // 4 * 4, dtype=torch.float32, device=index_q.device)
     _lib.check(_lib.lib().dsa_indexer_scan_f32(
         _ptr(index_q), _ptr(index_w), _ptr(index_k), _ptr(seq_lens), _ptr(out), R, rows_per_seq,
-        n_heads, d, ctx, ctx, out.shape[1], _stream()))
+        n_heads, d, ctx, cap, out.shape[1], _stream()))
     return out[:, :ctx]
 
 
@@ -652,6 +656,92 @@ def decode_prep(iq_raw, w_raw, ik_raw, kv_a, q_abs, q_pe, kv_norm_w, mla_cos, ml
         _ptr(mla_cos), _ptr(mla_sin), _ptr(idx_cos), _ptr(idx_sin), _ptr(positions), _ptr(index_q), _ptr(index_w),
         _ptr(q_full), _ptr(cache_index_k), _ptr(cache_k_scale), _ptr(cache_kv), B, H, n_idx, cap,
         1 if interleave else 0, float(eps), _stream()))
+
+
+# --------------------------------------------------------------------------- full-sequence preparation
+def _rows(t: Optional[torch.Tensor], name: str, dtype) -> int:
+    """Row stride of a 2-D operand with dense rows (0 for None)."""
+    if t is None:
+        return 0
+    _need(t.is_cuda and t.dtype == dtype and t.dim() == 2 and t.stride(1) == 1, f"{name} must be CUDA {dtype} [rows, n] with dense rows")
+    return t.stride(0)
+
+
+def prefill_latents(qa, kv_a, ik, q_norm_w, kv_norm_w, rope, c_q, kv_out, ik_out, ik_scale, seq: int,
+                    interleave: bool, eps: float) -> None:
+    """Behind the GEMM that reads x_norm (see ``dsa_prefill_latents`` in the header): ``qa`` / ``kv_a`` /
+    ``ik`` are 2-D row views (any may be None), ``kv_out`` ``[n_seq, cap, w]`` and ``ik_out``
+    ``[n_seq, cap, D]`` (e4m3 bytes with ``ik_scale``, else the operands' type) receive their rows in
+    place. ``rope``: tables of the operands' type (``RopeCaches``)."""
+    ref = next(t for t in (qa, kv_a, ik) if t is not None)
+    dt = ref.dtype
+    _need(dt in (torch.float32, torch.bfloat16), "operands must be fp32 or bf16")
+    strides = [_rows(t, n, dt) for t, n in ((qa, "qa"), (kv_a, "kv_a"), (ik, "ik"))]
+    rows = ref.shape[0]
+    _need(all(t is None or t.shape[0] == rows for t in (qa, kv_a, ik)), "operand rows disagree")
+    for t, n in ((rope.mla_cos, "mla_cos"), (rope.mla_sin, "mla_sin"), (rope.idx_cos, "idx_cos"), (rope.idx_sin, "idx_sin")):
+        _cuda_contig(t, n, (dt,))
+        _need(t.shape[0] >= seq, f"{n} is shorter than the sequence")
+    q_rank = kv_rank = rope_dim = idx_dim = kv_cap = ik_cap = 0
+    if qa is not None:
+        q_rank = qa.shape[1]
+        _cuda_contig(c_q, "c_q", (dt,))
+        _need(c_q.numel() == rows * q_rank and q_norm_w.numel() == q_rank and q_norm_w.dtype == dt, "c_q / q_norm_w shapes")
+    if kv_a is not None:
+        rope_dim = rope.mla_cos.shape[1]
+        kv_rank = kv_a.shape[1] - rope_dim
+        _cuda_contig(kv_out, "kv_out", (dt,))
+        _need(kv_out.dim() == 3 and kv_out.shape[2] == kv_a.shape[1] and kv_out.shape[0] * seq == rows
+              and kv_out.shape[1] >= seq and kv_norm_w.numel() == kv_rank and kv_norm_w.dtype == dt, "kv_out must be [n_seq, cap, w]")
+        kv_cap = kv_out.shape[1]
+    if ik is not None:
+        idx_dim = ik.shape[1]
+        _cuda_contig(ik_out, "ik_out", (torch.uint8, _FP8) if ik_scale is not None else (dt,))
+        _need(ik_out.dim() == 3 and ik_out.shape[2] == idx_dim and ik_out.shape[0] * seq == rows and ik_out.shape[1] >= seq
+              and rope.idx_cos.shape[1] == idx_dim, "ik_out must be [n_seq, cap, D]")
+        ik_cap = ik_out.shape[1]
+        if ik_scale is not None:
+            _cuda_contig(ik_scale, "ik_scale", (torch.float32,))
+            _need(ik_scale.shape == ik_out.shape[:2], "ik_scale must be [n_seq, cap]")
+    _lib.check(_lib.lib().dsa_prefill_latents(
+        _ptr(qa), strides[0], _ptr(kv_a), strides[1], _ptr(ik), strides[2], _ptr(q_norm_w), _ptr(kv_norm_w),
+        _ptr(rope.mla_cos), _ptr(rope.mla_sin), _ptr(rope.idx_cos), _ptr(rope.idx_sin), _ptr(c_q), _ptr(kv_out), kv_cap,
+        _ptr(ik_out), _ptr(ik_scale), ik_cap, rows, seq, q_rank, kv_rank, rope_dim, idx_dim, 1 if interleave else 0,
+        float(eps), 0 if dt == torch.float32 else 1, _stream()))
+
+
+def prefill_queries(q, nope: int, iq, w, rope, q_full, index_q, index_w, seq: int, interleave: bool) -> None:
+    """Behind the GEMM that reads c_q (see ``dsa_prefill_queries``): ``q`` ``[rows, H, nope + rope]`` (a
+    strided view is fine) or None, ``iq`` / ``w`` 2-D row views or None; the rope columns of ``q_full``
+    ``[rows, H, kv_rank + rope]`` and ``index_q`` ``[rows, Hidx, D]`` (e4m3 bytes with ``index_w``, else
+    the operands' type) are written."""
+    ref = q if q is not None else iq
+    dt, rows = ref.dtype, ref.shape[0]
+    _need(dt in (torch.float32, torch.bfloat16), "operands must be fp32 or bf16")
+    for t, n in ((rope.mla_cos, "mla_cos"), (rope.mla_sin, "mla_sin"), (rope.idx_cos, "idx_cos"), (rope.idx_sin, "idx_sin")):
+        _cuda_contig(t, n, (dt,))
+        _need(t.shape[0] >= seq, f"{n} is shorter than the sequence")
+    H = Hidx = kv_rank = rope_dim = idx_dim = qs = qh = 0
+    iq_stride, w_stride = _rows(iq, "iq", dt), _rows(w, "w", dt)
+    if q is not None:
+        rope_dim = rope.mla_cos.shape[1]
+        _need(q.is_cuda and q.dim() == 3 and q.stride(2) == 1 and q.shape[2] == nope + rope_dim, "q must be [rows, H, nope + rope]")
+        H, qs, qh = q.shape[1], q.stride(0), q.stride(1)
+        _cuda_contig(q_full, "q_full", (dt,))
+        _need(q_full.dim() == 3 and q_full.shape[0] == rows and q_full.shape[1] == H, "q_full must be [rows, H, kv_rank + rope]")
+        kv_rank = q_full.shape[2] - rope_dim
+    if iq is not None:
+        _cuda_contig(index_q, "index_q", (torch.uint8, _FP8) if index_w is not None else (dt,))
+        Hidx, idx_dim = index_q.shape[1], index_q.shape[2]
+        _need(iq.shape == (rows, Hidx * idx_dim) and index_q.shape[0] == rows and rope.idx_cos.shape[1] == idx_dim,
+              "iq must be [rows, Hidx * D]")
+        if index_w is not None:
+            _cuda_contig(index_w, "index_w", (torch.float32,))
+            _need(w is not None and tuple(w.shape) == (rows, Hidx) and tuple(index_w.shape) == (rows, Hidx), "w must be [rows, Hidx]")
+    _lib.check(_lib.lib().dsa_prefill_queries(
+        _ptr(q), qs, qh, nope, _ptr(iq), iq_stride, _ptr(w), w_stride, _ptr(rope.mla_cos), _ptr(rope.mla_sin),
+        _ptr(rope.idx_cos), _ptr(rope.idx_sin), _ptr(q_full), _ptr(index_q), _ptr(index_w), rows, seq, H, Hidx, kv_rank,
+        rope_dim, idx_dim, 1 if interleave else 0, 0 if dt == torch.float32 else 1, _stream()))
 
 
 # --------------------------------------------------------------------------- exchanges between GPUs

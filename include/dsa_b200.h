@@ -31,7 +31,7 @@
 extern "C" {
 #endif
 
-#define DSA_ABI_VERSION 9
+#define DSA_ABI_VERSION 10
 
 enum dsa_status {
   DSA_OK = 0,
@@ -442,6 +442,31 @@ int dsa_latent_append(const void* kv_a, const float* kv_norm_weight, float eps, 
                       const float* rope_sin, const int64_t* positions, const int64_t* slots, void* pool,
                       int B, int64_t cap, int64_t n_slots, int rope_interleave, int format,
                       int round_scale, void* stream);
+
+/* Full-sequence (prompt) preparation: what lies between a layer's projection GEMMs and the scan /
+ * attention for `rows` = n_seq * seq tokens, row r being position r % seq of sequence r / seq
+ * (src/lagged_indexer_dsa/dsa_layer.py:87-143). dtype 0 = fp32, 1 = bf16 for all operands; every
+ * product and sum of the rotary embeddings is rounded to that type on its own.
+ *
+ * dsa_prefill_latents, behind the GEMM that reads x_norm (any of qa / kv_a / ik may be NULL: skipped):
+ *   c_q [rows, q_rank] = rmsnorm(qa); kv_out row b * kv_cap + s = [rmsnorm(kv_a[:kv_rank]) |
+ *   RoPE(kv_a[kv_rank:])]; ik_out row b * ik_cap + s = RoPE(ik), as e4m3 bytes with ik_scale (dtype 1,
+ *   idx_dim 128) or, with ik_scale NULL, in dtype. Row strides in elements.
+ * dsa_prefill_queries, behind the GEMM that reads c_q: the rope columns of q_full
+ *   [rows, H, kv_rank + rope_dim] = RoPE(q[row, h, nope:]) (q_full NULL: skipped), and RoPE(iq) as
+ *   e4m3 bytes with index_w = q scale * w (dtype 1, idx_dim 128) or in dtype (index_w NULL); iq NULL:
+ *   skipped. dtype 1 needs kv_rank 512, rope_dim 64, idx_dim 128. */
+int dsa_prefill_latents(const void* qa, int64_t qa_stride, const void* kv_a, int64_t kv_a_stride,
+                        const void* ik, int64_t ik_stride, const void* q_norm_w, const void* kv_norm_w,
+                        const void* mla_cos, const void* mla_sin, const void* idx_cos, const void* idx_sin,
+                        void* c_q, void* kv_out, int64_t kv_cap, void* ik_out, float* ik_scale,
+                        int64_t ik_cap, int64_t rows, int seq, int q_rank, int kv_rank, int rope_dim,
+                        int idx_dim, int interleave, float eps, int dtype, void* stream);
+int dsa_prefill_queries(const void* q, int64_t q_stride, int64_t q_head_stride, int nope, const void* iq,
+                        int64_t iq_stride, const void* w, int64_t w_stride, const void* mla_cos,
+                        const void* mla_sin, const void* idx_cos, const void* idx_sin, void* q_full,
+                        void* index_q, float* index_w, int64_t rows, int seq, int H, int n_index_heads,
+                        int kv_rank, int rope_dim, int idx_dim, int interleave, int dtype, void* stream);
 
 /* ---- (a7) per-token e4m3 quantisation of index keys / queries --------------
  * scale = max(amax(row), clamp_min) / 448, q = sat(x / scale) -> e4m3 RN
