@@ -825,12 +825,14 @@ static int mla_prepare(const void* q, const void* kv, const int32_t* indices, co
 
 static int mla_partials_launch(const void* q, const void* kv, const int32_t* indices,
                                const int32_t* seq_lens, float* part_acc, float* part_m, float* part_l,
-                               int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale,
+                               void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale,
                                int64_t kv_seq_stride, int kv_fp8, bool beside, void* stream) {
+  // `out`: the caller wants the merged result and there is one split, so the kernel writes it itself
   mla::Params p;
   int rc0 = mla_prepare(q, kv, indices, seq_lens, part_acc, part_m, part_l, R, rows_per_seq, H, topk_k,
-                        nsplit, sm_scale, kv_seq_stride, kv_fp8, true, &p);
+                        nsplit, sm_scale, kv_seq_stride, kv_fp8, out == nullptr, &p);
   if (rc0) return rc0;
+  p.out = static_cast<__nv_bfloat16*>(out);
   // Head counts that fill 64-row blocks go to the tcgen05 kernel once there are enough
   // 64-head x 64-key tiles to give every SM more than one (a single row of 2048 keys
   // is faster on the mma.sync kernel's 16-head CTAs); its splits are whole 64-key tiles.
@@ -865,7 +867,7 @@ int dsa_sparse_mla_partials(const void* q, const void* kv, const int32_t* indice
                             const int32_t* seq_lens, float* part_acc, float* part_m, float* part_l,
                             int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale,
                             int64_t kv_seq_stride, int kv_fp8, void* stream) {
-  return mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, R, rows_per_seq, H, topk_k,
+  return mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, nullptr, R, rows_per_seq, H, topk_k,
                              nsplit, sm_scale, kv_seq_stride, kv_fp8, false, stream);
 }
 
@@ -895,10 +897,9 @@ int dsa_sparse_mla_decode(const void* q, const void* kv, const int32_t* indices,
                           void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit,
                           float sm_scale, int64_t kv_seq_stride, int kv_fp8, void* stream) {
   DSA_REQUIRE(out && aligned16(out), "sparse MLA: out must be a 16-byte aligned pointer");
-  int rc = dsa_sparse_mla_partials(q, kv, indices, seq_lens, part_acc, part_m, part_l, R,
-                                   rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8,
-                                   stream);
-  if (rc) return rc;
+  int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, nsplit == 1 ? out : nullptr, R,
+                               rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8, false, stream);
+  if (rc || nsplit == 1) return rc;
   return dsa_sparse_mla_combine(part_acc, part_m, part_l, out, R, H, nsplit, stream);
 }
 
@@ -907,9 +908,9 @@ int dsa_sparse_mla_decode_beside(const void* q, const void* kv, const int32_t* i
                                  void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit,
                                  float sm_scale, int64_t kv_seq_stride, int kv_fp8, void* stream) {
   DSA_REQUIRE(out && aligned16(out), "sparse MLA: out must be a 16-byte aligned pointer");
-  int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, R, rows_per_seq, H, topk_k,
-                               nsplit, sm_scale, kv_seq_stride, kv_fp8, true, stream);
-  if (rc) return rc;
+  int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, nsplit == 1 ? out : nullptr, R,
+                               rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8, true, stream);
+  if (rc || nsplit == 1) return rc;
   return dsa_sparse_mla_combine(part_acc, part_m, part_l, out, R, H, nsplit, stream);
 }
 

@@ -41,6 +41,7 @@ struct Params {
   float* part_acc;
   float* part_m;
   float* part_l;
+  __nv_bfloat16* out;     // one split only: the normalised result goes here and no partials are written
   int64_t kv_seq_stride;  // rows per cached sequence
   int64_t ctx;            // dense mode: key capacity
   int rows_per_seq;
@@ -434,6 +435,19 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
     drain_after_timeout();  // let outstanding copies land
   }
 
+  if (p.out) {  // the only split: what the merge kernel would make of its partials
+    __nv_bfloat16* out = p.out + (int64_t(r) * p.H + hg * kHB) * kDV;
+    const float inv0 = l_run[0] > 0.f ? 1.f / l_run[0] : 0.f, inv1 = l_run[1] > 0.f ? 1.f / l_run[1] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int col = warp * 128 + i * 8 + t4 * 2;
+      *reinterpret_cast<__nv_bfloat162*>(out + g * kDV + col) = __floats2bfloat162_rn(acc[i][0] * inv0, acc[i][1] * inv0);
+      *reinterpret_cast<__nv_bfloat162*>(out + (g + 8) * kDV + col) = __floats2bfloat162_rn(acc[i][2] * inv1, acc[i][3] * inv1);
+    }
+    if constexpr (kBeside) pdl_wait();
+    DSA_KTIME_END(2);
+    return;
+  }
   // ---- partials of this split: unnormalised accumulator, running max (base 2), sum
   const int64_t pbase = (int64_t(r) * p.nsplit + split) * p.H + hg * kHB;
 #pragma unroll

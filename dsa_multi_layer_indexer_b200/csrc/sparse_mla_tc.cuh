@@ -85,6 +85,7 @@ struct Smem {
   static constexpr int tmem_off = misc_off + 96;
   static constexpr int flag_off = misc_off + 104;      // int [2]
   static constexpr int valid_off = misc_off + 112;     // uint32 [2 stages][producer warps]
+  static constexpr int bound_off = misc_off + 248;     // int: end of the split's last visible key
   static constexpr int factor_off = misc_off + 256;    // float [64]
   static constexpr int max_off = misc_off + 512;       // float [2 parities][2 halves][64]
   static constexpr int bytes = misc_off + 1536 + 1024;  // + slack for the 1024-byte alignment
@@ -128,6 +129,7 @@ sparse_mla_tc_kernel(const mla::Params p) {
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + Smem::tmem_off);
   volatile int* s_flag = reinterpret_cast<volatile int*>(smem + Smem::flag_off);
   volatile uint32_t* s_validw = reinterpret_cast<volatile uint32_t*>(smem + Smem::valid_off);
+  int* s_bound = reinterpret_cast<int*>(smem + Smem::bound_off);
   volatile float* s_factor = reinterpret_cast<volatile float*>(smem + Smem::factor_off);
   volatile float* s_max = reinterpret_cast<volatile float*>(smem + Smem::max_off);
   auto bar = [&](int i) { return bars + 8u * uint32_t(i); };
@@ -148,6 +150,7 @@ sparse_mla_tc_kernel(const mla::Params p) {
     }
     mbar_init(bar(kBarPFull), 2 * kHG);
     mbar_init(bar(kBarOFull), 1);
+    *s_bound = 0;
     mbar_fence_init();
   }
   if (warp == kMmaWarp) {
@@ -167,26 +170,44 @@ sparse_mla_tc_kernel(const mla::Params p) {
   len = len < 0 ? 0 : (len > p.ctx ? p.ctx : len);
   const int k_begin = split * p.keys_per_split;
   const int k_end = min(k_begin + p.keys_per_split, p.topk);
-  const int n_tiles = (max(k_end - k_begin, 0) + kBN - 1) / kBN;
   bool failed = false;
   DSA_STAMP(scta, 14);
 
+  const int ptid = tid - kProducerWarp0 * 32;
+  const int v8 = ptid & 7, rsub = ptid >> 3;  // gather: 8 threads per row, kRowsPerPass rows per pass
+  if (warp >= kProducerWarp0) {
+    // queries of this head block: [64 heads][1152 B] -> swizzled chunks
+    const uint8_t* qsrc = reinterpret_cast<const uint8_t*>(p.q + (int64_t(r) * p.H + hg * kHG) * mla::kD);
+#pragma unroll
+    for (int k = 0; k < kPasses; ++k) {
+      const int row = rsub + kRowsPerPass * k;
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c)
+        cp_async16(s_q + swz(row, c * 8 + v8), qsrc + row * mla::kRowBytes + c * 128 + v8 * 16);
+    }
+    cp_async_commit();
+  }
+  // Where the split's last visible key ends: the padding behind it (a row with fewer keys than the list
+  // has entries, as most rows of a prompt) costs no tiles. The look at the list runs beside the query's
+  // way into shared memory, which the first product waits for anyway. (4099-token prompt, top-2048,
+  // 128 heads: a quarter of the tiles.)
+  int n_tiles;
+  if (p.indices) {
+    int bound = 0;
+    for (int j = k_begin + tid; j < k_end; j += kThreads) {
+      const int idx = p.indices[int64_t(r) * p.topk + j];
+      if (idx >= 0 && idx < len) bound = j + 1;
+    }
+    bound = __reduce_max_sync(0xffffffffu, bound);
+    if (lane == 0 && bound > 0) atomicMax(s_bound, bound);
+    __syncthreads();
+    n_tiles = (max(*s_bound - k_begin, 0) + kBN - 1) / kBN;
+  } else {
+    n_tiles = (max(int(min(int64_t(k_end), len)) - k_begin, 0) + kBN - 1) / kBN;
+  }
+
   if (warp >= kProducerWarp0) {
     // ===================================================================== gather
-    const int ptid = tid - kProducerWarp0 * 32;
-    const int v8 = ptid & 7, rsub = ptid >> 3;  // 8 threads per row, kRowsPerPass rows per pass
-    {
-      // queries of this head block: [64 heads][1152 B] -> swizzled chunks
-      const uint8_t* qsrc = reinterpret_cast<const uint8_t*>(p.q + (int64_t(r) * p.H + hg * kHG) * mla::kD);
-#pragma unroll
-      for (int k = 0; k < kPasses; ++k) {
-        const int row = rsub + kRowsPerPass * k;
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c)
-          cp_async16(s_q + swz(row, c * 8 + v8), qsrc + row * mla::kRowBytes + c * 128 + v8 * 16);
-      }
-      cp_async_commit();
-    }
     const int row_bytes = p.kv_fp8 ? mla::kFp8Row : mla::kRowBytes;
     const uint8_t* kv_seq = p.kv + int64_t(seq) * p.kv_seq_stride * row_bytes;
     // selection entries of this thread's four rows of tile t (-1 past the split)
@@ -495,10 +516,16 @@ sparse_mla_tc_kernel(const mla::Params p) {
     // the two column halves of a head add their sums
     if (soft && half == 1) s_factor[head] = l_run;
     group_sync();
-    if (soft && half == 0) l_run += s_factor[head];
+    if (soft && half == 0) {
+      l_run += s_factor[head];
+      s_factor[head] = l_run > 0.f ? 1.f / l_run : 0.f;  // (read only by this thread above)
+    }
+    if (p.out) group_sync();
 
     if (warp < 4) {
-      // ---- partials of this split: O^T (lane = value dim, column = head), reference m, sum l
+      // ---- partials of this split: O^T (lane = value dim, column = head), reference m, sum l; or,
+      // when there is only one split, the normalised bf16 result itself (what the merge kernel would
+      // make of the partials: 256 KB less traffic per row and 128 heads, and one launch less)
       const int64_t pbase = (int64_t(r) * p.nsplit + split) * p.H + hg * kHG;
       bool have = n_tiles > 0 && !__any_sync(0xffffffffu, failed);
       if (__any_sync(0xffffffffu, have && !mbar_wait(bar(kBarOFull), 0))) have = false, failed = true;
@@ -515,11 +542,18 @@ sparse_mla_tc_kernel(const mla::Params p) {
           for (int i = 0; i < 32; ++i) o[i] = 0u;
         }
         const int dim = (blk >> 1) * 128 + quad * 32 + lane;
-        float* dst = p.part_acc + (pbase + (blk & 1) * 32) * mla::kDV + dim;
+        if (p.out) {
+          __nv_bfloat16* dst = p.out + (int64_t(r) * p.H + hg * kHG + (blk & 1) * 32) * mla::kDV + dim;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) dst[int64_t(i) * mla::kDV] = __uint_as_float(o[i]);
+          for (int i = 0; i < 32; ++i)
+            dst[i * mla::kDV] = __float2bfloat16_rn(__uint_as_float(o[i]) * s_factor[(blk & 1) * 32 + i]);
+        } else {
+          float* dst = p.part_acc + (pbase + (blk & 1) * 32) * mla::kDV + dim;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) dst[int64_t(i) * mla::kDV] = __uint_as_float(o[i]);
+        }
       }
-      if (soft) {
+      if (soft && !p.out) {
         p.part_m[pbase + head] = have ? m_ref : -INFINITY;
         p.part_l[pbase + head] = have ? l_run : 0.f;
       }

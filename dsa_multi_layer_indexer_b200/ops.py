@@ -331,9 +331,11 @@ def sparse_mla_decode(
     seq_lens = _lens(seq_lens, R)
     if nsplit is None:
         nsplit = scratch.nsplit if scratch is not None else default_nsplit(R, H, topk)
-    if scratch is None:
+    if scratch is None and (nsplit > 1 or stage != "both"):  # (one split: the result is written at once)
         scratch = MlaScratch(R, H, nsplit, q.device)
-    _need(scratch.rows >= R and scratch.heads == H and scratch.nsplit == nsplit, "scratch does not match the launch")
+    _need(scratch is None or (scratch.rows >= R and scratch.heads == H and scratch.nsplit == nsplit),
+          "scratch does not match the launch")
+    acc, m, l = (None, None, None) if scratch is None else (scratch.acc, scratch.m, scratch.l)
     if out is None:
         out = torch.empty(R, H, VALUE_DIM, dtype=torch.bfloat16, device=q.device)
     _out_contig(out, "out", (torch.bfloat16,))
@@ -341,16 +343,16 @@ def sparse_mla_decode(
     if stage == "both":
         fn = _lib.lib().dsa_sparse_mla_decode_beside if beside_previous else _lib.lib().dsa_sparse_mla_decode
         _lib.check(fn(
-            _ptr(q), _ptr(kv), _ptr(indices), _ptr(seq_lens), _ptr(scratch.acc), _ptr(scratch.m),
-            _ptr(scratch.l), _ptr(out), R, rows_per_seq, H, topk, nsplit, float(sm_scale), cap, kv_fp8,
+            _ptr(q), _ptr(kv), _ptr(indices), _ptr(seq_lens), _ptr(acc), _ptr(m),
+            _ptr(l), _ptr(out), R, rows_per_seq, H, topk, nsplit, float(sm_scale), cap, kv_fp8,
             _stream()))
     elif stage == "partials":  # the two halves separately, as the reference schedules them
         _lib.check(_lib.lib().dsa_sparse_mla_partials(
-            _ptr(q), _ptr(kv), _ptr(indices), _ptr(seq_lens), _ptr(scratch.acc), _ptr(scratch.m),
-            _ptr(scratch.l), R, rows_per_seq, H, topk, nsplit, float(sm_scale), cap, kv_fp8, _stream()))
+            _ptr(q), _ptr(kv), _ptr(indices), _ptr(seq_lens), _ptr(acc), _ptr(m),
+            _ptr(l), R, rows_per_seq, H, topk, nsplit, float(sm_scale), cap, kv_fp8, _stream()))
     elif stage == "combine":
         _lib.check(_lib.lib().dsa_sparse_mla_combine(
-            _ptr(scratch.acc), _ptr(scratch.m), _ptr(scratch.l), _ptr(out), R, H, nsplit, _stream()))
+            _ptr(acc), _ptr(m), _ptr(l), _ptr(out), R, H, nsplit, _stream()))
     else:
         raise ValueError(f"unknown stage {stage!r}")
     return out
