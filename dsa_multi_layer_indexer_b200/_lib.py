@@ -36,6 +36,7 @@ SIGNATURES: Dict[str, Tuple[object, List[object]]] = {
     "dsa_indexer_scan_f32": (_i, [_p, _p, _p, _p, _p, _i, _i, _i, _i, _l, _l, _l, _p]),
     "dsa_topk_workspace_bytes": (_l, [_i, _l]),
     "dsa_topk_select": (_i, [_p, _p, _p, _p, _p, _p, _p, _l, _i, _l, _l, _i, C.c_int32, C.c_int32, _p]),
+    "dsa_topk_select_paged": (_i, [_p, _p, _p, _p, _l, _p, _i, _l, _l, _i, C.c_int32, _p]),
     "dsa_topk_select_push": (_i, [_p, _p, _p, _i, _l, _l, _i, C.c_int32, C.c_int32, _i, _i, _p, _p, _p, _p, _p]),
     "dsa_topk_merge_wait": (_i, [_p, _p, _p, _p, _p, _i, _i, _i, C.c_int32, _l, _p]),
     "dsa_allreduce_push": (_i, [_p, _i, _l, _i, _i, _p, _p, _p, _p]),
@@ -105,6 +106,26 @@ def lib() -> C.CDLL:
         raise ImportError(f"{LIB_PATH} has ABI version {got}, this package needs {ABI_VERSION}")
     _lib = handle
     return handle
+
+
+_host = None
+
+
+def host():
+    """The native half of ``ops``, bound to the loaded library; raises like :func:`lib` if it has not
+    been built."""
+    global _host
+    if _host is not None:
+        return _host
+    handle = lib()
+    try:
+        from . import _host as module
+    except ImportError as exc:
+        raise ImportError(f"{_PKG / '_host.so'} is missing or does not load: build it with "
+                          "`python -m dsa_multi_layer_indexer_b200.csrc.build` (there is no fallback path)") from exc
+    module.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in SIGNATURES}, check)
+    _host = module
+    return module
 
 
 def check(status: int) -> None:

@@ -453,10 +453,10 @@ int64_t dsa_topk_workspace_bytes(int R, int64_t n) {
 
 // Rows of up to topk_cluster_max_n() logits: one cluster of 1..8 (or 16) CTAs per row, no scratch.
 extern "C++" {
-template <bool kPlain, int kMaxC>
+template <bool kPlain, int kMaxC, bool kPages = false>
 static int launch_topk_cluster_as(const topk::Params& p, int R, int ctas, int nk, cudaStream_t st) {
   static bool done[64];
-  auto kernel = topk::topk_cluster_kernel<kPlain, kMaxC>;
+  auto kernel = topk::topk_cluster_kernel<kPlain, kMaxC, kPages>;
   constexpr size_t smem = sizeof(topk::ClSharedT<kMaxC>);
   int dev = 0;
   DSA_CUDA(cudaGetDevice(&dev));
@@ -497,6 +497,9 @@ static int launch_topk_cluster(const topk::Params& p, int R, int64_t n, cudaStre
     while (ctas < topk::kClMaxCtas && int64_t(ctas) * 2048 < n && 2 * ctas * R <= sm_count()) ctas *= 2;
   const int64_t per_key = int64_t(ctas) * topk::kClThreads;
   const int nk = int((n + per_key - 1) / per_key);
+  if (p.page_table)
+    return ctas > topk::kClMaxCtas ? launch_topk_cluster_as<true, topk::kClMaxCtasBig, true>(p, R, ctas, nk, st)
+                                   : launch_topk_cluster_as<true, topk::kClMaxCtas, true>(p, R, ctas, nk, st);
   if (ctas > topk::kClMaxCtas)
     return plain ? launch_topk_cluster_as<true, topk::kClMaxCtasBig>(p, R, ctas, nk, st)
                  : launch_topk_cluster_as<false, topk::kClMaxCtasBig>(p, R, ctas, nk, st);
@@ -508,7 +511,8 @@ int dsa_topk_select(const float* logits, const int32_t* seq_lens, uint32_t* hist
                     const int32_t* index_map, int32_t* out_idx, float* out_val, void* workspace,
                     int64_t workspace_bytes, int R, int64_t n, int64_t slab_stride, int topk_k,
                     int32_t pad_value, int32_t index_offset, void* stream) {
-  DSA_REQUIRE(logits && out_idx && workspace, "topk: null pointer");
+  // (rows that the cluster kernel takes need no workspace)
+  DSA_REQUIRE(logits && out_idx && (workspace || (R > 0 && n > 0 && n <= topk_cluster_max_n())), "topk: null pointer");
   DSA_REQUIRE(aligned16(logits) && aligned16(workspace), "topk: logits / workspace must be 16-byte aligned");
   DSA_REQUIRE(R > 0 && R <= 65535, "topk: R=%d out of range", R);
   DSA_REQUIRE(n > 0 && slab_stride >= n, "topk: need 0 < n <= slab_stride");
@@ -516,7 +520,7 @@ int dsa_topk_select(const float* logits, const int32_t* seq_lens, uint32_t* hist
   if (n > topk::kMaxN)
     return fail(DSA_ERR_UNSUPPORTED, "topk: n=%lld exceeds the %lld-per-row limit", (long long)n,
                 (long long)topk::kMaxN);
-  DSA_REQUIRE(workspace_bytes >= dsa_topk_workspace_bytes(R, n),
+  DSA_REQUIRE(!workspace || workspace_bytes >= dsa_topk_workspace_bytes(R, n),
               "topk: workspace of %lld bytes is smaller than dsa_topk_workspace_bytes = %lld",
               (long long)workspace_bytes, (long long)dsa_topk_workspace_bytes(R, n));
   if (n <= topk_cluster_max_n()) {
@@ -568,6 +572,33 @@ int dsa_topk_select(const float* logits, const int32_t* seq_lens, uint32_t* hist
   DSA_CUDA(launch_pdl(topk::topk_finish_kernel, dim3(R), dim3(topk::kFinThreads),
                       topk::fin_smem_bytes(p.words), st, p));
   return DSA_OK;
+}
+
+int dsa_topk_select_paged(const float* logits, const int32_t* seq_lens, uint32_t* hist, const int32_t* page_table,
+                          int64_t pt_stride, int32_t* out_idx, int R, int64_t n, int64_t slab_stride, int topk_k,
+                          int32_t pad_value, void* stream) {
+  DSA_REQUIRE(logits && hist && page_table && out_idx, "paged topk: null pointer");
+  DSA_REQUIRE(aligned16(logits), "paged topk: logits must be 16-byte aligned");
+  DSA_REQUIRE(R > 0 && R <= 65535, "paged topk: R=%d out of range", R);
+  DSA_REQUIRE(n > 0 && slab_stride >= n, "paged topk: need 0 < n <= slab_stride");
+  DSA_REQUIRE(topk_k > 0 && topk_k <= 65536, "paged topk: k=%d out of range [1, 65536]", topk_k);
+  DSA_REQUIRE(pt_stride * DSA_PAGE_TOKENS >= n, "paged topk: pt_stride=%lld pages cannot cover n=%lld", (long long)pt_stride,
+              (long long)n);
+  if (n > topk_cluster_max_n())
+    return fail(DSA_ERR_UNSUPPORTED, "paged topk: rows of %lld logits (the limit is %lld)", (long long)n,
+                (long long)topk_cluster_max_n());
+  topk::Params p{};
+  p.logits = logits;
+  p.seq_lens = seq_lens;
+  p.hist = hist;
+  p.page_table = page_table;
+  p.pt_stride = pt_stride;
+  p.out_idx = out_idx;
+  p.n = n;
+  p.slab_stride = slab_stride;
+  p.topk = topk_k;
+  p.pad = pad_value;
+  return launch_topk_cluster(p, R, n, static_cast<cudaStream_t>(stream));
 }
 
 // ------------------------------------------------------------------ candidate exchange between GPUs

@@ -1,0 +1,762 @@
+// Native half of ops.py: argument checks, allocation of results and the C-ABI calls of the entry
+// points that a decode step or a full-sequence layer makes eagerly, in one step from Python objects
+// to the launch. A ctypes call with its checks in Python cost 10-20 us per operation, more than the
+// kernels of a small step take; here an operation costs one to three microseconds plus its launches.
+// The library's functions arrive as addresses (bind), so the build that _lib.py loaded is the one that
+// runs. Nothing here computes: it checks, allocates with torch's allocator and launches on torch's
+// current stream.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <algorithm>
+#include <cmath>
+#include <initializer_list>
+#include <stdexcept>
+#include <string>
+#include <tuple>
+#include <type_traits>
+#include <utility>
+
+#include "../../include/dsa_b200.h"
+
+namespace {
+
+using at::Tensor;
+
+// ---------------------------------------------------------------- the library's functions
+#define DSA_HOST_API(X)                                                                                        \
+  X(dsa_indexer_scan_fp8) X(dsa_indexer_scan_fp8_paged) X(dsa_indexer_scan_f32) X(dsa_topk_workspace_bytes)    \
+  X(dsa_topk_select) X(dsa_topk_select_paged) X(dsa_sparse_mla_partials) X(dsa_sparse_mla_combine)             \
+  X(dsa_sparse_mla_decode) X(dsa_sparse_mla_decode_beside) X(dsa_sparse_mla_f32) X(dsa_rmsnorm)                \
+  X(dsa_add_rmsnorm_bf16) X(dsa_silu_mul_bf16) X(dsa_indexer_stage_fp8) X(dsa_latent_append)                   \
+  X(dsa_prefill_latents) X(dsa_prefill_queries)
+struct Api {
+#define X(name) decltype(&::name) name = nullptr;
+  DSA_HOST_API(X)
+#undef X
+} api;
+PyObject* status_check = nullptr;  // _lib.check: raises for a negative status
+
+// ---------------------------------------------------------------- errors
+struct PyErrorSet {};  // a Python exception is already set
+[[noreturn]] void bad(const std::string& msg) {
+  PyErr_SetString(PyExc_ValueError, msg.c_str());
+  throw PyErrorSet();
+}
+inline void need(bool cond, const char* msg) {
+  if (__builtin_expect(!cond, 0)) bad(msg);
+}
+void ok(int status) {
+  if (__builtin_expect(status == 0, 1)) return;
+  PyObject* r = PyObject_CallFunction(status_check, "i", status);
+  Py_XDECREF(r);
+  if (r) PyErr_SetString(PyExc_RuntimeError, "dsa_b200: call failed");
+  throw PyErrorSet();
+}
+
+// The call itself runs without the interpreter's lock (a full launch queue blocks it): its arguments
+// must not touch Python objects.
+#define LAUNCH(expr)                         \
+  do {                                       \
+    int status_;                             \
+    Py_BEGIN_ALLOW_THREADS status_ = (expr); \
+    Py_END_ALLOW_THREADS ok(status_);        \
+  } while (0)
+
+// ---------------------------------------------------------------- arguments
+inline const Tensor* opt(PyObject* o, const char* name) {
+  if (o == Py_None) return nullptr;
+  if (!THPVariable_Check(o)) {
+    PyErr_Format(PyExc_TypeError, "%s must be a tensor, got %s", name, Py_TYPE(o)->tp_name);
+    throw PyErrorSet();
+  }
+  return &THPVariable_Unpack(o);
+}
+inline const Tensor& ten(PyObject* o, const char* name) {
+  const Tensor* t = opt(o, name);
+  if (!t) {
+    PyErr_Format(PyExc_TypeError, "%s must be a tensor, got None", name);
+    throw PyErrorSet();
+  }
+  return *t;
+}
+inline int64_t integer(PyObject* o) {
+  int64_t v = PyLong_Check(o) ? PyLong_AsLongLong(o) : -1;
+  if (!PyLong_Check(o)) {  // numpy integers and the like
+    PyObject* i = PyNumber_Index(o);
+    if (!i) throw PyErrorSet();
+    v = PyLong_AsLongLong(i);
+    Py_DECREF(i);
+  }
+  if (v == -1 && PyErr_Occurred()) throw PyErrorSet();
+  return v;
+}
+inline double real(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw PyErrorSet();
+  return v;
+}
+inline bool truth(PyObject* o) { return PyObject_IsTrue(o) == 1; }
+void contig(const Tensor& t, const char* name, std::initializer_list<at::ScalarType> types, bool pinned_too = false) {
+  if (!t.is_cuda() && !(pinned_too && t.is_pinned()))
+    bad(std::string(name) + (pinned_too ? " must be a CUDA tensor or pinned host memory" : " must be a CUDA tensor"));
+  if (!t.is_contiguous()) bad(std::string(name) + " must be contiguous");
+  const at::ScalarType st = t.scalar_type();
+  for (at::ScalarType x : types)
+    if (x == st) return;
+  std::string msg = std::string(name) + " has dtype " + c10::toString(st) + ", expected one of";
+  for (at::ScalarType x : types) msg += std::string(" ") + c10::toString(x);
+  bad(msg);
+}
+inline void* ptr(const Tensor& t) { return t.data_ptr(); }
+inline void* ptr(const Tensor* t) { return t ? t->data_ptr() : nullptr; }
+template <class T>
+inline T* as(const Tensor& t) { return static_cast<T*>(t.data_ptr()); }
+template <class T>
+inline T* as(const Tensor* t) { return t ? static_cast<T*>(t->data_ptr()) : nullptr; }
+inline void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+inline Tensor fresh(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like) {
+  return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device()));
+}
+const Tensor* lens_of(PyObject* o, int64_t rows) {
+  const Tensor* t = opt(o, "seq_lens");
+  if (t) {
+    contig(*t, "seq_lens", {at::kInt});
+    if (t->numel() != rows)
+      bad("seq_lens has " + std::to_string(t->numel()) + " entries, expected " + std::to_string(rows));
+  }
+  return t;
+}
+const Tensor* hist_of(PyObject* o, int64_t rows) {
+  const Tensor* t = opt(o, "hist");
+  if (t) {
+    contig(*t, "hist", {at::kInt, at::kUInt32});
+    need(t->numel() == rows * DSA_TOPK_HIST_BINS, "hist must be [R, 4096]");
+  }
+  return t;
+}
+inline PyObject* same(PyObject* o) {
+  Py_INCREF(o);
+  return o;
+}
+// `given` when the caller passed the buffer, else a wrapper of the new tensor.
+inline PyObject* result(PyObject* given, const Tensor& t) { return given != Py_None ? same(given) : THPVariable_Wrap(t); }
+PyObject* columns(PyObject* given, const Tensor& t, int64_t n) {
+  if (t.size(1) == n) return result(given, t);
+  return THPVariable_Wrap(t.narrow(1, 0, n));
+}
+
+constexpr auto kFp8 = at::kFloat8_e4m3fn;
+
+// ---------------------------------------------------------------- indexer scan
+// (index_q, index_w, index_k, k_scale, seq_lens, rows_per_seq, ctx, out, hist, impl)
+PyObject* scan_fp8(PyObject* const* a) {
+  const Tensor &q = ten(a[0], "index_q"), &w = ten(a[1], "index_w"), &k = ten(a[2], "index_k"), &ks = ten(a[3], "k_scale");
+  contig(q, "index_q", {kFp8, at::kByte});
+  contig(w, "index_w", {at::kFloat});
+  contig(k, "index_k", {kFp8, at::kByte});
+  contig(ks, "k_scale", {at::kFloat});
+  need(q.dim() == 3 && q.size(2) == DSA_INDEX_DIM, "index_q must be [R, Hidx, 128]");
+  const int64_t R = q.size(0), heads = q.size(1), rps = integer(a[5]);
+  need(w.dim() == 2 && w.size(0) == R && w.size(1) == heads, "index_w must be [R, Hidx]");
+  int64_t n_seq = 1, cap;
+  if (k.dim() == 2) {
+    need(k.size(1) == DSA_INDEX_DIM, "index_k must be [n_seq, cap, 128]");
+    cap = k.size(0);
+    need(ks.numel() == cap, "k_scale must be [n_seq, cap]");
+  } else {
+    need(k.dim() == 3 && k.size(2) == DSA_INDEX_DIM, "index_k must be [n_seq, cap, 128]");
+    n_seq = k.size(0), cap = k.size(1);
+    need(ks.dim() == 2 && ks.size(0) == n_seq && ks.size(1) == cap, "k_scale must be [n_seq, cap]");
+  }
+  if (R != n_seq * rps)
+    bad("R=" + std::to_string(R) + " must equal n_seq=" + std::to_string(n_seq) + " * rows_per_seq=" + std::to_string(rps));
+  const int64_t ctx = a[6] == Py_None ? cap : integer(a[6]);
+  need(ctx > 0 && ctx <= cap, "ctx must be in (0, cap]");
+  const Tensor* lens = lens_of(a[4], R);
+  const Tensor* given = opt(a[7], "out");
+  const Tensor out = given ? *given : fresh({R, (ctx + 3) / 4 * 4}, at::kFloat, q);
+  contig(out, "out", {at::kFloat});
+  need(out.dim() == 2 && out.size(0) == R && out.size(1) >= ctx, "out must be [R, >= ctx]");
+  const Tensor* hist = hist_of(a[8], R);
+  const int impl = int(integer(a[9]));
+  void* st = stream();
+  LAUNCH(api.dsa_indexer_scan_fp8(as<uint8_t>(q), as<float>(w), as<uint8_t>(k), as<float>(ks), as<int32_t>(lens), as<float>(out),
+                              as<uint32_t>(hist), int(R), int(rps), int(heads), ctx, n_seq, cap, cap, out.size(1),
+                              impl, st));
+  return columns(a[7], out, ctx);
+}
+
+// (index_q, index_w, pages, page_table, seq_lens, ctx, out, hist)
+PyObject* scan_paged(PyObject* const* a) {
+  const Tensor &q = ten(a[0], "index_q"), &w = ten(a[1], "index_w"), &pages = ten(a[2], "index_k_pages"),
+               &table = ten(a[3], "page_table");
+  contig(q, "index_q", {kFp8, at::kByte});
+  contig(w, "index_w", {at::kFloat});
+  contig(pages, "index_k_pages", {at::kByte});
+  contig(table, "page_table", {at::kInt});
+  need(q.dim() == 3 && q.size(2) == DSA_INDEX_DIM, "index_q must be [R, Hidx, 128]");
+  const int64_t R = q.size(0), heads = q.size(1), ctx = integer(a[5]);
+  need(pages.dim() == 2 && pages.size(1) == DSA_INDEX_PAGE_BYTES, "index_k_pages must be [num_pages, 8448]");
+  need(table.dim() == 2 && table.size(0) == R, "page_table must be [R, pt_stride]");
+  const Tensor* lens = lens_of(a[4], R);
+  need(lens != nullptr, "paged scan needs seq_lens");
+  const Tensor* given = opt(a[6], "out");
+  const Tensor out = given ? *given : fresh({R, (ctx + 3) / 4 * 4}, at::kFloat, q);
+  contig(out, "out", {at::kFloat});
+  need(out.dim() == 2 && out.size(0) == R && out.size(1) >= ctx, "out must be [R, >= ctx]");
+  need(w.dim() == 2 && w.size(0) == R && w.size(1) == heads, "index_w must be [R, Hidx]");
+  need(table.size(1) * DSA_PAGE_TOKENS >= ctx, "page_table rows cannot cover ctx positions");
+  const Tensor* hist = hist_of(a[7], R);
+  void* st = stream();
+  LAUNCH(api.dsa_indexer_scan_fp8_paged(as<uint8_t>(q), as<float>(w), as<uint8_t>(pages), pages.size(0), as<int32_t>(table),
+                                    table.size(1), as<int32_t>(lens), as<float>(out), as<uint32_t>(hist), int(R), int(heads), ctx,
+                                    out.size(1), st));
+  return columns(a[6], out, ctx);
+}
+
+// (index_q, index_w, index_k, seq_lens, rows_per_seq, ctx, out)
+PyObject* scan_f32(PyObject* const* a) {
+  const Tensor &q = ten(a[0], "index_q"), &w = ten(a[1], "index_w"), &k = ten(a[2], "index_k");
+  contig(q, "index_q", {at::kFloat});
+  contig(w, "index_w", {at::kFloat});
+  contig(k, "index_k", {at::kFloat});
+  need(q.dim() == 3, "index_q must be [R, H, D]");
+  const int64_t R = q.size(0), heads = q.size(1), d = q.size(2), rps = integer(a[4]);
+  need(k.dim() == 2 || k.dim() == 3, "index_k must be [n_seq, cap, D]");
+  const int64_t n_seq = k.dim() == 2 ? 1 : k.size(0), cap = k.size(-2);
+  const int64_t ctx = a[5] == Py_None ? cap : integer(a[5]);
+  need(ctx > 0 && ctx <= cap, "ctx must be in (0, cap]");
+  need(k.size(-1) == d, "index_k width differs from index_q");
+  need(w.numel() == R * heads, "index_w must be [R, H]");
+  need(R == n_seq * rps, "R must equal n_seq * rows_per_seq");
+  const Tensor* lens = lens_of(a[3], R);
+  const Tensor* given = opt(a[6], "out");
+  const Tensor out = given ? *given : fresh({R, (ctx + 3) / 4 * 4}, at::kFloat, q);
+  contig(out, "out", {at::kFloat});
+  need(out.dim() == 2 && out.size(0) == R && out.size(1) >= ctx, "out must be [R, >= ctx]");
+  void* st = stream();
+  LAUNCH(api.dsa_indexer_scan_f32(as<float>(q), as<float>(w), as<float>(k), as<int32_t>(lens), as<float>(out), int(R), int(rps),
+                              int(heads), int(d), ctx, cap, out.size(1), st));
+  return columns(a[6], out, ctx);
+}
+
+// ---------------------------------------------------------------- top-k
+// Scratch of a call: the caller's, or a fresh zeroed one where rows of n logits need any.
+struct Workspace {
+  Tensor own;
+  void* data = nullptr;
+  int64_t bytes = 0;
+};
+Workspace workspace_for(PyObject* given, int64_t R, int64_t n, const Tensor& like) {
+  Workspace ws;
+  if (const Tensor* t = opt(given, "workspace")) {
+    contig(*t, "workspace", {at::kByte});
+    ws.data = ptr(*t), ws.bytes = t->numel();
+    return ws;
+  }
+  ws.bytes = api.dsa_topk_workspace_bytes(int(R), n);
+  if (ws.bytes > 16) {
+    ws.own = fresh({ws.bytes}, at::kByte, like).zero_();
+    ws.data = ptr(ws.own);
+  }
+  return ws;
+}
+
+// (logits, topk, seq_lens, hist, index_map, pad, offset, out_idx, out_val, return_values, workspace)
+PyObject* topk(PyObject* const* a) {
+  const Tensor& x = ten(a[0], "logits");
+  need(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 2, "logits must be CUDA fp32 [R, n]");
+  need(x.stride(1) == 1, "logits rows must be dense");
+  const int64_t R = x.size(0), n = x.size(1), k = integer(a[1]);
+  const int64_t slab = R > 1 ? x.stride(0) : std::max(x.stride(0), n);
+  const Tensor* lens = lens_of(a[2], R);
+  const Tensor* map = opt(a[4], "index_map");
+  if (map) {
+    contig(*map, "index_map", {at::kInt});
+    need(map->dim() == 2 && map->size(0) == R && map->size(1) == n, "index_map must be [R, n]");
+  }
+  need(k > 0 && k <= 65536, "topk must be in [1, 65536]");
+  const std::string shape = "[" + std::to_string(R) + ", " + std::to_string(k) + "]";
+  const Tensor* gi = opt(a[7], "out_idx");
+  const Tensor idx = gi ? *gi : fresh({R, k}, at::kInt, x);
+  contig(idx, "out_idx", {at::kInt});
+  if (!(idx.dim() == 2 && idx.size(0) == R && idx.size(1) == k)) bad("out_idx must be [R, topk] = " + shape);
+  const Tensor* gv = opt(a[8], "out_val");
+  Tensor val;
+  if (gv) val = *gv;
+  else if (truth(a[9])) val = fresh({R, k}, at::kFloat, x);
+  if (val.defined()) {
+    contig(val, "out_val", {at::kFloat});
+    if (!(val.dim() == 2 && val.size(0) == R && val.size(1) == k)) bad("out_val must be [R, topk] = " + shape);
+  }
+  const Tensor* hist = hist_of(a[3], R);
+  const Workspace ws = workspace_for(a[10], R, n, x);
+  const int32_t pad = int32_t(integer(a[5])), offset = int32_t(integer(a[6]));
+  void* st = stream();
+  LAUNCH(api.dsa_topk_select(as<float>(x), as<int32_t>(lens), as<uint32_t>(hist), as<int32_t>(map), as<int32_t>(idx),
+                         val.defined() ? as<float>(val) : nullptr, ws.data, ws.bytes, int(R), n, slab, int(k),
+                         pad, offset, st));
+  PyObject* pi = result(a[7], idx);
+  if (!val.defined()) return pi;
+  PyObject* pv = result(a[8], val);
+  PyObject* both = PyTuple_Pack(2, pi, pv);
+  Py_DECREF(pi);
+  Py_DECREF(pv);
+  return both;
+}
+
+// (logits, topk, seq_lens, hist, page_table, pad, out_idx): the selection as slots of the 64-token pages
+PyObject* topk_paged(PyObject* const* a) {
+  const Tensor &x = ten(a[0], "logits"), &table = ten(a[4], "page_table"), &idx = ten(a[6], "out_idx");
+  need(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 2 && x.stride(1) == 1, "logits must be CUDA fp32 [R, n] with dense rows");
+  const int64_t R = x.size(0), n = x.size(1), k = integer(a[1]);
+  const Tensor* lens = lens_of(a[2], R);
+  const Tensor* hist = hist_of(a[3], R);
+  contig(table, "page_table", {at::kInt});
+  need(table.dim() == 2 && table.size(0) == R && table.size(1) * DSA_PAGE_TOKENS >= n, "page_table rows cannot cover the logits");
+  contig(idx, "out_idx", {at::kInt});
+  need(idx.dim() == 2 && idx.size(0) == R && idx.size(1) == k, "out_idx must be [R, topk]");
+  const int32_t pad = int32_t(integer(a[5]));
+  void* st = stream();
+  LAUNCH(api.dsa_topk_select_paged(as<float>(x), as<int32_t>(lens), as<uint32_t>(hist), as<int32_t>(table), table.size(1),
+                               as<int32_t>(idx), int(R), n, R > 1 ? x.stride(0) : std::max(x.stride(0), n), int(k),
+                               pad, st));
+  return same(a[6]);
+}
+
+// ---------------------------------------------------------------- sparse MLA
+// ops.default_nsplit
+int64_t default_nsplit(int64_t rows, int64_t heads, int64_t k, int64_t sms) {
+  const int64_t tiles = std::max<int64_t>(1, (k + 63) / 64);
+  if (heads % 64 == 0 && rows * (heads / 64) * tiles >= 128) {
+    const int64_t blocks = std::max<int64_t>(1, rows * (heads / 64));
+    int64_t want = std::max<int64_t>(1, std::min(sms / blocks, tiles));
+    while (tiles % want) --want;
+    return want;
+  }
+  const int64_t blocks = std::max<int64_t>(1, rows * (heads / 16));
+  const int64_t want = std::max<int64_t>(1, 2 * sms / blocks);
+  return std::max<int64_t>(1, std::min(want, tiles));
+}
+
+// (q, kv, indices, sm_scale, seq_lens, rows_per_seq, nsplit, acc, m, l, out, dense_keys, stage 0 both / 1 partials /
+//  2 combine, beside)
+PyObject* mla(PyObject* const* a) {
+  const Tensor &q = ten(a[0], "q"), &kv = ten(a[1], "kv");
+  contig(q, "q", {at::kBFloat16});
+  need(q.dim() == 3 && q.size(2) == DSA_LATENT_DIM, "q must be [R, H, 576]");
+  const int64_t R = q.size(0), H = q.size(1), rps = integer(a[5]);
+  if (H % DSA_HEAD_BLOCK) bad("H=" + std::to_string(H) + " must be a multiple of 16 (pad heads with zero queries)");
+  need(kv.is_cuda() && kv.is_contiguous() && (kv.dim() == 3 || kv.dim() == 2), "kv must be a contiguous CUDA [n_seq, cap, w] tensor");
+  const bool fp8 = kv.scalar_type() != at::kBFloat16;
+  if (!fp8) need(kv.size(-1) == DSA_LATENT_DIM, "bf16 kv rows must be 576 wide");
+  else need(kv.scalar_type() == at::kByte && kv.size(-1) == DSA_FP8_LATENT_ROW, "fp8 kv rows must be 656 bytes of uint8");
+  const int64_t n_seq = kv.dim() == 2 ? 1 : kv.size(0), cap = kv.size(-2);
+  need(R == n_seq * rps, "R must equal n_seq * rows_per_seq");
+  const Tensor* idx = opt(a[2], "indices");
+  int64_t k;
+  if (idx) {
+    contig(*idx, "indices", {at::kInt});
+    need(idx->dim() == 2 && idx->size(0) == R, "indices must be [R, topk]");
+    k = idx->size(1);
+  } else {
+    k = a[11] == Py_None ? cap : integer(a[11]);
+  }
+  const Tensor* lens = lens_of(a[4], R);
+  const Tensor* ga = opt(a[7], "scratch.acc");
+  const int64_t nsplit = a[6] != Py_None ? integer(a[6]) : ga ? ga->size(1) : default_nsplit(R, H, k, 148);
+  const int64_t stage = integer(a[12]);
+  Tensor acc, m, l;
+  if (ga) {
+    need(ga->dim() == 4 && ga->size(0) >= R && ga->size(1) == nsplit && ga->size(2) == H, "scratch does not match the launch");
+    acc = *ga, m = ten(a[8], "scratch.m"), l = ten(a[9], "scratch.l");
+  } else if (nsplit > 1 || stage != 0) {  // (one split: the result is written at once)
+    acc = fresh({R, nsplit, H, DSA_VALUE_DIM}, at::kFloat, q);
+    m = fresh({R, nsplit, H}, at::kFloat, q);
+    l = fresh({R, nsplit, H}, at::kFloat, q);
+  }
+  const Tensor* go = opt(a[10], "out");
+  const Tensor out = go ? *go : fresh({R, H, DSA_VALUE_DIM}, at::kBFloat16, q);
+  contig(out, "out", {at::kBFloat16}, true);
+  need(out.numel() >= R * H * DSA_VALUE_DIM, "out must be [R, H, 512]");
+  float *pa = acc.defined() ? as<float>(acc) : nullptr, *pm = m.defined() ? as<float>(m) : nullptr,
+        *pl = l.defined() ? as<float>(l) : nullptr;
+  const float scale = float(real(a[3]));
+  const bool beside = truth(a[13]);
+  need(!beside || stage == 0, "beside_previous goes with stage='both'");
+  void* st = stream();
+  if (stage == 0)
+    LAUNCH((beside ? api.dsa_sparse_mla_decode_beside : api.dsa_sparse_mla_decode)(
+        ptr(q), ptr(kv), as<int32_t>(idx), as<int32_t>(lens), pa, pm, pl, ptr(out), int(R), int(rps), int(H), int(k), int(nsplit),
+        scale, cap, fp8 ? 1 : 0, st));
+  else if (stage == 1)
+    LAUNCH(api.dsa_sparse_mla_partials(ptr(q), ptr(kv), as<int32_t>(idx), as<int32_t>(lens), pa, pm, pl, int(R), int(rps), int(H),
+                                       int(k), int(nsplit), scale, cap, fp8 ? 1 : 0, st));
+  else
+    LAUNCH(api.dsa_sparse_mla_combine(pa, pm, pl, ptr(out), int(R), int(H), int(nsplit), st));
+  return result(a[10], out);
+}
+
+// (q, kv, indices, value_dim, sm_scale, seq_lens, rows_per_seq)
+PyObject* mla_f32(PyObject* const* a) {
+  const Tensor &q = ten(a[0], "q"), &kv = ten(a[1], "kv");
+  contig(q, "q", {at::kFloat});
+  contig(kv, "kv", {at::kFloat});
+  need(q.dim() == 3 && (kv.dim() == 2 || kv.dim() == 3), "q must be [R, H, Dqk], kv [n_seq, ctx, Dqk]");
+  const int64_t R = q.size(0), H = q.size(1), d = q.size(2), rps = integer(a[6]), vd = integer(a[3]);
+  const int64_t n_seq = kv.dim() == 2 ? 1 : kv.size(0), ctx = kv.size(-2);
+  need(kv.size(-1) == d && R == n_seq * rps, "q / kv shapes disagree");
+  const Tensor* idx = opt(a[2], "indices");
+  if (idx) {
+    contig(*idx, "indices", {at::kInt});
+    need(idx->dim() == 2 && idx->size(0) == R, "indices must be [R, topk]");
+  }
+  const Tensor* lens = lens_of(a[5], R);
+  const Tensor out = fresh({R, H, vd}, at::kFloat, q);
+  const float scale = float(real(a[4]));
+  void* st = stream();
+  LAUNCH(api.dsa_sparse_mla_f32(as<float>(q), as<float>(kv), as<int32_t>(idx), as<int32_t>(lens), as<float>(out), int(R), int(rps), int(H),
+                            int(d), int(vd), idx ? int(idx->size(1)) : 0, scale, ctx, st));
+  return THPVariable_Wrap(out);
+}
+
+// ---------------------------------------------------------------- norms and the MLP's product
+// (x, weight, eps)
+PyObject* rmsnorm(PyObject* const* a) {
+  const Tensor& x0 = ten(a[0], "x");
+  need(x0.is_cuda() && (x0.scalar_type() == at::kFloat || x0.scalar_type() == at::kBFloat16), "x must be CUDA fp32 / bf16");
+  const Tensor x = x0.contiguous();
+  const Tensor w = ten(a[1], "weight").to(x.scalar_type()).contiguous();
+  const Tensor out = at::empty_like(x);
+  const int64_t dim = x.size(-1);
+  const float eps = float(real(a[2]));
+  void* st = stream();
+  LAUNCH(api.dsa_rmsnorm(ptr(x), ptr(w), ptr(out), x.numel() / dim, int(dim), eps, x.scalar_type() == at::kFloat ? 0 : 1, st));
+  return THPVariable_Wrap(out);
+}
+
+// (x, delta, weight, eps)
+PyObject* add_rmsnorm(PyObject* const* a) {
+  const Tensor &x0 = ten(a[0], "x"), &d0 = ten(a[1], "delta");
+  need(x0.is_cuda() && x0.scalar_type() == at::kBFloat16 && d0.scalar_type() == at::kBFloat16 && x0.sizes() == d0.sizes(),
+       "x and delta must be CUDA bf16 tensors of one shape");
+  const int64_t dim = x0.size(-1);
+  need(dim % 8 == 0 && dim <= 8192, "the row length must be a multiple of 8 and at most 8192");
+  const Tensor x = x0.contiguous(), d = d0.contiguous();
+  const Tensor w = ten(a[2], "weight").to(x.scalar_type()).contiguous();
+  const Tensor s = at::empty_like(x), out = at::empty_like(x);
+  const float eps = float(real(a[3]));
+  void* st = stream();
+  LAUNCH(api.dsa_add_rmsnorm_bf16(ptr(x), ptr(d), ptr(w), ptr(s), ptr(out), x.numel() / dim, int(dim), eps, st));
+  PyObject *ps = THPVariable_Wrap(s), *po = THPVariable_Wrap(out);
+  PyObject* both = PyTuple_Pack(2, ps, po);
+  Py_DECREF(ps);
+  Py_DECREF(po);
+  return both;
+}
+
+// (gate, up)
+PyObject* silu_mul(PyObject* const* a) {
+  const Tensor &g0 = ten(a[0], "gate"), &u0 = ten(a[1], "up");
+  need(g0.is_cuda() && g0.scalar_type() == at::kBFloat16 && u0.scalar_type() == at::kBFloat16 && g0.sizes() == u0.sizes(),
+       "gate and up must be CUDA bf16 tensors of one shape");
+  const Tensor g = g0.contiguous(), u = u0.contiguous(), out = at::empty_like(g);
+  void* st = stream();
+  LAUNCH(api.dsa_silu_mul_bf16(ptr(g), ptr(u), ptr(out), g.numel(), st));
+  return THPVariable_Wrap(out);
+}
+
+// ---------------------------------------------------------------- staging of a new token
+// (q_raw, k_raw, w_raw, norm_w, norm_b, eps, cos, sin, positions, index_q, index_w, cache_k, cache_scale, pages, page_table,
+//  interleave, round_scale, softmax_scale)
+PyObject* indexer_stage(PyObject* const* a) {
+  const Tensor &q = ten(a[0], "q_raw"), &k = ten(a[1], "k_raw"), &w = ten(a[2], "w_raw"), &nw = ten(a[3], "k_norm_weight"),
+               &nb = ten(a[4], "k_norm_bias"), &cs = ten(a[6], "rope_cos"), &sn = ten(a[7], "rope_sin"), &pos = ten(a[8], "positions"),
+               &iq = ten(a[9], "index_q"), &iw = ten(a[10], "index_w");
+  contig(q, "q_raw", {at::kBFloat16});
+  contig(k, "k_raw", {at::kBFloat16});
+  contig(w, "w_raw", {at::kFloat});
+  contig(nw, "k_norm_weight", {at::kFloat});
+  contig(nb, "k_norm_bias", {at::kFloat});
+  contig(cs, "rope_cos", {at::kFloat});
+  contig(sn, "rope_sin", {at::kFloat});
+  contig(iw, "index_w", {at::kFloat});
+  contig(pos, "positions", {at::kLong});
+  contig(iq, "index_q", {at::kByte, kFp8});
+  need(q.dim() == 3 && q.size(2) == DSA_INDEX_DIM, "q_raw must be [B, heads, 128]");
+  const int64_t B = q.size(0), heads = q.size(1);
+  need(k.dim() == 2 && k.size(0) == B && k.size(1) == DSA_INDEX_DIM && w.dim() == 2 && w.size(0) == B && w.size(1) == heads &&
+           iw.sizes() == w.sizes() && iq.sizes() == q.sizes() && pos.dim() == 1 && pos.size(0) == B,
+       "operand shapes disagree");
+  need(nw.numel() == DSA_INDEX_DIM && nb.numel() == DSA_INDEX_DIM, "LayerNorm parameters must be [128]");
+  int64_t cap = cs.size(0);
+  need(cs.dim() == 2 && cs.size(1) == 32 && sn.sizes() == cs.sizes(), "rotary tables must be [cap, 32]");
+  const Tensor *pages = opt(a[13], "pages"), *table = nullptr, *ck = nullptr, *csc = nullptr;
+  if (pages) {
+    table = &ten(a[14], "page_table");
+    contig(*pages, "pages", {at::kByte});
+    contig(*table, "page_table", {at::kInt});
+    need(table->dim() == 2 && table->size(0) == B, "page_table must be [B, pages per sequence]");
+    need(pages->numel() % DSA_INDEX_PAGE_BYTES == 0, "page pool must be whole pages");
+    cap = std::min(cap, table->size(1) * DSA_PAGE_TOKENS);
+  } else {
+    ck = &ten(a[11], "cache_index_k"), csc = &ten(a[12], "cache_k_scale");
+    contig(*ck, "cache_index_k", {at::kByte, kFp8});
+    contig(*csc, "cache_k_scale", {at::kFloat});
+    need(ck->dim() == 3 && ck->size(0) == B && ck->size(2) == DSA_INDEX_DIM && csc->dim() == 2 && csc->size(0) == B &&
+             csc->size(1) == ck->size(1),
+         "caches must be [B, cap, 128] and [B, cap]");
+    cap = std::min(cap, ck->size(1));
+  }
+  const float eps = float(real(a[5])), head_scale = float(std::pow(double(heads), -0.5));
+  const float softmax_scale = float(a[17] == Py_None ? std::pow(double(DSA_INDEX_DIM), -0.5) : real(a[17]));
+  const int interleave = truth(a[15]), round_scale = truth(a[16]);
+  void* st = stream();
+  LAUNCH(api.dsa_indexer_stage_fp8(
+      ptr(q), ptr(k), as<float>(w), as<float>(nw), as<float>(nb), eps, as<float>(cs), as<float>(sn), as<int64_t>(pos), as<uint8_t>(iq),
+      as<float>(iw), as<uint8_t>(ck), as<float>(csc), as<uint8_t>(pages), pages ? pages->numel() / DSA_INDEX_PAGE_BYTES : 0,
+      as<int32_t>(table), table ? table->size(1) : 0, int(B), int(heads), cap, interleave, round_scale, head_scale, softmax_scale, st));
+  Py_RETURN_NONE;
+}
+
+// (kv_a, norm_w, eps, cos, sin, positions, slots, pool, interleave, format, round_scale)
+PyObject* latent_append(PyObject* const* a) {
+  const Tensor &kv = ten(a[0], "kv_a"), &nw = ten(a[1], "kv_norm_weight"), &cs = ten(a[3], "rope_cos"), &sn = ten(a[4], "rope_sin"),
+               &pos = ten(a[5], "positions"), &slots = ten(a[6], "slots"), &pool = ten(a[7], "pool");
+  contig(kv, "kv_a", {at::kBFloat16});
+  contig(nw, "kv_norm_weight", {at::kFloat});
+  contig(cs, "rope_cos", {at::kFloat});
+  contig(sn, "rope_sin", {at::kFloat});
+  contig(pos, "positions", {at::kLong});
+  contig(slots, "slots", {at::kLong});
+  need(kv.dim() == 2 && kv.size(1) == DSA_LATENT_DIM, "kv_a must be [B, 576]");
+  const int64_t B = kv.size(0);
+  need(pos.dim() == 1 && pos.size(0) == B && slots.dim() == 1 && slots.size(0) == B, "positions and slots must be [B]");
+  need(nw.numel() == DSA_VALUE_DIM, "kv_norm_weight must be [512]");
+  need(cs.dim() == 2 && cs.size(1) == 32 && sn.sizes() == cs.sizes(), "rotary tables must be [cap, 32]");
+  const int format = int(integer(a[9])), interleave = truth(a[8]), round_scale = truth(a[10]);
+  if (format == 2) {
+    contig(pool, "pool", {at::kByte});
+    need(pool.dim() == 2 && pool.size(1) == DSA_FP8_LATENT_ROW, "an fp8 pool is [n_slots, 656] uint8");
+  } else {
+    contig(pool, "pool", {at::kBFloat16});
+    need(pool.dim() == 2 && pool.size(1) == DSA_LATENT_DIM, "a bf16 pool is [n_slots, 576]");
+  }
+  const float eps = float(real(a[2]));
+  void* st = stream();
+  LAUNCH(api.dsa_latent_append(ptr(kv), as<float>(nw), eps, as<float>(cs), as<float>(sn), as<int64_t>(pos), as<int64_t>(slots), ptr(pool),
+                               int(B), cs.size(0), pool.size(0), interleave, format, round_scale, st));
+  Py_RETURN_NONE;
+}
+
+// ---------------------------------------------------------------- full-sequence preparation
+int64_t rows_of(const Tensor* t, const char* name, at::ScalarType type) {
+  if (!t) return 0;
+  if (!(t->is_cuda() && t->scalar_type() == type && t->dim() == 2 && t->stride(1) == 1))
+    bad(std::string(name) + " must be CUDA [rows, n] of the operands' type with dense rows");
+  return t->stride(0);
+}
+struct Rope {
+  const Tensor &mc, &ms, &ic, &is;
+};
+Rope rope_of(PyObject* const* a, at::ScalarType type, int64_t seq) {
+  Rope r{ten(a[0], "mla_cos"), ten(a[1], "mla_sin"), ten(a[2], "idx_cos"), ten(a[3], "idx_sin")};
+  for (const Tensor* t : {&r.mc, &r.ms, &r.ic, &r.is}) {
+    contig(*t, "rotary table", {type});
+    need(t->dim() == 2 && t->size(0) >= seq, "a rotary table is shorter than the sequence");
+  }
+  return r;
+}
+int dtype_of(at::ScalarType t) {
+  need(t == at::kFloat || t == at::kBFloat16, "operands must be fp32 or bf16");
+  return t == at::kFloat ? 0 : 1;
+}
+
+// (qa, kv_a, ik, q_norm_w, kv_norm_w, mla_cos, mla_sin, idx_cos, idx_sin, c_q, kv_out, ik_out, ik_scale, seq, interleave, eps)
+PyObject* prefill_latents(PyObject* const* a) {
+  const Tensor *qa = opt(a[0], "qa"), *kv = opt(a[1], "kv_a"), *ik = opt(a[2], "ik"), *qw = opt(a[3], "q_norm_w"),
+               *kw = opt(a[4], "kv_norm_w"), *cq = opt(a[9], "c_q"), *kvo = opt(a[10], "kv_out"), *iko = opt(a[11], "ik_out"),
+               *iks = opt(a[12], "ik_scale");
+  const Tensor* ref = qa ? qa : kv ? kv : ik;
+  need(ref != nullptr, "nothing to do");
+  const at::ScalarType type = ref->scalar_type();
+  const int dt = dtype_of(type);
+  const int64_t qs = rows_of(qa, "qa", type), kvs = rows_of(kv, "kv_a", type), iks_ = rows_of(ik, "ik", type);
+  const int64_t rows = ref->size(0), seq = integer(a[13]);
+  for (const Tensor* t : {qa, kv, ik}) need(!t || t->size(0) == rows, "operand rows disagree");
+  const Rope rope = rope_of(a + 5, type, seq);
+  int64_t q_rank = 0, kv_rank = 0, rope_dim = 0, idx_dim = 0, kv_cap = 0, ik_cap = 0;
+  if (qa) {
+    q_rank = qa->size(1);
+    need(cq && qw, "c_q and q_norm_w go with qa");
+    contig(*cq, "c_q", {type});
+    need(cq->numel() == rows * q_rank && qw->numel() == q_rank && qw->scalar_type() == type, "c_q / q_norm_w shapes");
+  }
+  if (kv) {
+    rope_dim = rope.mc.size(1), kv_rank = kv->size(1) - rope_dim;
+    need(kvo && kw, "kv_out and kv_norm_w go with kv_a");
+    contig(*kvo, "kv_out", {type});
+    need(kvo->dim() == 3 && kvo->size(2) == kv->size(1) && kvo->size(0) * seq == rows && kvo->size(1) >= seq && kw->numel() == kv_rank &&
+             kw->scalar_type() == type,
+         "kv_out must be [n_seq, cap, w]");
+    kv_cap = kvo->size(1);
+  }
+  if (ik) {
+    idx_dim = ik->size(1);
+    need(iko != nullptr, "ik_out goes with ik");
+    if (iks) contig(*iko, "ik_out", {at::kByte, kFp8});
+    else contig(*iko, "ik_out", {type});
+    need(iko->dim() == 3 && iko->size(2) == idx_dim && iko->size(0) * seq == rows && iko->size(1) >= seq && rope.ic.size(1) == idx_dim,
+         "ik_out must be [n_seq, cap, D]");
+    ik_cap = iko->size(1);
+    if (iks) {
+      contig(*iks, "ik_scale", {at::kFloat});
+      need(iks->dim() == 2 && iks->size(0) == iko->size(0) && iks->size(1) == ik_cap, "ik_scale must be [n_seq, cap]");
+    }
+  }
+  const int interleave = truth(a[14]);
+  const float eps = float(real(a[15]));
+  void* st = stream();
+  LAUNCH(api.dsa_prefill_latents(ptr(qa), qs, ptr(kv), kvs, ptr(ik), iks_, ptr(qw), ptr(kw), ptr(rope.mc), ptr(rope.ms), ptr(rope.ic),
+                                 ptr(rope.is), ptr(cq), ptr(kvo), kv_cap, ptr(iko), as<float>(iks), ik_cap, rows, int(seq), int(q_rank),
+                                 int(kv_rank), int(rope_dim), int(idx_dim), interleave, eps, dt, st));
+  Py_RETURN_NONE;
+}
+
+// (q, nope, iq, w, mla_cos, mla_sin, idx_cos, idx_sin, q_full, index_q, index_w, seq, interleave)
+PyObject* prefill_queries(PyObject* const* a) {
+  const Tensor *q = opt(a[0], "q"), *iq = opt(a[2], "iq"), *w = opt(a[3], "w"), *qf = opt(a[8], "q_full"), *iqo = opt(a[9], "index_q"),
+               *iwo = opt(a[10], "index_w");
+  const Tensor* ref = q ? q : iq;
+  need(ref != nullptr, "nothing to do");
+  const at::ScalarType type = ref->scalar_type();
+  const int dt = dtype_of(type);
+  const int64_t rows = ref->size(0), seq = integer(a[11]), nope = integer(a[1]);
+  const Rope rope = rope_of(a + 4, type, seq);
+  int64_t H = 0, Hidx = 0, kv_rank = 0, rope_dim = 0, idx_dim = 0, qs = 0, qh = 0;
+  const int64_t iqs = rows_of(iq, "iq", type), ws = rows_of(w, "w", type);
+  if (q) {
+    rope_dim = rope.mc.size(1);
+    need(q->is_cuda() && q->scalar_type() == type && q->dim() == 3 && q->stride(2) == 1 && q->size(2) == nope + rope_dim,
+         "q must be [rows, H, nope + rope]");
+    H = q->size(1), qs = q->stride(0), qh = q->stride(1);
+    need(qf != nullptr, "q_full goes with q");
+    contig(*qf, "q_full", {type});
+    need(qf->dim() == 3 && qf->size(0) == rows && qf->size(1) == H, "q_full must be [rows, H, kv_rank + rope]");
+    kv_rank = qf->size(2) - rope_dim;
+  }
+  if (iq) {
+    need(iqo != nullptr, "index_q goes with iq");
+    if (iwo) contig(*iqo, "index_q", {at::kByte, kFp8});
+    else contig(*iqo, "index_q", {type});
+    need(iqo->dim() == 3 && iqo->size(0) == rows, "index_q must be [rows, Hidx, D]");
+    Hidx = iqo->size(1), idx_dim = iqo->size(2);
+    need(iq->size(0) == rows && iq->size(1) == Hidx * idx_dim && rope.ic.size(1) == idx_dim, "iq must be [rows, Hidx * D]");
+    if (iwo) {
+      contig(*iwo, "index_w", {at::kFloat});
+      need(w && w->size(0) == rows && w->size(1) == Hidx && iwo->numel() == rows * Hidx, "w must be [rows, Hidx]");
+    }
+  }
+  const int interleave = truth(a[12]);
+  void* st = stream();
+  LAUNCH(api.dsa_prefill_queries(ptr(q), qs, qh, int(nope), ptr(iq), iqs, ptr(w), ws, ptr(rope.mc), ptr(rope.ms), ptr(rope.ic), ptr(rope.is),
+                                 ptr(qf), ptr(iqo), as<float>(iwo), rows, int(seq), int(H), int(Hidx), int(kv_rank), int(rope_dim),
+                                 int(idx_dim), interleave, dt, st));
+  Py_RETURN_NONE;
+}
+
+// ---------------------------------------------------------------- the ABI's functions as they are
+// abi_<name>(args without the stream): a pointer argument is a tensor, None or an address. For callers that
+// mirror another extension's argument lists and hand over what they were given (kernels_ext.py).
+template <class T>
+T from_py(PyObject* o) {
+  if constexpr (std::is_pointer_v<T>) {
+    if (o == Py_None) return nullptr;
+    if (THPVariable_Check(o)) return static_cast<T>(THPVariable_Unpack(o).data_ptr());
+    return reinterpret_cast<T>(static_cast<uintptr_t>(integer(o)));
+  } else if constexpr (std::is_floating_point_v<T>) {
+    return T(real(o));
+  } else {
+    return T(integer(o));
+  }
+}
+template <class... A, size_t... I>
+void call_abi(int (*fn)(A...), PyObject* const* a, std::index_sequence<I...>) {
+  using Types = std::tuple<A...>;
+  std::tuple<std::tuple_element_t<I, Types>...> v{from_py<std::tuple_element_t<I, Types>>(a[I])...};
+  void* st = stream();
+  LAUNCH(fn(std::get<I>(v)..., st));
+}
+template <class... A>
+PyObject* abi(int (*fn)(A...), PyObject* const* a) {
+  call_abi(fn, a, std::make_index_sequence<sizeof...(A) - 1>());
+  Py_RETURN_NONE;
+}
+template <class F>
+struct AbiArgs;
+template <class... A>
+struct AbiArgs<int(A...)> { static constexpr int value = int(sizeof...(A)) - 1; };
+PyObject* abi_scan(PyObject* const* a) { return abi(api.dsa_indexer_scan_fp8, a); }
+PyObject* abi_scan_paged(PyObject* const* a) { return abi(api.dsa_indexer_scan_fp8_paged, a); }
+PyObject* abi_topk(PyObject* const* a) { return abi(api.dsa_topk_select, a); }
+PyObject* abi_mla(PyObject* const* a) { return abi(api.dsa_sparse_mla_decode, a); }
+
+// ---------------------------------------------------------------- module
+template <PyObject* (*fn)(PyObject* const*), int n_args>
+PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != n_args) {
+    PyErr_Format(PyExc_TypeError, "expected %d arguments, got %zd", n_args, n);
+    return nullptr;
+  }
+  try {
+    return fn(args);
+  } catch (const PyErrorSet&) {
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+
+// bind({name: address}, check): the functions of the loaded library and the status check that raises
+PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 2 || !PyDict_Check(args[0])) {
+    PyErr_SetString(PyExc_TypeError, "bind(addresses, check)");
+    return nullptr;
+  }
+#define X(name)                                                                       \
+  {                                                                                   \
+    PyObject* v = PyDict_GetItemString(args[0], #name);                               \
+    if (!v) {                                                                         \
+      PyErr_SetString(PyExc_ImportError, "the library does not provide " #name);      \
+      return nullptr;                                                                 \
+    }                                                                                 \
+    void* p = PyLong_AsVoidPtr(v);                                                    \
+    if (!p && PyErr_Occurred()) return nullptr;                                       \
+    api.name = reinterpret_cast<decltype(&::name)>(p);                                \
+  }
+  DSA_HOST_API(X)
+#undef X
+  Py_INCREF(args[1]);
+  Py_XSETREF(status_check, args[1]);
+  Py_RETURN_NONE;
+}
+
+#define M(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&entry<name, n>)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {
+    {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&bind)), METH_FASTCALL, nullptr},
+    M(scan_fp8, 10), M(scan_paged, 8), M(scan_f32, 7), M(topk, 11), M(topk_paged, 7), M(mla, 14), M(mla_f32, 7), M(rmsnorm, 3),
+    M(add_rmsnorm, 4), M(silu_mul, 2), M(indexer_stage, 18), M(latent_append, 11), M(prefill_latents, 16), M(prefill_queries, 13),
+    M(abi_scan, AbiArgs<decltype(::dsa_indexer_scan_fp8)>::value), M(abi_scan_paged, AbiArgs<decltype(::dsa_indexer_scan_fp8_paged)>::value),
+    M(abi_topk, AbiArgs<decltype(::dsa_topk_select)>::value), M(abi_mla, AbiArgs<decltype(::dsa_sparse_mla_decode)>::value),
+    {nullptr, nullptr, 0, nullptr}};
+#undef M
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "native half of the tensor entry points", -1, methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module_def); }

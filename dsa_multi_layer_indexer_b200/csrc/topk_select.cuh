@@ -64,6 +64,8 @@ struct Params {
   int topk;
   int32_t pad;
   int32_t index_offset;
+  const int32_t* page_table;  // kPages only: the selection as slots page_table[r][position / 64] * 64 + position % 64
+  int64_t pt_stride;
   // ---- candidate exchange between the GPUs of a sequence-sharded indexer (cluster kernel only)
   // Push side (n_dest > 0): the selection of row r goes, as (index, logit), into slot `src_rank`
   // of every rank's gather buffers [2 parities][R][n_dest][topk], then flag word
@@ -815,7 +817,10 @@ __device__ __forceinline__ void cluster_sync_all(bool solo) {
 // map, indices only. It is the same code with those features compiled out, so that the kernel
 // every decode step runs is small (it alternates with three other kernels on the same SMs, and
 // its time in a step follows its size; alone, both forms take the same time).
-template <bool kPlain, int kMaxC = kClMaxCtas>
+// kPages: positions leave as slots of the row's 64-token pages (the serving form; seven elementwise
+// launches behind the top-k before). A mask word's 32 positions lie in one page, so a lane needs one
+// table entry, requested right after the dependency wait.
+template <bool kPlain, int kMaxC = kClMaxCtas, bool kPages = false>
 __global__ void __launch_bounds__(kClThreads, 1)
 topk_cluster_kernel(const Params p, const int nk) {
   extern __shared__ __align__(128) uint8_t topk_cl_smem[];
@@ -853,6 +858,13 @@ topk_cluster_kernel(const Params p, const int nk) {
   pdl_wait();
   DSA_STAMP(stamp_cta, 15);
   const int R = int(gridDim.y);
+  int32_t page = 0;  // kPages: the page of this lane's word of the emission
+  if constexpr (kPages) {
+    int G = 1;
+    while (2 * G * nk <= 32) G *= 2;
+    const int first = int(c) * kClThreads * nk + warp * (32 * nk) + (lane / G) * 32;
+    if (lane / G < nk && first < p.n) page = p.page_table[int64_t(r) * p.pt_stride + (first >> 6)];
+  }
   // ---- loads. The CTA's slice (positions slice_base .. + span) comes into shared memory as it
   // lies in global memory, by one bulk copy when the row is 16-byte aligned. Thread (warp, lane)
   // then owns positions warp_off + i * 32 + lane of the slice, i < nk: conflict-free reads, and
@@ -1319,7 +1331,9 @@ topk_cluster_kernel(const Params p, const int nk) {
         int b;
         uint32_t slot;
         next_bit(b, slot);
-        if (slot < topk_u) store(b, slot, imap_staged ? int32_t(wvals[span + b]) : word_base + b + p.index_offset);
+        if (slot < topk_u)
+          store(b, slot, kPages ? page * DSA_PAGE_TOKENS + ((word_base + b) & (DSA_PAGE_TOKENS - 1))
+                                : imap_staged ? int32_t(wvals[span + b]) : word_base + b + p.index_offset);
       }
     } else {
       // index map in global memory: four set bits at a time, so that their loads travel together

@@ -25,22 +25,13 @@ from . import _lib, ops
 
 _DQK, _DV, _DIDX = 576, 512, 128
 
-
-def _st() -> int:
-    return torch.cuda.current_stream().cuda_stream
-
-
-def _p(t):
-    return None if t is None else t.data_ptr()
-
-
 _LENS = {}
 
 
 def _causal_lens(S: int, Skv: int, device) -> torch.Tensor:
     """Visible keys of each of the S query rows of one sequence (row s sees Skv - S + s + 1),
     built once per (S, Skv, device): a launch then allocates nothing and stays capturable."""
-    key = (S, Skv, str(device))
+    key = (S, Skv, device)
     lens = _LENS.get(key)
     if lens is None:
         lens = _LENS[key] = torch.arange(Skv - S + 1, Skv + 1, dtype=torch.int32, device=device)
@@ -62,16 +53,15 @@ class FusedSparseSplitK:
                                    with_select, attn_on, win):
         """One sequence, S query rows; row s sees keys [0, Skv - S + s]."""
         _check_modes(with_select, win)
-        lib = _lib.lib()
+        host = _lib.host()
         lens = _causal_lens(S, Skv, Q.device)
         if attn_on:
-            _lib.check(lib.dsa_sparse_mla_decode(_p(Q), _p(KV), _p(Indices), _p(lens), _p(PartAcc), _p(PartM),
-                                                 _p(PartL), _p(Out), S, S, H, topk, nsplit, float(sm_scale), Skv, 0,
-                                                 _st()))
+            host.abi_mla(Q, KV, Indices, lens, PartAcc, PartM, PartL, Out, S, S, H, topk, nsplit, float(sm_scale),
+                         Skv, 0)
         if with_select:
             hist = SelHist if with_select == 2 else None
-            _lib.check(lib.dsa_indexer_scan_fp8(_p(IndexQ), _p(IndexW), _p(IndexK), _p(IndexKScale), _p(lens),
-                                                _p(SelSlab), _p(hist), S, S, Hidx, Skv, 1, Skv, Skv, Skv, 0, _st()))
+            host.abi_scan(IndexQ, IndexW, IndexK, IndexKScale, lens, SelSlab, hist, S, S, Hidx, Skv, 1, Skv, Skv, Skv,
+                          0)
 
     def launch_fused_sparse_splitk_batch_idx(self, Q, KV, Indices, IndexQ, IndexK, IndexW, IndexKScale, PartAcc,
                                              PartM, PartL, SelSlab, SelHist, Out, S, Skv, H, Hidx, topk, nsplit,
@@ -82,16 +72,14 @@ class FusedSparseSplitK:
         _check_modes(with_select, win)
         if kv_stride % _DQK or idx_k_stride % _DIDX:
             raise RuntimeError("kv_stride / idx_k_stride must be whole rows")
-        lib = _lib.lib()
+        host = _lib.host()
         if attn_on:
-            _lib.check(lib.dsa_sparse_mla_decode(_p(Q), _p(KV), _p(Indices), None, _p(PartAcc), _p(PartM), _p(PartL),
-                                                 _p(Out), S, 1, H, topk, nsplit, float(sm_scale), kv_stride // _DQK,
-                                                 0, _st()))
+            host.abi_mla(Q, KV, Indices, None, PartAcc, PartM, PartL, Out, S, 1, H, topk, nsplit, float(sm_scale),
+                         kv_stride // _DQK, 0)
         if with_select:
             hist = SelHist if with_select == 2 else None
-            _lib.check(lib.dsa_indexer_scan_fp8(_p(IndexQ), _p(IndexW), _p(IndexK), _p(IndexKScale), None,
-                                                _p(SelSlab), _p(hist), S, 1, Hidx, Skv, S, idx_k_stride // _DIDX,
-                                                idx_scale_stride, Skv, 0, _st()))
+            host.abi_scan(IndexQ, IndexW, IndexK, IndexKScale, None, SelSlab, hist, S, 1, Hidx, Skv, S, idx_k_stride
+                          // _DIDX, idx_scale_stride, Skv, 0)
 
     def launch_fused_sparse_splitk_paged(self, Q, KV, Indices, IndexQ, IndexKPaged, IndexW, SeqLens, PageTable,
                                          PartAcc, PartM, PartL, SelSlab, SelHist, Out, S, Skv, H, Hidx, topk, nsplit,
@@ -103,27 +91,23 @@ class FusedSparseSplitK:
         _check_modes(with_select, 0)
         if page_bytes != ops.INDEX_PAGE_BYTES:
             raise RuntimeError(f"page_bytes must be {ops.INDEX_PAGE_BYTES}")
-        lib = _lib.lib()
+        host = _lib.host()
         n_att = nsplit_attn if nsplit_attn and nsplit_attn > 0 else nsplit
         if attn_on:
             if kv_fp8:  # one shared pool of kv_rows slots; Indices are slot numbers
-                _lib.check(lib.dsa_sparse_mla_decode(_p(Q), _p(KV), _p(Indices), None, _p(PartAcc), _p(PartM),
-                                                     _p(PartL), _p(Out), S, S, H, topk, n_att, float(sm_scale),
-                                                     kv_rows, 1, _st()))
+                host.abi_mla(Q, KV, Indices, None, PartAcc, PartM, PartL, Out, S, S, H, topk, n_att, float(sm_scale),
+                             kv_rows, 1)
             else:
-                _lib.check(lib.dsa_sparse_mla_decode(_p(Q), _p(KV), _p(Indices), _p(SeqLens), _p(PartAcc), _p(PartM),
-                                                     _p(PartL), _p(Out), S, 1, H, topk, n_att, float(sm_scale),
-                                                     kv_stride // _DQK, 0, _st()))
+                host.abi_mla(Q, KV, Indices, SeqLens, PartAcc, PartM, PartL, Out, S, 1, H, topk, n_att,
+                             float(sm_scale), kv_stride // _DQK, 0)
         if with_select:
             hist = SelHist if (with_select == 2 or sel_on) else None
             slab = slab_stride if slab_stride and slab_stride > 0 else Skv
-            _lib.check(lib.dsa_indexer_scan_fp8_paged(_p(IndexQ), _p(IndexW), _p(IndexKPaged), IndexKPaged.shape[0],
-                                                      _p(PageTable), pt_stride, _p(SeqLens), _p(SelSlab), _p(hist),
-                                                      S, Hidx, Skv, slab, _st()))
+            host.abi_scan_paged(IndexQ, IndexW, IndexKPaged, IndexKPaged.shape[0], PageTable, pt_stride, SeqLens,
+                                SelSlab, hist, S, Hidx, Skv, slab)
             if sel_on:  # in-launch selection: SelScratch is the top-k workspace, NextIdx the result
-                _lib.check(lib.dsa_topk_select(_p(SelSlab), _p(SeqLens), _p(hist), None, _p(NextIdx), None,
-                                               _p(SelScratch), SelScratch.numel() * SelScratch.element_size(), S, Skv,
-                                               slab, topk, -1, 0, _st()))
+                host.abi_topk(SelSlab, SeqLens, hist, None, NextIdx, None, SelScratch, SelScratch.numel() *
+                              SelScratch.element_size(), S, Skv, slab, topk, -1, 0)
 
 
 def build() -> FusedSparseSplitK:

@@ -3,7 +3,8 @@ device pointers and the current CUDA stream to libdsa_b200.so.
 
 torch is used here for device memory and streams only. Nothing in this module
 computes on the host or falls back to torch kernels; a missing library raises
-at the first call (``_lib.lib()``).
+at the first call (``_lib.lib()``). The entry points of a step run their checks, allocations and
+the call natively (``_lib.host()``, csrc/host_ops.cpp); the rest goes through ctypes.
 """
 
 from __future__ import annotations
@@ -25,6 +26,9 @@ FP8_LATENT_ROW = 656
 HIST_BINS = 4096
 
 _FP8 = torch.float8_e4m3fn
+_STAGES = {"both": 0, "partials": 1, "combine": 2}
+_LATENT_FORMATS = {"bf16": 0, "bf16_quant": 1, "fp8": 2}
+_host = _lib.host
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -42,14 +46,6 @@ def _need(cond: bool, msg: str) -> None:
 
 def _cuda_contig(t: torch.Tensor, name: str, dtypes) -> None:
     _need(t.is_cuda, f"{name} must be a CUDA tensor")
-    _need(t.is_contiguous(), f"{name} must be contiguous")
-    _need(t.dtype in dtypes, f"{name} has dtype {t.dtype}, expected one of {dtypes}")
-
-
-def _out_contig(t: torch.Tensor, name: str, dtypes) -> None:
-    """An output may also live in pinned host memory (it is mapped into the device's
-    address space): the kernel then writes the result straight to the host."""
-    _need(t.is_cuda or t.is_pinned(), f"{name} must be a CUDA tensor or pinned host memory")
     _need(t.is_contiguous(), f"{name} must be contiguous")
     _need(t.dtype in dtypes, f"{name} has dtype {t.dtype}, expected one of {dtypes}")
 
@@ -95,34 +91,7 @@ def indexer_scan_fp8(
     with the query scale folded in, index_k ``[n_seq, cap, 128]`` (or ``[cap, 128]``),
     k_scale ``[n_seq, cap]`` fp32. Row r reads sequence ``r // rows_per_seq``.
     """
-    _cuda_contig(index_q, "index_q", (_FP8, torch.uint8))
-    _cuda_contig(index_w, "index_w", (torch.float32,))
-    _cuda_contig(index_k, "index_k", (_FP8, torch.uint8))
-    _cuda_contig(k_scale, "k_scale", (torch.float32,))
-    _need(index_q.dim() == 3 and index_q.shape[-1] == INDEX_DIM, "index_q must be [R, Hidx, 128]")
-    R, n_heads = index_q.shape[0], index_q.shape[1]
-    _need(tuple(index_w.shape) == (R, n_heads), "index_w must be [R, Hidx]")
-    if index_k.dim() == 2:
-        index_k = index_k.unsqueeze(0)
-        k_scale = k_scale.reshape(1, -1)
-    _need(index_k.dim() == 3 and index_k.shape[-1] == INDEX_DIM, "index_k must be [n_seq, cap, 128]")
-    n_seq, cap = index_k.shape[0], index_k.shape[1]
-    _need(tuple(k_scale.shape) == (n_seq, cap), "k_scale must be [n_seq, cap]")
-    _need(R == n_seq * rows_per_seq, f"R={R} must equal n_seq={n_seq} * rows_per_seq={rows_per_seq}")
-    ctx = cap if ctx is None else int(ctx)
-    _need(0 < ctx <= cap, "ctx must be in (0, cap]")
-    seq_lens = _lens(seq_lens, R)
-    if out is None:
-        out = torch.empty(R, (ctx + 3) // 4 * 4, dtype=torch.float32, device=index_q.device)
-    _cuda_contig(out, "out", (torch.float32,))
-    _need(out.dim() == 2 and out.shape[0] == R and out.shape[1] >= ctx, "out must be [R, >= ctx]")
-    if hist is not None:
-        _cuda_contig(hist, "hist", (torch.int32, torch.uint32))
-        _need(hist.numel() == R * HIST_BINS, "hist must be [R, 4096]")
-    _lib.check(_lib.lib().dsa_indexer_scan_fp8(
-        _ptr(index_q), _ptr(index_w), _ptr(index_k), _ptr(k_scale), _ptr(seq_lens), _ptr(out),
-        _ptr(hist), R, rows_per_seq, n_heads, ctx, n_seq, cap, cap, out.shape[1], impl, _stream()))
-    return out[:, :ctx]
+    return _host().scan_fp8(index_q, index_w, index_k, k_scale, seq_lens, rows_per_seq, ctx, out, hist, impl)
 
 
 def indexer_scan_fp8_paged(
@@ -137,31 +106,7 @@ def indexer_scan_fp8_paged(
     hist: Optional[torch.Tensor] = None,
 ) -> torch.Tensor:
     """Paged form: index_k_pages ``[num_pages, 8448]`` uint8, page_table ``[R, pt_stride]`` int32."""
-    _cuda_contig(index_q, "index_q", (_FP8, torch.uint8))
-    _cuda_contig(index_w, "index_w", (torch.float32,))
-    _cuda_contig(index_k_pages, "index_k_pages", (torch.uint8,))
-    _cuda_contig(page_table, "page_table", (torch.int32,))
-    _need(index_q.dim() == 3 and index_q.shape[-1] == INDEX_DIM, "index_q must be [R, Hidx, 128]")
-    R, n_heads = index_q.shape[0], index_q.shape[1]
-    _need(index_k_pages.dim() == 2 and index_k_pages.shape[1] == INDEX_PAGE_BYTES,
-          "index_k_pages must be [num_pages, 8448]")
-    _need(page_table.dim() == 2 and page_table.shape[0] == R, "page_table must be [R, pt_stride]")
-    seq_lens = _lens(seq_lens, R)
-    _need(seq_lens is not None, "paged scan needs seq_lens")
-    if out is None:
-        out = torch.empty(R, (ctx + 3) // 4 * 4, dtype=torch.float32, device=index_q.device)
-    _cuda_contig(out, "out", (torch.float32,))
-    _need(out.dim() == 2 and out.shape[0] == R and out.shape[1] >= ctx, "out must be [R, >= ctx]")
-    _need(tuple(index_w.shape) == (R, n_heads), "index_w must be [R, Hidx]")
-    _need(page_table.shape[1] * PAGE_TOKENS >= ctx, "page_table rows cannot cover ctx positions")
-    if hist is not None:
-        _cuda_contig(hist, "hist", (torch.int32, torch.uint32))
-        _need(hist.numel() == R * HIST_BINS, "hist must be [R, 4096]")
-    _lib.check(_lib.lib().dsa_indexer_scan_fp8_paged(
-        _ptr(index_q), _ptr(index_w), _ptr(index_k_pages), index_k_pages.shape[0], _ptr(page_table),
-        page_table.shape[1], _ptr(seq_lens), _ptr(out), _ptr(hist), R, n_heads, int(ctx),
-        out.shape[1], _stream()))
-    return out[:, :ctx]
+    return _host().scan_paged(index_q, index_w, index_k_pages, page_table, seq_lens, ctx, out, hist)
 
 
 def indexer_scan_f32(
@@ -176,23 +121,7 @@ def indexer_scan_f32(
 ) -> torch.Tensor:
     """fp32 logits for any head count / key width: q ``[R, H, D]``, k ``[n_seq, cap, D]`` of which
     the first ``ctx`` keys are scanned (default: all)."""
-    for t, n in ((index_q, "index_q"), (index_w, "index_w"), (index_k, "index_k")):
-        _cuda_contig(t, n, (torch.float32,))
-    R, n_heads, d = index_q.shape
-    if index_k.dim() == 2:
-        index_k = index_k.unsqueeze(0)
-    n_seq, cap = index_k.shape[0], index_k.shape[1]
-    ctx = cap if ctx is None else int(ctx)
-    _need(0 < ctx <= cap, "ctx must be in (0, cap]")
-    _need(index_k.shape[2] == d, "index_k width differs from index_q")
-    _need(R == n_seq * rows_per_seq, "R must equal n_seq * rows_per_seq")
-    seq_lens = _lens(seq_lens, R)
-    if out is None:
-        out = torch.empty(R, (ctx + 3) // 4 * 4, dtype=torch.float32, device=index_q.device)
-    _lib.check(_lib.lib().dsa_indexer_scan_f32(
-        _ptr(index_q), _ptr(index_w), _ptr(index_k), _ptr(seq_lens), _ptr(out), R, rows_per_seq,
-        n_heads, d, ctx, cap, out.shape[1], _stream()))
-    return out[:, :ctx]
+    return _host().scan_f32(index_q, index_w, index_k, seq_lens, rows_per_seq, ctx, out)
 
 
 # --------------------------------------------------------------------------- a3
@@ -221,38 +150,15 @@ def topk_select(
     """Exact top-k per row of ``logits[R, n]`` (a view of a wider slab is fine):
     int32 positions in ascending order, ties to the lower position, padded with
     ``pad_value``."""
-    _need(logits.is_cuda and logits.dtype == torch.float32 and logits.dim() == 2, "logits must be CUDA fp32 [R, n]")
-    _need(logits.stride(1) == 1, "logits rows must be dense")
-    R, n = logits.shape
-    slab_stride = logits.stride(0) if R > 1 else max(logits.stride(0), n)
-    seq_lens = _lens(seq_lens, R)
-    if index_map is not None:
-        _cuda_contig(index_map, "index_map", (torch.int32,))
-        _need(tuple(index_map.shape) == (R, n), "index_map must be [R, n]")
-    if out_idx is None:
-        out_idx = torch.empty(R, topk, dtype=torch.int32, device=logits.device)
-    _cuda_contig(out_idx, "out_idx", (torch.int32,))
-    _need(tuple(out_idx.shape) == (R, topk), f"out_idx must be [R, topk] = [{R}, {topk}]")
-    if out_val is None and return_values:
-        out_val = torch.empty(R, topk, dtype=torch.float32, device=logits.device)
-    if out_val is not None:
-        _cuda_contig(out_val, "out_val", (torch.float32,))
-        _need(tuple(out_val.shape) == (R, topk), f"out_val must be [R, topk] = [{R}, {topk}]")
-    if hist is not None:
-        _cuda_contig(hist, "hist", (torch.int32, torch.uint32))
-        _need(hist.numel() == R * HIST_BINS, "hist must be [R, 4096]")
-    if workspace is None:
-        # a fresh zeroed scratch per call is always safe; steady-state callers pass their own
-        workspace = topk_workspace(R, n, logits.device)
-    _cuda_contig(workspace, "workspace", (torch.uint8,))
-    _need(0 < int(topk) <= 65536, "topk must be in [1, 65536]")
-    _lib.check(_lib.lib().dsa_topk_select(
-        _ptr(logits), _ptr(seq_lens), _ptr(hist), _ptr(index_map), _ptr(out_idx), _ptr(out_val),
-        _ptr(workspace), workspace.numel(), R, n, slab_stride, int(topk), int(pad_value),
-        int(index_offset), _stream()))
-    if return_values or out_val is not None:
-        return out_idx, out_val
-    return out_idx
+    return _host().topk(logits, topk, seq_lens, hist, index_map, pad_value, index_offset, out_idx, out_val, return_values,
+                        workspace)
+
+
+def topk_select_paged(logits: torch.Tensor, topk: int, seq_lens: Optional[torch.Tensor], hist: torch.Tensor,
+                      page_table: torch.Tensor, out_idx: torch.Tensor, pad_value: int = -1) -> torch.Tensor:
+    """:func:`topk_select` over paged caches: ``out_idx`` receives cache slots,
+    ``page_table[r, p // 64] * 64 + p % 64`` for position p (rows that need no workspace)."""
+    return _host().topk_paged(logits, topk, seq_lens, hist, page_table, pad_value, out_idx)
 
 
 # --------------------------------------------------------------------------- a4, a5
@@ -307,55 +213,14 @@ def sparse_mla_decode(
     ``beside_previous``: none of the operands comes from the two kernels enqueued just before
     this call (the lagged schedule's attention behind this layer's scan and top-k); the attention
     then runs beside the top-k and completes after it."""
-    _cuda_contig(q, "q", (torch.bfloat16,))
-    _need(q.dim() == 3 and q.shape[2] == LATENT_DIM, "q must be [R, H, 576]")
-    R, H = q.shape[0], q.shape[1]
-    _need(H % HEAD_BLOCK == 0, f"H={H} must be a multiple of {HEAD_BLOCK} (pad heads with zero queries)")
-    if kv.dim() == 2:
-        kv = kv.unsqueeze(0)
-    _need(kv.is_cuda and kv.is_contiguous() and kv.dim() == 3, "kv must be a contiguous CUDA [n_seq, cap, w] tensor")
-    if kv.dtype == torch.bfloat16:
-        _need(kv.shape[2] == LATENT_DIM, "bf16 kv rows must be 576 wide")
-        kv_fp8 = 0
-    else:
-        _need(kv.dtype == torch.uint8 and kv.shape[2] == FP8_LATENT_ROW, "fp8 kv rows must be 656 bytes of uint8")
-        kv_fp8 = 1
-    n_seq, cap = kv.shape[0], kv.shape[1]
-    _need(R == n_seq * rows_per_seq, "R must equal n_seq * rows_per_seq")
-    if indices is not None:
-        _cuda_contig(indices, "indices", (torch.int32,))
-        _need(indices.dim() == 2 and indices.shape[0] == R, "indices must be [R, topk]")
-        topk = indices.shape[1]
-    else:
-        topk = int(dense_keys if dense_keys is not None else cap)
-    seq_lens = _lens(seq_lens, R)
-    if nsplit is None:
-        nsplit = scratch.nsplit if scratch is not None else default_nsplit(R, H, topk)
-    if scratch is None and (nsplit > 1 or stage != "both"):  # (one split: the result is written at once)
-        scratch = MlaScratch(R, H, nsplit, q.device)
-    _need(scratch is None or (scratch.rows >= R and scratch.heads == H and scratch.nsplit == nsplit),
-          "scratch does not match the launch")
-    acc, m, l = (None, None, None) if scratch is None else (scratch.acc, scratch.m, scratch.l)
-    if out is None:
-        out = torch.empty(R, H, VALUE_DIM, dtype=torch.bfloat16, device=q.device)
-    _out_contig(out, "out", (torch.bfloat16,))
-    _need(not beside_previous or stage == "both", "beside_previous goes with stage='both'")
-    if stage == "both":
-        fn = _lib.lib().dsa_sparse_mla_decode_beside if beside_previous else _lib.lib().dsa_sparse_mla_decode
-        _lib.check(fn(
-            _ptr(q), _ptr(kv), _ptr(indices), _ptr(seq_lens), _ptr(acc), _ptr(m),
-            _ptr(l), _ptr(out), R, rows_per_seq, H, topk, nsplit, float(sm_scale), cap, kv_fp8,
-            _stream()))
-    elif stage == "partials":  # the two halves separately, as the reference schedules them
-        _lib.check(_lib.lib().dsa_sparse_mla_partials(
-            _ptr(q), _ptr(kv), _ptr(indices), _ptr(seq_lens), _ptr(acc), _ptr(m),
-            _ptr(l), R, rows_per_seq, H, topk, nsplit, float(sm_scale), cap, kv_fp8, _stream()))
-    elif stage == "combine":
-        _lib.check(_lib.lib().dsa_sparse_mla_combine(
-            _ptr(acc), _ptr(m), _ptr(l), _ptr(out), R, H, nsplit, _stream()))
-    else:
+    if stage not in _STAGES:
         raise ValueError(f"unknown stage {stage!r}")
-    return out
+    if scratch is None:
+        acc = m = l = None
+    else:
+        acc, m, l = scratch.acc, scratch.m, scratch.l
+    return _host().mla(q, kv, indices, sm_scale, seq_lens, rows_per_seq, nsplit, acc, m, l, out, dense_keys, _STAGES[stage],
+                       beside_previous)
 
 
 def sparse_mla_f32(
@@ -370,23 +235,7 @@ def sparse_mla_f32(
 ) -> torch.Tensor:
     """fp32 attention for any width: q ``[R, H, Dqk]``, kv ``[n_seq, ctx, Dqk]``;
     indices None = dense causal over ``seq_lens``."""
-    _cuda_contig(q, "q", (torch.float32,))
-    _cuda_contig(kv, "kv", (torch.float32,))
-    if kv.dim() == 2:
-        kv = kv.unsqueeze(0)
-    R, H, dqk = q.shape
-    n_seq, ctx = kv.shape[0], kv.shape[1]
-    _need(kv.shape[2] == dqk and R == n_seq * rows_per_seq, "q / kv shapes disagree")
-    topk = 0
-    if indices is not None:
-        _cuda_contig(indices, "indices", (torch.int32,))
-        topk = indices.shape[1]
-    seq_lens = _lens(seq_lens, R)
-    out = torch.empty(R, H, value_dim, dtype=torch.float32, device=q.device)
-    _lib.check(_lib.lib().dsa_sparse_mla_f32(
-        _ptr(q), _ptr(kv), _ptr(indices), _ptr(seq_lens), _ptr(out), R, rows_per_seq, H, dqk,
-        value_dim, topk, float(sm_scale), ctx, _stream()))
-    return out
+    return _host().mla_f32(q, kv, indices, value_dim, sm_scale, seq_lens, rows_per_seq)
 
 
 # --------------------------------------------------------------------------- a6
@@ -456,40 +305,19 @@ def fused_decode(
 # --------------------------------------------------------------------------- decode-step preparation
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
     """RMSNorm over the last dimension in one launch (fp32 math, one rounding)."""
-    _need(x.is_cuda and x.dtype in (torch.float32, torch.bfloat16), "x must be CUDA fp32 / bf16")
-    x = x.contiguous()
-    w = weight if weight.dtype == x.dtype else weight.to(x.dtype)
-    out = torch.empty_like(x)
-    dim = x.shape[-1]
-    _lib.check(_lib.lib().dsa_rmsnorm(_ptr(x), _ptr(w.contiguous()), _ptr(out), x.numel() // dim, dim, float(eps),
-                                      0 if x.dtype == torch.float32 else 1, _stream()))
-    return out
+    return _host().rmsnorm(x, weight, eps)
 
 
 def add_rmsnorm(x: torch.Tensor, delta: torch.Tensor, weight: torch.Tensor, eps: float):
     """``s = x + delta`` and ``rmsnorm(s)`` in one launch (bf16 rows of at most 8192
     elements, a multiple of 8): returns ``(s, normed)``, both rounded exactly as the
     separate addition and norm would be."""
-    _need(x.is_cuda and x.dtype == torch.bfloat16 and delta.dtype == torch.bfloat16 and x.shape == delta.shape,
-          "x and delta must be CUDA bf16 tensors of one shape")
-    dim = x.shape[-1]
-    _need(dim % 8 == 0 and dim <= 8192, "the row length must be a multiple of 8 and at most 8192")
-    x, delta = x.contiguous(), delta.contiguous()
-    w = (weight if weight.dtype == x.dtype else weight.to(x.dtype)).contiguous()
-    s, out = torch.empty_like(x), torch.empty_like(x)
-    _lib.check(_lib.lib().dsa_add_rmsnorm_bf16(_ptr(x), _ptr(delta), _ptr(w), _ptr(s), _ptr(out), x.numel() // dim, dim,
-                                               float(eps), _stream()))
-    return s, out
+    return _host().add_rmsnorm(x, delta, weight, eps)
 
 
 def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     """``silu(gate) * up`` over bf16 tensors in one launch, rounded as the two separate operations."""
-    _need(gate.is_cuda and gate.dtype == torch.bfloat16 and up.dtype == torch.bfloat16 and gate.shape == up.shape,
-          "gate and up must be CUDA bf16 tensors of one shape")
-    gate, up = gate.contiguous(), up.contiguous()
-    out = torch.empty_like(gate)
-    _lib.check(_lib.lib().dsa_silu_mul_bf16(_ptr(gate), _ptr(up), _ptr(out), gate.numel(), _stream()))
-    return out
+    return _host().silu_mul(gate, up)
 
 
 def copy_bytes(dst: torch.Tensor, src: torch.Tensor, beside_previous: bool = False) -> None:
@@ -563,42 +391,9 @@ def indexer_stage_fp8(q_raw, k_raw, w_raw, k_norm_weight, k_norm_bias, k_norm_ep
     (``cache_index_k`` [B, cap, 128] u8 + ``cache_k_scale`` [B, cap]) or to 64-token
     ``pages`` through ``page_table``. ``q_raw`` [B, heads, 128] / ``k_raw`` [B, 128] bf16,
     ``w_raw`` [B, heads] fp32, ``rope_cos`` / ``rope_sin`` [cap, 32] fp32."""
-    _cuda_contig(q_raw, "q_raw", (torch.bfloat16,))
-    _cuda_contig(k_raw, "k_raw", (torch.bfloat16,))
-    for t, n in ((w_raw, "w_raw"), (k_norm_weight, "k_norm_weight"), (k_norm_bias, "k_norm_bias"),
-                 (rope_cos, "rope_cos"), (rope_sin, "rope_sin"), (index_w, "index_w")):
-        _cuda_contig(t, n, (torch.float32,))
-    _cuda_contig(positions, "positions", (torch.int64,))
-    _cuda_contig(index_q, "index_q", (torch.uint8, torch.float8_e4m3fn))
-    _need(q_raw.dim() == 3 and q_raw.shape[2] == INDEX_DIM, "q_raw must be [B, heads, 128]")
-    B, n_heads = q_raw.shape[0], q_raw.shape[1]
-    _need(k_raw.shape == (B, INDEX_DIM) and w_raw.shape == (B, n_heads) and index_w.shape == (B, n_heads)
-          and index_q.shape == q_raw.shape and positions.shape == (B,), "operand shapes disagree")
-    _need(k_norm_weight.numel() == INDEX_DIM and k_norm_bias.numel() == INDEX_DIM, "LayerNorm parameters must be [128]")
-    cap = rope_cos.shape[0]
-    _need(rope_cos.shape == (cap, 32) and rope_sin.shape == (cap, 32), "rotary tables must be [cap, 32]")
-    paged = pages is not None
-    if paged:
-        _cuda_contig(pages, "pages", (torch.uint8,))
-        _cuda_contig(page_table, "page_table", (torch.int32,))
-        _need(page_table.dim() == 2 and page_table.shape[0] == B, "page_table must be [B, pages per sequence]")
-        _need(pages.numel() % INDEX_PAGE_BYTES == 0, "page pool must be whole pages")
-        cap = min(cap, page_table.shape[1] * PAGE_TOKENS)
-    else:
-        _cuda_contig(cache_index_k, "cache_index_k", (torch.uint8, torch.float8_e4m3fn))
-        _cuda_contig(cache_k_scale, "cache_k_scale", (torch.float32,))
-        _need(cache_index_k.dim() == 3 and cache_index_k.shape[0] == B and cache_index_k.shape[2] == INDEX_DIM
-              and cache_k_scale.shape == cache_index_k.shape[:2], "caches must be [B, cap, 128] and [B, cap]")
-        cap = min(cap, cache_index_k.shape[1])
-    if softmax_scale is None:
-        softmax_scale = INDEX_DIM ** -0.5
-    _lib.check(_lib.lib().dsa_indexer_stage_fp8(
-        _ptr(q_raw), _ptr(k_raw), _ptr(w_raw), _ptr(k_norm_weight), _ptr(k_norm_bias), float(k_norm_eps),
-        _ptr(rope_cos), _ptr(rope_sin), _ptr(positions), _ptr(index_q), _ptr(index_w),
-        _ptr(cache_index_k) if not paged else None, _ptr(cache_k_scale) if not paged else None,
-        _ptr(pages) if paged else None, pages.numel() // INDEX_PAGE_BYTES if paged else 0,
-        _ptr(page_table) if paged else None, page_table.shape[1] if paged else 0, B, n_heads, cap, 1 if rope_interleave else 0,
-        0 if scale_fmt is None else 1, float(n_heads ** -0.5), float(softmax_scale), _stream()))
+    _host().indexer_stage(q_raw, k_raw, w_raw, k_norm_weight, k_norm_bias, k_norm_eps, rope_cos, rope_sin, positions, index_q,
+                          index_w, cache_index_k, cache_k_scale, pages, page_table, rope_interleave, scale_fmt is not None,
+                          softmax_scale)
 
 
 def latent_append(kv_a, kv_norm_weight, eps: float, rope_cos, rope_sin, positions, slots, pool,
@@ -608,29 +403,10 @@ def latent_append(kv_a, kv_norm_weight, eps: float, rope_cos, rope_sin, position
     embedding of its 64 rope dims, row written at ``slots[b]`` of ``pool``: ``fmt="bf16"``
     [n_slots, 576] bf16 as it is, ``"bf16_quant"`` the same with the latent dims passed
     through act_quant and back, ``"fp8"`` the 656-byte packed rows [n_slots, 656] uint8."""
-    _cuda_contig(kv_a, "kv_a", (torch.bfloat16,))
-    for t, n in ((kv_norm_weight, "kv_norm_weight"), (rope_cos, "rope_cos"), (rope_sin, "rope_sin")):
-        _cuda_contig(t, n, (torch.float32,))
-    _cuda_contig(positions, "positions", (torch.int64,))
-    _cuda_contig(slots, "slots", (torch.int64,))
-    _need(kv_a.dim() == 2 and kv_a.shape[1] == LATENT_DIM, "kv_a must be [B, 576]")
-    B = kv_a.shape[0]
-    _need(positions.shape == (B,) and slots.shape == (B,), "positions and slots must be [B]")
-    _need(kv_norm_weight.numel() == VALUE_DIM, "kv_norm_weight must be [512]")
-    cap = rope_cos.shape[0]
-    _need(rope_cos.shape == (cap, 32) and rope_sin.shape == (cap, 32), "rotary tables must be [cap, 32]")
-    formats = {"bf16": 0, "bf16_quant": 1, "fp8": 2}
-    _need(fmt in formats, f"fmt must be one of {sorted(formats)}")
-    if fmt == "fp8":
-        _cuda_contig(pool, "pool", (torch.uint8,))
-        _need(pool.dim() == 2 and pool.shape[1] == FP8_LATENT_ROW, "an fp8 pool is [n_slots, 656] uint8")
-    else:
-        _cuda_contig(pool, "pool", (torch.bfloat16,))
-        _need(pool.dim() == 2 and pool.shape[1] == LATENT_DIM, "a bf16 pool is [n_slots, 576]")
-    _lib.check(_lib.lib().dsa_latent_append(
-        _ptr(kv_a), _ptr(kv_norm_weight), float(eps), _ptr(rope_cos), _ptr(rope_sin), _ptr(positions), _ptr(slots),
-        _ptr(pool), B, cap, pool.shape[0], 1 if rope_interleave else 0, formats[fmt],
-        0 if scale_fmt is None else 1, _stream()))
+    if fmt not in _LATENT_FORMATS:
+        raise ValueError(f"fmt must be one of {sorted(_LATENT_FORMATS)}")
+    _host().latent_append(kv_a, kv_norm_weight, eps, rope_cos, rope_sin, positions, slots, pool, rope_interleave,
+                          _LATENT_FORMATS[fmt], scale_fmt is not None)
 
 
 def decode_prep(iq_raw, w_raw, ik_raw, kv_a, q_abs, q_pe, kv_norm_w, mla_cos, mla_sin, idx_cos, idx_sin,
@@ -661,55 +437,14 @@ def decode_prep(iq_raw, w_raw, ik_raw, kv_a, q_abs, q_pe, kv_norm_w, mla_cos, ml
 
 
 # --------------------------------------------------------------------------- full-sequence preparation
-def _rows(t: Optional[torch.Tensor], name: str, dtype) -> int:
-    """Row stride of a 2-D operand with dense rows (0 for None)."""
-    if t is None:
-        return 0
-    _need(t.is_cuda and t.dtype == dtype and t.dim() == 2 and t.stride(1) == 1, f"{name} must be CUDA {dtype} [rows, n] with dense rows")
-    return t.stride(0)
-
-
 def prefill_latents(qa, kv_a, ik, q_norm_w, kv_norm_w, rope, c_q, kv_out, ik_out, ik_scale, seq: int,
                     interleave: bool, eps: float) -> None:
     """Behind the GEMM that reads x_norm (see ``dsa_prefill_latents`` in the header): ``qa`` / ``kv_a`` /
     ``ik`` are 2-D row views (any may be None), ``kv_out`` ``[n_seq, cap, w]`` and ``ik_out``
     ``[n_seq, cap, D]`` (e4m3 bytes with ``ik_scale``, else the operands' type) receive their rows in
     place. ``rope``: tables of the operands' type (``RopeCaches``)."""
-    ref = next(t for t in (qa, kv_a, ik) if t is not None)
-    dt = ref.dtype
-    _need(dt in (torch.float32, torch.bfloat16), "operands must be fp32 or bf16")
-    strides = [_rows(t, n, dt) for t, n in ((qa, "qa"), (kv_a, "kv_a"), (ik, "ik"))]
-    rows = ref.shape[0]
-    _need(all(t is None or t.shape[0] == rows for t in (qa, kv_a, ik)), "operand rows disagree")
-    for t, n in ((rope.mla_cos, "mla_cos"), (rope.mla_sin, "mla_sin"), (rope.idx_cos, "idx_cos"), (rope.idx_sin, "idx_sin")):
-        _cuda_contig(t, n, (dt,))
-        _need(t.shape[0] >= seq, f"{n} is shorter than the sequence")
-    q_rank = kv_rank = rope_dim = idx_dim = kv_cap = ik_cap = 0
-    if qa is not None:
-        q_rank = qa.shape[1]
-        _cuda_contig(c_q, "c_q", (dt,))
-        _need(c_q.numel() == rows * q_rank and q_norm_w.numel() == q_rank and q_norm_w.dtype == dt, "c_q / q_norm_w shapes")
-    if kv_a is not None:
-        rope_dim = rope.mla_cos.shape[1]
-        kv_rank = kv_a.shape[1] - rope_dim
-        _cuda_contig(kv_out, "kv_out", (dt,))
-        _need(kv_out.dim() == 3 and kv_out.shape[2] == kv_a.shape[1] and kv_out.shape[0] * seq == rows
-              and kv_out.shape[1] >= seq and kv_norm_w.numel() == kv_rank and kv_norm_w.dtype == dt, "kv_out must be [n_seq, cap, w]")
-        kv_cap = kv_out.shape[1]
-    if ik is not None:
-        idx_dim = ik.shape[1]
-        _cuda_contig(ik_out, "ik_out", (torch.uint8, _FP8) if ik_scale is not None else (dt,))
-        _need(ik_out.dim() == 3 and ik_out.shape[2] == idx_dim and ik_out.shape[0] * seq == rows and ik_out.shape[1] >= seq
-              and rope.idx_cos.shape[1] == idx_dim, "ik_out must be [n_seq, cap, D]")
-        ik_cap = ik_out.shape[1]
-        if ik_scale is not None:
-            _cuda_contig(ik_scale, "ik_scale", (torch.float32,))
-            _need(ik_scale.shape == ik_out.shape[:2], "ik_scale must be [n_seq, cap]")
-    _lib.check(_lib.lib().dsa_prefill_latents(
-        _ptr(qa), strides[0], _ptr(kv_a), strides[1], _ptr(ik), strides[2], _ptr(q_norm_w), _ptr(kv_norm_w),
-        _ptr(rope.mla_cos), _ptr(rope.mla_sin), _ptr(rope.idx_cos), _ptr(rope.idx_sin), _ptr(c_q), _ptr(kv_out), kv_cap,
-        _ptr(ik_out), _ptr(ik_scale), ik_cap, rows, seq, q_rank, kv_rank, rope_dim, idx_dim, 1 if interleave else 0,
-        float(eps), 0 if dt == torch.float32 else 1, _stream()))
+    _host().prefill_latents(qa, kv_a, ik, q_norm_w, kv_norm_w, rope.mla_cos, rope.mla_sin, rope.idx_cos, rope.idx_sin, c_q,
+                            kv_out, ik_out, ik_scale, seq, interleave, eps)
 
 
 def prefill_queries(q, nope: int, iq, w, rope, q_full, index_q, index_w, seq: int, interleave: bool) -> None:
@@ -717,33 +452,8 @@ def prefill_queries(q, nope: int, iq, w, rope, q_full, index_q, index_w, seq: in
     strided view is fine) or None, ``iq`` / ``w`` 2-D row views or None; the rope columns of ``q_full``
     ``[rows, H, kv_rank + rope]`` and ``index_q`` ``[rows, Hidx, D]`` (e4m3 bytes with ``index_w``, else
     the operands' type) are written."""
-    ref = q if q is not None else iq
-    dt, rows = ref.dtype, ref.shape[0]
-    _need(dt in (torch.float32, torch.bfloat16), "operands must be fp32 or bf16")
-    for t, n in ((rope.mla_cos, "mla_cos"), (rope.mla_sin, "mla_sin"), (rope.idx_cos, "idx_cos"), (rope.idx_sin, "idx_sin")):
-        _cuda_contig(t, n, (dt,))
-        _need(t.shape[0] >= seq, f"{n} is shorter than the sequence")
-    H = Hidx = kv_rank = rope_dim = idx_dim = qs = qh = 0
-    iq_stride, w_stride = _rows(iq, "iq", dt), _rows(w, "w", dt)
-    if q is not None:
-        rope_dim = rope.mla_cos.shape[1]
-        _need(q.is_cuda and q.dim() == 3 and q.stride(2) == 1 and q.shape[2] == nope + rope_dim, "q must be [rows, H, nope + rope]")
-        H, qs, qh = q.shape[1], q.stride(0), q.stride(1)
-        _cuda_contig(q_full, "q_full", (dt,))
-        _need(q_full.dim() == 3 and q_full.shape[0] == rows and q_full.shape[1] == H, "q_full must be [rows, H, kv_rank + rope]")
-        kv_rank = q_full.shape[2] - rope_dim
-    if iq is not None:
-        _cuda_contig(index_q, "index_q", (torch.uint8, _FP8) if index_w is not None else (dt,))
-        Hidx, idx_dim = index_q.shape[1], index_q.shape[2]
-        _need(iq.shape == (rows, Hidx * idx_dim) and index_q.shape[0] == rows and rope.idx_cos.shape[1] == idx_dim,
-              "iq must be [rows, Hidx * D]")
-        if index_w is not None:
-            _cuda_contig(index_w, "index_w", (torch.float32,))
-            _need(w is not None and tuple(w.shape) == (rows, Hidx) and tuple(index_w.shape) == (rows, Hidx), "w must be [rows, Hidx]")
-    _lib.check(_lib.lib().dsa_prefill_queries(
-        _ptr(q), qs, qh, nope, _ptr(iq), iq_stride, _ptr(w), w_stride, _ptr(rope.mla_cos), _ptr(rope.mla_sin),
-        _ptr(rope.idx_cos), _ptr(rope.idx_sin), _ptr(q_full), _ptr(index_q), _ptr(index_w), rows, seq, H, Hidx, kv_rank,
-        rope_dim, idx_dim, 1 if interleave else 0, 0 if dt == torch.float32 else 1, _stream()))
+    _host().prefill_queries(q, nope, iq, w, rope.mla_cos, rope.mla_sin, rope.idx_cos, rope.idx_sin, q_full, index_q, index_w,
+                            seq, interleave)
 
 
 # --------------------------------------------------------------------------- exchanges between GPUs

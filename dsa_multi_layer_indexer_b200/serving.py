@@ -24,20 +24,49 @@ import torch
 from . import ops
 
 _FP8_ROW = ops.FP8_LATENT_ROW
-_scratch: Dict[Tuple, torch.Tensor] = {}
+_plans: Dict[Tuple, "_Plan"] = {}
+_SELECT = {True: "exact", False: "prod", "kernel": "exact", "approx": "exact", "exact": "exact", "prod": "prod",
+           "prod_side": "prod",  # the side-stream placement is the caller's business
+           "torch": "torch"}
 
 
-def _hide_scratch(key: Tuple, make):
-    """Persistent scratch keyed by static shape (patch :1274-1279): allocated on
-    first use, reused by every later call and by graph replays."""
-    buf = _scratch.get(key)
-    if buf is None:
-        buf = _scratch[key] = make()
-    return buf
+class _Plan:
+    """Persistent scratch of one static shape (patch :1274-1279), each buffer allocated on first use and
+    reused by every later call and by graph replays."""
+
+    def __init__(self, device, B: int, H_real: int, skv_cap: int, nsplit: int, topk: int) -> None:
+        self.device, self.B, self.skv_cap, self.nsplit, self.topk = device, B, skv_cap, nsplit, topk
+        # Head-geometry convention of the reference (:1443-1452): pad the heads to a multiple of 16
+        # with zero queries (a persistent buffer) and slice them off on return.
+        self.H_real, self.H = H_real, (H_real + 15) // 16 * 16
+        self.qpad = self.attn = self.attn_out = self.part = None
+        self.slab = self.logits = self.hist = None
+        self.next_idx = self.pos = self.topk_ws = self.paged = None
+
+    def attention_buffers(self) -> None:
+        dev, B, H = self.device, self.B, self.H
+        if H != self.H_real:
+            self.qpad = torch.zeros(1, B, H, ops.LATENT_DIM, dtype=torch.bfloat16, device=dev)
+        out = torch.zeros(1, B, H, ops.VALUE_DIM, dtype=torch.bfloat16, device=dev)
+        self.part = ops.MlaScratch(B, H, self.nsplit, dev)
+        self.attn_out = out if H == self.H_real else out[:, :, :self.H_real]
+        self.attn = out.view(B, H, ops.VALUE_DIM)
+
+    def scan_buffers(self) -> None:
+        self.slab = torch.empty(self.B, (self.skv_cap + 3) // 4 * 4, dtype=torch.float32, device=self.device)
+        self.logits = self.slab[:, :self.skv_cap]
+        self.hist = torch.zeros(self.B, ops.HIST_BINS, dtype=torch.int32, device=self.device)
+
+    def select_buffers(self) -> None:
+        self.next_idx = torch.full((self.B, self.topk), -1, dtype=torch.int32, device=self.device)
+        self.pos = torch.full((self.B, self.topk), -1, dtype=torch.int32, device=self.device)
+        self.topk_ws = ops.topk_workspace(self.B, self.skv_cap, self.device)
+        self.paged = self.topk_ws.numel() <= 16  # rows short enough for the top-k that emits slots itself
 
 
 def clear_scratch() -> None:
-    _scratch.clear()
+    _plans.clear()
+    _operands.clear()
 
 
 def fused_hide_decode_paged(
@@ -70,15 +99,8 @@ def fused_hide_decode_paged(
     ``select="torch"`` (torch.topk gate)."""
     if mode not in ("full", "attn_only", "scan_only"):
         raise ValueError(f"unknown mode={mode!r}")
-    if select is True:
-        sel_mode = "exact"
-    elif select is False:
-        sel_mode = "prod"
-    else:
-        sel_mode = "exact" if select in ("kernel", "approx") else str(select)
-    if sel_mode == "prod_side":
-        sel_mode = "prod"  # the side-stream placement is the caller's business
-    if sel_mode not in ("exact", "prod", "torch"):
+    sel_mode = _SELECT.get(select)
+    if sel_mode is None:
         raise ValueError(f"unknown select={select!r}")
     if q_all.dim() != 4 or q_all.shape[0] != 1:
         raise ValueError(f"q_all must be [1,B,H,dqk], got {tuple(q_all.shape)}")
@@ -93,9 +115,9 @@ def fused_hide_decode_paged(
         raise ValueError(f"unsupported indexer geometry Hidx={Hidx} didx={didx}")
     if index_q_fp8.dtype not in (torch.float8_e4m3fn, torch.uint8):
         raise ValueError(f"index_q_fp8 dtype {index_q_fp8.dtype}")
-    if tuple(index_weights.shape) != (B, Hidx):
+    if index_weights.shape != (B, Hidx):
         raise ValueError(f"index_weights must be [B,Hidx]=({B},{Hidx}), got {tuple(index_weights.shape)}")
-    if tuple(seq_lens.shape) != (B,) or seq_lens.dtype != torch.int32:
+    if seq_lens.shape != (B,) or seq_lens.dtype != torch.int32:
         raise ValueError(f"seq_lens must be int32 [B={B}], got {tuple(seq_lens.shape)} {seq_lens.dtype}")
     if page_table.dim() != 2 or page_table.shape[0] != B or page_table.dtype != torch.int32:
         raise ValueError(f"page_table must be int32 [B={B}, pt_stride], got {tuple(page_table.shape)} {page_table.dtype}")
@@ -117,44 +139,39 @@ def fused_hide_decode_paged(
         raise ValueError(f"kv_pool must be bf16 [S,{dqk}] or fp8-packed uint8 [S,{_FP8_ROW}], got "
                          f"{kv_pool.dtype} {tuple(kv_pool.shape)}")
 
-    # Head-geometry convention of the reference (:1443-1452): pad the heads to a multiple
-    # of 16 with zero queries (a persistent buffer) and slice them off on return.
-    H = (H_real + 15) // 16 * 16
-    if H != H_real:
-        qpad = _hide_scratch((str(device), B, H, "qpad"),
-                             lambda: torch.zeros(1, B, H, dqk, dtype=torch.bfloat16, device=device))
-        qpad[:, :, :H_real].copy_(q_all)
-        q_all = qpad
-    q = q_all.contiguous().view(B, H, dqk)
     if nsplit_attn is None:
-        nsplit_attn = nsplit if nsplit is not None else ops.default_nsplit(B, H, topk)
-    nsplit_attn = int(nsplit_attn)
-    key = (str(device), B, H, skv_cap, nsplit_attn, topk)
+        nsplit_attn = nsplit if nsplit is not None else ops.default_nsplit(B, (H_real + 15) // 16 * 16, topk)
+    key = (device, B, H_real, skv_cap, nsplit_attn, topk)
+    plan = _plans.get(key)
+    if plan is None:
+        plan = _plans[key] = _Plan(device, B, H_real, skv_cap, int(nsplit_attn), topk)
 
-    attn_out = logits = None
+    attn_out = None
     if mode != "scan_only":
+        if plan.attn is None:
+            plan.attention_buffers()
         # one shared pool of S_pool slots: every row is a query row of the same "sequence",
         # entries < 0 or >= S_pool are skipped in the kernel
+        if plan.qpad is not None:
+            plan.qpad[:, :, :H_real].copy_(q_all)
+            q_all = plan.qpad
         slots = incumbent_slots if incumbent_slots.dtype == torch.int32 else incumbent_slots.to(torch.int32)
-        kv = (kv_pool if kv_pool.dtype != torch.float8_e4m3fn else kv_pool.view(torch.uint8)).unsqueeze(0)
-        scratch = _hide_scratch(key + ("part",), lambda: ops.MlaScratch(B, H, nsplit_attn, device))
-        out = _hide_scratch(key + ("out",), lambda: torch.zeros(1, B, H, ops.VALUE_DIM, dtype=torch.bfloat16,
-                                                                 device=device))
-        ops.sparse_mla_decode(q, kv, slots.contiguous(), float(sm_scale), None, rows_per_seq=B, nsplit=nsplit_attn,
-                              scratch=scratch, out=out.view(B, H, ops.VALUE_DIM))
-        attn_out = out[:, :, :H_real] if H != H_real else out
+        kv = kv_pool if kv_pool.dtype != torch.float8_e4m3fn else kv_pool.view(torch.uint8)
+        ops.sparse_mla_decode(q_all.contiguous().view(B, plan.H, dqk), kv, slots.contiguous(), sm_scale, None, rows_per_seq=B,
+                              nsplit=plan.nsplit, scratch=plan.part, out=plan.attn)
+        attn_out = plan.attn_out
         if mode == "attn_only":
             return attn_out
 
-    slab = _hide_scratch(key + ("slab",), lambda: torch.empty(B, (skv_cap + 3) // 4 * 4, dtype=torch.float32,
-                                                              device=device))
+    if plan.slab is None:
+        plan.scan_buffers()
     use_hist = mode == "full" and sel_mode == "exact"
-    hist = _hide_scratch(key + ("hist",), lambda: torch.zeros(B, ops.HIST_BINS, dtype=torch.int32, device=device))
-    iq = index_q_fp8 if index_q_fp8.dtype == torch.uint8 else index_q_fp8.view(torch.uint8)
-    ops.indexer_scan_fp8_paged(iq.contiguous(), index_weights.to(torch.float32).contiguous(), index_k_paged,
-                               page_table.contiguous(), seq_lens.contiguous(), skv_cap, out=slab,
-                               hist=hist if use_hist else None)
-    logits = slab[:, :skv_cap]
+    iq = index_q_fp8 if index_q_fp8.is_contiguous() else index_q_fp8.contiguous()
+    weights = index_weights if index_weights.dtype == torch.float32 else index_weights.to(torch.float32)
+    table = page_table.contiguous()
+    logits = plan.logits
+    ops.indexer_scan_fp8_paged(iq, weights.contiguous(), index_k_paged, table, seq_lens.contiguous(), skv_cap, out=plan.slab,
+                               hist=plan.hist if use_hist else None)
     if mode == "scan_only":
         return logits
     if sel_mode == "prod":
@@ -163,19 +180,27 @@ def fused_hide_decode_paged(
     if sel_mode == "exact":
         if index_topk != topk:
             raise ValueError("the in-launch select emits exactly topk indices")
-        ws = _hide_scratch(key + ("topk_ws",), lambda: ops.topk_workspace(B, skv_cap, device))
-        pos = _hide_scratch(key + ("pos",), lambda: torch.full((B, topk), -1, dtype=torch.int32, device=device))
-        next_idx = _hide_scratch(key + ("nextidx",), lambda: torch.full((B, topk), -1, dtype=torch.int32,
-                                                                        device=device))
-        ops.topk_select(logits, topk, seq_lens, hist=hist, out_idx=pos, workspace=ws)
-        # positions -> KV slots: through out_index_pool, or page * 64 + offset from the page-64
-        # table (kernels/cuda_fused_sparse_splitk.py:1142-1144); padding stays -1
-        safe = pos.clamp(min=0).long()
-        if out_index_pool is not None:
-            mapped = torch.gather(out_index_pool[:, :skv_cap], 1, safe).to(torch.int32)
+        if plan.next_idx is None:
+            plan.select_buffers()
+        next_idx = plan.next_idx
+        if out_index_pool is None and plan.paged:
+            # the selection leaves the top-k as KV slots, page * 64 + offset from the page-64 table
+            # (kernels/cuda_fused_sparse_splitk.py:1142-1144)
+            ops.topk_select_paged(logits, topk, seq_lens, plan.hist, table, next_idx)
+        elif (out_index_pool is not None and out_index_pool.dtype == torch.int32 and plan.paged
+              and out_index_pool.shape[1] == skv_cap and out_index_pool.is_contiguous()):
+            # positions -> KV slots through out_index_pool, read by the top-k as its index map
+            ops.topk_select(logits, topk, seq_lens, hist=plan.hist, index_map=out_index_pool, out_idx=next_idx,
+                            workspace=plan.topk_ws)
         else:
-            mapped = torch.gather(page_table, 1, safe >> 6) * ops.PAGE_TOKENS + (pos & (ops.PAGE_TOKENS - 1))
-        torch.where(pos >= 0, mapped, pos, out=next_idx)
+            pos = plan.pos
+            ops.topk_select(logits, topk, seq_lens, hist=plan.hist, out_idx=pos, workspace=plan.topk_ws)
+            safe = pos.clamp(min=0).long()
+            if out_index_pool is not None:
+                mapped = torch.gather(out_index_pool[:, :skv_cap], 1, safe).to(torch.int32)
+            else:
+                mapped = torch.gather(page_table, 1, safe >> 6) * ops.PAGE_TOKENS + (pos & (ops.PAGE_TOKENS - 1))
+            torch.where(pos >= 0, mapped, pos, out=next_idx)  # padding stays -1
         if return_logits:
             return attn_out, next_idx, logits
         return attn_out, next_idx
@@ -192,6 +217,9 @@ def fused_hide_decode_paged(
     if return_logits:
         return attn_out, next_idx, logits.clone()
     return attn_out, next_idx
+
+
+_operands: Dict[Tuple, Tuple[torch.Tensor, torch.Tensor]] = {}
 
 
 def forward_hide_operands(
@@ -236,12 +264,14 @@ def forward_hide_operands(
         seq_lens = seq_lens.to(torch.int32)
     B, n_heads = q_proj.shape[0], q_proj.shape[1]
     device = q_proj.device
-    q_fp8 = _hide_scratch(("hide_q", B, n_heads, device),
-                          lambda: torch.empty(B, n_heads, ops.INDEX_DIM, dtype=torch.uint8, device=device))
-    weights = _hide_scratch(("hide_w", B, n_heads, device),
-                            lambda: torch.empty(B, n_heads, dtype=torch.float32, device=device))
+    key = (device, B, n_heads)
+    buffers = _operands.get(key)
+    if buffers is None:
+        buffers = _operands[key] = (torch.empty(B, n_heads, ops.INDEX_DIM, dtype=torch.uint8, device=device),
+                                    torch.empty(B, n_heads, dtype=torch.float32, device=device))
+    q_fp8, weights = buffers
     ops.indexer_stage_fp8(q_proj, k_proj, head_gates, k_norm_weight, k_norm_bias, k_norm_eps, rope_cos, rope_sin,
-                          positions, q_fp8, weights, pages=index_k_paged.view(-1), page_table=page_table_64,
+                          positions, q_fp8, weights, pages=index_k_paged, page_table=page_table_64,
                           rope_interleave=rope_interleave, scale_fmt=scale_fmt, softmax_scale=softmax_scale)
     skv_cap = int(page_table_64.shape[1]) * ops.PAGE_TOKENS
     return q_fp8, weights, index_k_paged, page_table_64, seq_lens, skv_cap

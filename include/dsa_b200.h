@@ -140,7 +140,8 @@ int dsa_indexer_scan_f32(const float* index_q, const float* index_w, const float
  *              index_map[r, p] (used to merge per-GPU candidate lists)
  *   out_idx    [R, topk] int32        out_val  NULL or [R, topk] fp32
  *   workspace  caller-owned scratch of at least dsa_topk_workspace_bytes(R, n)
- *              bytes, zero before its first use; every call leaves it re-armed
+ *              bytes, zero before its first use (NULL where that is no more than 16 bytes: such
+ *              rows need none); every call leaves it re-armed
  *              (the reference's self-resetting SelScratch, :2150-2153). Calls
  *              that share a workspace must not overlap on the device.
  *   index_offset is added to positions when index_map is NULL.
@@ -152,6 +153,13 @@ int dsa_topk_select(const float* logits, const int32_t* seq_lens, uint32_t* hist
                     void* workspace, int64_t workspace_bytes,
                     int R, int64_t n, int64_t slab_stride, int topk,
                     int32_t pad_value, int32_t index_offset, void* stream);
+/* The same selection for a paged cache, as cache slots: position p of row r is written as
+ * page_table[r, p / 64] * 64 + p % 64 (kernels/cuda_fused_sparse_splitk.py:1142-1144), padding as
+ * pad_value. hist as above, required; page_table [R, pt_stride] int32; rows that the workspace-free
+ * kernel takes (dsa_topk_workspace_bytes <= 16), else DSA_ERR_UNSUPPORTED. */
+int dsa_topk_select_paged(const float* logits, const int32_t* seq_lens, uint32_t* hist,
+                          const int32_t* page_table, int64_t pt_stride, int32_t* out_idx, int R,
+                          int64_t n, int64_t slab_stride, int topk, int32_t pad_value, void* stream);
 
 /* ---- candidate exchange of the KV-sequence-sharded indexer -------------------
  * One process per GPU, each scanning its own range of the keys. The reference has no
