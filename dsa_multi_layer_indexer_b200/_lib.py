@@ -53,6 +53,9 @@ SIGNATURES: Dict[str, Tuple[object, List[object]]] = {
     "dsa_sparse_mla_f32": (_i, [_p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _f, _l, _p]),
     "dsa_rmsnorm": (_i, [_p, _p, _p, _l, _i, _f, _i, _p]),
     "dsa_add_rmsnorm_bf16": (_i, [_p, _p, _p, _p, _p, _l, _i, _f, _p]),
+    "dsa_add_rmsnorm_f32": (_i, [_p, _p, _p, _p, _p, _l, _i, _f, _p]),
+    "dsa_linear_f32": (_i, [_p, _l, _i] + [_p, _i, _p] * 3 + [_i, _p]),
+    "dsa_silu_mul_f32": (_i, [_p, _p, _p, _l, _p]),
     "dsa_silu_mul_bf16": (_i, [_p, _p, _p, _l, _p]),
     "dsa_gemv_bf16": (_i, [_p, _p, _p, _i, _i, _i, _l, _l, _p]),
     "dsa_copy_bytes": (_i, [_p, _p, _l, _p]),

@@ -54,6 +54,43 @@ rmsnorm_kernel(const T* __restrict__ x, const T* __restrict__ weight, T* __restr
     out[row * dim + i] = from_f32<T>(to_f32<T>(xr[i]) * inv * to_f32<T>(weight[i]));
 }
 
+// s = x + delta and its norm, fp32 rows of any length: the residual addition and the norm behind it.
+__global__ void __launch_bounds__(256)
+add_rmsnorm_f32_kernel(const float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ weight,
+                       float* sum_out, float* __restrict__ out, int dim, float eps) {
+  __shared__ float s_part[8];
+  const int64_t row = blockIdx.x;
+  pdl_wait();
+  pdl_launch_dependents();
+  float* sr = sum_out + row * dim;
+  float ss = 0.f;
+  for (int i = threadIdx.x; i < dim; i += 256) {
+    const float v = x[row * dim + i] + delta[row * dim + i];
+    sr[i] = v;
+    ss = fmaf(v, v, ss);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float tot = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) tot += s_part[w];
+  const float inv = rsqrtf(tot / float(dim) + eps);
+  for (int i = threadIdx.x; i < dim; i += 256) out[row * dim + i] = sr[i] * inv * weight[i];  // (its own writes)
+}
+
+// out = silu(gate) * up over fp32, rounded as the two separate operations.
+__global__ void __launch_bounds__(256)
+silu_mul_f32_kernel(const float* __restrict__ gate, const float* __restrict__ up, float* __restrict__ out, int64_t n) {
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < n; i += int64_t(gridDim.x) * 256) {
+    const float g = gate[i];
+    out[i] = __fmul_rn(g / (1.f + expf(-g)), up[i]);
+  }
+}
+
 // bf16 rows of up to 8192 elements (a multiple of 8): each of the 256 threads keeps its
 // 16-byte pieces of the row in registers, so the row is read once. With kAdd the
 // kernel first forms s = x + delta (rounded to bf16 as the separate addition would

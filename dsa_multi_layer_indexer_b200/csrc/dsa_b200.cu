@@ -13,10 +13,12 @@
 #include "decode_prep.cuh"
 #include "fused_decode.cuh"
 #include "indexer_scan.cuh"
+#include "linear_f32.cuh"
 #include "peer_allreduce.cuh"
 #include "prefill_prep.cuh"
 #include "sparse_mla.cuh"
 #include "sparse_mla_tc.cuh"
+#include "topk_rows.cuh"
 #include "topk_select.cuh"
 
 namespace dsa {
@@ -103,7 +105,7 @@ static int opt_in_smem(K kernel, size_t bytes, bool (&done)[64]) {
   if (dev >= 0 && dev < 64) done[dev] = true;
   return DSA_OK;
 }
-static bool g_opt_fused[64], g_opt_mla[64], g_opt_mla_beside[64], g_opt_mla_tc[64], g_opt_scan_f32[64], g_opt_topk[64], g_opt_gemv[4][64];
+static bool g_opt_fused[64], g_opt_mla[64], g_opt_mla_beside[64], g_opt_mla_tc[64], g_opt_mla_f32[64], g_opt_topk[64], g_opt_gemv[4][64];
 
 // Launch with programmatic dependent launch allowed: the kernel may be scheduled
 // while its predecessor in the stream is still draining; it calls
@@ -392,18 +394,12 @@ int dsa_indexer_scan_f32(const float* index_q, const float* index_w, const float
               "f32 indexer scan: bad R=%d / rows_per_seq=%d", R, rows_per_seq);
   DSA_REQUIRE(n_heads > 0 && head_dim > 0 && ctx > 0, "f32 indexer scan: bad geometry");
   DSA_REQUIRE(k_seq_stride >= ctx && slab_stride >= ctx, "f32 indexer scan: strides must be >= ctx");
-  const size_t smem = (size_t(n_heads) * head_dim + n_heads) * sizeof(float);
-  DSA_REQUIRE(smem <= 200 * 1024, "f32 indexer scan: n_heads * head_dim too large for shared memory");
-  if (smem > 48 * 1024) {
-    int rc = opt_in_smem(scan::indexer_scan_f32_kernel, 200 * 1024, g_opt_scan_f32);
-    if (rc) return rc;
-  }
-  int gx = int((ctx + 7) / 8);
-  int cap = (16 * sm_count() + R - 1) / R;
-  if (gx > cap) gx = cap < 1 ? 1 : cap;
-  scan::indexer_scan_f32_kernel<<<dim3(gx, R), 256, smem, static_cast<cudaStream_t>(stream)>>>(
-      index_q, index_w, index_k, seq_lens, logits, rows_per_seq, n_heads, head_dim, ctx,
-      k_seq_stride, slab_stride);
+  const int groups = (rows_per_seq + scan::kF32Rows - 1) / scan::kF32Rows;
+  const dim3 grid(unsigned((ctx + scan::kF32Keys - 1) / scan::kF32Keys), unsigned(R / rows_per_seq * groups));  // (y <= R <= 65535)
+  // four rows or more of a sequence: the warps split the rows; fewer: the heads
+  auto kernel = rows_per_seq >= 4 ? scan::indexer_scan_f32_rows_kernel : scan::indexer_scan_f32_kernel;
+  kernel<<<grid, scan::kF32Warps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
+      index_q, index_w, index_k, seq_lens, logits, rows_per_seq, groups, n_heads, head_dim, ctx, k_seq_stride, slab_stride);
   DSA_CUDA(cudaGetLastError());
   return DSA_OK;
 }
@@ -484,7 +480,22 @@ static int launch_topk_cluster_as(const topk::Params& p, int R, int ctas, int nk
 }
 }  // extern "C++"
 
+// Many short rows without a histogram: one small CTA per row (topk_rows.cuh).
+static int launch_topk_rows(const topk::Params& p, int R, int64_t n, cudaStream_t st) {
+  const dim3 grid(R);
+  if (n <= 512) DSA_CUDA(launch_pdl(topk::topk_rows_kernel<128, 4>, grid, dim3(128), 0, st, p));
+  else if (n <= 2048) DSA_CUDA(launch_pdl(topk::topk_rows_kernel<256, 8>, grid, dim3(256), 0, st, p));
+  else if (n <= 4096) DSA_CUDA(launch_pdl(topk::topk_rows_kernel<256, 16>, grid, dim3(256), 0, st, p));
+  else if (n <= 6144) DSA_CUDA(launch_pdl(topk::topk_rows_kernel<256, 24>, grid, dim3(256), 0, st, p));
+  else if (n <= 8192) DSA_CUDA(launch_pdl(topk::topk_rows_kernel<256, 32>, grid, dim3(256), 0, st, p));
+  else DSA_CUDA(launch_pdl(topk::topk_rows_kernel<512, 32>, grid, dim3(512), 0, st, p));
+  return DSA_OK;
+}
+
 static int launch_topk_cluster(const topk::Params& p, int R, int64_t n, cudaStream_t st) {
+  // More rows than SMs: the cluster kernel holds one row per SM and would take several waves of its
+  // latency-bound chain, the row kernel keeps several rows per SM in flight.
+  if (!p.hist && !p.n_src && !p.n_dest && R > sm_count() && n <= topk::kRowsMaxN) return launch_topk_rows(p, R, n, st);
   const bool plain = p.hist && !p.n_src && !p.n_dest && !p.index_map && !p.out_val;
   // As few CTAs as hold the row at 32 logits per thread: every CTA added costs cluster barriers and
   // remote stores, and a row of up to 16384 logits needs none of either.
@@ -984,6 +995,56 @@ int dsa_add_rmsnorm_bf16(const void* x, const void* delta, const void* weight, v
   return DSA_OK;
 }
 
+int dsa_add_rmsnorm_f32(const float* x, const float* delta, const float* weight, float* sum_out, float* out, int64_t rows,
+                        int dim, float eps, void* stream) {
+  DSA_REQUIRE(x && delta && weight && sum_out && out, "add + rmsnorm: null pointer");
+  DSA_REQUIRE(rows > 0 && rows < (int64_t(1) << 31) && dim > 0, "add + rmsnorm: bad shape");
+  DSA_CUDA(launch_pdl(prep::add_rmsnorm_f32_kernel, dim3(unsigned(rows)), dim3(256), 0, static_cast<cudaStream_t>(stream), x, delta,
+                      weight, sum_out, out, dim, eps));
+  return DSA_OK;
+}
+
+int dsa_silu_mul_f32(const float* gate, const float* up, float* out, int64_t n, void* stream) {
+  DSA_REQUIRE(gate && up && out, "silu * up: null pointer");
+  DSA_REQUIRE(n > 0 && n < (int64_t(1) << 40), "silu * up: bad element count");
+  const int64_t blocks = std::min<int64_t>((n + 255) / 256, 16 * sm_count());
+  DSA_CUDA(launch_pdl(prep::silu_mul_f32_kernel, dim3(unsigned(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream), gate, up,
+                      out, n));
+  return DSA_OK;
+}
+
+extern "C++" {
+template <bool kSwiglu>
+static int launch_linear_f32(const lin::Params& p, int tiles, cudaStream_t st) {
+  static bool done[64];
+  constexpr size_t smem = lin::smem_bytes<kSwiglu>();
+  int rc = opt_in_smem(lin::linear_f32_kernel<kSwiglu>, smem, done);
+  if (rc) return rc;
+  const dim3 grid(unsigned((p.m + lin::kBM - 1) / lin::kBM), tiles);
+  DSA_CUDA(launch_pdl(lin::linear_f32_kernel<kSwiglu>, grid, dim3(lin::kThreads), smem, st, p));
+  return DSA_OK;
+}
+}  // extern "C++"
+
+int dsa_linear_f32(const float* x, int64_t m, int k, const float* w0, int n0, float* y0, const float* w1, int n1, float* y1,
+                   const float* w2, int n2, float* y2, int swiglu, void* stream) {
+  DSA_REQUIRE(x && w0 && y0 && (!w1 || swiglu || y1) && (!w2 || (w1 && y2)), "linear: null pointer");
+  DSA_REQUIRE(m > 0 && m < (int64_t(1) << 31) && k > 0 && k % 4 == 0 && n0 > 0 && (!w1 || n1 > 0) && (!w2 || n2 > 0), "linear: bad shape");
+  DSA_REQUIRE(!swiglu || (w1 && !w2 && n1 == n0), "linear: swiglu takes two weights of one shape");
+  DSA_REQUIRE(aligned16(x) && aligned16(w0) && aligned16(w1) && aligned16(w2), "linear: pointers must be 16-byte aligned");
+  lin::Params p{};
+  p.x = x, p.m = m, p.k = k;
+  p.w[0] = w0, p.w[1] = w1, p.w[2] = w2;
+  p.y[0] = y0, p.y[1] = y1, p.y[2] = y2;
+  p.n[0] = n0, p.n[1] = n1, p.n[2] = n2;
+  p.count = swiglu ? 1 : w2 ? 3 : w1 ? 2 : 1;
+  int tiles = 0;
+  for (int i = 0; i < p.count; ++i) tiles += p.tiles[i] = (p.n[i] + lin::kBN - 1) / lin::kBN;
+  DSA_REQUIRE(tiles <= 65535, "linear: too many output columns");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return swiglu ? launch_linear_f32<true>(p, tiles, st) : launch_linear_f32<false>(p, tiles, st);
+}
+
 int dsa_copy_bytes(void* dst, const void* src, int64_t bytes, void* stream) {
   DSA_REQUIRE(dst && src, "copy: null pointer");
   DSA_REQUIRE(bytes > 0 && bytes % 16 == 0 && aligned16(dst) && aligned16(src),
@@ -1340,6 +1401,19 @@ int dsa_sparse_mla_f32(const float* q, const float* kv, const int32_t* indices,
   DSA_REQUIRE(H > 0 && qk_dim > 0 && v_dim > 0 && v_dim <= qk_dim && v_dim <= 512,
               "f32 sparse MLA: need 0 < v_dim <= min(qk_dim, 512)");
   DSA_REQUIRE(indices == nullptr || topk_k > 0, "f32 sparse MLA: topk must be positive");
+  // Many rows: eight heads share the gathered keys; with fewer CTAs than SMs a CTA per head is faster.
+  const int head_blocks = (H + mla::kF32Heads - 1) / mla::kF32Heads;
+  const size_t rows_smem = mla::f32_rows_smem(qk_dim);
+  if (int64_t(R) * head_blocks >= sm_count() && rows_smem <= 200 * 1024) {
+    if (rows_smem > 48 * 1024) {
+      int rc = opt_in_smem(mla::sparse_mla_f32_rows_kernel, 200 * 1024, g_opt_mla_f32);
+      if (rc) return rc;
+    }
+    mla::sparse_mla_f32_rows_kernel<<<dim3(R, head_blocks), mla::kF32Threads, rows_smem, static_cast<cudaStream_t>(stream)>>>(
+        q, kv, indices, seq_lens, out, rows_per_seq, H, qk_dim, v_dim, topk_k, sm_scale, kv_seq_stride, kv_seq_stride);
+    DSA_CUDA(cudaGetLastError());
+    return DSA_OK;
+  }
   const size_t smem = (size_t(qk_dim) + 128 + 128 + 8) * sizeof(float);
   DSA_REQUIRE(smem <= 48 * 1024, "f32 sparse MLA: qk_dim too large");
   mla::sparse_mla_f32_kernel<<<dim3(H, R), 128, smem, static_cast<cudaStream_t>(stream)>>>(

@@ -32,7 +32,7 @@ using at::Tensor;
   X(dsa_indexer_scan_fp8) X(dsa_indexer_scan_fp8_paged) X(dsa_indexer_scan_f32) X(dsa_topk_workspace_bytes)    \
   X(dsa_topk_select) X(dsa_topk_select_paged) X(dsa_sparse_mla_partials) X(dsa_sparse_mla_combine)             \
   X(dsa_sparse_mla_decode) X(dsa_sparse_mla_decode_beside) X(dsa_sparse_mla_f32) X(dsa_rmsnorm)                \
-  X(dsa_add_rmsnorm_bf16) X(dsa_silu_mul_bf16) X(dsa_indexer_stage_fp8) X(dsa_latent_append)                   \
+  X(dsa_add_rmsnorm_bf16) X(dsa_silu_mul_bf16) X(dsa_add_rmsnorm_f32) X(dsa_silu_mul_f32) X(dsa_linear_f32) X(dsa_indexer_stage_fp8) X(dsa_latent_append)                   \
   X(dsa_prefill_latents) X(dsa_prefill_queries)
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
@@ -42,21 +42,25 @@ struct Api {
 PyObject* status_check = nullptr;  // _lib.check: raises for a negative status
 
 // ---------------------------------------------------------------- errors
+// Thrown without touching the interpreter (its lock may be released) and translated in entry().
 struct PyErrorSet {};  // a Python exception is already set
-[[noreturn]] void bad(const std::string& msg) {
-  PyErr_SetString(PyExc_ValueError, msg.c_str());
-  throw PyErrorSet();
-}
+struct ValueError {
+  std::string msg;
+};
+struct StatusError {
+  int status;
+};
+[[noreturn]] void bad(const std::string& msg) { throw ValueError{msg}; }
 inline void need(bool cond, const char* msg) {
   if (__builtin_expect(!cond, 0)) bad(msg);
 }
-void ok(int status) {
-  if (__builtin_expect(status == 0, 1)) return;
-  PyObject* r = PyObject_CallFunction(status_check, "i", status);
-  Py_XDECREF(r);
-  if (r) PyErr_SetString(PyExc_RuntimeError, "dsa_b200: call failed");
-  throw PyErrorSet();
+inline void ok(int status) {
+  if (__builtin_expect(status != 0, 0)) throw StatusError{status};
 }
+struct NoGil {  // the interpreter's lock is released while this lives
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
 
 // The call itself runs without the interpreter's lock (a full launch queue blocks it): its arguments
 // must not touch Python objects.
@@ -443,16 +447,20 @@ PyObject* rmsnorm(PyObject* const* a) {
 // (x, delta, weight, eps)
 PyObject* add_rmsnorm(PyObject* const* a) {
   const Tensor &x0 = ten(a[0], "x"), &d0 = ten(a[1], "delta");
-  need(x0.is_cuda() && x0.scalar_type() == at::kBFloat16 && d0.scalar_type() == at::kBFloat16 && x0.sizes() == d0.sizes(),
-       "x and delta must be CUDA bf16 tensors of one shape");
+  const at::ScalarType type = x0.scalar_type();
+  need(x0.is_cuda() && (type == at::kBFloat16 || type == at::kFloat) && d0.scalar_type() == type && x0.sizes() == d0.sizes(),
+       "x and delta must be CUDA bf16 or fp32 tensors of one shape");
   const int64_t dim = x0.size(-1);
-  need(dim % 8 == 0 && dim <= 8192, "the row length must be a multiple of 8 and at most 8192");
+  need(type == at::kFloat || (dim % 8 == 0 && dim <= 8192), "the row length must be a multiple of 8 and at most 8192");
   const Tensor x = x0.contiguous(), d = d0.contiguous();
-  const Tensor w = ten(a[2], "weight").to(x.scalar_type()).contiguous();
+  const Tensor w = ten(a[2], "weight").to(type).contiguous();
   const Tensor s = at::empty_like(x), out = at::empty_like(x);
   const float eps = float(real(a[3]));
   void* st = stream();
-  LAUNCH(api.dsa_add_rmsnorm_bf16(ptr(x), ptr(d), ptr(w), ptr(s), ptr(out), x.numel() / dim, int(dim), eps, st));
+  if (type == at::kFloat)
+    LAUNCH(api.dsa_add_rmsnorm_f32(as<float>(x), as<float>(d), as<float>(w), as<float>(s), as<float>(out), x.numel() / dim, int(dim), eps, st));
+  else
+    LAUNCH(api.dsa_add_rmsnorm_bf16(ptr(x), ptr(d), ptr(w), ptr(s), ptr(out), x.numel() / dim, int(dim), eps, st));
   PyObject *ps = THPVariable_Wrap(s), *po = THPVariable_Wrap(out);
   PyObject* both = PyTuple_Pack(2, ps, po);
   Py_DECREF(ps);
@@ -463,11 +471,13 @@ PyObject* add_rmsnorm(PyObject* const* a) {
 // (gate, up)
 PyObject* silu_mul(PyObject* const* a) {
   const Tensor &g0 = ten(a[0], "gate"), &u0 = ten(a[1], "up");
-  need(g0.is_cuda() && g0.scalar_type() == at::kBFloat16 && u0.scalar_type() == at::kBFloat16 && g0.sizes() == u0.sizes(),
-       "gate and up must be CUDA bf16 tensors of one shape");
+  const at::ScalarType type = g0.scalar_type();
+  need(g0.is_cuda() && (type == at::kBFloat16 || type == at::kFloat) && u0.scalar_type() == type && g0.sizes() == u0.sizes(),
+       "gate and up must be CUDA bf16 or fp32 tensors of one shape");
   const Tensor g = g0.contiguous(), u = u0.contiguous(), out = at::empty_like(g);
   void* st = stream();
-  LAUNCH(api.dsa_silu_mul_bf16(ptr(g), ptr(u), ptr(out), g.numel(), st));
+  if (type == at::kFloat) LAUNCH(api.dsa_silu_mul_f32(as<float>(g), as<float>(u), as<float>(out), g.numel(), st));
+  else LAUNCH(api.dsa_silu_mul_bf16(ptr(g), ptr(u), ptr(out), g.numel(), st));
   return THPVariable_Wrap(out);
 }
 
@@ -670,6 +680,178 @@ PyObject* prefill_queries(PyObject* const* a) {
   Py_RETURN_NONE;
 }
 
+// ---------------------------------------------------------------- a full-sequence layer
+// The chain DSALayer runs per layer of a prompt, without the interpreter between its launches: at a few
+// hundred tokens of the small preset a layer is some twenty launches of 3-8 us, and calling each from
+// Python took twice that.
+
+// Up to this many multiply-adds a product of fp32 matrices goes to the library's own small-tile kernel,
+// beyond it to the GEMM library (1024 x 1024 x 256,
+// two weights: 23 us against the library's 19; three weights of 2^25.6 in all: 6 us against 20).
+constexpr double kSmallLinear = double(1 << 28);
+
+bool small_f32(const Tensor& x, std::initializer_list<const Tensor*> ws) {
+  if (x.scalar_type() != at::kFloat || !x.is_contiguous() || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u)) return false;
+  double n = 0;
+  for (const Tensor* w : ws) {
+    if (!w->is_contiguous() || (reinterpret_cast<uintptr_t>(w->data_ptr()) & 15u)) return false;
+    n += double(w->size(0));
+  }
+  return x.size(1) % 4 == 0 && double(x.size(0)) * n * double(x.size(1)) <= kSmallLinear;
+}
+// y_i = x w_i^T for weights that read the same rows x.
+void linears(const Tensor& x, std::initializer_list<std::pair<const Tensor*, Tensor*>> jobs) {
+  const Tensor* w[3] = {};
+  Tensor* y[3] = {};
+  int n = 0;
+  bool small = x.scalar_type() == at::kFloat;
+  for (const auto& j : jobs)
+    if (j.first) w[n] = j.first, y[n++] = j.second;
+  if (n == 0) return;
+  small = small && (n == 1 ? small_f32(x, {w[0]}) : n == 2 ? small_f32(x, {w[0], w[1]}) : small_f32(x, {w[0], w[1], w[2]}));
+  if (!small) {
+    for (int i = 0; i < n; ++i) *y[i] = at::mm(x, w[i]->t());
+    return;
+  }
+  for (int i = 0; i < n; ++i) *y[i] = fresh({x.size(0), w[i]->size(0)}, at::kFloat, x);
+  void* st = stream();
+  ok(api.dsa_linear_f32(as<float>(x), x.size(0), int(x.size(1)), as<float>(w[0]), int(w[0]->size(0)), as<float>(*y[0]), as<float>(w[1]),
+                            w[1] ? int(w[1]->size(0)) : 0, y[1] ? as<float>(*y[1]) : nullptr, as<float>(w[2]),
+                            w[2] ? int(w[2]->size(0)) : 0, y[2] ? as<float>(*y[2]) : nullptr, 0, st));
+}
+Tensor linear_of(const Tensor& x, const Tensor& w) {
+  Tensor y;
+  linears(x, {{&w, &y}});
+  return y;
+}
+
+// (x_norm, seq, c_q | None, wx | None, wc | None, q_a, kv_a, ik, q_b, iq, w, q_norm, kv_norm, kv_b,
+//  mla_cos, mla_sin, idx_cos, idx_sin, kv | None, ik_out | None, ik_scale | None, attention, indexer, fp8,
+//  heads, nope, index_heads, interleave, eps) -> (q_full, kv, iq, iw, ik, ik_scale)
+PyObject* full_operands(PyObject* const* a) {
+  const Tensor& xn = ten(a[0], "x_norm");
+  const at::ScalarType type = xn.scalar_type();
+  const int dt = dtype_of(type);
+  const int64_t seq = integer(a[1]), hidden = xn.size(-1), rows = xn.numel() / hidden;
+  const Tensor *cq_in = opt(a[2], "c_q"), *wx = opt(a[3], "wx"), *wc = opt(a[4], "wc");
+  const Tensor &q_a = ten(a[5], "q_a"), &kv_a = ten(a[6], "kv_a"), &ik_w = ten(a[7], "ik"), &q_b = ten(a[8], "q_b"), &iq_w = ten(a[9], "iq"),
+               &w_w = ten(a[10], "w"), &q_norm = ten(a[11], "q_norm"), &kv_norm = ten(a[12], "kv_norm"), &kv_b = ten(a[13], "kv_b");
+  const Rope rope = rope_of(a + 14, type, seq);
+  const Tensor *kv_given = opt(a[18], "kv"), *ik_given = opt(a[19], "ik"), *iks_given = opt(a[20], "ik_scale");
+  const bool attention = truth(a[21]), indexer = truth(a[22]), fp8 = truth(a[23]);
+  const int64_t H = integer(a[24]), nope = integer(a[25]), Hidx = integer(a[26]);
+  const int interleave = truth(a[27]);
+  const float eps = float(real(a[28]));
+  Tensor q_full, kv, iq, iw, ik, iks;
+  {
+    NoGil unlocked;
+    const int64_t q_rank = q_a.size(0), width = kv_a.size(0), rope_dim = rope.mc.size(1), rank = width - rope_dim, D = ik_w.size(0);
+    const bool keep_kv = attention || kv_given, keep_ik = indexer || ik_given;
+    void* st = stream();
+
+    const Tensor x = xn.reshape({rows, hidden});
+    // what reads x_norm
+    Tensor qa, kva, ikr, c_q;
+    if (wx && !cq_in && keep_kv && keep_ik) {
+      const Tensor y = linear_of(x, *wx);
+      qa = y.narrow(1, 0, q_rank), kva = y.narrow(1, q_rank, width), ikr = y.narrow(1, q_rank + width, D);
+    } else {
+      linears(x, {{cq_in ? nullptr : &q_a, &qa}, {keep_kv ? &kv_a : nullptr, &kva}, {keep_ik ? &ik_w : nullptr, &ikr}});
+  }
+  c_q = cq_in ? cq_in->reshape({rows, q_rank}).contiguous() : fresh({rows, q_rank}, type, x);
+  if (kv_given) kv = *kv_given;
+  else if (keep_kv) kv = fresh({rows / seq, seq, width}, type, x);
+  if (ik_given) {
+    ik = *ik_given;
+    if (iks_given) iks = *iks_given;
+  } else if (keep_ik) {
+    ik = fresh({rows / seq, seq, D}, fp8 ? at::kByte : type, x);
+    if (fp8) iks = fresh({rows / seq, seq}, at::kFloat, x);
+  }
+  if (keep_kv) need(kv.is_contiguous() && kv.scalar_type() == type && kv.dim() == 3 && kv.size(0) * seq == rows && kv.size(1) >= seq && kv.size(2) == width, "latent cache: [n_seq, cap, w] of the operands' type");
+  if (keep_ik) need(ik.is_contiguous() && ik.dim() == 3 && ik.size(0) * seq == rows && ik.size(1) >= seq && ik.size(2) == D && (fp8 ? iks.defined() && iks.is_contiguous() : ik.scalar_type() == type), "index-key cache: [n_seq, cap, D]");
+  if (qa.defined() || keep_kv || keep_ik)
+    ok(api.dsa_prefill_latents(
+        qa.defined() ? ptr(qa) : nullptr, qa.defined() ? qa.stride(0) : 0, keep_kv ? ptr(kva) : nullptr, keep_kv ? kva.stride(0) : 0,
+        keep_ik ? ptr(ikr) : nullptr, keep_ik ? ikr.stride(0) : 0, ptr(q_norm), ptr(kv_norm), ptr(rope.mc), ptr(rope.ms), ptr(rope.ic),
+        ptr(rope.is), ptr(c_q), keep_kv ? ptr(kv) : nullptr, keep_kv ? kv.size(1) : 0, keep_ik ? ptr(ik) : nullptr,
+        iks.defined() ? as<float>(iks) : nullptr, keep_ik ? ik.size(1) : 0, rows, int(seq), int(q_rank), int(rank), int(rope_dim), int(D),
+        interleave, eps, dt, st));
+
+  // what reads c_q
+  Tensor q, iqr, w;
+  if (wc && attention && indexer) {
+    const Tensor y = linear_of(c_q, *wc);
+    q = y.narrow(1, 0, q_b.size(0)), iqr = y.narrow(1, q_b.size(0), iq_w.size(0)), w = y.narrow(1, q_b.size(0) + iq_w.size(0), Hidx);
+  } else {
+    linears(c_q, {{attention ? &q_b : nullptr, &q}, {indexer ? &iq_w : nullptr, &iqr}, {indexer ? &w_w : nullptr, &w}});
+  }
+  if (attention) {
+    q = q.unflatten(1, {H, nope + rope_dim});
+    q_full = fresh({rows, H, width}, type, x);
+    const Tensor w_uk = kv_b.view({H, kv_b.size(0) / H, rank}).narrow(1, 0, nope);
+    Tensor dst = q_full.narrow(2, 0, rank).transpose(0, 1);  // absorb W_UK: the GEMM writes its columns in place
+    at::bmm_out(dst, q.narrow(2, 0, nope).transpose(0, 1), w_uk);
+  }
+  if (indexer) {
+    iq = fresh({rows, Hidx, D}, fp8 ? at::kByte : type, x);
+    iw = fp8 ? fresh({rows, Hidx}, at::kFloat, x) : w.contiguous();
+  }
+  if (attention || indexer)
+    ok(api.dsa_prefill_queries(attention ? ptr(q) : nullptr, attention ? q.stride(0) : 0, attention ? q.stride(1) : 0, int(nope),
+                                   indexer ? ptr(iqr) : nullptr, indexer ? iqr.stride(0) : 0, indexer ? ptr(w) : nullptr,
+                                   indexer ? w.stride(0) : 0, ptr(rope.mc), ptr(rope.ms), ptr(rope.ic), ptr(rope.is),
+                                   attention ? ptr(q_full) : nullptr, indexer ? ptr(iq) : nullptr, indexer && fp8 ? as<float>(iw) : nullptr,
+                                   rows, int(seq), int(H), int(Hidx), int(rank), int(rope_dim), int(D), interleave, dt, st));
+  }
+  PyObject* t = PyTuple_New(6);
+  const Tensor* parts[6] = {&q_full, &kv, &iq, &iw, &ik, &iks};
+  for (int i = 0; i < 6; ++i) PyTuple_SET_ITEM(t, i, parts[i]->defined() ? THPVariable_Wrap(*parts[i]) : same(Py_None));
+  return t;
+}
+
+// (o [rows, H', rank], kv_b, o_proj, heads, v_dim) -> [rows, hidden]: W_UV per head, then o_proj
+PyObject* project_output(PyObject* const* a) {
+  const Tensor &o = ten(a[0], "o"), &kv_b = ten(a[1], "kv_b"), &o_proj = ten(a[2], "o_proj");
+  const int64_t H = integer(a[3]), v = integer(a[4]), rows = o.size(0);
+  Tensor y;
+  {
+    NoGil unlocked;
+    const Tensor ov = fresh({rows, H, v}, o.scalar_type(), o);
+    const int64_t per = kv_b.size(0) / H;
+    const Tensor w_uv = kv_b.view({H, per, kv_b.size(1)}).narrow(1, per - v, v);
+    Tensor dst = ov.transpose(0, 1);
+    at::bmm_out(dst, o.narrow(1, 0, H).transpose(0, 1), w_uv.transpose(1, 2));
+    y = linear_of(ov.view({rows, H * v}), o_proj);
+  }
+  return THPVariable_Wrap(y);
+}
+
+// (h_norm [rows, hidden], gate, up, down) -> [rows, hidden]: the SwiGLU MLP
+PyObject* mlp(PyObject* const* a) {
+  const Tensor &x = ten(a[0], "h_norm"), &gate = ten(a[1], "gate"), &up = ten(a[2], "up"), &down = ten(a[3], "down");
+  const at::ScalarType type = x.scalar_type();
+  dtype_of(type);
+  Tensor y;
+  {
+    NoGil unlocked;
+    Tensor act;
+    void* st = stream();
+    if (small_f32(x, {&gate, &up})) {
+      act = fresh({x.size(0), gate.size(0)}, type, x);
+      ok(api.dsa_linear_f32(as<float>(x), x.size(0), int(x.size(1)), as<float>(gate), int(gate.size(0)), as<float>(act), as<float>(up),
+                                int(up.size(0)), nullptr, nullptr, 0, nullptr, 1, st));
+    } else {
+      const Tensor g = at::mm(x, gate.t()), u = at::mm(x, up.t());
+      act = at::empty_like(g);
+      if (type == at::kFloat) ok(api.dsa_silu_mul_f32(as<float>(g), as<float>(u), as<float>(act), g.numel(), st));
+      else ok(api.dsa_silu_mul_bf16(ptr(g), ptr(u), ptr(act), g.numel(), st));
+  }
+  y = linear_of(act, down);
+  }
+  return THPVariable_Wrap(y);
+}
+
 // ---------------------------------------------------------------- the ABI's functions as they are
 // abi_<name>(args without the stream): a pointer argument is a tensor, None or an address. For callers that
 // mirror another extension's argument lists and hand over what they were given (kernels_ext.py).
@@ -716,6 +898,12 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
   try {
     return fn(args);
   } catch (const PyErrorSet&) {
+  } catch (const ValueError& e) {
+    PyErr_SetString(PyExc_ValueError, e.msg.c_str());
+  } catch (const StatusError& e) {
+    PyObject* r = PyObject_CallFunction(status_check, "i", e.status);  // raises with the library's message
+    if (r) PyErr_SetString(PyExc_RuntimeError, "dsa_b200: call failed");
+    Py_XDECREF(r);
   } catch (const std::exception& e) {
     PyErr_SetString(PyExc_RuntimeError, e.what());
   }
@@ -750,7 +938,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef methods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&bind)), METH_FASTCALL, nullptr},
     M(scan_fp8, 10), M(scan_paged, 8), M(scan_f32, 7), M(topk, 11), M(topk_paged, 7), M(mla, 14), M(mla_f32, 7), M(rmsnorm, 3),
-    M(add_rmsnorm, 4), M(silu_mul, 2), M(indexer_stage, 18), M(latent_append, 11), M(prefill_latents, 16), M(prefill_queries, 13),
+    M(add_rmsnorm, 4), M(silu_mul, 2), M(indexer_stage, 18), M(latent_append, 11), M(prefill_latents, 16), M(prefill_queries, 13), M(full_operands, 29), M(project_output, 5), M(mlp, 4),
     M(abi_scan, AbiArgs<decltype(::dsa_indexer_scan_fp8)>::value), M(abi_scan_paged, AbiArgs<decltype(::dsa_indexer_scan_fp8_paged)>::value),
     M(abi_topk, AbiArgs<decltype(::dsa_topk_select)>::value), M(abi_mla, AbiArgs<decltype(::dsa_sparse_mla_decode)>::value),
     {nullptr, nullptr, 0, nullptr}};

@@ -543,40 +543,194 @@ indexer_scan_legacy_kernel(const Params p) {
   }
 }
 
-// fp32 scan for any head count / key width: one warp per key, lanes stride the
-// key dimension per head. Accuracy path of the full-sequence layer API.
-__global__ void __launch_bounds__(256)
+// fp32 scan for any head count / key width (accuracy path of the full-sequence layer API). One CTA =
+// up to kF32Rows query rows of one sequence x 32 keys: the keys sit in shared memory once for all those
+// rows (padded rows: a lane's 16-byte reads are conflict-free), a lane owns a key, each of the four
+// warps a quarter of the heads, whose sums meet in shared memory. Bound: shared-memory reads of the
+// queries (one broadcast 16 bytes per 4 multiply-adds of a warp, eight heads per key read). The form
+// with one warp per key and a five-step reduction per head took 204 us for 1024 rows x 512 keys x
+// 8 heads x 16 (fp32 preset, two prompts of 512) against 10 us.
+constexpr int kF32Keys = 32, kF32Rows = 8, kF32Warps = 4, kF32HeadsPerWarp = 8;
+constexpr int kF32Heads = kF32Warps * kF32HeadsPerWarp;  // heads whose queries are staged at a time
+constexpr int kF32Dims = 128;                            // dims staged at a time
+constexpr int kF32Pitch = kF32Dims + 4;
+__global__ void __launch_bounds__(kF32Warps * 32)
 indexer_scan_f32_kernel(const float* __restrict__ q, const float* __restrict__ w,
                         const float* __restrict__ k, const int32_t* __restrict__ seq_lens,
-                        float* __restrict__ logits, int rows_per_seq, int n_heads, int head_dim,
+                        float* __restrict__ logits, int rows_per_seq, int groups_per_seq, int n_heads, int head_dim,
                         int64_t ctx, int64_t k_seq_stride, int64_t slab_stride) {
-  extern __shared__ float s_qf[];  // [n_heads][head_dim] then w[n_heads]
-  const int r = blockIdx.y;
-  const int seq = r / rows_per_seq;
-  float* s_wf = s_qf + size_t(n_heads) * head_dim;
-  for (int i = threadIdx.x; i < n_heads * head_dim; i += blockDim.x)
-    s_qf[i] = q[size_t(r) * n_heads * head_dim + i];
-  for (int i = threadIdx.x; i < n_heads; i += blockDim.x) s_wf[i] = w[size_t(r) * n_heads + i];
-  __syncthreads();
-  int64_t len = seq_lens ? seq_lens[r] : ctx;
-  len = len < 0 ? 0 : (len > ctx ? ctx : len);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+  __shared__ __align__(16) float s_k[kF32Keys * kF32Pitch];
+  __shared__ __align__(16) float s_q[kF32Heads * kF32Dims];
+  __shared__ float s_part[kF32Warps * kF32Keys];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int seq = blockIdx.y / groups_per_seq, grp = blockIdx.y - seq * groups_per_seq;
+  const int row0 = seq * rows_per_seq + grp * kF32Rows, row1 = min(row0 + kF32Rows, (seq + 1) * rows_per_seq);
+  const int64_t s0 = int64_t(blockIdx.x) * kF32Keys, s = s0 + lane;
   const float neg_inf = __int_as_float(0xff800000);
-  for (int64_t s = int64_t(blockIdx.x) * wpb + warp; s < ctx; s += int64_t(gridDim.x) * wpb) {
-    if (s >= len) {
-      if (lane == 0) logits[int64_t(r) * slab_stride + s] = neg_inf;
+  const float* mine = s_k + lane * kF32Pitch;
+  int staged = -1;  // first dim of the keys in shared memory
+  for (int r = row0; r < row1; ++r) {
+    int64_t len = seq_lens ? int64_t(seq_lens[r]) : ctx;
+    len = len < 0 ? 0 : (len > ctx ? ctx : len);
+    if (s0 >= len) {  // nothing of this row's part is visible
+      if (warp == 0 && s < ctx) logits[int64_t(r) * slab_stride + s] = neg_inf;
       continue;
     }
-    const float* kr = k + (int64_t(seq) * k_seq_stride + s) * head_dim;
     float total = 0.f;
-    for (int h = 0; h < n_heads; ++h) {
-      float dot = 0.f;
-      for (int d = lane; d < head_dim; d += 32) dot = fmaf(s_qf[h * head_dim + d], kr[d], dot);
+    for (int h0 = 0; h0 < n_heads; h0 += kF32Heads) {
+      const int heads = min(kF32Heads, n_heads - h0), per = (heads + kF32Warps - 1) / kF32Warps;
+      const int first = warp * per, mine_n = max(0, min(per, heads - first));
+      float dot[kF32HeadsPerWarp] = {};
+      for (int d0 = 0; d0 < head_dim; d0 += kF32Dims) {
+        const int dims = min(kF32Dims, head_dim - d0), dp = (dims + 3) & ~3;
+        __syncthreads();  // the previous queries (and keys) have been read
+        if (staged != d0) {
+          staged = d0;
+          for (int i = tid; i < kF32Keys * dp; i += kF32Warps * 32) {
+            const int j = i / dp, d = i - j * dp;
+            s_k[j * kF32Pitch + d] =
+                (d < dims && s0 + j < ctx) ? k[(int64_t(seq) * k_seq_stride + s0 + j) * head_dim + d0 + d] : 0.f;
+          }
+        }
+        for (int i = tid; i < heads * dp; i += kF32Warps * 32) {
+          const int h = i / dp, d = i - h * dp;
+          s_q[h * kF32Dims + d] = d < dims ? q[(int64_t(r) * n_heads + h0 + h) * head_dim + d0 + d] : 0.f;
+        }
+        __syncthreads();
+        const float* qh = s_q + first * kF32Dims;
+        if (mine_n == kF32HeadsPerWarp) {
+#pragma unroll 2
+          for (int d = 0; d < dp; d += 4) {
+            const float4 kv = *reinterpret_cast<const float4*>(mine + d);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-      total = fmaf(s_wf[h], fmaxf(dot, 0.f), total);
+            for (int u = 0; u < kF32HeadsPerWarp; ++u) {
+              const float4 qv = *reinterpret_cast<const float4*>(qh + u * kF32Dims + d);
+              dot[u] = fmaf(qv.x, kv.x, dot[u]);
+              dot[u] = fmaf(qv.y, kv.y, dot[u]);
+              dot[u] = fmaf(qv.z, kv.z, dot[u]);
+              dot[u] = fmaf(qv.w, kv.w, dot[u]);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < kF32HeadsPerWarp; ++u) {
+            if (u >= mine_n) break;
+            for (int d = 0; d < dp; d += 4) {
+              const float4 kv = *reinterpret_cast<const float4*>(mine + d);
+              const float4 qv = *reinterpret_cast<const float4*>(qh + u * kF32Dims + d);
+              dot[u] = fmaf(qv.x, kv.x, dot[u]);
+              dot[u] = fmaf(qv.y, kv.y, dot[u]);
+              dot[u] = fmaf(qv.z, kv.z, dot[u]);
+              dot[u] = fmaf(qv.w, kv.w, dot[u]);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kF32HeadsPerWarp; ++u)
+        if (u < mine_n) total = fmaf(w[int64_t(r) * n_heads + h0 + first + u], fmaxf(dot[u], 0.f), total);
     }
-    if (lane == 0) logits[int64_t(r) * slab_stride + s] = total;
+    s_part[warp * kF32Keys + lane] = total;
+    __syncthreads();
+    if (warp == 0 && s < ctx)
+      logits[int64_t(r) * slab_stride + s] =
+          s < len ? (s_part[lane] + s_part[32 + lane]) + (s_part[64 + lane] + s_part[96 + lane]) : neg_inf;
+  }
+}
+
+// The same scan where a sequence has many query rows (prompts): the four warps split the CTA's eight
+// rows instead of the heads, two rows a warp, so a key read serves two rows and four heads and nothing
+// is summed across warps. As many heads as fit 16 KB are staged for all eight rows at once: with the
+// small preset's 8 heads x 16 dims one staging and one barrier per CTA where the kernel above has two
+// barriers per row (33 us for 2 x 512 rows against 512 keys).
+constexpr int kF32StageFloats = 4096;
+__global__ void __launch_bounds__(kF32Warps * 32)
+indexer_scan_f32_rows_kernel(const float* __restrict__ q, const float* __restrict__ w,
+                             const float* __restrict__ k, const int32_t* __restrict__ seq_lens,
+                             float* __restrict__ logits, int rows_per_seq, int groups_per_seq, int n_heads, int head_dim,
+                             int64_t ctx, int64_t k_seq_stride, int64_t slab_stride) {
+  __shared__ __align__(16) float s_k[kF32Keys * kF32Pitch];
+  __shared__ __align__(16) float s_q[kF32StageFloats];
+  __shared__ int s_len[kF32Rows];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int seq = blockIdx.y / groups_per_seq, grp = blockIdx.y - seq * groups_per_seq;
+  const int row0 = seq * rows_per_seq + grp * kF32Rows, rows = min(kF32Rows, (seq + 1) * rows_per_seq - row0);
+  const int64_t s0 = int64_t(blockIdx.x) * kF32Keys, s = s0 + lane;
+  const float neg_inf = __int_as_float(0xff800000);
+  if (tid < kF32Rows) {
+    int64_t len = 0;
+    if (tid < rows) len = seq_lens ? int64_t(seq_lens[row0 + tid]) : ctx;
+    s_len[tid] = int(len < 0 ? 0 : (len > ctx ? ctx : len));
+  }
+  __syncthreads();
+  int longest = 0;
+#pragma unroll
+  for (int i = 0; i < kF32Rows; ++i) longest = max(longest, s_len[i]);
+  const int ra = 2 * warp, rb = ra + 1;
+  float ta = 0.f, tb = 0.f;
+  if (s0 < longest) {
+    const int chunk = min(head_dim, kF32Dims), cp = (chunk + 3) & ~3;
+    // heads staged at a time: a multiple of four (four exactly when the dims come in several chunks)
+    int hb = head_dim > kF32Dims ? 4 : max(4, (kF32StageFloats / (kF32Rows * cp)) & ~3);
+    hb = min(hb, (n_heads + 3) & ~3);
+    const float* mine = s_k + lane * kF32Pitch;
+    int staged = -1;
+    for (int h0 = 0; h0 < n_heads; h0 += hb) {
+      float da[4] = {}, db[4] = {};
+      for (int d0 = 0; d0 < head_dim; d0 += kF32Dims) {
+        const int dims = min(kF32Dims, head_dim - d0), dp = (dims + 3) & ~3;
+        __syncthreads();  // what is staged has been read
+        if (staged != d0) {
+          staged = d0;
+          for (int i = tid; i < kF32Keys * dp; i += kF32Warps * 32) {
+            const int j = i / dp, d = i - j * dp;
+            s_k[j * kF32Pitch + d] =
+                (d < dims && s0 + j < ctx) ? k[(int64_t(seq) * k_seq_stride + s0 + j) * head_dim + d0 + d] : 0.f;
+          }
+        }
+        for (int i = tid; i < kF32Rows * hb * dp; i += kF32Warps * 32) {
+          const int rh = i / dp, d = i - rh * dp, r = rh / hb, h = h0 + rh - r * hb;
+          s_q[i] = (r < rows && h < n_heads && d < dims) ? q[(int64_t(row0 + r) * n_heads + h) * head_dim + d0 + d] : 0.f;
+        }
+        __syncthreads();
+        for (int g = 0; g < hb; g += 4) {
+          if (head_dim <= kF32Dims) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) da[u] = db[u] = 0.f;
+          }
+          const float *qa = s_q + (ra * hb + g) * dp, *qb = s_q + (rb * hb + g) * dp;
+          for (int d = 0; d < dp; d += 4) {
+            const float4 kv = *reinterpret_cast<const float4*>(mine + d);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const float4 x = *reinterpret_cast<const float4*>(qa + u * dp + d), y = *reinterpret_cast<const float4*>(qb + u * dp + d);
+              da[u] = fmaf(x.x, kv.x, da[u]);
+              da[u] = fmaf(x.y, kv.y, da[u]);
+              da[u] = fmaf(x.z, kv.z, da[u]);
+              da[u] = fmaf(x.w, kv.w, da[u]);
+              db[u] = fmaf(y.x, kv.x, db[u]);
+              db[u] = fmaf(y.y, kv.y, db[u]);
+              db[u] = fmaf(y.z, kv.z, db[u]);
+              db[u] = fmaf(y.w, kv.w, db[u]);
+            }
+          }
+          if (d0 + kF32Dims >= head_dim) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int h = h0 + g + u;
+              if (h < n_heads) {
+                if (ra < rows) ta = fmaf(w[int64_t(row0 + ra) * n_heads + h], fmaxf(da[u], 0.f), ta);
+                if (rb < rows) tb = fmaf(w[int64_t(row0 + rb) * n_heads + h], fmaxf(db[u], 0.f), tb);
+              }
+            }
+          }
+        }
+      }
+    }
+  }
+  if (s < ctx) {
+    if (ra < rows) logits[int64_t(row0 + ra) * slab_stride + s] = s < s_len[ra] ? ta : neg_inf;
+    if (rb < rows) logits[int64_t(row0 + rb) * slab_stride + s] = s < s_len[rb] ? tb : neg_inf;
   }
 }
 

@@ -697,5 +697,116 @@ sparse_mla_f32_kernel(const float* __restrict__ q, const float* __restrict__ kv,
   }
 }
 
+// The same for many rows (full-sequence layers): one CTA per (row, block of eight heads). A tile of 16
+// latent rows is gathered into shared memory once for the eight heads (padded rows: conflict-free
+// 16-byte reads); a thread owns one (head, key) pair of the scores and every 128th value column of the
+// result for all eight heads. The kernel above gathers every row once per head and waits for a chunk of
+// 128 keys whatever the list's length: 66 us for 1024 rows x 8 heads x 16 keys x 80 against 12 us.
+constexpr int kF32Heads = 8, kF32Keys = 16, kF32Threads = kF32Heads * kF32Keys;
+__host__ __device__ inline int f32_rows_pitch(int qk_dim) { return (qk_dim + 7) / 8 * 8 + 4; }
+inline size_t f32_rows_smem(int qk_dim) {
+  return (size_t(kF32Heads + kF32Keys) * f32_rows_pitch(qk_dim) + kF32Heads * kF32Keys + 2 * kF32Heads) * 4;
+}
+__global__ void __launch_bounds__(kF32Threads)
+sparse_mla_f32_rows_kernel(const float* __restrict__ q, const float* __restrict__ kv,
+                           const int32_t* __restrict__ indices, const int32_t* __restrict__ seq_lens,
+                           float* __restrict__ out, int rows_per_seq, int H, int qk_dim, int v_dim,
+                           int topk, float sm_scale, int64_t kv_seq_stride, int64_t ctx) {
+  extern __shared__ __align__(16) float s_fr[];
+  const int pitch = f32_rows_pitch(qk_dim), dp = (qk_dim + 3) & ~3;
+  float* s_q = s_fr;                               // [8][pitch]
+  float* s_k = s_q + kF32Heads * pitch;            // [16][pitch]
+  float* s_p = s_k + kF32Keys * pitch;             // [16 keys][8 heads]
+  float* s_alpha = s_p + kF32Heads * kF32Keys;     // [8]
+  float* s_inv = s_alpha + kF32Heads;              // [8]
+  const int tid = threadIdx.x, key = tid & 15, head = tid >> 4;
+  const int r = blockIdx.x, h0 = blockIdx.y * kF32Heads, heads = min(kF32Heads, H - h0);
+  const int seq = r / rows_per_seq;
+  int64_t len = seq_lens ? int64_t(seq_lens[r]) : ctx;
+  len = len < 0 ? 0 : (len > ctx ? ctx : len);
+  const float* kvs = kv + int64_t(seq) * kv_seq_stride * qk_dim;
+  for (int i = tid; i < kF32Heads * dp; i += kF32Threads) {
+    const int h = i / dp, d = i - h * dp;
+    s_q[h * pitch + d] = (h < heads && d < qk_dim) ? q[(int64_t(r) * H + h0 + h) * qk_dim + d] : 0.f;
+  }
+  const int64_t n_keys = indices ? int64_t(topk) : len;
+  float m_run = -INFINITY, l_run = 0.f;            // of this thread's head (equal in its 16 lanes)
+  float o[kF32Heads][4] = {};                      // value columns tid, tid + 128, ... of every head
+  for (int64_t c0 = 0; c0 < n_keys; c0 += kF32Keys) {
+    // every thread looks at entry c0 + key, so that the 16 entries are known to each half-warp
+    const int64_t j = c0 + key;
+    int64_t idx = -1;
+    if (j < n_keys) idx = indices ? int64_t(indices[int64_t(r) * topk + j]) : j;
+    const bool ok = idx >= 0 && idx < len;
+    const uint32_t any = __ballot_sync(0xffffffffu, ok);
+    if ((any & 0xFFFFu) == 0u) continue;           // (the same 16 entries in both halves of every warp)
+    __syncthreads();                               // the previous tile and its probabilities have been read
+    for (int k = head; k < kF32Keys; k += kF32Heads) {  // 16 threads per latent row
+      const int64_t at = __shfl_sync(0xffffffffu, ok ? idx : int64_t(-1), k);
+      for (int d = key; d < dp; d += 16) s_k[k * pitch + d] = (at >= 0 && d < qk_dim) ? kvs[at * qk_dim + d] : 0.f;
+    }
+    __syncthreads();
+    float s = 0.f;
+    const float *qr = s_q + head * pitch, *kr = s_k + key * pitch;
+#pragma unroll 4
+    for (int d = 0; d < dp; d += 4) {
+      const float4 a = *reinterpret_cast<const float4*>(qr + d), b = *reinterpret_cast<const float4*>(kr + d);
+      s = fmaf(a.x, b.x, s);
+      s = fmaf(a.y, b.y, s);
+      s = fmaf(a.z, b.z, s);
+      s = fmaf(a.w, b.w, s);
+    }
+    s = ok ? s * sm_scale : -INFINITY;
+    float mx = s;
+#pragma unroll
+    for (int of = 8; of > 0; of >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, of));
+    const float m_new = fmaxf(m_run, mx);
+    const float pj = (ok && m_new != -INFINITY) ? expf(s - m_new) : 0.f;
+    float ps = pj;
+#pragma unroll
+    for (int of = 8; of > 0; of >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, of);
+    const float alpha = (m_new == -INFINITY) ? 1.f : expf(m_run - m_new);
+    l_run = l_run * alpha + ps;
+    m_run = m_new;
+    s_p[key * kF32Heads + head] = pj;
+    if (key == 0) s_alpha[head] = alpha;
+    __syncthreads();
+    float al[kF32Heads];
+#pragma unroll
+    for (int h = 0; h < kF32Heads; ++h) al[h] = s_alpha[h];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int col = tid + c * 128;
+      if (col >= v_dim) break;
+#pragma unroll
+      for (int h = 0; h < kF32Heads; ++h) o[h][c] *= al[h];
+#pragma unroll 4
+      for (int k = 0; k < kF32Keys; ++k) {
+        const float v = s_k[k * pitch + col];
+        const float4 p0 = *reinterpret_cast<const float4*>(s_p + k * kF32Heads);
+        const float4 p1 = *reinterpret_cast<const float4*>(s_p + k * kF32Heads + 4);
+        o[0][c] = fmaf(p0.x, v, o[0][c]);
+        o[1][c] = fmaf(p0.y, v, o[1][c]);
+        o[2][c] = fmaf(p0.z, v, o[2][c]);
+        o[3][c] = fmaf(p0.w, v, o[3][c]);
+        o[4][c] = fmaf(p1.x, v, o[4][c]);
+        o[5][c] = fmaf(p1.y, v, o[5][c]);
+        o[6][c] = fmaf(p1.z, v, o[6][c]);
+        o[7][c] = fmaf(p1.w, v, o[7][c]);
+      }
+    }
+  }
+  if (key == 0) s_inv[head] = l_run > 0.f ? 1.f / l_run : 0.f;
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int col = tid + c * 128;
+    if (col >= v_dim) break;
+#pragma unroll
+    for (int h = 0; h < kF32Heads; ++h)
+      if (h < heads) out[(int64_t(r) * H + h0 + h) * v_dim + col] = o[h][c] * s_inv[h];
+  }
+}
+
 }  // namespace mla
 }  // namespace dsa

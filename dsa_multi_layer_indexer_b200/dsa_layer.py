@@ -24,10 +24,16 @@ from typing import Optional, Tuple
 
 import torch
 from torch import nn
+from torch.nn.modules import module as _module_hooks
 
-from . import ops
+from . import _lib, ops
 from .config import DSAConfig
 from .rope import apply_rotary, apply_rotary_at
+
+
+# The linear projections of a layer, in construction order.
+_PROJECTIONS = ("q_a_proj", "q_b_proj", "kv_a_proj", "kv_b_proj", "o_proj", "index_q_proj", "index_k_proj",
+                "index_weights_proj", "gate_proj", "up_proj", "down_proj")
 
 
 @dataclasses.dataclass
@@ -48,9 +54,10 @@ class RMSNorm(nn.Module):
 
     def add_forward(self, x: torch.Tensor, delta: torch.Tensor):
         """``(x + delta, self(x + delta))``: the residual addition and this norm, one
-        launch for bf16 rows on a CUDA device, two separate steps otherwise."""
-        if (x.is_cuda and x.dtype == torch.bfloat16 and delta.dtype == torch.bfloat16 and x.shape == delta.shape
-                and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192 and not torch.is_grad_enabled()):
+        launch for bf16 and fp32 rows on a CUDA device, two separate steps otherwise."""
+        if (x.is_cuda and not torch.is_grad_enabled() and x.dtype == delta.dtype and x.shape == delta.shape
+                and (x.dtype == torch.float32
+                     or (x.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192))):
             return ops.add_rmsnorm(x, delta, self.weight, self.eps)
         s = x + delta
         return s, self(s)
@@ -103,19 +110,24 @@ class IndexerWorkspace:
 class FullOperands:
     """A full-sequence layer's operands of the scan and the attention (``DSALayer.full_operands``).
 
-    fused: ready for the kernels -- q [B*S,H,Dqk], kv [B,cap,Dqk], iq / iw / ik (/ ik_scale) of the FP8
-    scan (ik [B,cap,128] e4m3 bytes) or of the fp32 scan. Otherwise the torch tensors as computed."""
+    With ``weights`` (the fused chain's): ready for the kernels -- q [B*S,H,Dqk], kv [B,cap,Dqk], iq / iw /
+    ik (/ ik_scale) of the FP8 scan (ik [B,cap,128] e4m3 bytes) or of the fp32 scan. Otherwise the torch
+    tensors as computed."""
 
     b: int
     s: int
     lens: torch.Tensor  # int32 [B*S]: causally visible keys of every row
-    fused: bool
+    weights: Optional[Tuple[torch.Tensor, ...]]
     q: Optional[torch.Tensor]
     kv: Optional[torch.Tensor]
     iq: Optional[torch.Tensor]
     iw: Optional[torch.Tensor]
     ik: Optional[torch.Tensor]
     ik_scale: Optional[torch.Tensor]
+
+    @property
+    def fused(self) -> bool:
+        return self.weights is not None
 
 
 def _pad_heads(t: torch.Tensor, multiple: int) -> torch.Tensor:
@@ -270,14 +282,16 @@ class DSALayer(nn.Module):
 
     # ------------------------------------------------------------------ full sequence
     def full_operands(self, x_norm, rope: RopeCaches, c_q=None, attention: bool = True, indexer: bool = True,
-                      cache: Optional["LayerDecodeCache"] = None) -> "FullOperands":
+                      cache: Optional["LayerDecodeCache"] = None, lens: Optional[torch.Tensor] = None) -> "FullOperands":
         """Everything a full-sequence layer computes from x_norm [B,S,hidden] before its scan and its
         attention, once for both. With a ``cache`` the latent rows and index keys are written to (and
-        read from) the first S rows of the cache."""
-        c = self.config
+        read from) the first S rows of the cache. ``lens``: the causal lengths, if the caller has them."""
         b, s, _ = x_norm.shape
-        if self._fused_full(x_norm) and (cache is None or (cache.k_scale is not None) == self._fast_path(x_norm)):
-            return self._full_operands_fused(x_norm, rope, c_q, attention, indexer, cache)
+        if lens is None:
+            lens = self._causal_lens(b, s, x_norm.device)
+        weights = self._full_weights(x_norm)
+        if weights is not None and (cache is None or (cache.k_scale is not None) == self._fast_path(x_norm)):
+            return self._full_operands_fused(weights, x_norm, rope, c_q, attention, indexer, cache, lens)
         if c_q is None:
             c_q = self.q_latent(x_norm)
         q = kv = iq = ik = w = None
@@ -295,79 +309,53 @@ class DSALayer(nn.Module):
                 cache.k_scale[:, :s] = sk
             else:
                 cache.index_k[:, :s] = ik.float()
-        return FullOperands(b, s, self._causal_lens(b, s, x_norm.device), False, q, kv, iq, w, ik, None)
+        return FullOperands(b, s, lens, None, q, kv, iq, w, ik, None)
 
-    def _fused_full(self, t: torch.Tensor) -> bool:
-        """True when the fused full-sequence preparation applies: it has no autograd, and knows the
-        fp32 form of any geometry and the bf16 / e4m3 form of the production geometry."""
-        return (t.is_cuda and not torch.is_grad_enabled() and (t.dtype == torch.float32 or self._fast_path(t))
-                and self.q_a_proj.weight.dtype == t.dtype)
+    def _full_weights(self, t: torch.Tensor) -> Optional[Tuple[torch.Tensor, ...]]:
+        """The projections' weights, in construction order, where the fused full-sequence chain applies
+        to ``t``, else None: it has no autograd or autocast, knows the fp32 form of any geometry and the
+        bf16 / e4m3 form of the production geometry, and needs every projection to be a plain
+        ``nn.Linear`` (not replaced, no bias, no hooks on it)."""
+        dtype = t.dtype
+        if not (t.is_cuda and (dtype == torch.float32 or self._fast_path(t))) or torch.is_grad_enabled() or torch.is_autocast_enabled():
+            return None
+        if _module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks:
+            return None
+        mods, out = self._modules, []
+        for name in _PROJECTIONS:
+            m = mods[name]
+            d = m.__dict__
+            w = d["_parameters"].get("weight")
+            if (m.__class__ is not nn.Linear or w is None or w.dtype != dtype or d["_parameters"].get("bias") is not None
+                    or d["_forward_hooks"] or d["_forward_pre_hooks"]):
+                return None
+            out.append(w)
+        return tuple(out)
 
-    def _full_operands_fused(self, x_norm, rope, c_q, attention, indexer, cache) -> "FullOperands":
+    def _full_operands_fused(self, weights, x_norm, rope, c_q, attention, indexer, cache, lens) -> "FullOperands":
         c = self.config
         b, s, _ = x_norm.shape
-        rows, h, dev, dt = b * s, c.num_attention_heads, x_norm.device, x_norm.dtype
+        dt = x_norm.dtype
         fp8 = self._fast_path(x_norm)
-        linear = torch.nn.functional.linear
-        x2 = x_norm.reshape(rows, -1)
+        q_a, q_b, kv_a, kv_b, _, iq_w, ik_w, w_w = weights[:8]
         if rope.mla_cos.dtype != dt:
             rope = RopeCaches(*(t.to(dt) for t in (rope.mla_cos, rope.mla_sin, rope.idx_cos, rope.idx_sin)))
-        stacked = fp8 and self._stacked()
-        keep_kv, keep_ik = attention or cache is not None, indexer or cache is not None
-        # ---- what reads x_norm
-        qa = kv_a = ik_raw = kv = ik = ik_scale = None
-        if stacked and c_q is None and keep_kv and keep_ik:
-            qa, kv_a, ik_raw = linear(x2, self._wx).split([c.q_lora_rank, c.qk_head_dim, c.index_head_dim], dim=1)
-        else:
-            if c_q is None:
-                qa = self.q_a_proj(x2)
-            if keep_kv:
-                kv_a = self.kv_a_proj(x2)
-            if keep_ik:
-                ik_raw = self.index_k_proj(x2)
-        if qa is not None:
-            c_q = torch.empty(rows, c.q_lora_rank, dtype=dt, device=dev)
-        else:
-            c_q = c_q.reshape(rows, -1)
+        wx = wc = None
+        if fp8 and self._stacked():
+            wx, wc = self._wx, self._wc
+        kv = ik = ik_scale = None
         if cache is not None:
             kv, ik, ik_scale = cache.kv, cache.index_k, cache.k_scale
-        else:
-            if keep_kv:
-                kv = torch.empty(b, s, c.qk_head_dim, dtype=dt, device=dev)
-            if keep_ik:
-                ik = torch.empty(b, s, c.index_head_dim, dtype=torch.uint8 if fp8 else dt, device=dev)
-                ik_scale = torch.empty(b, s, dtype=torch.float32, device=dev) if fp8 else None
-        il = c.indexer_rope_interleave
-        if qa is not None or keep_kv or keep_ik:
-            ops.prefill_latents(qa, kv_a, ik_raw, self.q_a_layernorm.weight, self.kv_a_layernorm.weight, rope, c_q, kv, ik,
-                                ik_scale, s, il, c.rms_norm_eps)
-        # ---- what reads c_q
-        nope, rd = c.qk_nope_head_dim, c.qk_rope_head_dim
-        q = iq_raw = w = q_full = iq = iw = None
-        if stacked and attention and indexer:
-            q, iq_raw, w = linear(c_q, self._wc).split(
-                [h * (nope + rd), c.index_n_heads * c.index_head_dim, c.index_n_heads], dim=1)
-        else:
-            if attention:
-                q = self.q_b_proj(c_q)
-            if indexer:
-                iq_raw, w = self.index_q_proj(c_q), self.index_weights_proj(c_q)
-        if attention:
-            q = q.unflatten(1, (h, nope + rd))
-            q_full = torch.empty(rows, h, c.qk_head_dim, dtype=dt, device=dev)
-            w_uk, _ = self._w_uk_uv()  # absorb W_UK into the query: the GEMM writes its columns of q_full in place
-            torch.bmm(q[:, :, :nope].transpose(0, 1), w_uk, out=q_full[:, :, :c.kv_lora_rank].transpose(0, 1))
-        if indexer:
-            iq = torch.empty(rows, c.index_n_heads, c.index_head_dim, dtype=torch.uint8 if fp8 else dt, device=dev)
-            iw = torch.empty(rows, c.index_n_heads, dtype=torch.float32, device=dev) if fp8 else w.contiguous()
-        if attention or indexer:
-            ops.prefill_queries(q, nope, iq_raw, w, rope, q_full, iq, iw if fp8 else None, s, il)
-        return FullOperands(b, s, self._causal_lens(b, s, dev), True, q_full, kv, iq, iw, ik, ik_scale)
+        parts = _lib.host().full_operands(
+            x_norm, s, c_q, wx, wc, q_a, kv_a, ik_w, q_b, iq_w, w_w, self.q_a_layernorm.weight, self.kv_a_layernorm.weight,
+            kv_b, rope.mla_cos, rope.mla_sin, rope.idx_cos, rope.idx_sin, kv, ik, ik_scale, attention, indexer, fp8,
+            c.num_attention_heads, c.qk_nope_head_dim, c.index_n_heads, c.indexer_rope_interleave, c.rms_norm_eps)
+        return FullOperands(b, s, lens, weights, *parts)
 
     def full_select(self, op: "FullOperands", pad_value: int = -1, padded: bool = True) -> torch.Tensor:
         """int32 [B*S, topk] selected key positions of every row. ``padded`` False: without the columns
         that no row of a short sequence can fill (min(topk, S) columns)."""
-        if not op.fused:
+        if op.weights is None:
             return self._select(op.iq, op.ik, op.iw, op.lens, op.s, pad_value)
         topk = self.config.index_topk if padded else min(self.config.index_topk, op.s)
         if op.ik_scale is not None:
@@ -379,7 +367,7 @@ class DSALayer(nn.Module):
     def full_attend(self, op: "FullOperands", indices: Optional[torch.Tensor]) -> torch.Tensor:
         """Attention hidden output [B,S,hidden]; indices int32 [B*S, topk] or None (dense causal)."""
         c = self.config
-        if not op.fused:
+        if op.weights is None:
             o = self._attend(op.q, op.kv, indices, op.lens, op.s)
             return self._project_output(o.view(op.b, op.s, *o.shape[1:]))
         h = op.q.shape[1]
@@ -388,10 +376,7 @@ class DSALayer(nn.Module):
                                       rows_per_seq=op.s, dense_keys=op.s)
         else:
             o = ops.sparse_mla_f32(op.q, op.kv, indices, c.kv_lora_rank, self.sm_scale, op.lens, rows_per_seq=op.s)
-        _, w_uv = self._w_uk_uv()
-        ov = torch.empty(o.shape[0], h, c.v_head_dim, dtype=o.dtype, device=o.device)
-        torch.bmm(o[:, :h].transpose(0, 1), w_uv.transpose(1, 2), out=ov.transpose(0, 1))
-        return self._reduced(self.o_proj(ov.view(op.b, op.s, h * c.v_head_dim)))
+        return self._reduced(_lib.host().project_output(o, op.weights[3], op.weights[4], h, c.v_head_dim).view(op.b, op.s, -1))
 
     # ------------------------------------------------------------------ reference API (full sequence)
     def indexer_indices(self, x_norm, rope: RopeCaches, c_q=None) -> torch.Tensor:
@@ -413,13 +398,17 @@ class DSALayer(nn.Module):
         nxt = self.full_select(op, pad_value=op.s).view(op.b, op.s, -1).long() if produce_indexer else None
         return attn_hidden, nxt
 
-    def mlp(self, h_norm: torch.Tensor) -> torch.Tensor:
+    def mlp(self, h_norm: torch.Tensor, weights=None) -> torch.Tensor:
         if (h_norm.is_cuda and h_norm.dtype == torch.bfloat16 and h_norm.dim() == 2 and h_norm.shape[0] <= 2
                 and not torch.is_grad_enabled()):
             gate, up = ops.gemv(h_norm, self.gate_proj.weight), ops.gemv(h_norm, self.up_proj.weight)
             return self._reduced(self.down_proj(ops.silu_mul(gate, up)))
+        w = self._full_weights(h_norm) if h_norm.dim() == 3 and weights is None else weights
+        if w is not None:
+            y = _lib.host().mlp(h_norm.reshape(-1, h_norm.shape[2]), w[8], w[9], w[10])
+            return self._reduced(y.view(h_norm.shape[0], h_norm.shape[1], -1))
         gate, up = self.gate_proj(h_norm), self.up_proj(h_norm)
-        if gate.is_cuda and gate.dtype == torch.bfloat16 and not torch.is_grad_enabled():
+        if gate.is_cuda and gate.dtype in (torch.bfloat16, torch.float32) and not torch.is_grad_enabled():
             return self._reduced(self.down_proj(ops.silu_mul(gate, up)))  # one launch instead of two
         return self._reduced(self.down_proj(torch.nn.functional.silu(gate) * up))
 

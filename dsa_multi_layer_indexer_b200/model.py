@@ -129,6 +129,19 @@ class DSAModel(nn.Module):
                                    interleave=c.indexer_rope_interleave)
         return RopeCaches(mc, ms, ic, is_)
 
+    def _rope_for(self, seq_len: int, device, dtype) -> RopeCaches:
+        """Tables of at least ``seq_len`` rows for one full-sequence pass: the last pass's (a table row
+        depends on its position alone), rebuilt when it was shorter or made for another type, device or
+        stream. A graph capture gets tables of its own, which live as long as the graph."""
+        if torch.cuda.is_current_stream_capturing():
+            return self._build_rope(seq_len, device, dtype)
+        c = self.config
+        key = (device, dtype, torch.cuda.current_stream(device).cuda_stream, c.qk_rope_head_dim, c.index_head_dim, c.rope_theta, c.indexer_rope_interleave)
+        kept = getattr(self, "_rope_kept", None)
+        if kept is None or kept[0] != key or kept[1].mla_cos.shape[0] < seq_len:
+            kept = self._rope_kept = (key, self._build_rope(seq_len, device, dtype))
+        return kept[1]
+
     def _lagged_indexer_layers(self, types) -> List[bool]:
         return lagged_producers(types)
 
@@ -139,7 +152,7 @@ class DSAModel(nn.Module):
             raise ValueError(f"inputs_embeds must be [B,S,H], got {tuple(inputs_embeds.shape)}")
         if not inputs_embeds.is_cuda:
             raise RuntimeError("this implementation runs on a CUDA device only (there is no CPU path)")
-        rope = self._build_rope(inputs_embeds.shape[1], inputs_embeds.device, inputs_embeds.dtype)
+        rope = self._rope_for(inputs_embeds.shape[1], inputs_embeds.device, inputs_embeds.dtype)
         used, produced = ([], []) if record else (None, None)
         x = self._run_full(inputs_embeds, rope, mode, cold_start, None, used, produced)
         return ForwardTrace(x, used, produced) if record else x
@@ -156,6 +169,7 @@ class DSAModel(nn.Module):
         produces = lagged_producers(types)
         lagged = mode is not ScheduleMode.BASELINE
         prev: Optional[torch.Tensor] = None
+        lens = DSALayer._causal_lens(b, s, x.device)
         x_norm = self.layers[0].attn_norm(x)
         for li, layer in enumerate(self.layers):
             is_dsa = types[li] is AttentionType.DSA
@@ -164,7 +178,8 @@ class DSAModel(nn.Module):
                 raise ValueError(f"unknown cold start policy: {cold_start}")
             eager = cold and cold_start is ColdStartPolicy.EAGER  # layer 0 attends its own selection
             makes = produces[li] if lagged else is_dsa
-            op = layer.full_operands(x_norm, rope, indexer=makes or eager, cache=None if caches is None else caches[li])
+            op = layer.full_operands(x_norm, rope, indexer=makes or eager,
+                                     cache=None if caches is None else caches[li], lens=lens)
             own = layer.full_select(op, pad_value=s, padded=used is not None) if makes or eager else None
             made = own if makes else None
             if not is_dsa:
@@ -174,7 +189,7 @@ class DSAModel(nn.Module):
             else:
                 attend = prev  # (None at layer 0 with a dense cold start)
             attn = layer.full_attend(op, attend)
-            x, x_norm = self._residual_tail(li, x, attn)
+            x, x_norm = self._residual_tail(li, x, attn, op.weights)
             prev = made
             if used is not None:
                 used.append(None if attend is None else attend.view(b, s, -1).long())
@@ -311,14 +326,14 @@ class DSAModel(nn.Module):
             record["used"], record["produced"] = used, produced
         return x_norm  # the last layer's tail applied the final norm
 
-    def _residual_tail(self, li: int, x: torch.Tensor, attn: torch.Tensor):
+    def _residual_tail(self, li: int, x: torch.Tensor, attn: torch.Tensor, weights=None):
         """``h = x + attn; x' = h + mlp(ffn_norm(h))`` and the norm the next consumer
         applies to ``x'`` (the next layer's attn_norm, or the final norm after the last
         layer): each residual addition is fused with the norm that follows it."""
         layer = self.layers[li]
         h, h_norm = layer.ffn_norm.add_forward(x, attn)
         nxt = self.layers[li + 1].attn_norm if li + 1 < len(self.layers) else self.final_norm
-        return nxt.add_forward(h, layer.mlp(h_norm))
+        return nxt.add_forward(h, layer.mlp(h_norm, weights) if weights is not None else layer.mlp(h_norm))
 
     def _decode_step_depth(self, state: DecodeState, x: torch.Tensor, cold_start: ColdStartPolicy,
                            overlap: bool, record: Optional[dict], depth: int) -> torch.Tensor:

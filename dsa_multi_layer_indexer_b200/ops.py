@@ -310,13 +310,13 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
 
 def add_rmsnorm(x: torch.Tensor, delta: torch.Tensor, weight: torch.Tensor, eps: float):
     """``s = x + delta`` and ``rmsnorm(s)`` in one launch (bf16 rows of at most 8192
-    elements, a multiple of 8): returns ``(s, normed)``, both rounded exactly as the
+    elements, a multiple of 8, or fp32 rows): returns ``(s, normed)``, both rounded exactly as the
     separate addition and norm would be."""
     return _host().add_rmsnorm(x, delta, weight, eps)
 
 
 def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
-    """``silu(gate) * up`` over bf16 tensors in one launch, rounded as the two separate operations."""
+    """``silu(gate) * up`` over bf16 or fp32 tensors in one launch, rounded as the two separate operations."""
     return _host().silu_mul(gate, up)
 
 

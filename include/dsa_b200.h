@@ -357,6 +357,14 @@ int dsa_rmsnorm(const void* x, const void* weight, void* out, int64_t rows, int 
  * (a multiple of 8): sum_out = x + delta (rounded to bf16), out = rmsnorm(sum_out). */
 int dsa_add_rmsnorm_bf16(const void* x, const void* delta, const void* weight, void* sum_out, void* out,
                          int64_t rows, int dim, float eps, void* stream);
+/* The same for fp32 rows of any length. */
+int dsa_add_rmsnorm_f32(const float* x, const float* delta, const float* weight, float* sum_out, float* out,
+                        int64_t rows, int dim, float eps, void* stream);
+/* y_i [m, n_i] = x [m, k] w_i^T for up to three fp32 weights [n_i, k] that read the same x (w1, w2 may be
+ * NULL), in one launch; swiglu != 0: y0 = silu(x w0^T) * (x w1^T). The projections and the MLP of a small
+ * fp32 layer (src/lagged_indexer_dsa/dsa_layer.py:87-143, :194-196). k a multiple of 4. */
+int dsa_linear_f32(const float* x, int64_t m, int k, const float* w0, int n0, float* y0, const float* w1,
+                   int n1, float* y1, const float* w2, int n2, float* y2, int swiglu, void* stream);
 /* dst[0, bytes) = src[0, bytes) by a kernel (16-byte pieces; bytes and both pointers
  * multiples of 16). Either side may be pinned host memory: inside a CUDA graph a kernel
  * node starts sooner than a copy-engine node, which matters for the few KB a decode step
@@ -396,6 +404,8 @@ int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k
 /* out = silu(gate) * up over n bf16 elements: the SwiGLU between the MLP's GEMVs
  * (src/lagged_indexer_dsa/dsa_layer.py:194-196), rounded as the two separate operations. */
 int dsa_silu_mul_bf16(const void* gate, const void* up, void* out, int64_t n, void* stream);
+/* The same over fp32. */
+int dsa_silu_mul_f32(const float* gate, const float* up, float* out, int64_t n, void* stream);
 int dsa_decode_prep(const void* iq_raw, const void* w_raw, const void* ik_raw, const void* kv_a,
                     const void* q_abs, const void* q_pe, int64_t q_pe_stride, const void* kv_norm_w,
                     const void* mla_cos, const void* mla_sin, const void* idx_cos, const void* idx_sin,

@@ -1,0 +1,169 @@
+"""GPU tests of the kernels for many short rows (full-sequence layers): the one-CTA-per-row top-k
+against a stable sort, the fp32 scan and the fp32 attention that share keys between heads against
+plain fp32 arithmetic (1e-5: sums of at most a few hundred fp32 products in another order)."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ROWS = 160  # more rows than SMs: the row kernel
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from dsa_multi_layer_indexer_b200 import _lib, ops as _ops
+
+    yield _ops
+    _lib.check_device_status()
+
+
+def expected(x, lens, k, pad):
+    out = torch.full((x.shape[0], k), pad, dtype=torch.int32)
+    for r in range(x.shape[0]):
+        n = min(max(int(lens[r]), 0), x.shape[1])
+        order = torch.sort(x[r, :n], descending=True, stable=True).indices[:k]
+        order = order.sort().values
+        order = torch.where(torch.isinf(x[r, order]) & (x[r, order] < 0), torch.tensor(pad), order)
+        out[r, :order.numel()] = order.int()
+    return out
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (31, 16), (500, 16), (2048, 2048), (2049, 64), (4096, 512), (4099, 2048), (8192, 2048),
+                                 (8193, 2048), (16384, 300)])
+@pytest.mark.parametrize("kind", ["random", "ties", "equal", "inf"])
+def test_row_topk_matches_a_stable_sort(ops, n, k, kind):
+    torch.manual_seed(n + k)
+    x = torch.randn(ROWS, n)
+    if kind == "ties":
+        x = (x * 2).round() / 2
+        x[::2][x[::2] == 0] = -0.0
+    elif kind == "equal":
+        x[:] = 1.25
+    elif kind == "inf":
+        x[torch.rand_like(x) < 0.9] = float("-inf")
+        x[3, : n // 2] = float("inf")
+    lens = torch.randint(0, n + 1, (ROWS,), dtype=torch.int32)
+    lens[0], lens[1], lens[2] = n, 0, n + 5
+    got = ops.topk_select(x.cuda(), k, lens.cuda(), pad_value=-3).cpu()
+    assert torch.equal(got, expected(x, lens, k, -3))
+
+
+def test_row_topk_values_map_offset_and_strided_slab(ops):
+    torch.manual_seed(1)
+    n, k = 700, 64
+    slab = torch.randn(ROWS, n + 9, device="cuda")
+    x = slab[:, :n]
+    idx, val = ops.topk_select(x, k, return_values=True, index_offset=1000)
+    ref = expected(x.cpu(), [n] * ROWS, k, -1)
+    assert torch.equal(idx.cpu(), ref + 1000)
+    assert torch.equal(val, x.gather(1, ref.long().cuda()))
+    m = torch.randint(0, 1 << 20, (ROWS, n), dtype=torch.int32, device="cuda")
+    mapped = ops.topk_select(x, k, index_map=m)
+    assert torch.equal(mapped, m.gather(1, ref.long().cuda()))
+    nan = x.clone()
+    nan[5, 10:] = float("nan")
+    assert ops.topk_select(nan, k)[5].shape == (k,)  # terminates; the other rows are untouched
+    assert torch.equal(ops.topk_select(nan, k)[6].cpu(), ref[6])
+
+
+@pytest.mark.parametrize("rps,n_seq,heads,dim,ctx", [(1, 3, 64, 128, 100), (20, 2, 8, 16, 33), (9, 1, 5, 7, 64), (17, 2, 33, 130, 65),
+                                                     (3, 1, 70, 300, 31)])
+def test_f32_scan_matches_plain_arithmetic(ops, rps, n_seq, heads, dim, ctx):
+    torch.manual_seed(heads + dim)
+    R, cap = rps * n_seq, ctx + 5
+    q, w = torch.randn(R, heads, dim, device="cuda"), torch.randn(R, heads, device="cuda") / 8
+    k = torch.randn(n_seq, cap, dim, device="cuda")
+    lens = torch.randint(0, ctx + 1, (R,), dtype=torch.int32, device="cuda")
+    lens[0] = ctx
+    got = ops.indexer_scan_f32(q, w, k, lens, rows_per_seq=rps, ctx=ctx)
+    kk = k[:, :ctx].double().repeat_interleave(rps, 0)
+    dots = torch.einsum("rhd,rsd->rhs", q.double(), kk).clamp(min=0)
+    ref = (dots * w.double().unsqueeze(-1)).sum(1)
+    dead = torch.arange(ctx, device="cuda")[None, :] >= lens[:, None]
+    assert torch.isneginf(got[dead]).all() and torch.isfinite(got[~dead]).all()
+    scale = float((dots * w.double().abs().unsqueeze(-1)).sum(1).max())
+    assert float((got.double() - ref)[~dead].abs().max()) < 1e-5 * scale
+
+
+@pytest.mark.parametrize("H,qk,v,topk", [(8, 80, 64, 16), (3, 20, 20, 40), (17, 576, 512, 33), (8, 84, 70, None)])
+def test_f32_attention_rows_match_plain_arithmetic(ops, H, qk, v, topk):
+    torch.manual_seed(H + qk)
+    rps, n_seq, ctx = 90, 2, 120
+    R = rps * n_seq
+    q, kv = torch.randn(R, H, qk, device="cuda"), torch.randn(n_seq, ctx, qk, device="cuda")
+    lens = torch.arange(1, rps + 1, dtype=torch.int32, device="cuda").repeat(n_seq)
+    idx = None
+    if topk is not None:
+        idx = torch.stack([torch.randperm(ctx)[:topk] for _ in range(R)]).int().cuda()
+        idx[1] = -1
+    got = ops.sparse_mla_f32(q, kv, idx, v, 0.1, lens, rows_per_seq=rps)
+    keep = torch.zeros(R, ctx, dtype=torch.bool, device="cuda")
+    if idx is None:
+        keep[:] = True
+    else:
+        keep.scatter_(1, idx.clamp(min=0).long(), idx >= 0)
+    keep &= torch.arange(ctx, device="cuda")[None, :] < lens[:, None]
+    kk = kv.double().repeat_interleave(rps, 0)
+    s = torch.einsum("rhd,rsd->rhs", q.double(), kk) * 0.1
+    p = torch.softmax(s.masked_fill(~keep[:, None], float("-inf")), -1).nan_to_num(0.0)
+    ref = torch.einsum("rhs,rsd->rhd", p, kk[..., :v])
+    assert float((got.double() - ref).abs().max()) < 1e-5 * float(ref.abs().max())
+
+
+def test_f32_residual_norm_and_silu(ops):
+    torch.manual_seed(4)
+    x, d, w = torch.randn(5, 300, device="cuda"), torch.randn(5, 300, device="cuda"), torch.randn(300, device="cuda")
+    s, n = ops.add_rmsnorm(x, d, w, 1e-6)
+    assert torch.equal(s, x + d)
+    ref = (x + d).double()
+    ref = ref * torch.rsqrt(ref.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    assert float((n.double() - ref).abs().max()) < 1e-5 * float(ref.abs().max())
+    y = ops.silu_mul(x, d)
+    ref = torch.nn.functional.silu(x.double()) * d.double()
+    assert float((y.double() - ref).abs().max()) < 1e-6 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("m,k,ns", [(1, 4, (1,)), (64, 16, (32, 32, 32)), (65, 20, (33, 1, 70)), (1024, 256, (96, 80, 16)), (7, 300, (5, 9))])
+def test_small_f32_linears_match_fp64(m, k, ns):
+    """dsa_linear_f32 at the edges of its 64 x 32 x 16 tiles; 1e-6 of the row's sum of magnitudes."""
+    from dsa_multi_layer_indexer_b200 import _lib
+
+    torch.manual_seed(m + k)
+    x = torch.randn(m, k, device="cuda")
+    ws = [torch.randn(n, k, device="cuda") for n in ns]
+    ys = [torch.full((m, n), 7.0, device="cuda") for n in ns]
+    args = []
+    for i in range(3):
+        args += [ws[i].data_ptr(), ns[i], ys[i].data_ptr()] if i < len(ns) else [None, 0, None]
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(_lib.lib().dsa_linear_f32(x.data_ptr(), m, k, *args, 0, st))
+    bound = 1e-6 * k
+    for w, y in zip(ws, ys):
+        assert float((y.double() - x.double() @ w.double().T).abs().max()) < bound * 10
+    if len(ns) == 1 or ns[0] == ns[1]:
+        up = torch.randn(ns[0], k, device="cuda")
+        _lib.check(_lib.lib().dsa_linear_f32(x.data_ptr(), m, k, ws[0].data_ptr(), ns[0], ys[0].data_ptr(), up.data_ptr(), ns[0], None,
+                                             None, 0, None, 1, st))
+        g, u = x.double() @ ws[0].double().T, x.double() @ up.double().T
+        ref = torch.nn.functional.silu(g) * u
+        assert float((ys[0].double() - ref).abs().max()) < bound * 10 * max(1.0, float(u.abs().max()))
+
+
+def test_hooked_or_replaced_projections_keep_the_module_path():
+    import dsa_multi_layer_indexer_b200 as D
+
+    torch.manual_seed(9)
+    model = D.DSAModel(D.named_config("small")).eval().cuda()
+    x = torch.randn(1, 40, 256, device="cuda")
+    mode, cold = D.ScheduleMode.LAGGED_FUSED, D.ColdStartPolicy.EAGER
+    seen = []
+    with torch.no_grad():
+        plain = model(x, mode, cold)
+        handle = model.layers[2].gate_proj.register_forward_hook(lambda m, a, o: seen.append(o.shape))
+        hooked = model(x, mode, cold)
+        handle.remove()
+    assert seen == [torch.Size([1, 40, 512])]
+    assert float((plain - hooked).abs().max()) < 1e-4 * float(plain.abs().max())
