@@ -918,12 +918,13 @@ int dsa_sparse_mla_combine(const float* part_acc, const float* part_m, const flo
   DSA_REQUIRE(part_acc && part_m && part_l && out, "sparse MLA combine: null pointer");
   DSA_REQUIRE(aligned16(part_acc) && aligned16(out), "sparse MLA combine: misaligned pointer");
   DSA_REQUIRE(R > 0 && R <= 65535 && H > 0 && nsplit > 0, "sparse MLA combine: bad geometry");
-  if (nsplit <= mla::kFlatMaxSplit && int64_t(R) * H >= 512) {
-    // many (row, head) pairs, few splits: one thread per four output columns
-    const int64_t n_pairs = int64_t(R) * H;
-    DSA_CUDA(launch_pdl(mla::sparse_mla_combine_flat_kernel, dim3(unsigned((n_pairs * 128 + 255) / 256)), dim3(256),
-                        0, static_cast<cudaStream_t>(stream), part_acc, part_m, part_l,
-                        static_cast<__nv_bfloat16*>(out), H, nsplit, n_pairs));
+  if (int64_t(R) * H > sm_count() && (nsplit <= 16 || int64_t(R) * H >= 512)) {
+    // more (row, head) pairs than SMs: a small CTA per pair, one thread per four output columns
+    // (192 pairs x 24 splits: 15.6 us for the pair of launches against 16.5 this way)
+    // (partials + merge, 256 pairs x 16 splits: 12.8 us with 8 loads in flight, 13.7 with 16; 512 pairs: 15.3 / 14.9)
+    auto kernel = nsplit > 8 && int64_t(R) * H >= 512 ? mla::sparse_mla_combine_flat_kernel<16> : mla::sparse_mla_combine_flat_kernel<8>;
+    DSA_CUDA(launch_pdl(kernel, dim3(unsigned(int64_t(R) * H)), dim3(128), 0, static_cast<cudaStream_t>(stream), part_acc, part_m,
+                        part_l, static_cast<__nv_bfloat16*>(out), H, nsplit));
     return DSA_OK;
   }
   // one load group of 128 threads per split, up to four

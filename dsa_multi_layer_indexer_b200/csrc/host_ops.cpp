@@ -339,12 +339,13 @@ int64_t default_nsplit(int64_t rows, int64_t heads, int64_t k, int64_t sms) {
   const int64_t tiles = std::max<int64_t>(1, (k + 63) / 64);
   if (heads % 64 == 0 && rows * (heads / 64) * tiles >= 128) {
     const int64_t blocks = std::max<int64_t>(1, rows * (heads / 64));
-    int64_t want = std::max<int64_t>(1, std::min(sms / blocks, tiles));
+    int64_t want = std::max<int64_t>(1, std::min(std::min<int64_t>(sms / blocks, 16), tiles));
     while (tiles % want) --want;
     return want;
   }
   const int64_t blocks = std::max<int64_t>(1, rows * (heads / 16));
-  const int64_t want = std::max<int64_t>(1, 2 * sms / blocks);
+  int64_t want = std::max<int64_t>(1, 2 * sms / blocks);
+  if (rows * heads > sms) want = std::min<int64_t>(want, 16);
   return std::max<int64_t>(1, std::min(want, tiles));
 }
 

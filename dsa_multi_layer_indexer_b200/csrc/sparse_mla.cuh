@@ -567,56 +567,64 @@ sparse_mla_combine_kernel(const float* __restrict__ part_acc, const float* __res
   DSA_KTIME_END(3);
 }
 
-// The same merge for many (row, head) pairs with at most eight splits each (large
-// batches): one thread per four output columns, every load of a thread in flight
-// at once, no shared memory. Splits are folded in ascending order.
-constexpr int kFlatMaxSplit = 8;
-__global__ void __launch_bounds__(256)
+// The same merge for many (row, head) pairs: one thread per four output columns, kUnroll splits' loads
+// in flight at once, no shared memory; splits are folded in ascending order, kUnroll at a time. L2-bound:
+// 16.8 MB of partials (512 pairs x 16 splits) in 3.3 us, where a CTA per pair with its loads spread over
+// four thread groups takes 8.0.
+template <int kUnroll>
+__global__ void __launch_bounds__(128)
 sparse_mla_combine_flat_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_m,
                                const float* __restrict__ part_l, __nv_bfloat16* __restrict__ out, int H,
-                               int nsplit, int64_t n_pairs) {
+                               int nsplit) {
   DSA_KTIME_BEGIN(3);
   pdl_wait();
   pdl_launch_dependents();
-  const int64_t gid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t pair = gid >> 7;  // row * H + head
-  const int c4 = int(gid & 127);
-  if (pair < n_pairs) {
-    const int64_t r = pair / H, h = pair % H;
-    float ms[kFlatMaxSplit], ls[kFlatMaxSplit];
-    float4 a[kFlatMaxSplit];
+  const int64_t pair = blockIdx.x;  // row * H + head
+  const int64_t r = pair / H, h = pair % H;
+  const int c4 = threadIdx.x;
+  float m = -INFINITY, l = 0.f;
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = 0; s0 < nsplit; s0 += kUnroll) {
+    float ms[kUnroll], ls[kUnroll];
+    float4 a[kUnroll];
 #pragma unroll
-    for (int u = 0; u < kFlatMaxSplit; ++u) {
-      const bool ok = u < nsplit;
-      const int64_t row = (r * nsplit + u) * H + h;
+    for (int u = 0; u < kUnroll; ++u) {
+      const bool ok = s0 + u < nsplit;
+      const int64_t row = (r * nsplit + s0 + u) * H + h;
       ms[u] = ok ? part_m[row] : -INFINITY;
       ls[u] = ok ? part_l[row] : 0.f;
       a[u] = ok ? *reinterpret_cast<const float4*>(part_acc + row * kDV + c4 * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float m = ms[0];
+    float m_new = m;
 #pragma unroll
-    for (int u = 1; u < kFlatMaxSplit; ++u) m = fmaxf(m, ms[u]);
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    float l = 0.f;
-    if (m != -INFINITY) {
-#pragma unroll
-      for (int u = 0; u < kFlatMaxSplit; ++u) {
-        const float e = (ms[u] == -INFINITY) ? 0.f : exp2f(ms[u] - m);
-        l = fmaf(ls[u], e, l);
-        o.x = fmaf(a[u].x, e, o.x);
-        o.y = fmaf(a[u].y, e, o.y);
-        o.z = fmaf(a[u].z, e, o.z);
-        o.w = fmaf(a[u].w, e, o.w);
-      }
+    for (int u = 0; u < kUnroll; ++u) m_new = fmaxf(m_new, ms[u]);
+    if (m_new == -INFINITY) continue;
+    if (s0 > 0) {
+      const float keep = (m == -INFINITY) ? 0.f : exp2f(m - m_new);
+      l *= keep;
+      o.x *= keep;
+      o.y *= keep;
+      o.z *= keep;
+      o.w *= keep;
     }
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-    __nv_bfloat162 lo = __floats2bfloat162_rn(o.x * inv, o.y * inv);
-    __nv_bfloat162 hi = __floats2bfloat162_rn(o.z * inv, o.w * inv);
-    uint2 pk;
-    pk.x = *reinterpret_cast<uint32_t*>(&lo);
-    pk.y = *reinterpret_cast<uint32_t*>(&hi);
-    *reinterpret_cast<uint2*>(out + pair * kDV + c4 * 4) = pk;
+    m = m_new;
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const float e = (ms[u] == -INFINITY) ? 0.f : exp2f(ms[u] - m);
+      l = fmaf(ls[u], e, l);
+      o.x = fmaf(a[u].x, e, o.x);
+      o.y = fmaf(a[u].y, e, o.y);
+      o.z = fmaf(a[u].z, e, o.z);
+      o.w = fmaf(a[u].w, e, o.w);
+    }
   }
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+  __nv_bfloat162 lo = __floats2bfloat162_rn(o.x * inv, o.y * inv);
+  __nv_bfloat162 hi = __floats2bfloat162_rn(o.z * inv, o.w * inv);
+  uint2 pk;
+  pk.x = *reinterpret_cast<uint32_t*>(&lo);
+  pk.y = *reinterpret_cast<uint32_t*>(&hi);
+  *reinterpret_cast<uint2*>(out + pair * kDV + c4 * 4) = pk;
   DSA_KTIME_END(3);
 }
 
