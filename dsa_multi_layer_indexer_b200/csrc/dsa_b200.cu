@@ -492,11 +492,22 @@ static int launch_topk_rows(const topk::Params& p, int R, int64_t n, cudaStream_
   return DSA_OK;
 }
 
+// Rows of up to kSoloMaxN logits with the scan's histogram, indices only: one CTA per row, the row in registers.
+extern "C++" {
+template <bool kPages>
+static int launch_topk_solo(const topk::Params& p, int R, int64_t n, cudaStream_t st) {
+  if (n <= 2048) DSA_CUDA(launch_pdl(topk::topk_solo_kernel<4, kPages>, dim3(R), dim3(topk::kClThreads), 0, st, p));
+  else DSA_CUDA(launch_pdl(topk::topk_solo_kernel<8, kPages>, dim3(R), dim3(topk::kClThreads), 0, st, p));
+  return DSA_OK;
+}
+}  // extern "C++"
+
 static int launch_topk_cluster(const topk::Params& p, int R, int64_t n, cudaStream_t st) {
   // More rows than SMs: the cluster kernel holds one row per SM and would take several waves of its
   // latency-bound chain, the row kernel keeps several rows per SM in flight.
   if (!p.hist && !p.n_src && !p.n_dest && R > sm_count() && n <= topk::kRowsMaxN) return launch_topk_rows(p, R, n, st);
   const bool plain = p.hist && !p.n_src && !p.n_dest && !p.index_map && !p.out_val;
+  if (plain && n <= topk::kSoloMaxN) return p.page_table ? launch_topk_solo<true>(p, R, n, st) : launch_topk_solo<false>(p, R, n, st);
   // As few CTAs as hold the row at 32 logits per thread: every CTA added costs cluster barriers and
   // remote stores, and a row of up to 16384 logits needs none of either.
   // A row that comes without the scan's histogram counts its own first level with shared-memory

@@ -152,5 +152,166 @@ topk_rows_kernel(const Params p) {
   }
 }
 
+// ------------------------------------------------------------------------------
+// One row of up to kSoloMaxN logits that comes with the scan's histogram (a decode step at a short
+// context): one CTA of 512 threads with the row in registers. The cluster kernel's way for such a row is a
+// chain of phases laid out for 32 logits per thread and eight CTAs; here
+//   threshold bin from the histogram -> candidates of that bin counted by their next 7 key bits -> the
+//   second bin -> the few candidates in it ("survivors") ranked by comparison (key descending, position
+//   ascending) -> one pass of warp votes in position order gives each kept element its slot,
+// and candidates never leave their owner. More than kSoloSurv survivors (many equal logits): two more
+// counting rounds down to the k-th key, ties resolved in position order in the last pass.
+// Latency-bound: about a dozen dependent steps, and the unrolled code itself. scan + top-k of 4096 logits,
+// k = 2048: 9.3 -> 7.3 us; with 16 elements per thread (8192 logits) it is no faster than the cluster
+// kernel for one row and slower for eight (15.3 against 13.0 us), with 32 slower for one; the same kernel
+// with its elements in shared memory and rolled loops: 8.0 us at 4096, 14.8 at 16384. Hence the limit.
+constexpr int kSoloSurv = 256;
+constexpr int64_t kSoloMaxN = 4096;
+template <int ITEMS, bool kPages>
+__global__ void __launch_bounds__(kClThreads)
+topk_solo_kernel(const Params p) {
+  __shared__ uint32_t s_warp[kClWarps];
+  __shared__ uint32_t s_res[4];
+  __shared__ __align__(16) uint32_t s_h2[kL2Bins];
+  __shared__ uint32_t s_mask[kClWarps * ITEMS];  // survivors that are kept, word (warp, i), bit lane
+  __shared__ uint64_t s_surv[kSoloSurv];
+  __shared__ uint32_t s_nsurv;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t r = blockIdx.x;
+  for (int i = tid; i < kClWarps * ITEMS; i += kClThreads) s_mask[i] = 0u;
+  if (tid < kL2Bins) s_h2[tid] = 0u;
+  if (tid == 0) s_nsurv = 0u;
+  DSA_KTIME_BEGIN(1);
+  pdl_launch_dependents();  // (before the wait, as the cluster kernel does: see there)
+  pdl_wait();
+  const float* row = p.logits + r * p.slab_stride;
+  const int base = warp * (32 * ITEMS) + lane;   // element i of this thread is position base + 32 i
+  const int n = int(p.n);
+  uint32_t key[ITEMS];
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) key[i] = base + 32 * i < n ? __float_as_uint(__ldcg(row + base + 32 * i)) : 0xFFFFFFFFu;
+  uint4* gh = reinterpret_cast<uint4*>(p.hist + size_t(r) * kBins + (kBins - 8 * (tid + 1)));
+  const uint4 h1a = __ldcg(gh), h1b = __ldcg(gh + 1);
+  int64_t len64 = p.seq_lens ? int64_t(p.seq_lens[r]) : p.n;
+  const int len = int(len64 < 0 ? 0 : (len64 > p.n ? p.n : len64));
+  int32_t page[ITEMS / 2];                       // kPages: one table entry per two groups of 32 positions
+  if constexpr (kPages) {
+#pragma unroll
+    for (int i = 0; i < ITEMS / 2; ++i) {
+      const int first = warp * (32 * ITEMS) + 64 * i;
+      page[i] = first < n ? p.page_table[r * p.pt_stride + (first >> 6)] : 0;
+    }
+  }
+  // ordered keys; 0 (below every number) past the row's length
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) key[i] = base + 32 * i < len ? ordered_key(__uint_as_float(key[i])) : 0u;
+  gh[0] = make_uint4(0, 0, 0, 0);                // re-armed: every thread clears the bins that it has read
+  gh[1] = make_uint4(0, 0, 0, 0);
+
+  uint32_t kept = 0;                             // bit i: key[i] is certainly kept
+  uint32_t kstar = 0xFFFFFFFFu, ties_kept = 0;
+  bool pad_inf = true;                           // a kept -inf can only appear when the row has fewer than k finite logits
+  if (len <= p.topk) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+      if (base + 32 * i < len) kept |= 1u << i;
+    __syncthreads();
+  } else {
+    const uint32_t cnt8[8] = {h1b.w, h1b.z, h1b.y, h1b.x, h1a.w, h1a.z, h1a.y, h1a.x};  // highest bin first
+    find_kth_in_registers<kBins, 8>(cnt8, uint32_t(p.topk), s_warp, s_res);
+    const uint32_t T = s_res[0], need = s_res[1];
+    uint32_t cand = 0;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const uint32_t bin = key[i] >> kLowBits;
+      if (key[i] != 0u && bin > T) kept |= 1u << i;
+      if (key[i] != 0u && bin == T) {
+        cand |= 1u << i;
+        smem_red_add(&s_h2[(key[i] >> kL3Bits) & (kL2Bins - 1)], 1u);
+      }
+    }
+    __syncthreads();
+    find_kth_bin_warp<kL2Bins>(s_h2, need, s_res);
+    const uint32_t p19 = (T << kL2Bits) | s_res[0], need2 = s_res[1];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      if ((cand >> i) & 1u) {
+        const uint32_t k19 = key[i] >> kL3Bits;
+        if (k19 > p19) kept |= 1u << i;
+        if (k19 == p19) {
+          const uint32_t at = atomicAdd(&s_nsurv, 1u);
+          if (at < uint32_t(kSoloSurv)) s_surv[at] = (uint64_t(key[i]) << 32) | uint32_t(~uint32_t(base + 32 * i));
+        }
+      }
+    }
+    __syncthreads();
+    const uint32_t n_surv = s_nsurv;
+    if (n_surv <= uint32_t(kSoloSurv)) {
+      if (uint32_t(tid) < n_surv) {
+        const uint64_t mine = s_surv[tid];       // larger = earlier
+        uint32_t before = 0;
+        for (uint32_t j = 0; j < n_surv; ++j) before += uint32_t(s_surv[j] > mine);
+        const uint32_t pos = ~uint32_t(mine);
+        if (before < need2) atomicOr(&s_mask[pos >> 5], 1u << (pos & 31u));
+        if (before + 1u == need2) s_res[3] = uint32_t(mine >> 32);
+      }
+      __syncthreads();
+      pad_inf = s_res[3] <= 0x007FFFFFu;
+    } else {                                     // many equal logits: down to the k-th key itself
+      uint32_t prefix = p19, left = need2;
+#pragma unroll 1
+      for (int shift = 6; shift >= 0; shift -= 6) {  // 7 bits, then 6
+        const int bits = shift == 6 ? 7 : 6;
+        if (tid < kL2Bins) s_h2[tid] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i)
+          hist_add_warp(s_h2, ((cand >> i) & 1u) && (key[i] >> (shift + bits)) == prefix, (key[i] >> shift) & ((1u << bits) - 1u));
+        __syncthreads();
+        find_kth_bin_warp<kL2Bins>(s_h2, left, s_res);
+        prefix = (prefix << bits) | s_res[0];
+        left = s_res[1];
+      }
+      kstar = prefix;
+      ties_kept = left;
+      pad_inf = kstar <= 0x007FFFFFu;
+#pragma unroll
+      for (int i = 0; i < ITEMS; ++i)
+        if (((cand >> i) & 1u) && key[i] > kstar) kept |= 1u << i;
+    }
+  }
+  // ---- totals of the warps' shares, then the slots in position order
+  uint32_t cnt = uint32_t(__popc(kept));
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) cnt += (key[i] == kstar ? 0x10000u : 0u);
+  if (lane < ITEMS) cnt += uint32_t(__popc(s_mask[warp * ITEMS + lane]));
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if (lane == 0) s_warp[warp] = cnt;
+  __syncthreads();
+  const uint32_t wt = lane < kClWarps ? s_warp[lane] : 0u;
+  const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u), all = __reduce_add_sync(0xffffffffu, wt);
+  uint32_t g = before & 0xFFFFu, q = before >> 16;
+  const uint32_t below = (1u << lane) - 1u;
+  int32_t* out_idx = p.out_idx + r * p.topk;
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const uint32_t gm = __ballot_sync(0xffffffffu, (kept >> i) & 1u) | s_mask[warp * ITEMS + i];
+    const uint32_t qm = ties_kept ? __ballot_sync(0xffffffffu, key[i] == kstar) : 0u;
+    const uint32_t gb = g + __popc(gm & below), qb = q + __popc(qm & below);
+    const bool is_g = (gm >> lane) & 1u, is_q = ((qm >> lane) & 1u) && qb < ties_kept;
+    if (is_g || is_q) {
+      const int pos = base + 32 * i;
+      int32_t id = pos + p.index_offset;
+      if constexpr (kPages) id = page[i >> 1] * DSA_PAGE_TOKENS + (pos & (DSA_PAGE_TOKENS - 1));
+      if (pad_inf && key[i] == 0x007FFFFFu) id = p.pad;
+      out_idx[is_g ? gb + min(qb, ties_kept) : gb + qb] = id;
+    }
+    g += __popc(gm);
+    q += __popc(qm);
+  }
+  for (uint32_t i = (all & 0xFFFFu) + min(all >> 16, ties_kept) + tid; i < uint32_t(p.topk); i += kClThreads) out_idx[i] = p.pad;
+  DSA_KTIME_END(1);
+}
+
 }  // namespace topk
 }  // namespace dsa

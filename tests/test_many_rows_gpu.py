@@ -167,3 +167,41 @@ def test_hooked_or_replaced_projections_keep_the_module_path():
         handle.remove()
     assert seen == [torch.Size([1, 40, 512])]
     assert float((plain - hooked).abs().max()) < 1e-4 * float(plain.abs().max())
+
+
+def scan_histogram(x, lens):
+    """What the scan leaves for the top-k: counts of the top 12 bits of the order-preserving key."""
+    bits = (x + 0.0).view(torch.int32)
+    key = torch.where(bits < 0, ~bits, bits ^ -(1 << 31)).long() & 0xFFFFFFFF
+    hist = torch.zeros(x.shape[0], 4096, dtype=torch.int32)
+    for r in range(x.shape[0]):
+        n = min(max(int(lens[r]), 0), x.shape[1])
+        hist[r] = torch.bincount(key[r, :n] >> 20, minlength=4096).int()
+    return hist
+
+
+@pytest.mark.parametrize("n,k", [(1, 4), (60, 16), (2048, 512), (2049, 2048), (4096, 2048), (4097, 64), (8192, 2048), (8193, 2048),
+                                 (16384, 2048)])
+@pytest.mark.parametrize("kind", ["random", "ties", "equal", "inf", "close"])
+def test_solo_topk_with_the_scans_histogram(ops, n, k, kind):
+    """Rows with a histogram (up to 4096 logits: register kernel), at the edges of its sizes, with
+    more equal logits than it ranks by comparison, and with logits that share their top 19 bits."""
+    torch.manual_seed(n + k)
+    rows = 5
+    x = torch.randn(rows, n)
+    if kind == "ties":
+        x = (x * 2).round() / 2
+        x[::2][x[::2] == 0] = -0.0
+    elif kind == "equal":
+        x[:] = -2.5
+    elif kind == "inf":
+        x[torch.rand_like(x) < 0.9] = float("-inf")
+        x[3, : n // 2] = float("inf")
+    elif kind == "close":
+        x = 1.0 + torch.randint(0, 1 << 9, (rows, n)) * 2.0 ** -23
+    lens = torch.tensor([n, 0, n + 5, max(1, n - 3), n // 2], dtype=torch.int32)
+    hist = scan_histogram(x, lens).cuda()
+    got = ops.topk_select(x.cuda(), k, lens.cuda(), hist=hist, pad_value=-3, index_offset=7).cpu()
+    ref = expected(x, lens, k, -10)
+    assert torch.equal(got, torch.where(ref == -10, torch.tensor(-3, dtype=torch.int32), ref + 7))
+    assert int(hist.abs().sum()) == 0  # re-armed for the next scan
