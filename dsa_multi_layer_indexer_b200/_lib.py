@@ -58,6 +58,9 @@ SIGNATURES: Dict[str, Tuple[object, List[object]]] = {
     "dsa_silu_mul_f32": (_i, [_p, _p, _p, _l, _p]),
     "dsa_silu_mul_bf16": (_i, [_p, _p, _p, _l, _p]),
     "dsa_gemv_bf16": (_i, [_p, _p, _p, _i, _i, _i, _l, _l, _p]),
+    "dsa_gemv_swiglu_bf16": (_i, [_p, _p, _p, _p, _i, _i, _i, _l, _l, _p]),
+    "dsa_absorb_query": (_i, [_p, _p, _p, _i, _i, _i, _i, _l, _l, _p]),
+    "dsa_value_project": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _p]),
     "dsa_copy_bytes": (_i, [_p, _p, _l, _p]),
     "dsa_copy_bytes_beside": (_i, [_p, _p, _l, _p]),
     "dsa_post_epoch": (_i, [_p, _p, _p]),

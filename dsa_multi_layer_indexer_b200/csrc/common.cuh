@@ -51,6 +51,7 @@ constexpr unsigned int kStatusScanTimeout = DSA_STATUS_SCAN_TIMEOUT;
 constexpr unsigned int kStatusAttnTimeout = DSA_STATUS_ATTN_TIMEOUT;
 constexpr unsigned int kStatusSelectOverflow = DSA_STATUS_SELECT_OVERFLOW;
 constexpr unsigned int kStatusBadPage = DSA_STATUS_BAD_PAGE;  // a page-table entry outside [0, num_pages): the access was skipped
+constexpr unsigned int kStatusGemvTimeout = DSA_STATUS_GEMV_TIMEOUT;
 constexpr unsigned int kStatusExchangeTimeout = DSA_STATUS_EXCHANGE_TIMEOUT;  // a peer's candidates did not arrive in time
 
 #ifdef __CUDACC__

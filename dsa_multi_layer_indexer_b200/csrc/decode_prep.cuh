@@ -260,20 +260,169 @@ copy_post_epoch_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, i
 }
 
 // ------------------------------------------------------------------ skinny GEMV
-// y[b, n] = sum_k W[n, k] x[b, k] for 1..4 rows of x (decode batch): bf16 operands,
-// fp32 accumulation, one rounding. The weight matrix is streamed once with 16-byte
-// loads, eight per lane in flight, x staged in shared memory. This is the
-// projection GEMV of a decode step (src/lagged_indexer_dsa/dsa_layer.py:87-125) for
-// the shapes where the library GEMV is latency-bound (a few thousand output rows).
+// y[b, n] = sum_k W[n, k] x[b, k] for 1..4 rows of x (decode batch): bf16 operands, fp32 accumulation, one
+// rounding; as kSwiglu the MLP's product silu(W x) * (W2 x) with the roundings of its separate operations
+// (src/lagged_indexer_dsa/dsa_layer.py:87-143, :194-196).
+//
+// One or two rows of x (every decode step of a small batch). HBM-bound: the weights are streamed once, so
+// they are moved by the copy engine. A CTA per SM owns an even share of the rows, taken in pairs (for SwiGLU
+// the two matrices' rows of one output), so that x is read from shared memory and unpacked once for two
+// rows. Each of its sixteen warps keeps its own ring of two to four bulk copies of 2 x 2 KB and refills a slot as
+// soon as it has read it: no barrier between warps, no register holding a load in flight. A warp's pieces
+// are consecutive, its sum stays in registers until the pair changes, and the warps' sums of a pair are
+// folded in order at the end (a pair can span warps: the parts of a row are dealt out evenly).
+// The rings are filled BEFORE the dependency wait, which hides the launch and the latency of the kernel in
+// front: no kernel of this library writes weights, and any other kernel in front completes before its
+// successor starts.
+// One row of x, [2240, 7168] 13.0 -> 7.5 us, [32832, 1536] 18.5 -> 17.5 us (kernel below); against the
+// library's GEMV [7168, 16384] 39.7 -> 37.0 us (6.35 TB/s), [7168, 18432] 42.8 -> 41.2, SwiGLU 2 x [18432,
+// 7168] 41.3 + 41.3 + product -> 79.6. 96 KB in flight instead of 144 make [32832, 1536] 27 us behind another
+// kernel; eight warps 21.6 alone; pieces of 2 x 1 KB: [18432, 7168] 50.9 against 41.1; one producer warp for
+// the CTA's ring: 300 ns a copy, 3.5 TB/s; weights through registers: 4.2 - 5.7 TB/s. A ring of 200 KB keeps
+// the next kernel's CTA out and costs 1 % of a decode step.
 constexpr int kGemvThreads = 256;
-constexpr int kGemvLoads = 8;  // independent 16-byte weight loads per lane per step
-// R rows per warp, kGemvLoads / R consecutive 512-byte column blocks per step: the
-// launch picks R so that there are enough warps to fill the machine.
-template <int B, int R>
+constexpr int kGemvLoads = 8;        // gemv_rows_kernel: independent 16-byte weight loads per lane
+constexpr int kGemvChunks = 128;  // 16-byte chunks of a row in one piece, at most
+constexpr int kGemvWarps = 16;
+constexpr int kGemvMaxSlots = 4;     // pieces in flight per warp
+constexpr int kGemvRing = 160 << 10;  // bytes in flight per CTA, at most (and at least two pieces per warp)
+struct GemvParams {
+  const __nv_bfloat16* w;
+  const __nv_bfloat16* w2;
+  const __nv_bfloat16* x;
+  __nv_bfloat16* y;
+  int n, k, slots, ks, chunks;  // ks pieces of up to `chunks` 16-byte chunks per row
+  int64_t x_stride, y_stride;
+};
+// shared memory: ring [warps][slots][2][chunks] | x [B][k] | sums [units of a CTA][ks][2][B]
+template <int B, bool kSwiglu>
+__global__ void __launch_bounds__(kGemvWarps * 32, 1)
+gemv_stream_kernel(const GemvParams p) {
+  extern __shared__ __align__(128) uint8_t gemv_smem[];
+  __shared__ uint64_t s_full[kGemvWarps * kGemvMaxSlots];
+  __shared__ int s_abort;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int kv = p.k >> 3, ks = p.ks, pl = p.chunks, slots = p.slots;
+  // unit u: rows 2u, 2u + 1 of w, or row u of w and of w2; piece j of the CTA: part j % ks of unit j / ks
+  const int total = kSwiglu ? p.n : (p.n + 1) >> 1;
+  const int u0 = int(int64_t(total) * blockIdx.x / gridDim.x), nu = int(int64_t(total) * (blockIdx.x + 1) / gridDim.x) - u0;
+  const int p0 = nu * ks * warp / kGemvWarps, p1 = nu * ks * (warp + 1) / kGemvWarps;
+  uint4* ring = reinterpret_cast<uint4*>(gemv_smem) + warp * slots * 2 * pl;
+  uint4* s_x = reinterpret_cast<uint4*>(gemv_smem) + kGemvWarps * slots * 2 * pl;
+  float* s_sum = reinterpret_cast<float*>(s_x + B * kv);
+  uint64_t* full = s_full + warp * kGemvMaxSlots;
+  int unit = p0 / ks, part = p0 - unit * ks;  // of the piece that is consumed
+  int iu = unit, ip = part;                   // of the piece that is issued (lane 0)
+  const auto issue = [&](int slot) {
+    const int c0 = ip * pl, len = min(pl, kv - c0);
+    const int u = u0 + iu;
+    const __nv_bfloat16* r0 = p.w + int64_t(kSwiglu ? u : 2 * u) * p.k + c0 * 8;
+    const __nv_bfloat16* r1 = kSwiglu ? p.w2 + int64_t(u) * p.k + c0 * 8 : (2 * u + 1 < p.n ? r0 + p.k : r0);
+    const uint32_t bar = smem_u32(&full[slot]), dst = smem_u32(ring + slot * 2 * pl), bytes = uint32_t(len) * 16u;
+    mbar_arrive_expect_tx(bar, 2u * bytes);
+    bulk_g2s(dst, r0, bytes, bar);
+    bulk_g2s(dst + uint32_t(pl) * 16u, r1, bytes, bar);
+    if (++ip == ks) ip = 0, ++iu;
+  };
+  if (lane == 0) {
+    for (int i = 0; i < slots; ++i) mbar_init(smem_u32(&full[i]), 1);
+    mbar_fence_init();
+    for (int i = 0; i < slots && p0 + i < p1; ++i) issue(i);
+  }
+  if (tid == 0) s_abort = 0;
+  for (int i = tid; i < nu * ks * 2 * B; i += kGemvWarps * 32) s_sum[i] = 0.f;
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int b = 0; b < B; ++b)
+    for (int c = tid; c < kv; c += kGemvWarps * 32) s_x[b * kv + c] = *reinterpret_cast<const uint4*>(p.x + b * p.x_stride + c * 8);
+  __syncthreads();
+  float acc[2][B];
+#pragma unroll
+  for (int b = 0; b < B; ++b) acc[0][b] = acc[1][b] = 0.f;
+  int slot = 0;
+  uint32_t phase = 0;
+  for (int j = p0; j < p1; ++j) {
+    if (__any_sync(0xffffffffu, !mbar_wait(smem_u32(&full[slot]), phase))) {
+      s_abort = 1;
+      break;
+    }
+    const int c0 = part * pl, len = min(pl, kv - c0);
+    const uint4* wr = ring + slot * 2 * pl;
+    uint4 wv[2][4], xv[B][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int c = lane + 32 * i;
+      const bool in = c < len;
+      wv[0][i] = in ? wr[c] : make_uint4(0, 0, 0, 0);
+      wv[1][i] = in ? wr[pl + c] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int b = 0; b < B; ++b) xv[b][i] = in ? s_x[b * kv + c0 + c] : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int b = 0; b < B; ++b) {
+        const uint32_t xw[4] = {xv[b][i].x, xv[b][i].y, xv[b][i].z, xv[b][i].w};
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const uint32_t cw[4] = {wv[m][i].x, wv[m][i].y, wv[m][i].z, wv[m][i].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            acc[m][b] = fmaf(__uint_as_float(cw[e] << 16), __uint_as_float(xw[e] << 16), acc[m][b]);
+            acc[m][b] = fmaf(__uint_as_float(cw[e] & 0xFFFF0000u), __uint_as_float(xw[e] & 0xFFFF0000u), acc[m][b]);
+          }
+        }
+      }
+    }
+    __syncwarp();
+    if (lane == 0 && j + slots < p1) issue(slot);  // the same warp has read the slot: no barrier to wait for
+    if (++slot == slots) slot = 0, phase ^= 1;
+    const bool last = part == ks - 1 || j == p1 - 1;
+    if (last) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+          float v = acc[m][b];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (lane == 0) s_sum[((unit * ks + part) * 2 + m) * B + b] = v;
+          acc[m][b] = 0.f;
+        }
+    }
+    if (++part == ks) part = 0, ++unit;
+  }
+  __syncthreads();
+  if (s_abort) {
+    if (tid == 0) atomicOr(&g_device_status, kStatusGemvTimeout);
+    drain_after_timeout();  // let outstanding copies land
+  }
+  // the sums of a unit's parts (most are zero: a warp leaves one per unit that it met), in order
+  constexpr int kOut = kSwiglu ? 1 : 2;
+  for (int i = tid; i < nu * kOut * B; i += kGemvWarps * 32) {
+    const int u = i / (kOut * B), m0 = kSwiglu ? 0 : (i / B) % 2, b = i % B;
+    float v = 0.f, v2 = 0.f;
+    for (int q = 0; q < ks; ++q) {
+      v += s_sum[((u * ks + q) * 2 + m0) * B + b];
+      if (kSwiglu) v2 += s_sum[((u * ks + q) * 2 + 1) * B + b];
+    }
+    __nv_bfloat16 out = __float2bfloat16_rn(v);
+    const int row = kSwiglu ? u0 + u : 2 * (u0 + u) + m0;
+    if constexpr (kSwiglu) {
+      const float g = __bfloat162float(out), up = __bfloat162float(__float2bfloat16_rn(v2));
+      out = __float2bfloat16_rn(__bfloat162float(__float2bfloat16_rn(g / (1.f + __expf(-g)))) * up);
+    }
+    if (row < p.n) p.y[b * p.y_stride + row] = out;
+  }
+}
+
+// Three or four rows of x, and short rows of W: x staged in shared memory, one
+// row of W per warp with eight loads per lane in flight.
+template <int B>
 __global__ void __launch_bounds__(kGemvThreads)
-gemv_bf16_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ x,
+gemv_rows_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ x,
                  __nv_bfloat16* __restrict__ y, int n, int k, int64_t x_stride, int64_t y_stride) {
-  constexpr int UK = kGemvLoads / R;
+  constexpr int R = 1, UK = kGemvLoads;
   extern __shared__ __align__(16) uint8_t gemv_smem[];
   uint4* s_x = reinterpret_cast<uint4*>(gemv_smem);  // [B][k / 8]
   const int kv = k >> 3;
@@ -333,6 +482,111 @@ gemv_bf16_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __res
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane == 0 && row0 + r < n) y[b * y_stride + row0 + r] = __float2bfloat16_rn(v);
       }
+  }
+}
+
+// ------------------------------------------------------------------ per-head products of a decode row
+// The two absorbed projections of a decode step over kv_b_proj's weight [H, nope + v, 512]
+// (src/lagged_indexer_dsa/dsa_layer.py:96-125): q_abs[h] = q_nope[h] W_UK[h] into the first 512 columns of
+// q_full, and ov[h] = W_UV[h] o[h]. One token's 33 MB of weights are streamed once; as in the GEMV above the
+// first loads go out before the dependency wait. One CTA per (head, batch row).
+constexpr int kHeadThreads = 256;
+__global__ void __launch_bounds__(kHeadThreads)
+absorb_query_kernel(const __nv_bfloat16* __restrict__ kv_b, const __nv_bfloat16* q, __nv_bfloat16* __restrict__ q_full,
+                    int H, int nope, int per_head, int64_t q_row_stride, int64_t q_head_stride) {
+  // 64 column vectors of 8 x 4 groups of rows: thread (g, c) sums rows g, g + 4, ... of its eight columns
+  __shared__ float s_q[512];
+  __shared__ __align__(16) float s_o[4][512];
+  const int h = blockIdx.x, b = blockIdx.y, c = threadIdx.x & 63, g = threadIdx.x >> 6;
+  const uint4* wr = reinterpret_cast<const uint4*>(kv_b + int64_t(h) * per_head * DSA_VALUE_DIM) + c;
+  uint4 wv[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) wv[u] = g + 4 * u < nope ? __ldcs(wr + int64_t(g + 4 * u) * 64) : make_uint4(0, 0, 0, 0);
+  pdl_wait();
+  pdl_launch_dependents();
+  const __nv_bfloat16* qr = q + b * q_row_stride + h * q_head_stride;
+  for (int i = threadIdx.x; i < nope; i += kHeadThreads) s_q[i] = __bfloat162float(qr[i]);
+  __syncthreads();
+  float acc[8] = {};
+  for (int d0 = g; d0 < nope; d0 += 32) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float x = d0 + 4 * u < nope ? s_q[d0 + 4 * u] : 0.f;
+      const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wv[u]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 a = __bfloat1622float2(wp[e]);
+        acc[2 * e] = fmaf(a.x, x, acc[2 * e]);
+        acc[2 * e + 1] = fmaf(a.y, x, acc[2 * e + 1]);
+      }
+    }
+    if (d0 + 32 < nope) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        wv[u] = d0 + 32 + 4 * u < nope ? __ldcs(wr + int64_t(d0 + 32 + 4 * u) * 64) : make_uint4(0, 0, 0, 0);
+    }
+  }
+  *reinterpret_cast<float4*>(&s_o[g][8 * c]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  *reinterpret_cast<float4*>(&s_o[g][8 * c + 4]) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  __syncthreads();
+  __nv_bfloat162* dst = reinterpret_cast<__nv_bfloat162*>(q_full + (int64_t(b) * H + h) * DSA_LATENT_DIM);
+  const int i = 2 * threadIdx.x;
+  dst[threadIdx.x] = __floats2bfloat162_rn((s_o[0][i] + s_o[1][i]) + (s_o[2][i] + s_o[3][i]),
+                                           (s_o[0][i + 1] + s_o[1][i + 1]) + (s_o[2][i + 1] + s_o[3][i + 1]));
+}
+
+// ov[b, h, d] = sum_l W_UV[h, d, l] o[b, h, l]: four rows d per warp step, 512 columns = two vectors per lane and row.
+__global__ void __launch_bounds__(kHeadThreads)
+value_project_kernel(const __nv_bfloat16* __restrict__ kv_b, const __nv_bfloat16* o, __nv_bfloat16* __restrict__ ov, int H,
+                     int o_heads, int per_head, int v_dim) {
+  const int h = blockIdx.x, b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint4* wr = reinterpret_cast<const uint4*>(kv_b + (int64_t(h) * per_head + per_head - v_dim) * DSA_VALUE_DIM) + lane;
+  uint4 wv[4][2];
+  auto load = [&](int d) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        wv[u][j] = d + u < v_dim ? __ldcs(wr + int64_t(d + u) * 64 + 32 * j) : make_uint4(0, 0, 0, 0);
+  };
+  load(4 * warp);
+  pdl_wait();
+  pdl_launch_dependents();
+  const uint4* xr = reinterpret_cast<const uint4*>(o + (int64_t(b) * o_heads + h) * DSA_VALUE_DIM) + lane;
+  float xf[2][8];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const uint4 xv = xr[32 * j];
+    const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xv);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 v = __bfloat1622float2(xp[e]);
+      xf[j][2 * e] = v.x, xf[j][2 * e + 1] = v.y;
+    }
+  }
+  for (int d = 4 * warp; d < v_dim; d += 32) {
+    float acc[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      acc[u] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wv[u][j]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 a = __bfloat1622float2(wp[e]);
+          acc[u] = fmaf(a.x, xf[j][2 * e], acc[u]);
+          acc[u] = fmaf(a.y, xf[j][2 * e + 1], acc[u]);
+        }
+      }
+    }
+    if (d + 32 < v_dim) load(d + 32);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+#pragma unroll
+      for (int of = 16; of > 0; of >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], of);
+      if (lane == u && d + u < v_dim) ov[(int64_t(b) * H + h) * v_dim + d + u] = __float2bfloat16_rn(acc[u]);
+    }
   }
 }
 
@@ -473,11 +727,13 @@ decode_prep_kernel(const Params p) {
   } else {
     // ---- one MLA query head: absorbed 512 dims copied, rope part rotated
     const int h = item - p.Hidx - 2;
-    const uint4* src = reinterpret_cast<const uint4*>(p.q_abs + (int64_t(b) * p.H + h) * 512);
     __nv_bfloat16* dst = p.q_full + (int64_t(b) * p.H + h) * 576;
-    uint4* dst4 = reinterpret_cast<uint4*>(dst);
-    dst4[lane] = src[lane];            // 64 x 16 B = 512 bf16
-    dst4[lane + 32] = src[lane + 32];
+    if (p.q_abs) {                     // (nullptr: absorb_query_kernel has put them there)
+      const uint4* src = reinterpret_cast<const uint4*>(p.q_abs + (int64_t(b) * p.H + h) * 512);
+      uint4* dst4 = reinterpret_cast<uint4*>(dst);
+      dst4[lane] = src[lane];          // 64 x 16 B = 512 bf16
+      dst4[lane + 32] = src[lane + 32];
+    }
     const __nv_bfloat16* pe = p.q_pe + (int64_t(b) * p.H + h) * p.q_pe_stride;
     const float a0 = __bfloat162float(pe[2 * lane]), a1 = __bfloat162float(pe[2 * lane + 1]);
     const float p0 = __shfl_xor_sync(0xffffffffu, a0, 16), p1 = __shfl_xor_sync(0xffffffffu, a1, 16);

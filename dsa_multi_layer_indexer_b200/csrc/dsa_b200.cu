@@ -105,7 +105,7 @@ static int opt_in_smem(K kernel, size_t bytes, bool (&done)[64]) {
   if (dev >= 0 && dev < 64) done[dev] = true;
   return DSA_OK;
 }
-static bool g_opt_fused[64], g_opt_mla[64], g_opt_mla_beside[64], g_opt_mla_tc[64], g_opt_mla_f32[64], g_opt_topk[64], g_opt_gemv[4][64];
+static bool g_opt_fused[64], g_opt_mla[64], g_opt_mla_beside[64], g_opt_mla_tc[64], g_opt_mla_f32[64], g_opt_topk[64];
 
 // Launch with programmatic dependent launch allowed: the kernel may be scheduled
 // while its predecessor in the stream is still draining; it calls
@@ -1100,39 +1100,108 @@ int dsa_copy_post_epoch(void* dst, const void* src, int64_t bytes, uint32_t* cou
   return DSA_OK;
 }
 
-int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride,
-                  int64_t y_stride, void* stream) {
+extern "C++" {
+// 0: launched; 1: the shape is not for the streaming kernel (nothing is enqueued); else an error.
+template <int B, bool kSwiglu>
+static int launch_gemv_stream(const void* w, const void* w2, const void* x, void* y, int n, int k, int64_t x_stride, int64_t y_stride,
+                              cudaStream_t st) {
+  constexpr size_t kSmem = 226 * 1024, kSums = 16 * 1024;
+  prep::GemvParams p{};
+  // the fewest pieces per row, of even length (the last one may be shorter)
+  const int kv = k / 8;
+  p.ks = (kv + prep::kGemvChunks - 1) / prep::kGemvChunks;
+  p.chunks = (kv + p.ks - 1) / p.ks;
+  p.ks = (kv + p.chunks - 1) / p.chunks;
+  // a CTA per SM; several where one CTA's table of sums would be larger than its part of shared memory
+  const int units = kSwiglu ? n : (n + 1) / 2, most = int(kSums / (size_t(p.ks) * 2 * B * 4));
+  const int blocks = std::min(units, sm_count() * ((units + sm_count() * most - 1) / (sm_count() * most)));
+  const size_t fixed = size_t(B) * k * 2 + size_t((units + blocks - 1) / blocks) * p.ks * 2 * B * 4, piece = size_t(p.chunks) * 32;
+  if (fixed + prep::kGemvWarps * 2 * piece > kSmem) return 1;
+  p.slots = int(std::min<size_t>(std::max<size_t>(std::min<size_t>(prep::kGemvRing, kSmem - fixed) / (prep::kGemvWarps * piece), 2), prep::kGemvMaxSlots));
+  const size_t smem = prep::kGemvWarps * p.slots * piece + fixed;
+  p.w = static_cast<const __nv_bfloat16*>(w), p.w2 = static_cast<const __nv_bfloat16*>(w2), p.x = static_cast<const __nv_bfloat16*>(x);
+  p.y = static_cast<__nv_bfloat16*>(y), p.n = n, p.k = k, p.x_stride = x_stride, p.y_stride = y_stride;
+  static bool done[64];
+  int rc = opt_in_smem(prep::gemv_stream_kernel<B, kSwiglu>, kSmem, done);
+  if (rc) return rc;
+  DSA_CUDA(launch_pdl(prep::gemv_stream_kernel<B, kSwiglu>, dim3(blocks), dim3(prep::kGemvWarps * 32), smem, st, p));
+  return DSA_OK;
+}
+
+template <int B>
+static int launch_gemv_rows(const void* w, const void* x, void* y, int n, int k, int64_t x_stride, int64_t y_stride, cudaStream_t st) {
+  static bool done[64];
+  const size_t smem = size_t(B) * k * 2;
+  DSA_REQUIRE(smem <= 200 * 1024, "gemv: batch * k too large for the shared-memory copy of x");
+  if (smem > 48 * 1024) {
+    int rc = opt_in_smem(prep::gemv_rows_kernel<B>, 200 * 1024, done);
+    if (rc) return rc;
+  }
+  int blocks = (n * 32 + prep::kGemvThreads - 1) / prep::kGemvThreads;
+  if (blocks > 8 * sm_count()) blocks = 8 * sm_count();
+  DSA_CUDA(launch_pdl(prep::gemv_rows_kernel<B>, dim3(blocks), dim3(prep::kGemvThreads), smem, st, static_cast<const __nv_bfloat16*>(w),
+                      static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), n, k, x_stride, y_stride));
+  return DSA_OK;
+}
+}  // extern "C++"
+
+static int gemv_checks(const void* w, const void* x, const void* y, int batch, int n, int k, int64_t x_stride, int64_t y_stride) {
   DSA_REQUIRE(w && x && y, "gemv: null pointer");
   DSA_REQUIRE(batch >= 1 && batch <= 4, "gemv: batch=%d must be 1..4", batch);
   DSA_REQUIRE(n > 0 && k > 0 && k % 8 == 0, "gemv: k=%d must be a positive multiple of 8", k);
-  DSA_REQUIRE(int64_t(batch) * k * 2 <= 96 * 1024, "gemv: batch * k too large for the shared-memory copy of x");
   DSA_REQUIRE(x_stride >= k && x_stride % 8 == 0 && y_stride >= n, "gemv: bad row strides");
   DSA_REQUIRE(aligned16(w) && aligned16(x), "gemv: w and x must be 16-byte aligned");
-  const size_t smem = size_t(batch) * k * 2;
-  // One row per warp with eight 16-byte loads per lane in flight ([32832, 1536]: 18.5 us against
-  // 20.9 / 25.6 us with 2 / 4 rows per warp and fewer loads per row; [36864, 7168]: 79 / 84 / 107 us).
-  int blocks = (n * 32 + prep::kGemvThreads - 1) / prep::kGemvThreads;
-  if (blocks > 8 * sm_count()) blocks = 8 * sm_count();
+  return DSA_OK;
+}
+
+int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride,
+                  int64_t y_stride, void* stream) {
+  int rc = gemv_checks(w, x, y, batch, n, k, x_stride, y_stride);
+  if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const __nv_bfloat16* wp = static_cast<const __nv_bfloat16*>(w);
-  const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
-  __nv_bfloat16* yp = static_cast<__nv_bfloat16*>(y);
-#define DSA_GEMV_CASE(BV)                                                                                     \
-  case BV: {                                                                                                  \
-    if (smem > 48 * 1024) {                                                                                   \
-      int rc = opt_in_smem(prep::gemv_bf16_kernel<BV, 1>, 96 * 1024, g_opt_gemv[BV - 1]);                     \
-      if (rc) return rc;                                                                                      \
-    }                                                                                                         \
-    DSA_CUDA(launch_pdl(prep::gemv_bf16_kernel<BV, 1>, dim3(blocks), dim3(prep::kGemvThreads), smem, st, wp,  \
-                        xp, yp, n, k, x_stride, y_stride));                                                   \
-  } break;
-  switch (batch) {
-    DSA_GEMV_CASE(1)
-    DSA_GEMV_CASE(2)
-    DSA_GEMV_CASE(3)
-    DSA_GEMV_CASE(4)
+  if (batch <= 2) {
+    rc = batch == 1 ? launch_gemv_stream<1, false>(w, nullptr, x, y, n, k, x_stride, y_stride, st)
+                    : launch_gemv_stream<2, false>(w, nullptr, x, y, n, k, x_stride, y_stride, st);
+    if (rc != 1) return rc;
   }
-#undef DSA_GEMV_CASE
+  switch (batch) {
+    case 1: return launch_gemv_rows<1>(w, x, y, n, k, x_stride, y_stride, st);
+    case 2: return launch_gemv_rows<2>(w, x, y, n, k, x_stride, y_stride, st);
+    case 3: return launch_gemv_rows<3>(w, x, y, n, k, x_stride, y_stride, st);
+    default: return launch_gemv_rows<4>(w, x, y, n, k, x_stride, y_stride, st);
+  }
+}
+
+int dsa_gemv_swiglu_bf16(const void* w_gate, const void* w_up, const void* x, void* y, int batch, int n, int k, int64_t x_stride,
+                         int64_t y_stride, void* stream) {
+  int rc = gemv_checks(w_gate, x, y, batch, n, k, x_stride, y_stride);
+  if (rc) return rc;
+  DSA_REQUIRE(w_up && aligned16(w_up), "gemv: w_up must be a 16-byte aligned pointer");
+  DSA_REQUIRE(batch <= 2, "gemv + SwiGLU: batch=%d must be 1 or 2", batch);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  rc = batch == 1 ? launch_gemv_stream<1, true>(w_gate, w_up, x, y, n, k, x_stride, y_stride, st)
+                  : launch_gemv_stream<2, true>(w_gate, w_up, x, y, n, k, x_stride, y_stride, st);
+  return rc == 1 ? fail(DSA_ERR_UNSUPPORTED, "gemv + SwiGLU: [%d, %d] is outside the streaming kernel's range", n, k) : rc;
+}
+
+int dsa_absorb_query(const void* kv_b, const void* q, void* q_full, int B, int H, int nope, int per_head, int64_t q_row_stride,
+                     int64_t q_head_stride, void* stream) {
+  DSA_REQUIRE(kv_b && q && q_full, "absorb query: null pointer");
+  DSA_REQUIRE(aligned16(kv_b) && aligned16(q_full), "absorb query: pointers must be 16-byte aligned");
+  DSA_REQUIRE(B > 0 && B <= 65535 && H > 0 && nope > 0 && nope <= 512 && per_head >= nope, "absorb query: bad shape");
+  DSA_CUDA(launch_pdl(prep::absorb_query_kernel, dim3(H, B), dim3(prep::kHeadThreads), 0, static_cast<cudaStream_t>(stream),
+                      static_cast<const __nv_bfloat16*>(kv_b), static_cast<const __nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(q_full),
+                      H, nope, per_head, q_row_stride, q_head_stride));
+  return DSA_OK;
+}
+
+int dsa_value_project(const void* kv_b, const void* o, void* ov, int B, int H, int o_heads, int per_head, int v_dim, void* stream) {
+  DSA_REQUIRE(kv_b && o && ov, "value projection: null pointer");
+  DSA_REQUIRE(aligned16(kv_b) && aligned16(o), "value projection: pointers must be 16-byte aligned");
+  DSA_REQUIRE(B > 0 && B <= 65535 && H > 0 && o_heads >= H && v_dim > 0 && per_head >= v_dim, "value projection: bad shape");
+  DSA_CUDA(launch_pdl(prep::value_project_kernel, dim3(H, B), dim3(prep::kHeadThreads), 0, static_cast<cudaStream_t>(stream),
+                      static_cast<const __nv_bfloat16*>(kv_b), static_cast<const __nv_bfloat16*>(o), static_cast<__nv_bfloat16*>(ov), H,
+                      o_heads, per_head, v_dim));
   return DSA_OK;
 }
 
@@ -1237,7 +1306,7 @@ int dsa_decode_prep(const void* iq_raw, const void* w_raw, const void* ik_raw, c
                     const int64_t* positions, uint8_t* index_q, float* index_w, void* q_full,
                     uint8_t* cache_index_k, float* cache_k_scale, void* cache_kv, int B, int H,
                     int n_index_heads, int64_t cap, int interleave, float eps, void* stream) {
-  DSA_REQUIRE(iq_raw && w_raw && ik_raw && kv_a && q_abs && q_pe && kv_norm_w && mla_cos && mla_sin && idx_cos &&
+  DSA_REQUIRE(iq_raw && w_raw && ik_raw && kv_a && q_pe && kv_norm_w && mla_cos && mla_sin && idx_cos &&
                   idx_sin && positions && index_q && index_w && q_full && cache_index_k && cache_k_scale && cache_kv,
               "decode prep: null pointer");
   DSA_REQUIRE(aligned16(iq_raw) && aligned16(ik_raw) && aligned16(q_abs) && aligned16(q_full) && aligned16(index_q) &&

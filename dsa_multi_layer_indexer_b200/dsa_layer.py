@@ -401,8 +401,7 @@ class DSALayer(nn.Module):
     def mlp(self, h_norm: torch.Tensor, weights=None) -> torch.Tensor:
         if (h_norm.is_cuda and h_norm.dtype == torch.bfloat16 and h_norm.dim() == 2 and h_norm.shape[0] <= 2
                 and not torch.is_grad_enabled()):
-            gate, up = ops.gemv(h_norm, self.gate_proj.weight), ops.gemv(h_norm, self.up_proj.weight)
-            return self._reduced(self.down_proj(ops.silu_mul(gate, up)))
+            return self._reduced(self._skinny("down_proj", ops.gemv_swiglu(h_norm, self.gate_proj.weight, self.up_proj.weight)))
         w = self._full_weights(h_norm) if h_norm.dim() == 3 and weights is None else weights
         if w is not None:
             y = _lib.host().mlp(h_norm.reshape(-1, h_norm.shape[2]), w[8], w[9], w[10])
@@ -413,6 +412,16 @@ class DSALayer(nn.Module):
         return self._reduced(self.down_proj(torch.nn.functional.silu(gate) * up))
 
     # ------------------------------------------------------------------ decode form
+    def _skinny(self, name: str, x: torch.Tensor) -> torch.Tensor:
+        """A projection of one or two bf16 rows: the library's GEMV, which starts on its weights while the
+        kernel before it runs, unless the module is not a plain ``nn.Linear``."""
+        m = self._modules[name]
+        if (x.shape[0] > 2 or x.dtype != torch.bfloat16 or not x.is_cuda or torch.is_grad_enabled() or m.__class__ is not nn.Linear
+                or m.bias is not None or m.weight.dtype != torch.bfloat16 or m._forward_hooks or m._forward_pre_hooks
+                or m.in_features % 8 or not m.weight.is_contiguous()):
+            return m(x)
+        return ops.gemv(x, m.weight)
+
     def new_cache(self, n_seq: int, capacity: int, device, fp8: bool) -> LayerDecodeCache:
         c = self.config
         if fp8:
@@ -465,14 +474,20 @@ class DSALayer(nn.Module):
             ik_raw = self.index_k_proj(x_norm)
             w = self.index_weights_proj(c_q)
         q_nope, q_rope = q.split([c.qk_nope_head_dim, c.qk_rope_head_dim], dim=-1)
-        w_uk, _ = self._w_uk_uv()
-        q_abs = torch.einsum("bhd,hdl->bhl", q_nope, w_uk)
+        fused = cache.k_scale is not None and x_norm.dtype == torch.bfloat16
+        if fused and b <= 2 and c.qk_nope_head_dim <= 512 and not torch.is_grad_enabled():
+            q_abs = None  # absorbed straight into the first columns of the query below
+        else:
+            w_uk, _ = self._w_uk_uv()
+            q_abs = torch.einsum("bhd,hdl->bhl", q_nope, w_uk)
         if cache.k_scale is not None and x_norm.dtype == torch.bfloat16:
             index_q = torch.empty(b, c.index_n_heads, c.index_head_dim, dtype=torch.uint8, device=x_norm.device)
             index_w = torch.empty(b, c.index_n_heads, dtype=torch.float32, device=x_norm.device)
             q_full = torch.empty(b, h, c.qk_head_dim, dtype=torch.bfloat16, device=x_norm.device)
+            if q_abs is None:
+                ops.absorb_query(self.kv_b_proj.weight, q, c.qk_nope_head_dim, q_full)
             ops.decode_prep(iq_raw.contiguous(), w.contiguous(), ik_raw.contiguous(), kv_a.contiguous(),
-                            q_abs.contiguous(), q_rope, self.kv_a_layernorm.weight, rope.mla_cos, rope.mla_sin,
+                            None if q_abs is None else q_abs.contiguous(), q_rope, self.kv_a_layernorm.weight, rope.mla_cos, rope.mla_sin,
                             rope.idx_cos, rope.idx_sin, positions, index_q, index_w, q_full, cache.index_k,
                             cache.k_scale, cache.kv, il, c.rms_norm_eps)
             return q_full, index_q, index_w
@@ -525,8 +540,11 @@ class DSALayer(nn.Module):
             h = q.shape[1]
             direct = q.dtype == torch.bfloat16 and h % ops.HEAD_BLOCK == 0 and q.is_contiguous()
             o = ops.sparse_mla_decode(_pad_heads(q.to(torch.bfloat16), ops.HEAD_BLOCK).contiguous(), cache.kv,
-                                      indices, self.sm_scale, seq_lens,
-                                      beside_previous=beside_previous and direct)[:, :h].to(q.dtype)
+                                      indices, self.sm_scale, seq_lens, beside_previous=beside_previous and direct)
+            if q.dtype == torch.bfloat16 and q.shape[0] <= 2 and not torch.is_grad_enabled():
+                ov = ops.value_project(self.kv_b_proj.weight, o, h, c.v_head_dim)
+                return self._reduced(self._skinny("o_proj", ov.view(ov.shape[0], h * c.v_head_dim)))
+            o = o[:, :h].to(q.dtype)
         else:
             o = ops.sparse_mla_f32(q.float().contiguous(), cache.kv, indices, c.kv_lora_rank, self.sm_scale,
                                    seq_lens).to(q.dtype)

@@ -366,21 +366,62 @@ def copy_post_epoch(dst: torch.Tensor, src: torch.Tensor, counter: torch.Tensor,
                                               1 if beside_previous else 0, _stream()))
 
 
-def gemv(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """``x @ weight.T`` for a decode batch of 1..4 rows (bf16, fp32 accumulation): the weight
-    matrix ``[n, k]`` is streamed once. For the projection shapes where the library GEMV is
-    latency-bound."""
+def _gemv_operand(x: torch.Tensor, weight: torch.Tensor, most: int) -> torch.Tensor:
     _need(x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.dim() == 2,
           "x must be a CUDA bf16 [B, k] tensor and weight bf16")
-    b, k = x.shape
-    n = weight.shape[0]
-    _need(weight.dim() == 2 and weight.shape[1] == k and weight.is_contiguous(), "weight must be contiguous [n, k]")
-    _need(1 <= b <= 4 and k % 8 == 0 and b * k * 2 <= 96 * 1024, "batch 1..4, k a multiple of 8, batch * k <= 48K")
-    x = x if x.stride(1) == 1 and x.stride(0) % 8 == 0 else x.contiguous()
+    _need(weight.dim() == 2 and weight.shape[1] == x.shape[1] and weight.is_contiguous(), "weight must be contiguous [n, k]")
+    _need(1 <= x.shape[0] <= most and x.shape[1] % 8 == 0, f"batch 1..{most}, k a multiple of 8")
+    return x if x.stride(1) == 1 and x.stride(0) % 8 == 0 else x.contiguous()
+
+
+def gemv(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """``x @ weight.T`` for a decode batch of 1..4 rows (bf16, fp32 accumulation): the weight
+    matrix ``[n, k]`` is streamed once, its first part while the kernel before is still running."""
+    x = _gemv_operand(x, weight, 4)
+    (b, k), n = x.shape, weight.shape[0]
     y = torch.empty(b, n, dtype=torch.bfloat16, device=x.device)
     _lib.check(_lib.lib().dsa_gemv_bf16(_ptr(weight), _ptr(x), _ptr(y), b, n, k, x.stride(0) if b > 1 else k, n,
                                         _stream()))
     return y
+
+
+def gemv_swiglu(x: torch.Tensor, gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
+    """``silu(x @ gate.T) * (x @ up.T)`` for one or two rows in one launch, rounded as the separate operations."""
+    x = _gemv_operand(x, gate, 2)
+    _need(up.shape == gate.shape and up.dtype == torch.bfloat16 and up.is_contiguous(), "gate and up must have one shape")
+    (b, k), n = x.shape, gate.shape[0]
+    if b * k > 32768:  # x beside the weights' ring in shared memory: the streaming kernel's limit is a little above
+        return silu_mul(gemv(x, gate), gemv(x, up))
+    y = torch.empty(b, n, dtype=torch.bfloat16, device=x.device)
+    _lib.check(_lib.lib().dsa_gemv_swiglu_bf16(_ptr(gate), _ptr(up), _ptr(x), _ptr(y), b, n, k, x.stride(0) if b > 1 else k, n,
+                                               _stream()))
+    return y
+
+
+def absorb_query(kv_b: torch.Tensor, q: torch.Tensor, nope: int, q_full: torch.Tensor) -> None:
+    """Columns [0, 512) of ``q_full`` ``[B, H, 576]`` = ``q[b, h, :nope]`` through W_UK, the first ``nope`` rows
+    of every head of ``kv_b`` ``[H * per_head, 512]``; ``q`` ``[B, H, >= nope]`` may be a strided view."""
+    B, H = q.shape[0], q.shape[1]
+    _need(q.is_cuda and q.dtype == torch.bfloat16 and q.dim() == 3 and q.stride(2) == 1 and q.shape[2] >= nope, "q must be bf16 [B, H, >= nope]")
+    _cuda_contig(kv_b, "kv_b", (torch.bfloat16,))
+    _cuda_contig(q_full, "q_full", (torch.bfloat16,))
+    _need(kv_b.dim() == 2 and kv_b.shape[1] == VALUE_DIM and kv_b.shape[0] % H == 0 and tuple(q_full.shape) == (B, H, LATENT_DIM),
+          "kv_b must be [H * per_head, 512], q_full [B, H, 576]")
+    _lib.check(_lib.lib().dsa_absorb_query(_ptr(kv_b), _ptr(q), _ptr(q_full), B, H, nope, kv_b.shape[0] // H, q.stride(0), q.stride(1),
+                                           _stream()))
+
+
+def value_project(kv_b: torch.Tensor, o: torch.Tensor, heads: int, v_dim: int) -> torch.Tensor:
+    """``[B, heads, v_dim]``: every head's latent output ``o`` ``[B, >= heads, 512]`` through W_UV, the last
+    ``v_dim`` rows of the head's part of ``kv_b`` ``[heads * per_head, 512]``."""
+    _cuda_contig(kv_b, "kv_b", (torch.bfloat16,))
+    _cuda_contig(o, "o", (torch.bfloat16,))
+    _need(o.dim() == 3 and o.shape[2] == VALUE_DIM and o.shape[1] >= heads and kv_b.dim() == 2 and kv_b.shape[1] == VALUE_DIM
+          and kv_b.shape[0] % heads == 0, "kv_b must be [heads * per_head, 512], o [B, >= heads, 512]")
+    ov = torch.empty(o.shape[0], heads, v_dim, dtype=torch.bfloat16, device=o.device)
+    _lib.check(_lib.lib().dsa_value_project(_ptr(kv_b), _ptr(o), _ptr(ov), o.shape[0], heads, o.shape[1], kv_b.shape[0] // heads, v_dim,
+                                            _stream()))
+    return ov
 
 
 def indexer_stage_fp8(q_raw, k_raw, w_raw, k_norm_weight, k_norm_bias, k_norm_eps: float, rope_cos, rope_sin,
@@ -419,17 +460,20 @@ def decode_prep(iq_raw, w_raw, ik_raw, kv_a, q_abs, q_pe, kv_norm_w, mla_cos, ml
     """One launch for the chain between the projection GEMVs and the hot path
     (see ``dsa_decode_prep`` in the header). All operands bf16 CUDA tensors;
     ``q_pe`` may be a strided view ``q[..., nope:]`` of the q_b_proj output."""
-    for t, n in ((iq_raw, "iq_raw"), (w_raw, "w_raw"), (ik_raw, "ik_raw"), (kv_a, "kv_a"), (q_abs, "q_abs"),
+    for t, n in ((iq_raw, "iq_raw"), (w_raw, "w_raw"), (ik_raw, "ik_raw"), (kv_a, "kv_a"), (q_full, "q_full"),
                  (kv_norm_w, "kv_norm_w"), (mla_cos, "mla_cos"), (mla_sin, "mla_sin"), (idx_cos, "idx_cos"),
                  (idx_sin, "idx_sin")):
         _cuda_contig(t, n, (torch.bfloat16,))
+    if q_abs is not None:  # (None: those columns of q_full are filled already)
+        _cuda_contig(q_abs, "q_abs", (torch.bfloat16,))
+        _need(q_abs.shape[2] == VALUE_DIM, "q_abs must be [B, H, 512]")
     _need(q_pe.dtype == torch.bfloat16 and q_pe.dim() == 3 and q_pe.shape[2] == 64 and q_pe.stride(2) == 1
           and (q_pe.shape[0] == 1 or q_pe.stride(0) == q_pe.shape[1] * q_pe.stride(1)),
           "q_pe must be a [B, H, 64] bf16 view with dense rows")
     _cuda_contig(positions, "positions", (torch.int64,))
     B, n_idx = iq_raw.shape[0], iq_raw.shape[1]
-    H = q_abs.shape[1]
-    _need(iq_raw.shape[2] == INDEX_DIM and kv_a.shape[-1] == LATENT_DIM and q_abs.shape[2] == VALUE_DIM,
+    H = q_full.shape[1]
+    _need(iq_raw.shape[2] == INDEX_DIM and kv_a.shape[-1] == LATENT_DIM and q_full.shape[2] == LATENT_DIM,
           "decode prep needs the production geometry")
     cap = cache_kv.shape[1]
     _need(cache_kv.shape[0] == B and cache_index_k.shape[:2] == (B, cap), "caches must be [B, cap, ...]")

@@ -67,6 +67,7 @@ const char* dsa_status_string(int status);
 #define DSA_STATUS_SELECT_OVERFLOW 4u
 #define DSA_STATUS_BAD_PAGE 8u
 #define DSA_STATUS_EXCHANGE_TIMEOUT 16u
+#define DSA_STATUS_GEMV_TIMEOUT 32u
 int dsa_check_device_status(uint32_t* detail);
 
 /* Tracing builds only (compiled with -DDSA_STAMPS): copies the per-CTA phase
@@ -346,7 +347,7 @@ int dsa_sparse_mla_f32(const float* q, const float* kv, const int32_t* indices,
  *     index_w = q_scale * w_raw;
  *   - the token's index key: RoPE, e4m3 + scale, written at cache row positions[b];
  *   - the token's latent row: RMSNorm(512) | RoPE(64), written at positions[b];
- *   - the absorbed query: q_full = [q_abs | RoPE(q_pe)].
+ *   - the absorbed query: q_full = [q_abs | RoPE(q_pe)] (q_abs NULL: those columns are there already).
  * All inputs bf16 ([B,Hidx,128], [B,Hidx], [B,128], [B,576], [B,H,512],
  * [B,H,64] with row stride q_pe_stride elements); rotary tables bf16
  * [cap,64] / [cap,128]; caches as in dsa_indexer_scan_fp8 / dsa_sparse_mla_*. */
@@ -397,10 +398,23 @@ int dsa_copy_post_epoch(void* dst, const void* src, int64_t bytes, uint32_t* cou
 
 /* y[b, n] = sum_k w[n, k] x[b, k] for a decode batch of 1..4 rows: bf16 operands, fp32
  * accumulation, w [n, k] row-major streamed once (the projection GEMVs of
- * src/lagged_indexer_dsa/dsa_layer.py:87-125 at decode). k a multiple of 8,
- * batch * k * 2 <= 96 KB; row strides of x and y in elements. */
+ * src/lagged_indexer_dsa/dsa_layer.py:87-125 at decode). k a multiple of 8; row strides of x and y in
+ * elements. The kernel starts reading w before the kernel enqueued in front of it has completed: w must
+ * not be written by this library (by any other work, anything goes).
+ * dsa_gemv_swiglu_bf16: y = silu(x w_gate^T) * (x w_up^T), rounded as the separate operations, for one or
+ * two rows (:194-196). */
 int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride,
                   int64_t y_stride, void* stream);
+int dsa_gemv_swiglu_bf16(const void* w_gate, const void* w_up, const void* x, void* y, int batch, int n, int k,
+                         int64_t x_stride, int64_t y_stride, void* stream);
+/* The per-head products of a decode token with kv_b_proj's weight [H, per_head, 512] (per_head = nope +
+ * v_dim, bf16, src/lagged_indexer_dsa/dsa_layer.py:96-125), read like the weights of dsa_gemv_bf16:
+ * dsa_absorb_query: columns [0, 512) of q_full [B, H, 576] = q[b, h, 0:nope] W_UK[h] (element strides given);
+ * dsa_value_project: ov [B, H, v_dim] = W_UV[h] o[b, h, :], o [B, o_heads, 512]. */
+int dsa_absorb_query(const void* kv_b, const void* q, void* q_full, int B, int H, int nope, int per_head,
+                     int64_t q_row_stride, int64_t q_head_stride, void* stream);
+int dsa_value_project(const void* kv_b, const void* o, void* ov, int B, int H, int o_heads, int per_head,
+                      int v_dim, void* stream);
 /* out = silu(gate) * up over n bf16 elements: the SwiGLU between the MLP's GEMVs
  * (src/lagged_indexer_dsa/dsa_layer.py:194-196), rounded as the two separate operations. */
 int dsa_silu_mul_bf16(const void* gate, const void* up, void* out, int64_t n, void* stream);
