@@ -296,7 +296,7 @@ struct GemvParams {
 };
 // shared memory: ring [warps][slots][2][chunks] | x [B][k] | sums [units of a CTA][ks][2][B]
 template <int B, bool kSwiglu>
-__global__ void __launch_bounds__(kGemvWarps * 32, 1)
+__global__ void __launch_bounds__(kGemvWarps * 32, B == 1 ? 2 : 1)
 gemv_stream_kernel(const GemvParams p) {
   extern __shared__ __align__(128) uint8_t gemv_smem[];
   __shared__ uint64_t s_full[kGemvWarps * kGemvMaxSlots];
@@ -485,111 +485,6 @@ gemv_rows_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __res
   }
 }
 
-// ------------------------------------------------------------------ per-head products of a decode row
-// The two absorbed projections of a decode step over kv_b_proj's weight [H, nope + v, 512]
-// (src/lagged_indexer_dsa/dsa_layer.py:96-125): q_abs[h] = q_nope[h] W_UK[h] into the first 512 columns of
-// q_full, and ov[h] = W_UV[h] o[h]. One token's 33 MB of weights are streamed once; as in the GEMV above the
-// first loads go out before the dependency wait. One CTA per (head, batch row).
-constexpr int kHeadThreads = 256;
-__global__ void __launch_bounds__(kHeadThreads)
-absorb_query_kernel(const __nv_bfloat16* __restrict__ kv_b, const __nv_bfloat16* q, __nv_bfloat16* __restrict__ q_full,
-                    int H, int nope, int per_head, int64_t q_row_stride, int64_t q_head_stride) {
-  // 64 column vectors of 8 x 4 groups of rows: thread (g, c) sums rows g, g + 4, ... of its eight columns
-  __shared__ float s_q[512];
-  __shared__ __align__(16) float s_o[4][512];
-  const int h = blockIdx.x, b = blockIdx.y, c = threadIdx.x & 63, g = threadIdx.x >> 6;
-  const uint4* wr = reinterpret_cast<const uint4*>(kv_b + int64_t(h) * per_head * DSA_VALUE_DIM) + c;
-  uint4 wv[8];
-#pragma unroll
-  for (int u = 0; u < 8; ++u) wv[u] = g + 4 * u < nope ? __ldcs(wr + int64_t(g + 4 * u) * 64) : make_uint4(0, 0, 0, 0);
-  pdl_wait();
-  pdl_launch_dependents();
-  const __nv_bfloat16* qr = q + b * q_row_stride + h * q_head_stride;
-  for (int i = threadIdx.x; i < nope; i += kHeadThreads) s_q[i] = __bfloat162float(qr[i]);
-  __syncthreads();
-  float acc[8] = {};
-  for (int d0 = g; d0 < nope; d0 += 32) {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const float x = d0 + 4 * u < nope ? s_q[d0 + 4 * u] : 0.f;
-      const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wv[u]);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 a = __bfloat1622float2(wp[e]);
-        acc[2 * e] = fmaf(a.x, x, acc[2 * e]);
-        acc[2 * e + 1] = fmaf(a.y, x, acc[2 * e + 1]);
-      }
-    }
-    if (d0 + 32 < nope) {
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        wv[u] = d0 + 32 + 4 * u < nope ? __ldcs(wr + int64_t(d0 + 32 + 4 * u) * 64) : make_uint4(0, 0, 0, 0);
-    }
-  }
-  *reinterpret_cast<float4*>(&s_o[g][8 * c]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-  *reinterpret_cast<float4*>(&s_o[g][8 * c + 4]) = make_float4(acc[4], acc[5], acc[6], acc[7]);
-  __syncthreads();
-  __nv_bfloat162* dst = reinterpret_cast<__nv_bfloat162*>(q_full + (int64_t(b) * H + h) * DSA_LATENT_DIM);
-  const int i = 2 * threadIdx.x;
-  dst[threadIdx.x] = __floats2bfloat162_rn((s_o[0][i] + s_o[1][i]) + (s_o[2][i] + s_o[3][i]),
-                                           (s_o[0][i + 1] + s_o[1][i + 1]) + (s_o[2][i + 1] + s_o[3][i + 1]));
-}
-
-// ov[b, h, d] = sum_l W_UV[h, d, l] o[b, h, l]: four rows d per warp step, 512 columns = two vectors per lane and row.
-__global__ void __launch_bounds__(kHeadThreads)
-value_project_kernel(const __nv_bfloat16* __restrict__ kv_b, const __nv_bfloat16* o, __nv_bfloat16* __restrict__ ov, int H,
-                     int o_heads, int per_head, int v_dim) {
-  const int h = blockIdx.x, b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint4* wr = reinterpret_cast<const uint4*>(kv_b + (int64_t(h) * per_head + per_head - v_dim) * DSA_VALUE_DIM) + lane;
-  uint4 wv[4][2];
-  auto load = [&](int d) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        wv[u][j] = d + u < v_dim ? __ldcs(wr + int64_t(d + u) * 64 + 32 * j) : make_uint4(0, 0, 0, 0);
-  };
-  load(4 * warp);
-  pdl_wait();
-  pdl_launch_dependents();
-  const uint4* xr = reinterpret_cast<const uint4*>(o + (int64_t(b) * o_heads + h) * DSA_VALUE_DIM) + lane;
-  float xf[2][8];
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const uint4 xv = xr[32 * j];
-    const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xv);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 v = __bfloat1622float2(xp[e]);
-      xf[j][2 * e] = v.x, xf[j][2 * e + 1] = v.y;
-    }
-  }
-  for (int d = 4 * warp; d < v_dim; d += 32) {
-    float acc[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      acc[u] = 0.f;
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wv[u][j]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 a = __bfloat1622float2(wp[e]);
-          acc[u] = fmaf(a.x, xf[j][2 * e], acc[u]);
-          acc[u] = fmaf(a.y, xf[j][2 * e + 1], acc[u]);
-        }
-      }
-    }
-    if (d + 32 < v_dim) load(d + 32);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-#pragma unroll
-      for (int of = 16; of > 0; of >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], of);
-      if (lane == u && d + u < v_dim) ov[(int64_t(b) * H + h) * v_dim + d + u] = __float2bfloat16_rn(acc[u]);
-    }
-  }
-}
-
 // ------------------------------------------------------------------ decode prep
 struct Params {
   // inputs (bf16, outputs of the projection GEMVs), B rows
@@ -613,7 +508,8 @@ struct Params {
   float* cache_k_scale;          // [B, cap]
   __nv_bfloat16* cache_kv;       // [B, cap, 576]
   int64_t cap;
-  int64_t q_pe_stride;
+  int64_t q_pe_stride;           // elements between heads
+  int64_t iq_row, w_row, ik_row, kva_row, q_row;  // elements between the tokens of iq_raw, w_raw, ik_raw, kv_a, q_pe
   int B, H, Hidx;
   int interleave;                // indexer RoPE pairing (GLM-5) vs half split (DeepSeek)
   float eps;
@@ -663,22 +559,16 @@ __device__ __forceinline__ uint32_t quant128(const float (&v)[4], float& scale) 
   return packed;
 }
 
-__global__ void __launch_bounds__(128)
-decode_prep_kernel(const Params p) {
-  const int lane = threadIdx.x & 31;
-  const int item = blockIdx.x * 4 + (threadIdx.x >> 5);
-  const int b = blockIdx.y;
-  const int n_items = p.Hidx + 2 + p.H;
-  if (item >= n_items) return;
-  pdl_wait();
-  pdl_launch_dependents();
+// One warp per item of a token: an indexer query head, the token's index key, its latent row, or the rotary
+// part of an MLA query head (with the absorbed part where q_abs is given).
+__device__ __forceinline__ void prep_item(const Params& p, int b, int item, int lane) {
   const int64_t pos = p.positions[b];
   if (pos < 0 || pos >= p.cap) return;
 
   if (item < p.Hidx) {
     // ---- one indexer query head: RoPE, quantise, fold the scale into the head weight
     const int h = item;
-    const __nv_bfloat16* src = p.iq_raw + (int64_t(b) * p.Hidx + h) * 128 + 4 * lane;
+    const __nv_bfloat16* src = p.iq_raw + b * p.iq_row + h * 128 + 4 * lane;
     const uint2 raw = *reinterpret_cast<const uint2*>(src);
     const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&raw.x);
     const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
@@ -687,10 +577,10 @@ decode_prep_kernel(const Params p) {
     float scale;
     const uint32_t q = quant128(v, scale);
     *reinterpret_cast<uint32_t*>(p.index_q + (int64_t(b) * p.Hidx + h) * 128 + 4 * lane) = q;
-    if (lane == 0) p.index_w[int64_t(b) * p.Hidx + h] = scale * __bfloat162float(p.w_raw[int64_t(b) * p.Hidx + h]);
+    if (lane == 0) p.index_w[int64_t(b) * p.Hidx + h] = scale * __bfloat162float(p.w_raw[b * p.w_row + h]);
   } else if (item == p.Hidx) {
     // ---- the new token's index key: RoPE, quantise, append
-    const uint2 raw = *reinterpret_cast<const uint2*>(p.ik_raw + int64_t(b) * 128 + 4 * lane);
+    const uint2 raw = *reinterpret_cast<const uint2*>(p.ik_raw + b * p.ik_row + 4 * lane);
     const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&raw.x);
     const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
     float v[4] = {__bfloat162float(lo.x), __bfloat162float(lo.y), __bfloat162float(hi.x), __bfloat162float(hi.y)};
@@ -701,7 +591,7 @@ decode_prep_kernel(const Params p) {
     if (lane == 0) p.cache_k_scale[int64_t(b) * p.cap + pos] = scale;
   } else if (item == p.Hidx + 1) {
     // ---- the new token's latent row: RMSNorm(512) | RoPE(64), append
-    const __nv_bfloat16* src = p.kv_a + int64_t(b) * 576;
+    const __nv_bfloat16* src = p.kv_a + b * p.kva_row;
     __nv_bfloat16* dst = p.cache_kv + (int64_t(b) * p.cap + pos) * 576;
     float v[16];
     float ss = 0.f;
@@ -728,13 +618,13 @@ decode_prep_kernel(const Params p) {
     // ---- one MLA query head: absorbed 512 dims copied, rope part rotated
     const int h = item - p.Hidx - 2;
     __nv_bfloat16* dst = p.q_full + (int64_t(b) * p.H + h) * 576;
-    if (p.q_abs) {                     // (nullptr: absorb_query_kernel has put them there)
+    if (p.q_abs) {
       const uint4* src = reinterpret_cast<const uint4*>(p.q_abs + (int64_t(b) * p.H + h) * 512);
       uint4* dst4 = reinterpret_cast<uint4*>(dst);
       dst4[lane] = src[lane];          // 64 x 16 B = 512 bf16
       dst4[lane + 32] = src[lane + 32];
     }
-    const __nv_bfloat16* pe = p.q_pe + (int64_t(b) * p.H + h) * p.q_pe_stride;
+    const __nv_bfloat16* pe = p.q_pe + b * p.q_row + h * p.q_pe_stride;
     const float a0 = __bfloat162float(pe[2 * lane]), a1 = __bfloat162float(pe[2 * lane + 1]);
     const float p0 = __shfl_xor_sync(0xffffffffu, a0, 16), p1 = __shfl_xor_sync(0xffffffffu, a1, 16);
     const float sign = lane < 16 ? -1.f : 1.f;
@@ -742,6 +632,198 @@ decode_prep_kernel(const Params p) {
     const __nv_bfloat16* sr = p.mla_sin + pos * 64 + 2 * lane;
     dst[512 + 2 * lane] = __float2bfloat16_rn(a0 * __bfloat162float(cr[0]) + sign * p0 * __bfloat162float(sr[0]));
     dst[512 + 2 * lane + 1] = __float2bfloat16_rn(a1 * __bfloat162float(cr[1]) + sign * p1 * __bfloat162float(sr[1]));
+  }
+}
+
+__global__ void __launch_bounds__(128)
+decode_prep_kernel(const Params p) {
+  const int item = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (item >= p.Hidx + 2 + p.H) return;
+  pdl_wait();
+  pdl_launch_dependents();
+  prep_item(p, blockIdx.y, item, threadIdx.x & 31);
+}
+
+// ------------------------------------------------------------------ decode token: per-head products
+// A decode token's products with kv_b_proj's weight [H][nope + v][512] (src/lagged_indexer_dsa/dsa_layer.py:
+// 96-125) for NB tokens at a time: W_UK absorbed into the query (with every other item of decode_prep_kernel
+// in the same launch, nothing of which depends on it) and W_UV applied to the attention's output.
+// Bound by the latency of reading 128 - 256 KB per head in one CTA, so what can be read before the dependency
+// wait is: the first rows into registers, the rest of W_UK into L2, and W_UV, which the step needs two dozen
+// microseconds later, into L2 after the wait, while nothing else uses the memory.
+// One token of 128 heads of 128 + 128 behind its projection: 11.9 -> 6.7 us (absorption and the other items
+// were two launches), value projection 7.5 -> 5.2 us. Four / eight tokens: with the copies of the strided
+// projection outputs that decode_prep needs, 27 -> 8 us.
+constexpr int kHeadThreads = 512;
+constexpr int kHeadMaxTokens = 8;
+constexpr int kHeadMaxNope = 512;
+struct HeadParams {
+  const __nv_bfloat16* kv_b;
+  const __nv_bfloat16* q;  // [B] rows of H heads of nope + 64 (absorption) / [B, o_heads, 512] (value projection)
+  __nv_bfloat16* out;      // [B, H, v_dim] (value projection)
+  int64_t q_row, q_head;
+  int nope, v_dim, H, B, o_heads;
+};
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+// bytes a multiple of 16; one lane per 4 KB
+__device__ __forceinline__ void prefetch_l2_range(const char* p, int64_t bytes, int t, int threads) {
+  for (int64_t o = int64_t(t) * 4096; o < bytes; o += int64_t(threads) * 4096)
+    prefetch_l2(p + o, uint32_t(bytes - o < 4096 ? bytes - o : 4096));
+}
+
+template <int NB>
+__global__ void __launch_bounds__(kHeadThreads, NB <= 2 ? 2 : 1)
+decode_token_kernel(const Params p, const HeadParams hp) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (blockIdx.x >= unsigned(p.H)) {  // ---- a warp per indexer head, index key and latent row
+    const int i = (blockIdx.x - p.H) * (kHeadThreads / 32) + warp, b = i / (p.Hidx + 2);
+    pdl_wait();
+    pdl_launch_dependents();
+    if (b < p.B) prep_item(p, b, i - b * (p.Hidx + 2), lane);
+    return;
+  }
+  // ---- head h: 64 column vectors of 8 x 8 groups of rows: thread (g, c) sums rows g, g + 8, ... of its columns
+  extern __shared__ __align__(16) float head_smem[];  // q [NB][nope] | sums [8][NB <= 2 ? NB : 2][512]
+  constexpr int kRound = NB <= 2 ? NB : 2;            // tokens whose sums are folded at a time
+  float* s_q = head_smem;
+  float* s_o = head_smem + NB * kHeadMaxNope;
+  const int h = blockIdx.x, c = tid & 63, g = tid >> 6, nope = hp.nope;
+  const __nv_bfloat16* w_head = hp.kv_b + int64_t(h) * (nope + hp.v_dim) * DSA_VALUE_DIM;
+  const uint4* wr = reinterpret_cast<const uint4*>(w_head) + c;
+  uint4 wv[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) wv[u] = g + 8 * u < nope ? wr[int64_t(g + 8 * u) * 64] : make_uint4(0, 0, 0, 0);
+  if (nope > 64) prefetch_l2_range(reinterpret_cast<const char*>(w_head + 64 * DSA_VALUE_DIM), int64_t(nope - 64) * DSA_VALUE_DIM * 2, tid, kHeadThreads);
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int i = tid; i < NB * nope; i += kHeadThreads) {
+    const int b = i / nope, d = i - b * nope;
+    s_q[b * kHeadMaxNope + d] = b < hp.B ? __bfloat162float(hp.q[b * hp.q_row + h * hp.q_head + d]) : 0.f;
+  }
+  __syncthreads();
+  prefetch_l2_range(reinterpret_cast<const char*>(w_head + int64_t(nope) * DSA_VALUE_DIM), int64_t(hp.v_dim) * DSA_VALUE_DIM * 2, tid, kHeadThreads);
+  float acc[NB][8];
+#pragma unroll
+  for (int b = 0; b < NB; ++b)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[b][e] = 0.f;
+  for (int d0 = g; d0 < nope; d0 += 64) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int d = d0 + 8 * u;
+      const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wv[u]);
+      float2 a[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[e] = __bfloat1622float2(wp[e]);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        const float x = d < nope ? s_q[b * kHeadMaxNope + d] : 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          acc[b][2 * e] = fmaf(a[e].x, x, acc[b][2 * e]);
+          acc[b][2 * e + 1] = fmaf(a[e].y, x, acc[b][2 * e + 1]);
+        }
+      }
+    }
+    if (d0 - g + 64 < nope) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        wv[u] = d0 + 64 + 8 * u < nope ? wr[int64_t(d0 + 64 + 8 * u) * 64] : make_uint4(0, 0, 0, 0);
+    }
+  }
+  if (warp < hp.B) prep_item(p, warp, p.Hidx + 2 + h, lane);  // the rotary part of the head's query
+#pragma unroll
+  for (int b0 = 0; b0 < NB; b0 += kRound) {
+    if (b0 > 0) __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRound; ++r) {
+      float4* dst = reinterpret_cast<float4*>(s_o + (g * kRound + r) * DSA_VALUE_DIM + 8 * c);
+      dst[0] = make_float4(acc[b0 + r][0], acc[b0 + r][1], acc[b0 + r][2], acc[b0 + r][3]);
+      dst[1] = make_float4(acc[b0 + r][4], acc[b0 + r][5], acc[b0 + r][6], acc[b0 + r][7]);
+    }
+    __syncthreads();
+    for (int i = tid; i < kRound * DSA_VALUE_DIM / 2; i += kHeadThreads) {
+      const int r = i / (DSA_VALUE_DIM / 2), d = 2 * (i - r * (DSA_VALUE_DIM / 2)), b = b0 + r;
+      float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float2 t = *reinterpret_cast<const float2*>(s_o + (k * kRound + r) * DSA_VALUE_DIM + d);
+        v.x += t.x, v.y += t.y;
+      }
+      if (b < hp.B)
+        *reinterpret_cast<__nv_bfloat162*>(p.q_full + (int64_t(b) * p.H + h) * DSA_LATENT_DIM + d) = __floats2bfloat162_rn(v.x, v.y);
+    }
+  }
+}
+
+// ov[b, h, d] = sum_l W_UV[h, d, l] o[b, h, l]: four rows d per warp step, 512 columns = two vectors per lane
+// and row; the sums of the four rows and NB tokens are transposed into the lanes while they are reduced.
+template <int NB>
+__global__ void __launch_bounds__(kHeadThreads, NB == 1 ? 2 : 1)
+value_project_kernel(const HeadParams hp) {
+  __shared__ uint4 s_o[NB][64];
+  const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, v_dim = hp.v_dim;
+  const uint4* wr = reinterpret_cast<const uint4*>(hp.kv_b + (int64_t(h) * (hp.nope + v_dim) + hp.nope) * DSA_VALUE_DIM) + lane;
+  uint4 wv[4][2];
+  auto load = [&](int d) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) wv[u][j] = d + u < v_dim ? wr[int64_t(d + u) * 64 + 32 * j] : make_uint4(0, 0, 0, 0);
+  };
+  load(4 * warp);
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int i = tid; i < NB * 64; i += kHeadThreads) {
+    const int b = i >> 6;
+    s_o[b][i & 63] = b < hp.B ? reinterpret_cast<const uint4*>(hp.q + (int64_t(b) * hp.o_heads + h) * DSA_VALUE_DIM)[i & 63] : make_uint4(0, 0, 0, 0);
+  }
+  __syncthreads();
+  constexpr int kTokens = NB < 4 ? NB : 4, kSums = 4 * kTokens, kLanes = 32 / kSums;
+  for (int d = 4 * warp; d < v_dim; d += 4 * (kHeadThreads / 32)) {
+#pragma unroll 1
+    for (int b0 = 0; b0 < NB; b0 += kTokens) {
+      float acc[kSums];  // [token][row]
+#pragma unroll
+      for (int i = 0; i < kSums; ++i) acc[i] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        uint4 xv[kTokens];
+#pragma unroll
+        for (int b = 0; b < kTokens; ++b) xv[b] = s_o[b0 + b][lane + 32 * j];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float2 a[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) a[u] = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&wv[u][j])[e]);
+#pragma unroll
+          for (int b = 0; b < kTokens; ++b) {
+            const float2 x = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&xv[b])[e]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              acc[b * 4 + u] = fmaf(a[u].x, x.x, acc[b * 4 + u]);
+              acc[b * 4 + u] = fmaf(a[u].y, x.y, acc[b * 4 + u]);
+            }
+          }
+        }
+      }
+      if (b0 + kTokens == NB && d + 4 * (kHeadThreads / 32) < v_dim) load(d + 4 * (kHeadThreads / 32));
+#pragma unroll
+      for (int n = kSums / 2, o = 16; n >= 1; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          const float give = up ? acc[i] : acc[i + n], keep = up ? acc[i + n] : acc[i];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      }
+#pragma unroll
+      for (int w = kLanes / 2; w >= 1; w >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], w);  // (kLanes lanes hold parts of one sum)
+      const int i = lane / kLanes, b = b0 + (i >> 2), row = d + (i & 3);
+      if (lane % kLanes == 0 && b < hp.B && row < v_dim) hp.out[(int64_t(b) * hp.H + h) * v_dim + row] = __float2bfloat16_rn(acc[0]);
+    }
   }
 }
 

@@ -1184,25 +1184,33 @@ int dsa_gemv_swiglu_bf16(const void* w_gate, const void* w_up, const void* x, vo
   return rc == 1 ? fail(DSA_ERR_UNSUPPORTED, "gemv + SwiGLU: [%d, %d] is outside the streaming kernel's range", n, k) : rc;
 }
 
-int dsa_absorb_query(const void* kv_b, const void* q, void* q_full, int B, int H, int nope, int per_head, int64_t q_row_stride,
-                     int64_t q_head_stride, void* stream) {
-  DSA_REQUIRE(kv_b && q && q_full, "absorb query: null pointer");
-  DSA_REQUIRE(aligned16(kv_b) && aligned16(q_full), "absorb query: pointers must be 16-byte aligned");
-  DSA_REQUIRE(B > 0 && B <= 65535 && H > 0 && nope > 0 && nope <= 512 && per_head >= nope, "absorb query: bad shape");
-  DSA_CUDA(launch_pdl(prep::absorb_query_kernel, dim3(H, B), dim3(prep::kHeadThreads), 0, static_cast<cudaStream_t>(stream),
-                      static_cast<const __nv_bfloat16*>(kv_b), static_cast<const __nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(q_full),
-                      H, nope, per_head, q_row_stride, q_head_stride));
+// NB: the tokens whose products share one reading of the weights, 1, 2, 4 or 8.
+extern "C++" {
+template <int NB>
+static int launch_decode_token(const prep::Params& p, const prep::HeadParams& hp, cudaStream_t st) {
+  const int items = (p.Hidx + 2) * p.B, warps = prep::kHeadThreads / 32;
+  const size_t smem = (size_t(NB) * prep::kHeadMaxNope + 8 * (NB <= 2 ? NB : 2) * DSA_VALUE_DIM) * 4;
+  DSA_CUDA(launch_pdl(prep::decode_token_kernel<NB>, dim3(p.H + (items + warps - 1) / warps), dim3(prep::kHeadThreads), smem, st, p, hp));
   return DSA_OK;
 }
+template <int NB>
+static int launch_value_project(const prep::HeadParams& hp, cudaStream_t st) {
+  DSA_CUDA(launch_pdl(prep::value_project_kernel<NB>, dim3(hp.H), dim3(prep::kHeadThreads), 0, st, hp));
+  return DSA_OK;
+}
+}  // extern "C++"
 
-int dsa_value_project(const void* kv_b, const void* o, void* ov, int B, int H, int o_heads, int per_head, int v_dim, void* stream) {
+int dsa_value_project(const void* kv_b, const void* o, void* ov, int B, int H, int o_heads, int nope, int v_dim, void* stream) {
   DSA_REQUIRE(kv_b && o && ov, "value projection: null pointer");
   DSA_REQUIRE(aligned16(kv_b) && aligned16(o), "value projection: pointers must be 16-byte aligned");
-  DSA_REQUIRE(B > 0 && B <= 65535 && H > 0 && o_heads >= H && v_dim > 0 && per_head >= v_dim, "value projection: bad shape");
-  DSA_CUDA(launch_pdl(prep::value_project_kernel, dim3(H, B), dim3(prep::kHeadThreads), 0, static_cast<cudaStream_t>(stream),
-                      static_cast<const __nv_bfloat16*>(kv_b), static_cast<const __nv_bfloat16*>(o), static_cast<__nv_bfloat16*>(ov), H,
-                      o_heads, per_head, v_dim));
-  return DSA_OK;
+  DSA_REQUIRE(B > 0 && B <= prep::kHeadMaxTokens && H > 0 && o_heads >= H && v_dim > 0 && nope >= 0,
+              "value projection: bad shape (at most %d tokens)", prep::kHeadMaxTokens);
+  prep::HeadParams hp{};
+  hp.kv_b = static_cast<const __nv_bfloat16*>(kv_b), hp.q = static_cast<const __nv_bfloat16*>(o), hp.out = static_cast<__nv_bfloat16*>(ov);
+  hp.nope = nope, hp.v_dim = v_dim, hp.H = H, hp.B = B, hp.o_heads = o_heads;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return B == 1 ? launch_value_project<1>(hp, st) : B == 2 ? launch_value_project<2>(hp, st)
+         : B <= 4 ? launch_value_project<4>(hp, st) : launch_value_project<8>(hp, st);
 }
 
 int dsa_silu_mul_bf16(const void* gate, const void* up, void* out, int64_t n, void* stream) {
@@ -1340,10 +1348,46 @@ int dsa_decode_prep(const void* iq_raw, const void* w_raw, const void* ik_raw, c
   p.Hidx = n_index_heads;
   p.interleave = interleave;
   p.eps = eps;
+  p.iq_row = int64_t(n_index_heads) * 128, p.w_row = n_index_heads, p.ik_row = 128, p.kva_row = 576, p.q_row = H * q_pe_stride;
   const int items = n_index_heads + 2 + H;
   DSA_CUDA(launch_pdl(prep::decode_prep_kernel, dim3((items + 3) / 4, B), dim3(128), 0,
                       static_cast<cudaStream_t>(stream), p));
   return DSA_OK;
+}
+
+int dsa_decode_token(const void* iq_raw, int64_t iq_stride, const void* w_raw, int64_t w_stride, const void* ik_raw, int64_t ik_stride,
+                     const void* kv_a, int64_t kv_a_stride, const void* q, int64_t q_stride, const void* kv_b, const void* kv_norm_w,
+                     const void* mla_cos, const void* mla_sin, const void* idx_cos, const void* idx_sin, const int64_t* positions,
+                     uint8_t* index_q, float* index_w, void* q_full, uint8_t* cache_index_k, float* cache_k_scale, void* cache_kv, int B,
+                     int H, int nope, int v_dim, int n_index_heads, int64_t cap, int interleave, float eps, void* stream) {
+  DSA_REQUIRE(iq_raw && w_raw && ik_raw && kv_a && q && kv_b && kv_norm_w && mla_cos && mla_sin && idx_cos && idx_sin && positions &&
+                  index_q && index_w && q_full && cache_index_k && cache_k_scale && cache_kv,
+              "decode token: null pointer");
+  DSA_REQUIRE(aligned16(kv_b) && aligned16(q_full) && aligned16(index_q) && aligned16(cache_index_k) && aligned16(cache_kv) &&
+                  reinterpret_cast<uintptr_t>(iq_raw) % 8 == 0 && reinterpret_cast<uintptr_t>(ik_raw) % 8 == 0 &&
+                  iq_stride % 4 == 0 && ik_stride % 4 == 0,
+              "decode token: outputs and kv_b must be 16-byte aligned, index queries and keys 8-byte aligned");
+  DSA_REQUIRE(B > 0 && B <= prep::kHeadMaxTokens && H > 0 && n_index_heads > 0 && cap > 0 && nope > 0 && nope <= prep::kHeadMaxNope && v_dim > 0,
+              "decode token: bad shape (at most %d tokens, nope <= %d)", prep::kHeadMaxTokens, prep::kHeadMaxNope);
+  prep::Params p{};
+  p.iq_raw = static_cast<const __nv_bfloat16*>(iq_raw), p.iq_row = iq_stride;
+  p.w_raw = static_cast<const __nv_bfloat16*>(w_raw), p.w_row = w_stride;
+  p.ik_raw = static_cast<const __nv_bfloat16*>(ik_raw), p.ik_row = ik_stride;
+  p.kv_a = static_cast<const __nv_bfloat16*>(kv_a), p.kva_row = kv_a_stride;
+  p.q_pe = static_cast<const __nv_bfloat16*>(q) + nope, p.q_row = q_stride, p.q_pe_stride = nope + 64;
+  p.kv_norm_w = static_cast<const __nv_bfloat16*>(kv_norm_w);
+  p.mla_cos = static_cast<const __nv_bfloat16*>(mla_cos), p.mla_sin = static_cast<const __nv_bfloat16*>(mla_sin);
+  p.idx_cos = static_cast<const __nv_bfloat16*>(idx_cos), p.idx_sin = static_cast<const __nv_bfloat16*>(idx_sin);
+  p.positions = positions;
+  p.index_q = index_q, p.index_w = index_w, p.q_full = static_cast<__nv_bfloat16*>(q_full);
+  p.cache_index_k = cache_index_k, p.cache_k_scale = cache_k_scale, p.cache_kv = static_cast<__nv_bfloat16*>(cache_kv);
+  p.cap = cap, p.B = B, p.H = H, p.Hidx = n_index_heads, p.interleave = interleave, p.eps = eps;
+  prep::HeadParams hp{};
+  hp.kv_b = static_cast<const __nv_bfloat16*>(kv_b), hp.q = static_cast<const __nv_bfloat16*>(q), hp.q_row = q_stride, hp.q_head = nope + 64;
+  hp.nope = nope, hp.v_dim = v_dim, hp.H = H, hp.B = B;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return B == 1 ? launch_decode_token<1>(p, hp, st) : B == 2 ? launch_decode_token<2>(p, hp, st)
+         : B <= 4 ? launch_decode_token<4>(p, hp, st) : launch_decode_token<8>(p, hp, st);
 }
 
 // ------------------------------------------------------------------ full-sequence preparation

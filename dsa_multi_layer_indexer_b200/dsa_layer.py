@@ -422,6 +422,13 @@ class DSALayer(nn.Module):
             return m(x)
         return ops.gemv(x, m.weight)
 
+    def _absorbed_rows(self, x: torch.Tensor) -> bool:
+        """Whether a decode batch takes the kernels that read kv_b_proj's weight in place (one reading for all
+        tokens; beyond HEAD_TOKENS rows the products are GEMMs)."""
+        c, w = self.config, self.kv_b_proj.weight
+        return (x.shape[0] <= ops.HEAD_TOKENS and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_contiguous()
+                and c.qk_nope_head_dim <= 512 and c.qk_nope_head_dim % 8 == 0 and c.q_lora_rank % 8 == 0 and not torch.is_grad_enabled())
+
     def new_cache(self, n_seq: int, capacity: int, device, fp8: bool) -> LayerDecodeCache:
         c = self.config
         if fp8:
@@ -463,31 +470,31 @@ class DSALayer(nn.Module):
             q, iq_raw, w = (ops.gemv(c_q, self._wc) if wide else torch.nn.functional.linear(c_q, self._wc)).split(
                 [h * (c.qk_nope_head_dim + c.qk_rope_head_dim), c.index_n_heads * c.index_head_dim, c.index_n_heads],
                 dim=-1)
-            # (rows of a batch must be dense for the fused prep launch; one row already is)
-            q = (q if b == 1 else q.contiguous()).reshape(b, h, c.qk_nope_head_dim + c.qk_rope_head_dim)
-            iq_raw = iq_raw.reshape(b, c.index_n_heads, c.index_head_dim)
         else:
             c_q = self.q_latent(x_norm)
-            q = self.q_b_proj(c_q).view(b, h, c.qk_nope_head_dim + c.qk_rope_head_dim)
+            q = self.q_b_proj(c_q)
             kv_a = self.kv_a_proj(x_norm)
-            iq_raw = self.index_q_proj(c_q).view(b, c.index_n_heads, c.index_head_dim)
+            iq_raw = self.index_q_proj(c_q)
             ik_raw = self.index_k_proj(x_norm)
             w = self.index_weights_proj(c_q)
-        q_nope, q_rope = q.split([c.qk_nope_head_dim, c.qk_rope_head_dim], dim=-1)
         fused = cache.k_scale is not None and x_norm.dtype == torch.bfloat16
-        if fused and b <= 2 and c.qk_nope_head_dim <= 512 and not torch.is_grad_enabled():
-            q_abs = None  # absorbed straight into the first columns of the query below
-        else:
-            w_uk, _ = self._w_uk_uv()
-            q_abs = torch.einsum("bhd,hdl->bhl", q_nope, w_uk)
-        if cache.k_scale is not None and x_norm.dtype == torch.bfloat16:
+        if fused:
             index_q = torch.empty(b, c.index_n_heads, c.index_head_dim, dtype=torch.uint8, device=x_norm.device)
             index_w = torch.empty(b, c.index_n_heads, dtype=torch.float32, device=x_norm.device)
             q_full = torch.empty(b, h, c.qk_head_dim, dtype=torch.bfloat16, device=x_norm.device)
-            if q_abs is None:
-                ops.absorb_query(self.kv_b_proj.weight, q, c.qk_nope_head_dim, q_full)
+            if self._absorbed_rows(x_norm):
+                ops.decode_token(iq_raw, w, ik_raw, kv_a, q, self.kv_b_proj.weight, self.kv_a_layernorm.weight, rope.mla_cos,
+                                 rope.mla_sin, rope.idx_cos, rope.idx_sin, positions, index_q, index_w, q_full, cache.index_k,
+                                 cache.k_scale, cache.kv, il, c.rms_norm_eps)
+                return q_full, index_q, index_w
+        q = q.reshape(b, h, c.qk_nope_head_dim + c.qk_rope_head_dim)
+        iq_raw = iq_raw.reshape(b, c.index_n_heads, c.index_head_dim)
+        q_nope, q_rope = q.split([c.qk_nope_head_dim, c.qk_rope_head_dim], dim=-1)
+        w_uk, _ = self._w_uk_uv()
+        q_abs = torch.einsum("bhd,hdl->bhl", q_nope, w_uk)
+        if fused:
             ops.decode_prep(iq_raw.contiguous(), w.contiguous(), ik_raw.contiguous(), kv_a.contiguous(),
-                            None if q_abs is None else q_abs.contiguous(), q_rope, self.kv_a_layernorm.weight, rope.mla_cos, rope.mla_sin,
+                            q_abs.contiguous(), q_rope, self.kv_a_layernorm.weight, rope.mla_cos, rope.mla_sin,
                             rope.idx_cos, rope.idx_sin, positions, index_q, index_w, q_full, cache.index_k,
                             cache.k_scale, cache.kv, il, c.rms_norm_eps)
             return q_full, index_q, index_w
@@ -541,7 +548,7 @@ class DSALayer(nn.Module):
             direct = q.dtype == torch.bfloat16 and h % ops.HEAD_BLOCK == 0 and q.is_contiguous()
             o = ops.sparse_mla_decode(_pad_heads(q.to(torch.bfloat16), ops.HEAD_BLOCK).contiguous(), cache.kv,
                                       indices, self.sm_scale, seq_lens, beside_previous=beside_previous and direct)
-            if q.dtype == torch.bfloat16 and q.shape[0] <= 2 and not torch.is_grad_enabled():
+            if self._absorbed_rows(q):
                 ov = ops.value_project(self.kv_b_proj.weight, o, h, c.v_head_dim)
                 return self._reduced(self._skinny("o_proj", ov.view(ov.shape[0], h * c.v_head_dim)))
             o = o[:, :h].to(q.dtype)

@@ -398,30 +398,49 @@ def gemv_swiglu(x: torch.Tensor, gate: torch.Tensor, up: torch.Tensor) -> torch.
     return y
 
 
-def absorb_query(kv_b: torch.Tensor, q: torch.Tensor, nope: int, q_full: torch.Tensor) -> None:
-    """Columns [0, 512) of ``q_full`` ``[B, H, 576]`` = ``q[b, h, :nope]`` through W_UK, the first ``nope`` rows
-    of every head of ``kv_b`` ``[H * per_head, 512]``; ``q`` ``[B, H, >= nope]`` may be a strided view."""
-    B, H = q.shape[0], q.shape[1]
-    _need(q.is_cuda and q.dtype == torch.bfloat16 and q.dim() == 3 and q.stride(2) == 1 and q.shape[2] >= nope, "q must be bf16 [B, H, >= nope]")
-    _cuda_contig(kv_b, "kv_b", (torch.bfloat16,))
-    _cuda_contig(q_full, "q_full", (torch.bfloat16,))
-    _need(kv_b.dim() == 2 and kv_b.shape[1] == VALUE_DIM and kv_b.shape[0] % H == 0 and tuple(q_full.shape) == (B, H, LATENT_DIM),
-          "kv_b must be [H * per_head, 512], q_full [B, H, 576]")
-    _lib.check(_lib.lib().dsa_absorb_query(_ptr(kv_b), _ptr(q), _ptr(q_full), B, H, nope, kv_b.shape[0] // H, q.stride(0), q.stride(1),
-                                           _stream()))
+HEAD_TOKENS = 8  # tokens that share one reading of kv_b_proj's weight in decode_token / value_project
 
 
 def value_project(kv_b: torch.Tensor, o: torch.Tensor, heads: int, v_dim: int) -> torch.Tensor:
     """``[B, heads, v_dim]``: every head's latent output ``o`` ``[B, >= heads, 512]`` through W_UV, the last
-    ``v_dim`` rows of the head's part of ``kv_b`` ``[heads * per_head, 512]``."""
+    ``v_dim`` rows of the head's part of ``kv_b`` ``[heads * per_head, 512]``; at most HEAD_TOKENS rows."""
     _cuda_contig(kv_b, "kv_b", (torch.bfloat16,))
     _cuda_contig(o, "o", (torch.bfloat16,))
     _need(o.dim() == 3 and o.shape[2] == VALUE_DIM and o.shape[1] >= heads and kv_b.dim() == 2 and kv_b.shape[1] == VALUE_DIM
-          and kv_b.shape[0] % heads == 0, "kv_b must be [heads * per_head, 512], o [B, >= heads, 512]")
+          and kv_b.shape[0] % heads == 0 and kv_b.shape[0] // heads >= v_dim,
+          "kv_b must be [heads * per_head, 512], o [B, >= heads, 512]")
     ov = torch.empty(o.shape[0], heads, v_dim, dtype=torch.bfloat16, device=o.device)
-    _lib.check(_lib.lib().dsa_value_project(_ptr(kv_b), _ptr(o), _ptr(ov), o.shape[0], heads, o.shape[1], kv_b.shape[0] // heads, v_dim,
-                                            _stream()))
+    _lib.check(_lib.lib().dsa_value_project(_ptr(kv_b), _ptr(o), _ptr(ov), o.shape[0], heads, o.shape[1],
+                                            kv_b.shape[0] // heads - v_dim, v_dim, _stream()))
     return ov
+
+
+def decode_token(iq_raw, w_raw, ik_raw, kv_a, q, kv_b, kv_norm_w, mla_cos, mla_sin, idx_cos, idx_sin, positions, index_q,
+                 index_w, q_full, cache_index_k, cache_k_scale, cache_kv, interleave: bool, eps: float) -> None:
+    """:func:`decode_prep` for at most HEAD_TOKENS tokens with the query's absorption in the launch: ``q``
+    ``[B, H * (nope + 64)]`` and ``kv_b`` ``[H * per_head, 512]`` instead of ``q_abs`` and ``q_pe``. The five
+    inputs are 2-D and may be column ranges of a stacked projection's output (see ``dsa_decode_token``)."""
+    B, H = q_full.shape[0], q_full.shape[1]
+    n_idx = index_w.shape[1]
+    per_head = kv_b.shape[0] // H
+    nope = q.shape[1] // H - 64
+    for t, n, width in ((iq_raw, "iq_raw", n_idx * INDEX_DIM), (w_raw, "w_raw", n_idx), (ik_raw, "ik_raw", INDEX_DIM),
+                        (kv_a, "kv_a", LATENT_DIM), (q, "q", H * (nope + 64))):
+        _need(t.is_cuda and t.dtype == torch.bfloat16 and tuple(t.shape) == (B, width) and t.stride(1) == 1,
+              f"{n} must be a CUDA bf16 [B, {width}] tensor with dense rows")
+    for t, n in ((kv_b, "kv_b"), (q_full, "q_full"), (kv_norm_w, "kv_norm_w"), (mla_cos, "mla_cos"), (mla_sin, "mla_sin"),
+                 (idx_cos, "idx_cos"), (idx_sin, "idx_sin")):
+        _cuda_contig(t, n, (torch.bfloat16,))
+    _cuda_contig(positions, "positions", (torch.int64,))
+    _need(q_full.shape[2] == LATENT_DIM and kv_b.shape[1] == VALUE_DIM and kv_b.shape[0] == H * per_head and per_head > nope > 0,
+          "kv_b must be [H * (nope + v), 512], q [B, H * (nope + 64)], q_full [B, H, 576]")
+    cap = cache_kv.shape[1]
+    _need(cache_kv.shape[0] == B and cache_index_k.shape[:2] == (B, cap), "caches must be [B, cap, ...]")
+    _lib.check(_lib.lib().dsa_decode_token(
+        _ptr(iq_raw), iq_raw.stride(0), _ptr(w_raw), w_raw.stride(0), _ptr(ik_raw), ik_raw.stride(0), _ptr(kv_a), kv_a.stride(0),
+        _ptr(q), q.stride(0), _ptr(kv_b), _ptr(kv_norm_w), _ptr(mla_cos), _ptr(mla_sin), _ptr(idx_cos), _ptr(idx_sin),
+        _ptr(positions), _ptr(index_q), _ptr(index_w), _ptr(q_full), _ptr(cache_index_k), _ptr(cache_k_scale), _ptr(cache_kv),
+        B, H, nope, per_head - nope, n_idx, cap, 1 if interleave else 0, float(eps), _stream()))
 
 
 def indexer_stage_fp8(q_raw, k_raw, w_raw, k_norm_weight, k_norm_bias, k_norm_eps: float, rope_cos, rope_sin,
@@ -460,20 +479,17 @@ def decode_prep(iq_raw, w_raw, ik_raw, kv_a, q_abs, q_pe, kv_norm_w, mla_cos, ml
     """One launch for the chain between the projection GEMVs and the hot path
     (see ``dsa_decode_prep`` in the header). All operands bf16 CUDA tensors;
     ``q_pe`` may be a strided view ``q[..., nope:]`` of the q_b_proj output."""
-    for t, n in ((iq_raw, "iq_raw"), (w_raw, "w_raw"), (ik_raw, "ik_raw"), (kv_a, "kv_a"), (q_full, "q_full"),
+    for t, n in ((iq_raw, "iq_raw"), (w_raw, "w_raw"), (ik_raw, "ik_raw"), (kv_a, "kv_a"), (q_abs, "q_abs"),
                  (kv_norm_w, "kv_norm_w"), (mla_cos, "mla_cos"), (mla_sin, "mla_sin"), (idx_cos, "idx_cos"),
                  (idx_sin, "idx_sin")):
         _cuda_contig(t, n, (torch.bfloat16,))
-    if q_abs is not None:  # (None: those columns of q_full are filled already)
-        _cuda_contig(q_abs, "q_abs", (torch.bfloat16,))
-        _need(q_abs.shape[2] == VALUE_DIM, "q_abs must be [B, H, 512]")
     _need(q_pe.dtype == torch.bfloat16 and q_pe.dim() == 3 and q_pe.shape[2] == 64 and q_pe.stride(2) == 1
           and (q_pe.shape[0] == 1 or q_pe.stride(0) == q_pe.shape[1] * q_pe.stride(1)),
           "q_pe must be a [B, H, 64] bf16 view with dense rows")
     _cuda_contig(positions, "positions", (torch.int64,))
     B, n_idx = iq_raw.shape[0], iq_raw.shape[1]
-    H = q_full.shape[1]
-    _need(iq_raw.shape[2] == INDEX_DIM and kv_a.shape[-1] == LATENT_DIM and q_full.shape[2] == LATENT_DIM,
+    H = q_abs.shape[1]
+    _need(iq_raw.shape[2] == INDEX_DIM and kv_a.shape[-1] == LATENT_DIM and q_abs.shape[2] == VALUE_DIM,
           "decode prep needs the production geometry")
     cap = cache_kv.shape[1]
     _need(cache_kv.shape[0] == B and cache_index_k.shape[:2] == (B, cap), "caches must be [B, cap, ...]")

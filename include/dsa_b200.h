@@ -347,7 +347,7 @@ int dsa_sparse_mla_f32(const float* q, const float* kv, const int32_t* indices,
  *     index_w = q_scale * w_raw;
  *   - the token's index key: RoPE, e4m3 + scale, written at cache row positions[b];
  *   - the token's latent row: RMSNorm(512) | RoPE(64), written at positions[b];
- *   - the absorbed query: q_full = [q_abs | RoPE(q_pe)] (q_abs NULL: those columns are there already).
+ *   - the absorbed query: q_full = [q_abs | RoPE(q_pe)].
  * All inputs bf16 ([B,Hidx,128], [B,Hidx], [B,128], [B,576], [B,H,512],
  * [B,H,64] with row stride q_pe_stride elements); rotary tables bf16
  * [cap,64] / [cap,128]; caches as in dsa_indexer_scan_fp8 / dsa_sparse_mla_*. */
@@ -407,13 +407,10 @@ int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k
                   int64_t y_stride, void* stream);
 int dsa_gemv_swiglu_bf16(const void* w_gate, const void* w_up, const void* x, void* y, int batch, int n, int k,
                          int64_t x_stride, int64_t y_stride, void* stream);
-/* The per-head products of a decode token with kv_b_proj's weight [H, per_head, 512] (per_head = nope +
- * v_dim, bf16, src/lagged_indexer_dsa/dsa_layer.py:96-125), read like the weights of dsa_gemv_bf16:
- * dsa_absorb_query: columns [0, 512) of q_full [B, H, 576] = q[b, h, 0:nope] W_UK[h] (element strides given);
- * dsa_value_project: ov [B, H, v_dim] = W_UV[h] o[b, h, :], o [B, o_heads, 512]. */
-int dsa_absorb_query(const void* kv_b, const void* q, void* q_full, int B, int H, int nope, int per_head,
-                     int64_t q_row_stride, int64_t q_head_stride, void* stream);
-int dsa_value_project(const void* kv_b, const void* o, void* ov, int B, int H, int o_heads, int per_head,
+/* ov [B, H, v_dim] = W_UV[h] o[b, h, :] with kv_b_proj's weight kv_b [H, nope + v_dim, 512] (bf16,
+ * src/lagged_indexer_dsa/dsa_layer.py:118-125), o [B, o_heads, 512], 1..8 tokens. kv_b is read like the
+ * weights of dsa_gemv_bf16. */
+int dsa_value_project(const void* kv_b, const void* o, void* ov, int B, int H, int o_heads, int nope,
                       int v_dim, void* stream);
 /* out = silu(gate) * up over n bf16 elements: the SwiGLU between the MLP's GEMVs
  * (src/lagged_indexer_dsa/dsa_layer.py:194-196), rounded as the two separate operations. */
@@ -427,6 +424,17 @@ int dsa_decode_prep(const void* iq_raw, const void* w_raw, const void* ik_raw, c
                     uint8_t* cache_index_k, float* cache_k_scale, void* cache_kv,
                     int B, int H, int n_index_heads, int64_t cap, int interleave, float eps,
                     void* stream);
+/* The same for 1..8 tokens with the absorption of the query in the launch: q [B] rows of H heads of
+ * [nope | 64], q_full[b, h, 0:512] = q[b, h, 0:nope] W_UK[h] with kv_b as in dsa_value_project (read ahead
+ * of the kernel in front, as there). The inputs' rows may be strided (elements between tokens), so the
+ * outputs of stacked projections need no copies. */
+int dsa_decode_token(const void* iq_raw, int64_t iq_stride, const void* w_raw, int64_t w_stride,
+                     const void* ik_raw, int64_t ik_stride, const void* kv_a, int64_t kv_a_stride,
+                     const void* q, int64_t q_stride, const void* kv_b, const void* kv_norm_w,
+                     const void* mla_cos, const void* mla_sin, const void* idx_cos, const void* idx_sin,
+                     const int64_t* positions, uint8_t* index_q, float* index_w, void* q_full,
+                     uint8_t* cache_index_k, float* cache_k_scale, void* cache_kv, int B, int H, int nope,
+                     int v_dim, int n_index_heads, int64_t cap, int interleave, float eps, void* stream);
 
 /* Serving-form indexer staging: what the serving model's indexer does to the new
  * token between its projection GEMVs and the scan

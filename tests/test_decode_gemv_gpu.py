@@ -47,18 +47,36 @@ def test_gemv_and_swiglu(ops, b, n, k):
     assert torch.equal(ops.gemv(view, w), ops.gemv(view.contiguous(), w))
 
 
-@pytest.mark.parametrize("B,H,nope,v,pad", [(1, 128, 128, 128, 0), (2, 64, 192, 256, 0), (1, 5, 33, 7, 11), (2, 16, 512, 32, 0)])
+# one to eight tokens, remainders of the row groups (nope) and of the rows per warp step (v), padded heads
+@pytest.mark.parametrize("B,H,nope,v,pad", [(1, 128, 128, 128, 0), (2, 64, 192, 256, 0), (3, 5, 36, 7, 11), (8, 16, 512, 66, 0), (5, 8, 64, 128, 0)])
 def test_absorbed_projections(ops, B, H, nope, v, pad):
     torch.manual_seed(H + nope)
-    kv_b = torch.randn(H * (nope + v), 512, device="cuda").div_(16).to(torch.bfloat16)
-    q = torch.randn(B, H, nope + 64, device="cuda").to(torch.bfloat16)
-    q_full = torch.full((B, H, 576), 3.0, dtype=torch.bfloat16, device="cuda")
-    ops.absorb_query(kv_b, q, nope, q_full)
-    w = kv_b.view(H, nope + v, 512).double()
-    ref = torch.einsum("bhd,hdl->bhl", q[..., :nope].double(), w[:, :nope])
-    close(q_full[..., :512], ref, torch.einsum("bhd,hdl->bhl", q[..., :nope].double().abs(), w[:, :nope].abs()))
-    assert float((q_full[..., 512:].float() - 3.0).abs().max()) == 0.0
-    o = torch.randn(B, H + pad, 512, device="cuda").to(torch.bfloat16)
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    kv_b = bf(H * (nope + v), 512).div_(16)
+    n_idx, cap, d = 64, 40, H * (nope + 64)
+    yc, ya = bf(B, d + n_idx * 129), bf(B, 16 + 576 + 128)  # stacked projections; their ranges are strided
+    q, iq, w = yc.split([d, n_idx * 128, n_idx], dim=-1)
+    _, kv_a, ik = ya.split([16, 576, 128], dim=-1)
+    tab = [torch.rand(cap, n, device="cuda").to(torch.bfloat16) for n in (64, 64, 128, 128)]
+    pos = torch.randint(0, cap, (B,), device="cuda")
+    norm_w = bf(512)
+
+    def outputs():
+        return (torch.zeros(B, n_idx, 128, dtype=torch.uint8, device="cuda"), torch.zeros(B, n_idx, device="cuda"),
+                torch.zeros(B, H, 576, dtype=torch.bfloat16, device="cuda"), torch.zeros(B, cap, 128, dtype=torch.uint8, device="cuda"),
+                torch.zeros(B, cap, device="cuda"), torch.zeros(B, cap, 576, dtype=torch.bfloat16, device="cuda"))
+
+    got, want = outputs(), outputs()
+    ops.decode_token(iq, w, ik, kv_a, q, kv_b, norm_w, *tab, pos, *got, False, 1e-6)
+    q3 = q.reshape(B, H, nope + 64).contiguous()
+    weight = kv_b.view(H, nope + v, 512).double()
+    ref = torch.einsum("bhd,hdl->bhl", q3[..., :nope].double(), weight[:, :nope])
+    close(got[2][..., :512], ref, torch.einsum("bhd,hdl->bhl", q3[..., :nope].double().abs(), weight[:, :nope].abs()))
+    # everything else: the launch that takes the absorbed query, bit for bit
+    ops.decode_prep(iq.reshape(B, n_idx, 128).contiguous(), w.contiguous(), ik.contiguous(), kv_a.contiguous(),
+                    got[2][..., :512].contiguous(), q3[..., nope:], norm_w, *tab, pos, *want, False, 1e-6)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    o = bf(B, H + pad, 512)
     ov = ops.value_project(kv_b, o, H, v)
-    ref = torch.einsum("bhl,hdl->bhd", o[:, :H].double(), w[:, nope:])
-    close(ov, ref, torch.einsum("bhl,hdl->bhd", o[:, :H].double().abs(), w[:, nope:].abs()))
+    ref = torch.einsum("bhl,hdl->bhd", o[:, :H].double(), weight[:, nope:])
+    close(ov, ref, torch.einsum("bhl,hdl->bhd", o[:, :H].double().abs(), weight[:, nope:].abs()))
