@@ -59,6 +59,7 @@ SIGNATURES: Dict[str, Tuple[object, List[object]]] = {
     "dsa_silu_mul_bf16": (_i, [_p, _p, _p, _l, _p]),
     "dsa_gemv_bf16": (_i, [_p, _p, _p, _i, _i, _i, _l, _l, _p]),
     "dsa_gemv_swiglu_bf16": (_i, [_p, _p, _p, _p, _i, _i, _i, _l, _l, _p]),
+    "dsa_norm_gemv_bf16": (_i, [_p, _p, _p, _p, _p, _f, _p, _p, _i, _i, _i, _l, _l, _p]),
     "dsa_value_project": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _p]),
     "dsa_copy_bytes": (_i, [_p, _p, _l, _p]),
     "dsa_copy_bytes_beside": (_i, [_p, _p, _l, _p]),

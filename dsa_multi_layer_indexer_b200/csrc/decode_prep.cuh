@@ -284,6 +284,7 @@ constexpr int kGemvThreads = 256;
 constexpr int kGemvLoads = 8;        // gemv_rows_kernel: independent 16-byte weight loads per lane
 constexpr int kGemvChunks = 128;  // 16-byte chunks of a row in one piece, at most
 constexpr int kGemvWarps = 16;
+constexpr int kGemvNormVecs = 2;      // 16-byte vectors per thread of a row that is normed: k <= 8192
 constexpr int kGemvMaxSlots = 4;     // pieces in flight per warp
 constexpr int kGemvRing = 160 << 10;  // bytes in flight per CTA, at most (and at least two pieces per warp)
 struct GemvParams {
@@ -291,7 +292,12 @@ struct GemvParams {
   const __nv_bfloat16* w2;
   const __nv_bfloat16* x;
   __nv_bfloat16* y;
-  int n, k, slots, ks, chunks;  // ks pieces of up to `chunks` 16-byte chunks per row
+  // x staged as rmsnorm(x + delta) * norm_w where norm_w is given (delta may be null; CTA 0 writes the sum)
+  const __nv_bfloat16* delta;
+  const __nv_bfloat16* norm_w;
+  __nv_bfloat16* sum_out;
+  float eps;
+  int rows, n, k, slots, ks, chunks;  // rows <= B of x; ks pieces of up to `chunks` 16-byte chunks per row
   int64_t x_stride, y_stride;
 };
 // shared memory: ring [warps][slots][2][chunks] | x [B][k] | sums [units of a CTA][ks][2][B]
@@ -300,6 +306,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, B == 1 ? 2 : 1)
 gemv_stream_kernel(const GemvParams p) {
   extern __shared__ __align__(128) uint8_t gemv_smem[];
   __shared__ uint64_t s_full[kGemvWarps * kGemvMaxSlots];
+  __shared__ float s_sq[kGemvWarps][B];
   __shared__ int s_abort;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int kv = p.k >> 3, ks = p.ks, pl = p.chunks, slots = p.slots;
@@ -331,10 +338,76 @@ gemv_stream_kernel(const GemvParams p) {
   }
   if (tid == 0) s_abort = 0;
   for (int i = tid; i < nu * ks * 2 * B; i += kGemvWarps * 32) s_sum[i] = 0.f;
+  uint4 nw[kGemvNormVecs];
+  if (p.norm_w) {
+#pragma unroll
+    for (int i = 0; i < kGemvNormVecs; ++i) {
+      const int c = tid + i * kGemvWarps * 32;
+      nw[i] = c < kv ? reinterpret_cast<const uint4*>(p.norm_w)[c] : make_uint4(0, 0, 0, 0);
+    }
+  }
   pdl_wait();
   pdl_launch_dependents();
-  for (int b = 0; b < B; ++b)
-    for (int c = tid; c < kv; c += kGemvWarps * 32) s_x[b * kv + c] = *reinterpret_cast<const uint4*>(p.x + b * p.x_stride + c * 8);
+  if (p.norm_w) {
+    // every CTA norms the rows for itself: they come from L2, and a launch of its own for them costs 4 us
+    float ss[B];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      ss[b] = 0.f;
+#pragma unroll
+      for (int i = 0; i < kGemvNormVecs; ++i) {
+        const int c = tid + i * kGemvWarps * 32;
+        if (c >= kv || b >= p.rows) continue;
+        uint4 v = reinterpret_cast<const uint4*>(p.x + b * p.x_stride)[c];
+        __nv_bfloat162* vp = reinterpret_cast<__nv_bfloat162*>(&v);
+        if (p.delta) {
+          const uint4 d = reinterpret_cast<const uint4*>(p.delta + int64_t(b) * p.k)[c];
+          const __nv_bfloat162* dp = reinterpret_cast<const __nv_bfloat162*>(&d);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(vp[e]), g = __bfloat1622float2(dp[e]);
+            vp[e] = __floats2bfloat162_rn(f.x + g.x, f.y + g.y);
+          }
+          if (blockIdx.x == 0) reinterpret_cast<uint4*>(p.sum_out + int64_t(b) * p.k)[c] = v;
+        }
+        s_x[b * kv + c] = v;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __bfloat1622float2(vp[e]);
+          ss[b] = fmaf(f.x, f.x, ss[b]);
+          ss[b] = fmaf(f.y, f.y, ss[b]);
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss[b] += __shfl_xor_sync(0xffffffffu, ss[b], o);
+      if (lane == 0) s_sq[warp][b] = ss[b];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      float tot = 0.f;
+#pragma unroll
+      for (int w = 0; w < kGemvWarps; ++w) tot += s_sq[w][b];
+      const float inv = rsqrtf(tot / float(p.k) + p.eps);
+#pragma unroll
+      for (int i = 0; i < kGemvNormVecs; ++i) {
+        const int c = tid + i * kGemvWarps * 32;
+        if (c >= kv) continue;
+        uint4 v = b < p.rows ? s_x[b * kv + c] : make_uint4(0, 0, 0, 0);
+        __nv_bfloat162* vp = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __bfloat1622float2(vp[e]), g = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&nw[i])[e]);
+          vp[e] = __floats2bfloat162_rn(f.x * inv * g.x, f.y * inv * g.y);
+        }
+        s_x[b * kv + c] = v;
+      }
+    }
+  } else {
+    for (int b = 0; b < B; ++b)
+      for (int c = tid; c < kv; c += kGemvWarps * 32)
+        s_x[b * kv + c] = b < p.rows ? *reinterpret_cast<const uint4*>(p.x + b * p.x_stride + c * 8) : make_uint4(0, 0, 0, 0);
+  }
   __syncthreads();
   float acc[2][B];
 #pragma unroll
@@ -348,21 +421,20 @@ gemv_stream_kernel(const GemvParams p) {
     }
     const int c0 = part * pl, len = min(pl, kv - c0);
     const uint4* wr = ring + slot * 2 * pl;
-    uint4 wv[2][4], xv[B][4];
+    uint4 wv[2][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int c = lane + 32 * i;
-      const bool in = c < len;
-      wv[0][i] = in ? wr[c] : make_uint4(0, 0, 0, 0);
-      wv[1][i] = in ? wr[pl + c] : make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int b = 0; b < B; ++b) xv[b][i] = in ? s_x[b * kv + c0 + c] : make_uint4(0, 0, 0, 0);
+      wv[0][i] = c < len ? wr[c] : make_uint4(0, 0, 0, 0);
+      wv[1][i] = c < len ? wr[pl + c] : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
+      const int c = lane + 32 * i;
 #pragma unroll
       for (int b = 0; b < B; ++b) {
-        const uint32_t xw[4] = {xv[b][i].x, xv[b][i].y, xv[b][i].z, xv[b][i].w};
+        const uint4 xv = c < len ? s_x[b * kv + c0 + c] : make_uint4(0, 0, 0, 0);
+        const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
           const uint32_t cw[4] = {wv[m][i].x, wv[m][i].y, wv[m][i].z, wv[m][i].w};
@@ -412,7 +484,7 @@ gemv_stream_kernel(const GemvParams p) {
       const float g = __bfloat162float(out), up = __bfloat162float(__float2bfloat16_rn(v2));
       out = __float2bfloat16_rn(__bfloat162float(__float2bfloat16_rn(g / (1.f + __expf(-g)))) * up);
     }
-    if (row < p.n) p.y[b * p.y_stride + row] = out;
+    if (row < p.n && b < p.rows) p.y[b * p.y_stride + row] = out;
   }
 }
 
@@ -648,9 +720,9 @@ decode_prep_kernel(const Params p) {
 // A decode token's products with kv_b_proj's weight [H][nope + v][512] (src/lagged_indexer_dsa/dsa_layer.py:
 // 96-125) for NB tokens at a time: W_UK absorbed into the query (with every other item of decode_prep_kernel
 // in the same launch, nothing of which depends on it) and W_UV applied to the attention's output.
-// Bound by the latency of reading 128 - 256 KB per head in one CTA, so what can be read before the dependency
-// wait is: the first rows into registers, the rest of W_UK into L2, and W_UV, which the step needs two dozen
-// microseconds later, into L2 after the wait, while nothing else uses the memory.
+// Bound by the latency of reading 128 - 256 KB per head in one CTA; the first 64 KB are loaded before the
+// dependency wait. (Bulk prefetches of the rest into L2, of W_UV two launches ahead, or of the first 16 - 96 MB
+// of o_proj's weight while scan and top-k leave the memory idle: nothing gained, up to 1 % lost.)
 // One token of 128 heads of 128 + 128 behind its projection: 11.9 -> 6.7 us (absorption and the other items
 // were two launches), value projection 7.5 -> 5.2 us. Four / eight tokens: with the copies of the strided
 // projection outputs that decode_prep needs, 27 -> 8 us.
@@ -664,24 +736,15 @@ struct HeadParams {
   int64_t q_row, q_head;
   int nope, v_dim, H, B, o_heads;
 };
-__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-// bytes a multiple of 16; one lane per 4 KB
-__device__ __forceinline__ void prefetch_l2_range(const char* p, int64_t bytes, int t, int threads) {
-  for (int64_t o = int64_t(t) * 4096; o < bytes; o += int64_t(threads) * 4096)
-    prefetch_l2(p + o, uint32_t(bytes - o < 4096 ? bytes - o : 4096));
-}
-
 template <int NB>
 __global__ void __launch_bounds__(kHeadThreads, NB <= 2 ? 2 : 1)
 decode_token_kernel(const Params p, const HeadParams hp) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (blockIdx.x >= unsigned(p.H)) {  // ---- a warp per indexer head, index key and latent row
-    const int i = (blockIdx.x - p.H) * (kHeadThreads / 32) + warp, b = i / (p.Hidx + 2);
+  if (blockIdx.x >= unsigned(p.H)) {  // ---- a warp per indexer head, index key, latent row and rotary query part
+    const int n = p.Hidx + 2 + p.H, i = (blockIdx.x - p.H) * (kHeadThreads / 32) + warp, b = i / n;
     pdl_wait();
     pdl_launch_dependents();
-    if (b < p.B) prep_item(p, b, i - b * (p.Hidx + 2), lane);
+    if (b < p.B) prep_item(p, b, i - b * n, lane);
     return;
   }
   // ---- head h: 64 column vectors of 8 x 8 groups of rows: thread (g, c) sums rows g, g + 8, ... of its columns
@@ -695,7 +758,6 @@ decode_token_kernel(const Params p, const HeadParams hp) {
   uint4 wv[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) wv[u] = g + 8 * u < nope ? wr[int64_t(g + 8 * u) * 64] : make_uint4(0, 0, 0, 0);
-  if (nope > 64) prefetch_l2_range(reinterpret_cast<const char*>(w_head + 64 * DSA_VALUE_DIM), int64_t(nope - 64) * DSA_VALUE_DIM * 2, tid, kHeadThreads);
   pdl_wait();
   pdl_launch_dependents();
   for (int i = tid; i < NB * nope; i += kHeadThreads) {
@@ -703,7 +765,6 @@ decode_token_kernel(const Params p, const HeadParams hp) {
     s_q[b * kHeadMaxNope + d] = b < hp.B ? __bfloat162float(hp.q[b * hp.q_row + h * hp.q_head + d]) : 0.f;
   }
   __syncthreads();
-  prefetch_l2_range(reinterpret_cast<const char*>(w_head + int64_t(nope) * DSA_VALUE_DIM), int64_t(hp.v_dim) * DSA_VALUE_DIM * 2, tid, kHeadThreads);
   float acc[NB][8];
 #pragma unroll
   for (int b = 0; b < NB; ++b)
@@ -733,7 +794,6 @@ decode_token_kernel(const Params p, const HeadParams hp) {
         wv[u] = d0 + 64 + 8 * u < nope ? wr[int64_t(d0 + 64 + 8 * u) * 64] : make_uint4(0, 0, 0, 0);
     }
   }
-  if (warp < hp.B) prep_item(p, warp, p.Hidx + 2 + h, lane);  // the rotary part of the head's query
 #pragma unroll
   for (int b0 = 0; b0 < NB; b0 += kRound) {
     if (b0 > 0) __syncthreads();

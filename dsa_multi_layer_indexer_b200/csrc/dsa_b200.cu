@@ -1101,31 +1101,38 @@ int dsa_copy_post_epoch(void* dst, const void* src, int64_t bytes, uint32_t* cou
 }
 
 extern "C++" {
-// 0: launched; 1: the shape is not for the streaming kernel (nothing is enqueued); else an error.
+// 0: launched; 1: x does not fit beside the weights' ring (nothing is enqueued); else an error.
+// (p: operands, strides, rows, n, k; the split is added here.)
 template <int B, bool kSwiglu>
-static int launch_gemv_stream(const void* w, const void* w2, const void* x, void* y, int n, int k, int64_t x_stride, int64_t y_stride,
-                              cudaStream_t st) {
-  constexpr size_t kSmem = 226 * 1024, kSums = 16 * 1024;
-  prep::GemvParams p{};
-  // the fewest pieces per row, of even length (the last one may be shorter)
-  const int kv = k / 8;
-  p.ks = (kv + prep::kGemvChunks - 1) / prep::kGemvChunks;
-  p.chunks = (kv + p.ks - 1) / p.ks;
-  p.ks = (kv + p.chunks - 1) / p.chunks;
-  // a CTA per SM; several where one CTA's table of sums would be larger than its part of shared memory
-  const int units = kSwiglu ? n : (n + 1) / 2, most = int(kSums / (size_t(p.ks) * 2 * B * 4));
-  const int blocks = std::min(units, sm_count() * ((units + sm_count() * most - 1) / (sm_count() * most)));
-  const size_t fixed = size_t(B) * k * 2 + size_t((units + blocks - 1) / blocks) * p.ks * 2 * B * 4, piece = size_t(p.chunks) * 32;
-  if (fixed + prep::kGemvWarps * 2 * piece > kSmem) return 1;
-  p.slots = int(std::min<size_t>(std::max<size_t>(std::min<size_t>(prep::kGemvRing, kSmem - fixed) / (prep::kGemvWarps * piece), 2), prep::kGemvMaxSlots));
-  const size_t smem = prep::kGemvWarps * p.slots * piece + fixed;
-  p.w = static_cast<const __nv_bfloat16*>(w), p.w2 = static_cast<const __nv_bfloat16*>(w2), p.x = static_cast<const __nv_bfloat16*>(x);
-  p.y = static_cast<__nv_bfloat16*>(y), p.n = n, p.k = k, p.x_stride = x_stride, p.y_stride = y_stride;
-  static bool done[64];
-  int rc = opt_in_smem(prep::gemv_stream_kernel<B, kSwiglu>, kSmem, done);
-  if (rc) return rc;
-  DSA_CUDA(launch_pdl(prep::gemv_stream_kernel<B, kSwiglu>, dim3(blocks), dim3(prep::kGemvWarps * 32), smem, st, p));
-  return DSA_OK;
+static int launch_gemv_stream(prep::GemvParams p, cudaStream_t st) {
+  constexpr size_t kSmem = 224 * 1024, kSums = 16 * 1024;
+  const int kv = p.k / 8, units = kSwiglu ? p.n : (p.n + 1) / 2;
+  // pieces half as long where x leaves no room for two longer ones per warp
+  for (int longest = prep::kGemvChunks; longest >= prep::kGemvChunks / 2; longest /= 2) {
+    // the fewest pieces per row, of even length (the last one may be shorter)
+    p.ks = (kv + longest - 1) / longest;
+    p.chunks = (kv + p.ks - 1) / p.ks;
+    p.ks = (kv + p.chunks - 1) / p.chunks;
+    // a CTA per SM; several where one CTA's table of sums would be larger than its part of shared memory
+    const int most = int(kSums / (size_t(p.ks) * 2 * B * 4));
+    if (most < 1) return 1;
+    const int blocks = std::min(units, sm_count() * ((units + sm_count() * most - 1) / (sm_count() * most)));
+    const size_t fixed = size_t(B) * p.k * 2 + size_t((units + blocks - 1) / blocks) * p.ks * 2 * B * 4, piece = size_t(p.chunks) * 32;
+    if (fixed + prep::kGemvWarps * 2 * piece > kSmem) continue;
+    p.slots = int(std::min<size_t>(std::max<size_t>(std::min<size_t>(prep::kGemvRing, kSmem - fixed) / (prep::kGemvWarps * piece), 2), prep::kGemvMaxSlots));
+    const size_t smem = prep::kGemvWarps * p.slots * piece + fixed;
+    static bool done[64];
+    int rc = opt_in_smem(prep::gemv_stream_kernel<B, kSwiglu>, kSmem, done);
+    if (rc) return rc;
+    DSA_CUDA(launch_pdl(prep::gemv_stream_kernel<B, kSwiglu>, dim3(blocks), dim3(prep::kGemvWarps * 32), smem, st, p));
+    return DSA_OK;
+  }
+  return 1;
+}
+static int launch_gemv_stream(const prep::GemvParams& p, cudaStream_t st) {
+  if (p.w2) return p.rows == 1 ? launch_gemv_stream<1, true>(p, st) : launch_gemv_stream<2, true>(p, st);
+  return p.rows == 1 ? launch_gemv_stream<1, false>(p, st) : p.rows == 2 ? launch_gemv_stream<2, false>(p, st)
+                                                              : launch_gemv_stream<4, false>(p, st);
 }
 
 template <int B>
@@ -1145,25 +1152,25 @@ static int launch_gemv_rows(const void* w, const void* x, void* y, int n, int k,
 }
 }  // extern "C++"
 
-static int gemv_checks(const void* w, const void* x, const void* y, int batch, int n, int k, int64_t x_stride, int64_t y_stride) {
+static int gemv_checks(prep::GemvParams& p, const void* w, const void* x, void* y, int batch, int most, int n, int k, int64_t x_stride,
+                       int64_t y_stride) {
   DSA_REQUIRE(w && x && y, "gemv: null pointer");
-  DSA_REQUIRE(batch >= 1 && batch <= 4, "gemv: batch=%d must be 1..4", batch);
+  DSA_REQUIRE(batch >= 1 && batch <= most, "gemv: batch=%d must be 1..%d", batch, most);
   DSA_REQUIRE(n > 0 && k > 0 && k % 8 == 0, "gemv: k=%d must be a positive multiple of 8", k);
   DSA_REQUIRE(x_stride >= k && x_stride % 8 == 0 && y_stride >= n, "gemv: bad row strides");
   DSA_REQUIRE(aligned16(w) && aligned16(x), "gemv: w and x must be 16-byte aligned");
+  p.w = static_cast<const __nv_bfloat16*>(w), p.x = static_cast<const __nv_bfloat16*>(x), p.y = static_cast<__nv_bfloat16*>(y);
+  p.rows = batch, p.n = n, p.k = k, p.x_stride = x_stride, p.y_stride = y_stride;
   return DSA_OK;
 }
 
-int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride,
-                  int64_t y_stride, void* stream) {
-  int rc = gemv_checks(w, x, y, batch, n, k, x_stride, y_stride);
+int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride, int64_t y_stride, void* stream) {
+  prep::GemvParams p{};
+  int rc = gemv_checks(p, w, x, y, batch, 4, n, k, x_stride, y_stride);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (batch <= 2) {
-    rc = batch == 1 ? launch_gemv_stream<1, false>(w, nullptr, x, y, n, k, x_stride, y_stride, st)
-                    : launch_gemv_stream<2, false>(w, nullptr, x, y, n, k, x_stride, y_stride, st);
-    if (rc != 1) return rc;
-  }
+  rc = launch_gemv_stream(p, st);
+  if (rc != 1) return rc;
   switch (batch) {
     case 1: return launch_gemv_rows<1>(w, x, y, n, k, x_stride, y_stride, st);
     case 2: return launch_gemv_rows<2>(w, x, y, n, k, x_stride, y_stride, st);
@@ -1174,21 +1181,35 @@ int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k
 
 int dsa_gemv_swiglu_bf16(const void* w_gate, const void* w_up, const void* x, void* y, int batch, int n, int k, int64_t x_stride,
                          int64_t y_stride, void* stream) {
-  int rc = gemv_checks(w_gate, x, y, batch, n, k, x_stride, y_stride);
+  prep::GemvParams p{};
+  int rc = gemv_checks(p, w_gate, x, y, batch, 2, n, k, x_stride, y_stride);
   if (rc) return rc;
-  DSA_REQUIRE(w_up && aligned16(w_up), "gemv: w_up must be a 16-byte aligned pointer");
-  DSA_REQUIRE(batch <= 2, "gemv + SwiGLU: batch=%d must be 1 or 2", batch);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  rc = batch == 1 ? launch_gemv_stream<1, true>(w_gate, w_up, x, y, n, k, x_stride, y_stride, st)
-                  : launch_gemv_stream<2, true>(w_gate, w_up, x, y, n, k, x_stride, y_stride, st);
+  DSA_REQUIRE(w_up && aligned16(w_up), "gemv + SwiGLU: w_up must be a 16-byte aligned pointer");
+  p.w2 = static_cast<const __nv_bfloat16*>(w_up);
+  rc = launch_gemv_stream(p, static_cast<cudaStream_t>(stream));
   return rc == 1 ? fail(DSA_ERR_UNSUPPORTED, "gemv + SwiGLU: [%d, %d] is outside the streaming kernel's range", n, k) : rc;
+}
+
+int dsa_norm_gemv_bf16(const void* w, const void* w_up, const void* x, const void* delta, const void* norm_w, float eps, void* sum_out,
+                       void* y, int batch, int n, int k, int64_t x_stride, int64_t y_stride, void* stream) {
+  prep::GemvParams p{};
+  int rc = gemv_checks(p, w, x, y, batch, w_up ? 2 : 4, n, k, x_stride, y_stride);
+  if (rc) return rc;
+  DSA_REQUIRE(norm_w && (!delta || sum_out), "norm + gemv: null pointer");
+  DSA_REQUIRE(aligned16(w_up) && aligned16(delta) && aligned16(norm_w) && aligned16(sum_out), "norm + gemv: pointers must be 16-byte aligned");
+  DSA_REQUIRE(k <= prep::kGemvNormVecs * prep::kGemvWarps * 32 * 8, "norm + gemv: k=%d must be at most %d", k,
+              prep::kGemvNormVecs * prep::kGemvWarps * 32 * 8);
+  p.w2 = static_cast<const __nv_bfloat16*>(w_up), p.delta = static_cast<const __nv_bfloat16*>(delta);
+  p.norm_w = static_cast<const __nv_bfloat16*>(norm_w), p.sum_out = static_cast<__nv_bfloat16*>(sum_out), p.eps = eps;
+  rc = launch_gemv_stream(p, static_cast<cudaStream_t>(stream));
+  return rc == 1 ? fail(DSA_ERR_UNSUPPORTED, "norm + gemv: %d rows of %d do not fit into shared memory", batch, k) : rc;
 }
 
 // NB: the tokens whose products share one reading of the weights, 1, 2, 4 or 8.
 extern "C++" {
 template <int NB>
 static int launch_decode_token(const prep::Params& p, const prep::HeadParams& hp, cudaStream_t st) {
-  const int items = (p.Hidx + 2) * p.B, warps = prep::kHeadThreads / 32;
+  const int items = (p.Hidx + 2 + p.H) * p.B, warps = prep::kHeadThreads / 32;
   const size_t smem = (size_t(NB) * prep::kHeadMaxNope + 8 * (NB <= 2 ? NB : 2) * DSA_VALUE_DIM) * 4;
   DSA_CUDA(launch_pdl(prep::decode_token_kernel<NB>, dim3(p.H + (items + warps - 1) / warps), dim3(prep::kHeadThreads), smem, st, p, hp));
   return DSA_OK;

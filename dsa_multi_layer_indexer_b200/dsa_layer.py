@@ -416,11 +416,15 @@ class DSALayer(nn.Module):
         """A projection of one or two bf16 rows: the library's GEMV, which starts on its weights while the
         kernel before it runs, unless the module is not a plain ``nn.Linear``."""
         m = self._modules[name]
-        if (x.shape[0] > 2 or x.dtype != torch.bfloat16 or not x.is_cuda or torch.is_grad_enabled() or m.__class__ is not nn.Linear
-                or m.bias is not None or m.weight.dtype != torch.bfloat16 or m._forward_hooks or m._forward_pre_hooks
-                or m.in_features % 8 or not m.weight.is_contiguous()):
+        if x.shape[0] > 2 or x.dtype != torch.bfloat16 or not x.is_cuda or torch.is_grad_enabled() or not self._plain(name):
             return m(x)
         return ops.gemv(x, m.weight)
+
+    def _plain(self, name: str) -> bool:
+        """A bias-free bf16 ``nn.Linear`` without hooks, of a width that the GEMV takes."""
+        m = self._modules[name]
+        return (m.__class__ is nn.Linear and m.bias is None and m.weight.dtype == torch.bfloat16 and not m._forward_hooks
+                and not m._forward_pre_hooks and m.in_features % 8 == 0 and m.weight.is_contiguous())
 
     def _absorbed_rows(self, x: torch.Tensor) -> bool:
         """Whether a decode batch takes the kernels that read kv_b_proj's weight in place (one reading for all
@@ -444,30 +448,65 @@ class DSALayer(nn.Module):
         """Writes the keys of a whole prefix x_norm [B,S,hidden] (prefill)."""
         self.full_operands(x_norm, rope, attention=False, indexer=False, cache=cache)
 
-    def decode_project(self, x_norm, rope: RopeCaches, positions, cache: LayerDecodeCache, batch_index):
+    def _norm_folds(self, norm: RMSNorm, x: torch.Tensor) -> bool:
+        """Whether ``norm`` can run inside the projection that follows it (:func:`ops.norm_gemv`)."""
+        return (norm.__class__ is RMSNorm and not norm._forward_hooks and not norm._forward_pre_hooks
+                and x.is_cuda and x.dtype == torch.bfloat16 and norm.weight.dtype == torch.bfloat16
+                and not torch.is_grad_enabled() and ops.norm_gemv_fits(x.shape[0], x.shape[1]))
+
+    def decode_residual_project(self, x, delta, rope: RopeCaches, positions, cache: LayerDecodeCache, batch_index):
+        """``x + delta`` (``delta`` None: ``x``) and :func:`decode_project` of its attention norm."""
+        wide = self._wx.shape[0] if self._stacked() else 0
+        # One or two rows: the norm's launch goes. Four where the product has few outputs of long rows, which the
+        # library's GEMM runs at 1.4 TB/s (norm, [2240, 7168] and the copy of its strided columns 27 us, here 13).
+        if wide and x.dim() == 2 and (x.shape[0] <= 2 or (x.shape[0] <= 4 and wide <= 4096 <= x.shape[1])) and self._norm_folds(self.attn_norm, x):
+            x, ya = ops.norm_gemv(x, delta, self.attn_norm.weight, self.attn_norm.eps, self._wx)
+            return x, self.decode_project(x, rope, positions, cache, batch_index, ya)
+        if delta is None:
+            x_norm = self.attn_norm(x)
+        else:
+            x, x_norm = self.attn_norm.add_forward(x, delta)
+        return x, self.decode_project(x_norm, rope, positions, cache, batch_index)
+
+    def decode_mlp(self, x: torch.Tensor, attn: torch.Tensor):
+        """``(h, mlp(ffn_norm(h)))`` with ``h = x + attn``."""
+        if (x.shape == attn.shape and x.dim() == 2 and x.shape[0] <= 2 and attn.dtype == x.dtype and attn.is_contiguous()
+                and self._norm_folds(self.ffn_norm, x) and self._plain("gate_proj") and self._plain("up_proj")):
+            h, act = ops.norm_gemv(x, attn, self.ffn_norm.weight, self.ffn_norm.eps, self.gate_proj.weight, self.up_proj.weight)
+            return h, self._reduced(self._skinny("down_proj", act))
+        h, h_norm = self.ffn_norm.add_forward(x, attn)
+        return h, self.mlp(h_norm)
+
+    def decode_project(self, x_norm, rope: RopeCaches, positions, cache: LayerDecodeCache, batch_index, ya=None):
         """Projections of one new token per sequence, and its keys appended to
         the caches at ``positions`` [B]. Returns (q [B,H,Dqk], index_q, index_w).
 
         With FP8 caches and bf16 weights everything after the GEMVs (RoPE, e4m3
         quantisation with the scale folded into the head weights, both cache
         appends, assembly of the absorbed query) is ONE launch; index_q then
-        comes back already quantised (uint8) with index_w fp32."""
+        comes back already quantised (uint8) with index_w fp32. ``ya``: the stacked
+        projection of ``x_norm``, where the caller has it (then only x_norm's shape is read)."""
         c = self.config
         b = x_norm.shape[0]
         h = c.num_attention_heads
         il = c.indexer_rope_interleave
         if self._stacked():  # two GEMVs: everything that reads x_norm, then everything that reads c_q
-            # few output rows, long rows: the library GEMV is latency-bound there (measured 19-32 us
-            # against 13 us for the skinny kernel at one token); the other shapes stay with the library
-            skinny = b <= 2 and x_norm.dtype == torch.bfloat16 and self._wx.shape[0] <= 4096 <= self._wx.shape[1]
-            ya = ops.gemv(x_norm, self._wx) if skinny else torch.nn.functional.linear(x_norm, self._wx)
+            if ya is None:
+                # few output rows, long rows: the library GEMV is latency-bound there (measured 19-32 us
+                # against 13 us for the skinny kernel at one token); the other shapes stay with the library
+                skinny = b <= 2 and x_norm.dtype == torch.bfloat16 and self._wx.shape[0] <= 4096 <= self._wx.shape[1]
+                ya = ops.gemv(x_norm, self._wx) if skinny else torch.nn.functional.linear(x_norm, self._wx)
             qa, kv_a, ik_raw = ya.split(
                 [c.q_lora_rank, c.kv_lora_rank + c.qk_rope_head_dim, c.index_head_dim], dim=-1)
-            c_q = self.q_a_layernorm(qa)
+            n = self.q_a_layernorm
             # the c_q-side projection and the MLP's gate / up take the same kernel at one or two
             # tokens (252 against 255 us per layer of the 8-layer stack)
-            wide = b <= 2 and c_q.dtype == torch.bfloat16
-            q, iq_raw, w = (ops.gemv(c_q, self._wc) if wide else torch.nn.functional.linear(c_q, self._wc)).split(
+            if b <= 2 and self._norm_folds(n, qa):
+                yc = ops.norm_gemv(qa, None, n.weight, n.eps, self._wc)[1]
+            else:
+                c_q = n(qa)
+                yc = ops.gemv(c_q, self._wc) if b <= 2 and c_q.dtype == torch.bfloat16 else torch.nn.functional.linear(c_q, self._wc)
+            q, iq_raw, w = yc.split(
                 [h * (c.qk_nope_head_dim + c.qk_rope_head_dim), c.index_n_heads * c.index_head_dim, c.index_n_heads],
                 dim=-1)
         else:

@@ -275,11 +275,11 @@ class DSAModel(nn.Module):
         carried: Optional[torch.Tensor] = None
         pending = False  # an indexer is in flight on the side stream
         used, produced = [], []
-        x_norm = self.layers[0].attn_norm(x)
+        delta = None  # (the residual addition is left to the norm behind it)
         for li, layer in enumerate(self.layers):
             cache = state.caches[li]
             is_dsa = types[li] is AttentionType.DSA
-            q, iq, w = layer.decode_project(x_norm, state.rope, state.positions, cache, state.batch_index)
+            x, (q, iq, w) = layer.decode_residual_project(x, delta, state.rope, state.positions, cache, state.batch_index)
             made = None
             beside = False
             if not lagged:
@@ -312,7 +312,7 @@ class DSAModel(nn.Module):
                         beside = (chained and li > 0 and attend is not None and cache.k_scale is not None
                                   and iq.dtype == torch.uint8 and state.workspaces[li] is not None)
             attn = layer.decode_attention(q, cache, attend, state.seq_lens, beside_previous=beside)
-            x, x_norm = self._residual_tail(li, x, attn)
+            x, delta = layer.decode_mlp(x, attn)
             if lagged and made is not None:
                 carried = made  # becomes visible to layer li+1 after the join
             if record is not None:
@@ -324,7 +324,7 @@ class DSAModel(nn.Module):
         state.carried = carried
         if record is not None:
             record["used"], record["produced"] = used, produced
-        return x_norm  # the last layer's tail applied the final norm
+        return self.final_norm.add_forward(x, delta)[1]
 
     def _residual_tail(self, li: int, x: torch.Tensor, attn: torch.Tensor, weights=None):
         """``h = x + attn; x' = h + mlp(ffn_norm(h))`` and the norm the next consumer
@@ -356,11 +356,11 @@ class DSAModel(nn.Module):
         booted = False
         forked = False
         used, produced = [], []
-        x_norm = self.layers[0].attn_norm(x)
+        delta = None  # (the residual addition is left to the norm behind it)
         for li, layer in enumerate(self.layers):
             cache = state.caches[li]
             is_dsa = types[li] is AttentionType.DSA
-            q, iq, w = layer.decode_project(x_norm, state.rope, state.positions, cache, state.batch_index)
+            x, (q, iq, w) = layer.decode_residual_project(x, delta, state.rope, state.positions, cache, state.batch_index)
             made = None
 
             def dispatch():
@@ -401,7 +401,7 @@ class DSAModel(nn.Module):
             else:
                 attend = carried
             attn = layer.decode_attention(q, cache, attend, state.seq_lens)
-            x, x_norm = self._residual_tail(li, x, attn)
+            x, delta = layer.decode_mlp(x, attn)
             if record is not None:
                 used.append(attend)
                 produced.append(made)
@@ -411,7 +411,7 @@ class DSAModel(nn.Module):
         state.carried = carried
         if record is not None:
             record["used"], record["produced"] = used, produced
-        return x_norm  # the last layer's tail applied the final norm
+        return self.final_norm.add_forward(x, delta)[1]
 
     def capture_decode(self, state: DecodeState, mode: ScheduleMode,
                        cold_start: ColdStartPolicy = ColdStartPolicy.DENSE, overlap=True,

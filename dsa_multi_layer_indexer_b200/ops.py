@@ -398,6 +398,33 @@ def gemv_swiglu(x: torch.Tensor, gate: torch.Tensor, up: torch.Tensor) -> torch.
     return y
 
 
+def norm_gemv(x: torch.Tensor, delta: Optional[torch.Tensor], norm_weight: torch.Tensor, eps: float, weight: torch.Tensor,
+              up: Optional[torch.Tensor] = None):
+    """``(s, rmsnorm(s) @ weight.T)`` with ``s = x + delta`` (``x`` without a delta) in one launch, for 1..4
+    rows of at most 8192; with ``up`` the SwiGLU product of :func:`gemv_swiglu`."""
+    x = _gemv_operand(x, weight, 2 if up is not None else 4)
+    (b, k), n = x.shape, weight.shape[0]
+    _cuda_contig(norm_weight, "norm_weight", (torch.bfloat16,))
+    _need(norm_weight.numel() == k, "norm_weight must have k elements")
+    s = x
+    if delta is not None:
+        _cuda_contig(delta, "delta", (torch.bfloat16,))
+        _need(tuple(delta.shape) == (b, k), "delta must be [B, k]")
+        s = torch.empty(b, k, dtype=torch.bfloat16, device=x.device)
+    if up is not None:
+        _need(up.shape == weight.shape and up.dtype == torch.bfloat16 and up.is_contiguous(), "gate and up must have one shape")
+    y = torch.empty(b, n, dtype=torch.bfloat16, device=x.device)
+    _lib.check(_lib.lib().dsa_norm_gemv_bf16(_ptr(weight), _ptr(up), _ptr(x), _ptr(delta), _ptr(norm_weight), float(eps),
+                                             _ptr(s) if delta is not None else None, _ptr(y), b, n, k,
+                                             x.stride(0) if b > 1 else k, n, _stream()))
+    return s, y
+
+
+def norm_gemv_fits(b: int, k: int) -> bool:
+    """Rows that dsa_norm_gemv_bf16 takes."""
+    return 1 <= b <= 4 and k % 8 == 0 and k <= 8192
+
+
 HEAD_TOKENS = 8  # tokens that share one reading of kv_b_proj's weight in decode_token / value_project
 
 

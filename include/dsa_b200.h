@@ -402,11 +402,17 @@ int dsa_copy_post_epoch(void* dst, const void* src, int64_t bytes, uint32_t* cou
  * elements. The kernel starts reading w before the kernel enqueued in front of it has completed: w must
  * not be written by this library (by any other work, anything goes).
  * dsa_gemv_swiglu_bf16: y = silu(x w_gate^T) * (x w_up^T), rounded as the separate operations, for one or
- * two rows (:194-196). */
+ * two rows (:194-196).
+ * dsa_norm_gemv_bf16: either with x replaced by rmsnorm(x + delta) * norm_w, rounded as in
+ * dsa_add_rmsnorm_bf16 (delta NULL: rmsnorm(x)); sum_out [batch, k] receives x + delta and overlaps neither.
+ * w_up NULL: the plain product. k at most 8192; delta's rows are dense. */
 int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride,
                   int64_t y_stride, void* stream);
 int dsa_gemv_swiglu_bf16(const void* w_gate, const void* w_up, const void* x, void* y, int batch, int n, int k,
                          int64_t x_stride, int64_t y_stride, void* stream);
+int dsa_norm_gemv_bf16(const void* w, const void* w_up, const void* x, const void* delta, const void* norm_w,
+                       float eps, void* sum_out, void* y, int batch, int n, int k, int64_t x_stride,
+                       int64_t y_stride, void* stream);
 /* ov [B, H, v_dim] = W_UV[h] o[b, h, :] with kv_b_proj's weight kv_b [H, nope + v_dim, 512] (bf16,
  * src/lagged_indexer_dsa/dsa_layer.py:118-125), o [B, o_heads, 512], 1..8 tokens. kv_b is read like the
  * weights of dsa_gemv_bf16. */

@@ -47,6 +47,41 @@ def test_gemv_and_swiglu(ops, b, n, k):
     assert torch.equal(ops.gemv(view, w), ops.gemv(view.contiguous(), w))
 
 
+# one row per template, padded rows, a strided x, the widest row, with and without a residual and the second matrix
+@pytest.mark.parametrize("b,n,k,residual", [(1, 300, 7168, True), (2, 515, 1536, False), (3, 301, 6144, True), (4, 77, 8192, True),
+                                            (3, 148, 264, False), (1, 9, 8, True)])
+def test_norm_gemv(ops, b, n, k, residual):
+    torch.manual_seed(n + k)
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    assert ops.norm_gemv_fits(b, k)
+    wide, delta, nw = bf(b, k + 64), bf(b, k) if residual else None, bf(k)
+    x = wide[:, :k]
+    w, u = (torch.randn(n, k, device="cuda").div_(k ** 0.5).to(torch.bfloat16) for _ in range(2))
+    s, y = ops.norm_gemv(x, delta, nw, 1e-6, w)
+    if residual:
+        want_s, normed = ops.add_rmsnorm(x.contiguous(), delta, nw, 1e-6)
+        assert torch.equal(s, want_s)
+    else:
+        normed = ops.rmsnorm(x.contiguous(), nw, 1e-6)
+    # the sum of squares is taken in another order: 2^-20 relative in the factor, which may move a normed element
+    # to its neighbour (2^-8) - few of them, counted here as if all fell on the largest products
+    prod = normed.double().unsqueeze(1) * w.double().unsqueeze(0)
+    moved = prod.abs().topk(min(k, 4), dim=-1).values.sum(-1) * 2.0 ** -8
+    ref, mag = prod.sum(-1), prod.abs().sum(-1)
+    close(y, ref, mag + moved * 2.0 ** 20)
+    if b <= 2:
+        s2, act = ops.norm_gemv(x, delta, nw, 1e-6, w, u)
+        assert torch.equal(s2, s)
+        up = ops.norm_gemv(x, delta, nw, 1e-6, u)[1]
+        # as test_gemv_and_swiglu: the factors may lie one rounding from the single products
+        g, v = y.double(), up.double()
+        silu = torch.nn.functional.silu(g)
+        dg, dv = g.abs() * 2.0 ** -7 + mag * 2.0 ** -19, v.abs() * 2.0 ** -7 + mag * 2.0 ** -19
+        ds = 1.1 * dg + (silu.abs() + 1.1 * dg) * 2.0 ** -8
+        err = ds * (v.abs() + dv) + silu.abs() * dv
+        assert float(((act.double() - silu * v).abs() - err - ((silu * v).abs() + err) * 2.0 ** -8).max()) <= 0.0
+
+
 # one to eight tokens, remainders of the row groups (nope) and of the rows per warp step (v), padded heads
 @pytest.mark.parametrize("B,H,nope,v,pad", [(1, 128, 128, 128, 0), (2, 64, 192, 256, 0), (3, 5, 36, 7, 11), (8, 16, 512, 66, 0), (5, 8, 64, 128, 0)])
 def test_absorbed_projections(ops, B, H, nope, v, pad):
