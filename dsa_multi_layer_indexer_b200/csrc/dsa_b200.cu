@@ -1033,7 +1033,7 @@ static int launch_linear_f32(const lin::Params& p, int tiles, cudaStream_t st) {
   int rc = opt_in_smem(lin::linear_f32_kernel<kSwiglu>, smem, done);
   if (rc) return rc;
   const dim3 grid(unsigned((p.m + lin::kBM - 1) / lin::kBM), tiles);
-  DSA_CUDA(launch_pdl(lin::linear_f32_kernel<kSwiglu>, grid, dim3(lin::kThreads), smem, st, p));
+  DSA_CUDA(launch_pdl(lin::linear_f32_kernel<kSwiglu>, grid, dim3(lin::kGroup * lin::groups<kSwiglu>()), smem, st, p));
   return DSA_OK;
 }
 }  // extern "C++"
