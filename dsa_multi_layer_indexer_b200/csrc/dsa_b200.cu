@@ -105,7 +105,7 @@ static int opt_in_smem(K kernel, size_t bytes, bool (&done)[64]) {
   if (dev >= 0 && dev < 64) done[dev] = true;
   return DSA_OK;
 }
-static bool g_opt_fused[64], g_opt_mla[64], g_opt_mla_beside[64], g_opt_mla_tc[64], g_opt_mla_f32[64], g_opt_topk[64];
+static bool g_opt_fused[64], g_opt_mla[4][64], g_opt_mla_tc[64], g_opt_mla_f32[64], g_opt_topk[64];
 
 // Launch with programmatic dependent launch allowed: the kernel may be scheduled
 // while its predecessor in the stream is still draining; it calls
@@ -900,20 +900,14 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
     return DSA_OK;
   }
   const size_t smem = kv_fp8 ? mla::SmemLayout::bytes_fp8 : mla::SmemLayout::bytes_bf16;
-  if (beside) {
-    int rc = opt_in_smem(mla::sparse_mla_partials_beside_kernel, mla::SmemLayout::bytes_fp8, g_opt_mla_beside);
+  const auto launch = [&](auto kernel, bool (&done)[64]) {
+    int rc = opt_in_smem(kernel, mla::SmemLayout::bytes_fp8, done);
     if (rc) return rc;
-    DSA_CUDA(launch_pdl(mla::sparse_mla_partials_beside_kernel, dim3(nsplit, H / DSA_HEAD_BLOCK, R),
-                        dim3(mla::kThreads), smem, static_cast<cudaStream_t>(stream), p));
-    return DSA_OK;
-  }
-  {
-    int rc = opt_in_smem(mla::sparse_mla_partials_kernel, mla::SmemLayout::bytes_fp8, g_opt_mla);
-    if (rc) return rc;
-  }
-  DSA_CUDA(launch_pdl(mla::sparse_mla_partials_kernel, dim3(nsplit, H / DSA_HEAD_BLOCK, R),
-                      dim3(mla::kThreads), smem, static_cast<cudaStream_t>(stream), p));
-  return DSA_OK;
+    DSA_CUDA(launch_pdl(kernel, dim3(nsplit, H / DSA_HEAD_BLOCK, R), dim3(mla::kThreads), smem, static_cast<cudaStream_t>(stream), p));
+    return int(DSA_OK);
+  };
+  if (beside) return out ? launch(mla::sparse_mla_partials_beside_kernel<true>, g_opt_mla[3]) : launch(mla::sparse_mla_partials_beside_kernel<false>, g_opt_mla[2]);
+  return out ? launch(mla::sparse_mla_partials_kernel<true>, g_opt_mla[1]) : launch(mla::sparse_mla_partials_kernel<false>, g_opt_mla[0]);
 }
 
 int dsa_sparse_mla_partials(const void* q, const void* kv, const int32_t* indices,

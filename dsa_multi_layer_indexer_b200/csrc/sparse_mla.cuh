@@ -331,7 +331,7 @@ __device__ __forceinline__ void dequant_tile_inplace(uint8_t* s_k, const int* s_
 // schedule the attention reads the PREVIOUS layer's selection while this layer's top-k runs), so
 // it releases its own dependents and starts at once, beside that kernel, and waits for it only
 // before it exits: it still completes after it, and the next kernel's wait covers both.
-template <bool kBeside = false>
+template <bool kBeside = false, bool kDirect = false>
 __device__ __forceinline__ void mla_partials_body(const Params& p, const int split, const int hg, const int r,
                                                   uint8_t* smem) {
   uint8_t* s_q = smem + SmemLayout::q_off;
@@ -435,7 +435,7 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
     drain_after_timeout();  // let outstanding copies land
   }
 
-  if (p.out) {  // the only split: what the merge kernel would make of its partials
+  if constexpr (kDirect) {  // the only split: what the merge kernel would make of its partials
     __nv_bfloat16* out = p.out + (int64_t(r) * p.H + hg * kHB) * kDV;
     const float inv0 = l_run[0] > 0.f ? 1.f / l_run[0] : 0.f, inv1 = l_run[1] > 0.f ? 1.f / l_run[1] : 0.f;
 #pragma unroll
@@ -466,16 +466,18 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
   DSA_KTIME_END(2);
 }
 
+template <bool kDirect>
 __global__ void __launch_bounds__(kThreads)
-sparse_mla_partials_kernel(const Params p) {
+sparse_mla_partials_kernel(const Params p) {  // kDirect is an instantiation of its own: its code costs a step 0.1 us
   extern __shared__ __align__(16) uint8_t mla_smem[];
-  mla_partials_body<false>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
+  mla_partials_body<false, kDirect>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
 }
 
+template <bool kDirect>
 __global__ void __launch_bounds__(kThreads)
 sparse_mla_partials_beside_kernel(const Params p) {
   extern __shared__ __align__(16) uint8_t mla_smem[];
-  mla_partials_body<true>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
+  mla_partials_body<true, kDirect>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
 }
 
 // ------------------------------------------------------------------------------
