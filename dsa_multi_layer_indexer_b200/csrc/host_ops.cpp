@@ -9,12 +9,14 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <c10/core/GradMode.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
 #include <cmath>
 #include <initializer_list>
+#include <optional>
 #include <stdexcept>
 #include <string>
 #include <tuple>
@@ -897,6 +899,10 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return nullptr;
   }
   try {
+    // Without gradients the torch calls inside (allocations, views, library GEMMs) go straight to their
+    // kernels instead of through the autograd and view-tracking keys, about a microsecond each.
+    std::optional<at::AutoDispatchBelowADInplaceOrView> direct;
+    if (!c10::GradMode::is_enabled()) direct.emplace();
     return fn(args);
   } catch (const PyErrorSet&) {
   } catch (const ValueError& e) {
