@@ -41,7 +41,6 @@ struct Params {
   float* part_acc;
   float* part_m;
   float* part_l;
-  __nv_bfloat16* out;     // one split only: the normalised result goes here and no partials are written
   int64_t kv_seq_stride;  // rows per cached sequence
   int64_t ctx;            // dense mode: key capacity
   int rows_per_seq;
@@ -51,6 +50,7 @@ struct Params {
   int keys_per_split;
   int kv_fp8;
   float scale_log2;       // sm_scale * log2(e)
+  __nv_bfloat16* out;     // one split only: the normalised result goes here and no partials are written
 };
 
 struct SmemLayout {

@@ -64,8 +64,6 @@ struct Params {
   int topk;
   int32_t pad;
   int32_t index_offset;
-  const int32_t* page_table;  // kPages only: the selection as slots page_table[r][position / 64] * 64 + position % 64
-  int64_t pt_stride;
   // ---- candidate exchange between the GPUs of a sequence-sharded indexer (cluster kernel only)
   // Push side (n_dest > 0): the selection of row r goes, as (index, logit), into slot `src_rank`
   // of every rank's gather buffers [2 parities][R][n_dest][topk], then flag word
@@ -82,6 +80,8 @@ struct Params {
   const uint32_t* wait_flags;      // [n_src][R], written by the sources
   uint32_t* seen;                  // [R] steps merged so far (local)
   unsigned long long wait_limit_ns;
+  const int32_t* page_table;  // kPages only: the selection as slots page_table[r][position / 64] * 64 + position % 64
+  int64_t pt_stride;
 };
 
 // Workspace layout in 32-bit words: [R][words] mask | [R][slots] counts |
