@@ -750,6 +750,8 @@ PyObject* full_operands(PyObject* const* a) {
     NoGil unlocked;
     const int64_t q_rank = q_a.size(0), width = kv_a.size(0), rope_dim = rope.mc.size(1), rank = width - rope_dim, D = ik_w.size(0);
     const bool keep_kv = attention || kv_given, keep_ik = indexer || ik_given;
+    for (const Tensor* t : {&q_norm, &kv_norm}) contig(*t, "norm weight", {type});
+    need(q_norm.numel() == q_rank && kv_norm.numel() == rank, "the norms' weights must have q_rank and kv_rank elements");
     void* st = stream();
 
     const Tensor x = xn.reshape({rows, hidden});

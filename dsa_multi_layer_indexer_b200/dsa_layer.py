@@ -31,6 +31,12 @@ from .config import DSAConfig
 from .rope import apply_rotary, apply_rotary_at
 
 
+def _bare(m: nn.Module, cls: type) -> bool:
+    """Whether calling ``m`` is ``cls.forward`` and nothing else: no subclass, no hooks, no replaced ``forward``."""
+    d = m.__dict__
+    return m.__class__ is cls and not d["_forward_hooks"] and not d["_forward_pre_hooks"] and "forward" not in d
+
+
 # The linear projections of a layer, in construction order.
 _PROJECTIONS = ("q_a_proj", "q_b_proj", "kv_a_proj", "kv_b_proj", "o_proj", "index_q_proj", "index_k_proj",
                 "index_weights_proj", "gate_proj", "up_proj", "down_proj")
@@ -315,13 +321,17 @@ class DSALayer(nn.Module):
         """The projections' weights, in construction order, where the fused full-sequence chain applies
         to ``t``, else None: it has no autograd or autocast, knows the fp32 form of any geometry and the
         bf16 / e4m3 form of the production geometry, and needs every projection to be a plain
-        ``nn.Linear`` (not replaced, no bias, no hooks on it)."""
+        ``nn.Linear`` (not replaced, no bias, no hooks on it). It norms the two latents itself: their norms
+        must be plain too, with one eps and weights of ``t``'s type (the module converts them)."""
         dtype = t.dtype
         if not (t.is_cuda and (dtype == torch.float32 or self._fast_path(t))) or torch.is_grad_enabled() or torch.is_autocast_enabled():
             return None
         if _module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks:
             return None
         mods, out = self._modules, []
+        qn, kn = mods["q_a_layernorm"], mods["kv_a_layernorm"]
+        if not (_bare(qn, RMSNorm) and _bare(kn, RMSNorm) and qn.eps == kn.eps and qn.weight.dtype == dtype == kn.weight.dtype):
+            return None
         for name in _PROJECTIONS:
             m = mods[name]
             d = m.__dict__
@@ -349,7 +359,7 @@ class DSALayer(nn.Module):
         parts = _lib.host().full_operands(
             x_norm, s, c_q, wx, wc, q_a, kv_a, ik_w, q_b, iq_w, w_w, self.q_a_layernorm.weight, self.kv_a_layernorm.weight,
             kv_b, rope.mla_cos, rope.mla_sin, rope.idx_cos, rope.idx_sin, kv, ik, ik_scale, attention, indexer, fp8,
-            c.num_attention_heads, c.qk_nope_head_dim, c.index_n_heads, c.indexer_rope_interleave, c.rms_norm_eps)
+            c.num_attention_heads, c.qk_nope_head_dim, c.index_n_heads, c.indexer_rope_interleave, self.q_a_layernorm.eps)
         return FullOperands(b, s, lens, weights, *parts)
 
     def full_select(self, op: "FullOperands", pad_value: int = -1, padded: bool = True) -> torch.Tensor:

@@ -1,0 +1,113 @@
+"""GPU tests of full-sequence layers in the forms that the fused native chain does not take: whatever a
+module of the layer has been made into (other weight types, hooks, replacements), forward and prefill must
+give what calling the modules one after the other gives. That path still runs when autograd is on, so it is
+the reference here, bit for bit."""
+
+from __future__ import annotations
+
+import dataclasses
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def D():
+    import dsa_multi_layer_indexer_b200 as pkg
+    from dsa_multi_layer_indexer_b200 import _lib
+
+    _lib.lib()
+    yield pkg
+    _lib.check_device_status()
+
+
+def make_model(D, dtype, layers=1):
+    """Small layers whose norm weights are not ones (but numbers of every type used here)."""
+    if dtype == torch.bfloat16:
+        cfg = D.DSAConfig(hidden_size=192, num_hidden_layers=layers, num_attention_heads=16, q_lora_rank=96, index_n_heads=32,
+                          index_topk=64, intermediate_size=256, first_k_dense_replace=0)
+    else:
+        cfg = dataclasses.replace(D.named_config("small"), num_hidden_layers=layers, first_k_dense_replace=0)
+    torch.manual_seed(5)
+    model = D.DSAModel(cfg).eval()
+    with torch.no_grad():
+        for m in norms_of(model):
+            m.weight.copy_(1.0 + torch.randint(-32, 33, m.weight.shape) / 64.0)
+    return model.cuda().to(dtype)
+
+
+def norms_of(model):
+    return [m for m in model.modules() if type(m).__name__ == "RMSNorm"]
+
+
+def tokens(model, b, s):
+    torch.manual_seed(6)
+    return torch.randn(b, s, model.config.hidden_size, device="cuda").to(model.layers[0].q_a_proj.weight.dtype)
+
+
+def operands(model, x, cache=None):
+    """(q, kv, ik, iq, iw) of layer 0 as computed, whatever the path."""
+    op = model.layers[0].full_operands(x, model._build_rope(x.shape[1], x.device, x.dtype), cache=cache)
+    return op, [t.detach() for t in (op.q, op.kv, op.ik, op.iq, op.iw)]
+
+
+def check_against_modules(model, x):
+    """full_operands without gradients must be the modules' own results."""
+    with torch.no_grad():
+        op, got = operands(model, x)
+    ref_op, want = operands(model, x)  # autograd is on: the modules one by one
+    assert not op.fused and not ref_op.fused
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("dtype,other", [(torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("which", ["all", "q_a_layernorm", "kv_a_layernorm"])
+def test_norm_weights_of_another_type(D, dtype, other, which):
+    mode, cold = D.ScheduleMode.LAGGED_FUSED, D.ColdStartPolicy.DENSE  # (no selection, whose cutoff rounding moves)
+    model = make_model(D, dtype)
+    x = tokens(model, 2, 70)
+    with torch.no_grad():
+        same_type = model(x, mode, cold)
+    for m in norms_of(model) if which == "all" else [getattr(model.layers[0], which)]:
+        m.to(other)
+    check_against_modules(model, x)
+    with torch.no_grad():
+        got = model(x, mode, cold)
+    filled = model.prefill(model.init_decode(2, 80, fp8=dtype == torch.bfloat16), x, mode, cold)
+    # the same numbers as with weights of the activations' type, by other kernels: a handful of bf16 roundings
+    # (2^-8 each); fp32 sums in another order
+    tol = 3e-2 if dtype == torch.bfloat16 else 1e-4
+    for y in (got, filled):
+        assert float((y.float() - same_type.float()).norm()) <= tol * float(same_type.float().norm())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("name,row", [("q_a_layernorm", 0), ("kv_a_layernorm", 1)])
+@pytest.mark.parametrize("change", ["hook", "pre_hook", "subclass", "forward", "eps"])
+def test_changed_latent_norms_are_honoured(D, dtype, name, row, change):
+    model = make_model(D, dtype)
+    x = tokens(model, 1, 33)
+    with torch.no_grad():
+        plain = operands(model, x)[1]
+    m = getattr(model.layers[0], name)
+    if change == "hook":
+        m.register_forward_hook(lambda mod, a, o: o * 2)
+    elif change == "pre_hook":
+        m.register_forward_pre_hook(lambda mod, a: (a[0].sin(),))
+    elif change == "subclass":
+        class Doubled(type(m)):
+            def forward(self, t):
+                return super().forward(t) * 2
+
+        m.__class__ = Doubled
+    elif change == "forward":
+        inner = m.forward
+        m.forward = lambda t: inner(t) * 2
+    else:
+        m.eps = 0.5
+    check_against_modules(model, x)
+    with torch.no_grad():
+        changed = operands(model, x)[1]
+    assert not torch.allclose(changed[row].float(), plain[row].float(), rtol=2e-2, atol=1e-3)
