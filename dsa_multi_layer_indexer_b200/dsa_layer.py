@@ -536,7 +536,7 @@ class DSALayer(nn.Module):
                                  rope.mla_sin, rope.idx_cos, rope.idx_sin, positions, index_q, index_w, q_full, cache.index_k,
                                  cache.k_scale, cache.kv, il, c.rms_norm_eps)
                 return q_full, index_q, index_w
-        q = q.reshape(b, h, c.qk_nope_head_dim + c.qk_rope_head_dim)
+        q = q.contiguous().view(b, h, c.qk_nope_head_dim + c.qk_rope_head_dim)  # (a column range of a stacked product)
         iq_raw = iq_raw.reshape(b, c.index_n_heads, c.index_head_dim)
         q_nope, q_rope = q.split([c.qk_nope_head_dim, c.qk_rope_head_dim], dim=-1)
         w_uk, _ = self._w_uk_uv()
