@@ -132,14 +132,18 @@ class DSAModel(nn.Module):
     def _rope_for(self, seq_len: int, device, dtype) -> RopeCaches:
         """Tables of at least ``seq_len`` rows for one full-sequence pass: the last pass's (a table row
         depends on its position alone), rebuilt when it was shorter or made for another type, device or
-        stream. A graph capture gets tables of its own, which live as long as the graph."""
+        stream. A graph capture gets tables of its own, which live as long as the graph. What is kept are
+        ordinary tensors whatever mode this pass runs in: a later one may need them for its gradients."""
         if torch.cuda.is_current_stream_capturing():
             return self._build_rope(seq_len, device, dtype)
         c = self.config
         key = (device, dtype, torch.cuda.current_stream(device).cuda_stream, c.qk_rope_head_dim, c.index_head_dim, c.rope_theta, c.indexer_rope_interleave)
         kept = getattr(self, "_rope_kept", None)
         if kept is None or kept[0] != key or kept[1].mla_cos.shape[0] < seq_len:
-            kept = self._rope_kept = (key, self._build_rope(seq_len, device, dtype))
+            with torch.inference_mode(False):
+                kept = (key, self._build_rope(seq_len, device, dtype))
+            if type(kept[1].mla_cos) is torch.Tensor:  # (a dispatch mode may have made its own kind)
+                self._rope_kept = kept
         return kept[1]
 
     def _lagged_indexer_layers(self, types) -> List[bool]:

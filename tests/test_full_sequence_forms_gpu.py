@@ -111,3 +111,19 @@ def test_changed_latent_norms_are_honoured(D, dtype, name, row, change):
     with torch.no_grad():
         changed = operands(model, x)[1]
     assert not torch.allclose(changed[row].float(), plain[row].float(), rtol=2e-2, atol=1e-3)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gradients_after_a_pass_in_inference_mode(D, dtype):
+    """The rotary tables that one pass leaves for the next serve every mode."""
+    mode, cold = D.ScheduleMode.BASELINE, D.ColdStartPolicy.EAGER
+    model = make_model(D, dtype)
+    x = tokens(model, 1, 40)
+    with torch.inference_mode():
+        first = model(x, mode, cold)
+    x = x.clone().requires_grad_(True)
+    model(x, mode, cold)  # (apply_rotary saves its tables for the backward pass)
+    shorter = model(x[:, :17], mode, cold)
+    assert shorter.shape == (1, 17, model.config.hidden_size) and not model._rope_kept[1].mla_cos.is_inference()
+    with torch.inference_mode():
+        assert torch.equal(model(x, mode, cold), first)
