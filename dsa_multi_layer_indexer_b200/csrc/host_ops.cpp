@@ -583,6 +583,7 @@ Rope rope_of(PyObject* const* a, at::ScalarType type, int64_t seq) {
     contig(*t, "rotary table", {type});
     need(t->dim() == 2 && t->size(0) >= seq, "a rotary table is shorter than the sequence");
   }
+  need(r.mc.size(1) == r.ms.size(1) && r.ic.size(1) == r.is.size(1), "the rotary tables' widths disagree");
   return r;
 }
 int dtype_of(at::ScalarType t) {
@@ -693,11 +694,15 @@ PyObject* prefill_queries(PyObject* const* a) {
 // two weights: 23 us against the library's 19; three weights of 2^25.6 in all: 6 us against 20).
 constexpr double kSmallLinear = double(1 << 28);
 
+// (What the GEMM library would refuse - a weight of another device, type or inner dimension - goes to it.)
 bool small_f32(const Tensor& x, std::initializer_list<const Tensor*> ws) {
-  if (x.scalar_type() != at::kFloat || !x.is_contiguous() || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u)) return false;
+  if (!x.is_cuda() || x.dim() != 2 || x.scalar_type() != at::kFloat || !x.is_contiguous() || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u))
+    return false;
   double n = 0;
   for (const Tensor* w : ws) {
-    if (!w->is_contiguous() || (reinterpret_cast<uintptr_t>(w->data_ptr()) & 15u)) return false;
+    if (w->device() != x.device() || w->scalar_type() != at::kFloat || w->dim() != 2 || w->size(1) != x.size(1) || !w->is_contiguous() ||
+        (reinterpret_cast<uintptr_t>(w->data_ptr()) & 15u))
+      return false;
     n += double(w->size(0));
   }
   return x.size(1) % 4 == 0 && double(x.size(0)) * n * double(x.size(1)) <= kSmallLinear;
@@ -751,6 +756,9 @@ PyObject* full_operands(PyObject* const* a) {
     const int64_t q_rank = q_a.size(0), width = kv_a.size(0), rope_dim = rope.mc.size(1), rank = width - rope_dim, D = ik_w.size(0);
     const bool keep_kv = attention || kv_given, keep_ik = indexer || ik_given;
     for (const Tensor* t : {&q_norm, &kv_norm}) contig(*t, "norm weight", {type});
+    for (const Tensor* t : {&q_norm, &kv_norm, &rope.mc, &rope.ms, &rope.ic, &rope.is})
+      need(t->device() == xn.device(), "norm weights and rotary tables must be on the activations' device");
+    need(rope_dim > 0 && rank > 0 && rope.ic.size(1) == D, "the rotary tables' widths must be those of the projections");
     need(q_norm.numel() == q_rank && kv_norm.numel() == rank, "the norms' weights must have q_rank and kv_rank elements");
     void* st = stream();
 
@@ -799,6 +807,7 @@ PyObject* full_operands(PyObject* const* a) {
     at::bmm_out(dst, q.narrow(2, 0, nope).transpose(0, 1), w_uk);
   }
   if (indexer) {
+    need(iqr.size(1) == Hidx * D && w.size(1) == Hidx, "index_q_proj / index_weights_proj: wrong number of outputs");
     iq = fresh({rows, Hidx, D}, fp8 ? at::kByte : type, x);
     iw = fp8 ? fresh({rows, Hidx}, at::kFloat, x) : w.contiguous();
   }
@@ -842,12 +851,13 @@ PyObject* mlp(PyObject* const* a) {
     NoGil unlocked;
     Tensor act;
     void* st = stream();
-    if (small_f32(x, {&gate, &up})) {
+    if (small_f32(x, {&gate, &up}) && gate.size(0) == up.size(0)) {
       act = fresh({x.size(0), gate.size(0)}, type, x);
       ok(api.dsa_linear_f32(as<float>(x), x.size(0), int(x.size(1)), as<float>(gate), int(gate.size(0)), as<float>(act), as<float>(up),
                                 int(up.size(0)), nullptr, nullptr, 0, nullptr, 1, st));
     } else {
       const Tensor g = at::mm(x, gate.t()), u = at::mm(x, up.t());
+      need(g.is_cuda() && g.sizes() == u.sizes(), "gate and up must have one shape");
       act = at::empty_like(g);
       if (type == at::kFloat) ok(api.dsa_silu_mul_f32(as<float>(g), as<float>(u), as<float>(act), g.numel(), st));
       else ok(api.dsa_silu_mul_bf16(ptr(g), ptr(u), ptr(act), g.numel(), st));

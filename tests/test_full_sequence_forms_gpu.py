@@ -127,3 +127,42 @@ def test_gradients_after_a_pass_in_inference_mode(D, dtype):
     assert shorter.shape == (1, 17, model.config.hidden_size) and not model._rope_kept[1].mla_cos.is_inference()
     with torch.inference_mode():
         assert torch.equal(model(x, mode, cold), first)
+
+
+@pytest.mark.parametrize("name", ["q_a_proj", "kv_a_proj", "index_k_proj", "q_b_proj", "index_q_proj", "index_weights_proj", "kv_b_proj",
+                                  "o_proj", "gate_proj", "up_proj", "down_proj", "q_a_layernorm", "kv_a_layernorm"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_weights_on_another_device_are_refused(D, dtype, name):
+    """Never read by a kernel: torch's own error, or that of the argument checks."""
+    model = make_model(D, dtype)
+    x = tokens(model, 1, 33)
+    getattr(model.layers[0], name).cpu()
+    with torch.no_grad(), pytest.raises((RuntimeError, ValueError)):
+        model(x, D.ScheduleMode.BASELINE, D.ColdStartPolicy.EAGER)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_operands_of_other_widths_are_refused(D, dtype):
+    model = make_model(D, dtype)
+    layer, hidden = model.layers[0], model.config.hidden_size
+    x = tokens(model, 1, 33)
+    rope = model._build_rope(33, x.device, dtype)
+    refused = pytest.raises((RuntimeError, ValueError))
+    with torch.no_grad():
+        for width in (hidden - 4, hidden + 4, 2 * hidden):
+            with refused:
+                layer.full_operands(torch.zeros(1, 33, width, device="cuda", dtype=dtype), rope)
+            with refused:
+                layer.mlp(torch.zeros(1, 33, width, device="cuda", dtype=dtype))
+        c_q = layer.q_latent(x)
+        for bad in (c_q.cpu(), c_q[..., :-4], c_q.double()):
+            with refused:
+                layer.full_operands(x, rope, c_q=bad)
+        for field in ("mla_cos", "mla_sin", "idx_cos", "idx_sin"):
+            narrow = dataclasses.replace(rope, **{field: getattr(rope, field)[:, :-2].contiguous()})
+            with refused:
+                layer.full_operands(x, narrow)
+        wide = torch.nn.Linear(model.config.q_lora_rank, model.config.index_n_heads * model.config.index_head_dim - 4, bias=False)
+        layer.index_q_proj = wide.cuda().to(dtype)
+        with refused:
+            layer.full_operands(x, rope)
