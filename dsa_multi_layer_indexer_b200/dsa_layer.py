@@ -326,6 +326,8 @@ class DSALayer(nn.Module):
         dtype = t.dtype
         if not (t.is_cuda and (dtype == torch.float32 or self._fast_path(t))) or torch.is_grad_enabled() or torch.is_autocast_enabled():
             return None
+        if dtype == torch.bfloat16 and self.config.qk_nope_head_dim % 4:  # (8-byte reads behind the query heads' nope part)
+            return None
         if _module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks:
             return None
         mods, out = self._modules, []

@@ -23,13 +23,13 @@ def D():
     _lib.check_device_status()
 
 
-def make_model(D, dtype, layers=1):
+def make_model(D, dtype, layers=1, **kw):
     """Small layers whose norm weights are not ones (but numbers of every type used here)."""
     if dtype == torch.bfloat16:
         cfg = D.DSAConfig(hidden_size=192, num_hidden_layers=layers, num_attention_heads=16, q_lora_rank=96, index_n_heads=32,
-                          index_topk=64, intermediate_size=256, first_k_dense_replace=0)
+                          index_topk=64, intermediate_size=256, first_k_dense_replace=0, **kw)
     else:
-        cfg = dataclasses.replace(D.named_config("small"), num_hidden_layers=layers, first_k_dense_replace=0)
+        cfg = dataclasses.replace(D.named_config("small"), num_hidden_layers=layers, first_k_dense_replace=0, **kw)
     torch.manual_seed(5)
     model = D.DSAModel(cfg).eval()
     with torch.no_grad():
@@ -166,3 +166,20 @@ def test_operands_of_other_widths_are_refused(D, dtype):
         layer.index_q_proj = wide.cuda().to(dtype)
         with refused:
             layer.full_operands(x, rope)
+
+
+@pytest.mark.parametrize("nope", [30, 33, 36])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_query_heads_of_any_width(D, dtype, nope):
+    """Heads whose rotary part does not start on 8 bytes (bf16) take the modules, the others the fused chain."""
+    model = make_model(D, dtype, qk_nope_head_dim=nope)
+    x = tokens(model, 2, 41)
+    mode, cold = D.ScheduleMode.LAGGED_FUSED, D.ColdStartPolicy.DENSE
+    state = model.init_decode(2, 48, fp8=dtype == torch.bfloat16)  # (bf16: stacked projections)
+    filled = model.prefill(state, x, mode, cold)
+    with torch.no_grad():
+        got = model(x, mode, cold)
+    want = model(x, mode, cold).detach()  # autograd is on: the modules
+    tol = 3e-2 if dtype == torch.bfloat16 else 1e-4
+    for y in (got, filled):
+        assert float((y.float() - want.float()).norm()) <= tol * float(want.float().norm())
