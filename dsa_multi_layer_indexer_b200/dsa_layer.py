@@ -296,7 +296,7 @@ class DSALayer(nn.Module):
         if lens is None:
             lens = self._causal_lens(b, s, x_norm.device)
         weights = self._full_weights(x_norm)
-        if weights is not None and (cache is None or (cache.k_scale is not None) == self._fast_path(x_norm)):
+        if weights is not None and (cache is None or self._cache_fits(cache, x_norm)):
             return self._full_operands_fused(weights, x_norm, rope, c_q, attention, indexer, cache, lens)
         if c_q is None:
             c_q = self.q_latent(x_norm)
@@ -343,6 +343,18 @@ class DSALayer(nn.Module):
                 return None
             out.append(w)
         return tuple(out)
+
+    def _cache_fits(self, cache: "LayerDecodeCache", x: torch.Tensor) -> bool:
+        """Whether the fused chain can write ``cache`` in place: a dense cache of the scan's form and the
+        activations' type, one sequence each, on their device. Any other is filled by assignment, which
+        converts, broadcasts and copies across devices, or refuses."""
+        b, s, _ = x.shape
+        fp8 = self._fast_path(x)
+        kv, ik, scale = cache.kv, cache.index_k, cache.k_scale
+        return ((scale is not None) == fp8 and kv.dtype == x.dtype and ik.dtype == (torch.uint8 if fp8 else x.dtype)
+                and (not fp8 or scale.dtype == torch.float32)
+                and all(t.device == x.device and t.is_contiguous() and t.shape[0] == b and t.shape[1] >= s
+                        for t in (kv, ik, scale) if t is not None))
 
     def _full_operands_fused(self, weights, x_norm, rope, c_q, attention, indexer, cache, lens) -> "FullOperands":
         c = self.config

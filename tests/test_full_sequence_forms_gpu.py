@@ -183,3 +183,43 @@ def test_query_heads_of_any_width(D, dtype, nope):
     tol = 3e-2 if dtype == torch.bfloat16 else 1e-4
     for y in (got, filled):
         assert float((y.float() - want.float()).norm()) <= tol * float(want.float().norm())
+
+
+def _as(cache, change):
+    """A cache of another form than new_cache's, same contents after a fill."""
+    def strided(t):
+        return torch.zeros(t.shape[0], t.shape[1], 2, *t.shape[2:], dtype=t.dtype, device=t.device)[:, :, 1]
+
+    def wide(t):  # one prompt for three sequences
+        return torch.zeros(3, *t.shape[1:], dtype=t.dtype, device=t.device)
+
+    if change == "fp32 rows":
+        return dataclasses.replace(cache, kv=cache.kv.float())
+    if change == "bf16 rows":
+        return dataclasses.replace(cache, kv=cache.kv.to(torch.bfloat16))
+    make = {"broadcast": wide, "host": lambda t: torch.zeros_like(t, device="cpu"), "strided": strided}[change]
+    return type(cache)(make(cache.index_k), None if cache.k_scale is None else make(cache.k_scale), make(cache.kv))
+
+
+@pytest.mark.parametrize("dtype,change", [(torch.bfloat16, c) for c in ("broadcast", "host", "strided", "fp32 rows")] + [
+    (torch.float32, c) for c in ("broadcast", "host", "strided", "bf16 rows")])
+def test_caches_of_other_forms_are_filled(D, dtype, change):
+    model = make_model(D, dtype)
+    layer, x = model.layers[0], tokens(model, 1, 37)
+    rope = model._build_rope(37, x.device, dtype)
+    plain = layer.new_cache(1, 40, x.device, fp8=dtype == torch.bfloat16)
+    other = _as(plain, change)
+    with torch.no_grad():
+        layer.fill_cache(plain, x, rope)
+        layer.fill_cache(other, x, rope)
+    # (by other kernels: a unit in the last place of the type that is stored)
+    for a, b, scale in ((plain.kv, other.kv, None), (plain.index_k, other.index_k, (plain.k_scale, other.k_scale))):
+        a, b = a[:, :37], b[:, :37]
+        if scale and scale[0] is not None:
+            a, b = (t.view(torch.float8_e4m3fn).float() * s[:, :37, None] for t, s in ((a, scale[0]), (b.contiguous(), scale[1])))
+        tol = 2.0 ** -4 if scale and scale[0] is not None else 2.0 ** -7 if torch.bfloat16 in (a.dtype, b.dtype) else 1e-5
+        a, b = a.float().cpu().expand(b.shape), b.float().cpu()
+        assert float((a - b).abs().max()) <= tol * float(a.abs().max()) and float(b.abs().max()) > 0
+    short = type(plain)(plain.index_k[:, :30], None if plain.k_scale is None else plain.k_scale[:, :30], plain.kv[:, :30])
+    with torch.no_grad(), pytest.raises((RuntimeError, ValueError)):
+        layer.fill_cache(short, x, rope)
