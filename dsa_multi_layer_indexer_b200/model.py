@@ -156,6 +156,9 @@ class DSAModel(nn.Module):
             raise ValueError(f"inputs_embeds must be [B,S,H], got {tuple(inputs_embeds.shape)}")
         if not inputs_embeds.is_cuda:
             raise RuntimeError("this implementation runs on a CUDA device only (there is no CPU path)")
+        # (a plain "baseline" equals the member, but is not taken for it: it would run the lagged schedule)
+        if mode is not ScheduleMode.BASELINE and mode not in (ScheduleMode.LAGGED_REFERENCE, ScheduleMode.LAGGED_FUSED):
+            raise ValueError(f"unknown schedule mode: {mode}")
         rope = self._rope_for(inputs_embeds.shape[1], inputs_embeds.device, inputs_embeds.dtype)
         used, produced = ([], []) if record else (None, None)
         x = self._run_full(inputs_embeds, rope, mode, cold_start, None, used, produced)
@@ -166,8 +169,6 @@ class DSAModel(nn.Module):
         """The full-sequence layers under a schedule (reference model.py:92-144), filling ``caches`` on
         the way if given; returns the final norm's output. A layer's projections are computed once for
         the caches, its indexer and its attention; the selections stay int32 between the layers."""
-        if mode not in (ScheduleMode.BASELINE, ScheduleMode.LAGGED_REFERENCE, ScheduleMode.LAGGED_FUSED):
-            raise ValueError(f"unknown schedule mode: {mode}")
         b, s, _ = x.shape
         types = self.config.resolved_attention_types
         produces = lagged_producers(types)
@@ -178,7 +179,7 @@ class DSAModel(nn.Module):
         for li, layer in enumerate(self.layers):
             is_dsa = types[li] is AttentionType.DSA
             cold = lagged and is_dsa and li == 0
-            if cold and cold_start not in (ColdStartPolicy.DENSE, ColdStartPolicy.EAGER):
+            if cold and cold_start is not ColdStartPolicy.DENSE and cold_start is not ColdStartPolicy.EAGER:
                 raise ValueError(f"unknown cold start policy: {cold_start}")
             eager = cold and cold_start is ColdStartPolicy.EAGER  # layer 0 attends its own selection
             makes = produces[li] if lagged else is_dsa

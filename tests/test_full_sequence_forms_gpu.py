@@ -223,3 +223,19 @@ def test_caches_of_other_forms_are_filled(D, dtype, change):
     short = type(plain)(plain.index_k[:, :30], None if plain.k_scale is None else plain.k_scale[:, :30], plain.kv[:, :30])
     with torch.no_grad(), pytest.raises((RuntimeError, ValueError)):
         layer.fill_cache(short, x, rope)
+
+
+def test_schedules_and_policies_are_members_not_their_names(D):
+    """"baseline" and "eager" equal the members they name; taken by equality in one place and by identity in the
+    next they would run the other schedule."""
+    model = make_model(D, torch.float32, layers=2)
+    x = tokens(model, 1, 24)
+    with torch.no_grad():
+        for mode, cold in (("baseline", D.ColdStartPolicy.EAGER), ("unknown", D.ColdStartPolicy.EAGER),
+                           (D.ScheduleMode.LAGGED_FUSED, "eager"), (D.ScheduleMode.LAGGED_FUSED, "unknown")):
+            with pytest.raises(ValueError):
+                model(x, mode, cold)
+        want = model(x, D.ScheduleMode.LAGGED_FUSED, D.ColdStartPolicy.EAGER)
+        assert torch.equal(model(x, "lagged_fused", D.ColdStartPolicy.EAGER), want)
+    state = model.init_decode(1, 32, fp8=False)
+    assert torch.equal(model.prefill(state, x, "lagged", D.ColdStartPolicy.EAGER), want)  # (prefill: all but BASELINE lag)
