@@ -175,7 +175,7 @@ class DSAModel(nn.Module):
         lagged = mode is not ScheduleMode.BASELINE
         prev: Optional[torch.Tensor] = None
         lens = DSALayer._causal_lens(b, s, x.device)
-        x_norm = self.layers[0].attn_norm(x)
+        x_norm = (self.layers[0].attn_norm if len(self.layers) else self.final_norm)(x)
         for li, layer in enumerate(self.layers):
             is_dsa = types[li] is AttentionType.DSA
             cold = lagged and is_dsa and li == 0

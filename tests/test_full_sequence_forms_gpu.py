@@ -239,3 +239,10 @@ def test_schedules_and_policies_are_members_not_their_names(D):
         assert torch.equal(model(x, "lagged_fused", D.ColdStartPolicy.EAGER), want)
     state = model.init_decode(1, 32, fp8=False)
     assert torch.equal(model.prefill(state, x, "lagged", D.ColdStartPolicy.EAGER), want)  # (prefill: all but BASELINE lag)
+
+
+def test_a_model_without_layers_is_its_final_norm(D):
+    model = make_model(D, torch.float32, layers=0)
+    x = torch.randn(2, 9, model.config.hidden_size, device="cuda")
+    with torch.no_grad():
+        assert torch.equal(model(x, D.ScheduleMode.BASELINE), model.final_norm(x))
