@@ -32,9 +32,11 @@ from .rope import apply_rotary, apply_rotary_at
 
 
 def _bare(m: nn.Module, cls: type) -> bool:
-    """Whether calling ``m`` is ``cls.forward`` and nothing else: no subclass, no hooks, no replaced ``forward``."""
+    """Whether calling ``m`` is ``cls.forward`` and nothing else: no subclass, no hooks (its own or those of every
+    module), no replaced ``forward``."""
     d = m.__dict__
-    return m.__class__ is cls and not d["_forward_hooks"] and not d["_forward_pre_hooks"] and "forward" not in d
+    return (m.__class__ is cls and not d["_forward_hooks"] and not d["_forward_pre_hooks"] and "forward" not in d
+            and not _module_hooks._global_forward_hooks and not _module_hooks._global_forward_pre_hooks)
 
 
 # The linear projections of a layer, in construction order.
@@ -74,6 +76,14 @@ class RMSNorm(nn.Module):
         xf = x.float()
         inv = torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps)
         return (xf * inv * self.weight.float()).to(x.dtype)
+
+
+def add_norm(norm: nn.Module, x: torch.Tensor, delta: torch.Tensor):
+    """``(x + delta, norm(x + delta))``, in one launch where the norm is a plain RMSNorm (``add_forward``)."""
+    if _bare(norm, RMSNorm):
+        return norm.add_forward(x, delta)
+    s = x + delta
+    return s, norm(s)
 
 
 @dataclasses.dataclass
@@ -328,8 +338,6 @@ class DSALayer(nn.Module):
             return None
         if dtype == torch.bfloat16 and self.config.qk_nope_head_dim % 4:  # (8-byte reads behind the query heads' nope part)
             return None
-        if _module_hooks._global_forward_hooks or _module_hooks._global_forward_pre_hooks:
-            return None
         mods, out = self._modules, []
         qn, kn = mods["q_a_layernorm"], mods["kv_a_layernorm"]
         if not (_bare(qn, RMSNorm) and _bare(kn, RMSNorm) and qn.eps == kn.eps and qn.weight.dtype == dtype == kn.weight.dtype):
@@ -474,8 +482,7 @@ class DSALayer(nn.Module):
 
     def _norm_folds(self, norm: RMSNorm, x: torch.Tensor) -> bool:
         """Whether ``norm`` can run inside the projection that follows it (:func:`ops.norm_gemv`)."""
-        return (norm.__class__ is RMSNorm and not norm._forward_hooks and not norm._forward_pre_hooks
-                and x.is_cuda and x.dtype == torch.bfloat16 and norm.weight.dtype == torch.bfloat16
+        return (_bare(norm, RMSNorm) and x.is_cuda and x.dtype == torch.bfloat16 and norm.weight.dtype == torch.bfloat16
                 and not torch.is_grad_enabled() and ops.norm_gemv_fits(x.shape[0], x.shape[1]))
 
     def decode_residual_project(self, x, delta, rope: RopeCaches, positions, cache: LayerDecodeCache, batch_index):
@@ -489,7 +496,7 @@ class DSALayer(nn.Module):
         if delta is None:
             x_norm = self.attn_norm(x)
         else:
-            x, x_norm = self.attn_norm.add_forward(x, delta)
+            x, x_norm = add_norm(self.attn_norm, x, delta)
         return x, self.decode_project(x_norm, rope, positions, cache, batch_index)
 
     def decode_mlp(self, x: torch.Tensor, attn: torch.Tensor):
@@ -498,7 +505,7 @@ class DSALayer(nn.Module):
                 and self._norm_folds(self.ffn_norm, x) and self._plain("gate_proj") and self._plain("up_proj")):
             h, act = ops.norm_gemv(x, attn, self.ffn_norm.weight, self.ffn_norm.eps, self.gate_proj.weight, self.up_proj.weight)
             return h, self._reduced(self._skinny("down_proj", act))
-        h, h_norm = self.ffn_norm.add_forward(x, attn)
+        h, h_norm = add_norm(self.ffn_norm, x, attn)
         return h, self.mlp(h_norm)
 
     def decode_project(self, x_norm, rope: RopeCaches, positions, cache: LayerDecodeCache, batch_index, ya=None):

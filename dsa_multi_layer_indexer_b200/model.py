@@ -25,7 +25,7 @@ import torch
 from torch import nn
 
 from .config import AttentionType, ColdStartPolicy, DSAConfig, ScheduleMode
-from .dsa_layer import DSALayer, IndexerWorkspace, LayerDecodeCache, RMSNorm, RopeCaches
+from .dsa_layer import DSALayer, IndexerWorkspace, LayerDecodeCache, RMSNorm, RopeCaches, add_norm
 from .rope import build_rope_cache
 
 
@@ -329,16 +329,16 @@ class DSAModel(nn.Module):
         state.carried = carried
         if record is not None:
             record["used"], record["produced"] = used, produced
-        return self.final_norm.add_forward(x, delta)[1]
+        return add_norm(self.final_norm, x, delta)[1]
 
     def _residual_tail(self, li: int, x: torch.Tensor, attn: torch.Tensor, weights=None):
         """``h = x + attn; x' = h + mlp(ffn_norm(h))`` and the norm the next consumer
         applies to ``x'`` (the next layer's attn_norm, or the final norm after the last
         layer): each residual addition is fused with the norm that follows it."""
         layer = self.layers[li]
-        h, h_norm = layer.ffn_norm.add_forward(x, attn)
+        h, h_norm = add_norm(layer.ffn_norm, x, attn)
         nxt = self.layers[li + 1].attn_norm if li + 1 < len(self.layers) else self.final_norm
-        return nxt.add_forward(h, layer.mlp(h_norm, weights) if weights is not None else layer.mlp(h_norm))
+        return add_norm(nxt, h, layer.mlp(h_norm, weights) if weights is not None else layer.mlp(h_norm))
 
     def _decode_step_depth(self, state: DecodeState, x: torch.Tensor, cold_start: ColdStartPolicy,
                            overlap: bool, record: Optional[dict], depth: int) -> torch.Tensor:
@@ -416,7 +416,7 @@ class DSAModel(nn.Module):
         state.carried = carried
         if record is not None:
             record["used"], record["produced"] = used, produced
-        return self.final_norm.add_forward(x, delta)[1]
+        return add_norm(self.final_norm, x, delta)[1]
 
     def capture_decode(self, state: DecodeState, mode: ScheduleMode,
                        cold_start: ColdStartPolicy = ColdStartPolicy.DENSE, overlap=True,

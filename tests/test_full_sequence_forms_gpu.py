@@ -246,3 +246,49 @@ def test_a_model_without_layers_is_its_final_norm(D):
     x = torch.randn(2, 9, model.config.hidden_size, device="cuda")
     with torch.no_grad():
         assert torch.equal(model(x, D.ScheduleMode.BASELINE), model.final_norm(x))
+
+
+class ScaledNorm(torch.nn.Module):
+    """A norm that is no RMSNorm and knows nothing of residuals."""
+
+    def forward(self, t):
+        return (t.float() * torch.rsqrt(t.float().pow(2).mean(-1, keepdim=True) + 1e-6) * 1.5).to(t.dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("change", ["hook", "replaced", "global hook"])
+def test_residual_norms_are_called_as_modules(D, dtype, change):
+    """attn_norm, ffn_norm and final_norm: hooks see every call, replacements take their place."""
+    model = make_model(D, dtype, layers=2)
+    x = tokens(model, 2, 24)
+    mode, cold = D.ScheduleMode.BASELINE, D.ColdStartPolicy.DENSE
+    places = [(l, n) for l in model.layers for n in ("attn_norm", "ffn_norm")] + [(model, "final_norm")]
+    seen = []
+    if change == "replaced":
+        for owner, name in places:
+            setattr(owner, name, ScaledNorm())
+    elif change == "hook":
+        for owner, name in places:
+            getattr(owner, name).register_forward_hook(lambda m, a, o: seen.append(m) or o * 1.5)
+    else:
+        norms = [getattr(owner, name) for owner, name in places]
+        handle = torch.nn.modules.module.register_module_forward_hook(
+            lambda m, a, o: seen.append(m) if any(m is n for n in norms) else None)
+    try:
+        with torch.no_grad():
+            got = model(x, mode, cold)
+        calls = list(seen)
+        state = model.init_decode(2, 32, fp8=dtype == torch.bfloat16)
+        filled = model.prefill(state, x[:, :23], mode, cold)
+        seen.clear()
+        step = model.decode_step(state, x[:, 23], mode, cold)
+        if change != "replaced":
+            in_order = [getattr(owner, name) for owner, name in places]
+            assert [id(m) for m in calls] == [id(m) for m in in_order] == [id(m) for m in seen]
+        want = model(x, mode, cold).detach()  # autograd is on: the modules one by one
+    finally:
+        if change == "global hook":
+            handle.remove()
+    tol = 3e-2 if dtype == torch.bfloat16 else 1e-3  # (topk keys of a cutoff within rounding may change places)
+    for a, b in ((got, want), (filled, want[:, :23]), (step, want[:, 23])):
+        assert float((a.float() - b.float()).norm()) <= tol * float(b.float().norm())
