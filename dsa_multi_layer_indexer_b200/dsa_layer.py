@@ -39,6 +39,20 @@ def _bare(m: nn.Module, cls: type) -> bool:
             and not _module_hooks._global_forward_hooks and not _module_hooks._global_forward_pre_hooks)
 
 
+def _plain_weight(m: nn.Module, dtype: torch.dtype) -> Optional[torch.Tensor]:
+    """The weight of a bias-free ``nn.Linear`` that only multiplies by it - nothing hooked, replaced, patched or
+    quantised (a tensor subclass has its own product) - or None. (Hooks of every module: see ``_bare``.)"""
+    d = m.__dict__
+    p = d["_parameters"]
+    w = p.get("weight")
+    if (m.__class__ is not nn.Linear or w is None or w.dtype != dtype or p.get("bias") is not None or d["_forward_hooks"]
+            or d["_forward_pre_hooks"] or "forward" in d or w.__class__ not in _PLAIN_TENSORS):
+        return None
+    return w
+
+
+_PLAIN_TENSORS = (nn.Parameter, torch.Tensor)
+
 # The linear projections of a layer, in construction order.
 _PROJECTIONS = ("q_a_proj", "q_b_proj", "kv_a_proj", "kv_b_proj", "o_proj", "index_q_proj", "index_k_proj",
                 "index_weights_proj", "gate_proj", "up_proj", "down_proj")
@@ -343,11 +357,8 @@ class DSALayer(nn.Module):
         if not (_bare(qn, RMSNorm) and _bare(kn, RMSNorm) and qn.eps == kn.eps and qn.weight.dtype == dtype == kn.weight.dtype):
             return None
         for name in _PROJECTIONS:
-            m = mods[name]
-            d = m.__dict__
-            w = d["_parameters"].get("weight")
-            if (m.__class__ is not nn.Linear or w is None or w.dtype != dtype or d["_parameters"].get("bias") is not None
-                    or d["_forward_hooks"] or d["_forward_pre_hooks"]):
+            w = _plain_weight(mods[name], dtype)
+            if w is None:
                 return None
             out.append(w)
         return tuple(out)
@@ -453,16 +464,17 @@ class DSALayer(nn.Module):
         return ops.gemv(x, m.weight)
 
     def _plain(self, name: str) -> bool:
-        """A bias-free bf16 ``nn.Linear`` without hooks, of a width that the GEMV takes."""
+        """A bias-free bf16 ``nn.Linear`` that only multiplies, of a width that the GEMV takes."""
         m = self._modules[name]
-        return (m.__class__ is nn.Linear and m.bias is None and m.weight.dtype == torch.bfloat16 and not m._forward_hooks
-                and not m._forward_pre_hooks and m.in_features % 8 == 0 and m.weight.is_contiguous())
+        w = _plain_weight(m, torch.bfloat16)
+        return (w is not None and not _module_hooks._global_forward_hooks and not _module_hooks._global_forward_pre_hooks
+                and not torch.is_autocast_enabled() and m.in_features % 8 == 0 and w.is_contiguous())
 
     def _absorbed_rows(self, x: torch.Tensor) -> bool:
         """Whether a decode batch takes the kernels that read kv_b_proj's weight in place (one reading for all
         tokens; beyond HEAD_TOKENS rows the products are GEMMs)."""
         c, w = self.config, self.kv_b_proj.weight
-        return (x.shape[0] <= ops.HEAD_TOKENS and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.is_contiguous()
+        return (x.shape[0] <= ops.HEAD_TOKENS and x.dtype == torch.bfloat16 and w.__class__ in _PLAIN_TENSORS and w.dtype == torch.bfloat16 and w.is_contiguous()
                 and c.qk_nope_head_dim <= 512 and c.qk_nope_head_dim % 8 == 0 and c.q_lora_rank % 8 == 0 and not torch.is_grad_enabled())
 
     def new_cache(self, n_seq: int, capacity: int, device, fp8: bool) -> LayerDecodeCache:

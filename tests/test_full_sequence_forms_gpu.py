@@ -292,3 +292,52 @@ def test_residual_norms_are_called_as_modules(D, dtype, change):
     tol = 3e-2 if dtype == torch.bfloat16 else 1e-3  # (topk keys of a cutoff within rounding may change places)
     for a, b in ((got, want), (filled, want[:, :23]), (step, want[:, 23])):
         assert float((a.float() - b.float()).norm()) <= tol * float(b.float().norm())
+
+
+class ScaledWeight(torch.nn.Parameter):
+    """A weight with a product of its own, as quantised weights have: F.linear through __torch_function__."""
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        with torch._C.DisableTorchFunctionSubclass():
+            if func is torch.nn.functional.linear:
+                return func(args[0], args[1].as_subclass(torch.Tensor) * 1.5)
+            return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("change", ["forward", "weight", "global hook"])
+@pytest.mark.parametrize("name", ["o_proj", "gate_proj", "up_proj", "down_proj"])
+def test_changed_projections_are_honoured(D, dtype, change, name):
+    """A patched forward (as offloading and adapter libraries do), a weight of another tensor class, hooks of
+    every module: forward without gradients, prefill and the decode step against the module path."""
+    model = make_model(D, dtype)
+    x = tokens(model, 2, 24)
+    mode, cold = D.ScheduleMode.LAGGED_FUSED, D.ColdStartPolicy.DENSE
+    with torch.no_grad():
+        plain = model(x, mode, cold)
+    layer, fp8 = model.layers[0], dtype == torch.bfloat16
+    m = getattr(layer, name)
+    if change == "forward":
+        inner = m.forward
+        m.forward = lambda t: inner(t) * 1.5
+    elif change == "weight":
+        m.weight = ScaledWeight(m.weight.detach())
+    else:
+        handle = torch.nn.modules.module.register_module_forward_hook(lambda mod, a, o: o * 1.5 if mod is m else None)
+    try:
+        with torch.no_grad():
+            got = model(x, mode, cold)
+        state = model.init_decode(2, 32, fp8=fp8)
+        outs = [(got, slice(None)), (model.prefill(state, x[:, :23], mode, cold), slice(0, 23))]
+        if name in ("o_proj", "down_proj"):  # (the decode step reads the weights of gate and up itself)
+            outs.append((model.decode_step(state, x[:, 23], mode, cold)[:, None], slice(23, 24)))
+        want = model(x, mode, cold).detach()  # autograd is on: the modules one by one
+    finally:
+        if change == "global hook":
+            handle.remove()
+    tol = 3e-2 if dtype == torch.bfloat16 else 1e-3
+    for y, rows in outs:
+        ref = want[:, rows].float()
+        assert float((y.float() - ref).norm()) <= tol * float(ref.norm())
+    assert float((want.float() - plain.float()).norm()) > 5e-2 * float(plain.float().norm())
