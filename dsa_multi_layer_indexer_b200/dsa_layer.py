@@ -30,6 +30,9 @@ from . import _lib, ops
 from .config import DSAConfig
 from .rope import apply_rotary, apply_rotary_at
 
+# What fuse_decode_weights stacks: everything that reads x_norm, then everything that reads c_q.
+_STACKS = (("_wx", ("q_a_proj", "kv_a_proj", "index_k_proj")), ("_wc", ("q_b_proj", "index_q_proj", "index_weights_proj")))
+
 
 def _bare(m: nn.Module, cls: type) -> bool:
     """Whether calling ``m`` is ``cls.forward`` and nothing else: no subclass, no hooks (its own or those of every
@@ -227,8 +230,8 @@ class DSALayer(nn.Module):
         ``load_state_dict`` keep working, and moving or casting the module afterwards
         simply drops the stacking (``decode_project`` notices and uses the six)."""
         with torch.no_grad():
-            for name, mods in (("_wx", (self.q_a_proj, self.kv_a_proj, self.index_k_proj)),
-                               ("_wc", (self.q_b_proj, self.index_q_proj, self.index_weights_proj))):
+            for name, parts in _STACKS:
+                mods = [self._modules[p] for p in parts]
                 stacked = torch.cat([m.weight for m in mods], dim=0)
                 row = 0
                 for m in mods:
@@ -238,12 +241,20 @@ class DSALayer(nn.Module):
                 setattr(self, name, stacked)
 
     def _stacked(self) -> bool:
-        wx, wc = getattr(self, "_wx", None), getattr(self, "_wc", None)
-        return (wx is not None and wc is not None and self.q_a_proj.weight.data_ptr() == wx.data_ptr()
-                and self.q_b_proj.weight.data_ptr() == wc.data_ptr()
-                and self.index_k_proj.weight.data_ptr() == wx[wx.shape[0] - self.index_k_proj.weight.shape[0]:].data_ptr()
-                and self.index_weights_proj.weight.data_ptr()
-                == wc[wc.shape[0] - self.index_weights_proj.weight.shape[0]:].data_ptr())
+        """Whether the stacked weights are still the six parameters' own memory (any of them may have been given
+        other memory since, by assignment to the parameter or its data)."""
+        d, mods = self.__dict__, self._modules
+        for name, parts in _STACKS:
+            stack = d.get(name)
+            if stack is None:
+                return False
+            at, step = stack.data_ptr(), stack.stride(0) * stack.element_size()
+            for part in parts:
+                w = mods[part].weight
+                if w.data_ptr() != at or w.dtype != stack.dtype:
+                    return False
+                at += w.shape[0] * step
+        return True
 
     # ------------------------------------------------------------------ projections (torch)
     def q_latent(self, x_norm: torch.Tensor) -> torch.Tensor:

@@ -341,3 +341,39 @@ def test_changed_projections_are_honoured(D, dtype, change, name):
         ref = want[:, rows].float()
         assert float((y.float() - ref).norm()) <= tol * float(ref.norm())
     assert float((want.float() - plain.float()).norm()) > 5e-2 * float(plain.float().norm())
+
+
+@pytest.mark.parametrize("name", ["q_a_proj", "kv_a_proj", "index_k_proj", "q_b_proj", "index_q_proj", "index_weights_proj"])
+@pytest.mark.parametrize("how", ["parameter", "data"])
+def test_a_weight_replaced_after_stacking_is_the_one_that_runs(D, name, how):
+    """init_decode stacks three weights each; prompts and decode steps must notice that one of them (the middle
+    one too) has been given other memory."""
+    model = make_model(D, torch.bfloat16)
+    state = model.init_decode(1, 40)
+    layer, x = model.layers[0], tokens(model, 1, 24)
+    m = getattr(layer, name)
+    new = torch.randn_like(m.weight) * 0.2
+    if how == "parameter":
+        m.weight = torch.nn.Parameter(new)
+    else:
+        m.weight.data = new
+    rope = model._build_rope(24, x.device, x.dtype)
+    with torch.no_grad():
+        op = layer.full_operands(x, rope)
+        q, iq, iw = layer.decode_project(x[:, 5], state.rope, torch.full((1,), 5, device="cuda"), state.caches[0], state.batch_index)
+    want = layer.full_operands(x, rope)  # autograd is on: the modules
+    assert op.fused and not want.fused
+    f8 = lambda t: t.view(torch.float8_e4m3fn).float()
+
+    def near(a, b, tol=3e-2):
+        assert float((a.float() - b.detach().float()).norm()) <= tol * float(b.detach().float().norm())
+
+    # (a bf16 rounding apart; e4m3 bytes against the unquantised keys: half a step of 2^-3 at most)
+    near(op.q, want.q)
+    near(op.kv, want.kv)
+    near(f8(op.ik) * op.ik_scale[..., None], want.ik, 6e-2)
+    near(f8(op.iq) * op.iw[..., None], want.iq * want.iw[..., None], 6e-2)
+    near(q[0], want.q[5])
+    near(f8(iq[0]) * iw[0, :, None], want.iq[5] * want.iw[5, :, None], 6e-2)
+    near(state.caches[0].kv[0, 5], want.kv[0, 5])
+    near(f8(state.caches[0].index_k[0, 5]) * state.caches[0].k_scale[0, 5], want.ik[0, 5], 6e-2)
