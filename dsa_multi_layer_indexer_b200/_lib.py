@@ -58,9 +58,10 @@ SIGNATURES: Dict[str, Tuple[object, List[object]]] = {
     "dsa_silu_mul_f32": (_i, [_p, _p, _p, _l, _p]),
     "dsa_silu_mul_bf16": (_i, [_p, _p, _p, _l, _p]),
     "dsa_gemv_bf16": (_i, [_p, _p, _p, _i, _i, _i, _l, _l, _p]),
-    "dsa_gemv_swiglu_bf16": (_i, [_p, _p, _p, _p, _i, _i, _i, _l, _l, _p]),
-    "dsa_norm_gemv_bf16": (_i, [_p, _p, _p, _p, _p, _f, _p, _p, _i, _i, _i, _l, _l, _p]),
-    "dsa_value_project": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _p]),
+    "dsa_gemv_ahead_bf16": (_i, [_p, _p, _p, _i, _i, _i, _l, _l, _p]),
+    "dsa_gemv_swiglu_bf16": (_i, [_p, _p, _p, _p, _i, _i, _i, _l, _l, _i, _p]),
+    "dsa_norm_gemv_bf16": (_i, [_p, _p, _p, _p, _p, _f, _p, _p, _i, _i, _i, _l, _l, _i, _p]),
+    "dsa_value_project": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, _p]),
     "dsa_copy_bytes": (_i, [_p, _p, _l, _p]),
     "dsa_copy_bytes_beside": (_i, [_p, _p, _l, _p]),
     "dsa_post_epoch": (_i, [_p, _p, _p]),
@@ -68,14 +69,14 @@ SIGNATURES: Dict[str, Tuple[object, List[object]]] = {
     "dsa_indexer_stage_fp8": (_i, [_p, _p, _p, _p, _p, _f, _p, _p, _p, _p, _p, _p, _p, _p, _l, _p, _l,
                                    _i, _i, _l, _i, _i, _f, _f, _p]),
     "dsa_latent_append": (_i, [_p, _p, _f, _p, _p, _p, _p, _p, _i, _l, _l, _i, _i, _i, _p]),
-    "dsa_decode_token": (_i, [_p, _l, _p, _l, _p, _l, _p, _l, _p, _l] + [_p] * 13 + [_i] * 5 + [_l, _i, _f, _p]),
+    "dsa_decode_token": (_i, [_p, _l, _p, _l, _p, _l, _p, _l, _p, _l] + [_p] * 13 + [_i] * 5 + [_l, _i, _f, _i, _p]),
     "dsa_decode_prep": (_i, [_p, _p, _p, _p, _p, _p, _l] + [_p] * 12 + [_i, _i, _i, _l, _i, _f, _p]),
     "dsa_prefill_latents": (_i, [_p, _l, _p, _l, _p, _l] + [_p] * 8 + [_l, _p, _p, _l, _l] + [_i] * 6 + [_f, _i, _p]),
     "dsa_prefill_queries": (_i, [_p, _l, _l, _i, _p, _l, _p, _l] + [_p] * 7 + [_l] + [_i] * 8 + [_p]),
     "dsa_quantize_e4m3_rowwise": (_i, [_p, _p, _p, _l, _i, _f, _p]),
 }
 
-ABI_VERSION = 10
+ABI_VERSION = 11
 
 
 class DsaError(RuntimeError):

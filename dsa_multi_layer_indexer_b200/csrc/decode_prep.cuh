@@ -271,9 +271,11 @@ copy_post_epoch_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, i
 // soon as it has read it: no barrier between warps, no register holding a load in flight. A warp's pieces
 // are consecutive, its sum stays in registers until the pair changes, and the warps' sums of a pair are
 // folded in order at the end (a pair can span warps: the parts of a row are dealt out evenly).
-// The rings are filled BEFORE the dependency wait, which hides the launch and the latency of the kernel in
-// front: no kernel of this library writes weights, and any other kernel in front completes before its
-// successor starts.
+// With `ahead` the rings are filled BEFORE the dependency wait, which hides the launch and the latency of the
+// kernel in front. That is sound only if nothing that may still be running writes the weights: a kernel in
+// front that releases its dependents early (every kernel of this library, some of the GEMM library's) lets
+// this one start while its own stores, or those of the kernel before it, are still on their way. The caller
+// says so; without it the weights wait too.
 // One row of x, [2240, 7168] 13.0 -> 7.5 us, [32832, 1536] 18.5 -> 17.5 us (kernel below); against the
 // library's GEMV [7168, 16384] 39.7 -> 37.0 us (6.35 TB/s), [7168, 18432] 42.8 -> 41.2, SwiGLU 2 x [18432,
 // 7168] 41.3 + 41.3 + product -> 79.6. 96 KB in flight instead of 144 make [32832, 1536] 27 us behind another
@@ -297,6 +299,7 @@ struct GemvParams {
   const __nv_bfloat16* norm_w;
   __nv_bfloat16* sum_out;
   float eps;
+  int ahead;  // the weights (and norm_w) are read before the dependency wait
   int rows, n, k, slots, ks, chunks;  // rows <= B of x; ks pieces of up to `chunks` 16-byte chunks per row
   int64_t x_stride, y_stride;
 };
@@ -331,6 +334,7 @@ gemv_stream_kernel(const GemvParams p) {
     bulk_g2s(dst + uint32_t(pl) * 16u, r1, bytes, bar);
     if (++ip == ks) ip = 0, ++iu;
   };
+  if (!p.ahead) pdl_wait();
   if (lane == 0) {
     for (int i = 0; i < slots; ++i) mbar_init(smem_u32(&full[i]), 1);
     mbar_fence_init();
@@ -720,8 +724,8 @@ decode_prep_kernel(const Params p) {
 // A decode token's products with kv_b_proj's weight [H][nope + v][512] (src/lagged_indexer_dsa/dsa_layer.py:
 // 96-125) for NB tokens at a time: W_UK absorbed into the query (with every other item of decode_prep_kernel
 // in the same launch, nothing of which depends on it) and W_UV applied to the attention's output.
-// Bound by the latency of reading 128 - 256 KB per head in one CTA; the first 64 KB are loaded before the
-// dependency wait. (Bulk prefetches of the rest into L2, of W_UV two launches ahead, or of the first 16 - 96 MB
+// Bound by the latency of reading 128 - 256 KB per head in one CTA; with `ahead` (as in gemv_stream_kernel) the
+// first 64 KB are loaded before the dependency wait. (Bulk prefetches of the rest into L2, of W_UV two launches ahead, or of the first 16 - 96 MB
 // of o_proj's weight while scan and top-k leave the memory idle: nothing gained, up to 1 % lost.)
 // One token of 128 heads of 128 + 128 behind its projection: 11.9 -> 6.7 us (absorption and the other items
 // were two launches), value projection 7.5 -> 5.2 us. Four / eight tokens: with the copies of the strided
@@ -735,6 +739,7 @@ struct HeadParams {
   __nv_bfloat16* out;      // [B, H, v_dim] (value projection)
   int64_t q_row, q_head;
   int nope, v_dim, H, B, o_heads;
+  int ahead;               // kv_b is read before the dependency wait
 };
 template <int NB>
 __global__ void __launch_bounds__(kHeadThreads, NB <= 2 ? 2 : 1)
@@ -756,6 +761,7 @@ decode_token_kernel(const Params p, const HeadParams hp) {
   const __nv_bfloat16* w_head = hp.kv_b + int64_t(h) * (nope + hp.v_dim) * DSA_VALUE_DIM;
   const uint4* wr = reinterpret_cast<const uint4*>(w_head) + c;
   uint4 wv[8];
+  if (!hp.ahead) pdl_wait();
 #pragma unroll
   for (int u = 0; u < 8; ++u) wv[u] = g + 8 * u < nope ? wr[int64_t(g + 8 * u) * 64] : make_uint4(0, 0, 0, 0);
   pdl_wait();
@@ -833,6 +839,7 @@ value_project_kernel(const HeadParams hp) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) wv[u][j] = d + u < v_dim ? wr[int64_t(d + u) * 64 + 32 * j] : make_uint4(0, 0, 0, 0);
   };
+  if (!hp.ahead) pdl_wait();
   load(4 * warp);
   pdl_wait();
   pdl_launch_dependents();

@@ -1147,20 +1147,21 @@ static int launch_gemv_rows(const void* w, const void* x, void* y, int n, int k,
 }  // extern "C++"
 
 static int gemv_checks(prep::GemvParams& p, const void* w, const void* x, void* y, int batch, int most, int n, int k, int64_t x_stride,
-                       int64_t y_stride) {
+                       int64_t y_stride, int ahead) {
   DSA_REQUIRE(w && x && y, "gemv: null pointer");
   DSA_REQUIRE(batch >= 1 && batch <= most, "gemv: batch=%d must be 1..%d", batch, most);
   DSA_REQUIRE(n > 0 && k > 0 && k % 8 == 0, "gemv: k=%d must be a positive multiple of 8", k);
   DSA_REQUIRE(x_stride >= k && x_stride % 8 == 0 && y_stride >= n, "gemv: bad row strides");
   DSA_REQUIRE(aligned16(w) && aligned16(x), "gemv: w and x must be 16-byte aligned");
   p.w = static_cast<const __nv_bfloat16*>(w), p.x = static_cast<const __nv_bfloat16*>(x), p.y = static_cast<__nv_bfloat16*>(y);
-  p.rows = batch, p.n = n, p.k = k, p.x_stride = x_stride, p.y_stride = y_stride;
+  p.rows = batch, p.n = n, p.k = k, p.x_stride = x_stride, p.y_stride = y_stride, p.ahead = ahead != 0;
   return DSA_OK;
 }
 
-int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride, int64_t y_stride, void* stream) {
+static int gemv(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride, int64_t y_stride, int ahead,
+                void* stream) {
   prep::GemvParams p{};
-  int rc = gemv_checks(p, w, x, y, batch, 4, n, k, x_stride, y_stride);
+  int rc = gemv_checks(p, w, x, y, batch, 4, n, k, x_stride, y_stride, ahead);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   rc = launch_gemv_stream(p, st);
@@ -1173,10 +1174,19 @@ int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k
   }
 }
 
+int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride, int64_t y_stride, void* stream) {
+  return gemv(w, x, y, batch, n, k, x_stride, y_stride, 0, stream);
+}
+
+int dsa_gemv_ahead_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride, int64_t y_stride,
+                        void* stream) {
+  return gemv(w, x, y, batch, n, k, x_stride, y_stride, 1, stream);
+}
+
 int dsa_gemv_swiglu_bf16(const void* w_gate, const void* w_up, const void* x, void* y, int batch, int n, int k, int64_t x_stride,
-                         int64_t y_stride, void* stream) {
+                         int64_t y_stride, int ahead, void* stream) {
   prep::GemvParams p{};
-  int rc = gemv_checks(p, w_gate, x, y, batch, 2, n, k, x_stride, y_stride);
+  int rc = gemv_checks(p, w_gate, x, y, batch, 2, n, k, x_stride, y_stride, ahead);
   if (rc) return rc;
   DSA_REQUIRE(w_up && aligned16(w_up), "gemv + SwiGLU: w_up must be a 16-byte aligned pointer");
   p.w2 = static_cast<const __nv_bfloat16*>(w_up);
@@ -1185,9 +1195,9 @@ int dsa_gemv_swiglu_bf16(const void* w_gate, const void* w_up, const void* x, vo
 }
 
 int dsa_norm_gemv_bf16(const void* w, const void* w_up, const void* x, const void* delta, const void* norm_w, float eps, void* sum_out,
-                       void* y, int batch, int n, int k, int64_t x_stride, int64_t y_stride, void* stream) {
+                       void* y, int batch, int n, int k, int64_t x_stride, int64_t y_stride, int ahead, void* stream) {
   prep::GemvParams p{};
-  int rc = gemv_checks(p, w, x, y, batch, w_up ? 2 : 4, n, k, x_stride, y_stride);
+  int rc = gemv_checks(p, w, x, y, batch, w_up ? 2 : 4, n, k, x_stride, y_stride, ahead);
   if (rc) return rc;
   DSA_REQUIRE(norm_w && (!delta || sum_out), "norm + gemv: null pointer");
   DSA_REQUIRE(aligned16(w_up) && aligned16(delta) && aligned16(norm_w) && aligned16(sum_out), "norm + gemv: pointers must be 16-byte aligned");
@@ -1215,14 +1225,15 @@ static int launch_value_project(const prep::HeadParams& hp, cudaStream_t st) {
 }
 }  // extern "C++"
 
-int dsa_value_project(const void* kv_b, const void* o, void* ov, int B, int H, int o_heads, int nope, int v_dim, void* stream) {
+int dsa_value_project(const void* kv_b, const void* o, void* ov, int B, int H, int o_heads, int nope, int v_dim, int ahead,
+                      void* stream) {
   DSA_REQUIRE(kv_b && o && ov, "value projection: null pointer");
   DSA_REQUIRE(aligned16(kv_b) && aligned16(o), "value projection: pointers must be 16-byte aligned");
   DSA_REQUIRE(B > 0 && B <= prep::kHeadMaxTokens && H > 0 && o_heads >= H && v_dim > 0 && nope >= 0,
               "value projection: bad shape (at most %d tokens)", prep::kHeadMaxTokens);
   prep::HeadParams hp{};
   hp.kv_b = static_cast<const __nv_bfloat16*>(kv_b), hp.q = static_cast<const __nv_bfloat16*>(o), hp.out = static_cast<__nv_bfloat16*>(ov);
-  hp.nope = nope, hp.v_dim = v_dim, hp.H = H, hp.B = B, hp.o_heads = o_heads;
+  hp.nope = nope, hp.v_dim = v_dim, hp.H = H, hp.B = B, hp.o_heads = o_heads, hp.ahead = ahead != 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return B == 1 ? launch_value_project<1>(hp, st) : B == 2 ? launch_value_project<2>(hp, st)
          : B <= 4 ? launch_value_project<4>(hp, st) : launch_value_project<8>(hp, st);
@@ -1374,7 +1385,7 @@ int dsa_decode_token(const void* iq_raw, int64_t iq_stride, const void* w_raw, i
                      const void* kv_a, int64_t kv_a_stride, const void* q, int64_t q_stride, const void* kv_b, const void* kv_norm_w,
                      const void* mla_cos, const void* mla_sin, const void* idx_cos, const void* idx_sin, const int64_t* positions,
                      uint8_t* index_q, float* index_w, void* q_full, uint8_t* cache_index_k, float* cache_k_scale, void* cache_kv, int B,
-                     int H, int nope, int v_dim, int n_index_heads, int64_t cap, int interleave, float eps, void* stream) {
+                     int H, int nope, int v_dim, int n_index_heads, int64_t cap, int interleave, float eps, int ahead, void* stream) {
   DSA_REQUIRE(iq_raw && w_raw && ik_raw && kv_a && q && kv_b && kv_norm_w && mla_cos && mla_sin && idx_cos && idx_sin && positions &&
                   index_q && index_w && q_full && cache_index_k && cache_k_scale && cache_kv,
               "decode token: null pointer");
@@ -1399,7 +1410,7 @@ int dsa_decode_token(const void* iq_raw, int64_t iq_stride, const void* w_raw, i
   p.cap = cap, p.B = B, p.H = H, p.Hidx = n_index_heads, p.interleave = interleave, p.eps = eps;
   prep::HeadParams hp{};
   hp.kv_b = static_cast<const __nv_bfloat16*>(kv_b), hp.q = static_cast<const __nv_bfloat16*>(q), hp.q_row = q_stride, hp.q_head = nope + 64;
-  hp.nope = nope, hp.v_dim = v_dim, hp.H = H, hp.B = B;
+  hp.nope = nope, hp.v_dim = v_dim, hp.H = H, hp.B = B, hp.ahead = ahead != 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   return B == 1 ? launch_decode_token<1>(p, hp, st) : B == 2 ? launch_decode_token<2>(p, hp, st)
          : B <= 4 ? launch_decode_token<4>(p, hp, st) : launch_decode_token<8>(p, hp, st);

@@ -452,10 +452,11 @@ class DSALayer(nn.Module):
         nxt = self.full_select(op, pad_value=op.s).view(op.b, op.s, -1).long() if produce_indexer else None
         return attn_hidden, nxt
 
-    def mlp(self, h_norm: torch.Tensor, weights=None) -> torch.Tensor:
+    def mlp(self, h_norm: torch.Tensor, weights=None, ahead: bool = False) -> torch.Tensor:
         if (h_norm.is_cuda and h_norm.dtype == torch.bfloat16 and h_norm.dim() == 2 and h_norm.shape[0] <= 2
                 and not torch.is_grad_enabled()):
-            return self._reduced(self._skinny("down_proj", ops.gemv_swiglu(h_norm, self.gate_proj.weight, self.up_proj.weight)))
+            return self._reduced(self._skinny("down_proj", ops.gemv_swiglu(h_norm, self.gate_proj.weight, self.up_proj.weight,
+                                                                         ahead)))
         w = self._full_weights(h_norm) if h_norm.dim() == 3 and weights is None else weights
         if w is not None:
             y = _lib.host().mlp(h_norm.reshape(-1, h_norm.shape[2]), w[8], w[9], w[10])
@@ -467,12 +468,12 @@ class DSALayer(nn.Module):
 
     # ------------------------------------------------------------------ decode form
     def _skinny(self, name: str, x: torch.Tensor) -> torch.Tensor:
-        """A projection of one or two bf16 rows: the library's GEMV, which starts on its weights while the
-        kernel before it runs, unless the module is not a plain ``nn.Linear``."""
+        """A projection of one or two bf16 rows behind another launch of the same call: the library's GEMV, which
+        starts on its weights while the kernel before it runs, unless the module is not a plain ``nn.Linear``."""
         m = self._modules[name]
         if x.shape[0] > 2 or x.dtype != torch.bfloat16 or not x.is_cuda or torch.is_grad_enabled() or not self._plain(name):
             return m(x)
-        return ops.gemv(x, m.weight)
+        return ops.gemv(x, m.weight, ahead=True)
 
     def _plain(self, name: str) -> bool:
         """A bias-free bf16 ``nn.Linear`` that only multiplies, of a width that the GEMV takes."""
@@ -508,30 +509,36 @@ class DSALayer(nn.Module):
         return (_bare(norm, RMSNorm) and x.is_cuda and x.dtype == torch.bfloat16 and norm.weight.dtype == torch.bfloat16
                 and not torch.is_grad_enabled() and ops.norm_gemv_fits(x.shape[0], x.shape[1]))
 
-    def decode_residual_project(self, x, delta, rope: RopeCaches, positions, cache: LayerDecodeCache, batch_index):
-        """``x + delta`` (``delta`` None: ``x``) and :func:`decode_project` of its attention norm."""
+    def decode_residual_project(self, x, delta, rope: RopeCaches, positions, cache: LayerDecodeCache, batch_index,
+                                ahead: bool = False):
+        """``x + delta`` (``delta`` None: ``x``) and :func:`decode_project` of its attention norm. ``ahead`` (here
+        and in the methods below): this call's first launch may read its weights while the kernels in front still
+        run, as every later one does: nothing enqueued since the last launch that waited writes them (inside a
+        decode step; not at its start, where whatever updates weights may be in front)."""
         wide = self._wx.shape[0] if self._stacked() else 0
         # One or two rows: the norm's launch goes. Four where the product has few outputs of long rows, which the
         # library's GEMM runs at 1.4 TB/s (norm, [2240, 7168] and the copy of its strided columns 27 us, here 13).
         if wide and x.dim() == 2 and (x.shape[0] <= 2 or (x.shape[0] <= 4 and wide <= 4096 <= x.shape[1])) and self._norm_folds(self.attn_norm, x):
-            x, ya = ops.norm_gemv(x, delta, self.attn_norm.weight, self.attn_norm.eps, self._wx)
+            x, ya = ops.norm_gemv(x, delta, self.attn_norm.weight, self.attn_norm.eps, self._wx, ahead=ahead)
             return x, self.decode_project(x, rope, positions, cache, batch_index, ya)
         if delta is None:
             x_norm = self.attn_norm(x)
         else:
             x, x_norm = add_norm(self.attn_norm, x, delta)
-        return x, self.decode_project(x_norm, rope, positions, cache, batch_index)
+        return x, self.decode_project(x_norm, rope, positions, cache, batch_index, ahead=ahead)
 
-    def decode_mlp(self, x: torch.Tensor, attn: torch.Tensor):
+    def decode_mlp(self, x: torch.Tensor, attn: torch.Tensor, ahead: bool = False):
         """``(h, mlp(ffn_norm(h)))`` with ``h = x + attn``."""
         if (x.shape == attn.shape and x.dim() == 2 and x.shape[0] <= 2 and attn.dtype == x.dtype and attn.is_contiguous()
                 and self._norm_folds(self.ffn_norm, x) and self._plain("gate_proj") and self._plain("up_proj")):
-            h, act = ops.norm_gemv(x, attn, self.ffn_norm.weight, self.ffn_norm.eps, self.gate_proj.weight, self.up_proj.weight)
+            h, act = ops.norm_gemv(x, attn, self.ffn_norm.weight, self.ffn_norm.eps, self.gate_proj.weight, self.up_proj.weight,
+                                   ahead)
             return h, self._reduced(self._skinny("down_proj", act))
         h, h_norm = add_norm(self.ffn_norm, x, attn)
-        return h, self.mlp(h_norm)
+        return h, self.mlp(h_norm, ahead=ahead)
 
-    def decode_project(self, x_norm, rope: RopeCaches, positions, cache: LayerDecodeCache, batch_index, ya=None):
+    def decode_project(self, x_norm, rope: RopeCaches, positions, cache: LayerDecodeCache, batch_index, ya=None,
+                       ahead: bool = False):
         """Projections of one new token per sequence, and its keys appended to
         the caches at ``positions`` [B]. Returns (q [B,H,Dqk], index_q, index_w).
 
@@ -549,17 +556,17 @@ class DSALayer(nn.Module):
                 # few output rows, long rows: the library GEMV is latency-bound there (measured 19-32 us
                 # against 13 us for the skinny kernel at one token); the other shapes stay with the library
                 skinny = b <= 2 and x_norm.dtype == torch.bfloat16 and self._wx.shape[0] <= 4096 <= self._wx.shape[1]
-                ya = ops.gemv(x_norm, self._wx) if skinny else torch.nn.functional.linear(x_norm, self._wx)
+                ya = ops.gemv(x_norm, self._wx, ahead) if skinny else torch.nn.functional.linear(x_norm, self._wx)
             qa, kv_a, ik_raw = ya.split(
                 [c.q_lora_rank, c.kv_lora_rank + c.qk_rope_head_dim, c.index_head_dim], dim=-1)
             n = self.q_a_layernorm
             # the c_q-side projection and the MLP's gate / up take the same kernel at one or two
             # tokens (252 against 255 us per layer of the 8-layer stack)
             if b <= 2 and self._norm_folds(n, qa):
-                yc = ops.norm_gemv(qa, None, n.weight, n.eps, self._wc)[1]
+                yc = ops.norm_gemv(qa, None, n.weight, n.eps, self._wc, ahead=True)[1]
             else:
                 c_q = n(qa)
-                yc = ops.gemv(c_q, self._wc) if b <= 2 and c_q.dtype == torch.bfloat16 else torch.nn.functional.linear(c_q, self._wc)
+                yc = ops.gemv(c_q, self._wc, ahead=True) if b <= 2 and c_q.dtype == torch.bfloat16 else torch.nn.functional.linear(c_q, self._wc)
             q, iq_raw, w = yc.split(
                 [h * (c.qk_nope_head_dim + c.qk_rope_head_dim), c.index_n_heads * c.index_head_dim, c.index_n_heads],
                 dim=-1)
@@ -578,7 +585,7 @@ class DSALayer(nn.Module):
             if self._absorbed_rows(x_norm):
                 ops.decode_token(iq_raw, w, ik_raw, kv_a, q, self.kv_b_proj.weight, self.kv_a_layernorm.weight, rope.mla_cos,
                                  rope.mla_sin, rope.idx_cos, rope.idx_sin, positions, index_q, index_w, q_full, cache.index_k,
-                                 cache.k_scale, cache.kv, il, c.rms_norm_eps)
+                                 cache.k_scale, cache.kv, il, c.rms_norm_eps, ahead=True)
                 return q_full, index_q, index_w
         q = q.contiguous().view(b, h, c.qk_nope_head_dim + c.qk_rope_head_dim)  # (a column range of a stacked product)
         iq_raw = iq_raw.reshape(b, c.index_n_heads, c.index_head_dim)
@@ -642,7 +649,7 @@ class DSALayer(nn.Module):
             o = ops.sparse_mla_decode(_pad_heads(q.to(torch.bfloat16), ops.HEAD_BLOCK).contiguous(), cache.kv,
                                       indices, self.sm_scale, seq_lens, beside_previous=beside_previous and direct)
             if self._absorbed_rows(q):
-                ov = ops.value_project(self.kv_b_proj.weight, o, h, c.v_head_dim)
+                ov = ops.value_project(self.kv_b_proj.weight, o, h, c.v_head_dim, ahead=True)
                 return self._reduced(self._skinny("o_proj", ov.view(ov.shape[0], h * c.v_head_dim)))
             o = o[:, :h].to(q.dtype)
         else:

@@ -284,7 +284,8 @@ class DSAModel(nn.Module):
         for li, layer in enumerate(self.layers):
             cache = state.caches[li]
             is_dsa = types[li] is AttentionType.DSA
-            x, (q, iq, w) = layer.decode_residual_project(x, delta, state.rope, state.positions, cache, state.batch_index)
+            x, (q, iq, w) = layer.decode_residual_project(x, delta, state.rope, state.positions, cache, state.batch_index,
+                                                          ahead=li > 0)
             made = None
             beside = False
             if not lagged:
@@ -317,7 +318,7 @@ class DSAModel(nn.Module):
                         beside = (chained and li > 0 and attend is not None and cache.k_scale is not None
                                   and iq.dtype == torch.uint8 and state.workspaces[li] is not None)
             attn = layer.decode_attention(q, cache, attend, state.seq_lens, beside_previous=beside)
-            x, delta = layer.decode_mlp(x, attn)
+            x, delta = layer.decode_mlp(x, attn, ahead=True)
             if lagged and made is not None:
                 carried = made  # becomes visible to layer li+1 after the join
             if record is not None:
@@ -365,7 +366,8 @@ class DSAModel(nn.Module):
         for li, layer in enumerate(self.layers):
             cache = state.caches[li]
             is_dsa = types[li] is AttentionType.DSA
-            x, (q, iq, w) = layer.decode_residual_project(x, delta, state.rope, state.positions, cache, state.batch_index)
+            x, (q, iq, w) = layer.decode_residual_project(x, delta, state.rope, state.positions, cache, state.batch_index,
+                                                          ahead=li > 0)
             made = None
 
             def dispatch():
@@ -406,7 +408,7 @@ class DSAModel(nn.Module):
             else:
                 attend = carried
             attn = layer.decode_attention(q, cache, attend, state.seq_lens)
-            x, delta = layer.decode_mlp(x, attn)
+            x, delta = layer.decode_mlp(x, attn, ahead=True)
             if record is not None:
                 used.append(attend)
                 produced.append(made)

@@ -374,32 +374,33 @@ def _gemv_operand(x: torch.Tensor, weight: torch.Tensor, most: int) -> torch.Ten
     return x if x.stride(1) == 1 and x.stride(0) % 8 == 0 else x.contiguous()
 
 
-def gemv(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+def gemv(x: torch.Tensor, weight: torch.Tensor, ahead: bool = False) -> torch.Tensor:
     """``x @ weight.T`` for a decode batch of 1..4 rows (bf16, fp32 accumulation): the weight
-    matrix ``[n, k]`` is streamed once, its first part while the kernel before is still running."""
+    matrix ``[n, k]`` is streamed once. ``ahead`` (here and below): its first part while the kernels before
+    are still running, which the caller may say where none of them writes it (see ``dsa_gemv_ahead_bf16``)."""
     x = _gemv_operand(x, weight, 4)
     (b, k), n = x.shape, weight.shape[0]
     y = torch.empty(b, n, dtype=torch.bfloat16, device=x.device)
-    _lib.check(_lib.lib().dsa_gemv_bf16(_ptr(weight), _ptr(x), _ptr(y), b, n, k, x.stride(0) if b > 1 else k, n,
-                                        _stream()))
+    fn = _lib.lib().dsa_gemv_ahead_bf16 if ahead else _lib.lib().dsa_gemv_bf16
+    _lib.check(fn(_ptr(weight), _ptr(x), _ptr(y), b, n, k, x.stride(0) if b > 1 else k, n, _stream()))
     return y
 
 
-def gemv_swiglu(x: torch.Tensor, gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
+def gemv_swiglu(x: torch.Tensor, gate: torch.Tensor, up: torch.Tensor, ahead: bool = False) -> torch.Tensor:
     """``silu(x @ gate.T) * (x @ up.T)`` for one or two rows in one launch, rounded as the separate operations."""
     x = _gemv_operand(x, gate, 2)
     _need(up.shape == gate.shape and up.dtype == torch.bfloat16 and up.is_contiguous(), "gate and up must have one shape")
     (b, k), n = x.shape, gate.shape[0]
     if b * k > 32768:  # x beside the weights' ring in shared memory: the streaming kernel's limit is a little above
-        return silu_mul(gemv(x, gate), gemv(x, up))
+        return silu_mul(gemv(x, gate, ahead), gemv(x, up, ahead))
     y = torch.empty(b, n, dtype=torch.bfloat16, device=x.device)
     _lib.check(_lib.lib().dsa_gemv_swiglu_bf16(_ptr(gate), _ptr(up), _ptr(x), _ptr(y), b, n, k, x.stride(0) if b > 1 else k, n,
-                                               _stream()))
+                                               1 if ahead else 0, _stream()))
     return y
 
 
 def norm_gemv(x: torch.Tensor, delta: Optional[torch.Tensor], norm_weight: torch.Tensor, eps: float, weight: torch.Tensor,
-              up: Optional[torch.Tensor] = None):
+              up: Optional[torch.Tensor] = None, ahead: bool = False):
     """``(s, rmsnorm(s) @ weight.T)`` with ``s = x + delta`` (``x`` without a delta) in one launch, for 1..4
     rows of at most 8192; with ``up`` the SwiGLU product of :func:`gemv_swiglu`."""
     x = _gemv_operand(x, weight, 2 if up is not None else 4)
@@ -416,7 +417,7 @@ def norm_gemv(x: torch.Tensor, delta: Optional[torch.Tensor], norm_weight: torch
     y = torch.empty(b, n, dtype=torch.bfloat16, device=x.device)
     _lib.check(_lib.lib().dsa_norm_gemv_bf16(_ptr(weight), _ptr(up), _ptr(x), _ptr(delta), _ptr(norm_weight), float(eps),
                                              _ptr(s) if delta is not None else None, _ptr(y), b, n, k,
-                                             x.stride(0) if b > 1 else k, n, _stream()))
+                                             x.stride(0) if b > 1 else k, n, 1 if ahead else 0, _stream()))
     return s, y
 
 
@@ -428,7 +429,7 @@ def norm_gemv_fits(b: int, k: int) -> bool:
 HEAD_TOKENS = 8  # tokens that share one reading of kv_b_proj's weight in decode_token / value_project
 
 
-def value_project(kv_b: torch.Tensor, o: torch.Tensor, heads: int, v_dim: int) -> torch.Tensor:
+def value_project(kv_b: torch.Tensor, o: torch.Tensor, heads: int, v_dim: int, ahead: bool = False) -> torch.Tensor:
     """``[B, heads, v_dim]``: every head's latent output ``o`` ``[B, >= heads, 512]`` through W_UV, the last
     ``v_dim`` rows of the head's part of ``kv_b`` ``[heads * per_head, 512]``; at most HEAD_TOKENS rows."""
     _cuda_contig(kv_b, "kv_b", (torch.bfloat16,))
@@ -438,12 +439,13 @@ def value_project(kv_b: torch.Tensor, o: torch.Tensor, heads: int, v_dim: int) -
           "kv_b must be [heads * per_head, 512], o [B, >= heads, 512]")
     ov = torch.empty(o.shape[0], heads, v_dim, dtype=torch.bfloat16, device=o.device)
     _lib.check(_lib.lib().dsa_value_project(_ptr(kv_b), _ptr(o), _ptr(ov), o.shape[0], heads, o.shape[1],
-                                            kv_b.shape[0] // heads - v_dim, v_dim, _stream()))
+                                            kv_b.shape[0] // heads - v_dim, v_dim, 1 if ahead else 0, _stream()))
     return ov
 
 
 def decode_token(iq_raw, w_raw, ik_raw, kv_a, q, kv_b, kv_norm_w, mla_cos, mla_sin, idx_cos, idx_sin, positions, index_q,
-                 index_w, q_full, cache_index_k, cache_k_scale, cache_kv, interleave: bool, eps: float) -> None:
+                 index_w, q_full, cache_index_k, cache_k_scale, cache_kv, interleave: bool, eps: float,
+                 ahead: bool = False) -> None:
     """:func:`decode_prep` for at most HEAD_TOKENS tokens with the query's absorption in the launch: ``q``
     ``[B, H * (nope + 64)]`` and ``kv_b`` ``[H * per_head, 512]`` instead of ``q_abs`` and ``q_pe``. The five
     inputs are 2-D and may be column ranges of a stacked projection's output (see ``dsa_decode_token``)."""
@@ -467,7 +469,7 @@ def decode_token(iq_raw, w_raw, ik_raw, kv_a, q, kv_b, kv_norm_w, mla_cos, mla_s
         _ptr(iq_raw), iq_raw.stride(0), _ptr(w_raw), w_raw.stride(0), _ptr(ik_raw), ik_raw.stride(0), _ptr(kv_a), kv_a.stride(0),
         _ptr(q), q.stride(0), _ptr(kv_b), _ptr(kv_norm_w), _ptr(mla_cos), _ptr(mla_sin), _ptr(idx_cos), _ptr(idx_sin),
         _ptr(positions), _ptr(index_q), _ptr(index_w), _ptr(q_full), _ptr(cache_index_k), _ptr(cache_k_scale), _ptr(cache_kv),
-        B, H, nope, per_head - nope, n_idx, cap, 1 if interleave else 0, float(eps), _stream()))
+        B, H, nope, per_head - nope, n_idx, cap, 1 if interleave else 0, float(eps), 1 if ahead else 0, _stream()))
 
 
 def indexer_stage_fp8(q_raw, k_raw, w_raw, k_norm_weight, k_norm_bias, k_norm_eps: float, rope_cos, rope_sin,

@@ -31,7 +31,7 @@
 extern "C" {
 #endif
 
-#define DSA_ABI_VERSION 10
+#define DSA_ABI_VERSION 11
 
 enum dsa_status {
   DSA_OK = 0,
@@ -399,8 +399,11 @@ int dsa_copy_post_epoch(void* dst, const void* src, int64_t bytes, uint32_t* cou
 /* y[b, n] = sum_k w[n, k] x[b, k] for a decode batch of 1..4 rows: bf16 operands, fp32
  * accumulation, w [n, k] row-major streamed once (the projection GEMVs of
  * src/lagged_indexer_dsa/dsa_layer.py:87-125 at decode). k a multiple of 8; row strides of x and y in
- * elements. The kernel starts reading w before the kernel enqueued in front of it has completed: w must
- * not be written by this library (by any other work, anything goes).
+ * elements.
+ * dsa_gemv_ahead_bf16, and the functions below with ahead != 0, start reading w (and norm_w) before the
+ * kernels enqueued in front have completed. The caller states that none of them writes it, back to one that
+ * waited for its own predecessors before it released this one: a projection in the middle of a decode step
+ * qualifies, the first one behind unknown work does not. Otherwise nothing is read before they are done.
  * dsa_gemv_swiglu_bf16: y = silu(x w_gate^T) * (x w_up^T), rounded as the separate operations, for one or
  * two rows (:194-196).
  * dsa_norm_gemv_bf16: either with x replaced by rmsnorm(x + delta) * norm_w, rounded as in
@@ -408,16 +411,17 @@ int dsa_copy_post_epoch(void* dst, const void* src, int64_t bytes, uint32_t* cou
  * w_up NULL: the plain product. k at most 8192; delta's rows are dense. */
 int dsa_gemv_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride,
                   int64_t y_stride, void* stream);
+int dsa_gemv_ahead_bf16(const void* w, const void* x, void* y, int batch, int n, int k, int64_t x_stride,
+                        int64_t y_stride, void* stream);
 int dsa_gemv_swiglu_bf16(const void* w_gate, const void* w_up, const void* x, void* y, int batch, int n, int k,
-                         int64_t x_stride, int64_t y_stride, void* stream);
+                         int64_t x_stride, int64_t y_stride, int ahead, void* stream);
 int dsa_norm_gemv_bf16(const void* w, const void* w_up, const void* x, const void* delta, const void* norm_w,
                        float eps, void* sum_out, void* y, int batch, int n, int k, int64_t x_stride,
-                       int64_t y_stride, void* stream);
+                       int64_t y_stride, int ahead, void* stream);
 /* ov [B, H, v_dim] = W_UV[h] o[b, h, :] with kv_b_proj's weight kv_b [H, nope + v_dim, 512] (bf16,
- * src/lagged_indexer_dsa/dsa_layer.py:118-125), o [B, o_heads, 512], 1..8 tokens. kv_b is read like the
- * weights of dsa_gemv_bf16. */
+ * src/lagged_indexer_dsa/dsa_layer.py:118-125), o [B, o_heads, 512], 1..8 tokens. */
 int dsa_value_project(const void* kv_b, const void* o, void* ov, int B, int H, int o_heads, int nope,
-                      int v_dim, void* stream);
+                      int v_dim, int ahead, void* stream);
 /* out = silu(gate) * up over n bf16 elements: the SwiGLU between the MLP's GEMVs
  * (src/lagged_indexer_dsa/dsa_layer.py:194-196), rounded as the two separate operations. */
 int dsa_silu_mul_bf16(const void* gate, const void* up, void* out, int64_t n, void* stream);
@@ -431,8 +435,7 @@ int dsa_decode_prep(const void* iq_raw, const void* w_raw, const void* ik_raw, c
                     int B, int H, int n_index_heads, int64_t cap, int interleave, float eps,
                     void* stream);
 /* The same for 1..8 tokens with the absorption of the query in the launch: q [B] rows of H heads of
- * [nope | 64], q_full[b, h, 0:512] = q[b, h, 0:nope] W_UK[h] with kv_b as in dsa_value_project (read ahead
- * of the kernel in front, as there). The inputs' rows may be strided (elements between tokens), so the
+ * [nope | 64], q_full[b, h, 0:512] = q[b, h, 0:nope] W_UK[h] with kv_b as in dsa_value_project. The inputs' rows may be strided (elements between tokens), so the
  * outputs of stacked projections need no copies. */
 int dsa_decode_token(const void* iq_raw, int64_t iq_stride, const void* w_raw, int64_t w_stride,
                      const void* ik_raw, int64_t ik_stride, const void* kv_a, int64_t kv_a_stride,
@@ -440,7 +443,7 @@ int dsa_decode_token(const void* iq_raw, int64_t iq_stride, const void* w_raw, i
                      const void* mla_cos, const void* mla_sin, const void* idx_cos, const void* idx_sin,
                      const int64_t* positions, uint8_t* index_q, float* index_w, void* q_full,
                      uint8_t* cache_index_k, float* cache_k_scale, void* cache_kv, int B, int H, int nope,
-                     int v_dim, int n_index_heads, int64_t cap, int interleave, float eps, void* stream);
+                     int v_dim, int n_index_heads, int64_t cap, int interleave, float eps, int ahead, void* stream);
 
 /* Serving-form indexer staging: what the serving model's indexer does to the new
  * token between its projection GEMVs and the scan

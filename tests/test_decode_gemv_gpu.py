@@ -115,3 +115,41 @@ def test_absorbed_projections(ops, B, H, nope, v, pad):
     ov = ops.value_project(kv_b, o, H, v)
     ref = torch.einsum("bhl,hdl->bhd", o[:, :H].double(), weight[:, nope:])
     close(ov, ref, torch.einsum("bhl,hdl->bhd", o[:, :H].double().abs(), weight[:, nope:].abs()))
+
+
+def test_weights_may_come_from_the_launch_in_front(ops):
+    """Without ``ahead`` a weight is read when the kernels in front are done, also one that releases its
+    dependents before it has stored anything, as this library's norms do."""
+    torch.manual_seed(3)
+    n, k = 8192, 2048
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    x, ones, raw = bf(2, k), torch.ones(k, dtype=torch.bfloat16, device="cuda"), [bf(n, k) for _ in range(4)]
+    ref = [ops.rmsnorm(r, ones, 1e-6) for r in raw]
+    torch.cuda.synchronize()
+    fresh = lambda i: ops.rmsnorm(raw[i], ones, 1e-6)  # (into whatever memory the last one has left)
+    for i in range(4):
+        torch.cuda.synchronize()
+        assert torch.equal(ops.gemv(x, fresh(i)), ops.gemv(x, ref[i]))
+        assert torch.equal(ops.gemv_swiglu(x, fresh(i), ref[i]), ops.gemv_swiglu(x, ref[i], ref[i]))
+        assert torch.equal(ops.norm_gemv(x, None, ones, 1e-6, fresh(i))[1], ops.norm_gemv(x, None, ones, 1e-6, ref[i])[1])
+    heads = raw[0].view(-1, 512)[:16 * 256]
+    unit = torch.ones(512, dtype=torch.bfloat16, device="cuda")
+    o = bf(2, 16, 512)
+    want = ops.value_project(ops.rmsnorm(heads, unit, 1e-6).clone(), o, 16, 128)
+    torch.cuda.synchronize()
+    assert torch.equal(ops.value_project(ops.rmsnorm(heads, unit, 1e-6), o, 16, 128), want)
+
+
+@pytest.mark.parametrize("b", [1, 2, 4])
+def test_reading_ahead_changes_nothing_but_the_time(ops, b):
+    torch.manual_seed(b)
+    bf = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16)
+    x, w, u, nw = bf(b, 1024), bf(700, 1024), bf(700, 1024), bf(1024)
+    torch.cuda.synchronize()
+    assert torch.equal(ops.gemv(x, w), ops.gemv(x, w, ahead=True))
+    assert torch.equal(ops.norm_gemv(x, None, nw, 1e-6, w)[1], ops.norm_gemv(x, None, nw, 1e-6, w, ahead=True)[1])
+    if b <= 2:
+        assert torch.equal(ops.gemv_swiglu(x, w, u), ops.gemv_swiglu(x, w, u, ahead=True))
+    kv_b, o = bf(16 * 256, 512), bf(b, 16, 512)
+    torch.cuda.synchronize()
+    assert torch.equal(ops.value_project(kv_b, o, 16, 128), ops.value_project(kv_b, o, 16, 128, ahead=True))
