@@ -945,9 +945,10 @@ int dsa_sparse_mla_decode(const void* q, const void* kv, const int32_t* indices,
                           void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit,
                           float sm_scale, int64_t kv_seq_stride, int kv_fp8, void* stream) {
   DSA_REQUIRE(out && aligned16(out), "sparse MLA: out must be a 16-byte aligned pointer");
-  int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, nsplit == 1 ? out : nullptr, R,
+  const bool direct = nsplit == 1 && !part_acc;  // (a caller that hands over partials gets them)
+  int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, direct ? out : nullptr, R,
                                rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8, false, stream);
-  if (rc || nsplit == 1) return rc;
+  if (rc || direct) return rc;
   return dsa_sparse_mla_combine(part_acc, part_m, part_l, out, R, H, nsplit, stream);
 }
 
@@ -956,9 +957,10 @@ int dsa_sparse_mla_decode_beside(const void* q, const void* kv, const int32_t* i
                                  void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit,
                                  float sm_scale, int64_t kv_seq_stride, int kv_fp8, void* stream) {
   DSA_REQUIRE(out && aligned16(out), "sparse MLA: out must be a 16-byte aligned pointer");
-  int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, nsplit == 1 ? out : nullptr, R,
+  const bool direct = nsplit == 1 && !part_acc;  // (a caller that hands over partials gets them)
+  int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, direct ? out : nullptr, R,
                                rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8, true, stream);
-  if (rc || nsplit == 1) return rc;
+  if (rc || direct) return rc;
   return dsa_sparse_mla_combine(part_acc, part_m, part_l, out, R, H, nsplit, stream);
 }
 

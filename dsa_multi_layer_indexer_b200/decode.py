@@ -75,6 +75,8 @@ class HotPathState:
         self.topk_ws = ops.topk_workspace(rows, capacity, dev)
         self.nsplit = nsplit or ops.default_nsplit(rows, heads, topk)
         self.scratch = ops.MlaScratch(rows, heads, self.nsplit, dev)
+        # what the attention is handed: without partials a single split writes its result in one launch
+        self.partials = self.scratch if self.nsplit > 1 else None
 
     # -- the three launches, on the current stream -----------------------------
     def run_indexer(self, cache: LayerCache, impl: int = 0) -> torch.Tensor:
@@ -91,8 +93,8 @@ class HotPathState:
         """Sparse MLA over ``attend`` (any ``[rows, topk]`` int32 selection). ``beside_previous``:
         ``attend`` and the queries do not come from the kernel enqueued just before (see
         :func:`ops.sparse_mla_decode`)."""
-        return ops.sparse_mla_decode(self.q, cache.kv, attend, sm_scale, self.seq_lens,
-                                     scratch=self.scratch, out=self.out, beside_previous=beside_previous)
+        return ops.sparse_mla_decode(self.q, cache.kv, attend, sm_scale, self.seq_lens, nsplit=self.nsplit,
+                                     scratch=self.partials, out=self.out, beside_previous=beside_previous)
 
     def run_lagged_chained(self, cache: LayerCache, attend: torch.Tensor, sm_scale: float) -> torch.Tensor:
         """Lagged order on ONE stream: this layer's scan and top-k, then the attention over
@@ -205,8 +207,8 @@ class HostDecoder:
                     ops.copy_bytes(self.h_indices, s.indices)
                 else:
                     self.h_indices.copy_(s.indices, non_blocking=True)
-        ops.sparse_mla_decode(s.q, self.cache.kv, s.indices, sm_scale, s.seq_lens, scratch=s.scratch,
-                              out=self.h_out)
+        ops.sparse_mla_decode(s.q, self.cache.kv, s.indices, sm_scale, s.seq_lens, nsplit=s.nsplit,
+                              scratch=s.partials, out=self.h_out)
         if fused_tail:
             # (the selection was final three launches ago: it travels beside the merge kernel)
             ops.copy_post_epoch(self.h_indices, s.indices, self._epoch_dev, self._flag, beside_previous=True)

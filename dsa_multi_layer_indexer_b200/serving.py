@@ -48,7 +48,7 @@ class _Plan:
         if H != self.H_real:
             self.qpad = torch.zeros(1, B, H, ops.LATENT_DIM, dtype=torch.bfloat16, device=dev)
         out = torch.zeros(1, B, H, ops.VALUE_DIM, dtype=torch.bfloat16, device=dev)
-        self.part = ops.MlaScratch(B, H, self.nsplit, dev)
+        self.part = ops.MlaScratch(B, H, self.nsplit, dev) if self.nsplit > 1 else None  # (one split: no partials)
         self.attn_out = out if H == self.H_real else out[:, :, :self.H_real]
         self.attn = out.view(B, H, ops.VALUE_DIM)
 

@@ -267,8 +267,9 @@ int dsa_topk_select_static(const float* logits, const int32_t* seq_lens, int32_t
  *            (:1098-1104), dequantised fp8->f32 * scale -> bf16 RN (:1181-1196)
  *   indices  [R, topk] int32, or NULL to attend every key below seq_lens[r]
  *            (dense cold start; topk is then the key capacity to cover)
- *   part_acc [R, nsplit, H, 512] fp32, part_m / part_l [R, nsplit, H] fp32 (may be NULL for
- *            dsa_sparse_mla_decode with nsplit == 1, which writes the result without partials)
+ *   part_acc [R, nsplit, H, 512] fp32, part_m / part_l [R, nsplit, H] fp32, written by every call (all
+ *            three NULL with nsplit == 1: dsa_sparse_mla_decode then writes the result without partials,
+ *            in one launch)
  *   out      [R, H, 512] bf16
  * dsa_sparse_mla_decode = partials + combine; the two halves are exported for
  * callers that schedule them separately, as the reference does.

@@ -61,3 +61,28 @@ def test_one_split_dense_rows_of_a_prompt(ops, H):
     for r in (0, 63, 64, s - 1):
         ref = O.dense_mla_decode(q[r:r + 1].cpu(), kv[0].cpu(), [r + 1], sm)
         assert rel_err(got[r:r + 1].float().cpu(), ref) < 2e-2
+
+
+@pytest.mark.parametrize("H,rows", [(16, 3), (64, 130)])  # mma.sync kernel, tcgen05 kernel
+@pytest.mark.parametrize("beside", [False, True])
+def test_partials_that_a_caller_hands_over_are_written(ops, H, rows, beside):
+    """One split writes its result at once only where there is nothing else to write."""
+    from dsa_multi_layer_indexer_b200 import kernels_ext
+
+    torch.manual_seed(H)
+    n, topk, sm = 300, 128, 192 ** -0.5
+    q = torch.randn(rows, H, 576, device="cuda").to(torch.bfloat16)
+    kv = torch.randn(1, n, 576, device="cuda").to(torch.bfloat16)
+    idx = torch.stack([torch.randperm(n)[:topk] for _ in range(rows)]).int().cuda()
+    want, got = (ops.MlaScratch(rows, H, 1, "cuda") for _ in range(2))
+    ops.sparse_mla_decode(q, kv, idx, sm, rows_per_seq=rows, nsplit=1, scratch=want, stage="partials")
+    for s in (got.acc, got.m, got.l):
+        s.fill_(float("nan"))
+    out = ops.sparse_mla_decode(q, kv, idx, sm, rows_per_seq=rows, nsplit=1, scratch=got, beside_previous=beside)
+    for a, b in ((got.acc, want.acc), (got.m, want.m), (got.l, want.l)):
+        assert torch.equal(a, b)
+    assert torch.equal(out, ops.sparse_mla_decode(q, kv, idx, sm, rows_per_seq=rows, nsplit=1))
+    acc, m, l = kernels_ext.alloc_part(rows, H, 1, "cuda")  # the extension's own output arguments
+    kernels_ext.build().launch_fused_sparse_splitk(q, kv[0], idx, None, None, None, None, acc, m, l, None, None, out, rows, n, H, 16, topk,
+                                                   1, sm, 0, 1, 0)
+    assert float(l.min()) > 0 and float(acc.abs().sum()) > 0
