@@ -23,6 +23,10 @@ namespace topk {
 constexpr int kRowsBins = 2048;
 constexpr int64_t kRowsMaxN = 16384;  // 512 threads x 32 logits
 
+// Whether a key is that of a number. A NaN (key above +inf's) takes a rank, as it does in the scan's histogram,
+// but is never selected: the places that this leaves are padding. (topk_cluster_kernel compares numbers.)
+__device__ __forceinline__ bool key_is_number(uint32_t key) { return key - 0x007FFFFFu <= 0xFF800000u - 0x007FFFFFu; }
+
 // Bin (from the top) that holds the k-th largest of an NB-bin histogram; thread t owns the NB / T bins
 // below NB - t * NB / T. s_res: bin, rank inside it. Every thread calls it; ends with a barrier.
 template <int T, int NB>
@@ -89,40 +93,52 @@ topk_rows_kernel(const Params p) {
       if (out_val) out_val[i] = neg_inf;
     }
   };
-  if (len <= p.topk) {  // every visible key is kept, in place
-    for (int i = tid; i < len; i += T) emit(uint32_t(i), i, row[i] == neg_inf);
+  const bool take_all = len <= p.topk;
+  if (take_all) {  // every visible number is kept, in place unless there is a NaN among them
+    bool nan = false;
+    for (int i = tid; i < len; i += T) {
+      const float v = row[i];
+      nan |= v != v;
+      emit(uint32_t(i), i, v == neg_inf);
+    }
     pad_from(uint32_t(len));
-    return;
+    if (!__syncthreads_or(nan)) return;
   }
   const int base = warp * (32 * ITEMS) + lane;
   // keys, not values, stay in registers; 0 (below every number) past the row's length
   uint32_t key[ITEMS];
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) key[i] = base + 32 * i < len ? ordered_key(row[base + 32 * i]) : 0u;
-  __syncthreads();  // the histogram is clear
+  uint32_t kstar = 0u, ties_kept = 0u;  // (take_all: whatever is above 0)
+  if (!take_all) {
+    __syncthreads();  // the histogram is clear
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+      hist_add_warp(s_hist, key[i] != 0u, key[i] >> 21);
+    __syncthreads();
+    rows_find_bin<T, kRowsBins>(s_hist, uint32_t(p.topk), s_warp, s_res);
+    const uint32_t b1 = s_res[0];
+    uint32_t need = s_res[1];
+    clear();
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) hist_add_warp(s_hist, key[i] != 0u && (key[i] >> 21) == b1, (key[i] >> 10) & 2047u);
+    __syncthreads();
+    rows_find_bin<T, kRowsBins>(s_hist, need, s_warp, s_res);
+    const uint32_t p22 = (b1 << 11) | s_res[0];
+    need = s_res[1];
+    clear();
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) hist_add_warp(s_hist, key[i] != 0u && (key[i] >> 10) == p22, key[i] & 1023u);
+    __syncthreads();
+    rows_find_bin<T, 1024>(s_hist, need, s_warp, s_res);
+    kstar = (p22 << 10) | s_res[0];
+    ties_kept = s_res[1];
+  }
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i)
-    hist_add_warp(s_hist, key[i] != 0u, key[i] >> 21);
-  __syncthreads();
-  rows_find_bin<T, kRowsBins>(s_hist, uint32_t(p.topk), s_warp, s_res);
-  const uint32_t b1 = s_res[0];
-  uint32_t need = s_res[1];
-  clear();
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < ITEMS; ++i) hist_add_warp(s_hist, key[i] != 0u && (key[i] >> 21) == b1, (key[i] >> 10) & 2047u);
-  __syncthreads();
-  rows_find_bin<T, kRowsBins>(s_hist, need, s_warp, s_res);
-  const uint32_t p22 = (b1 << 11) | s_res[0];
-  need = s_res[1];
-  clear();
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < ITEMS; ++i) hist_add_warp(s_hist, key[i] != 0u && (key[i] >> 10) == p22, key[i] & 1023u);
-  __syncthreads();
-  rows_find_bin<T, 1024>(s_hist, need, s_warp, s_res);
-  const uint32_t kstar = (p22 << 10) | s_res[0];
-  const uint32_t ties_kept = kstar ? s_res[1] : 0u;  // (0: fewer than k numbers in the row, all of them kept)
+    if (!key_is_number(key[i])) key[i] = 0u;
 
   // (kept, tie) counts of the warps' shares in position order, then the slots
   uint32_t cnt = 0;
@@ -136,7 +152,8 @@ topk_rows_kernel(const Params p) {
   __syncthreads();
   const uint32_t wt = lane < kWarps ? s_warp[lane] : 0u;
   const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
-  if (kstar == 0u) pad_from(__reduce_add_sync(0xffffffffu, wt) & 0xFFFFu);
+  const uint32_t all = __reduce_add_sync(0xffffffffu, wt), total = (all & 0xFFFFu) + min(all >> 16, ties_kept);
+  if (total < uint32_t(p.topk)) pad_from(total);
   uint32_t g = before & 0xFFFFu, q = before >> 16;
   const uint32_t below = (1u << lane) - 1u;
 #pragma unroll
@@ -180,7 +197,7 @@ topk_solo_kernel(const Params p) {
   const int64_t r = blockIdx.x;
   for (int i = tid; i < kClWarps * ITEMS; i += kClThreads) s_mask[i] = 0u;
   if (tid < kL2Bins) s_h2[tid] = 0u;
-  if (tid == 0) s_nsurv = 0u;
+  if (tid == 0) s_nsurv = 0u, s_res[3] = 0u;
   DSA_KTIME_BEGIN(1);
   pdl_launch_dependents();  // (before the wait, as the cluster kernel does: see there)
   pdl_wait();
@@ -202,9 +219,12 @@ topk_solo_kernel(const Params p) {
       page[i] = first < n ? p.page_table[r * p.pt_stride + (first >> 6)] : 0;
     }
   }
-  // ordered keys; 0 (below every number) past the row's length
+  // ordered keys; 0 (below every number) for NaNs and past the row's length
 #pragma unroll
-  for (int i = 0; i < ITEMS; ++i) key[i] = base + 32 * i < len ? ordered_key(__uint_as_float(key[i])) : 0u;
+  for (int i = 0; i < ITEMS; ++i) {
+    key[i] = base + 32 * i < len ? ordered_key(__uint_as_float(key[i])) : 0u;
+    if (!key_is_number(key[i])) key[i] = 0u;
+  }
   gh[0] = make_uint4(0, 0, 0, 0);                // re-armed: every thread clears the bins that it has read
   gh[1] = make_uint4(0, 0, 0, 0);
 
@@ -214,7 +234,7 @@ topk_solo_kernel(const Params p) {
   if (len <= p.topk) {
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i)
-      if (base + 32 * i < len) kept |= 1u << i;
+      if (key[i] != 0u) kept |= 1u << i;
     __syncthreads();
   } else {
     const uint32_t cnt8[8] = {h1b.w, h1b.z, h1b.y, h1b.x, h1a.w, h1a.z, h1a.y, h1a.x};  // highest bin first

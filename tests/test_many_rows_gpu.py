@@ -205,3 +205,41 @@ def test_solo_topk_with_the_scans_histogram(ops, n, k, kind):
     ref = expected(x, lens, k, -10)
     assert torch.equal(got, torch.where(ref == -10, torch.tensor(-3, dtype=torch.int32), ref + 7))
     assert int(hist.abs().sum()) == 0  # re-armed for the next scan
+
+
+@pytest.mark.parametrize("n,k", [(60, 16), (60, 100), (512, 64), (2048, 300), (4096, 2048), (4096, 5000), (6000, 64)])
+def test_nans_are_ranked_and_not_selected_by_any_kernel(ops, n, k):
+    """Rows with NaNs by the three kernels that a row of this size can take (one CTA without a histogram, one with
+    the scan's, the cluster kernel): the same positions. A NaN takes a rank and is not selected."""
+    torch.manual_seed(n + k)
+    x = torch.randn(ROWS, n)
+    x[:, ::7] = float("-inf")
+    for r, share in enumerate((0.0, 0.01, 0.2, 0.9, 1.0)):
+        x[r][torch.rand(n) < share] = float("nan")
+    x[1, 0] = -float("nan")
+    lens = torch.full((ROWS,), n, dtype=torch.int32)
+    lens[5:8] = torch.tensor([0, n // 2, min(k, n)], dtype=torch.int32)
+    x[6, : n // 4] = float("nan")
+    x[7, 1::3] = float("nan")
+    few = 8
+    cluster = ops.topk_select(x[:few].cuda(), k, lens[:few].cuda(), pad_value=-3, index_offset=5).cpu()
+    for r in range(few):  # the rule itself
+        row = x[r, : int(lens[r])]
+        nans = int(row.isnan().sum())
+        kept = row.numel() if k >= row.numel() else max(0, k - nans)
+        numbers = torch.sort(row[~row.isnan()], descending=True, stable=True).indices[:kept]
+        pos = torch.nonzero(~row.isnan()).flatten()[numbers].sort().values
+        want = torch.full((k,), -3, dtype=torch.int32)
+        want[: pos.numel()] = torch.where(torch.isneginf(row[pos]), torch.tensor(-3), pos.int() + 5).int()
+        assert torch.equal(cluster[r], want), r
+    rows = ops.topk_select(x.cuda(), k, lens.cuda(), pad_value=-3, index_offset=5).cpu()
+    assert torch.equal(rows[:few], cluster)
+    hist = torch.zeros(few, 4096, dtype=torch.int32)
+    for r in range(few):  # (the scan counts a NaN in the last bin, whatever its sign)
+        row = x[r, : int(lens[r])]
+        bits = (row[~row.isnan()] + 0.0).view(torch.int32)
+        key = torch.where(bits < 0, ~bits, bits ^ -(1 << 31)).long() & 0xFFFFFFFF
+        hist[r] = torch.bincount(key >> 20, minlength=4096).int()
+        hist[r, 4095] += int(row.isnan().sum())
+    solo = ops.topk_select(x[:few].cuda(), k, lens[:few].cuda(), hist=hist.cuda(), pad_value=-3, index_offset=5).cpu()
+    assert torch.equal(solo, cluster)
