@@ -11,10 +11,12 @@
 #include <ATen/ATen.h>
 #include <c10/core/GradMode.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
 #include <cmath>
+#include <exception>
 #include <initializer_list>
 #include <optional>
 #include <stdexcept>
@@ -923,8 +925,8 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
     PyObject* r = PyObject_CallFunction(status_check, "i", e.status);  // raises with the library's message
     if (r) PyErr_SetString(PyExc_RuntimeError, "dsa_b200: call failed");
     Py_XDECREF(r);
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {  // torch's own errors, as its Python functions raise them (an allocation's OutOfMemoryError among them)
+    torch::translate_exception_to_python(std::current_exception());
   }
   return nullptr;
 }
