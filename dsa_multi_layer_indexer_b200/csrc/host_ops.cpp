@@ -443,6 +443,7 @@ PyObject* rmsnorm(PyObject* const* a) {
   const Tensor w = ten(a[1], "weight").to(x.scalar_type()).contiguous();
   const Tensor out = at::empty_like(x);
   const int64_t dim = x.size(-1);
+  need(dim > 0, "rows of no elements have no norm");
   const float eps = float(real(a[2]));
   void* st = stream();
   LAUNCH(api.dsa_rmsnorm(ptr(x), ptr(w), ptr(out), x.numel() / dim, int(dim), eps, x.scalar_type() == at::kFloat ? 0 : 1, st));
@@ -456,6 +457,7 @@ PyObject* add_rmsnorm(PyObject* const* a) {
   need(x0.is_cuda() && (type == at::kBFloat16 || type == at::kFloat) && d0.scalar_type() == type && x0.sizes() == d0.sizes(),
        "x and delta must be CUDA bf16 or fp32 tensors of one shape");
   const int64_t dim = x0.size(-1);
+  need(dim > 0, "rows of no elements have no norm");
   need(type == at::kFloat || (dim % 8 == 0 && dim <= 8192), "the row length must be a multiple of 8 and at most 8192");
   const Tensor x = x0.contiguous(), d = d0.contiguous();
   const Tensor w = ten(a[2], "weight").to(type).contiguous();
@@ -742,7 +744,9 @@ PyObject* full_operands(PyObject* const* a) {
   const Tensor& xn = ten(a[0], "x_norm");
   const at::ScalarType type = xn.scalar_type();
   const int dt = dtype_of(type);
-  const int64_t seq = integer(a[1]), hidden = xn.size(-1), rows = xn.numel() / hidden;
+  const int64_t seq = integer(a[1]), hidden = xn.size(-1);
+  need(seq > 0 && hidden > 0, "x_norm must be [B, S, hidden] with S, hidden > 0");
+  const int64_t rows = xn.numel() / hidden;
   const Tensor *cq_in = opt(a[2], "c_q"), *wx = opt(a[3], "wx"), *wc = opt(a[4], "wc");
   const Tensor &q_a = ten(a[5], "q_a"), &kv_a = ten(a[6], "kv_a"), &ik_w = ten(a[7], "ik"), &q_b = ten(a[8], "q_b"), &iq_w = ten(a[9], "iq"),
                &w_w = ten(a[10], "w"), &q_norm = ten(a[11], "q_norm"), &kv_norm = ten(a[12], "kv_norm"), &kv_b = ten(a[13], "kv_b");
@@ -750,6 +754,7 @@ PyObject* full_operands(PyObject* const* a) {
   const Tensor *kv_given = opt(a[18], "kv"), *ik_given = opt(a[19], "ik"), *iks_given = opt(a[20], "ik_scale");
   const bool attention = truth(a[21]), indexer = truth(a[22]), fp8 = truth(a[23]);
   const int64_t H = integer(a[24]), nope = integer(a[25]), Hidx = integer(a[26]);
+  need(H > 0, "no heads");
   const int interleave = truth(a[27]);
   const float eps = float(real(a[28]));
   Tensor q_full, kv, iq, iw, ik, iks;
@@ -830,6 +835,7 @@ PyObject* full_operands(PyObject* const* a) {
 PyObject* project_output(PyObject* const* a) {
   const Tensor &o = ten(a[0], "o"), &kv_b = ten(a[1], "kv_b"), &o_proj = ten(a[2], "o_proj");
   const int64_t H = integer(a[3]), v = integer(a[4]), rows = o.size(0);
+  need(H > 0, "no heads");
   Tensor y;
   {
     NoGil unlocked;
