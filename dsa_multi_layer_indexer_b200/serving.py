@@ -25,7 +25,7 @@ from . import ops
 
 _FP8_ROW = ops.FP8_LATENT_ROW
 _plans: Dict[Tuple, "_Plan"] = {}
-_SELECT = {True: "exact", False: "prod", "kernel": "exact", "approx": "exact", "exact": "exact", "prod": "prod",
+_SELECT = {"kernel": "exact", "approx": "exact", "exact": "exact", "prod": "prod",
            "prod_side": "prod",  # the side-stream placement is the caller's business
            "torch": "torch"}
 
@@ -99,7 +99,8 @@ def fused_hide_decode_paged(
     ``select="torch"`` (torch.topk gate)."""
     if mode not in ("full", "attn_only", "scan_only"):
         raise ValueError(f"unknown mode={mode!r}")
-    sel_mode = _SELECT.get(select)
+    # (by identity: 1 and 0 equal True and False, and are no selections)
+    sel_mode = "exact" if select is True else "prod" if select is False else _SELECT.get(select) if isinstance(select, str) else None
     if sel_mode is None:
         raise ValueError(f"unknown select={select!r}")
     if q_all.dim() != 4 or q_all.shape[0] != 1:
