@@ -1342,7 +1342,7 @@ int dsa_decode_prep(const void* iq_raw, const void* w_raw, const void* ik_raw, c
                     const int64_t* positions, uint8_t* index_q, float* index_w, void* q_full,
                     uint8_t* cache_index_k, float* cache_k_scale, void* cache_kv, int B, int H,
                     int n_index_heads, int64_t cap, int interleave, float eps, void* stream) {
-  DSA_REQUIRE(iq_raw && w_raw && ik_raw && kv_a && q_pe && kv_norm_w && mla_cos && mla_sin && idx_cos &&
+  DSA_REQUIRE(iq_raw && w_raw && ik_raw && kv_a && q_abs && q_pe && kv_norm_w && mla_cos && mla_sin && idx_cos &&
                   idx_sin && positions && index_q && index_w && q_full && cache_index_k && cache_k_scale && cache_kv,
               "decode prep: null pointer");
   DSA_REQUIRE(aligned16(iq_raw) && aligned16(ik_raw) && aligned16(q_abs) && aligned16(q_full) && aligned16(index_q) &&

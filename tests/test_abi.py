@@ -152,3 +152,18 @@ def test_default_nsplit_heuristic():
         assert 1 <= n <= tiles
         if rows * (heads // 64) * tiles >= 128:
             assert tiles % n == 0 and rows * (heads // 64) * n <= max(148, rows * (heads // 64))
+
+
+def test_decode_prep_needs_the_absorbed_query():
+    """Without q_abs nothing would write the latent columns of q_full (dsa_decode_token absorbs them itself)."""
+    from dsa_multi_layer_indexer_b200 import _lib
+
+    h = _lib.lib()
+    buf = (ctypes.c_char * 64)()
+    addr = ctypes.addressof(buf)
+    addr += (-addr) % 16
+    for missing in range(6):  # iq_raw, w_raw, ik_raw, kv_a, q_abs, q_pe
+        five = [addr] * 6
+        five[missing] = None
+        rc = h.dsa_decode_prep(*five, 64, *[addr] * 12, 1, 16, 64, 128, 0, 1e-6, None)
+        assert rc == -1 and b"null pointer" in h.dsa_last_error(), missing
