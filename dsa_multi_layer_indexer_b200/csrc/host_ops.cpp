@@ -103,6 +103,16 @@ inline int64_t integer(PyObject* o) {
   if (v == -1 && PyErr_Occurred()) throw PyErrorSet();
   return v;
 }
+// int(o): for the arguments that Python code converted so, where a float or a one-element tensor was taken.
+inline int64_t whole(PyObject* o) {
+  if (PyLong_Check(o)) return integer(o);
+  PyObject* i = PyNumber_Long(o);
+  if (!i) throw PyErrorSet();
+  const int64_t v = PyLong_AsLongLong(i);
+  Py_DECREF(i);
+  if (v == -1 && PyErr_Occurred()) throw PyErrorSet();
+  return v;
+}
 inline double real(PyObject* o) {
   const double v = PyFloat_AsDouble(o);
   if (v == -1.0 && PyErr_Occurred()) throw PyErrorSet();
@@ -183,7 +193,7 @@ PyObject* scan_fp8(PyObject* const* a) {
   }
   if (R != n_seq * rps)
     bad("R=" + std::to_string(R) + " must equal n_seq=" + std::to_string(n_seq) + " * rows_per_seq=" + std::to_string(rps));
-  const int64_t ctx = a[6] == Py_None ? cap : integer(a[6]);
+  const int64_t ctx = a[6] == Py_None ? cap : whole(a[6]);
   need(ctx > 0 && ctx <= cap, "ctx must be in (0, cap]");
   const Tensor* lens = lens_of(a[4], R);
   const Tensor* given = opt(a[7], "out");
@@ -240,13 +250,13 @@ PyObject* scan_f32(PyObject* const* a) {
   const int64_t ctx = a[5] == Py_None ? cap : integer(a[5]);
   need(ctx > 0 && ctx <= cap, "ctx must be in (0, cap]");
   need(k.size(-1) == d, "index_k width differs from index_q");
-  need(w.numel() == R * heads, "index_w must be [R, H]");
+  need(w.numel() >= R * heads, "index_w must be [R, H]");
   need(R == n_seq * rps, "R must equal n_seq * rows_per_seq");
   const Tensor* lens = lens_of(a[3], R);
   const Tensor* given = opt(a[6], "out");
   const Tensor out = given ? *given : fresh({R, (ctx + 3) / 4 * 4}, at::kFloat, q);
   contig(out, "out", {at::kFloat});
-  need(out.dim() == 2 && out.size(0) == R && out.size(1) >= ctx, "out must be [R, >= ctx]");
+  need(out.dim() == 2 && out.size(0) >= R && out.size(1) >= ctx, "out must be [>= R, >= ctx]");
   void* st = stream();
   LAUNCH(api.dsa_indexer_scan_f32(as<float>(q), as<float>(w), as<float>(k), as<int32_t>(lens), as<float>(out), int(R), int(rps),
                               int(heads), int(d), ctx, cap, out.size(1), st));
@@ -280,7 +290,7 @@ PyObject* topk(PyObject* const* a) {
   const Tensor& x = ten(a[0], "logits");
   need(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 2, "logits must be CUDA fp32 [R, n]");
   need(x.stride(1) == 1, "logits rows must be dense");
-  const int64_t R = x.size(0), n = x.size(1), k = integer(a[1]);
+  const int64_t R = x.size(0), n = x.size(1), k = a[7] == Py_None ? integer(a[1]) : whole(a[1]);
   const int64_t slab = R > 1 ? x.stride(0) : std::max(x.stride(0), n);
   const Tensor* lens = lens_of(a[2], R);
   const Tensor* map = opt(a[4], "index_map");
@@ -304,7 +314,7 @@ PyObject* topk(PyObject* const* a) {
   }
   const Tensor* hist = hist_of(a[3], R);
   const Workspace ws = workspace_for(a[10], R, n, x);
-  const int32_t pad = int32_t(integer(a[5])), offset = int32_t(integer(a[6]));
+  const int32_t pad = int32_t(whole(a[5])), offset = int32_t(whole(a[6]));
   void* st = stream();
   LAUNCH(api.dsa_topk_select(as<float>(x), as<int32_t>(lens), as<uint32_t>(hist), as<int32_t>(map), as<int32_t>(idx),
                          val.defined() ? as<float>(val) : nullptr, ws.data, ws.bytes, int(R), n, slab, int(k),
@@ -374,7 +384,7 @@ PyObject* mla(PyObject* const* a) {
     need(idx->dim() == 2 && idx->size(0) == R, "indices must be [R, topk]");
     k = idx->size(1);
   } else {
-    k = a[11] == Py_None ? cap : integer(a[11]);
+    k = a[11] == Py_None ? cap : whole(a[11]);
   }
   const Tensor* lens = lens_of(a[4], R);
   const Tensor* ga = opt(a[7], "scratch.acc");
@@ -423,7 +433,7 @@ PyObject* mla_f32(PyObject* const* a) {
   const Tensor* idx = opt(a[2], "indices");
   if (idx) {
     contig(*idx, "indices", {at::kInt});
-    need(idx->dim() == 2 && idx->size(0) == R, "indices must be [R, topk]");
+    need(idx->dim() == 2 && idx->size(0) >= R, "indices must be [>= R, topk]");
   }
   const Tensor* lens = lens_of(a[5], R);
   const Tensor out = fresh({R, H, vd}, at::kFloat, q);
