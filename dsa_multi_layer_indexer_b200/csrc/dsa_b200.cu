@@ -487,8 +487,7 @@ static int launch_topk_rows(const topk::Params& p, int R, int64_t n, cudaStream_
   else if (n <= 2048) DSA_CUDA(launch_pdl(topk::topk_rows_kernel<256, 8>, grid, dim3(256), 0, st, p));
   else if (n <= 4096) DSA_CUDA(launch_pdl(topk::topk_rows_kernel<256, 16>, grid, dim3(256), 0, st, p));
   else if (n <= 6144) DSA_CUDA(launch_pdl(topk::topk_rows_kernel<256, 24>, grid, dim3(256), 0, st, p));
-  else if (n <= 8192) DSA_CUDA(launch_pdl(topk::topk_rows_kernel<256, 32>, grid, dim3(256), 0, st, p));
-  else DSA_CUDA(launch_pdl(topk::topk_rows_kernel<512, 32>, grid, dim3(512), 0, st, p));
+  else DSA_CUDA(launch_pdl(topk::topk_rows_kernel<256, 32>, grid, dim3(256), 0, st, p));
   return DSA_OK;
 }
 
@@ -504,8 +503,13 @@ static int launch_topk_solo(const topk::Params& p, int R, int64_t n, cudaStream_
 
 static int launch_topk_cluster(const topk::Params& p, int R, int64_t n, cudaStream_t st) {
   // More rows than SMs: the cluster kernel holds one row per SM and would take several waves of its
-  // latency-bound chain, the row kernel keeps several rows per SM in flight.
-  if (!p.hist && !p.n_src && !p.n_dest && R > sm_count() && n <= topk::kRowsMaxN) return launch_topk_rows(p, R, n, st);
+  // latency-bound chain, the row kernel keeps several rows per SM in flight: four of up to 4096 logits, three of
+  // up to 8192, which pays from the cluster kernel's third wave on. (Row against cluster kernel, k = 2048, us:
+  // 149 rows of 4096 10.6 / 15.7, of 6000 15.8 / 18.0, of 8192 19.9 / 19.2; 296 rows 10.9 / 16.4, 17.6 / 18.9,
+  // 22.4 / 19.9; 400 rows of 8192 22.9 / 29.2, 2048 rows 113 / 134. Rows of 12000 and 16384 with one CTA of 512
+  // threads per SM: 149 rows 35 / 22, 2048 rows 306 / 159: no.)
+  if (!p.hist && !p.n_src && !p.n_dest && R > sm_count() && (n <= 6144 || (n <= topk::kRowsMaxN && R > 2 * sm_count())))
+    return launch_topk_rows(p, R, n, st);
   const bool plain = p.hist && !p.n_src && !p.n_dest && !p.index_map && !p.out_val;
   if (plain && n <= topk::kSoloMaxN) return p.page_table ? launch_topk_solo<true>(p, R, n, st) : launch_topk_solo<false>(p, R, n, st);
   // As few CTAs as hold the row at 32 logits per thread: every CTA added costs cluster barriers and

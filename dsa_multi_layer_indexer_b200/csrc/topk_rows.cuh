@@ -1,4 +1,4 @@
-// Exact top-k of MANY short rows (a prompt's indexer: one row per token, up to 16384 logits, no
+// Exact top-k of MANY short rows (a prompt's indexer: one row per token, up to 8192 logits, no
 // histogram from the scan): one small CTA per row instead of the cluster kernel's 512 threads and
 // 192 KB of shared memory, so that several rows share an SM and hide one another's latencies.
 //
@@ -21,7 +21,7 @@ namespace dsa {
 namespace topk {
 
 constexpr int kRowsBins = 2048;
-constexpr int64_t kRowsMaxN = 16384;  // 512 threads x 32 logits
+constexpr int64_t kRowsMaxN = 8192;  // 256 threads x 32 logits
 
 // Whether a key is that of a number. A NaN (key above +inf's) takes a rank, as it does in the scan's histogram,
 // but is never selected: the places that this leaves are padding. (topk_cluster_kernel compares numbers.)
@@ -62,7 +62,7 @@ __device__ __forceinline__ void rows_find_bin(const uint32_t* h, uint32_t k, uin
 }
 
 template <int T, int ITEMS>
-__global__ void __launch_bounds__(T, T > 256 ? 1 : T < 256 ? 8 : ITEMS > 16 ? 3 : ITEMS > 8 ? 4 : 6)
+__global__ void __launch_bounds__(T, T < 256 ? 8 : ITEMS > 16 ? 3 : ITEMS > 8 ? 4 : 6)
 topk_rows_kernel(const Params p) {
   constexpr int kWarps = T / 32;
   __shared__ __align__(16) uint32_t s_hist[kRowsBins];

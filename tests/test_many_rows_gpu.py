@@ -243,3 +243,17 @@ def test_nans_are_ranked_and_not_selected_by_any_kernel(ops, n, k):
         hist[r, 4095] += int(row.isnan().sum())
     solo = ops.topk_select(x[:few].cuda(), k, lens[:few].cuda(), hist=hist.cuda(), pad_value=-3, index_offset=5).cpu()
     assert torch.equal(solo, cluster)
+
+
+@pytest.mark.parametrize("n", [6144, 6145, 8192, 8193])
+@pytest.mark.parametrize("rows", [149, 296, 297])
+def test_row_topk_around_the_line_to_the_cluster_kernel(ops, rows, n):
+    """Longer rows change kernel at two rows per SM (148 of them here) and at 8192 logits."""
+    torch.manual_seed(rows + n)
+    x = (torch.randn(rows, n) * 4).round() / 4
+    lens = torch.randint(n - 700, n + 1, (rows,), dtype=torch.int32)
+    got = ops.topk_select(x.cuda(), 700, lens.cuda(), pad_value=-3).cpu()
+    some = [0, 1, rows // 2, rows - 1]
+    assert torch.equal(got[some], expected(x[some], lens[some], 700, -3))
+    values = torch.where(torch.arange(n)[None] < lens[:, None], x, torch.tensor(float("-inf"))).topk(700, -1).values
+    assert torch.equal(x.gather(1, got.long()).sort(-1, descending=True).values, values)
