@@ -105,7 +105,7 @@ static int opt_in_smem(K kernel, size_t bytes, bool (&done)[64]) {
   if (dev >= 0 && dev < 64) done[dev] = true;
   return DSA_OK;
 }
-static bool g_opt_fused[64], g_opt_mla[4][64], g_opt_mla_tc[64], g_opt_mla_f32[64], g_opt_topk[64];
+static bool g_opt_fused[64], g_opt_mla[4][64], g_opt_mla_tc[64], g_opt_mla_f32[64], g_opt_scan_f32[64], g_opt_topk[64];
 
 // Launch with programmatic dependent launch allowed: the kernel may be scheduled
 // while its predecessor in the stream is still draining; it calls
@@ -396,6 +396,33 @@ int dsa_indexer_scan_f32(const float* index_q, const float* index_w, const float
   DSA_REQUIRE(k_seq_stride >= ctx && slab_stride >= ctx, "f32 indexer scan: strides must be >= ctx");
   const int groups = (rows_per_seq + scan::kF32Rows - 1) / scan::kF32Rows;
   const dim3 grid(unsigned((ctx + scan::kF32Keys - 1) / scan::kF32Keys), unsigned(R / rows_per_seq * groups));  // (y <= R <= 65535)
+  // The kernels that stage keys for several rows or heads win by throughput; a launch of few CTAs lasts as long as
+  // one CTA's chain of stagings, where a warp per key has more in flight, and beyond 128 dims a CTA restages its
+  // keys for every four heads (or every row). Their times in ns on this device, fitted to 112 measured shapes
+  // (us, warp per key / staged: 8 rows of one sequence, 64 heads of 128, 100 keys 27 / 206, 4096 keys 193 / 207,
+  // 32768 keys 1349 / 598; 64 rows, 16 heads of 64, 100 keys 13.5 / 31, 4096 keys 346 / 77; one row, 8 heads of 16,
+  // 100 keys 4.4 / 3.6; 64 rows, 4 heads of 256, 512 keys 20 / 42, 32768 keys 846 / 547; one row each 121 / 399):
+  const size_t keys_smem = (size_t(n_heads) * head_dim + n_heads) * sizeof(float);
+  const double h = n_heads, d = head_dim, key_floats = scan::kF32Keys * d;
+  const bool by_rows = rows_per_seq >= 4, wide = head_dim > scan::kF32Dims;
+  const int group_rows = std::min(rows_per_seq, scan::kF32Rows);
+  const double busy = 0.084 * R * double(ctx) * h * std::max(1.0, d / 200);  // a warp per key, all SMs busy
+  const double keys_ns = std::max(busy, 2400 + h * (220 + 1.25 * d) + busy / 2);
+  const double chain = by_rows ? 2200 + 2.9 * (scan::kF32Rows * h * d + key_floats * (wide ? h / 4 : 1))
+                               : 1500 + 2.4 * (group_rows * h * d + key_floats * (wide ? group_rows * std::max(1.0, h / 32) : 1)) + 1000.0 * group_rows;
+  const double staged_ns = chain * std::max(1.0, double(grid.x) * grid.y / (3.5 * sm_count()));  // 3 to 4 CTAs at a time per SM
+  const bool staged = staged_ns <= keys_ns;
+  if (!staged && keys_smem <= 200 * 1024) {
+    if (keys_smem > 48 * 1024) {
+      int rc = opt_in_smem(scan::indexer_scan_f32_keys_kernel, 200 * 1024, g_opt_scan_f32);
+      if (rc) return rc;
+    }
+    const int64_t want = (ctx + 7) / 8, most = std::max(1, (16 * sm_count() + R - 1) / R);
+    scan::indexer_scan_f32_keys_kernel<<<dim3(unsigned(std::min(want, most)), R), 256, keys_smem, static_cast<cudaStream_t>(stream)>>>(
+        index_q, index_w, index_k, seq_lens, logits, rows_per_seq, n_heads, head_dim, ctx, k_seq_stride, slab_stride);
+    DSA_CUDA(cudaGetLastError());
+    return DSA_OK;
+  }
   // four rows or more of a sequence: the warps split the rows; fewer: the heads
   auto kernel = rows_per_seq >= 4 ? scan::indexer_scan_f32_rows_kernel : scan::indexer_scan_f32_kernel;
   kernel<<<grid, scan::kF32Warps * 32, 0, static_cast<cudaStream_t>(stream)>>>(

@@ -548,7 +548,7 @@ indexer_scan_legacy_kernel(const Params p) {
 // rows (padded rows: a lane's 16-byte reads are conflict-free), a lane owns a key, each of the four
 // warps a quarter of the heads, whose sums meet in shared memory. Bound: shared-memory reads of the
 // queries (one broadcast 16 bytes per 4 multiply-adds of a warp, eight heads per key read). The form
-// with one warp per key and a five-step reduction per head took 204 us for 1024 rows x 512 keys x
+// with one warp per key and a five-step reduction per head (below) takes 204 us for 1024 rows x 512 keys x
 // 8 heads x 16 (fp32 preset, two prompts of 512) against 10 us.
 constexpr int kF32Keys = 32, kF32Rows = 8, kF32Warps = 4, kF32HeadsPerWarp = 8;
 constexpr int kF32Heads = kF32Warps * kF32HeadsPerWarp;  // heads whose queries are staged at a time
@@ -731,6 +731,41 @@ indexer_scan_f32_rows_kernel(const float* __restrict__ q, const float* __restric
   if (s < ctx) {
     if (ra < rows) logits[int64_t(row0 + ra) * slab_stride + s] = s < s_len[ra] ? ta : neg_inf;
     if (rb < rows) logits[int64_t(row0 + rb) * slab_stride + s] = s < s_len[rb] ? tb : neg_inf;
+  }
+}
+
+// The same scan for few keys or wide ones: a warp per key of one row, the lanes share its dims. Many small
+// independent pieces of work where the kernels above are a chain of stagings: those stage all queries of a CTA
+// one block after the other, and restage the keys for every row and head block beyond 128 dims.
+__global__ void __launch_bounds__(256)
+indexer_scan_f32_keys_kernel(const float* __restrict__ q, const float* __restrict__ w,
+                             const float* __restrict__ k, const int32_t* __restrict__ seq_lens,
+                             float* __restrict__ logits, int rows_per_seq, int n_heads, int head_dim,
+                             int64_t ctx, int64_t k_seq_stride, int64_t slab_stride) {
+  extern __shared__ float s_rowq[];  // [n_heads][head_dim] queries, then [n_heads] weights
+  const int r = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int n_q = n_heads * head_dim;
+  for (int i = threadIdx.x; i < n_q; i += blockDim.x) s_rowq[i] = q[int64_t(r) * n_q + i];
+  for (int i = threadIdx.x; i < n_heads; i += blockDim.x) s_rowq[n_q + i] = w[int64_t(r) * n_heads + i];
+  __syncthreads();
+  int64_t len = seq_lens ? int64_t(seq_lens[r]) : ctx;
+  len = len < 0 ? 0 : (len > ctx ? ctx : len);
+  const float* keys = k + int64_t(r / rows_per_seq) * k_seq_stride * head_dim;
+  float* out = logits + int64_t(r) * slab_stride;
+  for (int64_t s = int64_t(blockIdx.x) * warps + warp; s < ctx; s += int64_t(gridDim.x) * warps) {
+    if (s >= len) {
+      if (lane == 0) out[s] = __int_as_float(0xff800000);
+      continue;
+    }
+    float total = 0.f;
+    for (int h = 0; h < n_heads; ++h) {
+      float dot = 0.f;
+      for (int d = lane; d < head_dim; d += 32) dot = fmaf(s_rowq[h * head_dim + d], keys[s * head_dim + d], dot);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+      total = fmaf(s_rowq[n_q + h], fmaxf(dot, 0.f), total);
+    }
+    if (lane == 0) out[s] = total;
   }
 }
 

@@ -257,3 +257,11 @@ def test_row_topk_around_the_line_to_the_cluster_kernel(ops, rows, n):
     assert torch.equal(got[some], expected(x[some], lens[some], 700, -3))
     values = torch.where(torch.arange(n)[None] < lens[:, None], x, torch.tensor(float("-inf"))).topk(700, -1).values
     assert torch.equal(x.gather(1, got.long()).sort(-1, descending=True).values, values)
+
+
+# on both sides of the line between the kernels: a warp per key (few CTAs, wide keys), rows or heads of a CTA staged
+@pytest.mark.parametrize("rps,n_seq,heads,dim,ctx", [(8, 1, 64, 128, 130), (8, 1, 16, 64, 4700), (8, 1, 16, 64, 9001), (1, 1, 8, 32, 70),
+                                                     (1, 4, 8, 16, 70), (1, 2, 4, 256, 300), (8, 2, 3, 129, 600), (64, 4, 4, 130, 3000),
+                                                     (1, 1, 300, 200, 40), (2, 1, 400, 128, 33)])
+def test_f32_scan_kernels_agree_with_plain_arithmetic(ops, rps, n_seq, heads, dim, ctx):
+    test_f32_scan_matches_plain_arithmetic(ops, rps, n_seq, heads, dim, ctx)
