@@ -23,9 +23,10 @@ namespace topk {
 constexpr int kRowsBins = 2048;
 constexpr int64_t kRowsMaxN = 8192;  // 256 threads x 32 logits
 
-// Whether a key is that of a number. A NaN (key above +inf's) takes a rank, as it does in the scan's histogram,
-// but is never selected: the places that this leaves are padding. (topk_cluster_kernel compares numbers.)
-__device__ __forceinline__ bool key_is_number(uint32_t key) { return key - 0x007FFFFFu <= 0xFF800000u - 0x007FFFFFu; }
+// A NaN takes a rank above every number, as in topk_cluster_kernel, but is never selected: the places that this
+// leaves are padding. (The bits of a NaN behind an addition are the compiler's choice: it is asked for by value.)
+constexpr uint32_t kNanKey = 0xFFFFFFFFu;
+__device__ __forceinline__ uint32_t rank_key(float v) { return v != v ? kNanKey : ordered_key(v); }
 
 // Bin (from the top) that holds the k-th largest of an NB-bin histogram; thread t owns the NB / T bins
 // below NB - t * NB / T. s_res: bin, rank inside it. Every thread calls it; ends with a barrier.
@@ -108,7 +109,7 @@ topk_rows_kernel(const Params p) {
   // keys, not values, stay in registers; 0 (below every number) past the row's length
   uint32_t key[ITEMS];
 #pragma unroll
-  for (int i = 0; i < ITEMS; ++i) key[i] = base + 32 * i < len ? ordered_key(row[base + 32 * i]) : 0u;
+  for (int i = 0; i < ITEMS; ++i) key[i] = base + 32 * i < len ? rank_key(row[base + 32 * i]) : 0u;
   uint32_t kstar = 0u, ties_kept = 0u;  // (take_all: whatever is above 0)
   if (!take_all) {
     __syncthreads();  // the histogram is clear
@@ -138,7 +139,7 @@ topk_rows_kernel(const Params p) {
   }
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i)
-    if (!key_is_number(key[i])) key[i] = 0u;
+    if (key[i] == kNanKey) key[i] = 0u;
 
   // (kept, tie) counts of the warps' shares in position order, then the slots
   uint32_t cnt = 0;
@@ -222,8 +223,8 @@ topk_solo_kernel(const Params p) {
   // ordered keys; 0 (below every number) for NaNs and past the row's length
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) {
-    key[i] = base + 32 * i < len ? ordered_key(__uint_as_float(key[i])) : 0u;
-    if (!key_is_number(key[i])) key[i] = 0u;
+    const float v = __uint_as_float(key[i]);
+    key[i] = base + 32 * i < len && v == v ? ordered_key(v) : 0u;
   }
   gh[0] = make_uint4(0, 0, 0, 0);                // re-armed: every thread clears the bins that it has read
   gh[1] = make_uint4(0, 0, 0, 0);
