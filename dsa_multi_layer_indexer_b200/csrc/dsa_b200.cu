@@ -1585,10 +1585,14 @@ int dsa_sparse_mla_f32(const float* q, const float* kv, const int32_t* indices,
   DSA_REQUIRE(H > 0 && qk_dim > 0 && v_dim > 0 && v_dim <= qk_dim && v_dim <= 512,
               "f32 sparse MLA: need 0 < v_dim <= min(qk_dim, 512)");
   DSA_REQUIRE(indices == nullptr || topk_k > 0, "f32 sparse MLA: topk must be positive");
-  // Many rows: eight heads share the gathered keys; with fewer CTAs than SMs a CTA per head is faster.
+  // Many rows: eight heads share the gathered keys; with fewer CTAs than SMs a CTA per head is faster, and with one
+  // head there is nothing to share unless the list is short (a CTA per head waits for a chunk of 128 keys). (us, CTA
+  // per head / shared, 80-wide rows: one head, 148 rows of 200 keys 21.7 / 29.2, of 16 keys 7.0 / 4.4; two heads, 148
+  // rows of up to 300 keys 38.7 / 41.8, 160 rows of 200 keys 36.5 / 32.9; three heads 36.8 / 29.5 at 148 rows.)
   const int head_blocks = (H + mla::kF32Heads - 1) / mla::kF32Heads;
   const size_t rows_smem = mla::f32_rows_smem(qk_dim);
-  if (int64_t(R) * head_blocks >= sm_count() && rows_smem <= 200 * 1024) {
+  const bool shares = H >= 3 || (H == 2 && R > sm_count()) || (indices ? topk_k : kv_seq_stride) <= 64;
+  if (shares && int64_t(R) * head_blocks >= sm_count() && rows_smem <= 200 * 1024) {
     if (rows_smem > 48 * 1024) {
       int rc = opt_in_smem(mla::sparse_mla_f32_rows_kernel, 200 * 1024, g_opt_mla_f32);
       if (rc) return rc;

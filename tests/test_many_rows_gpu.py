@@ -265,3 +265,9 @@ def test_row_topk_around_the_line_to_the_cluster_kernel(ops, rows, n):
                                                      (1, 1, 300, 200, 40), (2, 1, 400, 128, 33)])
 def test_f32_scan_kernels_agree_with_plain_arithmetic(ops, rps, n_seq, heads, dim, ctx):
     test_f32_scan_matches_plain_arithmetic(ops, rps, n_seq, heads, dim, ctx)
+
+
+# one and two heads: a CTA per head unless the list is short, or there are more rows than SMs
+@pytest.mark.parametrize("H,topk", [(1, 64), (1, 65), (2, 70), (1, None)])
+def test_f32_attention_of_few_heads(ops, H, topk):
+    test_f32_attention_rows_match_plain_arithmetic(ops, H, 80, 64, topk)
