@@ -264,7 +264,7 @@ copy_post_epoch_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, i
 // rounding; as kSwiglu the MLP's product silu(W x) * (W2 x) with the roundings of its separate operations
 // (src/lagged_indexer_dsa/dsa_layer.py:87-143, :194-196).
 //
-// One or two rows of x (every decode step of a small batch). HBM-bound: the weights are streamed once, so
+// gemv_stream_kernel, for all but the smallest and the widest products. HBM-bound: the weights are streamed once, so
 // they are moved by the copy engine. A CTA per SM owns an even share of the rows, taken in pairs (for SwiGLU
 // the two matrices' rows of one output), so that x is read from shared memory and unpacked once for two
 // rows. Each of its sixteen warps keeps its own ring of two to four bulk copies of 2 x 2 KB and refills a slot as
@@ -492,8 +492,9 @@ gemv_stream_kernel(const GemvParams p) {
   }
 }
 
-// Three or four rows of x, and short rows of W: x staged in shared memory, one
-// row of W per warp with eight loads per lane in flight.
+// A few hundred short rows of W (one CTA per SM holds them at a row per warp: see dsa_gemv_bf16), and rows so long
+// that x does not fit beside the streaming kernel's ring: x staged in shared memory, one row of W per warp with
+// eight loads per lane in flight.
 template <int B>
 __global__ void __launch_bounds__(kGemvThreads)
 gemv_rows_kernel(const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ x,

@@ -23,7 +23,7 @@ def close(got, ref, mag):
 
 
 # k below, at and above one piece of a row, uneven last pieces, odd row counts, fewer rows than SMs, more sums
-# than one CTA per SM holds, x too long for the streaming kernel, three and four rows
+# than one CTA per SM holds, x so long that the streaming kernel's pieces are half as long, three and four rows
 @pytest.mark.parametrize("b,n,k", [(1, 1, 8), (1, 515, 16384), (2, 2240, 7168), (1, 7168, 520), (2, 18432, 264), (4, 300, 2048),
                                    (3, 4097, 512), (1, 1001, 1024), (2, 77, 2056), (2, 320001, 64), (1, 600001, 8), (1, 9, 49152),
                                    (2, 31, 24576)])
@@ -153,3 +153,16 @@ def test_reading_ahead_changes_nothing_but_the_time(ops, b):
     kv_b, o = bf(16 * 256, 512), bf(b, 16, 512)
     torch.cuda.synchronize()
     assert torch.equal(ops.value_project(kv_b, o, 16, 128), ops.value_project(kv_b, o, 16, 128, ahead=True))
+
+
+# both sides of the lines between the row kernel and the streaming kernel: few short rows of W, and rows of x too
+# long to lie beside the streaming kernel's ring
+@pytest.mark.parametrize("b,n,k", [(1, 256, 512), (2, 256, 520), (3, 257, 2048), (4, 1184, 2048), (1, 1185, 2048), (2, 1184, 2056), (3, 5, 8),
+                                   (1, 9, 90112), (2, 9, 47104), (4, 9, 24576), (3, 9, 24576)])
+def test_gemv_by_either_kernel(ops, b, n, k):
+    torch.manual_seed(n + k)
+    x = torch.randn(b, k + 16, device="cuda").to(torch.bfloat16)[:, 8:k + 8]
+    w = torch.randn(n, k, device="cuda").div_(k ** 0.5).to(torch.bfloat16)
+    close(ops.gemv(x, w), x.double() @ w.double().T, x.double().abs() @ w.double().abs().T)
+    torch.cuda.synchronize()
+    assert torch.equal(ops.gemv(x, w), ops.gemv(x, w, ahead=True))
