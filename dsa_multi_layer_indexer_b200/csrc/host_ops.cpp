@@ -348,8 +348,14 @@ PyObject* topk_paged(PyObject* const* a) {
 }
 
 // ---------------------------------------------------------------- sparse MLA
-// ops.default_nsplit
-int64_t default_nsplit(int64_t rows, int64_t heads, int64_t k, int64_t sms) {
+// The split count where a caller gives none. Head counts that are a multiple of 64 run on the tcgen05 kernel (one CTA
+// per SM, 64 heads per CTA) once the launch has 128 tiles of 64 heads x 64 keys: about one CTA per SM in total, and a
+// split count that divides the tiles so no split is empty. Smaller launches and other head counts run on the mma.sync
+// kernel (16 heads per CTA, two CTAs per SM). With more (row, head) pairs than SMs at most 16 splits: the merge reads
+// every split's partials, and more of them cost more than the shorter splits save (2 rows x 128 heads: 12.8 us with 16
+// splits, 14.9 with 32).
+constexpr int64_t kSms = 148;  // the default of ops.default_nsplit, which plans are made with on any machine
+int64_t default_split_count(int64_t rows, int64_t heads, int64_t k, int64_t sms) {
   const int64_t tiles = std::max<int64_t>(1, (k + 63) / 64);
   if (heads % 64 == 0 && rows * (heads / 64) * tiles >= 128) {
     const int64_t blocks = std::max<int64_t>(1, rows * (heads / 64));
@@ -361,6 +367,11 @@ int64_t default_nsplit(int64_t rows, int64_t heads, int64_t k, int64_t sms) {
   int64_t want = std::max<int64_t>(1, 2 * sms / blocks);
   if (rows * heads > sms) want = std::min<int64_t>(want, 16);
   return std::max<int64_t>(1, std::min(want, tiles));
+}
+
+// (rows, heads, topk, sm_count)
+PyObject* default_nsplit(PyObject* const* a) {
+  return PyLong_FromLongLong(default_split_count(whole(a[0]), whole(a[1]), whole(a[2]), whole(a[3])));
 }
 
 // (q, kv, indices, sm_scale, seq_lens, rows_per_seq, nsplit, acc, m, l, out, dense_keys, stage 0 both / 1 partials /
@@ -388,7 +399,7 @@ PyObject* mla(PyObject* const* a) {
   }
   const Tensor* lens = lens_of(a[4], R);
   const Tensor* ga = opt(a[7], "scratch.acc");
-  const int64_t nsplit = a[6] != Py_None ? integer(a[6]) : ga ? ga->size(1) : default_nsplit(R, H, k, 148);
+  const int64_t nsplit = a[6] != Py_None ? integer(a[6]) : ga ? ga->size(1) : default_split_count(R, H, k, kSms);
   const int64_t stage = integer(a[12]);
   Tensor acc, m, l;
   if (ga) {
@@ -974,7 +985,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
 #define M(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&entry<name, n>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&bind)), METH_FASTCALL, nullptr},
-    M(scan_fp8, 10), M(scan_paged, 8), M(scan_f32, 7), M(topk, 11), M(topk_paged, 7), M(mla, 14), M(mla_f32, 7), M(rmsnorm, 3),
+    M(scan_fp8, 10), M(scan_paged, 8), M(scan_f32, 7), M(topk, 11), M(topk_paged, 7), M(default_nsplit, 4), M(mla, 14), M(mla_f32, 7), M(rmsnorm, 3),
     M(add_rmsnorm, 4), M(silu_mul, 2), M(indexer_stage, 18), M(latent_append, 11), M(prefill_latents, 16), M(prefill_queries, 13), M(full_operands, 29), M(project_output, 5), M(mlp, 4),
     M(abi_scan, AbiArgs<decltype(::dsa_indexer_scan_fp8)>::value), M(abi_scan_paged, AbiArgs<decltype(::dsa_indexer_scan_fp8_paged)>::value),
     M(abi_topk, AbiArgs<decltype(::dsa_topk_select)>::value), M(abi_mla, AbiArgs<decltype(::dsa_sparse_mla_decode)>::value),

@@ -9,7 +9,6 @@ the call natively (``_lib.host()``, csrc/host_ops.cpp); the rest goes through ct
 
 from __future__ import annotations
 
-import math
 from typing import Optional, Tuple
 
 import torch
@@ -174,26 +173,9 @@ class MlaScratch:
 
 
 def default_nsplit(rows: int, heads: int, topk: int, sm_count: int = 148) -> int:
-    """Splits of the index list, each a whole number of 64-key tiles. Head counts
-    that are a multiple of 64 run on the tcgen05 kernel (one CTA per SM, 64 heads
-    per CTA) once the launch has 128 tiles of 64 heads x 64 keys: about one CTA per
-    SM in total, and a split count that divides the tiles so no split is empty.
-    Smaller launches and other head counts run on the mma.sync kernel (16 heads
-    per CTA, two CTAs per SM). With more (row, head) pairs than SMs at most 16 splits: the
-    merge reads every split's partials, and more of them cost more than the shorter splits
-    save (2 rows x 128 heads: 12.8 us with 16 splits, 14.9 with 32)."""
-    tiles = max(1, math.ceil(topk / 64))
-    if heads % 64 == 0 and rows * (heads // 64) * tiles >= 128:
-        blocks = max(1, rows * (heads // 64))
-        want = max(1, min(sm_count // blocks, 16, tiles))
-        while tiles % want:
-            want -= 1
-        return want
-    blocks = max(1, rows * (heads // HEAD_BLOCK))
-    want = max(1, (2 * sm_count) // blocks)
-    if rows * heads > sm_count:
-        want = min(want, 16)
-    return max(1, min(want, tiles))
+    """Splits of the index list, each a whole number of 64-key tiles, that :func:`sparse_mla_decode` takes by
+    itself: enough CTAs for the SMs without more partials than the merge should read (csrc/host_ops.cpp)."""
+    return _host().default_nsplit(rows, heads, topk, sm_count)
 
 
 def sparse_mla_decode(
