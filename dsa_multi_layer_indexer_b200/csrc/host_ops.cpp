@@ -36,8 +36,8 @@ using at::Tensor;
   X(dsa_indexer_scan_fp8) X(dsa_indexer_scan_fp8_paged) X(dsa_indexer_scan_f32) X(dsa_topk_workspace_bytes)    \
   X(dsa_topk_select) X(dsa_topk_select_paged) X(dsa_sparse_mla_partials) X(dsa_sparse_mla_combine)             \
   X(dsa_sparse_mla_decode) X(dsa_sparse_mla_decode_beside) X(dsa_sparse_mla_f32) X(dsa_rmsnorm)                \
-  X(dsa_add_rmsnorm_bf16) X(dsa_silu_mul_bf16) X(dsa_add_rmsnorm_f32) X(dsa_silu_mul_f32) X(dsa_linear_f32) X(dsa_indexer_stage_fp8) X(dsa_latent_append)                   \
-  X(dsa_prefill_latents) X(dsa_prefill_queries)
+  X(dsa_add_rmsnorm_bf16) X(dsa_silu_mul_bf16) X(dsa_add_rmsnorm_f32) X(dsa_silu_mul_f32) X(dsa_linear_f32)                \
+  X(dsa_indexer_stage_fp8) X(dsa_latent_append) X(dsa_prefill_latents) X(dsa_prefill_queries)
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
   DSA_HOST_API(X)
@@ -798,53 +798,59 @@ PyObject* full_operands(PyObject* const* a) {
       qa = y.narrow(1, 0, q_rank), kva = y.narrow(1, q_rank, width), ikr = y.narrow(1, q_rank + width, D);
     } else {
       linears(x, {{cq_in ? nullptr : &q_a, &qa}, {keep_kv ? &kv_a : nullptr, &kva}, {keep_ik ? &ik_w : nullptr, &ikr}});
-  }
-  c_q = cq_in ? cq_in->reshape({rows, q_rank}).contiguous() : fresh({rows, q_rank}, type, x);
-  if (kv_given) kv = *kv_given;
-  else if (keep_kv) kv = fresh({rows / seq, seq, width}, type, x);
-  if (ik_given) {
-    ik = *ik_given;
-    if (iks_given) iks = *iks_given;
-  } else if (keep_ik) {
-    ik = fresh({rows / seq, seq, D}, fp8 ? at::kByte : type, x);
-    if (fp8) iks = fresh({rows / seq, seq}, at::kFloat, x);
-  }
-  if (keep_kv) need(kv.is_contiguous() && kv.scalar_type() == type && kv.dim() == 3 && kv.size(0) * seq == rows && kv.size(1) >= seq && kv.size(2) == width, "latent cache: [n_seq, cap, w] of the operands' type");
-  if (keep_ik) need(ik.is_contiguous() && ik.dim() == 3 && ik.size(0) * seq == rows && ik.size(1) >= seq && ik.size(2) == D && (fp8 ? iks.defined() && iks.is_contiguous() : ik.scalar_type() == type), "index-key cache: [n_seq, cap, D]");
-  if (qa.defined() || keep_kv || keep_ik)
-    ok(api.dsa_prefill_latents(
-        qa.defined() ? ptr(qa) : nullptr, qa.defined() ? qa.stride(0) : 0, keep_kv ? ptr(kva) : nullptr, keep_kv ? kva.stride(0) : 0,
-        keep_ik ? ptr(ikr) : nullptr, keep_ik ? ikr.stride(0) : 0, ptr(q_norm), ptr(kv_norm), ptr(rope.mc), ptr(rope.ms), ptr(rope.ic),
-        ptr(rope.is), ptr(c_q), keep_kv ? ptr(kv) : nullptr, keep_kv ? kv.size(1) : 0, keep_ik ? ptr(ik) : nullptr,
-        iks.defined() ? as<float>(iks) : nullptr, keep_ik ? ik.size(1) : 0, rows, int(seq), int(q_rank), int(rank), int(rope_dim), int(D),
-        interleave, eps, dt, st));
+    }
+    c_q = cq_in ? cq_in->reshape({rows, q_rank}).contiguous() : fresh({rows, q_rank}, type, x);
+    if (kv_given) kv = *kv_given;
+    else if (keep_kv) kv = fresh({rows / seq, seq, width}, type, x);
+    if (ik_given) {
+      ik = *ik_given;
+      if (iks_given) iks = *iks_given;
+    } else if (keep_ik) {
+      ik = fresh({rows / seq, seq, D}, fp8 ? at::kByte : type, x);
+      if (fp8) iks = fresh({rows / seq, seq}, at::kFloat, x);
+    }
+    if (keep_kv)
+      need(kv.is_contiguous() && kv.scalar_type() == type && kv.dim() == 3 && kv.size(0) * seq == rows && kv.size(1) >= seq &&
+               kv.size(2) == width,
+           "latent cache: [n_seq, cap, w] of the operands' type");
+    if (keep_ik)
+      need(ik.is_contiguous() && ik.dim() == 3 && ik.size(0) * seq == rows && ik.size(1) >= seq && ik.size(2) == D &&
+               (fp8 ? iks.defined() && iks.is_contiguous() : ik.scalar_type() == type),
+           "index-key cache: [n_seq, cap, D]");
+    if (qa.defined() || keep_kv || keep_ik)
+      ok(api.dsa_prefill_latents(
+          qa.defined() ? ptr(qa) : nullptr, qa.defined() ? qa.stride(0) : 0, keep_kv ? ptr(kva) : nullptr, keep_kv ? kva.stride(0) : 0,
+          keep_ik ? ptr(ikr) : nullptr, keep_ik ? ikr.stride(0) : 0, ptr(q_norm), ptr(kv_norm), ptr(rope.mc), ptr(rope.ms), ptr(rope.ic),
+          ptr(rope.is), ptr(c_q), keep_kv ? ptr(kv) : nullptr, keep_kv ? kv.size(1) : 0, keep_ik ? ptr(ik) : nullptr,
+          iks.defined() ? as<float>(iks) : nullptr, keep_ik ? ik.size(1) : 0, rows, int(seq), int(q_rank), int(rank), int(rope_dim), int(D),
+          interleave, eps, dt, st));
 
-  // what reads c_q
-  Tensor q, iqr, w;
-  if (wc && attention && indexer) {
-    const Tensor y = linear_of(c_q, *wc);
-    q = y.narrow(1, 0, q_b.size(0)), iqr = y.narrow(1, q_b.size(0), iq_w.size(0)), w = y.narrow(1, q_b.size(0) + iq_w.size(0), Hidx);
-  } else {
-    linears(c_q, {{attention ? &q_b : nullptr, &q}, {indexer ? &iq_w : nullptr, &iqr}, {indexer ? &w_w : nullptr, &w}});
-  }
-  if (attention) {
-    q = q.unflatten(1, {H, nope + rope_dim});
-    q_full = fresh({rows, H, width}, type, x);
-    const Tensor w_uk = kv_b.view({H, kv_b.size(0) / H, rank}).narrow(1, 0, nope);
-    Tensor dst = q_full.narrow(2, 0, rank).transpose(0, 1);  // absorb W_UK: the GEMM writes its columns in place
-    at::bmm_out(dst, q.narrow(2, 0, nope).transpose(0, 1), w_uk);
-  }
-  if (indexer) {
-    need(iqr.size(1) == Hidx * D && w.size(1) == Hidx, "index_q_proj / index_weights_proj: wrong number of outputs");
-    iq = fresh({rows, Hidx, D}, fp8 ? at::kByte : type, x);
-    iw = fp8 ? fresh({rows, Hidx}, at::kFloat, x) : w.contiguous();
-  }
-  if (attention || indexer)
-    ok(api.dsa_prefill_queries(attention ? ptr(q) : nullptr, attention ? q.stride(0) : 0, attention ? q.stride(1) : 0, int(nope),
-                                   indexer ? ptr(iqr) : nullptr, indexer ? iqr.stride(0) : 0, indexer ? ptr(w) : nullptr,
-                                   indexer ? w.stride(0) : 0, ptr(rope.mc), ptr(rope.ms), ptr(rope.ic), ptr(rope.is),
-                                   attention ? ptr(q_full) : nullptr, indexer ? ptr(iq) : nullptr, indexer && fp8 ? as<float>(iw) : nullptr,
-                                   rows, int(seq), int(H), int(Hidx), int(rank), int(rope_dim), int(D), interleave, dt, st));
+    // what reads c_q
+    Tensor q, iqr, w;
+    if (wc && attention && indexer) {
+      const Tensor y = linear_of(c_q, *wc);
+      q = y.narrow(1, 0, q_b.size(0)), iqr = y.narrow(1, q_b.size(0), iq_w.size(0)), w = y.narrow(1, q_b.size(0) + iq_w.size(0), Hidx);
+    } else {
+      linears(c_q, {{attention ? &q_b : nullptr, &q}, {indexer ? &iq_w : nullptr, &iqr}, {indexer ? &w_w : nullptr, &w}});
+    }
+    if (attention) {
+      q = q.unflatten(1, {H, nope + rope_dim});
+      q_full = fresh({rows, H, width}, type, x);
+      const Tensor w_uk = kv_b.view({H, kv_b.size(0) / H, rank}).narrow(1, 0, nope);
+      Tensor dst = q_full.narrow(2, 0, rank).transpose(0, 1);  // absorb W_UK: the GEMM writes its columns in place
+      at::bmm_out(dst, q.narrow(2, 0, nope).transpose(0, 1), w_uk);
+    }
+    if (indexer) {
+      need(iqr.size(1) == Hidx * D && w.size(1) == Hidx, "index_q_proj / index_weights_proj: wrong number of outputs");
+      iq = fresh({rows, Hidx, D}, fp8 ? at::kByte : type, x);
+      iw = fp8 ? fresh({rows, Hidx}, at::kFloat, x) : w.contiguous();
+    }
+    if (attention || indexer)
+      ok(api.dsa_prefill_queries(attention ? ptr(q) : nullptr, attention ? q.stride(0) : 0, attention ? q.stride(1) : 0, int(nope),
+                                     indexer ? ptr(iqr) : nullptr, indexer ? iqr.stride(0) : 0, indexer ? ptr(w) : nullptr,
+                                     indexer ? w.stride(0) : 0, ptr(rope.mc), ptr(rope.ms), ptr(rope.ic), ptr(rope.is),
+                                     attention ? ptr(q_full) : nullptr, indexer ? ptr(iq) : nullptr, indexer && fp8 ? as<float>(iw) : nullptr,
+                                     rows, int(seq), int(H), int(Hidx), int(rank), int(rope_dim), int(D), interleave, dt, st));
   }
   PyObject* t = PyTuple_New(6);
   const Tensor* parts[6] = {&q_full, &kv, &iq, &iw, &ik, &iks};
@@ -890,8 +896,8 @@ PyObject* mlp(PyObject* const* a) {
       act = at::empty_like(g);
       if (type == at::kFloat) ok(api.dsa_silu_mul_f32(as<float>(g), as<float>(u), as<float>(act), g.numel(), st));
       else ok(api.dsa_silu_mul_bf16(ptr(g), ptr(u), ptr(act), g.numel(), st));
-  }
-  y = linear_of(act, down);
+    }
+    y = linear_of(act, down);
   }
   return THPVariable_Wrap(y);
 }
@@ -986,7 +992,8 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef methods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&bind)), METH_FASTCALL, nullptr},
     M(scan_fp8, 10), M(scan_paged, 8), M(scan_f32, 7), M(topk, 11), M(topk_paged, 7), M(default_nsplit, 4), M(mla, 14), M(mla_f32, 7), M(rmsnorm, 3),
-    M(add_rmsnorm, 4), M(silu_mul, 2), M(indexer_stage, 18), M(latent_append, 11), M(prefill_latents, 16), M(prefill_queries, 13), M(full_operands, 29), M(project_output, 5), M(mlp, 4),
+    M(add_rmsnorm, 4), M(silu_mul, 2), M(indexer_stage, 18), M(latent_append, 11), M(prefill_latents, 16), M(prefill_queries, 13),
+    M(full_operands, 29), M(project_output, 5), M(mlp, 4),
     M(abi_scan, AbiArgs<decltype(::dsa_indexer_scan_fp8)>::value), M(abi_scan_paged, AbiArgs<decltype(::dsa_indexer_scan_fp8_paged)>::value),
     M(abi_topk, AbiArgs<decltype(::dsa_topk_select)>::value), M(abi_mla, AbiArgs<decltype(::dsa_sparse_mla_decode)>::value),
     {nullptr, nullptr, 0, nullptr}};
