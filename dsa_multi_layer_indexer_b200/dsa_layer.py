@@ -19,8 +19,7 @@ caches, which the reference layer lacks.
 from __future__ import annotations
 
 import dataclasses
-from typing import Optional, Tuple
-
+from typing import List, Optional, Tuple
 
 import torch
 from torch import nn
@@ -42,19 +41,26 @@ def _bare(m: nn.Module, cls: type) -> bool:
             and not _module_hooks._global_forward_hooks and not _module_hooks._global_forward_pre_hooks)
 
 
-def _plain_weight(m: nn.Module, dtype: torch.dtype) -> Optional[torch.Tensor]:
-    """The weight of a bias-free ``nn.Linear`` that only multiplies by it - nothing hooked, replaced, patched or
-    quantised (a tensor subclass has its own product) - or None. (Hooks of every module: see ``_bare``.)"""
-    d = m.__dict__
-    p = d["_parameters"]
-    w = p.get("weight")
-    if (m.__class__ is not nn.Linear or w is None or w.dtype != dtype or p.get("bias") is not None or d["_forward_hooks"]
-            or d["_forward_pre_hooks"] or "forward" in d or w.__class__ not in _PLAIN_TENSORS):
-        return None
-    return w
+_LINEAR, _PARAMETER, _TENSOR = nn.Linear, nn.Parameter, torch.Tensor
 
 
-_PLAIN_TENSORS = (nn.Parameter, torch.Tensor)
+def _plain_weights(mods, names, dtype: torch.dtype) -> Optional[list]:
+    """The weights of bias-free ``nn.Linear`` modules that only multiply by them - nothing hooked, replaced, patched
+    or quantised (a tensor subclass has its own product) - or None if one is not that. (Hooks of every module: see
+    ``_bare``.) Runs once per layer of a prompt, on the path of its launches: 0.3 us per module."""
+    out = []
+    for name in names:
+        m = mods[name]
+        d = m.__dict__
+        p = d["_parameters"]
+        w = p["weight"] if "weight" in p else None
+        kind = w.__class__
+        if (m.__class__ is not _LINEAR or d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d or p.get("bias") is not None
+                or (kind is not _PARAMETER and kind is not _TENSOR) or w.dtype is not dtype):
+            return None
+        out.append(w)
+    return out
+
 
 # The linear projections of a layer, in construction order.
 _PROJECTIONS = ("q_a_proj", "q_b_proj", "kv_a_proj", "kv_b_proj", "o_proj", "index_q_proj", "index_k_proj",
@@ -150,7 +156,7 @@ class FullOperands:
     b: int
     s: int
     lens: torch.Tensor  # int32 [B*S]: causally visible keys of every row
-    weights: Optional[Tuple[torch.Tensor, ...]]
+    weights: Optional[List[torch.Tensor]]
     q: Optional[torch.Tensor]
     kv: Optional[torch.Tensor]
     iq: Optional[torch.Tensor]
@@ -352,7 +358,7 @@ class DSALayer(nn.Module):
                 cache.index_k[:, :s] = ik.float()
         return FullOperands(b, s, lens, None, q, kv, iq, w, ik, None)
 
-    def _full_weights(self, t: torch.Tensor) -> Optional[Tuple[torch.Tensor, ...]]:
+    def _full_weights(self, t: torch.Tensor) -> Optional[List[torch.Tensor]]:
         """The projections' weights, in construction order, where the fused full-sequence chain applies
         to ``t``, else None: it has no autograd or autocast, knows the fp32 form of any geometry and the
         bf16 / e4m3 form of the production geometry, and needs every projection to be a plain
@@ -363,16 +369,11 @@ class DSALayer(nn.Module):
             return None
         if dtype == torch.bfloat16 and self.config.qk_nope_head_dim % 4:  # (8-byte reads behind the query heads' nope part)
             return None
-        mods, out = self._modules, []
+        mods = self._modules
         qn, kn = mods["q_a_layernorm"], mods["kv_a_layernorm"]
         if not (_bare(qn, RMSNorm) and _bare(kn, RMSNorm) and qn.eps == kn.eps and qn.weight.dtype == dtype == kn.weight.dtype):
             return None
-        for name in _PROJECTIONS:
-            w = _plain_weight(mods[name], dtype)
-            if w is None:
-                return None
-            out.append(w)
-        return tuple(out)
+        return _plain_weights(mods, _PROJECTIONS, dtype)
 
     def _cache_fits(self, cache: "LayerDecodeCache", x: torch.Tensor) -> bool:
         """Whether the fused chain can write ``cache`` in place: a dense cache of the scan's form and the
@@ -477,16 +478,15 @@ class DSALayer(nn.Module):
 
     def _plain(self, name: str) -> bool:
         """A bias-free bf16 ``nn.Linear`` that only multiplies, of a width that the GEMV takes."""
-        m = self._modules[name]
-        w = _plain_weight(m, torch.bfloat16)
+        w = _plain_weights(self._modules, (name,), torch.bfloat16)
         return (w is not None and not _module_hooks._global_forward_hooks and not _module_hooks._global_forward_pre_hooks
-                and not torch.is_autocast_enabled() and m.in_features % 8 == 0 and w.is_contiguous())
+                and not torch.is_autocast_enabled() and w[0].shape[1] % 8 == 0 and w[0].is_contiguous())
 
     def _absorbed_rows(self, x: torch.Tensor) -> bool:
         """Whether a decode batch takes the kernels that read kv_b_proj's weight in place (one reading for all
         tokens; beyond HEAD_TOKENS rows the products are GEMMs)."""
         c, w = self.config, self.kv_b_proj.weight
-        return (x.shape[0] <= ops.HEAD_TOKENS and x.dtype == torch.bfloat16 and w.__class__ in _PLAIN_TENSORS and w.dtype == torch.bfloat16 and w.is_contiguous()
+        return (x.shape[0] <= ops.HEAD_TOKENS and x.dtype == torch.bfloat16 and w.__class__ in (_PARAMETER, _TENSOR) and w.dtype == torch.bfloat16 and w.is_contiguous()
                 and c.qk_nope_head_dim <= 512 and c.qk_nope_head_dim % 8 == 0 and c.q_lora_rank % 8 == 0 and not torch.is_grad_enabled())
 
     def new_cache(self, n_seq: int, capacity: int, device, fp8: bool) -> LayerDecodeCache:
