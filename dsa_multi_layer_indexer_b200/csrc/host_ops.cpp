@@ -758,6 +758,46 @@ Tensor linear_of(const Tensor& x, const Tensor& w) {
   return y;
 }
 
+// (modules, names, nn.Linear, nn.Parameter, torch.Tensor, bf16) -> the weights of the named modules of a layer, or None
+// unless every one of them is a bias-free nn.Linear of fp32 or bf16 that only multiplies by its weight: nothing hooked,
+// replaced, patched (a `forward` of the instance) or quantised (a tensor subclass has its own product).
+PyObject* plain_weights(PyObject* const* a) {
+  static PyObject *s_hooks = PyUnicode_InternFromString("_forward_hooks"), *s_pre = PyUnicode_InternFromString("_forward_pre_hooks"),
+                  *s_forward = PyUnicode_InternFromString("forward"), *s_params = PyUnicode_InternFromString("_parameters"),
+                  *s_weight = PyUnicode_InternFromString("weight"), *s_bias = PyUnicode_InternFromString("bias");
+  if (!PyDict_Check(a[0]) || !PyTuple_Check(a[1])) bad("plain_weights(modules, names, ...)");
+  const at::ScalarType type = truth(a[5]) ? at::kBFloat16 : at::kFloat;
+  const Py_ssize_t n = PyTuple_GET_SIZE(a[1]);
+  PyObject* out = PyList_New(n);
+  if (!out) throw PyErrorSet();
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* m = PyDict_GetItem(a[0], PyTuple_GET_ITEM(a[1], i));
+    PyObject* w = nullptr;
+    if (m && reinterpret_cast<PyObject*>(Py_TYPE(m)) == a[2]) {
+      PyObject* d = PyObject_GenericGetDict(m, nullptr);  // a new reference; what is looked up in it lives as long
+      if (!d) PyErr_Clear();
+      const auto none = [&](PyObject* key) {  // no hooks
+        PyObject* h = PyDict_GetItem(d, key);
+        return h && PyDict_Check(h) && PyDict_Size(h) == 0;
+      };
+      PyObject* params = d ? PyDict_GetItem(d, s_params) : nullptr;
+      if (params && PyDict_Check(params) && none(s_hooks) && none(s_pre) && PyDict_Contains(d, s_forward) == 0) {
+        PyObject *weight = PyDict_GetItem(params, s_weight), *bias = PyDict_GetItem(params, s_bias);
+        PyObject* kind = weight ? reinterpret_cast<PyObject*>(Py_TYPE(weight)) : nullptr;
+        if ((!bias || bias == Py_None) && (kind == a[3] || kind == a[4]) && THPVariable_Unpack(weight).scalar_type() == type)
+          w = same(weight);
+      }
+      Py_XDECREF(d);
+    }
+    if (!w) {
+      Py_DECREF(out);
+      Py_RETURN_NONE;
+    }
+    PyList_SET_ITEM(out, i, w);
+  }
+  return out;
+}
+
 // (x_norm, seq, c_q | None, wx | None, wc | None, q_a, kv_a, ik, q_b, iq, w, q_norm, kv_norm, kv_b,
 //  mla_cos, mla_sin, idx_cos, idx_sin, kv | None, ik_out | None, ik_scale | None, attention, indexer, fp8,
 //  heads, nope, index_heads, interleave, eps) -> (q_full, kv, iq, iw, ik, ik_scale)
@@ -993,7 +1033,7 @@ PyMethodDef methods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&bind)), METH_FASTCALL, nullptr},
     M(scan_fp8, 10), M(scan_paged, 8), M(scan_f32, 7), M(topk, 11), M(topk_paged, 7), M(default_nsplit, 4), M(mla, 14), M(mla_f32, 7), M(rmsnorm, 3),
     M(add_rmsnorm, 4), M(silu_mul, 2), M(indexer_stage, 18), M(latent_append, 11), M(prefill_latents, 16), M(prefill_queries, 13),
-    M(full_operands, 29), M(project_output, 5), M(mlp, 4),
+    M(plain_weights, 6), M(full_operands, 29), M(project_output, 5), M(mlp, 4),
     M(abi_scan, AbiArgs<decltype(::dsa_indexer_scan_fp8)>::value), M(abi_scan_paged, AbiArgs<decltype(::dsa_indexer_scan_fp8_paged)>::value),
     M(abi_topk, AbiArgs<decltype(::dsa_topk_select)>::value), M(abi_mla, AbiArgs<decltype(::dsa_sparse_mla_decode)>::value),
     {nullptr, nullptr, 0, nullptr}};

@@ -41,25 +41,10 @@ def _bare(m: nn.Module, cls: type) -> bool:
             and not _module_hooks._global_forward_hooks and not _module_hooks._global_forward_pre_hooks)
 
 
-_LINEAR, _PARAMETER, _TENSOR = nn.Linear, nn.Parameter, torch.Tensor
-
-
-def _plain_weights(mods, names, dtype: torch.dtype) -> Optional[list]:
-    """The weights of bias-free ``nn.Linear`` modules that only multiply by them - nothing hooked, replaced, patched
-    or quantised (a tensor subclass has its own product) - or None if one is not that. (Hooks of every module: see
-    ``_bare``.) Runs once per layer of a prompt, on the path of its launches: 0.3 us per module."""
-    out = []
-    for name in names:
-        m = mods[name]
-        d = m.__dict__
-        p = d["_parameters"]
-        w = p["weight"] if "weight" in p else None
-        kind = w.__class__
-        if (m.__class__ is not _LINEAR or d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d or p.get("bias") is not None
-                or (kind is not _PARAMETER and kind is not _TENSOR) or w.dtype is not dtype):
-            return None
-        out.append(w)
-    return out
+def _plain_weights(mods, names, dtype: torch.dtype) -> Optional[List[torch.Tensor]]:
+    """The weights of the named modules, each a bias-free ``nn.Linear`` of ``dtype`` that only multiplies by its own -
+    nothing hooked, replaced, patched or quantised - or None. (Hooks of every module: see ``_bare``.)"""
+    return _lib.host().plain_weights(mods, names, nn.Linear, nn.Parameter, torch.Tensor, dtype == torch.bfloat16)
 
 
 # The linear projections of a layer, in construction order.
@@ -486,7 +471,7 @@ class DSALayer(nn.Module):
         """Whether a decode batch takes the kernels that read kv_b_proj's weight in place (one reading for all
         tokens; beyond HEAD_TOKENS rows the products are GEMMs)."""
         c, w = self.config, self.kv_b_proj.weight
-        return (x.shape[0] <= ops.HEAD_TOKENS and x.dtype == torch.bfloat16 and w.__class__ in (_PARAMETER, _TENSOR) and w.dtype == torch.bfloat16 and w.is_contiguous()
+        return (x.shape[0] <= ops.HEAD_TOKENS and x.dtype == torch.bfloat16 and w.__class__ in (nn.Parameter, torch.Tensor) and w.dtype == torch.bfloat16 and w.is_contiguous()
                 and c.qk_nope_head_dim <= 512 and c.qk_nope_head_dim % 8 == 0 and c.q_lora_rank % 8 == 0 and not torch.is_grad_enabled())
 
     def new_cache(self, n_seq: int, capacity: int, device, fp8: bool) -> LayerDecodeCache:
