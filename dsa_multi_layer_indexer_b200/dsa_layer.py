@@ -567,8 +567,11 @@ class DSALayer(nn.Module):
             index_q = torch.empty(b, c.index_n_heads, c.index_head_dim, dtype=torch.uint8, device=x_norm.device)
             index_w = torch.empty(b, c.index_n_heads, dtype=torch.float32, device=x_norm.device)
             q_full = torch.empty(b, h, c.qk_head_dim, dtype=torch.bfloat16, device=x_norm.device)
+            norm_w = self.kv_a_layernorm.weight
+            if norm_w.dtype != torch.bfloat16:  # (norms kept in fp32: the launch reads bf16, as ops.rmsnorm converts it)
+                norm_w = norm_w.to(torch.bfloat16)
             if self._absorbed_rows(x_norm):
-                ops.decode_token(iq_raw, w, ik_raw, kv_a, q, self.kv_b_proj.weight, self.kv_a_layernorm.weight, rope.mla_cos,
+                ops.decode_token(iq_raw, w, ik_raw, kv_a, q, self.kv_b_proj.weight, norm_w, rope.mla_cos,
                                  rope.mla_sin, rope.idx_cos, rope.idx_sin, positions, index_q, index_w, q_full, cache.index_k,
                                  cache.k_scale, cache.kv, il, c.rms_norm_eps, ahead=True)
                 return q_full, index_q, index_w
@@ -579,7 +582,7 @@ class DSALayer(nn.Module):
         q_abs = torch.einsum("bhd,hdl->bhl", q_nope, w_uk)
         if fused:
             ops.decode_prep(iq_raw.contiguous(), w.contiguous(), ik_raw.contiguous(), kv_a.contiguous(),
-                            q_abs.contiguous(), q_rope, self.kv_a_layernorm.weight, rope.mla_cos, rope.mla_sin,
+                            q_abs.contiguous(), q_rope, norm_w, rope.mla_cos, rope.mla_sin,
                             rope.idx_cos, rope.idx_sin, positions, index_q, index_w, q_full, cache.index_k,
                             cache.k_scale, cache.kv, il, c.rms_norm_eps)
             return q_full, index_q, index_w

@@ -48,3 +48,20 @@ def test_batches_decode_as_their_sequences_alone(D, batch, mode_name):
     for i in (0, batch - 1):
         alone = decode(model, prompt[i:i + 1], toks[:, i:i + 1], mode, cold)
         assert rel(got[:, i:i + 1], alone) < 2e-2  # a few bf16 roundings (2^-9 each) per layer
+
+
+@pytest.mark.parametrize("batch", [1, 3, 9])
+def test_norm_weights_in_fp32(D, batch):
+    """A bf16 model whose norms stay in fp32 decodes as one with the same numbers in bf16."""
+    mode, cold = D.ScheduleMode.LAGGED_FUSED, D.ColdStartPolicy.EAGER
+    model = make_model(D)
+    norms = [m for m in model.modules() if type(m).__name__ == "RMSNorm"]
+    with torch.no_grad():
+        for m in norms:
+            m.weight.copy_(1.0 + torch.randint(-32, 33, m.weight.shape) / 64.0)
+    prompt = torch.randn(batch, 20, 256, device="cuda").to(torch.bfloat16)
+    toks = torch.randn(3, batch, 256, device="cuda").to(torch.bfloat16)
+    want = decode(model, prompt, toks, mode, cold)
+    for m in norms:
+        m.float()
+    assert rel(decode(model, prompt, toks, mode, cold), want) < 2e-2  # (bf16 roundings of norms by other kernels)
