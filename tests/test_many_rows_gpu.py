@@ -128,7 +128,8 @@ def test_f32_residual_norm_and_silu(ops):
 
 @pytest.mark.parametrize("m,k,ns", [(1, 4, (1,)), (64, 16, (32, 32, 32)), (65, 20, (33, 1, 70)), (1024, 256, (96, 80, 16)), (7, 300, (5, 9))])
 def test_small_f32_linears_match_fp64(m, k, ns):
-    """dsa_linear_f32 at the edges of its 64 x 32 x 16 tiles; 1e-6 of the row's sum of magnitudes."""
+    """dsa_linear_f32 at the edges of its 64 x 32 tiles, 64 deep; 1e-5 per term of products of N(0, 1) numbers (a sum of k
+    fp32 products in another order; of magnitudes: test_small_f32_swiglu_matches_fp64)."""
     from dsa_multi_layer_indexer_b200 import _lib
 
     torch.manual_seed(m + k)
@@ -271,3 +272,24 @@ def test_f32_scan_kernels_agree_with_plain_arithmetic(ops, rps, n_seq, heads, di
 @pytest.mark.parametrize("H,topk", [(1, 64), (1, 65), (2, 70), (1, None)])
 def test_f32_attention_of_few_heads(ops, H, topk):
     test_f32_attention_rows_match_plain_arithmetic(ops, H, 80, 64, topk)
+
+
+# one, two and several 64-deep slices, a part of one, both groups of threads, partial row and column tiles
+@pytest.mark.parametrize("m,n,k", [(1, 1, 4), (64, 32, 16), (65, 33, 20), (1024, 96, 256), (7, 5, 300), (65, 31, 64), (63, 65, 68), (130, 40, 1028)])
+def test_small_f32_swiglu_matches_fp64(m, n, k):
+    """Both matrices' sums, their fold over the thread groups and the slices' ring: 2^-24 per term and step of the
+    order, bounded by (k / 16 + 4) 2^-23 of the sum of magnitudes of each factor, and |silu'| < 1.1."""
+    from dsa_multi_layer_indexer_b200 import _lib
+
+    torch.manual_seed(m + n + k)
+    x, wg, wu = (torch.randn(r, k, device="cuda") for r in (m, n, n))
+    y = torch.full((m, n), 7.0, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(_lib.lib().dsa_linear_f32(x.data_ptr(), m, k, wg.data_ptr(), n, y.data_ptr(), wu.data_ptr(), n, None, None, 0, None, 1, st))
+    x, wg, wu = x.double(), wg.double(), wu.double()
+    g, u = x @ wg.T, x @ wu.T
+    step = (k / 16 + 4) * 2.0 ** -23
+    dg, du = x.abs() @ wg.abs().T * step, x.abs() @ wu.abs().T * step
+    silu = torch.nn.functional.silu(g)
+    err = 1.1 * dg * (u.abs() + du) + silu.abs() * du + (silu * u).abs() * 2.0 ** -20  # (expf, the division, the product)
+    assert float(((y.double() - silu * u).abs() - err).max()) <= 0.0

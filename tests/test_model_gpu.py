@@ -86,6 +86,48 @@ def test_lagged_fused_equals_lagged_reference_and_is_causal(D):
     assert a.indices_produced[-1] is None  # the last layer has no consumer
 
 
+@pytest.mark.parametrize("cold_name", ["DENSE", "EAGER"])
+def test_forward_equals_the_layers_public_methods(D, cold_name):
+    """The schedules written out with the layer API, attention and indexer each by themselves
+    (attention_output, indexer_indices) and from one query latent (fused_attention_and_indices), against
+    DSAModel.forward: the same kernels on the same operands, so the same selections and, up to the order of fp32
+    sums in the MLP and norms, the same hidden states."""
+    model = small_model(D, 11)
+    cold = D.ColdStartPolicy[cold_name]
+    torch.manual_seed(12)
+    x = torch.randn(2, 40, D.SMALL_CONFIG.hidden_size, device="cuda")
+    rope = model._build_rope(40, x.device, x.dtype)
+    n = len(model.layers)
+
+    def tail(layer, h, attn):
+        h = h + attn
+        return h + layer.mlp(layer.ffn_norm(h))
+
+    with torch.no_grad():
+        for mode in D.ScheduleMode:
+            h, prev, used = x, None, []
+            for li, layer in enumerate(model.layers):
+                x_norm = layer.attn_norm(h)
+                if mode is D.ScheduleMode.BASELINE:
+                    attend = layer.indexer_indices(x_norm, rope)
+                    attn = layer.attention_output(x_norm, rope, attend)
+                else:
+                    attend = prev
+                    if li == 0:
+                        attend = layer.indexer_indices(x_norm, rope) if cold is D.ColdStartPolicy.EAGER else None
+                    if mode is D.ScheduleMode.LAGGED_FUSED:
+                        attn, prev = layer.fused_attention_and_indices(x_norm, rope, attend, produce_indexer=li + 1 < n)
+                    else:
+                        attn = layer.attention_output(x_norm, rope, attend)
+                        prev = layer.indexer_indices(x_norm, rope) if li + 1 < n else None
+                used.append(attend)
+                h = tail(layer, h, attn)
+            got = model(x, mode, cold, record=True)
+            for a, b in zip(got.indices_used, used):
+                assert (a is None) == (b is None) and (a is None or torch.equal(a, b))
+            assert rel_err(got.final_hidden.cpu(), model.final_norm(h).cpu()) < 1e-5
+
+
 @pytest.mark.parametrize("mode_name", ["BASELINE", "LAGGED_FUSED"])
 def test_decode_equals_full_forward(D, mode_name):
     mode = D.ScheduleMode[mode_name]
