@@ -962,7 +962,7 @@ topk_cluster_kernel(const Params p, const int nk) {
       for (int i = 0; i < nk; ++i) {
         const bool in = i * 32 + lane + warp_off < live;
         const float v = in ? __uint_as_float(flat[warp_off + i * 32 + lane]) : 0.f;
-        hist_add_warp(local1, in, v != v ? uint32_t(kBins - 1) : ordered_key(v) >> kLowBits);  // (a NaN takes a rank)
+        hist_add_warp(local1, in, ordered_key(v) >> kLowBits);
       }
       DSA_STAMP(stamp_cta, 12);
       __syncthreads();
