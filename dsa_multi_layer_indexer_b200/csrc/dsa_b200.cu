@@ -398,7 +398,7 @@ int dsa_indexer_scan_f32(const float* index_q, const float* index_w, const float
   const dim3 grid(unsigned((ctx + scan::kF32Keys - 1) / scan::kF32Keys), unsigned(R / rows_per_seq * groups));  // (y <= R <= 65535)
   // The kernels that stage keys for several rows or heads win by throughput; a launch of few CTAs lasts as long as
   // one CTA's chain of stagings, where a warp per key has more in flight, and beyond 128 dims a CTA restages its
-  // keys for every four heads (or every row). Their times in ns on this device, fitted to 112 measured shapes
+  // keys for every four heads (or every row). Their times in ns on this device, fitted to 200 measured shapes
   // (us, warp per key / staged: 8 rows of one sequence, 64 heads of 128, 100 keys 27 / 206, 4096 keys 193 / 207,
   // 32768 keys 1349 / 598; 64 rows, 16 heads of 64, 100 keys 13.5 / 31, 4096 keys 346 / 77; one row, 8 heads of 16,
   // 100 keys 4.4 / 3.6; 64 rows, 4 heads of 256, 512 keys 20 / 42, 32768 keys 846 / 547; one row each 121 / 399):
@@ -406,11 +406,13 @@ int dsa_indexer_scan_f32(const float* index_q, const float* index_w, const float
   const double h = n_heads, d = head_dim, key_floats = scan::kF32Keys * d;
   const bool by_rows = rows_per_seq >= 4, wide = head_dim > scan::kF32Dims;
   const int group_rows = std::min(rows_per_seq, scan::kF32Rows);
-  const double busy = 0.084 * R * double(ctx) * h * std::max(1.0, d / 200);  // a warp per key, all SMs busy
-  const double keys_ns = std::max(busy, 2400 + h * (220 + 1.25 * d) + busy / 2);
+  // a warp per key: all SMs busy (with room for few CTAs beside 48 KB of queries and more), or a head at a time
+  const double busy = R * double(ctx) * (0.1 + 0.09 * h) * std::max(1.0, d / 200) * (keys_smem > 48 * 1024 ? 1.6 : 1.0);
+  const double keys_ns = std::max(2000 + busy, 2400 + h * (220 + 1.25 * d) + busy / 2);
   const double chain = by_rows ? 2200 + 2.9 * (scan::kF32Rows * h * d + key_floats * (wide ? h / 4 : 1))
                                : 1500 + 2.4 * (group_rows * h * d + key_floats * (wide ? group_rows * std::max(1.0, h / 32) : 1)) + 1000.0 * group_rows;
-  const double staged_ns = chain * std::max(1.0, double(grid.x) * grid.y / (3.5 * sm_count()));  // 3 to 4 CTAs at a time per SM
+  // (CTAs that an SM has under way at a time: 5 to 6 of the shortest, else 3 to 4)
+  const double staged_ns = chain * std::max(1.0, double(grid.x) * grid.y / ((chain < 8000 ? 5.5 : 3.5) * sm_count()));
   const bool staged = staged_ns <= keys_ns;
   if (!staged && keys_smem <= 200 * 1024) {
     if (keys_smem > 48 * 1024) {
