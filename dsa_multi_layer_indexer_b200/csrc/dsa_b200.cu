@@ -1199,11 +1199,12 @@ static int gemv(const void* w, const void* x, void* y, int batch, int n, int k, 
   int rc = gemv_checks(p, w, x, y, batch, 4, n, k, x_stride, y_stride, ahead);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // No more rows of W than there are warps in one CTA of the row kernel per SM, and short ones: the streaming
-  // kernel's rings, barriers and table of sums cost more than they hide. (Row / streaming kernel, us, one row of x:
+  // About as many rows of W as there are warps in one CTA of the row kernel per SM, short ones, 4 MB in all: the
+  // streaming kernel's rings, barriers and table of sums cost more than they hide. (Row / streaming kernel, us, one row of x:
   // [512, 512] 2.1 / 2.5, [1024, 1024] 2.4 / 3.0, [1024, 4096] 4.8 / 3.3, [2048, 1024] 2.7 / 2.7, [64, 512] 2.0 / 2.2,
-  // [64, 2048] 2.6 / 2.5; four rows [1024, 512] 3.3 / 4.6, [2048, 512] 4.4 / 4.0.)
-  const bool small = n <= 8 * sm_count() && k <= (n <= 256 ? 512 : 2048);
+  // [64, 2048] 2.6 / 2.5, [1184, 2048] 3.5 / 3.0, [1200, 512] 2.6 / 2.8; four rows [1024, 512] 3.3 / 4.6, [1200, 512] 4.3 /
+  // 4.6, [2048, 512] 4.4 / 4.0.)
+  const bool small = n <= 10 * sm_count() && k <= (n <= 256 ? 512 : 2048) && int64_t(n) * k <= 1 << 21;
   rc = small ? 1 : launch_gemv_stream(p, st);
   if (rc != 1) return rc;
   switch (batch) {
