@@ -407,7 +407,7 @@ int dsa_indexer_scan_f32(const float* index_q, const float* index_w, const float
   const bool by_rows = rows_per_seq >= 4, wide = head_dim > scan::kF32Dims;
   const int group_rows = std::min(rows_per_seq, scan::kF32Rows);
   // a warp per key: all SMs busy (with room for few CTAs beside 48 KB of queries and more), or a head at a time
-  const double busy = R * double(ctx) * (0.1 + 0.09 * h) * std::max(1.0, d / 200) * (keys_smem > 48 * 1024 ? 1.6 : 1.0);
+  const double busy = R * double(ctx) * (0.1 + 0.09 * h) * std::max(1.0, d / 200) * (keys_smem > 48 * 1024 ? 1.3 : 1.0);
   const double keys_ns = std::max(2000 + busy, 2400 + h * (220 + 1.25 * d) + busy / 2);
   const double chain = by_rows ? 2200 + 2.9 * (scan::kF32Rows * h * d + key_floats * (wide ? h / 4 : 1))
                                : 1500 + 2.4 * (group_rows * h * d + key_floats * (wide ? group_rows * std::max(1.0, h / 32) : 1)) + 1000.0 * group_rows;
@@ -1199,12 +1199,12 @@ static int gemv(const void* w, const void* x, void* y, int batch, int n, int k, 
   int rc = gemv_checks(p, w, x, y, batch, 4, n, k, x_stride, y_stride, ahead);
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // About as many rows of W as there are warps in one CTA of the row kernel per SM, short ones, 4 MB in all: the
+  // About as many rows of W as there are warps in one CTA of the row kernel per SM, short ones, 4 or 5 MB in all: the
   // streaming kernel's rings, barriers and table of sums cost more than they hide. (Row / streaming kernel, us, one row of x:
   // [512, 512] 2.1 / 2.5, [1024, 1024] 2.4 / 3.0, [1024, 4096] 4.8 / 3.3, [2048, 1024] 2.7 / 2.7, [64, 512] 2.0 / 2.2,
   // [64, 2048] 2.6 / 2.5, [1184, 2048] 3.5 / 3.0, [1200, 512] 2.6 / 2.8; four rows [1024, 512] 3.3 / 4.6, [1200, 512] 4.3 /
-  // 4.6, [2048, 512] 4.4 / 4.0.)
-  const bool small = n <= 10 * sm_count() && k <= (n <= 256 ? 512 : 2048) && int64_t(n) * k <= 1 << 21;
+  // 4.6, [1184, 2048] 3.9 / 4.9, [2048, 512] 4.4 / 4.0.)
+  const bool small = n <= 10 * sm_count() && k <= (n <= 256 ? 512 : 2048) && int64_t(n) * k <= (batch < 3 ? 4 : 5) << 19;
   rc = small ? 1 : launch_gemv_stream(p, st);
   if (rc != 1) return rc;
   switch (batch) {

@@ -157,7 +157,7 @@ def test_reading_ahead_changes_nothing_but_the_time(ops, b):
 
 # both sides of the lines between the row kernel and the streaming kernel: few short rows of W, and rows of x too
 # long to lie beside the streaming kernel's ring
-@pytest.mark.parametrize("b,n,k", [(1, 256, 512), (2, 256, 520), (3, 257, 2048), (4, 1024, 2048), (1, 1025, 2048), (2, 1480, 1416), (2, 1481, 64), (3, 5, 8),
+@pytest.mark.parametrize("b,n,k", [(1, 256, 512), (2, 256, 520), (3, 257, 2048), (4, 1280, 2048), (3, 1281, 2048), (1, 1024, 2048), (1, 1025, 2048), (2, 1480, 1416), (2, 1481, 64), (3, 5, 8),
                                    (1, 9, 90112), (2, 9, 47104), (4, 9, 24576), (3, 9, 24576)])
 def test_gemv_by_either_kernel(ops, b, n, k):
     torch.manual_seed(n + k)
