@@ -93,7 +93,11 @@ constexpr int kQTmem = 6;
 #ifndef DSA_MLA_TC_MIN_TILES
 #define DSA_MLA_TC_MIN_TILES 128  // (a build flag, for measuring the crossover)
 #endif
-constexpr int kMinTiles = DSA_MLA_TC_MIN_TILES;  // fewer 64x64 tiles than this: the mma.sync kernel is faster
+// Fewer 64 x 64 tiles than this: the mma.sync kernel. With the merge, each with its own best split (us, this kernel /
+// mma.sync): 32 tiles 11.6 / 9.3 (bf16 rows), 14.0 / 11.9 (fp8); 64 of one row 12.0 / 9.7, 14.8 / 12.3; 96 (3 rows of 64
+// heads) 12.0 / 13.5, 14.5 / 18.6; 128 12.6 / 15.5, 15.1 / 20.7; 256 14.5 / 22.4, 17.4 / 32.1. (Between 64 and 128 tiles
+// the line lies by the rows; 64 tiles of two rows are 11.4 / 11.4 and 12.0 / 14.0.)
+constexpr int kMinTiles = DSA_MLA_TC_MIN_TILES;
 
 struct Smem {
   static constexpr int q_off = 0;
@@ -114,7 +118,10 @@ static_assert(Smem::bytes <= 232448, "tcgen05 sparse MLA: shared memory over the
 
 // First / Rest: the two parts of a tile have landed; RestFree / Free: the value product has read the second
 // part / everything; SFull / SRead: scores computed / read; PFull: probabilities stored; OFull: all done.
-enum { kBarQ = 0, kBarFirst = 1, kBarRest = 4, kBarRestFree = 6, kBarFree = 8, kBarSFull = 11, kBarSRead = 12, kBarPFull = 13, kBarOFull = 14, kBarQT = 15 /* queries in tensor memory */, kNumBars = 16 };
+enum {
+  kBarQ = 0, kBarFirst = 1, kBarRest = 4, kBarRestFree = 6, kBarFree = 8, kBarSFull = 11, kBarSRead = 12, kBarPFull = 13, kBarOFull = 14,
+  kBarQT = 15 /* queries in tensor memory */, kNumBars = 16
+};
 
 // Named barrier 2 over the 192 threads of warps 0-5, plain and with an OR reduction.
 __device__ __forceinline__ void group_sync() { asm volatile("bar.sync 2, 192;" ::: "memory"); }

@@ -2,9 +2,10 @@
 
 Same module tree, parameter names and construction order as the reference's
 ``DSALayer`` (src/lagged_indexer_dsa/dsa_layer.py:55-196), so a ``state_dict``
-(or a seed) gives identical weights in both. The projections, norms, RoPE and
-the SwiGLU MLP are torch ops (cuBLAS GEMV/GEMM); the three hot operations --
-indexer logits, top-k selection, sparse MLA -- go to the CUDA library:
+(or a seed) gives identical weights in both. Large projections are the GEMM library's; the three
+hot operations -- indexer logits, top-k selection, sparse MLA -- and, without gradients and with plain
+modules, the norms, rotary embeddings, quantisation, SwiGLU product, small fp32 products and the
+projections of a few decode rows go to the CUDA library (otherwise torch ops, module by module):
 
 * production geometry (576-wide latent, 128-wide index keys) in bf16: FP8
   tcgen05 scan, exact top-k, split-K bf16 attention;
@@ -471,8 +472,8 @@ class DSALayer(nn.Module):
         """Whether a decode batch takes the kernels that read kv_b_proj's weight in place (one reading for all
         tokens; beyond HEAD_TOKENS rows the products are GEMMs)."""
         c, w = self.config, self.kv_b_proj.weight
-        return (x.shape[0] <= ops.HEAD_TOKENS and x.dtype == torch.bfloat16 and w.__class__ in (nn.Parameter, torch.Tensor) and w.dtype == torch.bfloat16 and w.is_contiguous()
-                and c.qk_nope_head_dim <= 512 and c.qk_nope_head_dim % 8 == 0 and c.q_lora_rank % 8 == 0 and not torch.is_grad_enabled())
+        return (x.shape[0] <= ops.HEAD_TOKENS and x.dtype == torch.bfloat16 and w.__class__ in (nn.Parameter, torch.Tensor)
+                and w.dtype == torch.bfloat16 and w.is_contiguous() and c.qk_nope_head_dim <= 512 and c.qk_nope_head_dim % 8 == 0 and c.q_lora_rank % 8 == 0 and not torch.is_grad_enabled())
 
     def new_cache(self, n_seq: int, capacity: int, device, fp8: bool) -> LayerDecodeCache:
         c = self.config
@@ -538,15 +539,14 @@ class DSALayer(nn.Module):
         il = c.indexer_rope_interleave
         if self._stacked():  # two GEMVs: everything that reads x_norm, then everything that reads c_q
             if ya is None:
-                # few output rows, long rows: the library GEMV is latency-bound there (measured 19-32 us
-                # against 13 us for the skinny kernel at one token); the other shapes stay with the library
+                # few output rows, long rows: the GEMM library's GEMV is latency-bound there (19-32 us against
+                # 7.5 for [2240, 7168] at one token); the other shapes stay with it
                 skinny = b <= 2 and x_norm.dtype == torch.bfloat16 and self._wx.shape[0] <= 4096 <= self._wx.shape[1]
                 ya = ops.gemv(x_norm, self._wx, ahead) if skinny else torch.nn.functional.linear(x_norm, self._wx)
             qa, kv_a, ik_raw = ya.split(
                 [c.q_lora_rank, c.kv_lora_rank + c.qk_rope_head_dim, c.index_head_dim], dim=-1)
             n = self.q_a_layernorm
-            # the c_q-side projection and the MLP's gate / up take the same kernel at one or two
-            # tokens (252 against 255 us per layer of the 8-layer stack)
+            # one or two tokens: the norm runs inside the c_q-side projection, as attn_norm and ffn_norm do
             if b <= 2 and self._norm_folds(n, qa):
                 yc = ops.norm_gemv(qa, None, n.weight, n.eps, self._wc, ahead=True)[1]
             else:

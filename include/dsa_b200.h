@@ -146,6 +146,7 @@ int dsa_indexer_scan_f32(const float* index_q, const float* index_w, const float
  *              (the reference's self-resetting SelScratch, :2150-2153). Calls
  *              that share a workspace must not overlap on the device.
  *   index_offset is added to positions when index_map is NULL.
+ * A NaN is never selected; it takes a rank, and the places that this leaves are padding.
  * Limit: n <= 1048576 per row.
  */
 int64_t dsa_topk_workspace_bytes(int R, int64_t n);
