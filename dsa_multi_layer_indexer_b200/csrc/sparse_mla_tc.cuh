@@ -144,6 +144,7 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // Byte offset of 16-byte unit `u` (0..7) of row `row` inside a swizzled chunk.
 __device__ __forceinline__ uint32_t swz(int row, int u) { return uint32_t(row * 128 + ((u ^ (row & 7)) << 4)); }
 
+template <bool kBeside>  // as in mla_partials_body
 __global__ void __launch_bounds__(kThreads, 1)
 sparse_mla_tc_kernel(const mla::Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -200,7 +201,7 @@ sparse_mla_tc_kernel(const mla::Params p) {
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *s_tmem, 0);
 
-  pdl_wait();  // the selection, the queries and the lengths may come from the previous kernel
+  if constexpr (!kBeside) pdl_wait();  // the selection, the queries and the lengths may come from the previous kernel
   pdl_launch_dependents();
 
   const int seq = r / p.rows_per_seq;
@@ -683,6 +684,7 @@ sparse_mla_tc_kernel(const mla::Params p) {
   tc_fence_before();
   __syncthreads();
   if (warp == kMmaWarp) tmem_dealloc(tmem, kTmemCols);
+  if constexpr (kBeside) pdl_wait();
   DSA_STAMP(scta, 15);
   DSA_KTIME_END(2);
 }
