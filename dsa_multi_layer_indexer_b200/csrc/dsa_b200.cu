@@ -105,7 +105,7 @@ static int opt_in_smem(K kernel, size_t bytes, bool (&done)[64]) {
   if (dev >= 0 && dev < 64) done[dev] = true;
   return DSA_OK;
 }
-static bool g_opt_fused[64], g_opt_mla[4][64], g_opt_mla_tc[64], g_opt_mla_f32[64], g_opt_scan_f32[64], g_opt_topk[64];
+static bool g_opt_fused[64], g_opt_mla_tc[2][64], g_opt_mla_f32[64], g_opt_scan_f32[64], g_opt_topk[64];
 
 // Launch with programmatic dependent launch allowed: the kernel may be scheduled
 // while its predecessor in the stream is still draining; it calls
@@ -909,6 +909,24 @@ static int mla_prepare(const void* q, const void* kv, const int32_t* indices, co
   return DSA_OK;
 }
 
+extern "C++" {
+template <bool kBeside, bool kDirect, int MT, int W>
+static int launch_mla_partials_as(const mla::Params& p, int R, int nsplit, cudaStream_t st) {
+  static bool done[64];
+  auto kernel = mla::sparse_mla_partials_kernel<kBeside, kDirect, MT, W>;
+  constexpr int smem = mla::SmemLayout<MT, MT>::bytes;
+  int rc = opt_in_smem(kernel, smem, done);
+  if (rc) return rc;
+  DSA_CUDA(launch_pdl(kernel, dim3(nsplit, p.H / (MT * DSA_HEAD_BLOCK), R), dim3(32 * W), smem, st, p));
+  return DSA_OK;
+}
+template <int MT, int W>
+static int launch_mla_partials(const mla::Params& p, int R, int nsplit, bool beside, cudaStream_t st) {
+  if (beside) return p.out ? launch_mla_partials_as<true, true, MT, W>(p, R, nsplit, st) : launch_mla_partials_as<true, false, MT, W>(p, R, nsplit, st);
+  return p.out ? launch_mla_partials_as<false, true, MT, W>(p, R, nsplit, st) : launch_mla_partials_as<false, false, MT, W>(p, R, nsplit, st);
+}
+}  // extern "C++"
+
 static int mla_partials_launch(const void* q, const void* kv, const int32_t* indices,
                                const int32_t* seq_lens, float* part_acc, float* part_m, float* part_l,
                                void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale,
@@ -919,6 +937,7 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
                         nsplit, sm_scale, kv_seq_stride, kv_fp8, out == nullptr, &p);
   if (rc0) return rc0;
   p.out = static_cast<__nv_bfloat16*>(out);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
   // Head counts that fill 64-row blocks go to the tcgen05 kernel once there are enough
   // 64-head x 64-key tiles to give every SM more than one (a single row of 2048 keys
   // is faster on the mma.sync kernel's 16-head CTAs); its splits are whole 64-key tiles.
@@ -926,21 +945,18 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
   if (H % mla_tc::kHG == 0 && sm_scale > 0.f && tc_tiles >= mla_tc::kMinTiles) {
     int kps = (topk_k + nsplit - 1) / nsplit;
     p.keys_per_split = (kps + mla_tc::kBN - 1) / mla_tc::kBN * mla_tc::kBN;
-    int rc = opt_in_smem(mla_tc::sparse_mla_tc_kernel, mla_tc::Smem::bytes, g_opt_mla_tc);
+    auto kernel = beside ? mla_tc::sparse_mla_tc_kernel<true> : mla_tc::sparse_mla_tc_kernel<false>;
+    int rc = opt_in_smem(kernel, mla_tc::Smem::bytes, g_opt_mla_tc[beside]);
     if (rc) return rc;
-    DSA_CUDA(launch_pdl(mla_tc::sparse_mla_tc_kernel, dim3(nsplit, H / mla_tc::kHG, R), dim3(mla_tc::kThreads),
-                        mla_tc::Smem::bytes, static_cast<cudaStream_t>(stream), p));
+    DSA_CUDA(launch_pdl(kernel, dim3(nsplit, H / mla_tc::kHG, R), dim3(mla_tc::kThreads), mla_tc::Smem::bytes, st, p));
     return DSA_OK;
   }
-  const size_t smem = kv_fp8 ? mla::SmemLayout::bytes_fp8 : mla::SmemLayout::bytes_bf16;
-  const auto launch = [&](auto kernel, bool (&done)[64]) {
-    int rc = opt_in_smem(kernel, mla::SmemLayout::bytes_fp8, done);
-    if (rc) return rc;
-    DSA_CUDA(launch_pdl(kernel, dim3(nsplit, H / DSA_HEAD_BLOCK, R), dim3(mla::kThreads), smem, static_cast<cudaStream_t>(stream), p));
-    return int(DSA_OK);
-  };
-  if (beside) return out ? launch(mla::sparse_mla_partials_beside_kernel<true>, g_opt_mla[3]) : launch(mla::sparse_mla_partials_beside_kernel<false>, g_opt_mla[2]);
-  return out ? launch(mla::sparse_mla_partials_kernel<true>, g_opt_mla[1]) : launch(mla::sparse_mla_partials_kernel<false>, g_opt_mla[0]);
+  // Where 16-head CTAs would share the SMs, 32 heads per CTA: the rows are gathered once for both blocks and, of a split
+  // of several tiles, the next tile is on its way. Attention + merge inside a step, us, 16 / 32 heads per CTA: one row
+  // of 128 heads (256 CTAs of one tile) 9.8 / 9.5, 3 rows of 64 (two tiles each) 13.9 / 12.6, 8 rows of 32 15.3 / 13.3.
+  const int64_t ctas = int64_t(nsplit) * (H / DSA_HEAD_BLOCK) * R;
+  if (H % (2 * DSA_HEAD_BLOCK) == 0 && ctas > sm_count()) return launch_mla_partials<2, 8>(p, R, nsplit, beside, st);
+  return launch_mla_partials<1, 4>(p, R, nsplit, beside, st);
 }
 
 int dsa_sparse_mla_partials(const void* q, const void* kv, const int32_t* indices,
@@ -950,6 +966,17 @@ int dsa_sparse_mla_partials(const void* q, const void* kv, const int32_t* indice
   return mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, nullptr, R, rows_per_seq, H, topk_k,
                              nsplit, sm_scale, kv_seq_stride, kv_fp8, false, stream);
 }
+
+extern "C++" {
+template <int kParts>
+static int launch_combine(const float* part_acc, const float* part_m, const float* part_l, void* out, int R, int H, int nsplit,
+                          cudaStream_t st) {
+  const int threads = 128 / kParts * (nsplit < 4 ? nsplit : 4);  // one load group per split, up to four
+  DSA_CUDA(launch_pdl(mla::sparse_mla_combine_kernel<kParts>, dim3(unsigned(H) * kParts, R), dim3(threads), 0, st, part_acc, part_m,
+                      part_l, static_cast<__nv_bfloat16*>(out), H, nsplit));
+  return DSA_OK;
+}
+}  // extern "C++"
 
 int dsa_sparse_mla_combine(const float* part_acc, const float* part_m, const float* part_l,
                            void* out, int R, int H, int nsplit, void* stream) {
@@ -965,12 +992,12 @@ int dsa_sparse_mla_combine(const float* part_acc, const float* part_m, const flo
                         part_l, static_cast<__nv_bfloat16*>(out), H, nsplit));
     return DSA_OK;
   }
-  // one load group of 128 threads per split, up to four
-  const int combine_threads = 128 * (nsplit < 4 ? nsplit : 4);
-  DSA_CUDA(launch_pdl(mla::sparse_mla_combine_kernel, dim3(H, R), dim3(combine_threads), 0,
-                      static_cast<cudaStream_t>(stream), part_acc, part_m, part_l,
-                      static_cast<__nv_bfloat16*>(out), H, nsplit));
-  return DSA_OK;
+  // few (row, head) pairs: their columns over several CTAs (16 pairs x 32 splits, attention + merge 7.5 -> 6.6 us inside a
+  // step; 64 pairs 8.1 -> 7.8); with as many CTAs as SMs or more the extra ones wait for room (128 pairs 2.9 -> 3.9 us)
+  const int64_t pairs = int64_t(R) * H;
+  if (4 * pairs <= sm_count()) return launch_combine<4>(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
+  if (2 * pairs <= sm_count()) return launch_combine<2>(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
+  return launch_combine<1>(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
 }
 
 int dsa_sparse_mla_decode(const void* q, const void* kv, const int32_t* indices,

@@ -16,11 +16,11 @@
 namespace dsa {
 namespace fused {
 
-constexpr int kThreads = scan::kThreads;  // 192; an attention CTA uses its first 128 threads
+constexpr int kAttnWarps = 4, kThreads = scan::kThreads;  // 192; an attention CTA uses its first 128 threads
 constexpr size_t kSmemBytes =
-    scan::smem_bytes<scan::kStagesTwoPerSm>() > size_t(mla::SmemLayout::bytes_bf16)
+    scan::smem_bytes<scan::kStagesTwoPerSm>() > size_t(mla::SmemLayout<1, 1>::bytes)
         ? scan::smem_bytes<scan::kStagesTwoPerSm>()
-        : size_t(mla::SmemLayout::bytes_bf16);
+        : size_t(mla::SmemLayout<1, 1>::bytes);
 
 __global__ void __launch_bounds__(kThreads, 2)
 fused_decode_kernel(const __grid_constant__ CUtensorMap tmap, const scan::Params ps, const mla::Params pm,
@@ -40,11 +40,11 @@ fused_decode_kernel(const __grid_constant__ CUtensorMap tmap, const scan::Params
     scan_id = b - n_pair;
   }
   if (attn_id >= 0) {
-    if (threadIdx.x >= mla::kThreads) return;  // two spare warps leave; the rest synchronise among themselves
+    if (threadIdx.x >= 32 * kAttnWarps) return;  // two spare warps leave; the rest synchronise among themselves
     const int split = attn_id % attn_splits;
     const int hg = (attn_id / attn_splits) % attn_hgs;
     const int r = attn_id / (attn_splits * attn_hgs);
-    mla::mla_partials_body<false>(pm, split, hg, r, fused_smem);
+    mla::mla_partials_body<false, false, 1, kAttnWarps>(pm, split, hg, r, fused_smem);
   } else {
     scan::scan_tc_body<scan::kStagesTwoPerSm>(&tmap, ps, scan_id % scan_gx, scan_gx, scan_id / scan_gx, fused_smem);
   }

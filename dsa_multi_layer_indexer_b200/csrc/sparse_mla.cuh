@@ -8,13 +8,18 @@
 // ref_sparse_mla :2950-2966): bf16 operands, fp32 accumulation, base-2 online
 // softmax, probabilities rounded to bf16 before the value product.
 //
-// One CTA = (query row, block of 16 heads, one split of the index list). The
+// One CTA = (query row, one or two blocks of 16 heads, one split of the index list). The
 // 1152-byte latent rows are gathered with one bulk asynchronous copy per row
 // (TMA engine, completion counted on an mbarrier) into padded shared-memory
 // rows, so the gather costs one instruction per row instead of 72 16-byte
 // copies per row. FP8 latent rows (656 B) are staged the same way and
 // dequantised into the bf16 tile exactly as the reference does
 // (fp8 -> f32, x group scale, round to bf16; :1181-1196).
+//
+// What bounds it (one 64-key tile per CTA, cycles after the dependency wait, 16 heads alone on an SM / 32 heads):
+// selection entries 650-950, rows and queries landed 2500-2900 / 3150 (an SM gets 45-61 bytes a cycle from L2),
+// scores 1400 / 2000 and values 700 / 1100 (shared-memory reads: 148 / 221 KB and 65 KB), maximum, softmax and their
+// barriers 900 / 1250, partials 1200 / 2300 (28 bytes a cycle).
 #pragma once
 
 
@@ -27,7 +32,7 @@ constexpr int kD = DSA_LATENT_DIM;       // 576
 constexpr int kDV = DSA_VALUE_DIM;       // 512
 constexpr int kHB = DSA_HEAD_BLOCK;      // 16 heads per CTA
 constexpr int kBN = 64;                  // keys per tile
-constexpr int kThreads = 128;            // 4 warps
+constexpr int kSlices = 8;               // groups of eight keys of a tile, each summed by itself
 constexpr int kRowBytes = kD * 2;        // 1152
 constexpr int kRowPitch = kRowBytes + 16;  // 1168: 8 consecutive rows hit 8 distinct bank groups
 constexpr int kPPitch = (kBN + 8) * 2;   // bf16 probabilities, padded the same way
@@ -53,30 +58,39 @@ struct Params {
   __nv_bfloat16* out;     // one split only: the normalised result goes here and no partials are written
 };
 
+// MT blocks of 16 heads share a CTA's gathered rows, NB tiles are on their way or in use at once.
+template <int MT, int NB>
 struct SmemLayout {
   static constexpr int q_off = 0;
-  static constexpr int k_off = q_off + kHB * kRowPitch;
-  static constexpr int p_off = k_off + kBN * kRowPitch;
-  static constexpr int red_off = p_off + kHB * kPPitch;         // float [2][4][16]
-  static constexpr int valid_off = red_off + 2 * 4 * kHB * 4;   // int [64]
-  static constexpr int bar_off = valid_off + kBN * 4;           // 2 mbarriers
-  static constexpr int bytes_bf16 = (bar_off + 16 + 15) & ~15;
-  static constexpr int bytes_fp8 = bytes_bf16;  // fp8 rows are staged inside their own bf16 slots
+  static constexpr int k_off = q_off + MT * kHB * kRowPitch;
+  static constexpr int p_off = k_off + NB * kBN * kRowPitch;
+  static constexpr int red_off = p_off + MT * kHB * kPPitch;             // float [2][8][16 MT]
+  static constexpr int swap_off = red_off + 2 * kSlices * MT * kHB * 4;  // float4 [8][MT][32]
+  static constexpr int valid_off = swap_off + kSlices * MT * 32 * 16;    // int [NB][64]
+  static constexpr int bar_off = valid_off + NB * kBN * 4;               // 1 + 2 NB mbarriers
+  static constexpr int bytes = (bar_off + 8 * (1 + 2 * NB) + 15) & ~15;
 };
+static_assert(SmemLayout<1, 1>::bytes * 2 <= 231424, "sparse MLA: two CTAs of one head block share an SM");
+static_assert(SmemLayout<2, 2>::bytes <= 232448, "sparse MLA: shared memory over the per-CTA limit");
 
-// Barrier over the 128 attention threads (named barrier 1). The split-K body also
-// runs inside a 192-thread CTA of the fused launch, whose two spare warps have
-// left, so it must not use the whole-CTA barrier.
-__device__ __forceinline__ void cta128_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-// Barrier of the same 128 threads that also ORs a flag over them: every thread gets the same answer.
-__device__ __forceinline__ bool cta128_any(bool flag) {
+// Barrier over the attention CTA's W warps (named barrier 1: in the fused launch others may have left).
+template <int W>
+__device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * W) : "memory"); }
+// The same barrier that also ORs a flag over the threads: every thread gets the same answer.
+template <int W>
+__device__ __forceinline__ bool cta_any(bool flag) {
   uint32_t r;
   asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(r)
-      : "r"(uint32_t(flag))
+      : "r"(uint32_t(flag)), "n"(32 * W)
       : "memory");
   return r != 0;
+}
+// Barrier of the two warps that share a key group (named barriers 2..5).
+__device__ __forceinline__ void pair_sync(int key_group) {
+  asm volatile("bar.sync %0, 64;" ::"r"(2 + key_group) : "memory");
 }
 
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
@@ -112,164 +126,199 @@ __device__ __forceinline__ uint2 dequant4(uint32_t w, float s) {
   return r;
 }
 
-// One 64-key tile for the 16 heads of the CTA: S = Q K^T on bf16 tensor cores,
-// base-2 online softmax across the four warps, P rounded to bf16, O += P V.
-// Warp w owns keys [16 w, 16 w + 16) in S and value columns [128 w, 128 w + 128)
-// in O. All 128 threads call it; it contains two block barriers.
-__device__ __forceinline__ void attend_tile(const uint8_t* s_q, const uint8_t* s_k, uint8_t* s_p,
-                                            float* s_red, const int* s_valid, float scale_log2,
-                                            int warp, int lane, float (&m_run)[2], float (&l_run)[2],
-                                            float (&acc)[16][4]) {
-  const int g = lane >> 2, t4 = lane & 3;
-  // ---- S = Q K^T: warp w owns keys [16 w, 16 w + 16) for all 16 heads
-  float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+// One 64-key tile for the 16 MT heads of a CTA of W = 4 or 8 warps: S = Q K^T on bf16 tensor cores,
+// base-2 online softmax across the warps, P rounded to bf16, O += P V.
+// Scores: of eight warps (dh, kg) multiplies keys [16 kg, 16 kg + 16) with half dh of the dims; the two warps of
+// a key group then swap, so that each holds the sums of eight keys for the softmax. Of four warps each does both
+// halves and holds sixteen keys: the same sums, added in the same order. Values: warp w owns 512 / W columns.
+// `landed` is this thread's outcome of its wait for the tile; where one ran out, all threads leave together
+// with false. Contains two block barriers.
+template <int MT, int W>
+__device__ __forceinline__ bool attend_tile(const uint8_t* s_q, const uint8_t* s_k, uint8_t* s_p,
+                                            float* s_red, float4* s_swap, const int* s_valid, float scale_log2,
+                                            bool landed, int warp, int lane, float (&m_run)[MT][2],
+                                            float (&l_run)[MT][8 / W][2], float (&acc)[MT][kDV / 8 / W][4]) {
+  constexpr int kRows = MT * kHB, NS = kSlices / W;  // NS slices of eight keys per warp
+  const int g = lane >> 2, t4 = lane & 3, kg = warp & 3, dh = warp >> 2;  // (dh = 0 of four warps)
+  float x[MT][NS][4];
   {
-    const uint32_t a_base = smem_u32(s_q + (lane & 15) * kRowPitch + (lane >> 4) * 16);
-    const uint32_t b_base = smem_u32(s_k + (warp * 16 + (lane & 7) + 8 * (lane >> 4)) * kRowPitch +
-                                     ((lane >> 3) & 1) * 16);
-#pragma unroll 4
-    for (int k0 = 0; k0 < kD; k0 += 16) {
-      uint32_t a[4], b[4];
-      ldsm_x4(a_base + k0 * 2, a);
-      ldsm_x4(b_base + k0 * 2, b);
-      mma_bf16(sc[0], a, b[0], b[1]);
-      mma_bf16(sc[1], a, b[2], b[3]);
+    const uint32_t a_base = smem_u32(s_q + (lane & 15) * kRowPitch + (lane >> 4) * 16) + dh * kD;  // (half a row: kD bytes)
+    const uint32_t b_base = smem_u32(s_k + (kg * 16 + (lane & 7) + 8 * (lane >> 4)) * kRowPitch +
+                                     ((lane >> 3) & 1) * 16) + dh * kD;
+    float sc[NS][MT][2][4];  // [half of the dims][head block][slice]
+#pragma unroll
+    for (int hf = 0; hf < NS; ++hf)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sc[hf][mt][0][e] = sc[hf][mt][1][e] = 0.f;
+#pragma unroll 3
+    for (int k0 = 0; k0 < kD / 2; k0 += 16) {
+#pragma unroll
+      for (int hf = 0; hf < NS; ++hf) {
+        uint32_t b[4];
+        ldsm_x4(b_base + hf * kD + k0 * 2, b);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          uint32_t a[4];
+          ldsm_x4(a_base + hf * kD + mt * kHB * kRowPitch + k0 * 2, a);
+          mma_bf16(sc[hf][mt][0], a, b[0], b[1]);
+          mma_bf16(sc[hf][mt][1], a, b[2], b[3]);
+        }
+      }
+    }
+    if constexpr (W == 8) {  // this warp keeps keys [16 kg + 8 dh, + 8)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        float4 give;
+        give.x = dh ? sc[0][mt][0][0] : sc[0][mt][1][0];
+        give.y = dh ? sc[0][mt][0][1] : sc[0][mt][1][1];
+        give.z = dh ? sc[0][mt][0][2] : sc[0][mt][1][2];
+        give.w = dh ? sc[0][mt][0][3] : sc[0][mt][1][3];
+        s_swap[(warp * MT + mt) * 32 + lane] = give;
+      }
+      pair_sync(kg);
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        const float4 o = s_swap[((warp ^ 4) * MT + mt) * 32 + lane];
+        x[mt][0][0] = (dh ? sc[0][mt][1][0] : sc[0][mt][0][0]) + o.x;
+        x[mt][0][1] = (dh ? sc[0][mt][1][1] : sc[0][mt][0][1]) + o.y;
+        x[mt][0][2] = (dh ? sc[0][mt][1][2] : sc[0][mt][0][2]) + o.z;
+        x[mt][0][3] = (dh ? sc[0][mt][1][3] : sc[0][mt][0][3]) + o.w;
+      }
+    } else {
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int n = 0; n < NS; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[mt][n][e] = sc[0][mt][n][e] + sc[NS - 1][mt][n][e];
     }
   }
-  // scale, mask, tile max per head row (rows g and g + 8)
-  float tmax[2] = {-INFINITY, -INFINITY};
+  // scale, mask, tile max per head row (rows g and g + 8 of a block); slice `dh + n` of the key group
+  const auto column = [&](int n) { return kg * 16 + (dh + n) * 8 + t4 * 2; };
 #pragma unroll
-  for (int nt = 0; nt < 2; ++nt) {
+  for (int n = 0; n < NS; ++n) {
+    const bool v0 = s_valid[column(n)] != 0, v1 = s_valid[column(n) + 1] != 0;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int col = warp * 16 + nt * 8 + t4 * 2 + (e & 1);
-      const float v = s_valid[col] ? sc[nt][e] * scale_log2 : -INFINITY;
-      sc[nt][e] = v;
-      tmax[e >> 1] = fmaxf(tmax[e >> 1], v);
+    for (int mt = 0; mt < MT; ++mt) {
+      x[mt][n][0] = v0 ? x[mt][n][0] * scale_log2 : -INFINITY;
+      x[mt][n][1] = v1 ? x[mt][n][1] * scale_log2 : -INFINITY;
+      x[mt][n][2] = v0 ? x[mt][n][2] * scale_log2 : -INFINITY;
+      x[mt][n][3] = v1 ? x[mt][n][3] * scale_log2 : -INFINITY;
     }
   }
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    tmax[i] = fmaxf(tmax[i], __shfl_xor_sync(0xffffffffu, tmax[i], 1));
-    tmax[i] = fmaxf(tmax[i], __shfl_xor_sync(0xffffffffu, tmax[i], 2));
-  }
-  if (t4 == 0) {
-    s_red[warp * kHB + g] = tmax[0];
-    s_red[warp * kHB + g + 8] = tmax[1];
-  }
-  cta128_sync();
-  float alpha[2], m_new[2], psum[2] = {0.f, 0.f};
+  for (int mt = 0; mt < MT; ++mt) {
+    float tmax[2] = {fmaxf(x[mt][0][0], x[mt][0][1]), fmaxf(x[mt][0][2], x[mt][0][3])};
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int row = g + 8 * i;
-    float m = m_run[i];
-#pragma unroll
-    for (int w = 0; w < 4; ++w) m = fmaxf(m, s_red[w * kHB + row]);
-    m_new[i] = m;
-    alpha[i] = (m == -INFINITY) ? 1.f : exp2f(m_run[i] - m);
-  }
-#pragma unroll
-  for (int nt = 0; nt < 2; ++nt) {
-    float pr[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float m = m_new[e >> 1];
-      pr[e] = (m == -INFINITY) ? 0.f : exp2f(sc[nt][e] - m);
+    for (int n = 1; n < NS; ++n) {
+      tmax[0] = fmaxf(tmax[0], fmaxf(x[mt][n][0], x[mt][n][1]));
+      tmax[1] = fmaxf(tmax[1], fmaxf(x[mt][n][2], x[mt][n][3]));
     }
-    const __nv_bfloat162 p01 = __floats2bfloat162_rn(pr[0], pr[1]);
-    const __nv_bfloat162 p23 = __floats2bfloat162_rn(pr[2], pr[3]);
-    // the row sum uses the rounded probabilities that P.V will see
-    psum[0] += __bfloat162float(p01.x) + __bfloat162float(p01.y);
-    psum[1] += __bfloat162float(p23.x) + __bfloat162float(p23.y);
-    const int col = warp * 16 + nt * 8 + t4 * 2;
-    *reinterpret_cast<__nv_bfloat162*>(s_p + g * kPPitch + col * 2) = p01;
-    *reinterpret_cast<__nv_bfloat162*>(s_p + (g + 8) * kPPitch + col * 2) = p23;
-  }
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    psum[i] += __shfl_xor_sync(0xffffffffu, psum[i], 1);
-    psum[i] += __shfl_xor_sync(0xffffffffu, psum[i], 2);
+    for (int i = 0; i < 2; ++i) {
+      tmax[i] = fmaxf(tmax[i], __shfl_xor_sync(0xffffffffu, tmax[i], 1));
+      tmax[i] = fmaxf(tmax[i], __shfl_xor_sync(0xffffffffu, tmax[i], 2));
+    }
+    if (t4 == 0) {
+      s_red[warp * kRows + mt * kHB + g] = tmax[0];
+      s_red[warp * kRows + mt * kHB + g + 8] = tmax[1];
+    }
   }
-  if (t4 == 0) {
-    s_red[4 * kHB + warp * kHB + g] = psum[0];
-    s_red[4 * kHB + warp * kHB + g + 8] = psum[1];
-  }
-  cta128_sync();
+  if (cta_any<W>(!landed)) return false;
+  float alpha[MT][2];
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int row = g + 8 * i;
-    float s = 0.f;
+  for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
-    for (int w = 0; w < 4; ++w) s += s_red[4 * kHB + w * kHB + row];
-    l_run[i] = l_run[i] * alpha[i] + s;
-    m_run[i] = m_new[i];
-  }
+    for (int i = 0; i < 2; ++i) {
+      const int row = mt * kHB + g + 8 * i;
+      float m = m_run[mt][i];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    acc[i][0] *= alpha[0];
-    acc[i][1] *= alpha[0];
-    acc[i][2] *= alpha[1];
-    acc[i][3] *= alpha[1];
+      for (int w = 0; w < W; ++w) m = fmaxf(m, s_red[w * kRows + row]);
+      alpha[mt][i] = (m == -INFINITY) ? 1.f : exp2f(m_run[mt][i] - m);
+      m_run[mt][i] = m;
+    }
+#pragma unroll
+    for (int n = 0; n < NS; ++n) {
+      float pr[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float m = m_run[mt][e >> 1];
+        pr[e] = (m == -INFINITY) ? 0.f : exp2f(x[mt][n][e] - m);
+      }
+      const __nv_bfloat162 p01 = __floats2bfloat162_rn(pr[0], pr[1]);
+      const __nv_bfloat162 p23 = __floats2bfloat162_rn(pr[2], pr[3]);
+      // the row sum uses the rounded probabilities that P.V will see; each thread keeps the sum of its own keys,
+      // the CTA's are added up once, at the end
+      l_run[mt][n][0] = l_run[mt][n][0] * alpha[mt][0] + (__bfloat162float(p01.x) + __bfloat162float(p01.y));
+      l_run[mt][n][1] = l_run[mt][n][1] * alpha[mt][1] + (__bfloat162float(p23.x) + __bfloat162float(p23.y));
+      *reinterpret_cast<__nv_bfloat162*>(s_p + (mt * kHB + g) * kPPitch + column(n) * 2) = p01;
+      *reinterpret_cast<__nv_bfloat162*>(s_p + (mt * kHB + g + 8) * kPPitch + column(n) * 2) = p23;
+    }
   }
+  cta_sync<W>();
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int i = 0; i < kDV / 8 / W; ++i) {
+      acc[mt][i][0] *= alpha[mt][0];
+      acc[mt][i][1] *= alpha[mt][0];
+      acc[mt][i][2] *= alpha[mt][1];
+      acc[mt][i][3] *= alpha[mt][1];
+    }
 
-  // ---- O += P V: warp w owns value columns [128 w, 128 w + 128)
+  // ---- O += P V: warp w owns value columns [512 / W w, 512 / W (w + 1))
   {
     const uint32_t a_base = smem_u32(s_p + (lane & 15) * kPPitch + (lane >> 4) * 16);
     const uint32_t b_base = smem_u32(s_k + ((lane & 7) + 8 * ((lane >> 3) & 1)) * kRowPitch +
-                                     (warp * 128 + 8 * (lane >> 4)) * 2);
+                                     (warp * (kDV / W) + 8 * (lane >> 4)) * 2);
 #pragma unroll
     for (int ks = 0; ks < kBN / 16; ++ks) {
-      uint32_t a[4];
-      ldsm_x4(a_base + ks * 32, a);
+      uint32_t a[MT][4];
 #pragma unroll
-      for (int np = 0; np < 8; ++np) {
+      for (int mt = 0; mt < MT; ++mt) ldsm_x4(a_base + mt * kHB * kPPitch + ks * 32, a[mt]);
+#pragma unroll
+      for (int np = 0; np < kDV / 16 / W; ++np) {
         uint32_t b[4];
         ldsm_x4_t(b_base + ks * 16 * kRowPitch + np * 32, b);
-        mma_bf16(acc[2 * np], a, b[0], b[1]);
-        mma_bf16(acc[2 * np + 1], a, b[2], b[3]);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          mma_bf16(acc[mt][2 * np], a[mt], b[0], b[1]);
+          mma_bf16(acc[mt][2 * np + 1], a[mt], b[2], b[3]);
+        }
       }
     }
   }
+  return true;
 }
 
-// Dequantises a staged fp8 tile (656-B rows) into the bf16 K tile. Work item =
-// one 16-byte chunk of a row: 32 chunks of 16 e4m3 (-> 32 B of bf16) and 8 chunks
-// of rope that are copied. Items are independent and the loop is unrolled, so
-// each thread keeps several shared-memory loads in flight (the tile is
-// latency-bound with four warps per CTA). With zero_invalid the masked rows are
-// cleared here (they must be finite: 0 * NaN would poison P.V); otherwise the
-// caller has cleared them already.
-__device__ __forceinline__ void dequant_tile(const uint8_t* s_stage, uint8_t* s_k, const int* s_valid, int tid,
-                                             bool zero_invalid = false) {
-  constexpr int kChunks = 40;  // per row
-#pragma unroll 4
-  for (int i = tid; i < kBN * kChunks; i += kThreads) {
-    const int row = i / kChunks, c = i - row * kChunks;
-    const uint8_t* src = s_stage + row * kFp8Row;
-    uint8_t* dst = s_k + row * kRowPitch;
-    const bool ok = s_valid[row] != 0;
-    if (!ok && !zero_invalid) continue;
-    if (c < 32) {
-      uint4 lo = make_uint4(0, 0, 0, 0), hi = make_uint4(0, 0, 0, 0);
-      if (ok) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(src + c * 16);
-        const float sc = *reinterpret_cast<const float*>(src + 512 + (c >> 3) * 4);
-        const uint2 d0 = dequant4(raw.x, sc), d1 = dequant4(raw.y, sc);
-        const uint2 d2 = dequant4(raw.z, sc), d3 = dequant4(raw.w, sc);
-        lo = make_uint4(d0.x, d0.y, d1.x, d1.y);
-        hi = make_uint4(d2.x, d2.y, d3.x, d3.y);
+// Every thread's sums of its own keys, the four lanes of a head row added up, where sum_of can read them
+// behind a block barrier.
+template <int MT, int W>
+__device__ __forceinline__ void post_sums(float* s_red, int warp, int lane, const float (&l_run)[MT][8 / W][2]) {
+  float* s_sum = s_red + kSlices * MT * kHB;
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int n = 0; n < kSlices / W; ++n)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        float s = l_run[mt][n][i];
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        if ((lane & 3) == 0) s_sum[(warp + 4 * n) * MT * kHB + mt * kHB + (lane >> 2) + 8 * i] = s;
       }
-      *reinterpret_cast<uint4*>(dst + c * 32) = lo;
-      *reinterpret_cast<uint4*>(dst + c * 32 + 16) = hi;
-    } else {
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (ok) v = *reinterpret_cast<const uint4*>(src + 528 + (c - 32) * 16);
-      *reinterpret_cast<uint4*>(dst + 1024 + (c - 32) * 16) = v;
-    }
-  }
+}
+template <int MT>
+__device__ __forceinline__ float sum_of(const float* s_red, int row) {
+  float s = 0.f;
+#pragma unroll
+  for (int w = 0; w < kSlices; ++w) s += s_red[(kSlices + w) * MT * kHB + row];
+  return s;
 }
 
-// In-place variant for the split-K kernel: the 656 staged bytes of a row sit at
+// Dequantises a staged fp8 tile in place: the 656 staged bytes of a row sit at
 // the END of that row's 1152-byte bf16 slot (offset 496), so no separate staging
 // buffer is needed and the fp8 path keeps two CTAs per SM. Expanding a chunk
 // overwrites bytes other threads may still have to read, so the tile is done in
@@ -280,9 +329,9 @@ __device__ __forceinline__ void dequant_tile(const uint8_t* s_stage, uint8_t* s_
 //   chunks 24..31 + rope read [880,1152) write [768,1152)
 // The four group scales sit at [1008,1024) and are read before the last stores.
 constexpr int kFp8StageOff = kRowBytes - kFp8Row;  // 496
-template <int FIRST, int NDEQ, int NROPE>
+template <int FIRST, int NDEQ, int NROPE, int W>
 __device__ __forceinline__ void dequant_pass(uint8_t* s_k, const int* s_valid, int tid) {
-  constexpr int kPerRow = NDEQ + NROPE;
+  constexpr int kPerRow = NDEQ + NROPE, kThreads = 32 * W;
   constexpr int kPer = (kBN * kPerRow) / kThreads;
   static_assert((kBN * kPerRow) % kThreads == 0, "items must divide evenly");
   uint4 raw[kPer];
@@ -302,7 +351,7 @@ __device__ __forceinline__ void dequant_pass(uint8_t* s_k, const int* s_valid, i
       }
     }
   }
-  cta128_sync();
+  cta_sync<W>();
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int i = tid + u * kThreads, row = i / kPerRow, k = i - row * kPerRow;
@@ -319,42 +368,49 @@ __device__ __forceinline__ void dequant_pass(uint8_t* s_k, const int* s_valid, i
     }
   }
 }
+template <int W>
 __device__ __forceinline__ void dequant_tile_inplace(uint8_t* s_k, const int* s_valid, int tid) {
-  dequant_pass<0, 16, 0>(s_k, s_valid, tid);
-  dequant_pass<16, 8, 0>(s_k, s_valid, tid);
-  dequant_pass<24, 8, 8>(s_k, s_valid, tid);
+  dequant_pass<0, 16, 0, W>(s_k, s_valid, tid);
+  dequant_pass<16, 8, 0, W>(s_k, s_valid, tid);
+  dequant_pass<24, 8, 8, W>(s_k, s_valid, tid);
 }
 
 // Body of the split-K partials for CTA (split, hg, r); `smem` is the CTA's
-// dynamic shared memory. Threads 0..127 take part.
+// dynamic shared memory. Threads 0..32 W - 1 take part.
 // kBeside: the launch does not depend on the kernel enqueued just before it (under the lagged
 // schedule the attention reads the PREVIOUS layer's selection while this layer's top-k runs), so
 // it releases its own dependents and starts at once, beside that kernel, and waits for it only
 // before it exits: it still completes after it, and the next kernel's wait covers both.
-template <bool kBeside = false, bool kDirect = false>
+// kDirect: the split is the only one and writes the result itself.
+// MT: blocks of 16 heads per CTA; hg counts blocks of 16 MT heads.
+template <bool kBeside, bool kDirect, int MT, int W>
 __device__ __forceinline__ void mla_partials_body(const Params& p, const int split, const int hg, const int r,
                                                   uint8_t* smem) {
-  uint8_t* s_q = smem + SmemLayout::q_off;
-  uint8_t* s_k = smem + SmemLayout::k_off;
-  uint8_t* s_p = smem + SmemLayout::p_off;
-  float* s_red = reinterpret_cast<float*>(smem + SmemLayout::red_off);
-  int* s_valid = reinterpret_cast<int*>(smem + SmemLayout::valid_off);
-  uint64_t* s_bar = reinterpret_cast<uint64_t*>(smem + SmemLayout::bar_off);
+  constexpr int NB = MT;  // (one block: two CTAs share an SM and cover each other's gathers)
+  constexpr int kRowsPerWarp = kBN / W;  // latent rows of a tile that a warp requests
+  using L = SmemLayout<MT, NB>;
+  constexpr int kHeads = MT * kHB;
+  uint8_t* s_q = smem + L::q_off;
+  uint8_t* s_k = smem + L::k_off;
+  uint8_t* s_p = smem + L::p_off;
+  float* s_red = reinterpret_cast<float*>(smem + L::red_off);
+  float4* s_swap = reinterpret_cast<float4*>(smem + L::swap_off);
+  int* s_valid = reinterpret_cast<int*>(smem + L::valid_off);
+  const uint32_t bar_q = smem_u32(smem + L::bar_off);
+  const auto bar_k = [&](int buf, int half) { return bar_q + 8u * uint32_t(1 + 2 * buf + half); };  // rows 0..31, 32..63 of a tile
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   DSA_KTIME_BEGIN(2);
   const int seq = r / p.rows_per_seq;
-  const uint32_t bar_q = smem_u32(&s_bar[0]);
-  const uint32_t bar_k = smem_u32(&s_bar[1]);
   const int row_bytes = p.kv_fp8 ? kFp8Row : kRowBytes;
   const uint8_t* kv_seq = p.kv + int64_t(seq) * p.kv_seq_stride * row_bytes;
 
   if (tid == 0) {
-    mbar_init(bar_q, kHB);
-    mbar_init(bar_k, kBN);
+    mbar_init(bar_q, W);
+    for (int i = 0; i < 2 * NB; ++i) mbar_init(bar_k(i >> 1, i & 1), W / 2);
     mbar_fence_init();
   }
-  cta128_sync();
+  cta_sync<W>();
   if constexpr (!kBeside) pdl_wait();  // the selection, the queries and the lengths may come from the previous kernel
   pdl_launch_dependents();
   // The first tile's selection entries are requested before the row's length is looked at: two
@@ -362,145 +418,181 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
   const int k_begin = split * p.keys_per_split;
   const int k_end = min(k_begin + p.keys_per_split, p.topk);
   const int n_tiles = (max(k_end - k_begin, 0) + kBN - 1) / kBN;
-  int64_t idx_first = -1;
-  if (tid < kBN && k_begin + tid < k_end)
-    idx_first = p.indices ? int64_t(p.indices[int64_t(r) * p.topk + k_begin + tid]) : int64_t(k_begin + tid);
+  const int my_row = warp * kRowsPerWarp + lane;  // (lanes 0..7)
+  const auto entry = [&](int tile) {
+    const int j = k_begin + tile * kBN + my_row;
+    if (lane >= kRowsPerWarp || j >= k_end) return -1;
+    return p.indices ? int(p.indices[int64_t(r) * p.topk + j]) : j;
+  };
+  int idx_next = entry(0);
   int64_t len = p.seq_lens ? int64_t(p.seq_lens[r]) : p.ctx;
   len = len < 0 ? 0 : (len > p.ctx ? p.ctx : len);
 
-  // queries of this head block: 16 rows of 1152 B
-  if (tid >= kBN && tid < kBN + kHB) {
-    const int h = tid - kBN;
-    const __nv_bfloat16* src = p.q + (int64_t(r) * p.H + hg * kHB + h) * kD;
-    mbar_arrive_expect_tx(bar_q, kRowBytes);
-    bulk_g2s(smem_u32(s_q + h * kRowPitch), src, kRowBytes, bar_q);
+  // Gather up to 64 latent rows: one bulk copy per valid row, shared out over all warps. (A warp issues its lanes'
+  // copies one after the other, 60 cycles each: from two warps the 64 took 1900 cycles whether one CTA or two shared the SM.
+  // 16-byte asynchronous copies by all threads instead were slower still: 4608 of them per tile.)
+  const auto gather = [&](int tile) {
+    const int buf = NB == 1 ? 0 : tile & 1;
+    const int idx = idx_next;
+    const bool ok = idx >= 0 && idx < len;
+    const uint32_t seen = __ballot_sync(0xffffffffu, ok);
+    const uint32_t bar = bar_k(buf, warp / (W / 2));
+    uint8_t* dst = s_k + (buf * kBN + my_row) * kRowPitch;
+    if (lane < kRowsPerWarp) {
+      s_valid[buf * kBN + my_row] = ok;
+      if (!ok) {
+        // masked key: its row must be finite because 0 * NaN would poison P.V
+        uint4* z = reinterpret_cast<uint4*>(dst);
+        for (int i = 0; i < kRowBytes / 16; ++i) z[i] = make_uint4(0, 0, 0, 0);
+      }
+      fence_proxy_async_smem();  // earlier generic reads of these rows precede the async writes
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive_expect_tx(bar, uint32_t(__popc(seen)) * uint32_t(row_bytes));
+    __syncwarp();
+    if (ok) {
+      if (p.kv_fp8)  // staged at the end of the row's own slot, expanded in place below
+        bulk_g2s(smem_u32(dst + kFp8StageOff), kv_seq + int64_t(idx) * kFp8Row, kFp8Row, bar);
+      else
+        bulk_g2s(smem_u32(dst), kv_seq + int64_t(idx) * kRowBytes, kRowBytes, bar);
+    }
+    idx_next = entry(tile + 1);
+  };
+  if (n_tiles > 0) gather(0);
+  // queries of the head blocks: rows of 1152 B
+  {
+    constexpr int kPerWarp = kHeads / W;
+    if (lane == 0) mbar_arrive_expect_tx(bar_q, kPerWarp * kRowBytes);
+    __syncwarp();
+    if (lane < kPerWarp) {
+      const int h = warp * kPerWarp + lane;
+      bulk_g2s(smem_u32(s_q + h * kRowPitch), p.q + (int64_t(r) * p.H + hg * kHeads + h) * kD, kRowBytes, bar_q);
+    }
   }
 
   const int g = lane >> 2, t4 = lane & 3;
-  float m_run[2] = {-INFINITY, -INFINITY};
-  float l_run[2] = {0.f, 0.f};
-  float acc[16][4];
+  float m_run[MT][2], l_run[MT][kSlices / W][2];
+  float acc[MT][kDV / 8 / W][4];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+  for (int mt = 0; mt < MT; ++mt) {
+    m_run[mt][0] = m_run[mt][1] = -INFINITY;
+#pragma unroll
+    for (int n = 0; n < kSlices / W; ++n) l_run[mt][n][0] = l_run[mt][n][1] = 0.f;
+#pragma unroll
+    for (int i = 0; i < kDV / 8 / W; ++i) acc[mt][i][0] = acc[mt][i][1] = acc[mt][i][2] = acc[mt][i][3] = 0.f;
+  }
   bool timed_out = false;
 
   for (int tile = 0; tile < n_tiles; ++tile) {
-    // ---- gather up to 64 latent rows: one bulk copy per valid row. (The copy engine accepts about
-    // one such copy per 30 cycles, ~1900 cycles for the tile; 16-byte asynchronous copies by all
-    // 128 threads instead were slower still: 4608 of them per tile wait on one another's returns.)
-    if (tid < kBN) {
-      const int j = k_begin + tile * kBN + tid;
-      int64_t idx = idx_first;
-      if (tile > 0) {
-        idx = -1;
-        if (j < k_end) idx = p.indices ? int64_t(p.indices[int64_t(r) * p.topk + j]) : int64_t(j);
-      }
-      const bool ok = idx >= 0 && idx < len;
-      s_valid[tid] = ok;
-      uint8_t* dst_row = s_k + tid * kRowPitch;
-      if (ok) {
-        fence_proxy_async_smem();  // earlier generic reads of this row precede the async write
-        mbar_arrive_expect_tx(bar_k, row_bytes);
-        if (p.kv_fp8)  // staged at the end of the row's own slot, expanded in place below
-          bulk_g2s(smem_u32(dst_row + kFp8StageOff), kv_seq + idx * kFp8Row, kFp8Row, bar_k);
-        else
-          bulk_g2s(smem_u32(dst_row), kv_seq + idx * kRowBytes, kRowBytes, bar_k);
-      } else {
-        // masked key: its row must be finite because 0 * NaN would poison P.V
-        uint4* z = reinterpret_cast<uint4*>(dst_row);
-        for (int i = 0; i < kRowBytes / 16; ++i) z[i] = make_uint4(0, 0, 0, 0);
-        mbar_arrive(bar_k);
-      }
-    }
-    if (tile == 0 && !mbar_wait(bar_q, 0)) timed_out = true;
-    if (!mbar_wait(bar_k, tile & 1)) timed_out = true;
-    // Each thread ran its own clock: the 128 threads agree on leaving here, so nobody is left
-    // alone at the barriers below.
-    timed_out = cta128_any(timed_out);
-    if (timed_out) break;
+    const int buf = NB == 1 ? 0 : tile & 1, parity = (NB == 1 ? tile : tile >> 1) & 1;
+    if (NB > 1 && tile + 1 < n_tiles) gather(tile + 1);  // (its slot was read before the last barrier)
+    uint8_t* tile_k = s_k + buf * kBN * kRowPitch;
+    const int* valid = s_valid + buf * kBN;
+    // A warp waits for the half of the tile that its key group lies in; each thread runs its own clock, so the
+    // threads agree on leaving at the softmax's barrier (fp8 rows: here) and nobody is left alone at a later one.
+    bool landed = tile > 0 || mbar_wait(bar_q, 0);
+    if (!mbar_wait(bar_k(buf, (warp >> 1) & 1), parity)) landed = false;
     if (p.kv_fp8) {
-      dequant_tile_inplace(s_k, s_valid, tid);
-      cta128_sync();
+      if (!mbar_wait(bar_k(buf, ((warp >> 1) & 1) ^ 1), parity)) landed = false;
+      timed_out = cta_any<W>(!landed);
+      if (timed_out) break;
+      dequant_tile_inplace<W>(tile_k, valid, tid);
+      cta_sync<W>();
     }
-
-    attend_tile(s_q, s_k, s_p, s_red, s_valid, p.scale_log2, warp, lane, m_run, l_run, acc);
-    cta128_sync();  // the K tile and P are free for the next gather
+    timed_out = !attend_tile<MT, W>(s_q, tile_k, s_p, s_red, s_swap, valid, p.scale_log2, landed, warp, lane, m_run, l_run, acc);
+    if (timed_out) break;
+    if (tile + 1 < n_tiles) {
+      cta_sync<W>();  // the K tile and P are free for the next gather
+      if (NB == 1) gather(tile + 1);
+    }
   }
 
-  if (n_tiles == 0) timed_out = cta128_any(!mbar_wait(bar_q, 0));  // never leave with a copy in flight
+  if (n_tiles == 0) timed_out = cta_any<W>(!mbar_wait(bar_q, 0));  // never leave with a copy in flight
   if (timed_out) {
     atomicOr(&g_device_status, kStatusAttnTimeout);
-    m_run[0] = m_run[1] = -INFINITY;
-    l_run[0] = l_run[1] = 0.f;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      m_run[mt][0] = m_run[mt][1] = -INFINITY;
+#pragma unroll
+      for (int n = 0; n < kSlices / W; ++n) l_run[mt][n][0] = l_run[mt][n][1] = 0.f;
+    }
     drain_after_timeout();  // let outstanding copies land
   }
+  post_sums<MT, W>(s_red, warp, lane, l_run);
 
   if constexpr (kDirect) {  // the only split: what the merge kernel would make of its partials
-    __nv_bfloat16* out = p.out + (int64_t(r) * p.H + hg * kHB) * kDV;
-    const float inv0 = l_run[0] > 0.f ? 1.f / l_run[0] : 0.f, inv1 = l_run[1] > 0.f ? 1.f / l_run[1] : 0.f;
+    cta_sync<W>();
+    __nv_bfloat16* out = p.out + (int64_t(r) * p.H + hg * kHeads) * kDV;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int col = warp * 128 + i * 8 + t4 * 2;
-      *reinterpret_cast<__nv_bfloat162*>(out + g * kDV + col) = __floats2bfloat162_rn(acc[i][0] * inv0, acc[i][1] * inv0);
-      *reinterpret_cast<__nv_bfloat162*>(out + (g + 8) * kDV + col) = __floats2bfloat162_rn(acc[i][2] * inv1, acc[i][3] * inv1);
+    for (int mt = 0; mt < MT; ++mt) {
+      const float l0 = sum_of<MT>(s_red, mt * kHB + g), l1 = sum_of<MT>(s_red, mt * kHB + g + 8);
+      const float inv0 = l0 > 0.f ? 1.f / l0 : 0.f, inv1 = l1 > 0.f ? 1.f / l1 : 0.f;
+#pragma unroll
+      for (int i = 0; i < kDV / 8 / W; ++i) {
+        __nv_bfloat16* dst = out + (mt * kHB + g) * kDV + warp * (kDV / W) + i * 8 + t4 * 2;
+        *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(acc[mt][i][0] * inv0, acc[mt][i][1] * inv0);
+        *reinterpret_cast<__nv_bfloat162*>(dst + 8 * kDV) = __floats2bfloat162_rn(acc[mt][i][2] * inv1, acc[mt][i][3] * inv1);
+      }
     }
     if constexpr (kBeside) pdl_wait();
     DSA_KTIME_END(2);
     return;
   }
-  // ---- partials of this split: unnormalised accumulator, running max (base 2), sum
-  const int64_t pbase = (int64_t(r) * p.nsplit + split) * p.H + hg * kHB;
+  // ---- partials of this split: unnormalised accumulator, running max (base 2), sum. An SM writes about 28 bytes a
+  // cycle, so the 32 MT KB take 1200 MT cycles; the sums' barrier waits in their shadow.
+  const int64_t pbase = (int64_t(r) * p.nsplit + split) * p.H + hg * kHeads;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const int col = warp * 128 + i * 8 + t4 * 2;
-    *reinterpret_cast<float2*>(p.part_acc + (pbase + g) * kDV + col) = make_float2(acc[i][0], acc[i][1]);
-    *reinterpret_cast<float2*>(p.part_acc + (pbase + g + 8) * kDV + col) = make_float2(acc[i][2], acc[i][3]);
+  for (int mt = 0; mt < MT; ++mt) {
+    float* dst = p.part_acc + (pbase + mt * kHB + g) * kDV + warp * (kDV / W) + t4 * 2;
+#pragma unroll
+    for (int i = 0; i < kDV / 8 / W; ++i) {
+      *reinterpret_cast<float2*>(dst + i * 8) = make_float2(acc[mt][i][0], acc[mt][i][1]);
+      *reinterpret_cast<float2*>(dst + 8 * kDV + i * 8) = make_float2(acc[mt][i][2], acc[mt][i][3]);
+    }
+    if (warp == 0 && t4 == 0) {
+      p.part_m[pbase + mt * kHB + g] = m_run[mt][0];
+      p.part_m[pbase + mt * kHB + g + 8] = m_run[mt][1];
+    }
   }
-  if (warp == 0 && t4 == 0) {
-    p.part_m[pbase + g] = m_run[0];
-    p.part_m[pbase + g + 8] = m_run[1];
-    p.part_l[pbase + g] = l_run[0];
-    p.part_l[pbase + g + 8] = l_run[1];
-  }
+  cta_sync<W>();
+  if (tid < kHeads) p.part_l[pbase + tid] = sum_of<MT>(s_red, tid);
   if constexpr (kBeside) pdl_wait();
   DSA_KTIME_END(2);
 }
 
-template <bool kDirect>
-__global__ void __launch_bounds__(kThreads)
-sparse_mla_partials_kernel(const Params p) {  // kDirect is an instantiation of its own: its code costs a step 0.1 us
+// (instantiations of their own: the direct form's code costs a step 0.1 us)
+// (registers: what leaves room for the merge kernel's CTAs, which wait beside this kernel's)
+template <bool kBeside, bool kDirect, int MT, int W>
+__global__ void __launch_bounds__(32 * W, MT == 1 ? 3 : kDirect ? 1 : 2)
+sparse_mla_partials_kernel(const Params p) {
   extern __shared__ __align__(16) uint8_t mla_smem[];
-  mla_partials_body<false, kDirect>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
-}
-
-template <bool kDirect>
-__global__ void __launch_bounds__(kThreads)
-sparse_mla_partials_beside_kernel(const Params p) {
-  extern __shared__ __align__(16) uint8_t mla_smem[];
-  mla_partials_body<true, kDirect>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
+  mla_partials_body<kBeside, kDirect, MT, W>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
 }
 
 // ------------------------------------------------------------------------------
 // out = sum_s acc_s 2^(m_s - m) / sum_s l_s 2^(m_s - m); splits with m = -inf
 // (no visible key) are skipped, a row with none yields zeros. One CTA per (row,
-// head) of 1..4 groups of 128 threads (the launch picks min(nsplit, 4)): group g
-// folds splits g, g + ngrp, ... with all loads of a chunk of eight splits in
-// flight at once, then group 0 merges the group results in a fixed order.
-constexpr int kCombineThreads = 512;
-__global__ void __launch_bounds__(kCombineThreads)
+// head, 1 / kParts of the columns) of 1..4 groups of 128 / kParts threads (the launch picks min(nsplit, 4)):
+// group g folds splits g, g + ngrp, ... with all loads of a chunk of eight splits in
+// flight at once, then the groups' results are merged in a fixed order, the same for every kParts.
+// Bound by two dependent trips to L2 and by the 61 bytes a cycle that an SM gets from there.
+template <int kParts>
+__global__ void __launch_bounds__(512 / kParts)
 sparse_mla_combine_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_m,
                           const float* __restrict__ part_l, __nv_bfloat16* __restrict__ out, int H,
                           int nsplit) {
+  constexpr int kCols = kDV / kParts, kGroup = kCols / 4;  // columns of a CTA; threads of a group, four columns each
   __shared__ float s_m[4], s_l[4];
-  __shared__ __align__(16) float s_o[4][kDV];
-  const int h = blockIdx.x, r = blockIdx.y, tid = threadIdx.x & 127, grp = threadIdx.x >> 7;
-  const int ngrp = blockDim.x >> 7;  // 1..4 load groups of 128 threads, each taking every ngrp-th split
+  __shared__ __align__(16) float s_o[4][kCols];
+  const int h = blockIdx.x / kParts, c0 = (blockIdx.x % kParts) * kCols, r = blockIdx.y;
+  const int tid = threadIdx.x % kGroup, grp = threadIdx.x / kGroup;
+  const int ngrp = blockDim.x / kGroup;  // 1..4, each taking every ngrp-th split
   DSA_KTIME_BEGIN(3);
   pdl_wait();
   pdl_launch_dependents();
   const float* pm = part_m + int64_t(r) * nsplit * H + h;
   const float* pl = part_l + int64_t(r) * nsplit * H + h;
-  const float* pa = part_acc + (int64_t(r) * nsplit * H + h) * kDV + tid * 4;
+  const float* pa = part_acc + (int64_t(r) * nsplit * H + h) * kDV + c0 + tid * 4;
   float mg = -INFINITY, lg = 0.f;
   float4 og = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int s0 = grp; s0 < nsplit; s0 += 8 * ngrp) {
@@ -544,11 +636,14 @@ sparse_mla_combine_kernel(const float* __restrict__ part_acc, const float* __res
   __syncthreads();
   if (grp == 0) {
     float m = s_m[0];
-    for (int gi = 1; gi < ngrp; ++gi) m = fmaxf(m, s_m[gi]);
+#pragma unroll
+    for (int gi = 1; gi < 4; ++gi) m = gi < ngrp ? fmaxf(m, s_m[gi]) : m;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     float l = 0.f;
     if (m != -INFINITY) {
-      for (int gi = 0; gi < ngrp; ++gi) {
+#pragma unroll
+      for (int gi = 0; gi < 4; ++gi) {
+        if (gi >= ngrp) break;
         const float e = (s_m[gi] == -INFINITY) ? 0.f : exp2f(s_m[gi] - m);
         const float4 a = *reinterpret_cast<const float4*>(&s_o[gi][tid * 4]);
         l = fmaf(s_l[gi], e, l);
@@ -564,7 +659,7 @@ sparse_mla_combine_kernel(const float* __restrict__ part_acc, const float* __res
     uint2 pk;
     pk.x = *reinterpret_cast<uint32_t*>(&lo);
     pk.y = *reinterpret_cast<uint32_t*>(&hi);
-    *reinterpret_cast<uint2*>(out + (int64_t(r) * H + h) * kDV + tid * 4) = pk;
+    *reinterpret_cast<uint2*>(out + (int64_t(r) * H + h) * kDV + c0 + tid * 4) = pk;
   }
   DSA_KTIME_END(3);
 }
