@@ -278,7 +278,7 @@ int dsa_topk_select_static(const float* logits, const int32_t* seq_lens, int32_t
  * Two kernels serve the partials. Launches with H a multiple of 64 and at least
  * 128 tiles of 64 heads x 64 keys (R * H/64 * ceil(topk/64)) run on tcgen05 /
  * tensor memory with 64 heads per CTA; smaller launches and other head counts
- * run on mma.sync with 16 heads per CTA. Both write the same part_* layout;
+ * run on mma.sync with 16 or 32 heads per CTA. Both write the same part_* layout;
  * part_m is a base-2 softmax reference of the split (not necessarily its
  * maximum) consistent with part_l and part_acc, which is all
  * dsa_sparse_mla_combine needs. (bf16 partial accumulators were measured: the
@@ -305,9 +305,9 @@ int dsa_sparse_mla_decode(const void* q, const void* kv, const int32_t* indices,
  * enqueued before the call). The partials kernel releases its dependents and starts at once, and
  * waits for the kernel before it only before it exits: it completes after that kernel, and whatever
  * is enqueued next sees both. The whole lagged layer then stays one chain of programmatic
- * dependents on one stream (scan -> top-k -> this) instead of two streams and a join. Launches
- * that the tcgen05 kernel serves run as dsa_sparse_mla_decode does. The kernel before it must be
- * one of this library's; behind any other work the call behaves like dsa_sparse_mla_decode. */
+ * dependents on one stream (scan -> top-k -> this) instead of two streams and a join. Both
+ * kernels have this form. The kernel before it must be one of this library's; behind any
+ * other work the call behaves like dsa_sparse_mla_decode. */
 int dsa_sparse_mla_decode_beside(const void* q, const void* kv, const int32_t* indices,
                                  const int32_t* seq_lens, float* part_acc, float* part_m,
                                  float* part_l, void* out, int R, int rows_per_seq, int H, int topk,
