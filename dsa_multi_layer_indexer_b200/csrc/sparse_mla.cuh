@@ -66,11 +66,14 @@ struct SmemLayout {
   static constexpr int p_off = k_off + NB * kBN * kRowPitch;
   static constexpr int red_off = p_off + MT * kHB * kPPitch;             // float [2][8][16 MT]
   static constexpr int swap_off = red_off + 2 * kSlices * MT * kHB * 4;  // float4 [8][MT][32]
-  static constexpr int valid_off = swap_off + kSlices * MT * 32 * 16;    // int [NB][64]
+  static constexpr int valid_off = swap_off + (MT == 1 ? 0 : kSlices * MT * 32 * 16);  // int [NB][64] (four warps swap nothing)
   static constexpr int bar_off = valid_off + NB * kBN * 4;               // 1 + 2 NB mbarriers
   static constexpr int bytes = (bar_off + 8 * (1 + 2 * NB) + 15) & ~15;
 };
-static_assert(SmemLayout<1, 1>::bytes * 2 <= 231424, "sparse MLA: two CTAs of one head block share an SM");
+// Two CTAs of one head block (and 1 KB of the system's each) fit the 196 KB configuration that the scan and the top-k run
+// in. An SM is drained before its configuration changes: at 101 KB a CTA, which takes the 228 KB one, a layer of 128 heads
+// and 512 keys took 19.1 us instead of 17.2, its two-stream form 12.9 instead of 10.3.
+static_assert(2 * (SmemLayout<1, 1>::bytes + 1024) <= 196 * 1024, "sparse MLA: two CTAs of one head block share an SM");
 static_assert(SmemLayout<2, 2>::bytes <= 232448, "sparse MLA: shared memory over the per-CTA limit");
 
 // Barrier over the attention CTA's W warps (named barrier 1: in the fused launch others may have left).
