@@ -978,9 +978,8 @@ static int launch_combine(const float* part_acc, const float* part_m, const floa
 }
 }  // extern "C++"
 
-// `layer`: the attention of a decode layer's chain, behind whose merge the value projection already waits
-static int mla_combine(const float* part_acc, const float* part_m, const float* part_l, void* out, int R, int H, int nsplit,
-                       bool layer, void* stream) {
+int dsa_sparse_mla_combine(const float* part_acc, const float* part_m, const float* part_l,
+                           void* out, int R, int H, int nsplit, void* stream) {
   DSA_REQUIRE(part_acc && part_m && part_l && out, "sparse MLA combine: null pointer");
   DSA_REQUIRE(aligned16(part_acc) && aligned16(out), "sparse MLA combine: misaligned pointer");
   DSA_REQUIRE(R > 0 && R <= 65535 && H > 0 && nsplit > 0, "sparse MLA combine: bad geometry");
@@ -993,19 +992,16 @@ static int mla_combine(const float* part_acc, const float* part_m, const float* 
                         part_l, static_cast<__nv_bfloat16*>(out), H, nsplit));
     return DSA_OK;
   }
-  // few (row, head) pairs: their columns over four or two CTAs (attention + merge inside a step: 16 pairs x 32 splits
-  // 7.5 -> 6.6 us, 64 pairs 8.1 -> 7.9). With as many CTAs as SMs the extra ones wait for room (128 pairs 2.9 -> 3.9 us),
-  // and two a pair take that of the value projection in a layer's chain (two layers of the glm5 preset 333 -> 336 us).
+  // few (row, head) pairs: their columns over four or two CTAs (layers of the hot path in a row, one / this many CTAs a pair:
+  // 16 pairs 15.4 / 14.7 us, 32 pairs 19.5 / 18.8, 48 pairs 19.6 / 18.4; whole layers of the glm5 preset with 16 and 32
+  // heads 129.7 / 128.9 and 142.2 / 141.7). Not where two a pair would fill most SMs, since the launch behind the merge
+  // then finds no room (64 pairs: hot path 21.7 / 22.05, whole layers 160.7 / 162.2), nor with more CTAs than SMs (128
+  // pairs: the merge 2.9 / 3.9).
   const int64_t pairs = int64_t(R) * H;
   if (4 * pairs <= sm_count()) return launch_combine<4>(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
-  if (2 * pairs <= sm_count() && !layer)
+  if (3 * pairs <= sm_count())
     return launch_combine<2>(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
   return launch_combine<1>(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
-}
-
-int dsa_sparse_mla_combine(const float* part_acc, const float* part_m, const float* part_l,
-                           void* out, int R, int H, int nsplit, void* stream) {
-  return mla_combine(part_acc, part_m, part_l, out, R, H, nsplit, false, stream);
 }
 
 int dsa_sparse_mla_decode(const void* q, const void* kv, const int32_t* indices,
@@ -1029,7 +1025,7 @@ int dsa_sparse_mla_decode_beside(const void* q, const void* kv, const int32_t* i
   int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, direct ? out : nullptr, R,
                                rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8, true, stream);
   if (rc || direct) return rc;
-  return mla_combine(part_acc, part_m, part_l, out, R, H, nsplit, true, stream);
+  return dsa_sparse_mla_combine(part_acc, part_m, part_l, out, R, H, nsplit, stream);
 }
 
 // ------------------------------------------------------------------ decode-step preparation
