@@ -428,8 +428,9 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
     return p.indices ? int(p.indices[int64_t(r) * p.topk + j]) : j;
   };
   int idx_next = entry(0);
-  int64_t len = p.seq_lens ? int64_t(p.seq_lens[r]) : p.ctx;
-  len = len < 0 ? 0 : (len > p.ctx ? p.ctx : len);
+  // (32 bits, as the entries have: with 64 the 32-head form spilled 28 bytes and the one that shares a launch with the scan 4)
+  const int ctx = int(min(p.ctx, int64_t(0x7FFFFFFF)));
+  const int len = p.seq_lens ? min(max(p.seq_lens[r], 0), ctx) : ctx;
 
   // Gather up to 64 latent rows: one bulk copy per valid row, shared out over all warps. (A warp issues its lanes'
   // copies one after the other, 60 cycles each: from two warps the 64 took 1900 cycles whether one CTA or two shared the SM.
