@@ -95,13 +95,16 @@ int encode_tensor_map(CUtensorMap* map, CUtensorMapDataType dtype, int rank, con
   return DSA_OK;
 }
 
-// Raises a kernel's dynamic shared-memory limit, once per device.
+// Raises a kernel's dynamic shared-memory limit, once per device. `carveout`: the share of an SM's 228 KB, in percent,
+// that it prefers to run with where its own need would have the driver choose less.
 template <typename K>
-static int opt_in_smem(K kernel, size_t bytes, bool (&done)[64]) {
+static int opt_in_smem(K kernel, size_t bytes, bool (&done)[64], int carveout = cudaSharedmemCarveoutDefault) {
   int dev = 0;
   DSA_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && done[dev]) return DSA_OK;
   DSA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  if (carveout != cudaSharedmemCarveoutDefault)
+    DSA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, carveout));
   if (dev >= 0 && dev < 64) done[dev] = true;
   return DSA_OK;
 }
@@ -910,20 +913,23 @@ static int mla_prepare(const void* q, const void* kv, const int32_t* indices, co
 }
 
 extern "C++" {
-template <bool kBeside, bool kDirect, int MT, int W>
+template <bool kBeside, bool kDirect, int MT, int W, int NB>
 static int launch_mla_partials_as(const mla::Params& p, int R, int nsplit, cudaStream_t st) {
   static bool done[64];
-  auto kernel = mla::sparse_mla_partials_kernel<kBeside, kDirect, MT, W>;
-  constexpr int smem = mla::SmemLayout<MT, MT>::bytes;
-  int rc = opt_in_smem(kernel, smem, done);
+  auto kernel = mla::sparse_mla_partials_kernel<kBeside, kDirect, MT, W, NB>;
+  constexpr int smem = mla::SmemLayout<MT, NB>::bytes;
+  // 85: the 196 KB configuration of the scan and the top-k also for the form of 127 KB, beside which the merge's CTAs then
+  // find room to wait (attention + merge of 128 heads 10.2 us; in the 132 KB one of its own 11.3)
+  int rc = opt_in_smem(kernel, smem, done, MT == 2 && NB == 1 ? 85 : int(cudaSharedmemCarveoutDefault));
   if (rc) return rc;
   DSA_CUDA(launch_pdl(kernel, dim3(nsplit, p.H / (MT * DSA_HEAD_BLOCK), R), dim3(32 * W), smem, st, p));
   return DSA_OK;
 }
-template <int MT, int W>
+template <int MT, int W, int NB>
 static int launch_mla_partials(const mla::Params& p, int R, int nsplit, bool beside, cudaStream_t st) {
-  if (beside) return p.out ? launch_mla_partials_as<true, true, MT, W>(p, R, nsplit, st) : launch_mla_partials_as<true, false, MT, W>(p, R, nsplit, st);
-  return p.out ? launch_mla_partials_as<false, true, MT, W>(p, R, nsplit, st) : launch_mla_partials_as<false, false, MT, W>(p, R, nsplit, st);
+  if (beside)
+    return p.out ? launch_mla_partials_as<true, true, MT, W, NB>(p, R, nsplit, st) : launch_mla_partials_as<true, false, MT, W, NB>(p, R, nsplit, st);
+  return p.out ? launch_mla_partials_as<false, true, MT, W, NB>(p, R, nsplit, st) : launch_mla_partials_as<false, false, MT, W, NB>(p, R, nsplit, st);
 }
 }  // extern "C++"
 
@@ -951,12 +957,15 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
     DSA_CUDA(launch_pdl(kernel, dim3(nsplit, H / mla_tc::kHG, R), dim3(mla_tc::kThreads), mla_tc::Smem::bytes, st, p));
     return DSA_OK;
   }
-  // Where 16-head CTAs would share the SMs, 32 heads per CTA: the rows are gathered once for both blocks and, of a split
-  // of several tiles, the next tile is on its way. Attention + merge inside a step, us, 16 / 32 heads per CTA: one row
-  // of 128 heads (256 CTAs of one tile) 9.8 / 9.5, 3 rows of 64 (two tiles each) 13.9 / 12.6, 8 rows of 32 15.3 / 13.3.
+  // Where 16-head CTAs would share the SMs, 32 heads per CTA: the rows are gathered once for both blocks. Layers of the hot
+  // path in a row, us, 16 / 32 heads per CTA: one row of 128 heads (256 CTAs of one tile) 24.5 / 24.1, of fp8 rows 24.9 / 23.7.
+  // Of a split of several tiles the next one is on its way (3 rows of 64 heads, two tiles each, 29.0 / 26.9; 8 rows of 32
+  // 33.3 / 31.2); of one tile there is no second buffer: it would hold nothing and take the SM for itself (24.8).
   const int64_t ctas = int64_t(nsplit) * (H / DSA_HEAD_BLOCK) * R;
-  if (H % (2 * DSA_HEAD_BLOCK) == 0 && ctas > sm_count()) return launch_mla_partials<2, 8>(p, R, nsplit, beside, st);
-  return launch_mla_partials<1, 4>(p, R, nsplit, beside, st);
+  if (H % (2 * DSA_HEAD_BLOCK) == 0 && ctas > sm_count())
+    return p.keys_per_split > mla::kBN ? launch_mla_partials<2, 8, 2>(p, R, nsplit, beside, st)
+                                       : launch_mla_partials<2, 8, 1>(p, R, nsplit, beside, st);
+  return launch_mla_partials<1, 4, 1>(p, R, nsplit, beside, st);
 }
 
 int dsa_sparse_mla_partials(const void* q, const void* kv, const int32_t* indices,

@@ -385,11 +385,11 @@ __device__ __forceinline__ void dequant_tile_inplace(uint8_t* s_k, const int* s_
 // it releases its own dependents and starts at once, beside that kernel, and waits for it only
 // before it exits: it still completes after it, and the next kernel's wait covers both.
 // kDirect: the split is the only one and writes the result itself.
-// MT: blocks of 16 heads per CTA; hg counts blocks of 16 MT heads.
-template <bool kBeside, bool kDirect, int MT, int W>
+// MT: blocks of 16 heads per CTA; hg counts blocks of 16 MT heads. NB: row buffers (one block: one, since two CTAs share an SM
+// and cover each other's gathers).
+template <bool kBeside, bool kDirect, int MT, int W, int NB>
 __device__ __forceinline__ void mla_partials_body(const Params& p, const int split, const int hg, const int r,
                                                   uint8_t* smem) {
-  constexpr int NB = MT;  // (one block: two CTAs share an SM and cover each other's gathers)
   constexpr int kRowsPerWarp = kBN / W;  // latent rows of a tile that a warp requests
   using L = SmemLayout<MT, NB>;
   constexpr int kHeads = MT * kHB;
@@ -569,11 +569,11 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
 
 // (instantiations of their own: the direct form's code costs a step 0.1 us)
 // (registers: what leaves room for the merge kernel's CTAs, which wait beside this kernel's)
-template <bool kBeside, bool kDirect, int MT, int W>
+template <bool kBeside, bool kDirect, int MT, int W, int NB>
 __global__ void __launch_bounds__(32 * W, MT == 1 ? 3 : kDirect ? 1 : 2)
 sparse_mla_partials_kernel(const Params p) {
   extern __shared__ __align__(16) uint8_t mla_smem[];
-  mla_partials_body<kBeside, kDirect, MT, W>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
+  mla_partials_body<kBeside, kDirect, MT, W, NB>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
 }
 
 // ------------------------------------------------------------------------------

@@ -22,6 +22,10 @@ ATTN_TOL = 2e-2
     (3, 96, 700, 9),     # 96-key splits
     (19, 32, 64, 4),     # 16 keys per split
     (75, 32, 130, 1),    # one split, no partials; three tiles
+    (75, 32, 64, 1),     # one tile
+    (75, 32, 260, 1),    # five tiles: both buffers are refilled, the last tile is short
+    (75, 32, 330, 1),    # six
+    (75, 32, 420, 1),    # seven
     (5, 32, 330, 2),     # five heads' CTAs, merges of two splits
 ])
 @pytest.mark.parametrize("fp8", [False, True])
