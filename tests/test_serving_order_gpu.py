@@ -1,5 +1,5 @@
-"""The serving entry runs its attention beside the top-k where that is safe: the results are those of the
-separate modes, also where the incumbents are the very buffer that the selection is written to."""
+"""The serving entry runs its attention behind scan and top-k, beside the top-k, unless the incumbents are the very
+buffer that the selection is written to: then in front of them. The results are those of the separate modes."""
 
 from __future__ import annotations
 
@@ -13,22 +13,38 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("heads,topk,cap,fp8", [(16, 512, 2048, False), (64, 512, 2048, True), (128, 2048, 4096, False)])
 @pytest.mark.parametrize("mapped", [False, True])
-def test_incumbents_that_are_the_selection_buffer(heads, topk, cap, fp8, mapped):
-    from dsa_multi_layer_indexer_b200 import _lib, serving
+def test_incumbents_that_are_the_selection_buffer(heads, topk, cap, fp8, mapped, monkeypatch):
+    from dsa_multi_layer_indexer_b200 import _lib, ops, serving
 
+    order = []
+
+    def noted(name, fn):
+        def f(*a, **kw):
+            order.append((name, kw.get("beside_previous", False)))
+            return fn(*a, **kw)
+        return f
+
+    for name, what in (("sparse_mla_decode", "attention"), ("indexer_scan_fp8_paged", "scan"), ("topk_select", "select"),
+                       ("topk_select_paged", "select")):
+        monkeypatch.setattr(ops, name, noted(what, getattr(ops, name)))
     serving.clear_scratch()
     c = build_case(fp8, cap=cap, heads=heads, topk=topk, lens=[cap, cap - 300, cap - 7])
     kw = {} if mapped else {"pool_map": None}
-    attn, nxt = call(c, **kw)
-    assert torch.equal(attn, call(c, mode="attn_only", **kw))
+    old = c["inc"].cuda()
+    attn, nxt = call(c, **kw)  # (plan buffers)
+    selected = nxt.clone()
+    assert not torch.equal(old, selected)
+    want = call(c, mode="attn_only", **kw).clone()
+    over_selected = call({**c, "inc": selected}, mode="attn_only", **kw).clone()
+    assert not torch.equal(want, over_selected)
     for _ in range(3):
-        attn, nxt = call(c, **kw)
-        own = {**c, "inc": nxt.clone()}
-        want = call(own, mode="attn_only", **kw).clone()
-        selected = nxt.clone()
-        attn, again = call({**c, "inc": nxt}, **kw)  # reads and writes one buffer
-        assert again.data_ptr() == nxt.data_ptr()
-        assert torch.equal(attn, want) and torch.equal(again, selected)
-        attn, again = call(own, **kw)
-        assert torch.equal(attn, want) and torch.equal(again, selected)
+        for aliased in (True, False):
+            nxt.copy_(old)
+            attn.fill_(float("nan"))
+            order.clear()
+            got, again = call({**c, "inc": nxt if aliased else old.clone()}, **kw)
+            assert again.data_ptr() == nxt.data_ptr() and got.data_ptr() == attn.data_ptr()
+            assert torch.equal(got, want) and torch.equal(again, selected)
+            assert order == ([("attention", False), ("scan", False), ("select", False)] if aliased else
+                             [("scan", False), ("select", False), ("attention", True)])
     _lib.check_device_status()
