@@ -75,6 +75,12 @@ def _overlap(a: torch.Tensor, b: torch.Tensor) -> bool:
             and b.data_ptr() < a.data_ptr() + a.numel() * a.element_size())
 
 
+def _attention_ready(q: torch.Tensor, kv: torch.Tensor, slots: torch.Tensor, sm_scale) -> bool:
+    """Whether the attention will take its operands, so that it may be enqueued last."""
+    return (q.is_cuda and q.dtype == torch.bfloat16 and q.data_ptr() % 16 == 0 and kv.is_cuda and kv.is_contiguous()
+            and kv.data_ptr() % 16 == 0 and kv.shape[0] > 0 and slots.is_cuda and hasattr(sm_scale, "__float__"))
+
+
 def clear_scratch() -> None:
     _plans.clear()
     _operands.clear()
@@ -180,12 +186,13 @@ def fused_hide_decode_paged(
         # The attention needs neither the scan nor the top-k. Where the selection is one launch it goes
         # behind the two and runs beside the top-k (3 requests of 9152 tokens, the whole step 34.4 -> 25.8 us;
         # 32 of up to 64K, where the attention fills the device by itself, 108.3 -> 106.9); not where it
-        # reads the list that the top-k writes.
+        # reads the list that the top-k writes, nor where it will refuse its operands: a refused call
+        # leaves the selection of the one before it alone.
         if mode == "full" and sel_mode == "exact" and index_topk == topk:
             if plan.next_idx is None:
                 plan.select_buffers()
-            behind = plan.paged and (out_index_pool is None or _is_slot_map(out_index_pool, skv_cap)) and not _overlap(
-                slots, plan.next_idx)
+            behind = (plan.paged and (out_index_pool is None or _is_slot_map(out_index_pool, skv_cap))
+                      and _attention_ready(q_rows, kv, slots, sm_scale) and not _overlap(slots, plan.next_idx))
         else:
             behind = False
         if not behind:
