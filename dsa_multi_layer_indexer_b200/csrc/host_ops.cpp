@@ -432,6 +432,22 @@ PyObject* mla(PyObject* const* a) {
   return result(a[10], out);
 }
 
+// (q, kv, slots, sm_scale, next_idx, out_index_pool, skv_cap): whether the serving entry may enqueue the attention behind
+// scan and top-k. Not where it will refuse its operands (a refused call leaves the last selection alone), where it
+// reads the list that the top-k writes, or where the pool cannot be the top-k's index map (the selection then takes
+// further launches). One call: in Python these checks took 2 us of a pass whose enqueueing takes 25.
+PyObject* attention_last(PyObject* const* a) {
+  const Tensor &q = ten(a[0], "q"), &kv = ten(a[1], "kv"), &slots = ten(a[2], "slots"), &next = ten(a[4], "next_idx");
+  const Tensor* map = opt(a[5], "out_index_pool");
+  const auto begin = [](const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()); };
+  const PyNumberMethods* number = Py_TYPE(a[3])->tp_as_number;
+  const bool taken = q.is_cuda() && q.scalar_type() == at::kBFloat16 && begin(q) % 16 == 0 && kv.is_cuda() && kv.is_contiguous() &&
+                     kv.numel() > 0 && begin(kv) % 16 == 0 && slots.is_cuda() && number && number->nb_float;
+  const bool mapped = !map || (map->scalar_type() == at::kInt && map->size(1) == integer(a[6]) && map->is_contiguous());
+  const bool apart = begin(slots) + slots.nbytes() <= begin(next) || begin(next) + next.nbytes() <= begin(slots);
+  return PyBool_FromLong(taken && mapped && apart);
+}
+
 // (q, kv, indices, value_dim, sm_scale, seq_lens, rows_per_seq)
 PyObject* mla_f32(PyObject* const* a) {
   const Tensor &q = ten(a[0], "q"), &kv = ten(a[1], "kv");
@@ -1031,7 +1047,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
 #define M(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&entry<name, n>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&bind)), METH_FASTCALL, nullptr},
-    M(scan_fp8, 10), M(scan_paged, 8), M(scan_f32, 7), M(topk, 11), M(topk_paged, 7), M(default_nsplit, 4), M(mla, 14), M(mla_f32, 7), M(rmsnorm, 3),
+    M(scan_fp8, 10), M(scan_paged, 8), M(scan_f32, 7), M(topk, 11), M(topk_paged, 7), M(default_nsplit, 4), M(mla, 14), M(attention_last, 7), M(mla_f32, 7), M(rmsnorm, 3),
     M(add_rmsnorm, 4), M(silu_mul, 2), M(indexer_stage, 18), M(latent_append, 11), M(prefill_latents, 16), M(prefill_queries, 13),
     M(plain_weights, 6), M(full_operands, 29), M(project_output, 5), M(mlp, 4),
     M(abi_scan, AbiArgs<decltype(::dsa_indexer_scan_fp8)>::value), M(abi_scan_paged, AbiArgs<decltype(::dsa_indexer_scan_fp8_paged)>::value),

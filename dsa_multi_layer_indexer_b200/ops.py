@@ -209,6 +209,11 @@ def sparse_mla_decode(
                        beside_previous)
 
 
+def attention_last(q, kv, slots, sm_scale, next_idx, index_map, cap) -> bool:
+    """Whether the serving entry may enqueue the attention behind scan and top-k (csrc/host_ops.cpp)."""
+    return _host().attention_last(q, kv, slots, sm_scale, next_idx, index_map, cap)
+
+
 def sparse_mla_f32(
     q: torch.Tensor,
     kv: torch.Tensor,

@@ -69,18 +69,6 @@ def _is_slot_map(out_index_pool: torch.Tensor, skv_cap: int) -> bool:
     return out_index_pool.dtype == torch.int32 and out_index_pool.shape[1] == skv_cap and out_index_pool.is_contiguous()
 
 
-def _overlap(a: torch.Tensor, b: torch.Tensor) -> bool:
-    """Whether two contiguous tensors share memory."""
-    return (a.data_ptr() < b.data_ptr() + b.numel() * b.element_size()
-            and b.data_ptr() < a.data_ptr() + a.numel() * a.element_size())
-
-
-def _attention_ready(q: torch.Tensor, kv: torch.Tensor, slots: torch.Tensor, sm_scale) -> bool:
-    """Whether the attention will take its operands, so that it may be enqueued last."""
-    return (q.is_cuda and q.dtype == torch.bfloat16 and q.data_ptr() % 16 == 0 and kv.is_cuda and kv.is_contiguous()
-            and kv.data_ptr() % 16 == 0 and kv.shape[0] > 0 and slots.is_cuda and hasattr(sm_scale, "__float__"))
-
-
 def clear_scratch() -> None:
     _plans.clear()
     _operands.clear()
@@ -120,15 +108,17 @@ def fused_hide_decode_paged(
     sel_mode = "exact" if select is True else "prod" if select is False else _SELECT.get(select) if isinstance(select, str) else None
     if sel_mode is None:
         raise ValueError(f"unknown select={select!r}")
-    if q_all.dim() != 4 or q_all.shape[0] != 1:
-        raise ValueError(f"q_all must be [1,B,H,dqk], got {tuple(q_all.shape)}")
-    _, B, H_real, dqk = q_all.shape
+    q_shape = q_all.shape
+    if len(q_shape) != 4 or q_shape[0] != 1:
+        raise ValueError(f"q_all must be [1,B,H,dqk], got {tuple(q_shape)}")
+    _, B, H_real, dqk = q_shape
     device = q_all.device
     if dqk != ops.LATENT_DIM:
         raise ValueError(f"dqk must be {ops.LATENT_DIM}, got {dqk}")
-    if index_q_fp8.dim() != 3 or index_q_fp8.shape[0] != B:
-        raise ValueError(f"index_q_fp8 must be [B={B},Hidx,didx], got {tuple(index_q_fp8.shape)}")
-    Hidx, didx = int(index_q_fp8.shape[1]), int(index_q_fp8.shape[2])
+    iq_shape = index_q_fp8.shape
+    if len(iq_shape) != 3 or iq_shape[0] != B:
+        raise ValueError(f"index_q_fp8 must be [B={B},Hidx,didx], got {tuple(iq_shape)}")
+    Hidx, didx = int(iq_shape[1]), int(iq_shape[2])
     if didx != ops.INDEX_DIM or Hidx % 16:
         raise ValueError(f"unsupported indexer geometry Hidx={Hidx} didx={didx}")
     if index_q_fp8.dtype not in (torch.float8_e4m3fn, torch.uint8):
@@ -137,9 +127,10 @@ def fused_hide_decode_paged(
         raise ValueError(f"index_weights must be [B,Hidx]=({B},{Hidx}), got {tuple(index_weights.shape)}")
     if seq_lens.shape != (B,) or seq_lens.dtype != torch.int32:
         raise ValueError(f"seq_lens must be int32 [B={B}], got {tuple(seq_lens.shape)} {seq_lens.dtype}")
-    if page_table.dim() != 2 or page_table.shape[0] != B or page_table.dtype != torch.int32:
-        raise ValueError(f"page_table must be int32 [B={B}, pt_stride], got {tuple(page_table.shape)} {page_table.dtype}")
-    pt_stride = int(page_table.shape[1])
+    pt_shape = page_table.shape
+    if len(pt_shape) != 2 or pt_shape[0] != B or page_table.dtype != torch.int32:
+        raise ValueError(f"page_table must be int32 [B={B}, pt_stride], got {tuple(pt_shape)} {page_table.dtype}")
+    pt_stride = int(pt_shape[1])
     skv_cap = int(skv_cap)
     if pt_stride * ops.PAGE_TOKENS < skv_cap:
         raise ValueError(f"page table ({pt_stride} pages) does not cover skv_cap={skv_cap}")
@@ -147,9 +138,10 @@ def fused_hide_decode_paged(
         raise ValueError(f"index_k_paged must be uint8 [num_pages, {ops.INDEX_PAGE_BYTES}]")
     if out_index_pool is not None and (out_index_pool.shape[0] != B or out_index_pool.shape[1] < skv_cap):
         raise ValueError(f"out_index_pool must be [B={B}, >= {skv_cap}], got {tuple(out_index_pool.shape)}")
-    if incumbent_slots.shape[0] != B:
-        raise ValueError(f"incumbent batch {incumbent_slots.shape[0]} != {B}")
-    topk = int(incumbent_slots.shape[1])
+    inc_shape = incumbent_slots.shape
+    if inc_shape[0] != B:
+        raise ValueError(f"incumbent batch {inc_shape[0]} != {B}")
+    topk = int(inc_shape[1])
     index_topk = topk if index_topk is None else int(index_topk)
     S_pool, row_w = kv_pool.shape
     kv_fp8 = row_w == _FP8_ROW and kv_pool.dtype in (torch.uint8, torch.float8_e4m3fn)
@@ -164,7 +156,8 @@ def fused_hide_decode_paged(
     if plan is None:
         plan = _plans[key] = _Plan(device, B, H_real, skv_cap, int(nsplit_attn), topk)
 
-    attn_out = attend = None
+    attn_out = None
+    behind = False
     if mode != "scan_only":
         if plan.attn is None:
             plan.attention_buffers()
@@ -179,10 +172,6 @@ def fused_hide_decode_paged(
         kv = kv_pool if kv_pool.dtype != torch.float8_e4m3fn else kv_pool.view(torch.uint8)
         attn_out = plan.attn_out
 
-        def attend(beside: bool) -> None:
-            ops.sparse_mla_decode(q_rows, kv, slots, sm_scale, None, rows_per_seq=B, nsplit=plan.nsplit,
-                                  scratch=plan.part, out=plan.attn, beside_previous=beside)
-
         # The attention needs neither the scan nor the top-k. Where the selection is one launch it goes
         # behind the two and runs beside the top-k (3 requests of 9152 tokens, the whole step 34.4 -> 25.8 us;
         # 32 of up to 64K, where the attention fills the device by itself, 108.3 -> 106.9); not where it
@@ -191,13 +180,10 @@ def fused_hide_decode_paged(
         if mode == "full" and sel_mode == "exact" and index_topk == topk:
             if plan.next_idx is None:
                 plan.select_buffers()
-            behind = (plan.paged and (out_index_pool is None or _is_slot_map(out_index_pool, skv_cap))
-                      and _attention_ready(q_rows, kv, slots, sm_scale) and not _overlap(slots, plan.next_idx))
-        else:
-            behind = False
+            behind = plan.paged and ops.attention_last(q_rows, kv, slots, sm_scale, plan.next_idx, out_index_pool, skv_cap)
         if not behind:
-            attend(False)
-            attend = None
+            ops.sparse_mla_decode(q_rows, kv, slots, sm_scale, None, rows_per_seq=B, nsplit=plan.nsplit, scratch=plan.part,
+                                  out=plan.attn)
         if mode == "attn_only":
             return attn_out
 
@@ -225,14 +211,10 @@ def fused_hide_decode_paged(
             # the selection leaves the top-k as KV slots, page * 64 + offset from the page-64 table
             # (kernels/cuda_fused_sparse_splitk.py:1142-1144)
             ops.topk_select_paged(logits, topk, seq_lens, plan.hist, table, next_idx)
-            if attend is not None:
-                attend(True)
-        elif out_index_pool is not None and plan.paged and _is_slot_map(out_index_pool, skv_cap):
+        elif out_index_pool is not None and plan.paged and (behind or _is_slot_map(out_index_pool, skv_cap)):
             # positions -> KV slots through out_index_pool, read by the top-k as its index map
             ops.topk_select(logits, topk, seq_lens, hist=plan.hist, index_map=out_index_pool, out_idx=next_idx,
                             workspace=plan.topk_ws)
-            if attend is not None:
-                attend(True)
         else:
             pos = plan.pos
             ops.topk_select(logits, topk, seq_lens, hist=plan.hist, out_idx=pos, workspace=plan.topk_ws)
@@ -242,6 +224,9 @@ def fused_hide_decode_paged(
             else:
                 mapped = torch.gather(page_table, 1, safe >> 6) * ops.PAGE_TOKENS + (pos & (ops.PAGE_TOKENS - 1))
             torch.where(pos >= 0, mapped, pos, out=next_idx)  # padding stays -1
+        if behind:
+            ops.sparse_mla_decode(q_rows, kv, slots, sm_scale, None, rows_per_seq=B, nsplit=plan.nsplit, scratch=plan.part,
+                                  out=plan.attn, beside_previous=True)
         if return_logits:
             return attn_out, next_idx, logits
         return attn_out, next_idx

@@ -48,3 +48,14 @@ def test_incumbents_that_are_the_selection_buffer(heads, topk, cap, fp8, mapped,
             assert order == ([("attention", False), ("scan", False), ("select", False)] if aliased else
                              [("scan", False), ("select", False), ("attention", True)])
     _lib.check_device_status()
+
+
+def test_attention_goes_first_where_the_lists_share_memory():
+    from dsa_multi_layer_indexer_b200 import ops
+
+    q, kv = (torch.zeros(n, 16, 576, dtype=torch.bfloat16, device="cuda") for n in (8, 1))
+    last = lambda a, b: ops.attention_last(q, kv[0], a, 1.0, b, None, 64)
+    whole, other = (torch.zeros(8, 16, dtype=torch.int32, device="cuda") for _ in range(2))
+    assert not last(whole, whole) and not last(whole[2:5], whole[4:]) and not last(whole[4:], whole[2:5])
+    assert not last(whole[3:4], whole) and not last(whole, whole[7:])
+    assert last(whole[:4], whole[4:]) and last(whole[4:], whole[:4]) and last(whole, other)
