@@ -977,11 +977,11 @@ int dsa_sparse_mla_partials(const void* q, const void* kv, const int32_t* indice
 }
 
 extern "C++" {
-template <int kParts>
+template <int kParts, bool kUnrolled>
 static int launch_combine(const float* part_acc, const float* part_m, const float* part_l, void* out, int R, int H, int nsplit,
                           cudaStream_t st) {
   const int threads = 128 / kParts * (nsplit < 4 ? nsplit : 4);  // one load group per split, up to four
-  DSA_CUDA(launch_pdl(mla::sparse_mla_combine_kernel<kParts>, dim3(unsigned(H) * kParts, R), dim3(threads), 0, st, part_acc, part_m,
+  DSA_CUDA(launch_pdl(mla::sparse_mla_combine_kernel<kParts, kUnrolled>, dim3(unsigned(H) * kParts, R), dim3(threads), 0, st, part_acc, part_m,
                       part_l, static_cast<__nv_bfloat16*>(out), H, nsplit));
   return DSA_OK;
 }
@@ -1007,10 +1007,11 @@ int dsa_sparse_mla_combine(const float* part_acc, const float* part_m, const flo
   // then finds no room (64 pairs: hot path 21.7 / 22.05, whole layers 160.7 / 162.2), nor with more CTAs than SMs (128
   // pairs: the merge 2.9 / 3.9).
   const int64_t pairs = int64_t(R) * H;
-  if (4 * pairs <= sm_count()) return launch_combine<4>(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
-  if (3 * pairs <= sm_count())
-    return launch_combine<2>(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
-  return launch_combine<1>(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
+  auto launch = 4 * pairs <= sm_count()   ? launch_combine<4, true>
+                : 3 * pairs <= sm_count() ? launch_combine<2, true>
+                : pairs <= sm_count()     ? launch_combine<1, false>
+                                          : launch_combine<1, true>;
+  return launch(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
 }
 
 int dsa_sparse_mla_decode(const void* q, const void* kv, const int32_t* indices,

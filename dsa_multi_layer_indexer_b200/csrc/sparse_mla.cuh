@@ -568,9 +568,10 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
 }
 
 // (instantiations of their own: the direct form's code costs a step 0.1 us)
-// (registers: what leaves room for the merge kernel's CTAs, which wait beside this kernel's)
+// (registers: what leaves room for the merge kernel's CTAs, which wait beside this kernel's; nothing waits beside the direct
+// form: one fp8 tile of 16 heads 7.6 us with 242 registers, 7.95 with 168)
 template <bool kBeside, bool kDirect, int MT, int W, int NB>
-__global__ void __launch_bounds__(32 * W, MT == 1 ? 3 : kDirect ? 1 : 2)
+__global__ void __launch_bounds__(32 * W, MT == 1 ? (kDirect ? 2 : 3) : kDirect ? 1 : 2)
 sparse_mla_partials_kernel(const Params p) {
   extern __shared__ __align__(16) uint8_t mla_smem[];
   mla_partials_body<kBeside, kDirect, MT, W, NB>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
@@ -583,7 +584,7 @@ sparse_mla_partials_kernel(const Params p) {
 // group g folds splits g, g + ngrp, ... with all loads of a chunk of eight splits in
 // flight at once, then the groups' results are merged in a fixed order, the same for every kParts.
 // Bound by two dependent trips to L2 and by the 61 bytes a cycle that an SM gets from there.
-template <int kParts>
+template <int kParts, bool kUnrolled>
 __global__ void __launch_bounds__(512 / kParts)
 sparse_mla_combine_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_m,
                           const float* __restrict__ part_l, __nv_bfloat16* __restrict__ out, int H,
@@ -594,10 +595,11 @@ sparse_mla_combine_kernel(const float* __restrict__ part_acc, const float* __res
   const int h = blockIdx.x / kParts, c0 = (blockIdx.x % kParts) * kCols, r = blockIdx.y;
   const int tid = threadIdx.x % kGroup, grp = threadIdx.x / kGroup;
   const int ngrp = blockDim.x / kGroup;  // 1..4, each taking every ngrp-th split
-  // (final loops unrolled: 0.1-0.2 us less with part of the columns per CTA, but with all of them 64 registers instead of 74
-  // and 25.2 instead of 24.5 us a layer of 128 heads, though the merge alone is as fast; presumably the next launch's CTAs
-  // then come to lie beside these)
-  const int groups = kParts == 1 ? ngrp : 4;
+  // Final loops unrolled: 0.1-0.2 us less with part of the columns per CTA. With all of them it takes 64 registers instead
+  // of 74, and two such CTAs share an SM: with more pairs than SMs that is a wave less (2 rows of 128 heads, 32 splits,
+  // attention + merge 13.0 instead of 14.3 us), with fewer a layer of 128 heads takes 25.2 instead of 24.5, though the merge
+  // alone is as fast; presumably the next launch's CTAs then come to lie beside these.
+  const int groups = kUnrolled ? 4 : ngrp;
   DSA_KTIME_BEGIN(3);
   pdl_wait();
   pdl_launch_dependents();
