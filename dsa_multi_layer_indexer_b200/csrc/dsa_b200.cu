@@ -913,10 +913,10 @@ static int mla_prepare(const void* q, const void* kv, const int32_t* indices, co
 }
 
 extern "C++" {
-template <bool kBeside, bool kDirect, int MT, int W, int NB>
+template <bool kBeside, bool kDirect, bool kMayExpand, int MT, int W, int NB>
 static int launch_mla_partials_as(const mla::Params& p, int R, int nsplit, cudaStream_t st) {
   static bool done[64];
-  auto kernel = mla::sparse_mla_partials_kernel<kBeside, kDirect, MT, W, NB>;
+  auto kernel = mla::sparse_mla_partials_kernel<kBeside, kDirect, kMayExpand, MT, W, NB>;
   constexpr int smem = mla::SmemLayout<MT, NB>::bytes;
   // 85: the 196 KB configuration of the scan and the top-k also for the form of 127 KB, beside which the merge's CTAs then
   // find room to wait (attention + merge of 128 heads 10.2 us; in the 132 KB one of its own 11.3)
@@ -925,11 +925,18 @@ static int launch_mla_partials_as(const mla::Params& p, int R, int nsplit, cudaS
   DSA_CUDA(launch_pdl(kernel, dim3(nsplit, p.H / (MT * DSA_HEAD_BLOCK), R), dim3(32 * W), smem, st, p));
   return DSA_OK;
 }
+template <bool kMayExpand, int MT, int W, int NB>
+static int launch_mla_partials_of(const mla::Params& p, int R, int nsplit, bool beside, cudaStream_t st) {
+  if (beside)
+    return p.out ? launch_mla_partials_as<true, true, kMayExpand, MT, W, NB>(p, R, nsplit, st)
+                 : launch_mla_partials_as<true, false, kMayExpand, MT, W, NB>(p, R, nsplit, st);
+  return p.out ? launch_mla_partials_as<false, true, kMayExpand, MT, W, NB>(p, R, nsplit, st)
+               : launch_mla_partials_as<false, false, kMayExpand, MT, W, NB>(p, R, nsplit, st);
+}
 template <int MT, int W, int NB>
 static int launch_mla_partials(const mla::Params& p, int R, int nsplit, bool beside, cudaStream_t st) {
-  if (beside)
-    return p.out ? launch_mla_partials_as<true, true, MT, W, NB>(p, R, nsplit, st) : launch_mla_partials_as<true, false, MT, W, NB>(p, R, nsplit, st);
-  return p.out ? launch_mla_partials_as<false, true, MT, W, NB>(p, R, nsplit, st) : launch_mla_partials_as<false, false, MT, W, NB>(p, R, nsplit, st);
+  return p.kv_fp8 ? launch_mla_partials_of<true, MT, W, NB>(p, R, nsplit, beside, st)
+                  : launch_mla_partials_of<false, MT, W, NB>(p, R, nsplit, beside, st);
 }
 }  // extern "C++"
 

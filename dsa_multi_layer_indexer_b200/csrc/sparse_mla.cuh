@@ -386,8 +386,10 @@ __device__ __forceinline__ void dequant_tile_inplace(uint8_t* s_k, const int* s_
 // before it exits: it still completes after it, and the next kernel's wait covers both.
 // kDirect: the split is the only one and writes the result itself.
 // MT: blocks of 16 heads per CTA; hg counts blocks of 16 MT heads. NB: row buffers (one block: one, since two CTAs share an SM
-// and cover each other's gathers).
-template <bool kBeside, bool kDirect, int MT, int W, int NB>
+// and cover each other's gathers). kMayExpand: rows may be fp8. A launch over bf16 rows carries no code for that: one row of
+// 64 heads 21.7 -> 21.45 us a layer, 8 of 16 heads chained 21.8 -> 20.85, 16 of 32 37.6 -> 37.0; fp8 rows in an instantiation of
+// their own were slower (one row of 128 heads 23.65 -> 24.0: the 32-head form then spills 112 bytes).
+template <bool kBeside, bool kDirect, bool kMayExpand, int MT, int W, int NB>
 __device__ __forceinline__ void mla_partials_body(const Params& p, const int split, const int hg, const int r,
                                                   uint8_t* smem) {
   constexpr int kRowsPerWarp = kBN / W;  // latent rows of a tile that a warp requests
@@ -405,7 +407,8 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   DSA_KTIME_BEGIN(2);
   const int seq = r / p.rows_per_seq;
-  const int row_bytes = p.kv_fp8 ? kFp8Row : kRowBytes;
+  const bool fp8 = kMayExpand && p.kv_fp8;
+  const int row_bytes = fp8 ? kFp8Row : kRowBytes;
   const uint8_t* kv_seq = p.kv + int64_t(seq) * p.kv_seq_stride * row_bytes;
 
   if (tid == 0) {
@@ -455,7 +458,7 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
     if (lane == 0) mbar_arrive_expect_tx(bar, uint32_t(__popc(seen)) * uint32_t(row_bytes));
     __syncwarp();
     if (ok) {
-      if (p.kv_fp8)  // staged at the end of the row's own slot, expanded in place below
+      if (fp8)  // staged at the end of the row's own slot, expanded in place below
         bulk_g2s(smem_u32(dst + kFp8StageOff), kv_seq + int64_t(idx) * kFp8Row, kFp8Row, bar);
       else
         bulk_g2s(smem_u32(dst), kv_seq + int64_t(idx) * kRowBytes, kRowBytes, bar);
@@ -499,7 +502,7 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
     // threads agree on leaving at the softmax's barrier (fp8 rows: here) and nobody is left alone at a later one.
     bool landed = tile > 0 || mbar_wait(bar_q, 0);
     if (!mbar_wait(bar_k(buf, (warp >> 1) & 1), parity)) landed = false;
-    if (p.kv_fp8) {
+    if (fp8) {
       if (!mbar_wait(bar_k(buf, ((warp >> 1) & 1) ^ 1), parity)) landed = false;
       timed_out = cta_any<W>(!landed);
       if (timed_out) break;
@@ -570,11 +573,11 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
 // (instantiations of their own: the direct form's code costs a step 0.1 us)
 // (registers: what leaves room for the merge kernel's CTAs, which wait beside this kernel's; nothing waits beside the direct
 // form: one fp8 tile of 16 heads 7.6 us with 242 registers, 7.95 with 168)
-template <bool kBeside, bool kDirect, int MT, int W, int NB>
+template <bool kBeside, bool kDirect, bool kMayExpand, int MT, int W, int NB>
 __global__ void __launch_bounds__(32 * W, MT == 1 ? (kDirect ? 2 : 3) : kDirect ? 1 : 2)
 sparse_mla_partials_kernel(const Params p) {
   extern __shared__ __align__(16) uint8_t mla_smem[];
-  mla_partials_body<kBeside, kDirect, MT, W, NB>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
+  mla_partials_body<kBeside, kDirect, kMayExpand, MT, W, NB>(p, blockIdx.x, blockIdx.y, blockIdx.z, mla_smem);
 }
 
 // ------------------------------------------------------------------------------
