@@ -919,7 +919,7 @@ static int launch_mla_partials_as(const mla::Params& p, int R, int nsplit, cudaS
   auto kernel = mla::sparse_mla_partials_kernel<kBeside, kDirect, kMayExpand, MT, W, NB>;
   constexpr int smem = mla::SmemLayout<MT, NB>::bytes;
   // 85: the 196 KB configuration of the scan and the top-k also for the form of 127 KB, beside which the merge's CTAs then
-  // find room to wait (attention + merge of 128 heads 10.2 us; in the 132 KB one of its own 11.3)
+  // find room to wait (attention + merge of 128 heads over bf16 rows 10.2 us; in the 132 KB one of its own 11.3)
   int rc = opt_in_smem(kernel, smem, done, MT == 2 && NB == 1 ? 85 : int(cudaSharedmemCarveoutDefault));
   if (rc) return rc;
   DSA_CUDA(launch_pdl(kernel, dim3(nsplit, p.H / (MT * DSA_HEAD_BLOCK), R), dim3(32 * W), smem, st, p));
@@ -964,14 +964,17 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
     DSA_CUDA(launch_pdl(kernel, dim3(nsplit, H / mla_tc::kHG, R), dim3(mla_tc::kThreads), mla_tc::Smem::bytes, st, p));
     return DSA_OK;
   }
-  // Where 16-head CTAs would share the SMs, 32 heads per CTA: the rows are gathered once for both blocks. Layers of the hot
-  // path in a row, us, 16 / 32 heads per CTA: one row of 128 heads (256 CTAs of one tile) 24.5 / 24.1, of fp8 rows 24.9 / 23.7.
-  // Of a split of several tiles the next one is on its way (3 rows of 64 heads, two tiles each, 29.0 / 26.9; 8 rows of 32
-  // 33.3 / 31.2); of one tile there is no second buffer: it would hold nothing and take the SM for itself (24.8).
+  // Where 16-head CTAs would share the SMs, 32 heads per CTA if that pays: the rows are gathered (and fp8 rows expanded)
+  // once for both blocks and, of a split of several tiles, the next one is on its way. Layers of the hot path in a row,
+  // us, 16 / 32 heads per CTA: splits of several tiles, 3 rows of 64 heads 28.0 / 26.85, 8 of 32 32.2 / 31.2, 16 of 32 41.9 / 39.0;
+  // one fp8 tile, a row of 128 heads 25.0 / 23.7 (one row buffer: a second would hold nothing and take the SM for itself).
+  // Not one bf16 tile, whose phases two CTAs on an SM overlap: a row of 128 heads 24.0 / 24.05, of 96 20.25 / 20.7, 2 rows
+  // of 64 24.15 / 24.4, 16 of 32 over 512 keys 25.7 / 26.4; 7 of 32 over 1024 25.4 / 25.2.
   const int64_t ctas = int64_t(nsplit) * (H / DSA_HEAD_BLOCK) * R;
-  if (H % (2 * DSA_HEAD_BLOCK) == 0 && ctas > sm_count())
-    return p.keys_per_split > mla::kBN ? launch_mla_partials<2, 8, 2>(p, R, nsplit, beside, st)
-                                       : launch_mla_partials<2, 8, 1>(p, R, nsplit, beside, st);
+  if (H % (2 * DSA_HEAD_BLOCK) == 0 && ctas > sm_count()) {
+    if (p.keys_per_split > mla::kBN) return launch_mla_partials<2, 8, 2>(p, R, nsplit, beside, st);
+    if (kv_fp8) return launch_mla_partials_of<true, 2, 8, 1>(p, R, nsplit, beside, st);
+  }
   return launch_mla_partials<1, 4, 1>(p, R, nsplit, beside, st);
 }
 

@@ -15,8 +15,9 @@ ATTN_TOL = 2e-2
 SM = 192 ** -0.5
 
 
+@pytest.mark.parametrize("fp8", [False, True])
 @pytest.mark.parametrize("rows,heads,ctx,topk,nsplit", [
-    (1, 128, 20000, 2048, None),  # 32 heads per CTA, one tile per split
+    (1, 128, 20000, 2048, None),  # one tile per split: 16 heads per CTA, fp8 rows 32
     (10, 32, 6000, 2048, None),   # 32 heads per CTA, three tiles per split
     (80, 32, 3000, 256, 1),       # the same without partials, four tiles
     (80, 32, 3000, 64, 1),        # one tile
@@ -24,7 +25,7 @@ SM = 192 ** -0.5
     (4, 128, 6000, 2048, None),   # tcgen05
     (80, 64, 3000, 256, 1),       # tcgen05 without partials
 ])
-def test_beside_the_topk_equals_alone(rows, heads, ctx, topk, nsplit):
+def test_beside_the_topk_equals_alone(rows, heads, ctx, topk, nsplit, fp8):
     from dsa_multi_layer_indexer_b200 import _lib, ops
     from dsa_multi_layer_indexer_b200.decode import HotPathState, LayerCache
 
@@ -32,7 +33,10 @@ def test_beside_the_topk_equals_alone(rows, heads, ctx, topk, nsplit):
     rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g)
     st = HotPathState(rows, heads, 64, ctx, topk, "cuda", nsplit=nsplit)
     k8, ks = ops.quantize_e4m3_rowwise(rand(rows, ctx, 128))
-    cache = LayerCache(k8.view(torch.uint8), ks, rand(rows, ctx, 576).to(torch.bfloat16))
+    lat = rand(rows * ctx, 576)
+    kv = O.pack_fp8_latent(lat.cpu()).cuda() if fp8 else lat.to(torch.bfloat16)
+    kv_ref = O.unpack_fp8_latent(kv.cpu()) if fp8 else kv.cpu()
+    cache = LayerCache(k8.view(torch.uint8), ks, kv.view(rows, ctx, -1))
     q8, sq = ops.quantize_e4m3_rowwise(rand(rows, 64, 128))
     st.index_q.copy_(q8.view(torch.uint8))
     st.index_w.copy_(sq * rand(rows, 64) / 8)
@@ -42,7 +46,7 @@ def test_beside_the_topk_equals_alone(rows, heads, ctx, topk, nsplit):
     selected = st.run_indexer(cache).clone()
     want = st.run_attention(cache, attend, SM).clone()
     for r in (0, rows - 1):
-        ref = O.sparse_mla_decode(st.q[r:r + 1].cpu(), cache.kv[r].cpu(), attend[r:r + 1].cpu(), [int(st.seq_lens[r])], SM)
+        ref = O.sparse_mla_decode(st.q[r:r + 1].cpu(), kv_ref.view(rows, ctx, 576)[r], attend[r:r + 1].cpu(), [int(st.seq_lens[r])], SM)
         assert rel_err(want[r:r + 1].float().cpu(), ref) < ATTN_TOL
 
     def check():
