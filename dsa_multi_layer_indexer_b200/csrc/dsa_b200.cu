@@ -953,7 +953,7 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // Head counts that fill 64-row blocks go to the tcgen05 kernel once there are enough
   // 64-head x 64-key tiles to give every SM more than one (a single row of 2048 keys
-  // is faster on the mma.sync kernel's 16-head CTAs); its splits are whole 64-key tiles.
+  // is faster on the mma.sync kernel's narrower CTAs); its splits are whole 64-key tiles.
   const int64_t tc_tiles = int64_t(R) * (H / mla_tc::kHG) * ((topk_k + mla_tc::kBN - 1) / mla_tc::kBN);
   if (H % mla_tc::kHG == 0 && sm_scale > 0.f && tc_tiles >= mla_tc::kMinTiles) {
     int kps = (topk_k + nsplit - 1) / nsplit;
@@ -1013,7 +1013,7 @@ int dsa_sparse_mla_combine(const float* part_acc, const float* part_m, const flo
   }
   // few (row, head) pairs: their columns over four or two CTAs (layers of the hot path in a row, one / this many CTAs a pair:
   // 16 pairs 15.4 / 14.7 us, 32 pairs 19.5 / 18.8, 48 pairs 19.6 / 18.4; whole layers of the glm5 preset with 16 and 32
-  // heads 129.7 / 128.9 and 142.2 / 141.7). Not where two a pair would fill most SMs, since the launch behind the merge
+  // heads 129.7 / 128.3 and 142.2 / 141.6). Not where two a pair would fill most SMs, since the launch behind the merge
   // then finds no room (64 pairs: hot path 21.7 / 22.05, whole layers 160.7 / 162.2), nor with more CTAs than SMs (128
   // pairs: the merge 2.9 / 3.9).
   const int64_t pairs = int64_t(R) * H;

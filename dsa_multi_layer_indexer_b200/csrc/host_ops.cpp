@@ -351,7 +351,7 @@ PyObject* topk_paged(PyObject* const* a) {
 // The split count where a caller gives none. Head counts that are a multiple of 64 run on the tcgen05 kernel (one CTA
 // per SM, 64 heads per CTA) once the launch has 128 tiles of 64 heads x 64 keys: about one CTA per SM in total, and a
 // split count that divides the tiles so no split is empty. Smaller launches and other head counts run on the mma.sync
-// kernel (16 heads per CTA, two CTAs per SM). With more (row, head) pairs than SMs at most 16 splits: the merge reads
+// kernel: two CTAs of 16 heads per SM, or one of 32 where a split has several tiles or fp8 rows. With more (row, head) pairs than SMs at most 16 splits: the merge reads
 // every split's partials, and more of them cost more than the shorter splits save (2 rows x 128 heads: 12.8 us with 16
 // splits, 14.9 with 32).
 constexpr int64_t kSms = 148;  // the default of ops.default_nsplit, which plans are made with on any machine

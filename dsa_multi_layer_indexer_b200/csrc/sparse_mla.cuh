@@ -16,10 +16,10 @@
 // dequantised into the bf16 tile exactly as the reference does
 // (fp8 -> f32, x group scale, round to bf16; :1181-1196).
 //
-// What bounds it (one 64-key tile per CTA, cycles after the dependency wait, 16 heads alone on an SM / 32 heads):
-// selection entries 650-950, rows and queries landed 2500-2900 / 3150 (an SM gets 45-61 bytes a cycle from L2),
-// scores 1400 / 2000 and values 700 / 1100 (shared-memory reads: 148 / 221 KB and 65 KB), maximum, softmax and their
-// barriers 900 / 1250, partials 1200 / 2300 (28 bytes a cycle).
+// What bounds it (one 64-key bf16 tile per CTA, cycles after the dependency wait; 16 heads alone on an SM / two such CTAs on it):
+// selection entries 900, rows and queries landed 2400-3400 / 3550 (an SM gets 45-61 bytes a cycle from L2), scores 1250 / 2280
+// and values 750 / 1170 (shared-memory reads: 148 and 65 KB a CTA), maximum, softmax and their barriers 600 / 800, partials
+// 1280-1390 / 1500, and 200 / 920 until the CTA's last warp has stored and added up.
 #pragma once
 
 
@@ -30,7 +30,7 @@ namespace mla {
 
 constexpr int kD = DSA_LATENT_DIM;       // 576
 constexpr int kDV = DSA_VALUE_DIM;       // 512
-constexpr int kHB = DSA_HEAD_BLOCK;      // 16 heads per CTA
+constexpr int kHB = DSA_HEAD_BLOCK;      // heads of a block
 constexpr int kBN = 64;                  // keys per tile
 constexpr int kSlices = 8;               // groups of eight keys of a tile, each summed by itself
 constexpr int kRowBytes = kD * 2;        // 1152
@@ -424,7 +424,7 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
   const int k_begin = split * p.keys_per_split;
   const int k_end = min(k_begin + p.keys_per_split, p.topk);
   const int n_tiles = (max(k_end - k_begin, 0) + kBN - 1) / kBN;
-  const int my_row = warp * kRowsPerWarp + lane;  // (lanes 0..7)
+  const int my_row = warp * kRowsPerWarp + lane;  // (lanes 0..kRowsPerWarp - 1)
   const auto entry = [&](int tile) {
     const int j = k_begin + tile * kBN + my_row;
     if (lane >= kRowsPerWarp || j >= k_end) return -1;
@@ -548,8 +548,8 @@ __device__ __forceinline__ void mla_partials_body(const Params& p, const int spl
     DSA_KTIME_END(2);
     return;
   }
-  // ---- partials of this split: unnormalised accumulator, running max (base 2), sum. An SM writes about 28 bytes a
-  // cycle, so the 32 MT KB take 1200 MT cycles; the sums' barrier waits in their shadow.
+  // ---- partials of this split: unnormalised accumulator, running max (base 2), sum. The 32 MT KB take 1300-1500
+  // cycles with 16 heads, 2050-2400 with 32 (25-32 bytes a cycle and SM); the sums' barrier waits in their shadow.
   const int64_t pbase = (int64_t(r) * p.nsplit + split) * p.H + hg * kHeads;
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) {

@@ -91,8 +91,8 @@ class HotPathState:
     def run_attention(self, cache: LayerCache, attend: torch.Tensor, sm_scale: float,
                       beside_previous: bool = False) -> torch.Tensor:
         """Sparse MLA over ``attend`` (any ``[rows, topk]`` int32 selection). ``beside_previous``:
-        ``attend`` and the queries do not come from the kernel enqueued just before (see
-        :func:`ops.sparse_mla_decode`)."""
+        neither ``attend`` nor the queries come from the two kernels enqueued just before, of which the
+        top-k lets its successor start before it has waited for the scan (see :func:`ops.sparse_mla_decode`)."""
         return ops.sparse_mla_decode(self.q, cache.kv, attend, sm_scale, self.seq_lens, nsplit=self.nsplit,
                                      scratch=self.partials, out=self.out, beside_previous=beside_previous)
 

@@ -101,7 +101,13 @@ def fused_hide_decode_paged(
     ``select=False/"prod"``, ``(attn_out, next_idx int32 [B, topk])`` under
     ``select=True/"kernel"/"exact"/"approx"`` (KV-slot space, ``-1`` padded;
     plus ``logits`` with ``return_logits``), ``(attn_out, next_idx int64)`` under
-    ``select="torch"`` (torch.topk gate)."""
+    ``select="torch"`` (torch.topk gate).
+
+    The returned tensors are buffers of the call's static shape, overwritten by the next call of that shape.
+    The attention is enqueued last and runs beside the top-k, unless ``incumbent_slots`` is the ``next_idx`` that
+    the call before returned: the selection is then written over it, so the attention has to come first (3
+    requests of 9152 tokens: 34.4 us instead of 24.7). A caller that chains layers of one shape gets the shorter
+    order by keeping the selection in a tensor of its own."""
     if mode not in ("full", "attn_only", "scan_only"):
         raise ValueError(f"unknown mode={mode!r}")
     # (by identity: 1 and 0 equal True and False, and are no selections)

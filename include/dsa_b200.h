@@ -278,7 +278,8 @@ int dsa_topk_select_static(const float* logits, const int32_t* seq_lens, int32_t
  * Two kernels serve the partials. Launches with H a multiple of 64 and at least
  * 128 tiles of 64 heads x 64 keys (R * H/64 * ceil(topk/64)) run on tcgen05 /
  * tensor memory with 64 heads per CTA; smaller launches and other head counts
- * run on mma.sync with 16 or 32 heads per CTA. Both write the same part_* layout;
+ * run on mma.sync with 16 heads per CTA, or 32 (CTA counts above the SMs', H a
+ * multiple of 32, and splits of several tiles or fp8 rows). Both write the same part_* layout;
  * part_m is a base-2 softmax reference of the split (not necessarily its
  * maximum) consistent with part_l and part_acc, which is all
  * dsa_sparse_mla_combine needs. (bf16 partial accumulators were measured: the
@@ -319,7 +320,8 @@ int dsa_sparse_mla_decode_beside(const void* q, const void* kv, const int32_t* i
  * `attend_indices` (under the lagged schedule: the PREVIOUS layer's selection)
  * and whose remaining CTAs run this layer's indexer scan into `logits` (+ `hist`),
  * followed by the LSE merge. Same results as dsa_sparse_mla_decode +
- * dsa_indexer_scan_fp8, bit for bit. Replaces launch_fused_sparse_splitk with
+ * dsa_indexer_scan_fp8, bit for bit (the attention where that call runs on
+ * mma.sync). Replaces launch_fused_sparse_splitk with
  * attn_on=1, with_select=1|2 (kernels/cuda_fused_sparse_splitk.py:178-683,
  * :2634-2655); the top-k stays a separate call. Dense bf16 caches only. */
 int dsa_fused_decode(const void* q, const void* kv, const int32_t* attend_indices,
