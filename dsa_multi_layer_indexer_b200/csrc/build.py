@@ -17,7 +17,7 @@ CSRC = Path(__file__).resolve().parent
 PKG = CSRC.parent
 LIB = PKG / "libdsa_b200.so"
 SOURCES = ["dsa_b200.cu"]
-HEADERS = ["common.cuh", "indexer_scan.cuh", "topk_select.cuh", "topk_rows.cuh", "sparse_mla.cuh", "sparse_mla_tc.cuh",
+HEADERS = ["common.cuh", "indexer_scan.cuh", "topk_select.cuh", "topk_rows.cuh", "sparse_mla.cuh", "sparse_mla_tc.cuh", "sparse_mla_pair.cuh",
            "fused_decode.cuh", "decode_prep.cuh", "prefill_prep.cuh", "linear_f32.cuh", "peer_allreduce.cuh"]
 HOST_LIB = PKG / "_host.so"
 HOST_SOURCE = CSRC / "host_ops.cpp"

@@ -17,6 +17,7 @@
 #include "peer_allreduce.cuh"
 #include "prefill_prep.cuh"
 #include "sparse_mla.cuh"
+#include "sparse_mla_pair.cuh"
 #include "sparse_mla_tc.cuh"
 #include "topk_rows.cuh"
 #include "topk_select.cuh"
@@ -108,7 +109,7 @@ static int opt_in_smem(K kernel, size_t bytes, bool (&done)[64], int carveout = 
   if (dev >= 0 && dev < 64) done[dev] = true;
   return DSA_OK;
 }
-static bool g_opt_fused[64], g_opt_mla_tc[2][64], g_opt_mla_f32[64], g_opt_scan_f32[64], g_opt_topk[64];
+static bool g_opt_fused[64], g_opt_mla_tc[2][64], g_opt_mla_pair[2][64], g_opt_mla_f32[64], g_opt_scan_f32[64], g_opt_topk[64];
 
 // Launch with programmatic dependent launch allowed: the kernel may be scheduled
 // while its predecessor in the stream is still draining; it calls
@@ -940,6 +941,44 @@ static int launch_mla_partials(const mla::Params& p, int R, int nsplit, bool bes
 }
 }  // extern "C++"
 
+// One pair of CTAs (sparse_mla_pair.cuh) per two SMs at most; each takes (row, 128 heads, split) triples in turn.
+static int launch_mla_pair(const mla::Params& m, int R, bool beside, cudaStream_t st) {
+  CUtensorMap kv_map, q_map, out_map;
+  const uint64_t kv_dims[2] = {DSA_LATENT_DIM, uint64_t(R / m.rows_per_seq) * uint64_t(m.kv_seq_stride)};
+  const uint64_t q_dims[2] = {DSA_LATENT_DIM, uint64_t(R) * uint64_t(m.H)};
+  const uint64_t strides[1] = {mla::kRowBytes};
+  // the result's rows, or the partials': 64 bytes of 32 rows are stored at a time
+  const uint64_t out_dims[2] = {DSA_VALUE_DIM, uint64_t(R) * uint64_t(m.H) * (m.out ? 1 : m.nsplit)};
+  const uint64_t out_strides[1] = {DSA_VALUE_DIM * (m.out ? 2 : 4)};
+  const uint32_t row_box[2] = {64, 1}, q_box[2] = {64, 64}, out_box[2] = {m.out ? 32u : 16u, 32};
+  int rc = encode_tensor_map(&kv_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, m.kv, kv_dims, strides, row_box, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (!rc) rc = encode_tensor_map(&q_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, m.q, q_dims, strides, q_box, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (!rc)
+    rc = encode_tensor_map(&out_map, m.out ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+                           m.out ? static_cast<const void*>(m.out) : m.part_acc, out_dims, out_strides, out_box, CU_TENSOR_MAP_SWIZZLE_64B);
+  if (rc) return rc;
+  auto kernel = beside ? mla_pair::sparse_mla_pair_kernel<true> : mla_pair::sparse_mla_pair_kernel<false>;
+  rc = opt_in_smem(kernel, mla_pair::Smem::bytes, g_opt_mla_pair[beside]);
+  if (rc) return rc;
+  mla_pair::Params p{m, int(int64_t(R) * (m.H / mla_pair::kHeads) * m.nsplit)};
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(2 * unsigned(std::min(p.items, std::max(1, sm_count() / 2))));
+  cfg.blockDim = dim3(mla_pair::kThreads);
+  cfg.dynamicSmemBytes = mla_pair::Smem::bytes;
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  DSA_CUDA(cudaLaunchKernelEx(&cfg, kernel, kv_map, q_map, out_map, p));
+  return DSA_OK;
+}
+
 static int mla_partials_launch(const void* q, const void* kv, const int32_t* indices,
                                const int32_t* seq_lens, float* part_acc, float* part_m, float* part_l,
                                void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale,
@@ -957,6 +996,19 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
   const int64_t tc_tiles = int64_t(R) * (H / mla_tc::kHG) * ((topk_k + mla_tc::kBN - 1) / mla_tc::kBN);
   if (H % mla_tc::kHG == 0 && sm_scale > 0.f && tc_tiles >= mla_tc::kMinTiles) {
     int kps = (topk_k + nsplit - 1) / nsplit;
+    // 128 heads on a pair of CTAs where a split has four of its 128-key tiles, or where the pairs take several splits each
+    // (us, pair / one CTA per 64 heads, 128 heads, the default split count): 16 rows x 2048 keys in 4 splits 23.2 / 24.8, 32 in
+    // 2 34.8 / 41.1, 40 in 1 41.4 / 59.5, 200 x 1024 64.3 / 95.1, 40 x 512 17.2 / 19.6, 96 x 256 21.3 / 24.7, 96 x 128 16.7 / 17.2.
+    // Not below, where the start and the end of a pair outweigh its products: 8 rows x 2048 in 8 splits 17.6 / 16.9, 4 in 16
+    // 16.2 / 14.3, 16 x 1024 in 4 19.0 / 18.1, 64 x 256 13.3 / 13.0, 64 x 128 11.0 / 9.2.
+    const int64_t pair_items = int64_t(R) * (H / mla_pair::kHeads) * nsplit;
+    const bool pair_pays = kps >= 4 * mla_pair::kBN || pair_items > sm_count() / 2;
+    // (the rows of cache, queries, result and partials are coordinates of tensor maps)
+    const bool pair_fits = R / rows_per_seq * kv_seq_stride < (int64_t(1) << 31) && int64_t(R) * H * nsplit < (int64_t(1) << 31);
+    if (H % mla_pair::kHeads == 0 && !kv_fp8 && pair_pays && pair_fits) {
+      p.keys_per_split = (kps + mla_pair::kBN - 1) / mla_pair::kBN * mla_pair::kBN;
+      return launch_mla_pair(p, R, beside, st);
+    }
     p.keys_per_split = (kps + mla_tc::kBN - 1) / mla_tc::kBN * mla_tc::kBN;
     auto kernel = beside ? mla_tc::sparse_mla_tc_kernel<true> : mla_tc::sparse_mla_tc_kernel<false>;
     int rc = opt_in_smem(kernel, mla_tc::Smem::bytes, g_opt_mla_tc[beside]);

@@ -1,0 +1,152 @@
+"""GPU tests of the sparse MLA kernel that runs 128 heads on a pair of CTAs (bf16 rows), at the sizes where it can go wrong:
+a tile's last keys, one tile, several triples per pair, splits of unequal length, masked entries at either end of the list,
+scores that run away from the softmax reference.
+
+Tolerance, relative 2-norm against the same computation in 64 bits: probabilities and results are rounded to bf16, at most
+2^-9 each, and their errors add up like the values themselves: 2 x 2^-9 = 3.9e-3, and 5e-3 with what the 32-bit sums add.
+"""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+TOL = 5e-3
+SM = 192 ** -0.5
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from dsa_multi_layer_indexer_b200 import _lib, ops as _ops
+
+    _lib.lib()
+    yield _ops
+    _lib.check_device_status()
+
+
+def reference(q, kv, idx, lens, rows_per_seq):
+    out = torch.zeros(*q.shape[:2], 512, dtype=torch.float64, device=q.device)
+    for r in range(q.shape[0]):
+        i = idx[r].long()
+        i = i[(i >= 0) & (i < int(lens[r]))]
+        if i.numel():
+            k = kv[r // rows_per_seq][i].double()
+            out[r] = torch.softmax(q[r].double() @ k.T * SM, -1) @ k[:, :512]
+    return out
+
+
+def operands(R, H, n, topk, rows_per_seq=1, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    q = torch.randn(R, H, 576, device="cuda", generator=gen).bfloat16()
+    kv = torch.randn(R // rows_per_seq, n, 576, device="cuda", generator=gen).bfloat16()
+    idx = torch.full((R, topk), -1, dtype=torch.int32, device="cuda")
+    take = min(n, topk)
+    for r in range(R):
+        idx[r, :take] = torch.randperm(n, device="cuda", generator=gen)[:take].sort().values.int()
+    return q, kv, idx, torch.full((R,), n, dtype=torch.int32, device="cuda")
+
+
+def check(ops, q, kv, idx, lens, rows_per_seq, nsplit):
+    from dsa_multi_layer_indexer_b200 import _lib
+
+    got = ops.sparse_mla_decode(q, kv, idx, SM, lens, rows_per_seq=rows_per_seq, nsplit=nsplit)
+    _lib.check_device_status()
+    want = reference(q, kv, idx, lens, rows_per_seq)
+    assert torch.isfinite(got).all()
+    for r in range(q.shape[0]):
+        norm = float(want[r].norm())
+        assert float((got[r].double() - want[r]).norm()) <= TOL * norm, r
+        if norm == 0.0:
+            assert float(got[r].abs().max()) == 0.0
+
+
+# (rows, heads, keys, list, splits): one split of 4 tiles, with a last tile of 1, 64, 65 and 127 keys; one tile of few keys
+# and two in which more triples than pairs exist; splits of which the last is short; several head blocks; several triples
+# a pair of very different length
+@pytest.mark.parametrize("R,H,n,topk,nsplit,rows_per_seq", [
+    (8, 128, 3000, 512, 1, 1), (8, 128, 700, 513, 1, 2), (8, 128, 600, 576, 1, 8), (4, 256, 900, 577, 1, 4), (8, 128, 700, 639, 1, 1),
+    (150, 128, 40, 40, 1, 150), (76, 128, 300, 64, 1, 76), (100, 128, 300, 129, 1, 100), (20, 512, 300, 200, 1, 1),
+    (3, 128, 5000, 2048, 3, 1), (40, 128, 500, 129, 2, 1), (6, 384, 3000, 1100, 2, 3), (160, 128, 2100, 2048, 1, 160)])
+def test_against_64_bits(ops, R, H, n, topk, nsplit, rows_per_seq):
+    q, kv, idx, lens = operands(R, H, n, topk, rows_per_seq, seed=R + topk)
+    check(ops, q, kv, idx, lens, rows_per_seq, nsplit)
+
+
+@pytest.mark.parametrize("nsplit", [1, 3])
+def test_masked_entries_and_rows(ops, nsplit):
+    R, n, topk = 90, 2500, 1600
+    q, kv, idx, lens = operands(R, 128, n, topk, seed=5)
+    idx[:, ::17] = n + 5           # beyond the sequence
+    idx[:, 3::29] = -1
+    lens[1], lens[2] = 0, 1
+    idx[3] = -1
+    idx[4, :-3] = -1               # only the list's end
+    idx[5, 1:] = -1                # only its start
+    idx[6, :64] = -1               # the reference comes from the tile's other half,
+    idx[7, :130] = -1              # from the next tile
+    idx[8, 200:1400] = -1          # tiles without a key in between
+    for r in range(9, 40):         # lengths as those of a prompt
+        idx[r, 40 * (r - 8):] = -1
+    check(ops, q, kv, idx, lens, 1, nsplit)
+
+
+def test_scores_that_run_away(ops):
+    R, n, topk = 8, 2048, 2048
+    q, kv, idx, lens = operands(R, 128, n, topk, seed=9)
+    grow = torch.linspace(0.01, 3, n, device="cuda")[None, :, None]
+    q = (q.float() * 60).bfloat16()
+    kv = (kv.float() * grow).bfloat16()
+    kv[3] = kv[3].flip(0)          # largest first
+    kv[4, :64] *= 0.001            # the first half of the first tile is far below the second
+    check(ops, q, kv, idx, lens, 1, 1)
+    check(ops, q, kv, idx, lens, 1, 2)
+
+
+def test_no_list_attends_every_key(ops):
+    from dsa_multi_layer_indexer_b200 import _lib
+
+    q, kv, _, _ = operands(8, 128, 1000, 8, seed=3)
+    lens = torch.tensor([1000, 999, 513, 1, 0, 128, 129, 700], dtype=torch.int32, device="cuda")
+    got = ops.sparse_mla_decode(q, kv, None, SM, lens, nsplit=1, dense_keys=1000)
+    _lib.check_device_status()
+    every = torch.arange(1000, dtype=torch.int32, device="cuda").expand(8, -1)
+    want = reference(q, kv, every, lens, 1)
+    assert float((got.double() - want).norm()) <= TOL * float(want.norm())
+    assert float(got[4].abs().max()) == 0.0
+
+
+def test_agrees_with_one_cta_per_64_heads(ops):
+    """64 heads at a time run on the other kernel: the same reference, the same rounded probabilities and products added in
+    the same order, so only the row sums' order can round a result the other way."""
+    q, kv, idx, lens = operands(40, 128, 3000, 2048, seed=7)
+    both = ops.sparse_mla_decode(q, kv, idx, SM, lens, nsplit=1)
+    for h in (0, 64):
+        half = ops.sparse_mla_decode(q[:, h:h + 64].contiguous(), kv, idx, SM, lens, nsplit=1)
+        same = both[:, h:h + 64]
+        assert float((same != half).float().mean()) < 0.01
+        assert float((same.float() - half.float()).norm()) <= 2.0 ** -9 * float(half.float().norm())
+
+
+def test_several_launches_in_a_graph_and_on_two_streams(ops):
+    from dsa_multi_layer_indexer_b200 import _lib
+
+    a = operands(90, 128, 900, 600, 90, seed=1)
+    b = operands(90, 128, 900, 600, 90, seed=2)
+    run = lambda o: ops.sparse_mla_decode(*o[:3], SM, o[3], rows_per_seq=90, nsplit=1)
+    want = [run(a), run(b)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = [run(a), run(b), run(a)]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and torch.equal(got[2], want[0])
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        other = run(b)
+    mine = run(a)
+    torch.cuda.synchronize()
+    assert torch.equal(mine, want[0]) and torch.equal(other, want[1])
+    _lib.check_device_status()
