@@ -1,4 +1,4 @@
-// Sparse MLA of 128 heads on a pair of CTAs (tcgen05 with cta_group::2), bf16 rows.
+// Sparse MLA of 128 heads, or of two rows' 64, on a pair of CTAs (tcgen05 with cta_group::2), bf16 rows.
 //
 // Same contract and the same partials as sparse_mla_tc.cuh. A persistent pair takes (row, 128 heads, split) triples in
 // turn; 128-key tiles, 64 heads in each CTA:
@@ -33,6 +33,12 @@
 // Tried: registers moved to the softmax warps by setmaxnreg (it needs whole groups of four warps; not needed since), two
 // softmax groups on alternate tiles (564 us: longer in total, and not what a tile waits for), eight gather warps (539).
 //
+// kTwoRows: 64 heads. Neighbouring rows of a prompt that is no longer than the list attend the same keys, the second one
+// its own as well: two rows' heads fill the pair's 128, with one list and each row's own view of what is masked. The plan
+// compares the two lists entry by entry; rows that do not nest, or whose one key more is not finite, go through their
+// own list alone, with the other CTA's result dropped. Prompt of 700 tokens 82 -> 65 us, 2048 465 -> 331 (four passes over
+// each list with a few loads under way instead of one with sixteen: 127 us, the plan was what everything waited for).
+//
 // Warps (864 threads): 0-7 softmax, queries to tensor memory, result; 8 products (in CTA 0); 9 plans the triples and loads
 // the rest of the queries; 10-25 gather; 26 lays out a tile's rows and gathers its last chunk.
 #pragma once
@@ -59,6 +65,7 @@ constexpr uint32_t kColQ = 320;                // Q: kQTmem x 32 columns
 constexpr int kLists = 4;                      // tiles whose rows are laid out
 constexpr int kPlan = 4;                       // entries of the plan ring
 constexpr float kRescaleLog2 = mla_tc::kRescaleLog2;
+enum { kBoth = 0, kFirst = 1, kSecond = 2 };  // rows of a plan entry
 constexpr float kAway = 1099511627776.f;       // 2^40: a tile's sum above it asks for another softmax reference
 
 // The first kNumPolled are what the MMA warp waits for.
@@ -178,7 +185,7 @@ struct Params {
   int items;  // (row, block of 128 heads, split) triples
 };
 
-template <bool kBeside>
+template <bool kBeside, bool kTwoRows>
 __global__ void __launch_bounds__(kThreads, 1)
 sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap out_map, const Params pp) {
   const mla::Params& p = pp.m;
@@ -223,27 +230,37 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
   if constexpr (!kBeside) pdl_wait();
   pdl_launch_dependents();
 
-  const int hps = p.H / kHeads;
-  struct Item { int r, hp, split, k_begin, k_end; };
+  // r: the row (kTwoRows: the first of two rows, the second CTA has the other), heads0: this CTA's 64 heads among all rows'
+  const int hps = kTwoRows ? 1 : p.H / kHeads;
+  struct Item { int r, split, k_begin, k_end; int64_t heads0; bool second; };
   auto item_of = [&](int i) {
     Item it;
     it.split = i % p.nsplit;
-    const int u = i / p.nsplit;
-    it.hp = u % hps;
-    it.r = pp.items / (p.nsplit * hps) - 1 - u / hps;  // last rows first: those of a prompt grow
+    int u = pp.items / p.nsplit - 1 - i / p.nsplit;  // last rows first: those of a prompt grow
+    it.second = true;
+    if constexpr (kTwoRows) {
+      const int per_seq = (p.rows_per_seq + 1) / 2, seq = u / per_seq;
+      u -= seq * per_seq;
+      it.r = seq * p.rows_per_seq + 2 * u;
+      it.second = 2 * u + 1 < p.rows_per_seq;
+      it.heads0 = (int64_t(it.r) + rank) * 64;
+    } else {
+      it.r = u / hps;
+      it.heads0 = int64_t(it.r) * p.H + u % hps * kHeads + rank * 64;
+    }
     it.k_begin = it.split * p.keys_per_split;
     it.k_end = min(it.k_begin + p.keys_per_split, p.topk);
     return it;
   };
   bool failed = false;
-  // the plan's entry n: item (-1: no more), tiles, length
+  // the plan's entry n: item (-1: no more), tiles, length of the row whose list counts, which rows (kBoth, kFirst, kSecond)
   auto next_plan = [&](int n, int4& e) {
     if (__any_sync(0xffffffffu, !mbar_wait(bar(kBarPlan + (n & (kPlan - 1))), (n / kPlan) & 1))) {
       failed = true;
       return false;
     }
     e = s_plan[n & (kPlan - 1)];
-    e.x = __shfl_sync(0xffffffffu, e.x, 0), e.y = __shfl_sync(0xffffffffu, e.y, 0), e.z = __shfl_sync(0xffffffffu, e.z, 0);
+    e.x = __shfl_sync(0xffffffffu, e.x, 0), e.y = __shfl_sync(0xffffffffu, e.y, 0), e.z = __shfl_sync(0xffffffffu, e.z, 0), e.w = __shfl_sync(0xffffffffu, e.w, 0);
     return e.x >= 0;
   };
 
@@ -389,14 +406,17 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
       const float l = (s_sum[head] + s_sum[64 + head]) + (s_sum[128 + head] + s_sum[192 + head]);
       const float inv = l > 0.f ? 1.f / l : 0.f;
       // (the item is read again: kept over the tiles, its numbers would cost registers)
-      const Item done = item_of(*reinterpret_cast<volatile int*>(smem + Smem::plan_off + 16 * (n & (kPlan - 1))));
-      const int64_t hrow = int64_t(done.r) * p.H + done.hp * kHeads + rank * 64;
-      const int64_t pb = (int64_t(done.r) * p.nsplit + done.split) * p.H + done.hp * kHeads + rank * 64;
+      const volatile int* entry = reinterpret_cast<volatile int*>(smem + Smem::plan_off + 16 * (n & (kPlan - 1)));
+      const Item done = item_of(entry[0]);
+      const bool mine = !kTwoRows || entry[3] == kBoth || entry[3] == kFirst + rank;  // (else the other row's list went through)
+      // first of this CTA's 64 rows of partials: [row][split][head]
+      const int64_t pb = kTwoRows ? ((int64_t(done.r) + rank) * p.nsplit + done.split) * 64
+                                  : (int64_t(done.r) * p.nsplit + done.split) * p.H + (done.heads0 - int64_t(done.r) * p.H);
       // 64 bytes of 32 rows at a time through this warp's 2 KB of the probabilities' place and out by TMA. (Stored straight
       // from the lanes, whose rows are a kilobyte or two apart, an instruction takes as many cycles as it has lanes: 5700
       // cycles an item.)
       const uint32_t s_stage = s_p + uint32_t(warp) * 2048u;
-      const int srow = int((p.out ? hrow : pb) + (quad & 1) * 32);
+      const int srow = int((p.out ? done.heads0 : pb) + (quad & 1) * 32);
       auto put = [&](const uint32_t (&w)[16], int col) {
         if (lane == 0) bulk_wait_read();
         __syncwarp();
@@ -405,7 +425,7 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
           st_shared_v4(s_stage + uint32_t(lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)), make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]));
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) tma_store_2d(s_stage, &out_map, col, srow);
+        if (lane == 0 && mine) tma_store_2d(s_stage, &out_map, col, srow);
       };
 #pragma unroll 1
       for (int blk = 4 * group; blk < 4 * group + 4; ++blk) {
@@ -431,7 +451,7 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
       tc_fence_before();
       __syncwarp();
       if (lane == 0) arrive_at(leader_bar(kBarOFree));
-      if (!p.out && part == 0) {
+      if (!p.out && part == 0 && mine) {
         p.part_m[pb + head] = m_ref;
         p.part_l[pb + head] = l;
       }
@@ -445,66 +465,134 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
       const bool leader = elect_one();
       int n = 0;
       // entry n; the one in its place has been read by all, since the last score product of item n - 2 is done
-      auto publish = [&](int item, int tiles, int len) {
+      auto publish = [&](int item, int tiles, int len, int rows) {
         if (leader) {
-          *reinterpret_cast<int4*>(smem + Smem::plan_off + 16 * (n & (kPlan - 1))) = make_int4(item, tiles, len, 0);
+          *reinterpret_cast<int4*>(smem + Smem::plan_off + 16 * (n & (kPlan - 1))) = make_int4(item, tiles, len, rows);
           mbar_arrive(bar(kBarPlan + (n & (kPlan - 1))));
         }
         __syncwarp();
       };
-      for (int k = 0; k * clusters < pp.items; ++k) {
-        // clusters take items in turn, every other time in reverse: the longer rows are spread over all
-        const int i = k * clusters + ((k & 1) ? clusters - 1 - cid : cid);
-        if (i >= pp.items) continue;
-        const Item it = item_of(i);
-        const int32_t* list = p.indices ? p.indices + int64_t(it.r) * p.topk : nullptr;
-        int last = -1;  // the list's last entries, on their way together with the length
-        if (list && it.k_end - 32 + lane >= it.k_begin) last = list[it.k_end - 32 + lane];
-        int64_t len64 = p.seq_lens ? int64_t(p.seq_lens[it.r]) : p.ctx;
-        len64 = len64 < 0 ? 0 : (len64 > p.ctx ? p.ctx : len64);
-        const int len = int(len64);
-        int bound = min(it.k_end, len);
-        if (list) {  // end of the last visible key, from the list's end
-          bound = __reduce_max_sync(0xffffffffu, last >= 0 && last < len ? it.k_end - 31 + lane : 0);
-          for (int j0 = it.k_end - 32; j0 > it.k_begin && bound == 0; j0 -= 512) {
+      auto list_of = [&](int r) { return p.indices ? p.indices + int64_t(r) * p.topk : nullptr; };
+      auto length_of = [&](int r) {
+        const int64_t len = p.seq_lens ? int64_t(p.seq_lens[r]) : p.ctx;
+        return int(len < 0 ? 0 : (len > p.ctx ? p.ctx : len));
+      };
+      // where the last visible key of row r's part of the list ends; `last`: the list's last entries, requested together with the length
+      auto tail_of = [&](const Item& it, int r) {
+        const int32_t* list = list_of(r);
+        return list && it.k_end - 32 + lane >= it.k_begin ? list[it.k_end - 32 + lane] : -1;
+      };
+      auto bound_of = [&](const Item& it, int r, int len, int last) {
+        const int32_t* list = list_of(r);
+        if (!list) return min(it.k_end, len);
+        int bound = __reduce_max_sync(0xffffffffu, last >= 0 && last < len ? it.k_end - 31 + lane : 0);
+        for (int j0 = it.k_end - 32; j0 > it.k_begin && bound == 0; j0 -= 512) {
 #pragma unroll 4
-            for (int c = 0; c < 16; ++c) {
-              const int j = j0 - 32 * (c + 1) + lane;
-              if (j >= it.k_begin) {
-                const int idx = list[j];
-                if (idx >= 0 && idx < len) bound = max(bound, j + 1);
-              }
+          for (int c = 0; c < 16; ++c) {
+            const int j = j0 - 32 * (c + 1) + lane;
+            if (j >= it.k_begin) {
+              const int idx = list[j];
+              if (idx >= 0 && idx < len) bound = max(bound, j + 1);
             }
-            bound = __reduce_max_sync(0xffffffffu, bound);
+          }
+          bound = __reduce_max_sync(0xffffffffu, bound);
+        }
+        return bound;
+      };
+      // kTwoRows: the bounds of both rows, and whether they nest: row r's visible keys are row r + 1's, in the same places, but
+      // for one at most, and that one's value is finite. Then both go through the second one's list together. (The first row's
+      // probability of the key is zero, and zero times an infinity would not be.) One pass over both lists, 16 loads under way.
+      auto survey = [&](const Item& it, int len0, int len1, int& bound0, int& bound1) {
+        const int32_t *list0 = list_of(it.r), *list1 = list_of(it.r + (it.second ? 1 : 0));
+        int extras = 0, extra = -1;
+        bool same = true;
+        bound0 = bound1 = 0;
+#pragma unroll 1
+        for (int j0 = it.k_begin; j0 < it.k_end; j0 += 256) {
+          int i0[8], i1[8];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const int j = j0 + 32 * c + lane;
+            i0[c] = i1[c] = -1;
+            if (j < it.k_end) i0[c] = list0 ? list0[j] : j, i1[c] = list1 ? list1[j] : j;
+          }
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const int j = j0 + 32 * c + lane;
+            const bool see0 = i0[c] >= 0 && i0[c] < len0, see1 = i1[c] >= 0 && i1[c] < len1;
+            if (see0) bound0 = j + 1;
+            if (see1) bound1 = j + 1;
+            if (see0 && !(see1 && i0[c] == i1[c])) same = false;
+            if (see1 && !see0) ++extras, extra = i1[c];
           }
         }
-        const int tiles = (max(bound - it.k_begin, 0) + kBN - 1) / kBN;
-        const int head0 = it.hp * kHeads + rank * 64;
-        if (tiles == 0) {  // nothing visible: nobody else hears of it
-          const uint4 zero = make_uint4(0, 0, 0, 0);
-          if (p.out) {
-            uint4* dst = reinterpret_cast<uint4*>(p.out + (int64_t(it.r) * p.H + head0) * mla::kDV);
-            for (int j = lane; j < 64 * mla::kDV / 8; j += 32) dst[j] = zero;
-          } else {
-            const int64_t pb = (int64_t(it.r) * p.nsplit + it.split) * p.H + head0;
-            uint4* dst = reinterpret_cast<uint4*>(p.part_acc + pb * mla::kDV);
-            for (int j = lane; j < 64 * mla::kDV / 4; j += 32) dst[j] = zero;
-            for (int j = lane; j < 64; j += 32) p.part_m[pb + j] = -INFINITY, p.part_l[pb + j] = 0.f;
+        bound0 = __reduce_max_sync(0xffffffffu, bound0), bound1 = __reduce_max_sync(0xffffffffu, bound1);
+        if (!__all_sync(0xffffffffu, same) || __reduce_add_sync(0xffffffffu, extras) > 1) return false;
+        extra = __reduce_max_sync(0xffffffffu, extra);
+        bool finite = true;
+        if (extra >= 0) {
+          const uint8_t* row = p.kv + (int64_t(it.r / p.rows_per_seq) * p.kv_seq_stride + extra) * mla::kRowBytes;
+#pragma unroll
+          for (int c = 0; c < mla::kDV / 64; ++c) {  // (two value dims a word; the others do not enter the value product)
+            const uint32_t w = reinterpret_cast<const uint32_t*>(row)[32 * c + lane];
+            finite = finite && (w & 0x7F80u) != 0x7F80u && (w & 0x7F800000u) != 0x7F800000u;
           }
-          continue;
         }
-        publish(i, tiles, len);
-        if (n >= 1 && __any_sync(0xffffffffu, !mbar_wait(bar(kBarQFree), (n - 1) & 1))) { failed = true; break; }
+        return __all_sync(0xffffffffu, finite) && bound1 > it.k_begin;
+      };
+      auto store_zeros = [&](const Item& it) {  // nothing visible: the plan does not mention the row
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        if (p.out) {
+          uint4* dst = reinterpret_cast<uint4*>(p.out + it.heads0 * mla::kDV);
+          for (int j = lane; j < 64 * mla::kDV / 8; j += 32) dst[j] = zero;
+        } else {
+          const int64_t pb = kTwoRows ? ((int64_t(it.r) + rank) * p.nsplit + it.split) * 64
+                                      : (int64_t(it.r) * p.nsplit + it.split) * p.H + (it.heads0 - int64_t(it.r) * p.H);
+          uint4* dst = reinterpret_cast<uint4*>(p.part_acc + pb * mla::kDV);
+          for (int j = lane; j < 64 * mla::kDV / 4; j += 32) dst[j] = zero;
+          for (int j = lane; j < 64; j += 32) p.part_m[pb + j] = -INFINITY, p.part_l[pb + j] = 0.f;
+        }
+      };
+      auto tiles_of = [&](const Item& it, int bound) { return (max(bound - it.k_begin, 0) + kBN - 1) / kBN; };
+      // puts an item into the plan and requests the rest of its queries
+      auto enter = [&](int i, const Item& it, int tiles, int len, int rows) {
+        publish(i, tiles, len, rows);
+        if (n >= 1 && __any_sync(0xffffffffu, !mbar_wait(bar(kBarQFree), (n - 1) & 1))) return !(failed = true);
         if (leader) {
           if (rank == 0) mbar_arrive_expect_tx(bar(kBarQ), 2 * (9 - kQTmem) * kChunkBytes);
           const uint32_t at = leader_bar(kBarQ);
           for (int c = kQTmem; c < 9; ++c)
-            tma_load_2d_pair(s_q + uint32_t(c - kQTmem) * kChunkBytes, &q_map, c * 64, it.r * p.H + head0, at);
+            tma_load_2d_pair(s_q + uint32_t(c - kQTmem) * kChunkBytes, &q_map, c * 64, int(it.heads0), at);
         }
         __syncwarp();
         ++n;
+        return true;
+      };
+      for (int k = 0; k * clusters < pp.items && !failed; ++k) {
+        // clusters take items in turn, every other time in reverse: the longer rows are spread over all
+        const int i = k * clusters + ((k & 1) ? clusters - 1 - cid : cid);
+        if (i >= pp.items) continue;
+        const Item it = item_of(i);
+        const int last = kTwoRows ? 0 : tail_of(it, it.r);
+        const int len = length_of(it.r), len1 = kTwoRows && it.second ? length_of(it.r + 1) : 0;
+        if constexpr (kTwoRows) {
+          int bound, bound1;
+          if (survey(it, len, len1, bound, bound1)) {
+            if (!enter(i, it, tiles_of(it, bound1), len1, kBoth)) break;
+            continue;
+          }
+          for (int row = 0; row < (it.second ? 2 : 1) && !failed; ++row) {
+            const int tiles = tiles_of(it, row ? bound1 : bound);
+            if (tiles > 0) enter(i, it, tiles, row ? len1 : len, row ? kSecond : kFirst);
+            else if (rank == row) store_zeros(it);
+          }
+        } else {
+          const int tiles = tiles_of(it, bound_of(it, it.r, len, last));
+          if (tiles > 0) enter(i, it, tiles, len, kBoth);
+          else store_zeros(it);
+        }
       }
-      if (!failed) publish(-1, 0, 0);
+      if (!failed) publish(-1, 0, 0, kBoth);
     } else if (warp >= kGatherWarp0) {
       // ===================================================================== gather
       // Four warps bring unit j of a tile's keys and unit j of its values, 32 rows of one chunk each. The seventeenth lays out
@@ -548,7 +636,7 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
               mbar_arrive_expect_tx(bar(kBarQStage), kUnitBytes);
               for (int c = 0; c < 2; ++c)
                 tma_load_2d(s_ring + uint32_t(at.slot) * kUnitBytes + uint32_t(c) * kChunkBytes, &q_map, 128 * quad + 64 * c,
-                            it.r * p.H + it.hp * kHeads + rank * 64, bar(kBarQStage));
+                            int(it.heads0), bar(kBarQStage));
             }
             __syncwarp();
           }
@@ -566,8 +654,16 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
           // The rows of a tile for everybody, once the products of the scores two tiles before are done: the value product four
           // tiles before, the last to need the place's rows, was issued before those. Then the tile's last chunk.
           const int64_t seq_row = int64_t(it.r / p.rows_per_seq) * p.kv_seq_stride;
-          const int32_t* list = p.indices ? p.indices + int64_t(it.r) * p.topk : nullptr;
-          auto load = [&](int t, int (&idx)[4]) {
+          // kTwoRows: both CTAs go through one list, but the first CTA's row sees what its own list says
+          const int lrow = it.r + (kTwoRows && e.w != kFirst ? 1 : 0);
+          const bool own = kTwoRows && e.w == kBoth && rank == 0;
+          int own_len = 0;
+          if (own) {
+            const int64_t len = p.seq_lens ? int64_t(p.seq_lens[it.r]) : p.ctx;
+            own_len = int(len < 0 ? 0 : (len > p.ctx ? p.ctx : len));
+          }
+          auto load = [&](int r, int t, int (&idx)[4]) {
+            const int32_t* list = p.indices ? p.indices + int64_t(r) * p.topk : nullptr;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const int j = it.k_begin + t * kBN + 32 * i + lane;
@@ -575,22 +671,24 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
               if (t < e.y && j < it.k_end) idx[i] = list ? list[j] : j;
             }
           };
-          int idx[4];
-          load(0, idx);
+          int idx[4], mine[4];
+          load(lrow, 0, idx);
+          if (own) load(it.r, 0, mine);
           for (int t = 0; t < e.y && !failed; ++t) {
             const int u = gt + t, b = u & 1, l = u & (kLists - 1);
             if (__any_sync(0xffffffffu, !mbar_wait(bar(kBarRopeFree + b), ((u >> 1) & 1) ^ 1))) { failed = true; break; }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const bool ok = idx[i] >= 0 && idx[i] < e.z;
-              const uint32_t seen = __ballot_sync(0xffffffffu, ok);
+              const uint32_t seen = __ballot_sync(0xffffffffu, own ? mine[i] >= 0 && mine[i] < own_len : ok);
               *reinterpret_cast<volatile int*>(smem + Smem::list_off + (l * kBN + 32 * i + lane) * 4) = ok ? int(seq_row + idx[i]) : -1;
               if (lane == 0) *reinterpret_cast<volatile uint32_t*>(smem + Smem::seen_off + (l * 4 + i) * 4) = seen;
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(kBarList + l));
             if (rank == 0 && leader) mbar_arrive_expect_tx(bar(kBarRope + b), 2 * kChunkBytes);
-            load(t + 1, idx);
+            load(lrow, t + 1, idx);
+            if (own) load(it.r, t + 1, mine);
             gather(s_rope + uint32_t(b) * kChunkBytes, 512, leader_bar(kBarRope + b), u, 64 * rank);
             gather(s_rope + uint32_t(b) * kChunkBytes + kChunkBytes / 2, 512, leader_bar(kBarRope + b), u, 64 * rank + 32);
           }

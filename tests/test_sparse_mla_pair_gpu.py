@@ -150,3 +150,64 @@ def test_several_launches_in_a_graph_and_on_two_streams(ops):
     torch.cuda.synchronize()
     assert torch.equal(mine, want[0]) and torch.equal(other, want[1])
     _lib.check_device_status()
+
+
+# ---- 64 heads: two rows of a prompt on a pair, where the second row sees what the first one sees and one key more
+def prompt(batch, n, topk, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    q = torch.randn(batch * n, 64, 576, device="cuda", generator=gen).bfloat16()
+    kv = torch.randn(batch, n, 576, device="cuda", generator=gen).bfloat16()
+    pos = torch.arange(topk, dtype=torch.int32, device="cuda")
+    row = torch.arange(n, dtype=torch.int32, device="cuda")
+    idx = torch.where(pos[None] <= row[:, None], pos[None], -1).repeat(batch, 1).contiguous()
+    return q, kv, idx, (row + 1).repeat(batch)
+
+
+@pytest.mark.parametrize("batch,n,topk", [(1, 256, 256), (1, 257, 300), (2, 193, 193), (3, 200, 256), (1, 385, 385), (1, 700, 703)])
+def test_two_rows_of_a_prompt(ops, batch, n, topk):
+    check(ops, *prompt(batch, n, topk, seed=n), n, 1)
+
+
+def test_two_rows_that_differ(ops):
+    """Lists that do not nest, rows of which one or both see nothing, lengths that shrink: row by row then."""
+    n = 260
+    q, kv, idx, lens = prompt(1, n, 400, seed=4)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    for r in range(20, 60):                                    # unrelated lists
+        idx[r] = -1
+        idx[r, :100] = torch.randperm(n, device="cuda", generator=gen)[:100].int()
+        lens[r] = n
+    idx[60, :3] = torch.tensor([2, 0, 1], dtype=torch.int32)   # the second row's list in another order
+    idx[70] = -1
+    idx[73] = -1
+    idx[74:76] = -1
+    lens[80] = 0
+    lens[83] = 5                                               # shorter than the row before it
+    idx[85, 84:90] = torch.tensor([84, 85, 86, 87, 88, 89], dtype=torch.int32)  # more than one key more
+    lens[85] = n
+    idx[90, 10] = -1                                           # the first row misses one in the middle,
+    idx[93, 10] = -1                                           # the second one does
+    check(ops, q, kv, idx, lens, n, 1)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("dim", [0, 511, 512])
+def test_a_key_that_is_not_finite_stays_out_of_the_rows_before_it(ops, bad, dim):
+    n, at = 256, 101  # the second row of its pair
+    q, kv, idx, lens = prompt(1, n, n, seed=6)
+    clean = ops.sparse_mla_decode(q, kv, idx, SM, lens, rows_per_seq=n, nsplit=1).clone()
+    kv[0, at, dim] = bad
+    got = ops.sparse_mla_decode(q, kv, idx, SM, lens, rows_per_seq=n, nsplit=1)
+    assert torch.equal(got[:at], clean[:at])
+    assert not torch.isfinite(got[at:]).all()
+
+
+def test_two_rows_agree_with_one_at_a_time(ops):
+    n = 640
+    q, kv, idx, lens = prompt(1, n, n, seed=8)
+    both = ops.sparse_mla_decode(q, kv, idx, SM, lens, rows_per_seq=n, nsplit=1)
+    for r in range(0, n, 80):  # (fewer rows run on the other kernel)
+        some = slice(r, r + 80)
+        alone = ops.sparse_mla_decode(q[some].contiguous(), kv, idx[some].contiguous(), SM, lens[some].contiguous(), rows_per_seq=80, nsplit=1)
+        assert float((both[some] != alone).float().mean()) < 0.01
+        assert float((both[some].float() - alone.float()).norm()) <= 2.0 ** -9 * float(alone.float().norm())
