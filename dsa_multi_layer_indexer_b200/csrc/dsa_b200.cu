@@ -1000,18 +1000,18 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
   const int64_t tc_tiles = int64_t(R) * (H / mla_tc::kHG) * ((topk_k + mla_tc::kBN - 1) / mla_tc::kBN);
   if (H % mla_tc::kHG == 0 && sm_scale > 0.f && tc_tiles >= mla_tc::kMinTiles) {
     int kps = (topk_k + nsplit - 1) / nsplit;
-    // 128 heads on a pair of CTAs where a split has four of its 128-key tiles, or where the pairs take several splits each
-    // (us, pair / one CTA per 64 heads, 128 heads, the default split count): 16 rows x 2048 keys in 4 splits 23.2 / 24.8, 32 in
-    // 2 34.8 / 41.1, 40 in 1 41.4 / 59.5, 200 x 1024 64.3 / 95.1, 40 x 512 17.2 / 19.6, 96 x 256 21.3 / 24.7, 96 x 128 16.7 / 17.2.
-    // Not below, where the start and the end of a pair outweigh its products: 8 rows x 2048 in 8 splits 17.6 / 16.9, 4 in 16
-    // 16.2 / 14.3, 16 x 1024 in 4 19.0 / 18.1, 64 x 256 13.3 / 13.0, 64 x 128 11.0 / 9.2.
+    // 128 heads on a pair of CTAs where a split has four of its 128-key tiles, the only split two, or where the pairs take several
+    // splits each (us, pair / one CTA per 64 heads, 128 heads, the default split count): 16 rows x 2048 keys in 4 splits
+    // 21.9 / 24.8, 32 in 2 32.7 / 41.1, 40 in 1 38.4 / 59.5, 200 x 1024 59.0 / 95.1, 40 x 512 15.8 / 19.6, 40 x 256 11.9 / 12.9,
+    // 96 x 128 16.0 / 17.2. Not below, where the start and the end of a pair weigh as much as its products: 8 rows x 2048 in 8
+    // splits 16.8 / 16.9, 4 in 16 16.0 / 14.3, 16 x 1024 in 4 18.3 / 18.1, 32 x 512 in 2 21.5 / 21.5, 64 x 128 10.6 / 9.2.
     const int64_t pair_items = int64_t(R) * (H / mla_pair::kHeads) * nsplit;
-    const bool pair_pays = kps >= 4 * mla_pair::kBN || pair_items > sm_count() / 2;
+    const bool pair_pays = kps >= (nsplit == 1 ? 2 : 4) * mla_pair::kBN || pair_items > sm_count() / 2;
     // (the rows of cache, queries, result and partials are coordinates of tensor maps)
     const bool pair_fits = R / rows_per_seq * kv_seq_stride < (int64_t(1) << 31) && int64_t(R) * H * nsplit < (int64_t(1) << 31);
     // Two rows of 64 heads on a pair for a prompt that is no longer than the list: neighbouring rows then attend the same keys
-    // but one (us, pair / one CTA a row: prompts of 256 tokens 20.3 / 20.8, 700 65 / 82, 2048 331 / 465, two of 200 28.4 / 29.0;
-    // 220 19.4 / 18.6, two of 150 24.3 / 23.7). What tells a prompt: many rows of one sequence, a length for each, and a list
+    // but one (us, pair / one CTA a row: prompts of 256 tokens 19.4 / 20.8, 700 61 / 82, 2048 320 / 465, two of 200 26.7 / 29.0;
+    // 220 18.7 / 18.6, two of 150 23.8 / 23.7). What tells a prompt: many rows of one sequence, a length for each, and a list
     // with room for them all (a pool of many requests' rows comes without lengths). Rows whose lists turn out not to nest take
     // half of a pair each, a third slower than here below (1024 rows of 2048 random keys 534 / 402).
     const bool two_rows = H == 64 && !beside && nsplit == 1 && seq_lens && rows_per_seq <= topk_k && rows_per_seq >= 192 && R >= 256;

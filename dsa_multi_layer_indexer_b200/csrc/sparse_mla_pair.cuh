@@ -14,8 +14,8 @@
 //
 // What bounds it. The products of a tile take 2180 cycles (32 a piece at M 128 N 128 K 16, 68 at N 256, measured alone) and
 // their operands, the rows' 139 KB and P 2900 cycles of shared memory; a tile takes 2300 with a few pairs at work and 3000 -
-// 3500 with all of them, where the board's power limit also lowers the clock (1.6 GHz at 1000 W). 1024 rows of 128 heads x
-// 2048 keys 803 -> 521 us, 700 x 700 250 -> 168 us (one CTA per 64 heads / this kernel). What it took:
+// 3400 with all of them, where the board's power limit also lowers the clock (1.6 GHz at 1000 W). 1024 rows of 128 heads x
+// 2048 keys 803 -> 495 us, 700 x 700 250 -> 155 us (one CTA per 64 heads / this kernel). What it took:
 //   * rows come by TMA row gathers (tile::gather4), four rows of one 64-dim chunk each. A gather costs a warp 35 - 60 cycles
 //     behind other gathers and 85 - 140 where it waits, looks something up or shuffles indices in between, so a warp issues
 //     eight in a row, from indices laid out in shared memory: 340 -> 270 cycles per 16 KB. (16-byte asynchronous copies with
@@ -24,19 +24,20 @@
 //     the same offset, and at the offset of a K chunk the other CTA has another chunk;
 //   * one ring of 16 KB units in the order of use, keys of tile t + 1 before values of tile t. A place is loaded again about
 //     2400 cycles before it is needed, which the loads just meet: nine units and two S buffers 532, ten and one 514 us;
+//   * the softmax takes S into registers and gives its buffer back at once, since the next score product waits for it: given
+//     back behind the exponentials 523, now 503 us. The heads' maxima are compared only where one ran away;
 //   * the MMA warp tests all its barriers in one look (a wait per unit, ready or not, took 200 cycles: 589 -> 548 us);
-//   * the softmax takes no maximum: a tile's row sums tell whether the reference still fits. Arrivals at the other CTA's
-//     barriers without cluster scope (they order nothing but shared memory of the arriving CTA, whose proxy fence precedes
-//     them): 1400 cycles each, twice a tile, before: 794 -> 580 us;
-//   * result and partials leave through shared memory and TMA stores: 5700 -> 1500 cycles a triple, 4 rows in 16 splits
-//     18.0 -> 16.1 us.
-// Tried: registers moved to the softmax warps by setmaxnreg (it needs whole groups of four warps; not needed since), two
-// softmax groups on alternate tiles (564 us: longer in total, and not what a tile waits for), eight gather warps (539).
+//   * arrivals at the other CTA's barriers without cluster scope (they order nothing but shared memory of the arriving CTA,
+//     whose proxy fence precedes them): 1400 cycles each, twice a tile, before: 794 -> 580 us;
+//   * result and partials leave through shared memory and TMA stores: 4 rows in 16 splits 18.0 -> 16.1 us.
+// Tried: two softmax groups on alternate tiles (564 us: longer in total, and not what a tile waits for), eight gather warps
+// (539), fp8 rows converted by the gather warps (32 rows 48.9 us against 45.8 with one CTA per 64 heads: of a tile's 17 chunks
+// eight are converted a second time).
 //
 // kTwoRows: 64 heads. Neighbouring rows of a prompt that is no longer than the list attend the same keys, the second one
 // its own as well: two rows' heads fill the pair's 128, with one list and each row's own view of what is masked. The plan
 // compares the two lists entry by entry; rows that do not nest, or whose one key more is not finite, go through their
-// own list alone, with the other CTA's result dropped. Prompt of 700 tokens 82 -> 65 us, 2048 465 -> 331 (four passes over
+// own list alone, with the other CTA's result dropped. Prompt of 700 tokens 82 -> 61 us, 2048 465 -> 320 (four passes over
 // each list with a few loads under way instead of one with sixteen: 127 us, the plan was what everything waited for).
 //
 // Warps (864 threads): 0-7 softmax, queries to tensor memory, result; 8 products (in CTA 0); 9 plans the triples and loads
@@ -66,7 +67,6 @@ constexpr int kLists = 4;                      // tiles whose rows are laid out
 constexpr int kPlan = 4;                       // entries of the plan ring
 constexpr float kRescaleLog2 = mla_tc::kRescaleLog2;
 enum { kBoth = 0, kFirst = 1, kSecond = 2 };  // rows of a plan entry
-constexpr float kAway = 1099511627776.f;       // 2^40: a tile's sum above it asks for another softmax reference
 
 // The first kNumPolled are what the MMA warp waits for.
 enum {
@@ -313,12 +313,14 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
         failed = __any_sync(0xffffffffu, failed);
         tc_fence_after();
         const uint32_t seen = *reinterpret_cast<volatile uint32_t*>(smem + Smem::seen_off + ((u & (kLists - 1)) * 4 + part) * 4);
-        uint32_t pk[16];
-        float psum = 0.f;
-        auto scores = [&](float (&x)[32]) {  // this lane's 32 keys, -inf where masked
+        float x[32];  // this lane's 32 keys, -inf where masked; then its probabilities, two to a register
+        {
           uint32_t raw[32];
           tmem_ld_32x32(ts, raw);
           tmem_ld_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) arrive_at(leader_bar(kBarSRead));
 #pragma unroll
           for (int i = 0; i < 32; ++i) x[i] = __uint_as_float(raw[i]);
           if (seen != 0xffffffffu) {
@@ -326,32 +328,14 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
             for (int i = 0; i < 32; ++i)
               if (!((seen >> i) & 1u)) x[i] = -INFINITY;
           }
-        };
-        auto probabilities = [&]() {
-          const float mr = m_ref == -INFINITY ? 0.f : m_ref;  // every key so far masked: all p = 0
-          float x[32], ps[2] = {0.f, 0.f};
-          scores(x);
-          // the row sum uses the rounded probabilities that the value product will see
+        }
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const __nv_bfloat162 b = __floats2bfloat162_rn(mla_tc::ex2_approx(fmaf(x[2 * i], p.scale_log2, -mr)),
-                                                           mla_tc::ex2_approx(fmaf(x[2 * i + 1], p.scale_log2, -mr)));
-            pk[i] = *reinterpret_cast<const uint32_t*>(&b);
-            ps[0] += __uint_as_float(pk[i] << 16);
-            ps[1] += __uint_as_float(pk[i] & 0xFFFF0000u);
-          }
-          psum = ps[0] + ps[1];
-        };
-        if (!failed && t > 0) probabilities();
-        // A sum that ran away from the reference (or no reference yet): the group looks at the tile's maximum. Any other tile
-        // needs none.
-        if (group_sync_or(failed || m_ref == -INFINITY || !(psum <= kAway))) {
-          float x[32];
-          scores(x);
-          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-          for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], x[i]);
-          s_max[part * 64 + head] = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
+        for (int i = 0; i < 32; ++i) m4[i & 3] = fmaxf(m4[i & 3], x[i]);
+        const float m_loc = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * p.scale_log2;
+        // No reference yet, or a maximum that ran away from it: the heads' quarters are compared.
+        if (group_sync_or(failed || m_ref == -INFINITY || m_loc > m_ref + kRescaleLog2)) {
+          s_max[part * 64 + head] = m_loc;
           if (group_sync_or(failed)) { failed = true; break; }
           float f = 1.f;
           const float m_first = fmaxf(s_max[head], s_max[64 + head]);
@@ -377,14 +361,23 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
               tmem_st_32x8(tq + kColO + 8u * blk, o);
             }
             tmem_st_wait();
+            tc_fence_before();
           }
           group_sync();  // (the maxima have been read)
-          probabilities();
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) arrive_at(leader_bar(kBarSRead));
-        l_run += psum;
+        const float mr = m_ref == -INFINITY ? 0.f : m_ref;  // every key so far masked: all p = 0
+        // the row sum uses the rounded probabilities that the value product will see
+        uint32_t pk[16];
+        float ps[2] = {0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const __nv_bfloat162 b = __floats2bfloat162_rn(mla_tc::ex2_approx(fmaf(x[2 * i], p.scale_log2, -mr)),
+                                                         mla_tc::ex2_approx(fmaf(x[2 * i + 1], p.scale_log2, -mr)));
+          pk[i] = *reinterpret_cast<const uint32_t*>(&b);
+          ps[0] += __uint_as_float(pk[i] << 16);
+          ps[1] += __uint_as_float(pk[i] & 0xFFFF0000u);
+        }
+        l_run += ps[0] + ps[1];
         // P is single-buffered: the previous tile's value product must have read it
         if (u >= 1 && !mbar_wait(bar(kBarPV), (u - 1) & 1)) failed = true;
 #pragma unroll
@@ -412,9 +405,9 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
       // first of this CTA's 64 rows of partials: [row][split][head]
       const int64_t pb = kTwoRows ? ((int64_t(done.r) + rank) * p.nsplit + done.split) * 64
                                   : (int64_t(done.r) * p.nsplit + done.split) * p.H + (done.heads0 - int64_t(done.r) * p.H);
-      // 64 bytes of 32 rows at a time through this warp's 2 KB of the probabilities' place and out by TMA. (Stored straight
-      // from the lanes, whose rows are a kilobyte or two apart, an instruction takes as many cycles as it has lanes: 5700
-      // cycles an item.)
+      // 64 bytes of 32 rows at a time through this warp's 2 KB of the probabilities' place and out by TMA: 4400 cycles an item.
+      // (Straight from the lanes, whose rows are a kilobyte or two apart, an instruction takes as many cycles as it has
+      // lanes: 5700, and as much in the way of the others. Both in turn: 3 % slower for short rows.)
       const uint32_t s_stage = s_p + uint32_t(warp) * 2048u;
       const int srow = int((p.out ? done.heads0 : pb) + (quad & 1) * 32);
       auto put = [&](const uint32_t (&w)[16], int col) {
