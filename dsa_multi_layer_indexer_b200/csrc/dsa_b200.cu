@@ -1014,12 +1014,29 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
     // 220 18.7 / 18.6, two of 150 23.8 / 23.7). What tells a prompt: many rows of one sequence, a length for each, and a list
     // with room for them all (a pool of many requests' rows comes without lengths). Rows whose lists turn out not to nest take
     // half of a pair each, a third slower than here below (1024 rows of 2048 random keys 534 / 402).
-    const bool two_rows = H == 64 && !beside && nsplit == 1 && seq_lens && rows_per_seq <= topk_k && rows_per_seq >= 192 && R >= 256;
+    const bool prompt = H == 64 && !kv_fp8 && !beside && nsplit == 1 && seq_lens;
+    const bool two_rows = prompt && rows_per_seq <= topk_k && rows_per_seq >= 192 && R >= 256;
+    const bool two_rows_first = prompt && indices && out && R == rows_per_seq && R > topk_k && topk_k >= 256;
     if (!kv_fp8 && pair_fits && (two_rows || (H % mla_pair::kHeads == 0 && pair_pays))) {
       p.keys_per_split = (kps + mla_pair::kBN - 1) / mla_pair::kBN * mla_pair::kBN;
       return launch_mla_pair(p, R, beside, st);
     }
     p.keys_per_split = (kps + mla_tc::kBN - 1) / mla_tc::kBN * mla_tc::kBN;
+    // Of a prompt that is longer than the list, the rows that it has room for go two by two, the others behind them as before:
+    // beside them, since neither depends on the other (us, all one by one / this: 2100 tokens 490 / 365, 4000 1294 / 1126).
+    if (two_rows_first && pair_fits) {
+      mla::Params head = p;
+      head.rows_per_seq = topk_k;
+      head.keys_per_split = (kps + mla_pair::kBN - 1) / mla_pair::kBN * mla_pair::kBN;
+      int rc = launch_mla_pair(head, topk_k, false, st);
+      if (rc) return rc;
+      p.q += int64_t(topk_k) * H * mla::kD;
+      p.indices += int64_t(topk_k) * topk_k;
+      p.seq_lens += topk_k;
+      p.out += int64_t(topk_k) * H * mla::kDV;
+      p.rows_per_seq = R = R - topk_k;
+      beside = true;
+    }
     auto kernel = beside ? mla_tc::sparse_mla_tc_kernel<true> : mla_tc::sparse_mla_tc_kernel<false>;
     int rc = opt_in_smem(kernel, mla_tc::Smem::bytes, g_opt_mla_tc[beside]);
     if (rc) return rc;

@@ -168,6 +168,18 @@ def test_two_rows_of_a_prompt(ops, batch, n, topk):
     check(ops, *prompt(batch, n, topk, seed=n), n, 1)
 
 
+@pytest.mark.parametrize("n,topk", [(257, 256), (400, 256), (700, 301)])
+def test_a_prompt_longer_than_its_lists(ops, n, topk):
+    """The rows that the list has room for go two by two, the others one by one beside them."""
+    q, kv, _, lens = prompt(1, n, n, seed=n)
+    gen = torch.Generator(device="cuda").manual_seed(topk)
+    idx = torch.full((n, topk), -1, dtype=torch.int32, device="cuda")
+    for r in range(n):
+        k = min(r + 1, topk)
+        idx[r, :k] = torch.randperm(r + 1, device="cuda", generator=gen)[:k].sort().values.int()
+    check(ops, q, kv, idx, lens, n, 1)
+
+
 def test_two_rows_that_differ(ops):
     """Lists that do not nest, rows of which one or both see nothing, lengths that shrink: row by row then."""
     n = 260
