@@ -98,7 +98,9 @@ __device__ __forceinline__ void tmem_alloc2(uint32_t smem_result_addr, uint32_t 
 __device__ __forceinline__ void tmem_free2(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void tmem_relinquish2() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_relinquish2() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
 // arrives at `bar` of both CTAs once every product issued so far is done
 __device__ __forceinline__ void commit2(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
@@ -126,8 +128,8 @@ __device__ __forceinline__ void gather4(uint32_t dst, const CUtensorMap* map, in
 }
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t cluster_bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(map), "r"(x), "r"(y), "r"(cluster_bar)
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+      "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(cluster_bar)
       : "memory");
 }
 __device__ __forceinline__ void arrive_at(uint32_t cluster_bar) {
@@ -141,8 +143,8 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&v)[8]) {
                : "memory");
 }
 __device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&v)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
-               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
 // Named barrier 2 over the softmax warps, plain and with an OR reduction.
@@ -161,7 +163,8 @@ __device__ __forceinline__ bool group_sync_or(bool x) {
 // [32 rows][64 bytes] of shared memory (64-byte swizzle) to global memory, and the waits for this thread's stores: until
 // shared memory has been read, until all is written.
 __device__ __forceinline__ void tma_store_2d(uint32_t src, const CUtensorMap* map, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src) : "memory");
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(src)
+               : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -187,7 +190,8 @@ struct Params {
 
 template <bool kBeside, bool kTwoRows>
 __global__ void __launch_bounds__(kThreads, 1)
-sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap out_map, const Params pp) {
+sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap q_map,
+                       const __grid_constant__ CUtensorMap out_map, const Params pp) {
   const mla::Params& p = pp.m;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
@@ -205,8 +209,10 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
   DSA_KTIME_BEGIN(2);
 
   if (tid == 0) {
-    for (int i = 0; i < kNumBars; ++i)
-      mbar_init(bar(i), i == kBarQT || i == kBarSRead || i == kBarP || i == kBarOFree ? uint32_t(2 * kSoftWarps) : i == kBarQStage ? uint32_t(kQTmem / 2) : 1u);
+    for (int i = 0; i < kNumBars; ++i) {
+      const bool softmax = i == kBarQT || i == kBarSRead || i == kBarP || i == kBarOFree;
+      mbar_init(bar(i), softmax ? 2 * kSoftWarps : i == kBarQStage ? kQTmem / 2 : 1);
+    }
     mbar_fence_init();
   }
   if (warp == kMmaWarp) {
@@ -260,7 +266,8 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
       return false;
     }
     e = s_plan[n & (kPlan - 1)];
-    e.x = __shfl_sync(0xffffffffu, e.x, 0), e.y = __shfl_sync(0xffffffffu, e.y, 0), e.z = __shfl_sync(0xffffffffu, e.z, 0), e.w = __shfl_sync(0xffffffffu, e.w, 0);
+    e.x = __shfl_sync(0xffffffffu, e.x, 0), e.y = __shfl_sync(0xffffffffu, e.y, 0);
+    e.z = __shfl_sync(0xffffffffu, e.z, 0), e.w = __shfl_sync(0xffffffffu, e.w, 0);
     return e.x >= 0;
   };
 
@@ -382,7 +389,8 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
         if (u >= 1 && !mbar_wait(bar(kBarPV), (u - 1) & 1)) failed = true;
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-          st_shared_v4(s_prow + uint32_t(((4 * group + c) ^ (head & 7)) << 4), make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]));
+          st_shared_v4(s_prow + uint32_t(((4 * group + c) ^ (head & 7)) << 4),
+                       make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]));
         fence_proxy_async_smem();
         tc_fence_before();
         __syncwarp();
@@ -415,7 +423,8 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
         __syncwarp();
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-          st_shared_v4(s_stage + uint32_t(lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)), make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]));
+          st_shared_v4(s_stage + uint32_t(lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)),
+                       make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]));
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && mine) tma_store_2d(s_stage, &out_map, col, srow);
@@ -760,7 +769,8 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
                 const uint64_t v0 = smem_desc_mn128(s_ring + uint32_t(slot) * kUnitBytes, kChunkBytes, 1024);
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                  mma2(tmem + kColO + 128u * i, smem_desc_k128(s_p + uint32_t(b) * kChunkBytes) + uint64_t(2 * ks), v0 + uint64_t(ks * (2048 >> 4)),
+                  mma2(tmem + kColO + 128u * i, smem_desc_k128(s_p + uint32_t(b) * kChunkBytes) + uint64_t(2 * ks),
+                       v0 + uint64_t(ks * (2048 >> 4)),
                        idesc_pv, (first && b == 0 && ks == 0) ? 0u : 1u);
                 commit2(bar(kBarEmpty + slot));
               }

@@ -275,11 +275,12 @@ int dsa_topk_select_static(const float* logits, const int32_t* seq_lens, int32_t
  * dsa_sparse_mla_decode = partials + combine; the two halves are exported for
  * callers that schedule them separately, as the reference does.
  *
- * Two kernels serve the partials. Launches with H a multiple of 64 and at least
+ * Three kernels serve the partials. Launches with H a multiple of 64 and at least
  * 128 tiles of 64 heads x 64 keys (R * H/64 * ceil(topk/64)) run on tcgen05 /
- * tensor memory with 64 heads per CTA; smaller launches and other head counts
+ * tensor memory with 64 heads per CTA, larger ones over bf16 rows with 128 heads
+ * (or two neighbouring rows' 64, of a prompt) per pair of CTAs; smaller launches and other head counts
  * run on mma.sync with 16 heads per CTA, or 32 (CTA counts above the SMs', H a
- * multiple of 32, and splits of several tiles or fp8 rows). Both write the same part_* layout;
+ * multiple of 32, and splits of several tiles or fp8 rows). All write the same part_* layout;
  * part_m is a base-2 softmax reference of the split (not necessarily its
  * maximum) consistent with part_l and part_acc, which is all
  * dsa_sparse_mla_combine needs. (bf16 partial accumulators were measured: the

@@ -168,6 +168,14 @@ def test_two_rows_of_a_prompt(ops, batch, n, topk):
     check(ops, *prompt(batch, n, topk, seed=n), n, 1)
 
 
+def test_two_rows_without_a_list(ops):
+    n = 259
+    q, kv, idx, lens = prompt(1, n, n, seed=11)
+    got = ops.sparse_mla_decode(q, kv, None, SM, lens, rows_per_seq=n, nsplit=1, dense_keys=n)
+    want = ops.sparse_mla_decode(q, kv, idx, SM, lens, rows_per_seq=n, nsplit=1)
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("n,topk", [(257, 256), (400, 256), (700, 301)])
 def test_a_prompt_longer_than_its_lists(ops, n, topk):
     """The rows that the list has room for go two by two, the others one by one beside them."""
