@@ -983,23 +983,16 @@ static int launch_mla_pair(const mla::Params& m, int R, bool beside, cudaStream_
   return DSA_OK;
 }
 
-static int mla_partials_launch(const void* q, const void* kv, const int32_t* indices,
-                               const int32_t* seq_lens, float* part_acc, float* part_m, float* part_l,
-                               void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale,
-                               int64_t kv_seq_stride, int kv_fp8, bool beside, void* stream) {
-  // `out`: the caller wants the merged result and there is one split, so the kernel writes it itself
-  mla::Params p;
-  int rc0 = mla_prepare(q, kv, indices, seq_lens, part_acc, part_m, part_l, R, rows_per_seq, H, topk_k,
-                        nsplit, sm_scale, kv_seq_stride, kv_fp8, out == nullptr, &p);
-  if (rc0) return rc0;
-  p.out = static_cast<__nv_bfloat16*>(out);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
+// The kernel(s) of a launch; `flags`: DSA_MLA_LIST and so on.
+static int mla_form(int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale, int64_t kv_seq_stride, bool kv_fp8, int flags) {
+  const int kps = (topk_k + nsplit - 1) / nsplit;
   // Head counts that fill 64-row blocks go to the tcgen05 kernel once there are enough
   // 64-head x 64-key tiles to give every SM more than one (a single row of 2048 keys
   // is faster on the mma.sync kernel's narrower CTAs); its splits are whole 64-key tiles.
   const int64_t tc_tiles = int64_t(R) * (H / mla_tc::kHG) * ((topk_k + mla_tc::kBN - 1) / mla_tc::kBN);
   if (H % mla_tc::kHG == 0 && sm_scale > 0.f && tc_tiles >= mla_tc::kMinTiles) {
-    int kps = (topk_k + nsplit - 1) / nsplit;
+    // (bf16 rows; the rows of cache, queries, result and partials are coordinates of tensor maps)
+    if (kv_fp8 || R / rows_per_seq * kv_seq_stride >= (int64_t(1) << 31) || int64_t(R) * H * nsplit >= (int64_t(1) << 31)) return DSA_MLA_TC;
     // 128 heads on a pair of CTAs where a split has four of its 128-key tiles, the only split two, or where the pairs take several
     // splits each (us, pair / one CTA per 64 heads, 128 heads, the default split count): 16 rows x 2048 keys in 4 splits
     // 21.9 / 24.8, 32 in 2 32.7 / 41.1, 40 in 1 38.4 / 59.5, 200 x 1024 59.0 / 95.1, 40 x 512 15.8 / 19.6, 40 x 256 11.9 / 12.9,
@@ -1007,41 +1000,21 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
     // splits 16.8 / 16.9, 4 in 16 16.0 / 14.3, 16 x 1024 in 4 18.3 / 18.1, 32 x 512 in 2 21.5 / 21.5, 64 x 128 10.6 / 9.2.
     const int64_t pair_items = int64_t(R) * (H / mla_pair::kHeads) * nsplit;
     const bool pair_pays = kps >= (nsplit == 1 ? 2 : 4) * mla_pair::kBN || pair_items > sm_count() / 2;
-    // (the rows of cache, queries, result and partials are coordinates of tensor maps)
-    const bool pair_fits = R / rows_per_seq * kv_seq_stride < (int64_t(1) << 31) && int64_t(R) * H * nsplit < (int64_t(1) << 31);
+    if (H % mla_pair::kHeads == 0 && pair_pays) return DSA_MLA_PAIR;
     // Two rows of 64 heads on a pair for a prompt that is no longer than the list: neighbouring rows then attend the same keys
     // but one (us, pair / one CTA a row: prompts of 256 tokens 19.4 / 20.8, 700 61 / 82, 2048 320 / 465, two of 200 26.7 / 29.0;
-    // 220 18.7 / 18.6, two of 150 23.8 / 23.7). What tells a prompt: many rows of one sequence, a length for each, and a list
-    // with room for them all (a pool of many requests' rows comes without lengths). Rows whose lists turn out not to nest take
-    // half of a pair each, a third slower than here below (1024 rows of 2048 random keys 534 / 402).
-    const bool prompt = H == 64 && !kv_fp8 && !beside && nsplit == 1 && seq_lens;
-    const bool two_rows = prompt && rows_per_seq <= topk_k && rows_per_seq >= 192 && R >= 256;
-    const bool two_rows_first = prompt && indices && out && R == rows_per_seq && R > topk_k && topk_k >= 256;
-    if (!kv_fp8 && pair_fits && (two_rows || (H % mla_pair::kHeads == 0 && pair_pays))) {
-      p.keys_per_split = (kps + mla_pair::kBN - 1) / mla_pair::kBN * mla_pair::kBN;
-      return launch_mla_pair(p, R, beside, st);
-    }
-    p.keys_per_split = (kps + mla_tc::kBN - 1) / mla_tc::kBN * mla_tc::kBN;
-    // Of a prompt that is longer than the list, the rows that it has room for go two by two, the others behind them as before:
+    // 220 18.7 / 18.6, two of 150 23.8 / 23.7). Rows whose lists do not nest take half of a pair each, a third slower than one
+    // CTA a row (512 rows behind 32K keys 300 / 233, 1024 of them 532 / 405): so only where the caller says that the rows are
+    // their sequence's first, or where the list has room for the whole cache (a selection then lists every key that a row sees).
+    const bool rows_of_a_prompt = H == 64 && (flags & DSA_MLA_LENGTHS) && !(flags & DSA_MLA_BESIDE) && nsplit == 1;
+    if (rows_of_a_prompt && ((flags & DSA_MLA_PROMPT) || kv_seq_stride <= topk_k) && rows_per_seq <= topk_k && rows_per_seq >= 192 && R >= 256)
+      return DSA_MLA_PAIR_TWO_ROWS;
+    // Of a prompt that is longer than the list, the rows that it has room for go two by two, the others behind them one by one:
     // beside them, since neither depends on the other (us, all one by one / this: 2100 tokens 490 / 365, 4000 1294 / 1126).
-    if (two_rows_first && pair_fits) {
-      mla::Params head = p;
-      head.rows_per_seq = topk_k;
-      head.keys_per_split = (kps + mla_pair::kBN - 1) / mla_pair::kBN * mla_pair::kBN;
-      int rc = launch_mla_pair(head, topk_k, false, st);
-      if (rc) return rc;
-      p.q += int64_t(topk_k) * H * mla::kD;
-      p.indices += int64_t(topk_k) * topk_k;
-      p.seq_lens += topk_k;
-      p.out += int64_t(topk_k) * H * mla::kDV;
-      p.rows_per_seq = R = R - topk_k;
-      beside = true;
-    }
-    auto kernel = beside ? mla_tc::sparse_mla_tc_kernel<true> : mla_tc::sparse_mla_tc_kernel<false>;
-    int rc = opt_in_smem(kernel, mla_tc::Smem::bytes, g_opt_mla_tc[beside]);
-    if (rc) return rc;
-    DSA_CUDA(launch_pdl(kernel, dim3(nsplit, H / mla_tc::kHG, R), dim3(mla_tc::kThreads), mla_tc::Smem::bytes, st, p));
-    return DSA_OK;
+    if (rows_of_a_prompt && (flags & DSA_MLA_PROMPT) && (flags & DSA_MLA_LIST) && (flags & DSA_MLA_DIRECT) && R == rows_per_seq &&
+        R > topk_k && topk_k >= 256)
+      return DSA_MLA_PAIR_FIRST_ROWS;
+    return DSA_MLA_TC;
   }
   // Where 16-head CTAs would share the SMs, 32 heads per CTA if that pays: the rows are gathered (and fp8 rows expanded)
   // once for both blocks and, of a split of several tiles, the next one is on its way. Layers of the hot path in a row,
@@ -1051,10 +1024,65 @@ static int mla_partials_launch(const void* q, const void* kv, const int32_t* ind
   // of 64 24.15 / 24.4, 16 of 32 over 512 keys 25.7 / 26.4; 7 of 32 over 1024 25.4 / 25.2.
   const int64_t ctas = int64_t(nsplit) * (H / DSA_HEAD_BLOCK) * R;
   if (H % (2 * DSA_HEAD_BLOCK) == 0 && ctas > sm_count()) {
-    if (p.keys_per_split > mla::kBN) return launch_mla_partials<2, 8, 2>(p, R, nsplit, beside, st);
-    if (kv_fp8) return launch_mla_partials_of<true, 2, 8, 1>(p, R, nsplit, beside, st);
+    if ((kps + 15) / 16 * 16 > mla::kBN) return DSA_MLA_32_HEADS;
+    if (kv_fp8) return DSA_MLA_32_HEADS_ONE_TILE;
   }
-  return launch_mla_partials<1, 4, 1>(p, R, nsplit, beside, st);
+  return DSA_MLA_16_HEADS;
+}
+
+int dsa_sparse_mla_form(int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale, int64_t kv_seq_stride, int kv_fp8, int flags) {
+  DSA_REQUIRE(R > 0 && rows_per_seq > 0 && R % rows_per_seq == 0 && H > 0 && H % DSA_HEAD_BLOCK == 0 && topk_k > 0 && nsplit > 0 &&
+                  kv_seq_stride > 0,
+              "sparse MLA: bad geometry");
+  return mla_form(R, rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8 != 0, flags);
+}
+
+// `flags`: DSA_MLA_BESIDE and DSA_MLA_PROMPT, as the caller has it; the others follow from the operands.
+static int mla_partials_launch(const void* q, const void* kv, const int32_t* indices,
+                               const int32_t* seq_lens, float* part_acc, float* part_m, float* part_l,
+                               void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale,
+                               int64_t kv_seq_stride, int kv_fp8, int flags, void* stream) {
+  // `out`: the caller wants the merged result and there is one split, so the kernel writes it itself
+  mla::Params p;
+  int rc0 = mla_prepare(q, kv, indices, seq_lens, part_acc, part_m, part_l, R, rows_per_seq, H, topk_k,
+                        nsplit, sm_scale, kv_seq_stride, kv_fp8, out == nullptr, &p);
+  if (rc0) return rc0;
+  p.out = static_cast<__nv_bfloat16*>(out);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  bool beside = flags & DSA_MLA_BESIDE;
+  flags |= (indices ? DSA_MLA_LIST : 0) | (seq_lens ? DSA_MLA_LENGTHS : 0) | (out ? DSA_MLA_DIRECT : 0);
+  const int form = mla_form(R, rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8 != 0, flags);
+  const int kps = (topk_k + nsplit - 1) / nsplit;
+  const auto whole_tiles = [&](int tile) { return (kps + tile - 1) / tile * tile; };
+  switch (form) {
+    case DSA_MLA_32_HEADS: return launch_mla_partials<2, 8, 2>(p, R, nsplit, beside, st);
+    case DSA_MLA_32_HEADS_ONE_TILE: return launch_mla_partials_of<true, 2, 8, 1>(p, R, nsplit, beside, st);
+    case DSA_MLA_16_HEADS: return launch_mla_partials<1, 4, 1>(p, R, nsplit, beside, st);
+    case DSA_MLA_PAIR:
+    case DSA_MLA_PAIR_TWO_ROWS:
+      p.keys_per_split = whole_tiles(mla_pair::kBN);
+      return launch_mla_pair(p, R, beside, st);
+    default: break;
+  }
+  p.keys_per_split = whole_tiles(mla_tc::kBN);
+  if (form == DSA_MLA_PAIR_FIRST_ROWS) {
+    mla::Params head = p;
+    head.rows_per_seq = topk_k;
+    head.keys_per_split = whole_tiles(mla_pair::kBN);
+    int rc = launch_mla_pair(head, topk_k, false, st);
+    if (rc) return rc;
+    p.q += int64_t(topk_k) * H * mla::kD;
+    p.indices += int64_t(topk_k) * topk_k;
+    p.seq_lens += topk_k;
+    p.out += int64_t(topk_k) * H * mla::kDV;
+    p.rows_per_seq = R = R - topk_k;
+    beside = true;
+  }
+  auto kernel = beside ? mla_tc::sparse_mla_tc_kernel<true> : mla_tc::sparse_mla_tc_kernel<false>;
+  int rc = opt_in_smem(kernel, mla_tc::Smem::bytes, g_opt_mla_tc[beside]);
+  if (rc) return rc;
+  DSA_CUDA(launch_pdl(kernel, dim3(nsplit, H / mla_tc::kHG, R), dim3(mla_tc::kThreads), mla_tc::Smem::bytes, st, p));
+  return DSA_OK;
 }
 
 int dsa_sparse_mla_partials(const void* q, const void* kv, const int32_t* indices,
@@ -1062,7 +1090,7 @@ int dsa_sparse_mla_partials(const void* q, const void* kv, const int32_t* indice
                             int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale,
                             int64_t kv_seq_stride, int kv_fp8, void* stream) {
   return mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, nullptr, R, rows_per_seq, H, topk_k,
-                             nsplit, sm_scale, kv_seq_stride, kv_fp8, false, stream);
+                             nsplit, sm_scale, kv_seq_stride, kv_fp8, 0, stream);
 }
 
 extern "C++" {
@@ -1103,28 +1131,39 @@ int dsa_sparse_mla_combine(const float* part_acc, const float* part_m, const flo
   return launch(part_acc, part_m, part_l, out, R, H, nsplit, static_cast<cudaStream_t>(stream));
 }
 
+static int mla_decode(const void* q, const void* kv, const int32_t* indices, const int32_t* seq_lens, float* part_acc, float* part_m,
+                      float* part_l, void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit, float sm_scale,
+                      int64_t kv_seq_stride, int kv_fp8, int flags, void* stream) {
+  DSA_REQUIRE(out && aligned16(out), "sparse MLA: out must be a 16-byte aligned pointer");
+  const bool direct = nsplit == 1 && !part_acc;  // (a caller that hands over partials gets them)
+  int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, direct ? out : nullptr, R,
+                               rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8, flags, stream);
+  if (rc || direct) return rc;
+  return dsa_sparse_mla_combine(part_acc, part_m, part_l, out, R, H, nsplit, stream);
+}
+
 int dsa_sparse_mla_decode(const void* q, const void* kv, const int32_t* indices,
                           const int32_t* seq_lens, float* part_acc, float* part_m, float* part_l,
                           void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit,
                           float sm_scale, int64_t kv_seq_stride, int kv_fp8, void* stream) {
-  DSA_REQUIRE(out && aligned16(out), "sparse MLA: out must be a 16-byte aligned pointer");
-  const bool direct = nsplit == 1 && !part_acc;  // (a caller that hands over partials gets them)
-  int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, direct ? out : nullptr, R,
-                               rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8, false, stream);
-  if (rc || direct) return rc;
-  return dsa_sparse_mla_combine(part_acc, part_m, part_l, out, R, H, nsplit, stream);
+  return mla_decode(q, kv, indices, seq_lens, part_acc, part_m, part_l, out, R, rows_per_seq, H, topk_k, nsplit, sm_scale,
+                    kv_seq_stride, kv_fp8, 0, stream);
 }
 
 int dsa_sparse_mla_decode_beside(const void* q, const void* kv, const int32_t* indices,
                                  const int32_t* seq_lens, float* part_acc, float* part_m, float* part_l,
                                  void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit,
                                  float sm_scale, int64_t kv_seq_stride, int kv_fp8, void* stream) {
-  DSA_REQUIRE(out && aligned16(out), "sparse MLA: out must be a 16-byte aligned pointer");
-  const bool direct = nsplit == 1 && !part_acc;  // (a caller that hands over partials gets them)
-  int rc = mla_partials_launch(q, kv, indices, seq_lens, part_acc, part_m, part_l, direct ? out : nullptr, R,
-                               rows_per_seq, H, topk_k, nsplit, sm_scale, kv_seq_stride, kv_fp8, true, stream);
-  if (rc || direct) return rc;
-  return dsa_sparse_mla_combine(part_acc, part_m, part_l, out, R, H, nsplit, stream);
+  return mla_decode(q, kv, indices, seq_lens, part_acc, part_m, part_l, out, R, rows_per_seq, H, topk_k, nsplit, sm_scale,
+                    kv_seq_stride, kv_fp8, DSA_MLA_BESIDE, stream);
+}
+
+int dsa_sparse_mla_prompt(const void* q, const void* kv, const int32_t* indices,
+                          const int32_t* seq_lens, float* part_acc, float* part_m, float* part_l,
+                          void* out, int R, int rows_per_seq, int H, int topk_k, int nsplit,
+                          float sm_scale, int64_t kv_seq_stride, int kv_fp8, void* stream) {
+  return mla_decode(q, kv, indices, seq_lens, part_acc, part_m, part_l, out, R, rows_per_seq, H, topk_k, nsplit, sm_scale,
+                    kv_seq_stride, kv_fp8, DSA_MLA_PROMPT, stream);
 }
 
 // ------------------------------------------------------------------ decode-step preparation

@@ -35,7 +35,7 @@ using at::Tensor;
 #define DSA_HOST_API(X)                                                                                        \
   X(dsa_indexer_scan_fp8) X(dsa_indexer_scan_fp8_paged) X(dsa_indexer_scan_f32) X(dsa_topk_workspace_bytes)    \
   X(dsa_topk_select) X(dsa_topk_select_paged) X(dsa_sparse_mla_partials) X(dsa_sparse_mla_combine)             \
-  X(dsa_sparse_mla_decode) X(dsa_sparse_mla_decode_beside) X(dsa_sparse_mla_f32) X(dsa_rmsnorm)                \
+  X(dsa_sparse_mla_decode) X(dsa_sparse_mla_decode_beside) X(dsa_sparse_mla_prompt) X(dsa_sparse_mla_f32) X(dsa_rmsnorm)                \
   X(dsa_add_rmsnorm_bf16) X(dsa_silu_mul_bf16) X(dsa_add_rmsnorm_f32) X(dsa_silu_mul_f32) X(dsa_linear_f32)                \
   X(dsa_indexer_stage_fp8) X(dsa_latent_append) X(dsa_prefill_latents) X(dsa_prefill_queries)
 struct Api {
@@ -375,7 +375,7 @@ PyObject* default_nsplit(PyObject* const* a) {
 }
 
 // (q, kv, indices, sm_scale, seq_lens, rows_per_seq, nsplit, acc, m, l, out, dense_keys, stage 0 both / 1 partials /
-//  2 combine, beside)
+//  2 combine, beside, prompt)
 PyObject* mla(PyObject* const* a) {
   const Tensor &q = ten(a[0], "q"), &kv = ten(a[1], "kv");
   contig(q, "q", {at::kBFloat16});
@@ -421,7 +421,7 @@ PyObject* mla(PyObject* const* a) {
   need(!beside || stage == 0, "beside_previous goes with stage='both'");
   void* st = stream();
   if (stage == 0)
-    LAUNCH((beside ? api.dsa_sparse_mla_decode_beside : api.dsa_sparse_mla_decode)(
+    LAUNCH((beside ? api.dsa_sparse_mla_decode_beside : truth(a[14]) ? api.dsa_sparse_mla_prompt : api.dsa_sparse_mla_decode)(
         ptr(q), ptr(kv), as<int32_t>(idx), as<int32_t>(lens), pa, pm, pl, ptr(out), int(R), int(rps), int(H), int(k), int(nsplit),
         scale, cap, fp8 ? 1 : 0, st));
   else if (stage == 1)
@@ -1047,7 +1047,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
 #define M(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&entry<name, n>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&bind)), METH_FASTCALL, nullptr},
-    M(scan_fp8, 10), M(scan_paged, 8), M(scan_f32, 7), M(topk, 11), M(topk_paged, 7), M(default_nsplit, 4), M(mla, 14), M(attention_last, 7), M(mla_f32, 7), M(rmsnorm, 3),
+    M(scan_fp8, 10), M(scan_paged, 8), M(scan_f32, 7), M(topk, 11), M(topk_paged, 7), M(default_nsplit, 4), M(mla, 15), M(attention_last, 7), M(mla_f32, 7), M(rmsnorm, 3),
     M(add_rmsnorm, 4), M(silu_mul, 2), M(indexer_stage, 18), M(latent_append, 11), M(prefill_latents, 16), M(prefill_queries, 13),
     M(plain_weights, 6), M(full_operands, 29), M(project_output, 5), M(mlp, 4),
     M(abi_scan, AbiArgs<decltype(::dsa_indexer_scan_fp8)>::value), M(abi_scan_paged, AbiArgs<decltype(::dsa_indexer_scan_fp8_paged)>::value),

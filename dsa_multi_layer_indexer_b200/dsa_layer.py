@@ -302,12 +302,13 @@ class DSALayer(nn.Module):
         return ops.topk_select(logits, topk, seq_lens, pad_value=pad_value)
 
     def _attend(self, q, kv, indices, seq_lens, rows_per_seq: int) -> torch.Tensor:
-        """Latent attention output [R,H,Dv]. q [R,H,Dqk], kv [n_seq,N,Dqk]; indices int32 or None (dense)."""
+        """Latent attention output [R,H,Dv] of sequences from their first position. q [R,H,Dqk], kv [n_seq,N,Dqk];
+        indices int32 or None (dense)."""
         c = self.config
         if self._fast_path(q):
             h = q.shape[1]
             out = ops.sparse_mla_decode(_pad_heads(q, ops.HEAD_BLOCK).contiguous(), kv.contiguous(), indices,
-                                        self.sm_scale, seq_lens, rows_per_seq=rows_per_seq)
+                                        self.sm_scale, seq_lens, rows_per_seq=rows_per_seq, prompt=True)
             return out[:, :h]
         out = ops.sparse_mla_f32(q.float().contiguous(), kv.float().contiguous(), indices, c.kv_lora_rank,
                                  self.sm_scale, seq_lens, rows_per_seq=rows_per_seq)
@@ -414,7 +415,7 @@ class DSALayer(nn.Module):
         h = op.q.shape[1]
         if op.q.dtype == torch.bfloat16:
             o = ops.sparse_mla_decode(_pad_heads(op.q, ops.HEAD_BLOCK), op.kv, indices, self.sm_scale, op.lens,
-                                      rows_per_seq=op.s, dense_keys=op.s)
+                                      rows_per_seq=op.s, dense_keys=op.s, prompt=True)
         else:
             o = ops.sparse_mla_f32(op.q, op.kv, indices, c.kv_lora_rank, self.sm_scale, op.lens, rows_per_seq=op.s)
         return self._reduced(_lib.host().project_output(o, op.weights[3], op.weights[4], h, c.v_head_dim).view(op.b, op.s, -1))

@@ -192,13 +192,16 @@ def sparse_mla_decode(
     dense_keys: Optional[int] = None,
     stage: str = "both",
     beside_previous: bool = False,
+    prompt: bool = False,
 ) -> torch.Tensor:
     """Sparse MLA decode: q ``[R, H, 576]`` bf16, kv ``[n_seq, cap, 576]`` bf16 or
     ``[n_seq, cap, 656]`` uint8 (fp8-packed rows), indices ``[R, topk]`` int32 or
     None for dense attention over ``dense_keys`` positions. Returns ``[R, H, 512]`` bf16.
     ``beside_previous``: none of the operands comes from the two kernels enqueued just before
     this call (the lagged schedule's attention behind this layer's scan and top-k); the attention
-    then runs beside the top-k and completes after it."""
+    then runs beside the top-k and completes after it. ``prompt``: the rows of each sequence are its
+    first positions (row i sees at most its first i + 1 keys), so that neighbours attend nearly the same
+    keys and may share a launch's CTAs; for speed alone, the results are the same without it."""
     if stage not in _STAGES:
         raise ValueError(f"unknown stage {stage!r}")
     if scratch is None:
@@ -206,7 +209,7 @@ def sparse_mla_decode(
     else:
         acc, m, l = scratch.acc, scratch.m, scratch.l
     return _host().mla(q, kv, indices, sm_scale, seq_lens, rows_per_seq, nsplit, acc, m, l, out, dense_keys, _STAGES[stage],
-                       beside_previous)
+                       beside_previous, prompt)
 
 
 def attention_last(q, kv, slots, sm_scale, next_idx, index_map, cap) -> bool:

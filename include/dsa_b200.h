@@ -316,6 +316,31 @@ int dsa_sparse_mla_decode_beside(const void* q, const void* kv, const int32_t* i
                                  int nsplit, float sm_scale, int64_t kv_seq_stride, int kv_fp8,
                                  void* stream);
 
+/* dsa_sparse_mla_decode for the rows of a prompt: the rows of each sequence are its first positions, so row i of a
+ * sequence sees at most its first i + 1 keys. Neighbouring rows then attend nearly the same keys, and those of 64 heads
+ * may share a pair of CTAs. The promise is for speed alone: rows that do not keep it get the same results. */
+int dsa_sparse_mla_prompt(const void* q, const void* kv, const int32_t* indices,
+                          const int32_t* seq_lens, float* part_acc, float* part_m,
+                          float* part_l, void* out, int R, int rows_per_seq, int H, int topk,
+                          int nsplit, float sm_scale, int64_t kv_seq_stride, int kv_fp8,
+                          void* stream);
+
+/* The kernel that these entry points take for a launch of the given sizes, a dsa_mla_form (nothing is launched; without a
+ * GPU, that of a device of 148 SMs). `flags` say what the launch has: a list, lengths, one split whose result
+ * is written without partials, and which of the entry points above it comes through. */
+enum dsa_mla_form {
+  DSA_MLA_16_HEADS = 0,          /* mma.sync, 16 heads per CTA                                                  */
+  DSA_MLA_32_HEADS = 1,          /* mma.sync, 32 heads per CTA, several tiles per split                         */
+  DSA_MLA_32_HEADS_ONE_TILE = 2, /* mma.sync, 32 heads per CTA                                                  */
+  DSA_MLA_TC = 3,                /* tcgen05, 64 heads per CTA                                                   */
+  DSA_MLA_PAIR = 4,              /* tcgen05, 128 heads per pair of CTAs                                         */
+  DSA_MLA_PAIR_TWO_ROWS = 5,     /* tcgen05, two rows of 64 heads per pair of CTAs                              */
+  DSA_MLA_PAIR_FIRST_ROWS = 6    /* the same for the rows that the list has room for, DSA_MLA_TC for the others */
+};
+enum { DSA_MLA_LIST = 1, DSA_MLA_LENGTHS = 2, DSA_MLA_DIRECT = 4, DSA_MLA_BESIDE = 8, DSA_MLA_PROMPT = 16 };
+int dsa_sparse_mla_form(int R, int rows_per_seq, int H, int topk, int nsplit, float sm_scale, int64_t kv_seq_stride,
+                        int kv_fp8, int flags);
+
 /* ---- (a6) fused indexer + attention launch -----------------------------------
  * One launch whose first CTAs compute the split-K attention partials over
  * `attend_indices` (under the lagged schedule: the PREVIOUS layer's selection)

@@ -1,0 +1,41 @@
+"""Which kernel a sparse MLA launch runs on, by its sizes (no GPU needed)."""
+
+from __future__ import annotations
+
+import pytest
+
+HEADS_16, HEADS_32, HEADS_32_ONE_TILE, TC, PAIR, TWO_ROWS, FIRST_ROWS = range(7)
+LIST, LENGTHS, DIRECT, BESIDE, PROMPT = 1, 2, 4, 8, 16
+
+
+def form(R, rows_per_seq, H, topk, nsplit, cap, flags=LIST | LENGTHS | DIRECT, fp8=0, scale=0.07):
+    from dsa_multi_layer_indexer_b200 import _lib
+
+    return _lib.lib().dsa_sparse_mla_form(R, rows_per_seq, H, topk, nsplit, scale, cap, fp8, flags)
+
+
+@pytest.mark.parametrize("R,rows_per_seq,topk,cap", [
+    (256, 256, 2048, 8192), (1024, 1024, 2048, 32768), (2048, 2048, 2048, 32768), (300, 300, 300, 4096), (900, 300, 300, 556),
+    (2500, 2500, 2048, 32768), (4000, 4000, 2048, 4000)])
+def test_rows_behind_a_context_do_not_share_a_pair(R, rows_per_seq, topk, cap):
+    """Lists that are selections from more keys than they have room for hardly ever nest."""
+    assert form(R, rows_per_seq, 64, topk, 1, cap) == TC
+    assert form(R, rows_per_seq, 64, topk, 1, cap, LIST | LENGTHS) == TC
+
+
+@pytest.mark.parametrize("R,rows_per_seq,topk,cap,with_prompt,without", [
+    (700, 700, 2048, 956, TWO_ROWS, TWO_ROWS), (700, 700, 700, 956, TWO_ROWS, TC), (600, 200, 200, 456, TWO_ROWS, TC),
+    (256, 256, 256, 256, TWO_ROWS, TWO_ROWS), (2048, 2048, 2048, 2304, TWO_ROWS, TC), (255, 255, 255, 255, TC, TC),
+    (382, 191, 191, 191, TC, TC), (2049, 2049, 2048, 2305, FIRST_ROWS, TC), (4002, 2001, 2000, 4096, TC, TC), (700, 700, 255, 700, TC, TC)])
+def test_rows_of_a_prompt(R, rows_per_seq, topk, cap, with_prompt, without):
+    every = LIST | LENGTHS | DIRECT
+    assert form(R, rows_per_seq, 64, topk, 1, cap, every | PROMPT) == with_prompt
+    assert form(R, rows_per_seq, 64, topk, 1, cap, every) == without
+    # not without lengths, in several splits, over fp8 rows, beside the top-k or with another head count; the first rows of a
+    # longer prompt not into partials either
+    assert form(R, rows_per_seq, 64, topk, 1, cap, LIST | DIRECT | PROMPT) == TC
+    assert form(R, rows_per_seq, 64, topk, 2, cap, LIST | LENGTHS | PROMPT) == TC
+    assert form(R, rows_per_seq, 64, topk, 1, cap, every | PROMPT, fp8=1) == TC
+    assert form(R, rows_per_seq, 64, topk, 1, cap, every | BESIDE) == TC
+    assert form(R, rows_per_seq, 192, topk, 1, cap, every | PROMPT) == TC
+    assert form(R, rows_per_seq, 64, topk, 1, cap, LIST | LENGTHS | PROMPT) == (TC if with_prompt == FIRST_ROWS else with_prompt)

@@ -48,10 +48,10 @@ def operands(R, H, n, topk, rows_per_seq=1, seed=0):
     return q, kv, idx, torch.full((R,), n, dtype=torch.int32, device="cuda")
 
 
-def check(ops, q, kv, idx, lens, rows_per_seq, nsplit):
+def check(ops, q, kv, idx, lens, rows_per_seq, nsplit, **kw):
     from dsa_multi_layer_indexer_b200 import _lib
 
-    got = ops.sparse_mla_decode(q, kv, idx, SM, lens, rows_per_seq=rows_per_seq, nsplit=nsplit)
+    got = ops.sparse_mla_decode(q, kv, idx, SM, lens, rows_per_seq=rows_per_seq, nsplit=nsplit, **kw)
     _lib.check_device_status()
     want = reference(q, kv, idx, lens, rows_per_seq)
     assert torch.isfinite(got).all()
@@ -228,7 +228,29 @@ def test_a_prompt_longer_than_its_lists(ops, n, topk):
     for r in range(n):
         k = min(r + 1, topk)
         idx[r, :k] = torch.randperm(r + 1, device="cuda", generator=gen)[:k].sort().values.int()
+    check(ops, q, kv, idx, lens, n, 1, prompt=True)
     check(ops, q, kv, idx, lens, n, 1)
+
+
+def test_what_is_called_a_prompt_and_is_none(ops):
+    """Rows behind a context, lists that do not nest: the caller's word changes the launch, not the result."""
+    q, kv, idx, lens = operands(400, 64, 900, 256, 400, seed=13)
+    check(ops, q, kv, idx, lens, 400, 1, prompt=True)
+
+
+def test_a_prefill_says_that_its_rows_are_a_prompt(ops, monkeypatch):
+    import dataclasses
+
+    import dsa_multi_layer_indexer_b200 as dsa
+
+    said, decode = [], ops.sparse_mla_decode
+    monkeypatch.setattr(ops, "sparse_mla_decode", lambda *a, **kw: said.append(kw.get("prompt", False)) or decode(*a, **kw))
+    cfg = dataclasses.replace(dsa.named_config("glm5"), num_hidden_layers=1, first_k_dense_replace=0)
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        model = dsa.DSAModel(cfg).to(torch.bfloat16).eval()
+    model.prefill(model.init_decode(1, 128), torch.randn(1, 70, cfg.hidden_size, device="cuda").bfloat16())
+    assert said == [True]
 
 
 def test_two_rows_that_differ(ops):
