@@ -997,9 +997,14 @@ static int mla_form(int R, int rows_per_seq, int H, int topk_k, int nsplit, floa
     // splits each (us, pair / one CTA per 64 heads, 128 heads, the default split count): 16 rows x 2048 keys in 4 splits
     // 21.9 / 24.8, 32 in 2 32.7 / 41.1, 40 in 1 38.4 / 59.5, 200 x 1024 59.0 / 95.1, 40 x 512 15.8 / 19.6, 40 x 256 11.9 / 12.9,
     // 96 x 128 16.0 / 17.2. Not below, where the start and the end of a pair weigh as much as its products: 8 rows x 2048 in 8
-    // splits 16.8 / 16.9, 4 in 16 16.0 / 14.3, 16 x 1024 in 4 18.3 / 18.1, 32 x 512 in 2 21.5 / 21.5, 64 x 128 10.6 / 9.2.
+    // splits 16.8 / 16.9, 4 in 16 16.0 / 14.3, 16 x 1024 in 4 18.3 / 18.1, 32 x 512 in 2 21.5 / 21.5, 64 x 128 10.6 / 9.2. Nor
+    // splits of up to 64 keys, half a tile, unless there are more of them than SMs or two to four of a list: 75 rows x 64 16.3 / 14.9, 128
+    // 16.9 / 15.9, 150 20.9 / 22.4, 512 47.2 / 62.7; 10 x 512 in 8 21.9 / 19.9, 16 23.3 / 22.2, 19 24.4 / 29.8; 19 x 256 in 4 18.4 / 21.4,
+    // 40 x 128 in 2 24.1 / 25.7. (What a row sees of its list is not known here: rows of 40 keys in lists of 2048 take 11.2 / 8.4
+    // with 38 rows, 12.5 / 8.8 with 74 and 21.9 / 23.5 with 150; of 200 keys 12.7 / 13.0, 14.2 / 13.7 and 26.1 / 37.3.)
     const int64_t pair_items = int64_t(R) * (H / mla_pair::kHeads) * nsplit;
-    const bool pair_pays = kps >= (nsplit == 1 ? 2 : 4) * mla_pair::kBN || pair_items > sm_count() / 2;
+    const bool half_tiles = kps <= mla_pair::kBN / 2 && (nsplit == 1 || nsplit > 4);
+    const bool pair_pays = kps >= (nsplit == 1 ? 2 : 4) * mla_pair::kBN || pair_items > (half_tiles ? sm_count() : sm_count() / 2);
     if (H % mla_pair::kHeads == 0 && pair_pays) return DSA_MLA_PAIR;
     // Two rows of 64 heads on a pair for a prompt that is no longer than the list: neighbouring rows then attend the same keys
     // but one (us, pair / one CTA a row: prompts of 256 tokens 19.4 / 20.8, 700 61 / 82, 2048 320 / 465, two of 200 26.7 / 29.0;

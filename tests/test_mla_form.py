@@ -39,3 +39,12 @@ def test_rows_of_a_prompt(R, rows_per_seq, topk, cap, with_prompt, without):
     assert form(R, rows_per_seq, 64, topk, 1, cap, every | BESIDE) == TC
     assert form(R, rows_per_seq, 192, topk, 1, cap, every | PROMPT) == TC
     assert form(R, rows_per_seq, 64, topk, 1, cap, LIST | LENGTHS | PROMPT) == (TC if with_prompt == FIRST_ROWS else with_prompt)
+
+
+@pytest.mark.parametrize("R,H,topk,nsplit,want", [
+    (75, 128, 64, 1, TC), (148, 128, 40, 1, TC), (149, 128, 64, 1, PAIR), (512, 128, 64, 1, PAIR), (38, 256, 64, 1, TC), (16, 128, 512, 8, TC),
+    (19, 128, 512, 8, PAIR), (19, 128, 256, 4, PAIR), (18, 128, 256, 4, TC), (38, 128, 128, 2, PAIR), (75, 128, 65, 1, PAIR),
+    (74, 128, 65, 1, TC), (76, 128, 128, 1, PAIR), (38, 256, 128, 1, PAIR), (16, 128, 640, 8, PAIR)])
+def test_half_tiles_on_pairs(R, H, topk, nsplit, want):
+    for rows_per_seq in (1, R):
+        assert form(R, rows_per_seq, H, topk, nsplit, 4096) == want

@@ -67,7 +67,8 @@ def check(ops, q, kv, idx, lens, rows_per_seq, nsplit, **kw):
 # a pair of very different length
 @pytest.mark.parametrize("R,H,n,topk,nsplit,rows_per_seq", [
     (8, 128, 3000, 512, 1, 1), (8, 128, 700, 513, 1, 2), (8, 128, 600, 576, 1, 8), (4, 256, 900, 577, 1, 4), (8, 128, 700, 639, 1, 1),
-    (150, 128, 40, 40, 1, 150), (76, 128, 300, 64, 1, 76), (100, 128, 300, 129, 1, 100), (20, 512, 300, 200, 1, 1), (33, 128, 300, 256, 1, 1),
+    (150, 128, 40, 40, 1, 150), (76, 128, 300, 64, 1, 76), (150, 128, 40, 70, 1, 150), (76, 128, 300, 65, 1, 76),
+    (100, 128, 300, 129, 1, 100), (20, 512, 300, 200, 1, 1), (33, 128, 300, 256, 1, 1),
     (3, 128, 5000, 2048, 3, 1), (40, 128, 500, 129, 2, 1), (6, 384, 3000, 1100, 2, 3), (160, 128, 2100, 2048, 1, 160)])
 def test_against_64_bits(ops, R, H, n, topk, nsplit, rows_per_seq):
     q, kv, idx, lens = operands(R, H, n, topk, rows_per_seq, seed=R + topk)
