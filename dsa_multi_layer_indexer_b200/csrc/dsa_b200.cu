@@ -534,6 +534,13 @@ static int launch_topk_solo(const topk::Params& p, int R, int64_t n, cudaStream_
 }
 }  // extern "C++"
 
+// As few CTAs as hold the row at 32 logits per thread.
+static int topk_row_ctas(int64_t n) {
+  int ctas = 1;
+  while (ctas < topk::kClMaxCtasBig && int64_t(ctas) * topk::kClThreads * topk::kClMaxKeys < n) ctas *= 2;
+  return ctas;
+}
+
 static int launch_topk_cluster(const topk::Params& p, int R, int64_t n, cudaStream_t st) {
   // More rows than SMs: the cluster kernel holds one row per SM and would take several waves of its
   // latency-bound chain, the row kernel keeps several rows per SM in flight: four of up to 4096 logits, three of
@@ -545,13 +552,11 @@ static int launch_topk_cluster(const topk::Params& p, int R, int64_t n, cudaStre
     return launch_topk_rows(p, R, n, st);
   const bool plain = p.hist && !p.n_src && !p.n_dest && !p.index_map && !p.out_val;
   if (plain && n <= topk::kSoloMaxN) return p.page_table ? launch_topk_solo<true>(p, R, n, st) : launch_topk_solo<false>(p, R, n, st);
-  // As few CTAs as hold the row at 32 logits per thread: every CTA added costs cluster barriers and
-  // remote stores, and a row of up to 16384 logits needs none of either.
+  // Every CTA added costs cluster barriers and remote stores, and a row of up to 16384 logits needs none of either.
   // A row that comes without the scan's histogram counts its own first level with shared-memory
   // atomics, about one per cycle per SM: it is spread over as many SMs as the cluster has (2048 logits
   // per CTA or more).
-  int ctas = 1;
-  while (ctas < topk::kClMaxCtasBig && int64_t(ctas) * topk::kClThreads * topk::kClMaxKeys < n) ctas *= 2;
+  int ctas = topk_row_ctas(n);
   if (!p.hist)  // (as long as the launch still fits the device in one wave)
     while (ctas < topk::kClMaxCtas && int64_t(ctas) * 2048 < n && 2 * ctas * R <= sm_count()) ctas *= 2;
   const int64_t per_key = int64_t(ctas) * topk::kClThreads;
@@ -1005,7 +1010,20 @@ static int mla_form(int R, int rows_per_seq, int H, int topk_k, int nsplit, floa
     const int64_t pair_items = int64_t(R) * (H / mla_pair::kHeads) * nsplit;
     const bool half_tiles = kps <= mla_pair::kBN / 2 && (nsplit == 1 || nsplit > 4);
     const bool pair_pays = kps >= (nsplit == 1 ? 2 : 4) * mla_pair::kBN || pair_items > (half_tiles ? sm_count() : sm_count() / 2);
-    if (H % mla_pair::kHeads == 0 && pair_pays) return DSA_MLA_PAIR;
+    // Beside the top-k of the same rows, whose CTAs have the SMs first: a pair needs both SMs of a TPC at once. Where the pairs
+    // that are left no room wait for the top-k and CTAs of 64 heads would not, splits of four tiles or fewer go to those (lagged
+    // layer, us, pair / 64 heads: 16 rows x 2048 keys over 16K 37.7 / 34.1, 15 35.6 / 33.3, 12 over 40K 38.7 / 35.9, 28 x 1024 over 8K
+    // 39.6 / 35.9; both wait: 17 rows over 16K 38.8 / 40.5; splits of eight tiles: 28 x 2048 over 16K 51.0 / 54.3). The kernel for
+    // short rows is over too soon (16 rows over 4K 28.3 / 30.8). The rows' contexts are taken to be the cache's length, or their
+    // share of a pool that all rows read.
+    const int64_t ctx = R == rows_per_seq ? kv_seq_stride / R : kv_seq_stride;
+    bool pair_waits = false;
+    if ((flags & DSA_MLA_BESIDE) && kps <= 4 * mla_pair::kBN && ctx > topk::kSoloMaxN) {
+      const int ctas = topk_row_ctas(ctx);
+      const int64_t tpcs = std::max<int64_t>(R, int64_t(R) * ctas * 5 / 8);  // (a cluster of four has CTAs in two or three)
+      pair_waits = pair_items + tpcs > sm_count() / 2 && 2 * pair_items + int64_t(R) * ctas <= sm_count();
+    }
+    if (H % mla_pair::kHeads == 0 && pair_pays && !pair_waits) return DSA_MLA_PAIR;
     // Two rows of 64 heads on a pair for a prompt that is no longer than the list: neighbouring rows then attend the same keys
     // but one (us, pair / one CTA a row: prompts of 256 tokens 19.4 / 20.8, 700 61 / 82, 2048 320 / 465, two of 200 26.7 / 29.0;
     // 220 18.7 / 18.6, two of 150 23.8 / 23.7). Rows whose lists do not nest take half of a pair each, a third slower than one

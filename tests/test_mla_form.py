@@ -48,3 +48,14 @@ def test_rows_of_a_prompt(R, rows_per_seq, topk, cap, with_prompt, without):
 def test_half_tiles_on_pairs(R, H, topk, nsplit, want):
     for rows_per_seq in (1, R):
         assert form(R, rows_per_seq, H, topk, nsplit, 4096) == want
+
+
+@pytest.mark.parametrize("R,H,topk,nsplit,cap,want", [
+    (16, 128, 2048, 4, 16384, TC), (15, 128, 2048, 4, 8192, TC), (14, 128, 2048, 4, 16384, PAIR), (17, 128, 2048, 4, 16384, PAIR),
+    (11, 128, 2048, 4, 40000, PAIR), (7, 256, 2048, 4, 40000, PAIR), (12, 128, 2048, 4, 40000, TC), (10, 128, 2048, 4, 40000, PAIR), (13, 128, 2048, 4, 40000, PAIR),
+    (28, 128, 1024, 2, 8192, TC), (28, 128, 2048, 2, 16384, PAIR), (16, 256, 1024, 2, 8192, TC), (9, 256, 2048, 4, 8192, PAIR),
+    (75, 128, 2048, 1, 16384, PAIR), (200, 128, 512, 1, 16384, PAIR), (16, 128, 2048, 4, 4096, PAIR), (16, 128, 2048, 4, 4097, TC)])
+def test_pairs_beside_the_topk_need_room(R, H, topk, nsplit, cap, want):
+    for rows_per_seq, stride in ((1, cap), (R, cap * R)):  # a cache each, one pool
+        assert form(R, rows_per_seq, H, topk, nsplit, stride) == PAIR
+        assert form(R, rows_per_seq, H, topk, nsplit, stride, LIST | LENGTHS | BESIDE) == want
