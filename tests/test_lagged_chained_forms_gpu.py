@@ -16,22 +16,27 @@ SM = 192 ** -0.5
 
 
 @pytest.mark.parametrize("fp8", [False, True])
-@pytest.mark.parametrize("rows,heads,ctx,topk,nsplit", [
-    (1, 128, 20000, 2048, None),  # one tile per split: 16 heads per CTA, fp8 rows 32
-    (10, 32, 6000, 2048, None),   # 32 heads per CTA, three tiles per split
-    (80, 32, 3000, 256, 1),       # the same without partials, four tiles
-    (80, 32, 3000, 64, 1),        # one tile
-    (10, 48, 6000, 2048, None),   # 16 heads per CTA, two CTAs on an SM
-    (4, 128, 6000, 2048, None),   # tcgen05
-    (80, 64, 3000, 256, 1),       # tcgen05 without partials
+@pytest.mark.parametrize("rows,heads,ctx,topk,nsplit,forms", [  # (forms: over bf16 rows and fp8 rows)
+    (1, 128, 20000, 2048, None, (0, 2)),  # one tile per split: 16 heads per CTA, fp8 rows 32
+    (10, 32, 6000, 2048, None, (1, 1)),   # 32 heads per CTA, three tiles per split
+    (80, 32, 3000, 256, 1, (1, 1)),       # the same without partials, four tiles
+    (80, 32, 3000, 64, 1, (0, 2)),        # one tile
+    (10, 48, 6000, 2048, None, (0, 0)),   # 16 heads per CTA, two CTAs on an SM
+    (4, 128, 6000, 2048, None, (3, 3)),   # tcgen05
+    (80, 64, 3000, 256, 1, (3, 3)),       # tcgen05 without partials
+    (14, 128, 6000, 2048, None, (4, 3)),  # pairs of CTAs, bf16 rows
+    (80, 128, 3000, 256, 1, (4, 3)),      # the same without partials, two rows for some pairs
+    (40, 128, 3000, 256, 2, (4, 3)),      # the same, splits of one tile
 ])
-def test_beside_the_topk_equals_alone(rows, heads, ctx, topk, nsplit, fp8):
+def test_beside_the_topk_equals_alone(rows, heads, ctx, topk, nsplit, forms, fp8):
     from dsa_multi_layer_indexer_b200 import _lib, ops
     from dsa_multi_layer_indexer_b200.decode import HotPathState, LayerCache
 
     g = torch.Generator(device="cuda").manual_seed(rows + heads + topk)
     rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g)
     st = HotPathState(rows, heads, 64, ctx, topk, "cuda", nsplit=nsplit)
+    beside = 1 | 2 | 8  # a list, lengths, beside the kernel in front
+    assert _lib.lib().dsa_sparse_mla_form(rows, 1, heads, topk, st.nsplit, SM, ctx, fp8, beside) == forms[fp8]
     k8, ks = ops.quantize_e4m3_rowwise(rand(rows, ctx, 128))
     lat = rand(rows * ctx, 576)
     kv = O.pack_fp8_latent(lat.cpu()).cuda() if fp8 else lat.to(torch.bfloat16)

@@ -254,9 +254,8 @@ def test_a_prefill_says_that_its_rows_are_a_prompt(ops, monkeypatch):
     assert said == [True]
 
 
-def test_two_rows_that_differ(ops):
-    """Lists that do not nest, rows of which one or both see nothing, lengths that shrink: row by row then."""
-    n = 260
+def rows_that_differ(n):
+    """Lists that do not nest, rows of which one or both see nothing, lengths that shrink."""
     q, kv, idx, lens = prompt(1, n, 400, seed=4)
     gen = torch.Generator(device="cuda").manual_seed(5)
     for r in range(20, 60):                                    # unrelated lists
@@ -273,7 +272,70 @@ def test_two_rows_that_differ(ops):
     lens[85] = n
     idx[90, 10] = -1                                           # the first row misses one in the middle,
     idx[93, 10] = -1                                           # the second one does
-    check(ops, q, kv, idx, lens, n, 1)
+    return q, kv, idx, lens
+
+
+def test_two_rows_that_differ(ops):
+    check(ops, *rows_that_differ(260), 260, 1)
+
+
+@pytest.mark.parametrize("operands_of", [lambda: (*prompt(1, 257, 300, seed=3), 257), lambda: (*prompt(2, 193, 193, seed=4), 193),
+                                         lambda: (*rows_that_differ(260), 260), lambda: (*rows_that_differ(261), 261)])
+def test_two_rows_into_partials(ops, operands_of):
+    """The two-row form with a caller's scratch: of one split, the merge makes the same result of it bit for bit."""
+    from dsa_multi_layer_indexer_b200 import _lib
+
+    q, kv, idx, lens, rows_per_seq = operands_of()
+    R, cap = q.shape[0], kv.shape[1]
+    assert _lib.lib().dsa_sparse_mla_form(R, rows_per_seq, 64, idx.shape[1], 1, SM, cap, 0, 1 | 2) == 5
+    want = ops.sparse_mla_decode(q, kv, idx, SM, lens, rows_per_seq=rows_per_seq, nsplit=1)
+    scratch = ops.MlaScratch(R + 1, 64, 1, "cuda")
+    for t in (scratch.acc, scratch.m, scratch.l):
+        t.fill_(float("nan"))
+    kw = dict(rows_per_seq=rows_per_seq, nsplit=1, scratch=scratch)
+    ops.sparse_mla_decode(q, kv, idx, SM, lens, stage="partials", **kw)
+    _lib.check_device_status()
+    assert torch.isfinite(scratch.acc[:R]).all() and not torch.isnan(scratch.m[:R]).any() and torch.isfinite(scratch.l[:R]).all()
+    assert torch.isnan(scratch.acc[R]).all() and torch.isnan(scratch.m[R]).all() and torch.isnan(scratch.l[R]).all()
+    assert torch.equal(ops.sparse_mla_decode(q, kv, idx, SM, lens, stage="combine", **kw), want)
+    assert torch.equal(ops.sparse_mla_decode(q, kv, idx, SM, lens, **kw), want)
+
+
+def test_a_long_prompt_right_behind_its_selection(ops):
+    """Both launches of a prompt longer than its lists read what the kernel in front of them writes: the second one starts
+    without a wait of its own, behind the first one's. Replayed over changing logits."""
+    from dsa_multi_layer_indexer_b200 import _lib
+
+    n, topk = 900, 300
+    q, kv, _, lens = prompt(1, n, n, seed=21)
+    gen = torch.Generator(device="cuda").manual_seed(22)
+    logits = torch.zeros(n, n, device="cuda")
+    lists = torch.empty(n, topk, dtype=torch.int32, device="cuda")
+    out = torch.empty(n, 64, 512, dtype=torch.bfloat16, device="cuda")
+
+    def both():
+        ops.topk_select(logits, topk, lens, out_idx=lists)
+        ops.sparse_mla_decode(q, kv, lists, SM, lens, rows_per_seq=n, nsplit=1, out=out, prompt=True)
+
+    assert _lib.lib().dsa_sparse_mla_form(n, n, 64, topk, 1, SM, n, 0, 1 | 2 | 4 | 16) == 6
+    both()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(2):
+            both()
+    for _ in range(4):
+        logits.copy_(torch.randn(n, n, device="cuda", generator=gen))
+        ops.topk_select(logits, topk, lens, out_idx=lists)
+        torch.cuda.synchronize()
+        want = ops.sparse_mla_decode(q, kv, lists, SM, lens, rows_per_seq=n, nsplit=1, prompt=True)
+        torch.cuda.synchronize()
+        lists.fill_(-1)
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    _lib.check_device_status()
+    check(ops, q, kv, lists, lens, n, 1, prompt=True)
 
 
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
