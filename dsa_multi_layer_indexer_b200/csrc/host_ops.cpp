@@ -348,9 +348,10 @@ PyObject* topk_paged(PyObject* const* a) {
 }
 
 // ---------------------------------------------------------------- sparse MLA
-// The split count where a caller gives none. Head counts that are a multiple of 64 run on the tcgen05 kernel (one CTA
-// per SM, 64 heads per CTA) once the launch has 128 tiles of 64 heads x 64 keys: about one CTA per SM in total, and a
-// split count that divides the tiles so no split is empty. Smaller launches and other head counts run on the mma.sync
+// The split count where a caller gives none. Head counts that are a multiple of 64 run on the tcgen05 kernels once the launch
+// has 128 tiles of 64 heads x 64 keys: about one CTA per SM in total with 64 heads per CTA, and a split count that divides
+// the tiles so no split is empty. (128 heads over bf16 rows may run on persistent pairs of CTAs, for which other counts have not
+// been measured: 10-14, 19-28 and 38-56 rows of 2048 keys occupy half to three quarters of the pairs.) Smaller launches and other head counts run on the mma.sync
 // kernel: two CTAs of 16 heads per SM, or one of 32 where a split has several tiles or fp8 rows. With more (row, head) pairs than SMs at most 16 splits: the merge reads
 // every split's partials, and more of them cost more than the shorter splits save (2 rows x 128 heads: 12.8 us with 16
 // splits, 14.9 with 32).

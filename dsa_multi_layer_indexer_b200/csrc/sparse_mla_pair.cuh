@@ -12,10 +12,11 @@
 // The other 192 hold the first six chunks of Q, in both lane halves. One S buffer is enough: the score product of tile t + 1
 // is issued behind the value product of tile t - 1, by when the softmax has read S(t).
 //
-// What bounds it. The products of a tile take 2180 cycles (32 a piece at M 128 N 128 K 16, 68 at N 256, measured alone) and
-// their operands, the rows' 139 KB and P 2900 cycles of shared memory; a tile takes 2300 with a few pairs at work and 3000 -
-// 3400 with all of them, where the board's power limit also lowers the clock (1.6 GHz at 1000 W). 1024 rows of 128 heads x
-// 2048 keys 803 -> 495 us, 700 x 700 250 -> 155 us (one CTA per 64 heads / this kernel). What it took:
+// What bounds it. The products of a tile take 2280 cycles (36 of 32.6 at M 128 N 128 K 16 and 16 of 68.9 at N 256, each measured
+// alone). A tile takes 3300 - 3450 with up to 37 pairs at work and 3600 - 4000 with all 74 (times of 2048 and 4096 keys, at the
+// clock sampled meanwhile): the products wait for rows and probabilities, and with all pairs at work the board's power limit
+// also lowers the clock (1.6 GHz at 1000 W). 1024 rows of 128 heads x 2048 keys 803 -> 500 us, 700 x 700 250 -> 155 us (one CTA
+// per 64 heads / this kernel). What it took:
 //   * rows come by TMA row gathers (tile::gather4), four rows of one 64-dim chunk each. A gather costs a warp 35 - 60 cycles
 //     behind other gathers and 85 - 140 where it waits, looks something up or shuffles indices in between, so a warp issues
 //     eight in a row, from indices laid out in shared memory: 340 -> 270 cycles per 16 KB. (16-byte asynchronous copies with
@@ -25,7 +26,7 @@
 //   * one ring of 16 KB units in the order of use, keys of tile t + 1 before values of tile t. A place is loaded again about
 //     2400 cycles before it is needed, which the loads just meet: nine units and two S buffers 532, ten and one 514 us;
 //   * the softmax takes S into registers and gives its buffer back at once, since the next score product waits for it: given
-//     back behind the exponentials 523, now 503 us. The heads' maxima are compared only where one ran away;
+//     back behind the exponentials 523 us. The heads' maxima are compared only where one ran away;
 //   * the MMA warp tests all its barriers in one look (a wait per unit, ready or not, took 200 cycles: 589 -> 548 us);
 //   * arrivals at the other CTA's barriers without cluster scope (they order nothing but shared memory of the arriving CTA,
 //     whose proxy fence precedes them): 1400 cycles each, twice a tile, before: 794 -> 580 us;
@@ -369,7 +370,9 @@ sparse_mla_pair_kernel(const __grid_constant__ CUtensorMap kv_map, const __grid_
           float f = 1.f;
           const float m_first = fmaxf(s_max[head], s_max[64 + head]);
           const float m_tile = fmaxf(m_first, fmaxf(s_max[128 + head], s_max[192 + head]));
-          if (m_ref == -INFINITY) {  // the first 64 visible keys' maximum, as the kernel of one CTA has it: the same roundings of p
+          // The maximum of the first 64 places of the first tile with a visible key, as the kernel of one CTA has it where its
+          // first such tile is those 64: then the same roundings of p. The whole tile's where they are masked or it runs away.
+          if (m_ref == -INFINITY) {
             m_ref = m_first == -INFINITY || m_tile > m_first + kRescaleLog2 ? m_tile : m_first;
           } else if (m_tile > m_ref + kRescaleLog2) {
             f = exp2f(m_ref - m_tile);
