@@ -1005,10 +1005,11 @@ static int mla_form(int R, int rows_per_seq, int H, int topk_k, int nsplit, floa
     // splits 16.8 / 16.9, 4 in 16 16.0 / 14.3, 16 x 1024 in 4 18.3 / 18.1, 32 x 512 in 2 21.5 / 21.5, 64 x 128 10.6 / 9.2. Nor
     // splits of up to 64 keys, half a tile, unless there are more of them than SMs or two to four of a list: 75 rows x 64 16.3 / 14.9, 128
     // 16.9 / 15.9, 150 20.9 / 22.4, 512 47.2 / 62.7; 10 x 512 in 8 21.9 / 19.9, 16 23.3 / 22.2, 19 24.4 / 29.8; 19 x 256 in 4 18.4 / 21.4,
-    // 40 x 128 in 2 24.1 / 25.7. (What a row sees of its list is not known here: rows of 40 keys in lists of 2048 take 11.2 / 8.4
+    // 40 x 128 in 2 24.1 / 25.7. Of a prompt's rows the list holds half on average: 75 tokens 17.2 / 15.7, 100 17.5 / 16.8, 128 17.5 / 17.7, 150
+    // 22.8 / 24.6. (What a row sees of its list is not known here: rows of 40 keys in lists of 2048 take 11.2 / 8.4
     // with 38 rows, 12.5 / 8.8 with 74 and 21.9 / 23.5 with 150; of 200 keys 12.7 / 13.0, 14.2 / 13.7 and 26.1 / 37.3.)
     const int64_t pair_items = int64_t(R) * (H / mla_pair::kHeads) * nsplit;
-    const bool half_tiles = kps <= mla_pair::kBN / 2 && (nsplit == 1 || nsplit > 4);
+    const bool half_tiles = (flags & DSA_MLA_PROMPT ? kps / 2 : kps) <= mla_pair::kBN / 2 && (nsplit == 1 || nsplit > 4);
     const bool pair_pays = kps >= (nsplit == 1 ? 2 : 4) * mla_pair::kBN || pair_items > (half_tiles ? sm_count() : sm_count() / 2);
     // Beside the top-k of the same rows, whose CTAs have the SMs first: a pair needs both SMs of a TPC at once. Where the pairs
     // that are left no room wait for the top-k and CTAs of 64 heads would not, splits of four tiles or fewer go to those (lagged

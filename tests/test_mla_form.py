@@ -50,6 +50,12 @@ def test_half_tiles_on_pairs(R, H, topk, nsplit, want):
         assert form(R, rows_per_seq, H, topk, nsplit, 4096) == want
 
 
+@pytest.mark.parametrize("batch,n,H,want", [(1, 75, 128, TC), (1, 128, 128, TC), (1, 149, 128, PAIR), (2, 74, 128, TC), (2, 75, 128, PAIR),
+                                            (1, 74, 256, TC), (1, 75, 256, PAIR), (1, 700, 128, PAIR)])
+def test_short_prompts_are_half_tiles(batch, n, H, want):
+    assert form(batch * n, n, H, n, 1, n + 256, LIST | LENGTHS | DIRECT | PROMPT) == want
+
+
 @pytest.mark.parametrize("R,H,topk,nsplit,cap,want", [
     (16, 128, 2048, 4, 16384, TC), (15, 128, 2048, 4, 8192, TC), (14, 128, 2048, 4, 16384, PAIR), (17, 128, 2048, 4, 16384, PAIR),
     (11, 128, 2048, 4, 40000, PAIR), (7, 256, 2048, 4, 40000, PAIR), (12, 128, 2048, 4, 40000, TC), (10, 128, 2048, 4, 40000, PAIR), (13, 128, 2048, 4, 40000, PAIR),
